@@ -26,7 +26,7 @@ class GdnArgs(ctypes.Structure):
                 + [(n, I32) for n in ("B", "T", "Hk", "Hv", "dk", "dv", "n_seqs", "num_slots", "chunk", "max_seqlen")]
                 + [(f"{t}_stride_{d}", I64) for t in ("q", "k", "v", "z", "o") for d in ("b", "t", "h")]
                 + [("g_stride_b", I64), ("g_stride_t", I64), ("scale", F32), ("norm_eps", F32),
-                   ("o_peers", P), ("n_peers", I32), ("reserved1", I32)])
+                   ("o_peers", P), ("n_peers", I32), ("token_begin", I32)])
 
 
 class NormArgs(ctypes.Structure):
@@ -128,6 +128,27 @@ def load():
             raise ImportError("libave_gdn_b200.so has an unexpected ABI version")
         _LIB = lib
     return _LIB
+
+
+class _Host:
+    """The native host side (module ``_host``, csrc/host.cpp), loaded and bound to the C library at first use."""
+
+    def __getattr__(self, name):
+        path = lib_path()
+        load()
+        try:
+            from . import _host
+        except ImportError as e:
+            raise ImportError(f"avelang_b200._host cannot be loaded ({e}): run `python -m avelang_b200.build`; "
+                              "this package has no fallback implementation") from e
+        _host.bind(os.path.abspath(path))
+        for key in dir(_host):
+            if not key.startswith("__"):
+                self.__dict__[key] = getattr(_host, key)  # later calls find the function without coming here
+        return getattr(_host, name)
+
+
+host = _Host()
 
 
 def check(rc: int, what: str) -> None:

@@ -390,10 +390,11 @@ static int launch_prefill_t(const AveGdnArgs& a, cudaStream_t stream) {
     // the norm kernel indexes rows as (token, head); batches are folded in one launch per batch row
     for (int b = 0; b < a.B; ++b) {
       AveGdnNormArgs nb = na;
-      nb.rows = (int64_t)a.T * a.Hv;
-      nb.x = o_f32 + (int64_t)b * a.T * a.Hv * DV;
-      nb.z = reinterpret_cast<const __nv_bfloat16*>(a.z) + b * a.z_stride_b;
-      nb.y = reinterpret_cast<__nv_bfloat16*>(a.o) + b * a.o_stride_b;
+      const int64_t t0 = a.token_begin;  // 0 except in the prefill part of a mixed batch
+      nb.rows = ((int64_t)a.T - t0) * a.Hv;
+      nb.x = o_f32 + ((int64_t)b * a.T + t0) * a.Hv * DV;
+      nb.z = reinterpret_cast<const __nv_bfloat16*>(a.z) + b * a.z_stride_b + t0 * a.z_stride_t;
+      nb.y = reinterpret_cast<__nv_bfloat16*>(a.o) + b * a.o_stride_b + t0 * a.o_stride_t;
       nb.z_stride_t = a.z_stride_t; nb.z_stride_h = a.z_stride_h;
       nb.y_stride_t = a.o_stride_t; nb.y_stride_h = a.o_stride_h;
       const int rc = launch_gated_rmsnorm_f32in(nb, stream);

@@ -1751,7 +1751,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     AVE_CUDA_TRY(cudaGetLastError());
     if (a.z != nullptr) {
       // packed layouts: the norm covers every row (rows of later parts are rewritten by the fix-up, which runs after it)
-      const int rc = norm_rows(a, o_f32, 0, a.cu_seqlens ? a.T : part0_tokens, stream);
+      const int rc = norm_rows(a, o_f32, a.token_begin, a.cu_seqlens ? a.T : part0_tokens, stream);
       if (rc != AVE_GDN_OK) return rc;
     }
     return finish_parts(stream, nullptr, nullptr, nullptr);
@@ -1787,7 +1787,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     }
   }
   if (rc == AVE_GDN_OK) {
-    if (a.z != nullptr && !norm_per_range) rc = norm_rows(a, o_f32, 0, a.T, side->scan);  // packed layout: after the last scan
+    if (a.z != nullptr && !norm_per_range) rc = norm_rows(a, o_f32, a.token_begin, a.T, side->scan);  // packed layout: after the last scan
     if (rc == AVE_GDN_OK) rc = finish_parts(side->scan, side->prep, side->chains_done, side->combined);
   }
   step(cudaEventRecord(side->join, side->scan));

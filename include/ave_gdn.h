@@ -103,7 +103,8 @@ typedef struct AveGdnArgs {
    * the layout.  The caller orders the stores against the peers' readers (a barrier after the call). */
   const void* const* o_peers;
   int32_t n_peers;
-  int32_t reserved1;
+  int32_t token_begin; /* prefill, packed layout: the sequences start at this token (cu_seqlens[0]); rows before it belong to
+                          somebody else (the decode part of a mixed batch) and are not written */
 } AveGdnArgs;
 
 /* Chunked prefill (chunk 64, WY/UT form), dense [B,T] or packed varlen via cu_seqlens. */
