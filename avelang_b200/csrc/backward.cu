@@ -1,234 +1,949 @@
-// Backward pass of the gated delta rule (d_k = d_v = 128), token by token in reverse, fp32 on the CUDA cores.
+// Backward pass of the gated delta rule (d_k = d_v = 128), chunked (64 tokens), with fp32-level accuracy.
 //
-// Forward, per token (M is the key-major state [dk][dv], a = exp(g)):
-//     Mb = a M;   r = Mb^T k;   u = beta (v - r);   M' = Mb + k u^T;   o = scale M'^T q
-// Backward, given do and the gradient dM' that flows in from the future:
-//     dM' += scale q do^T;          dq = scale M' do
-//     du = dM'^T k;                 dk = dM' u + Mb dr        (dr = -beta du)
-//     dbeta = du . (v - r);         dv = beta du
-//     dMb = dM' + k dr^T;           dg = <dMb, Mb>;           dM = a dMb
-// so the reverse sweep needs Mb of every token.  One CTA walks one (sequence, value head): a forward sweep leaves the
-// state at every 64-token boundary in the checkpoint area; then, chunk by chunk from the end, the chunk's 64 Mb tiles
-// are recomputed from its checkpoint into a per-CTA scratch ring and consumed in reverse.  The state tile and its
-// gradient stay in registers (a warp owns 16 rows, a lane 4 columns); column reductions (r, du) cross warps through
-// shared memory, row reductions (dq, dk) are one 32-value butterfly per warp and token.
-// This is the correct-first form of the pass: every token costs a 64 KiB tile written and read back, and a handful of
-// CTA barriers; a chunked (WY) backward on the tensor cores is the faster successor.
+// Per chunk (M0 the state that enters it, b the in-chunk cumulative gate, G_ij = e^{b_i - b_j}, S the output scale):
+//     A = strict_lower(beta_i G_ij k_i.k_j)    T = (I + A)^-1      P = lower(G_ij q_i.k_j)      D_i = e^{b_C - b_i}
+//     Vn = T diag(beta) (V - diag(e^b) K M0)   O = S (diag(e^b) Q M0 + P Vn)    M1 = e^{b_C} M0 + K^T diag(D) Vn
+// and in reverse, with E the gradient of M1:
+//     dVn = S P^T dO + diag(D) K E             Ut = T^T dVn
+//     dM0 = e^{b_C} E + S Q^T diag(e^b) dO - K^T diag(beta e^b) Ut
+//     dV  = diag(beta) Ut
+//     dQ  = S diag(e^b) dO M0^T + X K          X = S lower(dO Vn^T) o G
+//     dK  = row + col,  row = Y K - diag(beta e^b) Ut M0^T,   col = Y^T K + X^T Q + diag(D) Vn E^T,
+//           Y = -diag(beta) strict_lower(Ut Vn^T) o G     (the gradient of A collapses to -strict_lower(Ut Vn^T))
+//     dbeta_i = Ut_i.v_i + (k_i.row_i) / beta_i
+//     db_i    = q_i.dq_i + k_i.row_i - k_i.col_i,  and  dg_t = sum_{i >= t} db_i + sum_j k_j.(D_j (Vn E^T)_j) + e^{b_C} <E, M0>
+//           (b_i rides on q_i and on the row side of k_i with a plus sign, on the column side of k_i with a minus sign).
+//
+// Four launches.  bwd_prep: T, P and b of every (chunk, value head), in parallel.  bwd_forward: the states and Vn, chunk
+// after chunk; bwd_reverse: the state gradients and Ut, chunk after chunk from the end (it needs nothing of bwd_forward).
+// bwd_grads: everything else, in parallel over (chunk, key head), summing over the value heads that share the key head.
+//
+// The contractions run on warp-level bf16 MMAs with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
+// every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with one fp32 operand is
+// three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which the gradient of
+// the gate needs, because it is a difference of large sums.
+// The scans hold the state transposed, H = M^T: a warp owns 16 of the 128 d_v rows for the whole sequence, every product
+// is (its rows) x (a tile all warps read), and the accumulator of one product is, in place, the left operand of the next,
+// so the warps of a chain never exchange anything and only meet where a tile buffer is refilled.
+// Two sequences of 4096 tokens, 32 value heads: 1.49 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.73)
+// against 22.1 ms for the token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
+#include "blockalg.cuh"
 #include "common.cuh"
+#include "tc.cuh"
 
 namespace ave {
 namespace {
 
-constexpr int BD = 128, BW = 8, BROWS = BD / BW, BCH = 64;  // head dim, warps, rows per warp, tokens per checkpoint
+constexpr int BD = 128, BCH = 64;
+constexpr int IMG = BCH * BCH * 2;              // one bf16 [64][64] tile
+constexpr int PREP_P = 3 * IMG, PREP_SC = 6 * IMG, SC_BYTES = 3 * BCH * 4, PREP_BYTES = PREP_SC + SC_BYTES;  // T h m l | P h m l | b | beta | b's low part
+constexpr int STATE_FLOATS = BD * BD, VEC_FLOATS = BD * BCH;
 
-struct Tok {
-  float alpha, beta;
-  float v4[4], do4[4];
+struct BwdScratch {
+  uint8_t* prep;   // [slots][Hv][PREP_BYTES]; the tiles are stored as the swizzled shared-memory images the scans read
+  float *m0, *e;   // [slots][Hv][d_v][d_k]: H = M0^T and E^T of every chunk
+  float *vn, *u;   // [slots][Hv][d_v][64 tokens]: Vn^T and Ut^T
 };
 
-__global__ void __launch_bounds__(256, 1) gdn_backward_kernel(const AveGdnBwdArgs a, int n_units) {
-  __shared__ __align__(16) float k_s[BD];
-  __shared__ __align__(16) float q_s[BD];
-  __shared__ __align__(16) float red[2][BW][BD];
-  __shared__ float red_g[BW];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int col = lane * 4, row0 = warp * BROWS;
-  const int r_heads = a.Hv / a.Hk;
-  float* ckpt = reinterpret_cast<float*>(a.workspace);
-  const int64_t ckpt_tiles = ((int64_t)a.B * a.T / BCH + a.n_seqs + 1) * a.Hv;
-  float* ring = ckpt + ckpt_tiles * (int64_t)(BD * BD) + (int64_t)blockIdx.x * BCH * (int64_t)(BD * BD);  // this CTA's 64 tiles
+// Chunk j of sequence n has record slot floor(first token of n / 64) + n + j: unique, needs no table, and the sequence of a
+// slot is found by bisection because the first slots of the sequences increase strictly.
+struct BwdChunk { int n, b, t0, len; bool ok; };
+__device__ __forceinline__ int64_t first_slot(const AveGdnBwdArgs& a, int n) {
+  return (a.cu_seqlens ? (int64_t)a.cu_seqlens[n] : (int64_t)n * a.T) / BCH + n;
+}
+__device__ __forceinline__ BwdChunk chunk_of_slot(const AveGdnBwdArgs& a, int64_t slot) {
+  int lo = 0, hi = a.n_seqs;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (first_slot(a, mid) <= slot) lo = mid; else hi = mid;
+  }
+  BwdChunk c{lo, 0, 0, 0, false};
+  const SeqSpan sp = seq_span(a.cu_seqlens, lo, a.T, nullptr);
+  const int64_t j = slot - first_slot(a, lo);
+  if (!sp.ok || j < 0 || j * BCH >= sp.len) return c;
+  c.b = sp.b; c.t0 = sp.t0 + (int)j * BCH; c.len = min(BCH, sp.len - (int)j * BCH); c.ok = true;
+  return c;
+}
 
-  for (int unit = blockIdx.x; unit < n_units; unit += gridDim.x) {
-    const int n = unit / a.Hv, h = unit % a.Hv, hk = h / r_heads;
-    const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
-    if (!sp.ok || sp.len == 0) {
-      if (sp.ok && a.d_initial_state != nullptr) {  // empty sequence: the state gradient passes through
-        const int64_t tile = ((int64_t)n * a.Hv + h) * (int64_t)(BD * BD);
-        for (int e = tid; e < BD * BD; e += 256) a.d_initial_state[tile + e] = a.d_final_state ? a.d_final_state[tile + e] : 0.f;
-      }
-      continue;
-    }
-    const int64_t tile = ((int64_t)n * a.Hv + h) * (int64_t)(BD * BD);
-    const __nv_bfloat16* q_base = reinterpret_cast<const __nv_bfloat16*>(a.q) + sp.b * a.q_stride_b + (int64_t)hk * a.q_stride_h;
-    const __nv_bfloat16* k_base = reinterpret_cast<const __nv_bfloat16*>(a.k) + sp.b * a.k_stride_b + (int64_t)hk * a.k_stride_h;
-    const __nv_bfloat16* v_base = reinterpret_cast<const __nv_bfloat16*>(a.v) + sp.b * a.v_stride_b + (int64_t)h * a.v_stride_h;
-    const __nv_bfloat16* do_base = reinterpret_cast<const __nv_bfloat16*>(a.d_o) + sp.b * a.do_stride_b + (int64_t)h * a.do_stride_h;
-    const float* g_base = a.g + sp.b * a.g_stride_b + h;
-    const float* beta_base = a.beta + sp.b * a.g_stride_b + h;
-    const int n_chunks = (sp.len + BCH - 1) / BCH;
-    auto ckpt_of = [&](int j) {  // unique per (sequence, chunk): chunks of later sequences get later indices
-      return ckpt + ((((int64_t)sp.b * a.T + sp.t0 + j * BCH) / BCH + n) * a.Hv + h) * (int64_t)(BD * BD);
-    };
-    // vectors of token `tok` into shared memory / registers; the caller synchronises
-    auto load_token = [&](int64_t tok, Tok& tk, bool need_q) {
-      if (tid < BD) k_s[tid] = bf2f(k_base[tok * a.k_stride_t + tid]);
-      else if (need_q) q_s[tid - BD] = bf2f(q_base[tok * a.q_stride_t + tid - BD]);
-      unpack_bf16x4(*reinterpret_cast<const uint2*>(v_base + tok * a.v_stride_t + col), tk.v4);
-      if (need_q) unpack_bf16x4(*reinterpret_cast<const uint2*>(do_base + tok * a.do_stride_t + col), tk.do4);
-      tk.alpha = __expf(g_base[tok * a.g_stride_t]);
-      tk.beta = beta_base[tok * a.g_stride_t];
-    };
-    // column reduction over the 128 rows of per-thread partials p (this thread's 16 rows): total per column, in all threads
-    auto col_reduce = [&](int which, const float (&p)[4], float (&out)[4]) {
-      *reinterpret_cast<float4*>(&red[which][warp][col]) = make_float4(p[0], p[1], p[2], p[3]);
-      __syncthreads();
-      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int w = 0; w < BW; ++w) {
-        const float4 x = *reinterpret_cast<const float4*>(&red[which][w][col]);
-        s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
-      }
-      out[0] = s.x; out[1] = s.y; out[2] = s.z; out[3] = s.w;
-    };
-    // one forward token on the state in registers: S <- Mb = a S (optionally stored), then S <- Mb + k u^T
-    float4 S[BROWS];
-    auto forward_token = [&](int64_t tok, float* store_mb) {
-      Tok tk;
-      __syncthreads();  // the shared vectors of the previous token are no longer read
-      load_token(tok, tk, false);
-      __syncthreads();
-      float p[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < BROWS; ++i) {
-        S[i].x *= tk.alpha; S[i].y *= tk.alpha; S[i].z *= tk.alpha; S[i].w *= tk.alpha;
-        if (store_mb != nullptr) *reinterpret_cast<float4*>(store_mb + (row0 + i) * BD + col) = S[i];
-        const float kr = k_s[row0 + i];
-        p[0] += S[i].x * kr; p[1] += S[i].y * kr; p[2] += S[i].z * kr; p[3] += S[i].w * kr;
-      }
-      float r[4];
-      col_reduce(0, p, r);
-      float u[4];
-#pragma unroll
-      for (int c = 0; c < 4; ++c) u[c] = tk.beta * (tk.v4[c] - r[c]);
-#pragma unroll
-      for (int i = 0; i < BROWS; ++i) {
-        const float kr = k_s[row0 + i];
-        S[i].x += kr * u[0]; S[i].y += kr * u[1]; S[i].z += kr * u[2]; S[i].w += kr * u[3];
-      }
-    };
+// ---------------------------------------------------------------------------------------------- warp MMA helpers
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// Tiles are stored in rows of ROWB bytes; the 16-byte piece c of row r sits at piece c ^ (r & 7).
+template <int ROWB>
+__device__ __forceinline__ uint32_t piece(int row, int c) { return (uint32_t)(row * ROWB + ((c ^ (row & 7)) << 4)); }
+// Lane addresses of the four ldmatrix patterns (r0, c0: first row and first 16-byte piece of the 16x16 block in the tile)
+template <int ROWB>  // left operand, tile rows = its rows
+__device__ __forceinline__ uint32_t at_a(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 15), c0 + (lane >> 4)); }
+template <int ROWB>  // left operand, tile rows = contraction index (with .trans)
+__device__ __forceinline__ uint32_t at_at(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
+template <int ROWB>  // right operand of two adjacent column tiles, tile rows = its columns
+__device__ __forceinline__ uint32_t at_b(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
+template <int ROWB>  // right operand of two adjacent column tiles, tile rows = contraction index (with .trans)
+__device__ __forceinline__ uint32_t at_bt(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 15), c0 + (lane >> 4)); }
 
-    // ---- forward sweep: checkpoints at every chunk boundary
-    {
-      const float* s0 = a.initial_state ? a.initial_state + tile : nullptr;
-#pragma unroll
-      for (int i = 0; i < BROWS; ++i)
-        S[i] = s0 ? *reinterpret_cast<const float4*>(s0 + (row0 + i) * BD + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-      for (int j = 0; j < n_chunks; ++j) {
-        float* dst = ckpt_of(j);
-#pragma unroll
-        for (int i = 0; i < BROWS; ++i) *reinterpret_cast<float4*>(dst + (row0 + i) * BD + col) = S[i];
-        if (j == n_chunks - 1) break;  // the last chunk is recomputed below anyway
-        for (int t = 0; t < BCH; ++t) forward_token(sp.t0 + j * BCH + t, nullptr);
-      }
-    }
+// e^{b_i - b_j} for i >= j (at most 1 elsewhere); sc: b[64] | beta[64] | low part of b[64]
+__device__ __forceinline__ float gate_between(const float* sc, int i, int j) {
+  return __expf(fminf((sc[i] - sc[j]) + (sc[2 * BCH + i] - sc[2 * BCH + j]), 0.f));
+}
 
-    // ---- reverse sweep
-    float4 dM[BROWS];
-    {
-      const float* ds = a.d_final_state ? a.d_final_state + tile : nullptr;
+// x = h + m + l in bf16, exact to 24 bits
+__device__ __forceinline__ void split3(float2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
+  const float2 m1 = make_float2(-1.f, -1.f);
+  h = pack_bf16x2(x.x, x.y);
+  const float2 r = __ffma2_rn(bf16x2_to_float2(h), m1, x);
+  m = pack_bf16x2(r.x, r.y);
+  const float2 s = __ffma2_rn(bf16x2_to_float2(m), m1, r);
+  l = pack_bf16x2(s.x, s.y);
+}
+// two adjacent accumulator tiles (columns 0..15) -> left operand of a product over those columns, three terms
+__device__ __forceinline__ void split_acc(const float (&c0)[4], const float (&c1)[4], uint32_t (&h)[4], uint32_t (&m)[4], uint32_t (&l)[4]) {
+  split3(make_float2(c0[0], c0[1]), h[0], m[0], l[0]);
+  split3(make_float2(c0[2], c0[3]), h[1], m[1], l[1]);
+  split3(make_float2(c1[0], c1[1]), h[2], m[2], l[2]);
+  split3(make_float2(c1[2], c1[3]), h[3], m[3], l[3]);
+}
+// d += (h + m + l) * b with b exact
+__device__ __forceinline__ void mma3(float (&d)[4], const uint32_t (&h)[4], const uint32_t (&m)[4], const uint32_t (&l)[4], uint32_t b0, uint32_t b1) {
+  mma_bf16(d, h, b0, b1);
+  mma_bf16(d, m, b0, b1);
+  mma_bf16(d, l, b0, b1);
+}
+// d += (ah + am + al) (bh + bm + bl), the terms below 2^-24 left out
+__device__ __forceinline__ void mma6(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
+                                     uint32_t bh0, uint32_t bh1, uint32_t bm0, uint32_t bm1, uint32_t bl0, uint32_t bl1) {
+  mma_bf16(d, ah, bh0, bh1);
+  mma_bf16(d, ah, bm0, bm1);
+  mma_bf16(d, am, bh0, bh1);
+  mma_bf16(d, ah, bl0, bl1);
+  mma_bf16(d, al, bh0, bh1);
+  mma_bf16(d, am, bm0, bm1);
+}
+__device__ __forceinline__ void zero(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
+
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
+  const int bytes = valid ? 16 : 0;  // the rest of the 16 bytes is zero-filled
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+// `rows` x `PIECES` 16-byte pieces of a strided bf16 matrix into a tile; rows from `len` on are zero
+template <int PIECES, int THREADS>
+__device__ __forceinline__ void load_tile(uint32_t dst, const __nv_bfloat16* src, int64_t stride, int len, int tid) {
 #pragma unroll
-      for (int i = 0; i < BROWS; ++i)
-        dM[i] = ds ? *reinterpret_cast<const float4*>(ds + (row0 + i) * BD + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i = 0; i < BCH * PIECES / THREADS; ++i) {
+    const int e = tid + i * THREADS, row = e / PIECES, c = e % PIECES;
+    cp16(dst + piece<PIECES * 16>(row, c), src + (int64_t)(row < len ? row : 0) * stride + c * 8, row < len);
+  }
+}
+template <int BYTES, int THREADS>
+__device__ __forceinline__ void load_flat(uint32_t dst, const uint8_t* src, int tid) {
+#pragma unroll
+  for (int i = 0; i < (BYTES / 16 + THREADS - 1) / THREADS; ++i) {
+    const int e = tid + i * THREADS;
+    if (BYTES / 16 % THREADS == 0 || e < BYTES / 16) cp16(dst + e * 16, src + e * 16, true);
+  }
+}
+__device__ __forceinline__ const __nv_bfloat16* bf(const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); }
+
+// ---------------------------------------------------------------------------------------------- T, P and b of every chunk
+constexpr int PREP_T = 256;
+constexpr int PR_K = 0, PR_Q = 16384, PR_A = 32768, PR_D = PR_A + 10 * BLK_FLOATS * 4, PR_E = PR_D + 4 * BLK_FLOATS * 4,
+              PR_SC = PR_E + 10 * BLK_FLOATS * 4, PR_SMEM = PR_SC + SC_BYTES;
+
+__global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  float* Ab = reinterpret_cast<float*>(smem + PR_A);
+  float* Di = reinterpret_cast<float*>(smem + PR_D);
+  float* Eb = reinterpret_cast<float*>(smem + PR_E);
+  float* E2b = Eb + 6 * BLK_FLOATS;
+  float* E3b = E2b + 3 * BLK_FLOATS;
+  float* bs = reinterpret_cast<float*>(smem + PR_SC);
+  float* betas = bs + BCH;
+  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const BwdChunk c = chunk_of_slot(a, blockIdx.x);
+  if (!c.ok) return;
+  const int hk = h / (a.Hv / a.Hk);
+  uint8_t* rec = ws.prep + ((int64_t)blockIdx.x * a.Hv + h) * PREP_BYTES;
+  const uint32_t sb = tc::smem_u32(smem);
+  load_tile<16, PREP_T>(sb + PR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
+  load_tile<16, PREP_T>(sb + PR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
+  cp_commit();
+  if (warp == 0) {  // inclusive scan of the gates; beyond the end of the sequence b stays and beta is 0
+    // b reaches hundreds while e^{b_i - b_j} of near tokens matters: it is summed in double and kept as two floats, so that
+    // the differences are as exact as the gates themselves
+    const int64_t off = c.b * a.g_stride_b + (int64_t)c.t0 * a.g_stride_t + h;
+    double v0 = lane < c.len ? a.g[off + lane * a.g_stride_t] : 0.f, v1 = lane + 32 < c.len ? a.g[off + (lane + 32) * a.g_stride_t] : 0.f;
+    const float be0 = lane < c.len ? a.beta[off + lane * a.g_stride_t] : 0.f, be1 = lane + 32 < c.len ? a.beta[off + (lane + 32) * a.g_stride_t] : 0.f;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double t0 = __shfl_up_sync(0xffffffffu, v0, o), t1 = __shfl_up_sync(0xffffffffu, v1, o);
+      if (lane >= o) { v0 += t0; v1 += t1; }
     }
-    for (int j = n_chunks - 1; j >= 0; --j) {
-      const int len = min(BCH, sp.len - j * BCH);
-      const float* src = ckpt_of(j);
+    v1 += __shfl_sync(0xffffffffu, v0, 31);
+    float* sc = reinterpret_cast<float*>(rec + PREP_SC);
+    const float h0 = (float)v0, h1 = (float)v1, l0 = (float)(v0 - h0), l1 = (float)(v1 - h1);
+    bs[lane] = sc[lane] = h0; bs[lane + 32] = sc[lane + 32] = h1;
+    betas[lane] = sc[BCH + lane] = be0; betas[lane + 32] = sc[BCH + lane + 32] = be1;
+    bs[2 * BCH + lane] = sc[2 * BCH + lane] = l0; bs[2 * BCH + lane + 32] = sc[2 * BCH + lane + 32] = l1;
+  }
+  cp_wait<0>();
+  __syncthreads();
+  {  // warps 0..3: rows 16m.. of K K^T -> A;  warps 4..7: rows 16m.. of Q K^T -> P.  Blocks above the diagonal are skipped.
+    const int m = warp & 3, g = lane >> 2, t = lane & 3;
+    const bool is_p = warp >= 4;
+    float acc[8][4];
 #pragma unroll
-      for (int i = 0; i < BROWS; ++i) S[i] = *reinterpret_cast<const float4*>(src + (row0 + i) * BD + col);
-      for (int t = 0; t < len; ++t) forward_token(sp.t0 + j * BCH + t, ring + (int64_t)t * (BD * BD));
-      // every thread re-reads only the tile elements it wrote itself, so no fence is needed around the ring
-      for (int t = len - 1; t >= 0; --t) {
-        const int64_t tok = sp.t0 + j * BCH + t;
-        const float* mb = ring + (int64_t)t * (BD * BD);
-        Tok tk;
-        __syncthreads();
-        load_token(tok, tk, true);
+    for (int i = 0; i < 8; ++i) zero(acc[i]);
 #pragma unroll
-        for (int i = 0; i < BROWS; ++i) S[i] = *reinterpret_cast<const float4*>(mb + (row0 + i) * BD + col);  // Mb of this token
-        __syncthreads();
-        // r = Mb^T k, u = beta (v - r)
-        float p[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int ks = 0; ks < 8; ++ks) {
+      uint32_t af[4];
+      ldsm4(af, sb + (is_p ? PR_Q : PR_K) + at_a<256>(16 * m, 2 * ks, lane));
 #pragma unroll
-        for (int i = 0; i < BROWS; ++i) {
-          const float kr = k_s[row0 + i];
-          p[0] += S[i].x * kr; p[1] += S[i].y * kr; p[2] += S[i].z * kr; p[3] += S[i].w * kr;
-        }
-        float r[4], u[4], vr[4];
-        col_reduce(0, p, r);
+      for (int np = 0; np < 4; ++np) {
+        if (np > m) break;
+        uint32_t b[4];
+        ldsm4(b, sb + PR_K + at_b<256>(16 * np, 2 * ks, lane));
+        mma_bf16(acc[2 * np], af, b[0], b[1]);
+        mma_bf16(acc[2 * np + 1], af, b[2], b[3]);
+      }
+    }
 #pragma unroll
-        for (int c = 0; c < 4; ++c) { vr[c] = tk.v4[c] - r[c]; u[c] = tk.beta * vr[c]; }
-        // dM' += scale q do^T;  rows of dq = scale M' do and the first half of dk = dM' u;  du = dM'^T k
-        float rowv[32];
-        float pu[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int nt = 0; nt < 8; ++nt) {
 #pragma unroll
-        for (int i = 0; i < BROWS; ++i) {
-          const float kr = k_s[row0 + i], qs = a.scale * q_s[row0 + i];
-          dM[i].x += qs * tk.do4[0]; dM[i].y += qs * tk.do4[1]; dM[i].z += qs * tk.do4[2]; dM[i].w += qs * tk.do4[3];
-          const float m0 = S[i].x + kr * u[0], m1 = S[i].y + kr * u[1], m2 = S[i].z + kr * u[2], m3 = S[i].w + kr * u[3];
-          rowv[i] = a.scale * (m0 * tk.do4[0] + m1 * tk.do4[1] + m2 * tk.do4[2] + m3 * tk.do4[3]);
-          rowv[16 + i] = dM[i].x * u[0] + dM[i].y * u[1] + dM[i].z * u[2] + dM[i].w * u[3];
-          pu[0] += dM[i].x * kr; pu[1] += dM[i].y * kr; pu[2] += dM[i].z * kr; pu[3] += dM[i].w * kr;
-        }
-        float du[4], dr[4];
-        col_reduce(1, pu, du);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) dr[c] = -tk.beta * du[c];
-        // dMb = dM' + k dr^T;  second half of dk = Mb dr;  dg = <dMb, Mb>;  dM = a dMb
-        float gpart = 0.f;
-#pragma unroll
-        for (int i = 0; i < BROWS; ++i) {
-          const float kr = k_s[row0 + i];
-          rowv[16 + i] += S[i].x * dr[0] + S[i].y * dr[1] + S[i].z * dr[2] + S[i].w * dr[3];
-          dM[i].x += kr * dr[0]; dM[i].y += kr * dr[1]; dM[i].z += kr * dr[2]; dM[i].w += kr * dr[3];
-          gpart += dM[i].x * S[i].x + dM[i].y * S[i].y + dM[i].z * S[i].z + dM[i].w * S[i].w;
-          dM[i].x *= tk.alpha; dM[i].y *= tk.alpha; dM[i].z *= tk.alpha; dM[i].w *= tk.alpha;
-        }
-        const float rowsum = reduce32(rowv, lane);  // lanes 0..15: dq of rows row0 + lane; lanes 16..31: dk of rows row0 + lane - 16
-        const int64_t kq_off = (((int64_t)sp.b * a.T + tok) * a.Hv + h) * BD + row0 + (lane & 15);
-        if (lane < 16) a.d_q[kq_off] = rowsum; else a.d_k[kq_off] = rowsum;
-        gpart = warp_sum(gpart);
-        if (lane == 0) red_g[warp] = gpart;
-        if (warp == 0) {  // every warp holds every column once; warp 0 writes the per-column and per-token results
-          float db = du[0] * vr[0] + du[1] * vr[1] + du[2] * vr[2] + du[3] * vr[3];
-          db = warp_sum(db);
-          const int64_t v_off = (((int64_t)sp.b * a.T + tok) * a.Hv + h) * BD + col;
-          *reinterpret_cast<float4*>(a.d_v + v_off) = make_float4(tk.beta * du[0], tk.beta * du[1], tk.beta * du[2], tk.beta * du[3]);
-          if (lane == 0) a.d_beta[((int64_t)sp.b * a.T + tok) * a.Hv + h] = db;
-        }
-        __syncthreads();
-        if (tid == 0) {
-          float gs = 0.f;
-#pragma unroll
-          for (int w = 0; w < BW; ++w) gs += red_g[w];
-          a.d_g[((int64_t)sp.b * a.T + tok) * a.Hv + h] = gs;
+      for (int half = 0; half < 2; ++half) {
+        const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
+        const float x0 = gate_between(bs, i, j) * acc[nt][2 * half], x1 = gate_between(bs, i, j + 1) * acc[nt][2 * half + 1];
+        if (is_p) {
+          uint32_t ph, pm, pl;
+          split3(make_float2(i >= j ? x0 : 0.f, i > j ? x1 : 0.f), ph, pm, pl);
+          uint8_t* dst = rec + PREP_P + piece<128>(i, nt) + 4 * t;
+          *reinterpret_cast<uint32_t*>(dst) = ph;
+          *reinterpret_cast<uint32_t*>(dst + IMG) = pm;
+          *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = pl;
+        } else if (nt <= 2 * m + 1) {
+          const float be = betas[i];
+          *reinterpret_cast<float2*>(Ab + tri(m, nt >> 1) * BLK_FLOATS + (i & 15) * BLK_LD + (j & 15)) =
+              make_float2(i > j ? be * x0 : 0.f, i > j + 1 ? be * x1 : 0.f);
         }
       }
     }
-    if (a.d_initial_state != nullptr) {
-      float* dst = a.d_initial_state + tile;
+  }
+  __syncthreads();
+  // T = (I + A)^-1 by 16x16 blocks, as in the forward pass: D = blockdiag(I + A_rr), E = D^-1 (A - A_D),
+  // T = (I - E + E^2 - E^3) D^-1
+  if (tid < 64) {
+    const int r = tid >> 4, k = tid & 15;
+    const float* Arr = Ab + tri(r, r) * BLK_FLOATS;
+    float x[16];
 #pragma unroll
-      for (int i = 0; i < BROWS; ++i) *reinterpret_cast<float4*>(dst + (row0 + i) * BD + col) = dM[i];
+    for (int i = 0; i < 16; ++i) {
+      float s0 = (i == k) ? 1.f : 0.f, s1 = 0.f;
+#pragma unroll
+      for (int j = 0; j < i; ++j) {
+        const float av = Arr[i * BLK_LD + j];
+        if (j & 1) s1 = fmaf(-av, x[j], s1); else s0 = fmaf(-av, x[j], s0);
+      }
+      x[i] = s0 + s1;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) Di[r * BLK_FLOATS + i * BLK_LD + k] = x[i];
+  }
+  __syncthreads();
+  constexpr int RR[6] = {1, 2, 2, 3, 3, 3}, CC[6] = {0, 0, 1, 0, 1, 2};
+  auto Eblk = [&](int r, int cc) { return Eb + (tri(r, cc) - r) * BLK_FLOATS; };
+  auto plain = [](const float* L) { return [L](int row, int col) { return L[row * BLK_LD + col]; }; };
+  if (warp < 6) {
+    const int r = RR[warp], cc = CC[warp];
+    float acc[2][4] = {};
+    block_mma(acc, plain(Di + r * BLK_FLOATS), Ab + tri(r, cc) * BLK_FLOATS, lane);
+    block_store(Eblk(r, cc), acc, lane);
+  }
+  __syncthreads();
+  if (warp < 3) {  // E^2: (2,0), (3,1), (3,0)
+    float acc[2][4] = {};
+    if (warp == 0) block_mma(acc, plain(Eblk(2, 1)), Eblk(1, 0), lane);
+    else if (warp == 1) block_mma(acc, plain(Eblk(3, 2)), Eblk(2, 1), lane);
+    else { block_mma(acc, plain(Eblk(3, 1)), Eblk(1, 0), lane); block_mma(acc, plain(Eblk(3, 2)), Eblk(2, 0), lane); }
+    block_store(E2b + warp * BLK_FLOATS, acc, lane);
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float acc[2][4] = {};
+    block_mma(acc, plain(Eblk(3, 2)), E2b, lane);
+    block_store(E3b, acc, lane);
+  }
+  __syncthreads();
+  if (warp < 6) {
+    const int r = RR[warp], cc = CC[warp];
+    const float* e1 = Eblk(r, cc);
+    const float* e2 = (r - cc >= 2) ? E2b + ((r == 2) ? 0 : (cc == 1 ? 1 : 2)) * BLK_FLOATS : nullptr;
+    const float* e3 = (r - cc == 3) ? E3b : nullptr;
+    float acc[2][4] = {};
+    block_mma(acc, [&](int row, int col) {
+      float v = -e1[row * BLK_LD + col];
+      if (e2 != nullptr) v += e2[row * BLK_LD + col];
+      if (e3 != nullptr) v -= e3[row * BLK_LD + col];
+      return v;
+    }, Di + cc * BLK_FLOATS, lane);
+    block_store(Ab + tri(r, cc) * BLK_FLOATS, acc, lane);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int it = 0; it < 2; ++it) {
+    const int i = (tid >> 3) + 32 * it, rb = i >> 4, pc = tid & 7, cb = pc >> 1;
+    uint32_t th[4] = {}, tm[4] = {}, tl[4] = {};
+    if (cb <= rb) {
+      const float* src = ((rb == cb) ? Di + rb * BLK_FLOATS : Ab + tri(rb, cb) * BLK_FLOATS) + (i & 15) * BLK_LD + (pc & 1) * 8;
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const int j = 8 * pc + 2 * w;
+        split3(make_float2(j <= i ? src[2 * w] : 0.f, j + 1 <= i ? src[2 * w + 1] : 0.f), th[w], tm[w], tl[w]);
+      }
+    }
+    uint8_t* dst = rec + piece<128>(i, pc);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(th[0], th[1], th[2], th[3]);
+    *reinterpret_cast<uint4*>(dst + IMG) = make_uint4(tm[0], tm[1], tm[2], tm[3]);
+    *reinterpret_cast<uint4*>(dst + 2 * IMG) = make_uint4(tl[0], tl[1], tl[2], tl[3]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- the two scans
+// One CTA of four warps per (sequence, value head, half of d_v): a warp owns 16 rows of the transposed state.
+constexpr int SC_T = 128;
+constexpr int FW_K = 0, FW_V = 16384, FW_TI = FW_V + 8192, FW_SC = FW_TI + 3 * IMG, FW_STAGE = FW_SC + SC_BYTES;
+constexpr int RV_K = 0, RV_Q = 16384, RV_DO = 32768, RV_TI = RV_DO + 8192, RV_PI = RV_TI + 3 * IMG, RV_SC = RV_PI + 3 * IMG,
+              RV_STAGE = RV_SC + SC_BYTES;
+
+struct ScanUnit { SeqSpan sp; int n, h, hk, row0; int64_t slot0, tile; };
+__device__ __forceinline__ ScanUnit scan_unit(const AveGdnBwdArgs& a, int block, int warp) {
+  ScanUnit u;
+  const int unit = block >> 1;
+  u.n = unit / a.Hv; u.h = unit % a.Hv; u.hk = u.h / (a.Hv / a.Hk);
+  u.row0 = (block & 1) * 64 + warp * 16;
+  u.sp = seq_span(a.cu_seqlens, u.n, a.T, a.status);
+  u.slot0 = u.sp.ok ? first_slot(a, u.n) : 0;
+  u.tile = ((int64_t)u.n * a.Hv + u.h) * STATE_FLOATS;
+  return u;
+}
+// rows row0 + g (+ 8), columns 8 nt + 2 t (+ 1) of the transposed state <-> a key-major [d_k][d_v] state in memory
+__device__ __forceinline__ void load_state(float (&H)[16][4], const float* src, int row0, int lane) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) H[nt][e] = src != nullptr ? src[(int64_t)(8 * nt + 2 * t + (e & 1)) * BD + row0 + g + 8 * (e >> 1)] : 0.f;
+}
+__device__ __forceinline__ void store_rows(float* dst, const float (&H)[16][4], int lane) {  // dst: first of this warp's rows, [d_v][d_k]
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < 16; ++nt) {
+    *reinterpret_cast<float2*>(dst + g * BD + 8 * nt + 2 * t) = make_float2(H[nt][0], H[nt][1]);
+    *reinterpret_cast<float2*>(dst + (g + 8) * BD + 8 * nt + 2 * t) = make_float2(H[nt][2], H[nt][3]);
+  }
+}
+__device__ __forceinline__ void store_vec(float* dst, const float (&v)[8][4], int lane) {  // [d_v][64 tokens]
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) {
+    *reinterpret_cast<float2*>(dst + g * BCH + 8 * nt + 2 * t) = make_float2(v[nt][0], v[nt][1]);
+    *reinterpret_cast<float2*>(dst + (g + 8) * BCH + 8 * nt + 2 * t) = make_float2(v[nt][2], v[nt][3]);
+  }
+}
+// acc[16 rows][64 tokens] = H K^T, K a [64][128] tile
+__device__ __forceinline__ void state_times_kt(float (&acc)[8][4], const float (&H)[16][4], uint32_t k_tile, int lane) {
+#pragma unroll
+  for (int nt = 0; nt < 8; ++nt) zero(acc[nt]);
+#pragma unroll
+  for (int ks = 0; ks < 8; ++ks) {
+    uint32_t ah[4], am[4], al[4];
+    split_acc(H[2 * ks], H[2 * ks + 1], ah, am, al);
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {
+      uint32_t b[4];
+      ldsm4(b, k_tile + at_b<256>(16 * np, 2 * ks, lane));
+      mma3(acc[2 * np], ah, am, al, b[0], b[1]);
+      mma3(acc[2 * np + 1], ah, am, al, b[2], b[3]);
+    }
+  }
+}
+// H[16 rows][128] += X[16 rows][64 tokens] K, K a [64][128] tile
+__device__ __forceinline__ void add_times_k(float (&H)[16][4], const float (&X)[8][4], uint32_t k_tile, int lane) {
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) {
+    uint32_t ah[4], am[4], al[4];
+    split_acc(X[2 * ks], X[2 * ks + 1], ah, am, al);
+#pragma unroll
+    for (int np = 0; np < 8; ++np) {
+      uint32_t b[4];
+      ldsm4t(b, k_tile + at_bt<256>(16 * ks, 2 * np, lane));
+      mma3(H[2 * np], ah, am, al, b[0], b[1]);
+      mma3(H[2 * np + 1], ah, am, al, b[2], b[3]);
     }
   }
 }
 
-int backward_grid(const AveGdnBwdArgs& a) {
-  const int64_t units = (int64_t)a.n_seqs * a.Hv;
-  return (int)(units < 148 ? units : 148);
+__global__ void __launch_bounds__(SC_T, 2) bwd_forward_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = lane & 3;
+  const ScanUnit u = scan_unit(a, blockIdx.x, warp);
+  if (!u.sp.ok || u.sp.len == 0) return;
+  const int n_chunks = (u.sp.len + BCH - 1) / BCH;
+  const __nv_bfloat16* kp = bf(a.k) + u.sp.b * a.k_stride_b + (int64_t)u.sp.t0 * a.k_stride_t + u.hk * a.k_stride_h;
+  const __nv_bfloat16* vp = bf(a.v) + u.sp.b * a.v_stride_b + (int64_t)u.sp.t0 * a.v_stride_t + u.h * a.v_stride_h + (blockIdx.x & 1) * 64;
+  const uint32_t sb = tc::smem_u32(smem);
+  auto load = [&](int c) {
+    const uint32_t st = sb + (c & 1) * FW_STAGE;
+    const int len = min(BCH, u.sp.len - c * BCH);
+    const uint8_t* rec = ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES;
+    load_tile<16, SC_T>(st + FW_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
+    load_tile<8, SC_T>(st + FW_V, vp + (int64_t)c * BCH * a.v_stride_t, a.v_stride_t, len, tid);
+    load_flat<3 * IMG, SC_T>(st + FW_TI, rec, tid);
+    load_flat<SC_BYTES, SC_T>(st + FW_SC, rec + PREP_SC, tid);
+  };
+  load(0);
+  cp_commit();
+  float H[16][4];
+  load_state(H, a.initial_state ? a.initial_state + u.tile : nullptr, u.row0, lane);
+  for (int c = 0; c < n_chunks; ++c) {
+    if (c + 1 < n_chunks) load(c + 1);
+    cp_commit();
+    cp_wait<1>();
+    __syncthreads();
+    const uint32_t st = sb + (c & 1) * FW_STAGE;
+    const float* bs = reinterpret_cast<const float*>(smem + (c & 1) * FW_STAGE + FW_SC);
+    const float* betas = bs + BCH;
+    const int64_t rec = (u.slot0 + c) * a.Hv + u.h;
+    store_rows(ws.m0 + rec * STATE_FLOATS + (int64_t)u.row0 * BD, H, lane);
+    float x[8][4], vn[8][4];
+    state_times_kt(x, H, st + FW_K, lane);
+#pragma unroll
+    for (int np = 0; np < 4; ++np) {  // X^T = beta (V^T - e^b (K M0)^T)
+      uint32_t v[4];
+      ldsm4t(v, st + FW_V + piece<128>(16 * np + (lane & 7) + ((lane >> 4) << 3), (u.row0 & 63) / 8 + ((lane >> 3) & 1)));
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int nt = 2 * np + e;
+        const float2 b = *reinterpret_cast<const float2*>(bs + 8 * nt + 2 * t), be = *reinterpret_cast<const float2*>(betas + 8 * nt + 2 * t);
+        const float e0 = __expf(b.x), e1 = __expf(b.y);
+        const float2 v0 = bf16x2_to_float2(v[2 * e]), v1 = bf16x2_to_float2(v[2 * e + 1]);
+        x[nt][0] = be.x * (v0.x - e0 * x[nt][0]); x[nt][1] = be.y * (v0.y - e1 * x[nt][1]);
+        x[nt][2] = be.x * (v1.x - e0 * x[nt][2]); x[nt][3] = be.y * (v1.y - e1 * x[nt][3]);
+      }
+    }
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) zero(vn[nt]);
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {  // Vn^T = X^T T^T
+      uint32_t ah[4], am[4], al[4];
+      split_acc(x[2 * ks], x[2 * ks + 1], ah, am, al);
+#pragma unroll
+      for (int np = ks; np < 4; ++np) {
+        uint32_t th[4], tm[4], tl[4];
+        const uint32_t at = st + FW_TI + at_b<128>(16 * np, 2 * ks, lane);
+        ldsm4(th, at); ldsm4(tm, at + IMG); ldsm4(tl, at + 2 * IMG);
+        mma6(vn[2 * np], ah, am, al, th[0], th[1], tm[0], tm[1], tl[0], tl[1]);
+        mma6(vn[2 * np + 1], ah, am, al, th[2], th[3], tm[2], tm[3], tl[2], tl[3]);
+      }
+    }
+    store_vec(ws.vn + rec * VEC_FLOATS + u.row0 * BCH, vn, lane);
+    if (c + 1 == n_chunks) break;
+    const float bC = bs[BCH - 1], decay = __expf(bC);
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float d0 = gate_between(bs, BCH - 1, 8 * nt + 2 * t), d1 = gate_between(bs, BCH - 1, 8 * nt + 2 * t + 1);
+      vn[nt][0] *= d0; vn[nt][1] *= d1; vn[nt][2] *= d0; vn[nt][3] *= d1;
+    }
+#pragma unroll
+    for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) H[nt][e] *= decay;
+    add_times_k(H, vn, st + FW_K, lane);
+    __syncthreads();  // every warp is done with this stage before it is refilled
+  }
+}
+
+__global__ void __launch_bounds__(SC_T, 1) bwd_reverse_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const ScanUnit u = scan_unit(a, blockIdx.x, warp);
+  if (!u.sp.ok) return;
+  if (u.sp.len == 0) {  // empty sequence: the state gradient passes through
+    if (a.d_initial_state != nullptr)
+      for (int e = tid + (blockIdx.x & 1) * (STATE_FLOATS / 2); e < ((int)(blockIdx.x & 1) + 1) * (STATE_FLOATS / 2); e += SC_T)
+        a.d_initial_state[u.tile + e] = a.d_final_state ? a.d_final_state[u.tile + e] : 0.f;
+    return;
+  }
+  const int n_chunks = (u.sp.len + BCH - 1) / BCH;
+  const __nv_bfloat16* kp = bf(a.k) + u.sp.b * a.k_stride_b + (int64_t)u.sp.t0 * a.k_stride_t + u.hk * a.k_stride_h;
+  const __nv_bfloat16* qp = bf(a.q) + u.sp.b * a.q_stride_b + (int64_t)u.sp.t0 * a.q_stride_t + u.hk * a.q_stride_h;
+  const __nv_bfloat16* dop = bf(a.d_o) + u.sp.b * a.do_stride_b + (int64_t)u.sp.t0 * a.do_stride_t + u.h * a.do_stride_h + (blockIdx.x & 1) * 64;
+  const uint32_t sb = tc::smem_u32(smem);
+  auto load = [&](int c) {
+    const uint32_t st = sb + (c & 1) * RV_STAGE;
+    const int len = min(BCH, u.sp.len - c * BCH);
+    load_tile<16, SC_T>(st + RV_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
+    load_tile<16, SC_T>(st + RV_Q, qp + (int64_t)c * BCH * a.q_stride_t, a.q_stride_t, len, tid);
+    load_tile<8, SC_T>(st + RV_DO, dop + (int64_t)c * BCH * a.do_stride_t, a.do_stride_t, len, tid);
+    load_flat<PREP_BYTES, SC_T>(st + RV_TI, ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES, tid);
+  };
+  load(n_chunks - 1);
+  cp_commit();
+  float E[16][4];
+  load_state(E, a.d_final_state ? a.d_final_state + u.tile : nullptr, u.row0, lane);
+  for (int c = n_chunks - 1; c >= 0; --c) {
+    if (c > 0) load(c - 1);
+    cp_commit();
+    cp_wait<1>();
+    __syncthreads();
+    const uint32_t st = sb + (c & 1) * RV_STAGE;
+    const float* bs = reinterpret_cast<const float*>(smem + (c & 1) * RV_STAGE + RV_SC);
+    const float* betas = bs + BCH;
+    const int64_t rec = (u.slot0 + c) * a.Hv + u.h;
+    store_rows(ws.e + rec * STATE_FLOATS + (int64_t)u.row0 * BD, E, lane);
+    const float bC = bs[BCH - 1], decay = __expf(bC);
+    float x[8][4], ut[8][4];
+    state_times_kt(x, E, st + RV_K, lane);
+    // x = dVn^T = D (E^T K^T) + S (dO^T P)
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float d0 = gate_between(bs, BCH - 1, 8 * nt + 2 * t), d1 = gate_between(bs, BCH - 1, 8 * nt + 2 * t + 1);
+      x[nt][0] *= d0; x[nt][1] *= d1; x[nt][2] *= d0; x[nt][3] *= d1;
+      zero(ut[nt]);
+    }
+    uint32_t doa[4][4];  // dO^T, this warp's rows x 64 tokens
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) ldsm4t(doa[ks], st + RV_DO + at_at<128>(16 * ks, (u.row0 & 63) / 8, lane));
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks)
+#pragma unroll
+      for (int np = 0; np <= ks; ++np) {
+        const uint32_t at = st + RV_PI + at_bt<128>(16 * ks, 2 * np, lane);
+#pragma unroll
+        for (int term = 0; term < 3; ++term) {
+          uint32_t b[4];
+          ldsm4t(b, at + term * IMG);
+          mma_bf16(ut[2 * np], doa[ks], b[0], b[1]);
+          mma_bf16(ut[2 * np + 1], doa[ks], b[2], b[3]);
+        }
+      }
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[nt][e] = fmaf(a.scale, ut[nt][e], x[nt][e]);
+      zero(ut[nt]);
+    }
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {  // Ut^T = dVn^T T
+      uint32_t ah[4], am[4], al[4];
+      split_acc(x[2 * ks], x[2 * ks + 1], ah, am, al);
+#pragma unroll
+      for (int np = 0; np <= ks; ++np) {
+        uint32_t th[4], tm[4], tl[4];
+        const uint32_t at = st + RV_TI + at_bt<128>(16 * ks, 2 * np, lane);
+        ldsm4t(th, at); ldsm4t(tm, at + IMG); ldsm4t(tl, at + 2 * IMG);
+        mma6(ut[2 * np], ah, am, al, th[0], th[1], tm[0], tm[1], tl[0], tl[1]);
+        mma6(ut[2 * np + 1], ah, am, al, th[2], th[3], tm[2], tm[3], tl[2], tl[3]);
+      }
+    }
+    store_vec(ws.u + rec * VEC_FLOATS + u.row0 * BCH, ut, lane);
+    if (c == 0 && a.d_initial_state == nullptr) break;
+    // E <- e^{b_C} E + (S e^b dO)^T Q - (beta e^b Ut)^T K
+#pragma unroll
+    for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) E[nt][e] *= decay;
+#pragma unroll
+    for (int nt = 0; nt < 8; ++nt) {
+      const float2 b = *reinterpret_cast<const float2*>(bs + 8 * nt + 2 * t), be = *reinterpret_cast<const float2*>(betas + 8 * nt + 2 * t);
+      const float f0 = __expf(b.x), f1 = __expf(b.y);
+      const float2 o0 = bf16x2_to_float2(doa[nt >> 1][2 * (nt & 1)]), o1 = bf16x2_to_float2(doa[nt >> 1][2 * (nt & 1) + 1]);
+      const float s0 = a.scale * f0, s1 = a.scale * f1;
+      x[nt][0] = s0 * o0.x; x[nt][1] = s1 * o0.y; x[nt][2] = s0 * o1.x; x[nt][3] = s1 * o1.y;
+      const float u0 = -be.x * f0, u1 = -be.y * f1;
+      ut[nt][0] *= u0; ut[nt][1] *= u1; ut[nt][2] *= u0; ut[nt][3] *= u1;
+    }
+    add_times_k(E, x, st + RV_Q, lane);
+    add_times_k(E, ut, st + RV_K, lane);
+    __syncthreads();
+  }
+  if (a.d_initial_state != nullptr) {
+    float* dst = a.d_initial_state + u.tile;
+#pragma unroll
+    for (int nt = 0; nt < 16; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) dst[(int64_t)(8 * nt + 2 * t + (e & 1)) * BD + u.row0 + g + 8 * (e >> 1)] = E[nt][e];
+  }
+}
+
+// ---------------------------------------------------------------------------------------------- the gradients of one chunk
+// 16 warps; a warp owns 32 tokens x 16 d_k columns of dQ and dK.  M0 and E, each element used by exactly one warp column
+// (two warps), go from global memory straight into right-operand registers; everything several warps read is a tile.
+constexpr int GR_T = 512;
+constexpr int GR_K = 0, GR_Q = 16384, GR_DO = 32768, GR_VN = 49152, GR_U = GR_VN + 3 * 16384, GR_X = GR_U + 3 * 16384,
+              GR_Y = GR_X + 3 * IMG, GR_RED = GR_Y + 3 * IMG, GR_SC = GR_RED + 8 * BCH * 20, GR_SMEM = GR_SC + SC_BYTES + 64;
+
+// fp32 [128][64] -> three bf16 tiles of 128-byte rows
+__device__ __forceinline__ void split_tile(uint8_t* dst, const float* src, int tid) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int e = tid + i * GR_T, row = e >> 4, q4 = e & 15;
+    const float4 x = __ldcs(reinterpret_cast<const float4*>(src + row * BCH + 4 * q4));
+    uint32_t h[2], m[2], l[2];
+    split3(make_float2(x.x, x.y), h[0], m[0], l[0]);
+    split3(make_float2(x.z, x.w), h[1], m[1], l[1]);
+    uint8_t* p = dst + piece<128>(row, q4 >> 1) + 8 * (q4 & 1);
+    *reinterpret_cast<uint2*>(p) = make_uint2(h[0], h[1]);
+    *reinterpret_cast<uint2*>(p + 16384) = make_uint2(m[0], m[1]);
+    *reinterpret_cast<uint2*>(p + 32768) = make_uint2(l[0], l[1]);
+  }
+}
+__device__ __forceinline__ float quad_sum(float x) {
+  x += __shfl_xor_sync(0xffffffffu, x, 1);
+  return x + __shfl_xor_sync(0xffffffffu, x, 2);
+}
+// per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16
+template <bool kSum>
+__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const BwdChunk& c, int head, int tok, int col, float x, float y) {
+  if (tok >= c.len) return;
+  const int64_t row = (int64_t)c.b * a.T + c.t0 + tok;
+  if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(dst) + (row * a.Hk + head) * BD + col) = pack_bf16x2(x, y);
+  else *reinterpret_cast<float2*>(dst + (row * a.Hv + head) * BD + col) = make_float2(x, y);
+}
+
+template <bool kSum>
+__global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int hk = blockIdx.y, r = a.Hv / a.Hk;
+  const int64_t slot = blockIdx.x;
+  const BwdChunk c = chunk_of_slot(a, slot);
+  if (!c.ok) return;
+  const uint32_t sb = tc::smem_u32(smem);
+  float* red = reinterpret_cast<float*>(smem + GR_RED);  // [8 column blocks][64 tokens][q.dq, k.row, k.col, k.state, u.v]
+  float* bs = reinterpret_cast<float*>(smem + GR_SC);
+  float* betas = bs + BCH;
+  float* dots = bs + 3 * BCH;  // [8] partial <E, M0>, then [8] the carry of the suffix sum
+  const int wm = warp & 1, wn = warp >> 1;  // token half, 16-column block
+  const int64_t row0 = (int64_t)c.b * a.T + c.t0;
+
+  load_tile<16, GR_T>(sb + GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
+  load_tile<16, GR_T>(sb + GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
+  float dq[2][2][4], dk[2][2][4];  // [16-token tile][8-column tile], summed over the value heads
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) { zero(dq[i][j]); zero(dk[i][j]); }
+
+#pragma unroll 1
+  for (int hh = 0; hh < r; ++hh) {
+    const int h = hk * r + hh;
+    const int64_t rec = slot * a.Hv + h;
+    if (hh > 0) __syncthreads();  // the tiles and sums of the previous head are no longer read
+    load_tile<16, GR_T>(sb + GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t, c.len, tid);
+    cp_commit();
+    split_tile(smem + GR_VN, ws.vn + rec * VEC_FLOATS, tid);
+    split_tile(smem + GR_U, ws.u + rec * VEC_FLOATS, tid);
+    if (tid < 3 * BCH) bs[tid] = reinterpret_cast<const float*>(ws.prep + rec * PREP_BYTES + PREP_SC)[tid];
+    cp_wait<0>();
+    __syncthreads();
+
+    {  // X = S lower(dO Vn^T) o G and Y = -beta strict_lower(Ut Vn^T) o G: warp = (16-row tile, column tiles nq and nq + 4)
+      const int m = warp >> 2, nq = warp & 3, last = 2 * m + 1;
+      if (nq <= last) {
+        float ax[2][4], ay[2][4];
+        zero(ax[0]); zero(ax[1]); zero(ay[0]); zero(ay[1]);
+        const bool two = nq + 4 <= last;
+#pragma unroll 2
+        for (int ks = 0; ks < 8; ++ks) {
+          uint32_t o[4], uh[4], um[4], ul[4], vh[4], vm[4], vl[4];
+          ldsm4(o, sb + GR_DO + at_a<256>(16 * m, 2 * ks, lane));
+          const uint32_t ua = sb + GR_U + at_at<128>(16 * ks, 2 * m, lane);
+          ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
+          const uint32_t va = sb + GR_VN + piece<128>(16 * ks + (lane & 15), nq + 4 * (lane >> 4));
+          ldsm4t(vh, va); ldsm4t(vm, va + 16384); ldsm4t(vl, va + 32768);
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            if (e == 1 && !two) break;
+            mma_bf16(ax[e], o, vh[2 * e], vh[2 * e + 1]);
+            mma_bf16(ax[e], o, vm[2 * e], vm[2 * e + 1]);
+            mma_bf16(ax[e], o, vl[2 * e], vl[2 * e + 1]);
+            mma6(ay[e], uh, um, ul, vh[2 * e], vh[2 * e + 1], vm[2 * e], vm[2 * e + 1], vl[2 * e], vl[2 * e + 1]);
+          }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (e == 1 && !two) break;
+          const int nt = nq + 4 * e;
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
+            const float e0 = gate_between(bs, i, j), e1 = gate_between(bs, i, j + 1);
+            const float be = -(fabsf(betas[i]) < 1e-20f ? 1e-20f : betas[i]);
+            uint32_t xh, xm, xl;
+            uint8_t* dst = smem + GR_X + piece<128>(i, nt) + 4 * t;
+            split3(make_float2(i >= j ? a.scale * e0 * ax[e][2 * half] : 0.f, i > j ? a.scale * e1 * ax[e][2 * half + 1] : 0.f), xh, xm, xl);
+            *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
+            dst += GR_Y - GR_X;
+            split3(make_float2(i > j ? be * e0 * ay[e][2 * half] : 0.f, i > j + 1 ? be * e1 * ay[e][2 * half + 1] : 0.f), xh, xm, xl);
+            *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
+          }
+        }
+      }
+    }
+    {  // dV = beta Ut and the row sums of Ut o V: this warp's 16 d_v columns and 32 tokens
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt) {
+        uint32_t uh[4], um[4], ul[4];
+        const uint32_t ua = sb + GR_U + at_at<128>(16 * wn, 4 * wm + 2 * mt, lane);
+        ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int tok = 32 * wm + 16 * mt + g + 8 * half;
+          float s = 0.f;
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const int idx = half + 2 * kk, col = 16 * wn + 8 * kk + 2 * t;
+            const float2 x = bf16x2_to_float2(uh[idx]), y = bf16x2_to_float2(um[idx]), z = bf16x2_to_float2(ul[idx]);
+            const float2 ut = make_float2(x.x + (y.x + z.x), x.y + (y.y + z.y));
+            if (tok < c.len) {
+              const float2 v = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(bf(a.v) + c.b * a.v_stride_b + (int64_t)(c.t0 + tok) * a.v_stride_t + h * a.v_stride_h + col));
+              s = fmaf(ut.x, v.x, fmaf(ut.y, v.y, s));
+              const float be = betas[tok];
+              if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.d_v) + ((row0 + tok) * a.Hv + h) * BD + col) = pack_bf16x2(be * ut.x, be * ut.y);
+              else *reinterpret_cast<float2*>(a.d_v + ((row0 + tok) * a.Hv + h) * BD + col) = make_float2(be * ut.x, be * ut.y);
+            }
+          }
+          s = quad_sum(s);
+          if (t == 0) red[(wn * BCH + tok) * 5 + 4] = s;
+        }
+      }
+    }
+    // dO M0^T, Ut M0^T, Vn E^T over d_v
+    float qa[2][2][4], ra[2][2][4], sa[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) { zero(qa[i][j]); zero(ra[i][j]); zero(sa[i][j]); }
+    float dot = 0.f;
+    {
+      // right-operand element (k = 16 ks + 2 t (+1, +8, +9), column 16 wn + 8 nt + g)
+      const float* hp = ws.m0 + rec * STATE_FLOATS + 2 * t * BD + 16 * wn + g;
+      const float* ep = ws.e + rec * STATE_FLOATS + 2 * t * BD + 16 * wn + g;
+      float hx[8], ex[8];
+      auto fetch = [&](int ks) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int off = (16 * ks + (e & 1) + 8 * ((e >> 1) & 1)) * BD + 8 * (e >> 2);
+          hx[e] = __ldcs(hp + off);
+          ex[e] = __ldcs(ep + off);
+        }
+      };
+      fetch(0);
+#pragma unroll 1
+      for (int ks = 0; ks < 8; ++ks) {
+        uint32_t hh_[4], hm[4], hl[4], eh[4], em[4], el[4];  // [column tile][b0, b1]
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          split3(make_float2(hx[2 * e], hx[2 * e + 1]), hh_[e], hm[e], hl[e]);
+          split3(make_float2(ex[2 * e], ex[2 * e + 1]), eh[e], em[e], el[e]);
+          dot = fmaf(hx[2 * e], ex[2 * e], fmaf(hx[2 * e + 1], ex[2 * e + 1], dot));
+        }
+        if (ks < 7) fetch(ks + 1);
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+          const int m0 = 32 * wm + 16 * mt;
+          uint32_t x[4], y[4], z[4];
+          ldsm4(x, sb + GR_DO + at_a<256>(m0, 2 * ks, lane));
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            mma_bf16(qa[mt][nt], x, hh_[2 * nt], hh_[2 * nt + 1]);
+            mma_bf16(qa[mt][nt], x, hm[2 * nt], hm[2 * nt + 1]);
+            mma_bf16(qa[mt][nt], x, hl[2 * nt], hl[2 * nt + 1]);
+          }
+          const uint32_t ua = sb + GR_U + at_at<128>(16 * ks, m0 >> 3, lane);
+          ldsm4t(x, ua); ldsm4t(y, ua + 16384); ldsm4t(z, ua + 32768);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+            mma6(ra[mt][nt], x, y, z, hh_[2 * nt], hh_[2 * nt + 1], hm[2 * nt], hm[2 * nt + 1], hl[2 * nt], hl[2 * nt + 1]);
+          const uint32_t va = ua - (GR_U - GR_VN);
+          ldsm4t(x, va); ldsm4t(y, va + 16384); ldsm4t(z, va + 32768);
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt)
+            mma6(sa[mt][nt], x, y, z, eh[2 * nt], eh[2 * nt + 1], em[2 * nt], em[2 * nt + 1], el[2 * nt], el[2 * nt + 1]);
+        }
+      }
+    }
+    dot = warp_sum(dot);
+    if (lane == 0 && wm == 0) dots[wn] = dot;
+    __syncthreads();  // X and Y are complete
+    const float bC = bs[BCH - 1];
+#pragma unroll
+    for (int mt = 0; mt < 2; ++mt) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int tok = 32 * wm + 16 * mt + g + 8 * half;
+        const float eb = __expf(bs[tok]), fq = a.scale * eb, fd = gate_between(bs, BCH - 1, tok);
+        const float be = fabsf(betas[tok]) < 1e-20f ? 1e-20f : betas[tok], fr = -be * eb;
+        float st = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          float* q4 = qa[mt][nt] + 2 * half; float* r4 = ra[mt][nt] + 2 * half; float* s4 = sa[mt][nt] + 2 * half;
+          q4[0] *= fq; q4[1] *= fq; r4[0] *= fr; r4[1] *= fr; s4[0] *= fd; s4[1] *= fd;
+          const float2 k = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_K + piece<256>(tok, 2 * wn + nt) + 4 * t));
+          st = fmaf(k.x, s4[0], fmaf(k.y, s4[1], st));
+        }
+        st = quad_sum(st);
+        if (t == 0) red[(wn * BCH + tok) * 5 + 3] = st;
+      }
+      const int m = 2 * wm + mt;  // 16-token tile
+#pragma unroll 1
+      for (int ks = 0; ks <= m; ++ks) {  // rows of tile m need the tokens up to it
+        uint32_t kb[4], x[4], y[4], z[4];
+        ldsm4t(kb, sb + GR_K + at_bt<256>(16 * ks, 2 * wn, lane));
+        const uint32_t xa = sb + GR_X + at_a<128>(16 * m, 2 * ks, lane);
+        ldsm4(x, xa); ldsm4(y, xa + IMG); ldsm4(z, xa + 2 * IMG);
+        mma3(qa[mt][0], x, y, z, kb[0], kb[1]);
+        mma3(qa[mt][1], x, y, z, kb[2], kb[3]);
+        const uint32_t ya = xa + (GR_Y - GR_X);
+        ldsm4(x, ya); ldsm4(y, ya + IMG); ldsm4(z, ya + 2 * IMG);
+        mma3(ra[mt][0], x, y, z, kb[0], kb[1]);
+        mma3(ra[mt][1], x, y, z, kb[2], kb[3]);
+      }
+#pragma unroll 1
+      for (int ks = m; ks < 4; ++ks) {  // columns of tile m take from the tokens from it on
+        uint32_t kb[4], qb[4], x[4], y[4], z[4];
+        ldsm4t(kb, sb + GR_K + at_bt<256>(16 * ks, 2 * wn, lane));
+        ldsm4t(qb, sb + GR_Q + at_bt<256>(16 * ks, 2 * wn, lane));
+        const uint32_t xa = sb + GR_X + at_at<128>(16 * ks, 2 * m, lane);
+        ldsm4t(x, xa); ldsm4t(y, xa + IMG); ldsm4t(z, xa + 2 * IMG);
+        mma3(sa[mt][0], x, y, z, qb[0], qb[1]);
+        mma3(sa[mt][1], x, y, z, qb[2], qb[3]);
+        const uint32_t ya = xa + (GR_Y - GR_X);
+        ldsm4t(x, ya); ldsm4t(y, ya + IMG); ldsm4t(z, ya + 2 * IMG);
+        mma3(sa[mt][0], x, y, z, kb[0], kb[1]);
+        mma3(sa[mt][1], x, y, z, kb[2], kb[3]);
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int tok = 32 * wm + 16 * mt + g + 8 * half;
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int nt = 0; nt < 2; ++nt) {
+          const uint32_t off = piece<256>(tok, 2 * wn + nt) + 4 * t;
+          const float2 k = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_K + off));
+          const float2 q = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_Q + off));
+          const float* q4 = qa[mt][nt] + 2 * half; const float* r4 = ra[mt][nt] + 2 * half; const float* s4 = sa[mt][nt] + 2 * half;
+          s0 = fmaf(q.x, q4[0], fmaf(q.y, q4[1], s0));
+          s1 = fmaf(k.x, r4[0], fmaf(k.y, r4[1], s1));
+          s2 = fmaf(k.x, s4[0], fmaf(k.y, s4[1], s2));
+          dq[mt][nt][2 * half] += q4[0]; dq[mt][nt][2 * half + 1] += q4[1];
+          dk[mt][nt][2 * half] += r4[0] + s4[0]; dk[mt][nt][2 * half + 1] += r4[1] + s4[1];
+        }
+        s0 = quad_sum(s0); s1 = quad_sum(s1); s2 = quad_sum(s2);
+        if (t == 0) {
+          float* dst = red + (wn * BCH + tok) * 5;
+          dst[0] = s0; dst[1] = s1; dst[2] = s2;
+        }
+        if (!kSum || hh == r - 1) {
+#pragma unroll
+          for (int nt = 0; nt < 2; ++nt) {
+            const int col = 16 * wn + 8 * nt + 2 * t;
+            float* q4 = dq[mt][nt] + 2 * half; float* k4 = dk[mt][nt] + 2 * half;
+            store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok, col, q4[0], q4[1]);
+            store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok, col, k4[0], k4[1]);
+            if (!kSum) q4[0] = q4[1] = k4[0] = k4[1] = 0.f;
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (tid < BCH) {  // dbeta, and dg as a suffix sum of db
+      float s[5] = {};
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+#pragma unroll
+        for (int e = 0; e < 5; ++e) s[e] += red[(w * BCH + tid) * 5 + e];
+      const float be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
+      const int64_t off = (row0 + tid) * a.Hv + h;
+      if (tid < c.len) a.d_beta[off] = s[4] + s[1] / be;
+      float db = s[0] + s[1] - s[2];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float x = __shfl_down_sync(0xffffffffu, db, o);
+        if (lane + o < 32) db += x;
+      }
+      const float st = warp_sum(s[3]);
+      if (lane == 0) { dots[8 + 2 * warp] = db; dots[9 + 2 * warp] = st; }
+      asm volatile("bar.sync 1, 64;" ::: "memory");
+      float em = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) em += dots[w];
+      if (warp == 0) db += dots[10];
+      if (tid < c.len) a.d_g[off] = db + (dots[9] + dots[11]) + __expf(bC) * em;
+    }
+  }
+}
+
+int64_t backward_slots(const AveGdnBwdArgs& a) { return (int64_t)a.B * a.T / BCH + a.n_seqs + 1; }
+
+BwdScratch scratch_layout(const AveGdnBwdArgs& a, size_t* total) {
+  const size_t recs = (size_t)backward_slots(a) * a.Hv;
+  uint8_t* p = reinterpret_cast<uint8_t*>(a.workspace);
+  BwdScratch ws;
+  size_t off = 0;
+  auto take = [&](size_t bytes) { uint8_t* q = p + off; off += (bytes + 255) & ~(size_t)255; return q; };
+  ws.prep = take(recs * PREP_BYTES);
+  ws.m0 = reinterpret_cast<float*>(take(recs * STATE_FLOATS * 4));
+  ws.e = reinterpret_cast<float*>(take(recs * STATE_FLOATS * 4));
+  ws.vn = reinterpret_cast<float*>(take(recs * VEC_FLOATS * 4));
+  ws.u = reinterpret_cast<float*>(take(recs * VEC_FLOATS * 4));
+  if (total != nullptr) *total = off;
+  return ws;
 }
 
 }  // namespace
 
 size_t backward_workspace_bytes(const AveGdnBwdArgs& a) {
-  const size_t tile = (size_t)BD * BD * 4;
-  const size_t ckpt = ((size_t)a.B * a.T / BCH + (size_t)a.n_seqs + 1) * (size_t)a.Hv * tile;
-  return ckpt + (size_t)backward_grid(a) * BCH * tile;
+  size_t total = 0;
+  scratch_layout(a, &total);
+  return total;
 }
 
 int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
   const int units = a.n_seqs * a.Hv;
   if (units == 0 || a.T == 0) return AVE_GDN_OK;
-  gdn_backward_kernel<<<backward_grid(a), 256, 0, stream>>>(a, units);
+  static bool attr_set_dev[64] = {};
+  int dev = 0;
+  AVE_CUDA_TRY(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) return AVE_GDN_UNSUPPORTED;
+  if (!attr_set_dev[dev]) {
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * FW_STAGE));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * RV_STAGE));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_grads_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_grads_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
+    attr_set_dev[dev] = true;  // repeating the calls from another thread is harmless
+  }
+  const BwdScratch ws = scratch_layout(a, nullptr);
+  const unsigned slots = (unsigned)backward_slots(a);
+  bwd_prep_kernel<<<dim3(slots, (unsigned)a.Hv), PREP_T, PR_SMEM, stream>>>(a, ws);
+  AVE_CUDA_TRY(cudaGetLastError());
+  bwd_forward_kernel<<<2 * units, SC_T, 2 * FW_STAGE, stream>>>(a, ws);
+  AVE_CUDA_TRY(cudaGetLastError());
+  bwd_reverse_kernel<<<2 * units, SC_T, 2 * RV_STAGE, stream>>>(a, ws);
+  AVE_CUDA_TRY(cudaGetLastError());
+  const bool sum = (a.flags & AVE_GDN_FLAG_BWD_SUMMED) != 0;
+  (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<dim3(slots, (unsigned)a.Hk), GR_T, GR_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }

@@ -638,6 +638,60 @@ PyObject* gemm(PyObject* const* p) {
   return wrap(c);
 }
 
+AveGdnBwdArgs bwd_args(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& d_o,
+                       double scale, const Tensor* s0, const Tensor* ds, const Tensor* cu, const Tensor& dq, const Tensor& dk,
+                       const Tensor& dv, const Tensor& dg, const Tensor& dbeta, const Tensor* ds0, uint32_t flags) {
+  AveGdnBwdArgs a{};
+  a.struct_size = sizeof(a);
+  a.flags = flags;
+  a.q = ptr(&q); a.k = ptr(&k); a.v = ptr(&v); a.g = ptr_as<float>(&g); a.beta = ptr_as<float>(&beta); a.d_o = ptr(&d_o);
+  a.initial_state = ptr_as<float>(s0); a.d_final_state = ptr_as<float>(ds); a.cu_seqlens = ptr_as<int32_t>(cu);
+  a.d_q = ptr_as<float>(&dq); a.d_k = ptr_as<float>(&dk); a.d_v = ptr_as<float>(&dv);
+  a.d_g = ptr_as<float>(&dg); a.d_beta = ptr_as<float>(&dbeta); a.d_initial_state = ptr_as<float>(ds0);
+  a.status = reinterpret_cast<uint32_t*>(status_word(q.device()).data_ptr());
+  a.B = (int32_t)q.size(0); a.T = (int32_t)q.size(1); a.Hk = (int32_t)q.size(2); a.Hv = (int32_t)v.size(2);
+  a.dk = (int32_t)q.size(3); a.dv = (int32_t)v.size(3);
+  a.n_seqs = (int32_t)(cu != nullptr ? cu->numel() - 1 : q.size(0));
+  STRIDES4(a, q, q); STRIDES4(a, k, k); STRIDES4(a, v, v); STRIDES4(a, do, d_o);
+  a.g_stride_b = g.stride(0); a.g_stride_t = g.stride(1); a.scale = (float)scale;
+  return a;
+}
+void enqueue_backward(AveGdnBwdArgs& a, const Tensor& q) {
+  Launch launch(q);
+  a.workspace = workspace(q, launch.stream, api.backward_workspace_bytes(&a), &a.workspace_bytes);
+  check(launch([&] { return api.recurrent_backward(&a, launch.stream); }), "gated_delta_rule_backward");
+}
+
+// backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens) -> (dq, dk, dv, dg, dbeta, ds0 or None)
+PyObject* backward(PyObject* const* p) {
+  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta"),
+               &d_o = tensor(p[5], "d_o");
+  const Tensor *s0 = opt_tensor(p[7], "initial_state"), *ds = opt_tensor(p[8], "d_final_state"), *cu = opt_tensor(p[9], "cu_seqlens");
+  const Shape s = check_common(q, k, v, g, beta, nullptr, cu);
+  REQ(s.dk == 128 && s.dv == 128, "the backward pass is built for head dims (128, 128), got (", s.dk, ", ", s.dv, ").");
+  REQ(d_o.scalar_type() == at::kBFloat16 && d_o.sizes() == v.sizes() && d_o.device() == q.device() && d_o.stride(3) == 1,
+      "d_o must be a bf16 tensor of shape ", shape_of(v.sizes()), " on ", q.device());
+  const std::pair<const char*, const Tensor*> states[] = {{"initial_state", s0}, {"d_final_state", ds}};
+  for (const auto& [name, t] : states)
+    if (t != nullptr)
+      REQ(t->scalar_type() == at::kFloat && t->dim() == 4 && t->size(0) == s.n && t->size(1) == s.Hv && t->size(2) == s.dk &&
+              t->size(3) == s.dv && t->is_contiguous() && t->device() == q.device(),
+          name, " must be a contiguous fp32 tensor (", s.n, ", ", s.Hv, ", ", s.dk, ", ", s.dv, ") on ", q.device());
+  const Tensor dq = empty(q.sizes(), at::kBFloat16, q), dk = empty(q.sizes(), at::kBFloat16, q), dv = empty(v.sizes(), at::kBFloat16, v);
+  const Tensor dg = empty(g.sizes(), at::kFloat, q), dbeta = empty(g.sizes(), at::kFloat, q);
+  const Tensor ds0 = s0 != nullptr ? empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, q) : Tensor();
+  AveGdnBwdArgs a = bwd_args(q, k, v, g, beta, d_o, scale_or(p[6], s.dk), s0, ds, cu, dq, dk, dv, dg, dbeta, some(ds0), AVE_GDN_FLAG_BWD_SUMMED);
+  enqueue_backward(a, q);
+  PyObject* r = PyTuple_New(6);
+  if (r == nullptr) throw python_error();
+  const Tensor* out[] = {&dq, &dk, &dv, &dg, &dbeta, &ds0};
+  for (int i = 0; i < 6; ++i) {
+    if (!out[i]->defined()) Py_INCREF(Py_None);
+    PyTuple_SET_ITEM(r, i, out[i]->defined() ? wrap(*out[i]) : Py_None);
+  }
+  return r;
+}
+
 // ---------------------------------------------------------------------------------------------- torch.ops.avelang_gdn.*
 // The operators take tensors the caller has laid out; the library checks what they pass on.
 int64_t n_sequences(const Tensor& q, const Tensor* cu) { return cu != nullptr ? cu->numel() - 1 : q.size(0); }
@@ -693,6 +747,18 @@ PyObject* op_gate(PyObject* const* p) {
 }
 PyObject* op_gemm(PyObject* const* p) {
   enqueue_gemm(tensor(p[0], "A"), tensor(p[1], "B"), tensor(p[2], "out"));
+  return none();
+}
+
+// op_backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens, dq, dk, dv, dg, dbeta, d_initial_state): dq, dk
+// and dv in fp32 per value head, contiguous
+PyObject* op_backward(PyObject* const* p) {
+  const Tensor &q = tensor(p[0], "q");
+  AveGdnBwdArgs a = bwd_args(q, tensor(p[1], "k"), tensor(p[2], "v"), tensor(p[3], "g"), tensor(p[4], "beta"), tensor(p[5], "d_o"), number(p[6]),
+                             opt_tensor(p[7], "initial_state"), opt_tensor(p[8], "d_final_state"), opt_tensor(p[9], "cu_seqlens"),
+                             tensor(p[10], "dq"), tensor(p[11], "dk"), tensor(p[12], "dv"), tensor(p[13], "dg"), tensor(p[14], "dbeta"),
+                             opt_tensor(p[15], "d_initial_state"), 0);
+  enqueue_backward(a, q);
   return none();
 }
 
@@ -755,6 +821,8 @@ PyMethodDef methods[] = {
     ENTRY("conv_update", conv_update, 6),
     ENTRY("gate", gate, 4),
     ENTRY("gemm", gemm, 3),
+    ENTRY("backward", backward, 10),
+    ENTRY("op_backward", op_backward, 16),
     ENTRY("op_prefill", op_prefill, 17),
     ENTRY("op_decode", op_decode, 15),
     ENTRY("op_rmsnorm", op_rmsnorm, 6),

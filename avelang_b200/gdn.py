@@ -44,56 +44,6 @@ def read_status(device=None, reset: bool = True) -> int:
     return val
 
 
-_workspaces: dict[tuple[int, int], torch.Tensor] = {}
-
-
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Scratch owned by the Python layer, grown on demand and reused (one per device and stream)."""
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
-    cur = _workspaces.get(key)
-    if cur is None or cur.numel() < nbytes:
-        cur = torch.empty(max(nbytes, 1), dtype=torch.uint8, device=device)
-        _workspaces[key] = cur
-    return cur
-
-
-def _req(cond: bool, msg: str) -> None:
-    if not cond:
-        raise ValueError(msg)
-
-
-def _check_common(q, k, v, g, beta, z, cu_seqlens):
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        _req(isinstance(t, torch.Tensor) and t.dim() == 4, f"{name} must be a 4-D tensor [B, T, H, d]")
-        _req(t.dtype == torch.bfloat16, f"{name} must have dtype torch.bfloat16, got {t.dtype}.")
-        _req(t.is_cuda, f"{name} must be a CUDA tensor")
-        _req(t.stride(-1) == 1, f"{name} must be contiguous in its last dimension")
-        _req(t.device == q.device, f"{name} must be on device {q.device}, got {t.device}.")
-    B, T, Hk, dk = q.shape
-    _req(k.shape == q.shape, f"k must have shape {tuple(q.shape)}, got {tuple(k.shape)}.")
-    _req(v.shape[0] == B and v.shape[1] == T, f"v must have leading shape {(B, T)}, got {tuple(v.shape[:2])}.")
-    Hv, dv = v.shape[2], v.shape[3]
-    _req(Hv % Hk == 0, f"value heads ({Hv}) must be a multiple of key heads ({Hk}).")
-    _req((dk, dv) in ((128, 128), (64, 64)), f"head dims (dk, dv) must be (128, 128) or (64, 64), got {(dk, dv)}.")
-    for name, t in (("g", g), ("beta", beta)):
-        _req(t.dtype == torch.float32, f"{name} must have dtype torch.float32, got {t.dtype}.")
-        _req(tuple(t.shape) == (B, T, Hv), f"{name} must have shape {(B, T, Hv)}, got {tuple(t.shape)}.")
-        _req(t.device == q.device, f"{name} must be on device {q.device}, got {t.device}.")
-        _req(t.stride(-1) == 1 or Hv == 1, f"{name} must be contiguous in its last dimension")
-    _req(g.stride() == beta.stride(), "g and beta must share strides")
-    if z is not None:
-        _req(z.dtype == torch.bfloat16 and z.shape == v.shape and z.device == q.device and z.stride(-1) == 1,
-             f"z must be a bf16 tensor of shape {tuple(v.shape)} on {q.device}")
-    n_seqs = B
-    if cu_seqlens is not None:
-        _req(B == 1, "cu_seqlens requires B == 1 (packed layout)")
-        _req(cu_seqlens.dtype == torch.int32 and cu_seqlens.dim() == 1 and cu_seqlens.numel() >= 1,
-             "cu_seqlens must be a 1-D int32 tensor [N+1]")
-        _req(cu_seqlens.device == q.device and cu_seqlens.is_contiguous(), f"cu_seqlens must be contiguous on {q.device}")
-        n_seqs = cu_seqlens.numel() - 1
-    return B, T, Hk, Hv, dk, dv, n_seqs
-
-
 def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, output_final_state=False,
                            use_qk_l2norm_in_kernel=False, cu_seqlens=None, *, z=None, norm_weight=None,
                            norm_eps=1e-6, state_indices=None, inplace_state=True, chunk_size=64, out=None, out_peers=None,
@@ -183,56 +133,20 @@ def gated_delta_rule_backward(q, k, v, g, beta, d_o, scale=None, initial_state=N
     without the fused gated norm) for d = 128.  ``d_o``: bf16, shaped like ``v``; ``d_final_state``: optional fp32 gradient
     of the final states.  Returns ``(dq, dk, dv, dg, dbeta, d_initial_state)``: dq, dk in the dtype and shape of q, k (the
     value heads sharing a key head are summed), dv in the dtype of v, dg, dbeta fp32, ``d_initial_state`` fp32 or None
-    when no initial state was given.  A token-by-token reverse sweep in fp32 (recomputing the states from 64-token
-    checkpoints): exact to fp32 rounding, and far slower than the chunked forward pass."""
-    B, T, Hk, Hv, dk, dv, n_seqs = _check_common(q, k, v, g, beta, None, cu_seqlens)
-    _req((dk, dv) == (128, 128), f"the backward pass is built for head dims (128, 128), got {(dk, dv)}.")
-    _req(d_o.dtype == torch.bfloat16 and d_o.shape == v.shape and d_o.device == q.device and d_o.stride(-1) == 1,
-         f"d_o must be a bf16 tensor of shape {tuple(v.shape)} on {q.device}")
-    for name, t in (("initial_state", initial_state), ("d_final_state", d_final_state)):
-        if t is not None:
-            _req(t.dtype == torch.float32 and tuple(t.shape) == (n_seqs, Hv, dk, dv) and t.is_contiguous() and t.device == q.device,
-                 f"{name} must be a contiguous fp32 tensor ({n_seqs}, {Hv}, {dk}, {dv}) on {q.device}")
-    f32 = dict(dtype=torch.float32, device=q.device)
-    dq_v, dk_v = torch.empty(B, T, Hv, dk, **f32), torch.empty(B, T, Hv, dk, **f32)
-    dv_f, dg, dbeta = torch.empty(B, T, Hv, dv, **f32), torch.empty(B, T, Hv, **f32), torch.empty(B, T, Hv, **f32)
-    ds0 = torch.empty(n_seqs, Hv, dk, dv, **f32) if initial_state is not None else None
-    torch_ops.op("recurrent_backward")(q, k, v, g, beta, d_o, float(dk ** -0.5 if scale is None else scale), initial_state,
-                                       d_final_state, cu_seqlens, dq_v, dk_v, dv_f, dg, dbeta, ds0)
-    r = Hv // Hk
-    dq = dq_v.view(B, T, Hk, r, dk).sum(3).to(q.dtype)
-    dk_ = dk_v.view(B, T, Hk, r, dk).sum(3).to(k.dtype)
-    return dq, dk_, dv_f.to(v.dtype), dg, dbeta, ds0
+    when no initial state was given.  Chunked like the forward pass (64 tokens), every fp32 operand carried to 24 bits."""
+    return _native.backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens)
 
 
 @torch_ops.implement("recurrent_backward")
-def _recurrent_backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens, dq, dk, dv, dg, dbeta, d_initial_state):
-    """torch.ops.avelang_gdn.recurrent_backward -> ave_gdn_recurrent_backward on the current stream."""
-    B, T, Hk, dkk = q.shape
-    Hv, dvv = v.shape[2], v.shape[3]
-    a = _lib.BwdArgs()
-    a.struct_size = ctypes.sizeof(_lib.BwdArgs)
-    ptr = lambda t: t.data_ptr() if t is not None and t.numel() > 0 else None
-    a.q, a.k, a.v, a.g, a.beta, a.d_o = ptr(q), ptr(k), ptr(v), ptr(g), ptr(beta), ptr(d_o)
-    a.initial_state, a.d_final_state, a.cu_seqlens = ptr(initial_state), ptr(d_final_state), ptr(cu_seqlens)
-    a.d_q, a.d_k, a.d_v, a.d_g, a.d_beta, a.d_initial_state = ptr(dq), ptr(dk), ptr(dv), ptr(dg), ptr(dbeta), ptr(d_initial_state)
-    a.status = _status_word(q.device).data_ptr()
-    a.B, a.T, a.Hk, a.Hv, a.dk, a.dv = B, T, Hk, Hv, dkk, dvv
-    a.n_seqs = B if cu_seqlens is None else cu_seqlens.numel() - 1
-    for name, t in (("q", q), ("k", k), ("v", v), ("do", d_o)):
-        setattr(a, f"{name}_stride_b", t.stride(0)); setattr(a, f"{name}_stride_t", t.stride(1)); setattr(a, f"{name}_stride_h", t.stride(2))
-    a.g_stride_b, a.g_stride_t, a.scale = g.stride(0), g.stride(1), float(scale)
-    lib = _lib.load()
-    with torch.cuda.device(q.device):
-        ws = _workspace(q.device, lib.ave_gdn_backward_workspace_bytes(ctypes.byref(a)))
-        a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
-        rc = lib.ave_gdn_recurrent_backward(ctypes.byref(a), torch.cuda.current_stream(q.device).cuda_stream)
-    _lib.check(rc, "gated_delta_rule_backward")
+def _recurrent_backward(*args):
+    """torch.ops.avelang_gdn.recurrent_backward -> ave_gdn_recurrent_backward on the current stream (dq, dk, dv in fp32 per
+    value head)."""
+    _native.op_backward(*args)
 
 
 class GatedDeltaRuleFunction(torch.autograd.Function):
     """``o, final_state = GatedDeltaRuleFunction.apply(q, k, v, g, beta, scale, initial_state)``: the chunked forward pass
-    with the reverse-sweep backward pass attached (d = 128, dense batches, no in-kernel L2 norm, no fused gated norm)."""
+    with the chunked backward pass attached (d = 128, dense batches, no in-kernel L2 norm, no fused gated norm)."""
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, scale, initial_state):

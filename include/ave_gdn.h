@@ -60,6 +60,7 @@ typedef enum AveGdnStatus {
 
 /* flags */
 #define AVE_GDN_FLAG_QK_L2NORM 1u    /* normalise q and k per head vector (eps 1e-6) inside the kernel */
+#define AVE_GDN_FLAG_BWD_SUMMED 4u   /* backward: d_q, d_k are bf16 [B,T,Hk,dk], summed over the value heads, and d_v is bf16 */
 #define AVE_GDN_FLAG_GATE_FIRST 2u   /* gated norm computes rmsnorm(o * silu(z)) instead of rmsnorm(o) * silu(z) */
 
 /* One argument block for both recurrences (chunked prefill and token-by-token decode). */
@@ -259,8 +260,9 @@ int ave_gdn_decode_layer_step(const AveGdnDecodeLayerArgs* args, void* stream);
  * fused gated norm: those two are differentiated by the caller's framework around this call).  Inputs as for the
  * forward pass plus d_o (bf16, laid out like v) and the optional gradient of the final states; outputs in fp32:
  * dq, dk [B,T,Hv,dk] PER VALUE HEAD (the caller sums the value heads that share a key head), dv [B,T,Hv,dv],
- * dg, dbeta [B,T,Hv], and optionally d_initial_state [n_seqs,Hv,dk,dv]; all contiguous.  Token-by-token reverse sweep
- * in fp32 with the state recomputed from 64-token checkpoints held in `workspace`. */
+ * dg, dbeta [B,T,Hv], and optionally d_initial_state [n_seqs,Hv,dk,dv]; all contiguous.  With AVE_GDN_FLAG_BWD_SUMMED
+ * d_q and d_k point to bf16 [B,T,Hk,dk] (the value heads of a key head summed in fp32) and d_v to bf16 [B,T,Hv,dv].
+ * Chunked like the forward pass, with fp32-level accuracy; the states and their gradients of all chunks live in `workspace`. */
 typedef struct AveGdnBwdArgs {
   uint32_t struct_size;
   uint32_t flags;
