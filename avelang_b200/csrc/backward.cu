@@ -30,6 +30,7 @@
 #include "blockalg.cuh"
 #include "common.cuh"
 #include "tc.cuh"
+#include "warpmma.cuh"
 
 namespace ave {
 namespace {
@@ -65,95 +66,10 @@ __device__ __forceinline__ BwdChunk chunk_of_slot(const AveGdnBwdArgs& a, int64_
   return c;
 }
 
-// ---------------------------------------------------------------------------------------------- warp MMA helpers
-__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm4t(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-// Tiles are stored in rows of ROWB bytes; the 16-byte piece c of row r sits at piece c ^ (r & 7).
-template <int ROWB>
-__device__ __forceinline__ uint32_t piece(int row, int c) { return (uint32_t)(row * ROWB + ((c ^ (row & 7)) << 4)); }
-// Lane addresses of the four ldmatrix patterns (r0, c0: first row and first 16-byte piece of the 16x16 block in the tile)
-template <int ROWB>  // left operand, tile rows = its rows
-__device__ __forceinline__ uint32_t at_a(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 15), c0 + (lane >> 4)); }
-template <int ROWB>  // left operand, tile rows = contraction index (with .trans)
-__device__ __forceinline__ uint32_t at_at(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
-template <int ROWB>  // right operand of two adjacent column tiles, tile rows = its columns
-__device__ __forceinline__ uint32_t at_b(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 7) + ((lane >> 4) << 3), c0 + ((lane >> 3) & 1)); }
-template <int ROWB>  // right operand of two adjacent column tiles, tile rows = contraction index (with .trans)
-__device__ __forceinline__ uint32_t at_bt(int r0, int c0, int lane) { return piece<ROWB>(r0 + (lane & 15), c0 + (lane >> 4)); }
-
 // e^{b_i - b_j} for i >= j (at most 1 elsewhere); sc: b[64] | beta[64] | low part of b[64]
 __device__ __forceinline__ float gate_between(const float* sc, int i, int j) {
   return __expf(fminf((sc[i] - sc[j]) + (sc[2 * BCH + i] - sc[2 * BCH + j]), 0.f));
 }
-
-// x = h + m + l in bf16, exact to 24 bits
-__device__ __forceinline__ void split3(float2 x, uint32_t& h, uint32_t& m, uint32_t& l) {
-  const float2 m1 = make_float2(-1.f, -1.f);
-  h = pack_bf16x2(x.x, x.y);
-  const float2 r = __ffma2_rn(bf16x2_to_float2(h), m1, x);
-  m = pack_bf16x2(r.x, r.y);
-  const float2 s = __ffma2_rn(bf16x2_to_float2(m), m1, r);
-  l = pack_bf16x2(s.x, s.y);
-}
-// two adjacent accumulator tiles (columns 0..15) -> left operand of a product over those columns, three terms
-__device__ __forceinline__ void split_acc(const float (&c0)[4], const float (&c1)[4], uint32_t (&h)[4], uint32_t (&m)[4], uint32_t (&l)[4]) {
-  split3(make_float2(c0[0], c0[1]), h[0], m[0], l[0]);
-  split3(make_float2(c0[2], c0[3]), h[1], m[1], l[1]);
-  split3(make_float2(c1[0], c1[1]), h[2], m[2], l[2]);
-  split3(make_float2(c1[2], c1[3]), h[3], m[3], l[3]);
-}
-// d += (h + m + l) * b with b exact
-__device__ __forceinline__ void mma3(float (&d)[4], const uint32_t (&h)[4], const uint32_t (&m)[4], const uint32_t (&l)[4], uint32_t b0, uint32_t b1) {
-  mma_bf16(d, h, b0, b1);
-  mma_bf16(d, m, b0, b1);
-  mma_bf16(d, l, b0, b1);
-}
-// d += (ah + am + al) (bh + bm + bl), the terms below 2^-24 left out
-__device__ __forceinline__ void mma6(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
-                                     uint32_t bh0, uint32_t bh1, uint32_t bm0, uint32_t bm1, uint32_t bl0, uint32_t bl1) {
-  mma_bf16(d, ah, bh0, bh1);
-  mma_bf16(d, ah, bm0, bm1);
-  mma_bf16(d, am, bh0, bh1);
-  mma_bf16(d, ah, bl0, bl1);
-  mma_bf16(d, al, bh0, bh1);
-  mma_bf16(d, am, bm0, bm1);
-}
-__device__ __forceinline__ void zero(float (&d)[4]) { d[0] = d[1] = d[2] = d[3] = 0.f; }
-
-__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool valid) {
-  const int bytes = valid ? 16 : 0;  // the rest of the 16 bytes is zero-filled
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// `rows` x `PIECES` 16-byte pieces of a strided bf16 matrix into a tile; rows from `len` on are zero
-template <int PIECES, int THREADS>
-__device__ __forceinline__ void load_tile(uint32_t dst, const __nv_bfloat16* src, int64_t stride, int len, int tid) {
-#pragma unroll
-  for (int i = 0; i < BCH * PIECES / THREADS; ++i) {
-    const int e = tid + i * THREADS, row = e / PIECES, c = e % PIECES;
-    cp16(dst + piece<PIECES * 16>(row, c), src + (int64_t)(row < len ? row : 0) * stride + c * 8, row < len);
-  }
-}
-template <int BYTES, int THREADS>
-__device__ __forceinline__ void load_flat(uint32_t dst, const uint8_t* src, int tid) {
-#pragma unroll
-  for (int i = 0; i < (BYTES / 16 + THREADS - 1) / THREADS; ++i) {
-    const int e = tid + i * THREADS;
-    if (BYTES / 16 % THREADS == 0 || e < BYTES / 16) cp16(dst + e * 16, src + e * 16, true);
-  }
-}
-__device__ __forceinline__ const __nv_bfloat16* bf(const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); }
 
 // ---------------------------------------------------------------------------------------------- T, P and b of every chunk
 constexpr int PREP_T = 256;
@@ -175,8 +91,8 @@ __global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a,
   const int hk = h / (a.Hv / a.Hk);
   uint8_t* rec = ws.prep + ((int64_t)blockIdx.x * a.Hv + h) * PREP_BYTES;
   const uint32_t sb = tc::smem_u32(smem);
-  load_tile<16, PREP_T>(sb + PR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
-  load_tile<16, PREP_T>(sb + PR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
+  load_tile<BCH, 16, PREP_T>(sb + PR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
+  load_tile<BCH, 16, PREP_T>(sb + PR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
   cp_commit();
   if (warp == 0) {  // inclusive scan of the gates; beyond the end of the sequence b stays and beta is 0
     // b reaches hundreds while e^{b_i - b_j} of near tokens matters: it is summed in double and kept as two floats, so that
@@ -405,8 +321,8 @@ __global__ void __launch_bounds__(SC_T, 2) bwd_forward_kernel(const AveGdnBwdArg
     const uint32_t st = sb + (c & 1) * FW_STAGE;
     const int len = min(BCH, u.sp.len - c * BCH);
     const uint8_t* rec = ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES;
-    load_tile<16, SC_T>(st + FW_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
-    load_tile<8, SC_T>(st + FW_V, vp + (int64_t)c * BCH * a.v_stride_t, a.v_stride_t, len, tid);
+    load_tile<BCH, 16, SC_T>(st + FW_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
+    load_tile<BCH, 8, SC_T>(st + FW_V, vp + (int64_t)c * BCH * a.v_stride_t, a.v_stride_t, len, tid);
     load_flat<3 * IMG, SC_T>(st + FW_TI, rec, tid);
     load_flat<SC_BYTES, SC_T>(st + FW_SC, rec + PREP_SC, tid);
   };
@@ -491,9 +407,9 @@ __global__ void __launch_bounds__(SC_T, 1) bwd_reverse_kernel(const AveGdnBwdArg
   auto load = [&](int c) {
     const uint32_t st = sb + (c & 1) * RV_STAGE;
     const int len = min(BCH, u.sp.len - c * BCH);
-    load_tile<16, SC_T>(st + RV_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
-    load_tile<16, SC_T>(st + RV_Q, qp + (int64_t)c * BCH * a.q_stride_t, a.q_stride_t, len, tid);
-    load_tile<8, SC_T>(st + RV_DO, dop + (int64_t)c * BCH * a.do_stride_t, a.do_stride_t, len, tid);
+    load_tile<BCH, 16, SC_T>(st + RV_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
+    load_tile<BCH, 16, SC_T>(st + RV_Q, qp + (int64_t)c * BCH * a.q_stride_t, a.q_stride_t, len, tid);
+    load_tile<BCH, 8, SC_T>(st + RV_DO, dop + (int64_t)c * BCH * a.do_stride_t, a.do_stride_t, len, tid);
     load_flat<PREP_BYTES, SC_T>(st + RV_TI, ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES, tid);
   };
   load(n_chunks - 1);
@@ -636,8 +552,8 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
   const int wm = warp & 1, wn = warp >> 1;  // token half, 16-column block
   const int64_t row0 = (int64_t)c.b * a.T + c.t0;
 
-  load_tile<16, GR_T>(sb + GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
-  load_tile<16, GR_T>(sb + GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
+  load_tile<BCH, 16, GR_T>(sb + GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
+  load_tile<BCH, 16, GR_T>(sb + GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
   float dq[2][2][4], dk[2][2][4];  // [16-token tile][8-column tile], summed over the value heads
 #pragma unroll
   for (int i = 0; i < 2; ++i)
@@ -649,7 +565,7 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
     const int h = hk * r + hh;
     const int64_t rec = slot * a.Hv + h;
     if (hh > 0) __syncthreads();  // the tiles and sums of the previous head are no longer read
-    load_tile<16, GR_T>(sb + GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t, c.len, tid);
+    load_tile<BCH, 16, GR_T>(sb + GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t, c.len, tid);
     cp_commit();
     split_tile(smem + GR_VN, ws.vn + rec * VEC_FLOATS, tid);
     split_tile(smem + GR_U, ws.u + rec * VEC_FLOATS, tid);

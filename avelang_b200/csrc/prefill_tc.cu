@@ -1,10 +1,9 @@
 // Chunked gated-delta-rule prefill on the tensor cores (d_k = d_v = 128, chunk 64).
 //
-// Pass 1, chunk_prep (one CTA per (chunk, value head), fully parallel, four CTAs per SM): in-chunk cumulative gate b,
-//   [K; Q] K^T on tcgen05 -> A = strict_lower(beta_i e^{b_i-b_j} k_i.k_j) and P = scale * lower_incl(e^{b_i-b_j} q_i.k_j);
-//   T = (I+A)^-1 by 16x16 blocks (warp-level tf32 MMAs); W^T = K^T (T diag(beta e^b))^T on tcgen05.  W^T, P and
-//   Tu = T diag(beta) leave as bf16 hi+lo pairs (the tensor cores then see 16 significant bits), each as the swizzled
-//   shared-memory image of its tile so that a bulk copy moves it out here and in again in pass 2, plus per-token
+// Pass 1, chunk_prep (prefill_prep.cuh; parallel over chunks): in-chunk cumulative gate b, T = (I+A)^-1 with
+//   A = strict_lower(beta_i e^{b_i-b_j} k_i.k_j), P = scale * lower_incl(e^{b_i-b_j} q_i.k_j), W^T = K^T (T diag(beta e^b))^T.
+//   W^T, P and Tu = T diag(beta) leave as bf16 hi+lo pairs (the tensor cores then see 16 significant bits), each as the
+//   swizzled shared-memory image of its tile so that a bulk copy moves it out here and in again in pass 2, plus per-token
 //   scale vectors.
 // Pass 2, chunk_scan (one CTA per (sequence, value head)): the recurrence over chunks with the state kept
 //   on chip, transposed (H = M^T, rows = d_v = TMEM lanes) so that every MMA has M = 128:
@@ -20,7 +19,6 @@
 // All waits are bounded; on give-up the CTA drains, frees its tensor memory and sets a status bit.
 #include <mutex>
 
-#include "blockalg.cuh"
 #include "common.cuh"
 #include "tc.cuh"
 
@@ -151,439 +149,13 @@ __device__ __forceinline__ uint32_t kmajor_piece_off(int row, int k8) {
   return (uint32_t)((k8 >> 3) * 16384 + row * 128 + (((k8 & 7) ^ (row & 7)) << 4));
 }
 
-// ------------------------------------------------------------------------------------------------ pass 1
-// Shared memory of chunk_prep (offsets from a 1024-byte aligned base).  The K and Q tiles are interleaved by
-// 64-wide halves, [K_h0 | Q_h0 | K_h1 | Q_h1], so that one M = 128 MMA reads [K; Q] as its A operand (rows 0..63 =
-// K, 64..127 = Q) and the K rows alone as its N = 64 B operand: lanes 0..63 of the accumulator are K K^T, lanes
-// 64..127 are Q K^T.
+}  // namespace
+}  // namespace ave
 
-// bf16 hi + lo images of a pair of fp32 values: hi = round-to-bf16, lo = bf16(x - hi); packed math on the pair
-__device__ __forceinline__ void split_pair(float2 x, uint32_t& hi, uint32_t& lo) {
-  hi = pack_bf16x2(x.x, x.y);
-  const float2 h = make_float2(__uint_as_float(hi << 16), __uint_as_float(hi & 0xffff0000u));
-  const float2 l = __ffma2_rn(h, make_float2(-1.f, -1.f), x);
-  lo = pack_bf16x2(l.x, l.y);
-}
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-// Four gated Gram entries f_i kn_j e^{b_i - b_j} acc_j for columns j0..j0+3 (packed fp32 pairs); entry e is kept when
-// keep > e, where the caller passes keep = i - j0 for a strictly lower mask and i - j0 + 1 for a lower one.  The
-// difference b_i - b_j is formed before the scaling by log2(e), so nearby tokens lose no accuracy to large |b|.
-__device__ __forceinline__ void gate4(float (&out)[4], const uint32_t* acc, float bi, float fi, const float* bs_j, const float* kn_j,
-                                      int keep) {
-  const float4 b4 = *reinterpret_cast<const float4*>(bs_j), k4 = *reinterpret_cast<const float4*>(kn_j);
-  const float2 m1 = make_float2(-1.f, -1.f), bi2 = make_float2(bi, bi), fi2 = make_float2(fi, fi);
-  const float2 l2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
-  const float2 x0 = __fmul2_rn(__ffma2_rn(make_float2(b4.x, b4.y), m1, bi2), l2e);
-  const float2 x1 = __fmul2_rn(__ffma2_rn(make_float2(b4.z, b4.w), m1, bi2), l2e);
-  const float2 e0 = make_float2(ex2_approx(x0.x), ex2_approx(x0.y)), e1 = make_float2(ex2_approx(x1.x), ex2_approx(x1.y));
-  const float2 r0 = __fmul2_rn(__fmul2_rn(fi2, make_float2(__uint_as_float(acc[0]), __uint_as_float(acc[1]))),
-                               __fmul2_rn(make_float2(k4.x, k4.y), e0));
-  const float2 r1 = __fmul2_rn(__fmul2_rn(fi2, make_float2(__uint_as_float(acc[2]), __uint_as_float(acc[3]))),
-                               __fmul2_rn(make_float2(k4.z, k4.w), e1));
-  out[0] = keep > 0 ? r0.x : 0.f; out[1] = keep > 1 ? r0.y : 0.f;
-  out[2] = keep > 2 ? r1.x : 0.f; out[3] = keep > 3 ? r1.y : 0.f;
-}
+#include "prefill_prep.cuh"  // pass 1
 
-constexpr int PREP_THREADS = 256;
-// Regions are reused as their contents die, which keeps a CTA at 52 KB so that four fit on an SM:
-//   PP_KQ  [K_h0 | Q_h0 | K_h1 | Q_h1]   once the Gram MMA is done the Q halves hold the store images of P hi / P lo, then
-//                                        the E, E^2, E^3 block scratch, then Tw hi / Tw lo; after the W MMA the whole
-//                                        region is the store image of W^T hi | W^T lo
-//   PP_R2  A -> T blocks and D^-1 blocks
-constexpr int PP_KQ = 0, PP_TWH = PP_KQ + 8192, PP_TWL = PP_KQ + 24576,
-              PP_WHI = PP_KQ, PP_WLO = PP_KQ + 16384,
-              PP_R2 = 32768, PP_A = PP_R2, PP_DI = PP_A + 10 * BLK_FLOATS * 4,
-              PP_SC = PP_R2 + 18432, PP_BARS = PP_SC + 4 * C * 4;
-constexpr int PP_PHI = PP_TWH, PP_PLO = PP_TWL;        // P hi / P lo tile images, before the block scratch
-constexpr int PP_E = PP_TWH, PP_E2 = PP_TWL, PP_E3 = PP_E2 + 3 * BLK_FLOATS * 4;
-static_assert(6 * BLK_FLOATS * 4 <= 8192 && 4 * BLK_FLOATS * 4 <= 8192, "block scratch must fit inside the Q halves");
-static_assert(PP_DI + 4 * BLK_FLOATS * 4 <= PP_R2 + 18432, "T and D^-1 blocks must fit inside their region");
-constexpr size_t PREP_SMEM = PP_BARS + 64 + 1024;
-constexpr uint32_t PT_GRAM = 0, PT_W = 0;               // TMEM columns (64 allocated; W^T reuses the Gram columns)
-
-// Pass 1 per (chunk, value head):
-//   tensor cores: [K; Q] K^T                                   -> A (strict lower, gated) and P (lower, gated)
-//   CUDA cores  : T = (I + A)^-1 by 16x16 blocks (warp-level tf32 MMAs for the block products)
-//   tensor cores: W^T = K^T (T diag(beta e^b))^T   (M = 128 = d_k, N = 64 tokens)
-// W^T leaves as bf16 hi + lo, as the 128-byte-swizzled shared-memory image of a [128][64] tile (one bulk copy out here,
-// one bulk copy in by the scan, which reads it as an MN-major B operand); Tu = T diag(beta) leaves as bf16 hi + lo
-// [64][64] tiles in the same swizzled layout: the scan forms U^T = V^T Tu^T itself, straight into its Vn accumulator.
-__global__ void __launch_bounds__(PREP_THREADS, 4)
-chunk_prep_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, const int32_t* __restrict__ chunk_start, PrepOut out,
-                  const __grid_constant__ ScanPlan plan, int compact_grid) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  float* Ab = reinterpret_cast<float*>(smem + PP_A);   // A as 16x16 blocks (r >= c), block tri(r,c); later T
-  float* Di = reinterpret_cast<float*>(smem + PP_DI);  // (I + A_rr)^-1
-  float* Eb = reinterpret_cast<float*>(smem + PP_E);
-  float* E2b = reinterpret_cast<float*>(smem + PP_E2);
-  float* E3b = reinterpret_cast<float*>(smem + PP_E3);
-  float* bs = reinterpret_cast<float*>(smem + PP_SC);
-  float* betas = bs + C;
-  float* qn = betas + C;
-  float* kn = qn + C;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + PP_BARS);
-  uint64_t* tma_bar = bars;
-  uint64_t* mma_bar = bars + 1;
-  uint64_t* mma2_bar = bars + 2;   // W^T accumulated
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 4);
-  volatile uint32_t* abort_flag = tmem_slot + 1;
-
-  const int h = blockIdx.y, tid = threadIdx.x;
-  const int warp = tid >> 5, lane = tid & 31;
-  // Whole-batch launches index every chunk of the batch; range launches use the compact grid
-  // n_seqs x parts x rn so that no CTA is spent on chunks outside the range.
-  int c = blockIdx.x;
-  if (compact_grid) {
-    const int per_seq = plan.parts * plan.rn;
-    const int n = blockIdx.x / per_seq, rest = blockIdx.x % per_seq;
-    const int cis = plan.part_begin[rest / plan.rn] + plan.r0 + rest % plan.rn;
-    if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;  // table rejected
-    const int per = a.cu_seqlens ? (chunk_start[n + 1] - chunk_start[n]) : (a.T + C - 1) / C;
-    if (cis >= per || cis >= plan.part_begin[rest / plan.rn + 1]) return;
-    c = (a.cu_seqlens ? chunk_start[n] : n * per) + cis;
-  }
-  const ChunkRef cr = find_chunk(a, chunk_start, c);  // (a compact grid only ever names chunks of this launch's range)
-  if (!cr.ok) return;
-  const int hk = h / (a.Hv / a.Hk);
-  const int64_t rec = (int64_t)c * a.Hv + h;
-
-  if (tid == 0) {
-    tc::mbar_init(tma_bar, 1);
-    tc::mbar_init(mma_bar, 1);
-    tc::mbar_init(mma2_bar, 1);
-    *abort_flag = 0;
-    tc::fence_barrier_init();
-    tc::mbar_expect_tx(tma_bar, 32768);
-    tc::tma_load_4d(smem + PP_KQ, &maps.k, tma_bar, 0, hk, cr.t0, cr.b);
-    tc::tma_load_4d(smem + PP_KQ + 8192, &maps.q, tma_bar, 0, hk, cr.t0, cr.b);
-    tc::tma_load_4d(smem + PP_KQ + 16384, &maps.k, tma_bar, 64, hk, cr.t0, cr.b);
-    tc::tma_load_4d(smem + PP_KQ + 24576, &maps.q, tma_bar, 64, hk, cr.t0, cr.b);
-  }
-  if (warp == 2) tc::tmem_alloc(tmem_slot, 64);
-  if (tid < C) {
-    const bool valid = tid < cr.len;
-    const int64_t off = cr.b * a.g_stride_b + (int64_t)(cr.t0 + tid) * a.g_stride_t + h;
-    bs[tid] = valid ? a.g[off] : 0.f;
-    betas[tid] = valid ? a.beta[off] : 0.f;
-  }
-  tc::tc_fence_before_sync();
-  __syncthreads();
-  tc::tc_fence_after_sync();
-  const uint32_t tm = *tmem_slot;
-  if (warp == 1) {  // in-chunk cumulative gate: inclusive scan of 64 values by one warp
-    float v0 = bs[lane], v1 = bs[32 + lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float t0 = __shfl_up_sync(0xffffffffu, v0, o), t1 = __shfl_up_sync(0xffffffffu, v1, o);
-      if (lane >= o) { v0 += t0; v1 += t1; }
-    }
-    v1 += __shfl_sync(0xffffffffu, v0, 31);
-    bs[lane] = v0; bs[32 + lane] = v1;
-  }
-
-  // Only warp 0 polls an mbarrier; the other warps park at the next CTA barrier (a hardware barrier costs no issue
-  // slots, a polling loop does) and learn of a failed wait through the abort flag.
-  bool ok = true;
-  if (warp == 0) {
-    ok = tc::mbar_wait_warp(tma_bar, 0, abort_flag);
-    tc::tc_fence_after_sync();
-    const bool leader = tc::elect_one();
-    if (ok && leader) {
-      constexpr uint32_t idesc = tc::idesc_f16(128, 64, 1, 1, false, false);
-      const uint32_t base = tc::smem_u32(smem + PP_KQ);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const uint64_t d = tc::smem_desc_sw128(base + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024);
-        tc::mma_ss(tm + PT_GRAM, d, d, idesc, k != 0 ? 1u : 0u);
-      }
-      tc::mma_commit(mma_bar);
-    }
-    __syncwarp();
-  }
-  // row norms of k and q (the swizzle only permutes 16-byte pieces inside a 128-byte row, so a row sum needs no decode)
-  if (a.flags & AVE_GDN_FLAG_QK_L2NORM) {
-    __syncthreads();  // warp 0 has seen the tiles land
-    const int i = tid >> 2, part = tid & 3;
-    float sk = 0.f, sq = 0.f;
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const uint4 kr = *reinterpret_cast<const uint4*>(smem + PP_KQ + half * 16384 + i * 128 + part * 32);
-      const uint4 kr2 = *reinterpret_cast<const uint4*>(smem + PP_KQ + half * 16384 + i * 128 + part * 32 + 16);
-      const uint4 qr = *reinterpret_cast<const uint4*>(smem + PP_KQ + 8192 + half * 16384 + i * 128 + part * 32);
-      const uint4 qr2 = *reinterpret_cast<const uint4*>(smem + PP_KQ + 8192 + half * 16384 + i * 128 + part * 32 + 16);
-      const uint32_t kw[8] = {kr.x, kr.y, kr.z, kr.w, kr2.x, kr2.y, kr2.z, kr2.w};
-      const uint32_t qw[8] = {qr.x, qr.y, qr.z, qr.w, qr2.x, qr2.y, qr2.z, qr2.w};
-#pragma unroll
-      for (int w = 0; w < 8; ++w) {
-        const float k0 = __uint_as_float(kw[w] << 16), k1 = __uint_as_float(kw[w] & 0xffff0000u);
-        const float q0 = __uint_as_float(qw[w] << 16), q1 = __uint_as_float(qw[w] & 0xffff0000u);
-        sk += k0 * k0 + k1 * k1; sq += q0 * q0 + q1 * q1;
-      }
-    }
-    sk += __shfl_xor_sync(0xffffffffu, sk, 1); sk += __shfl_xor_sync(0xffffffffu, sk, 2);
-    sq += __shfl_xor_sync(0xffffffffu, sq, 1); sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-    if (part == 0) { kn[i] = rsqrtf(sk + 1e-6f); qn[i] = rsqrtf(sq + 1e-6f); }
-  } else if (tid < C) { kn[tid] = 1.f; qn[tid] = 1.f; }
-  __syncthreads();
-  const float bC = bs[C - 1];
-  float* fwv = qn;  // q's norm is consumed below; afterwards the slot holds beta_j e^{b_j} kn_j, the column factor of Tw
-  if (tid < C) {
-    float* sc = out.scal + rec * SCAL_FLOATS;
-    sc[tid] = __expf(bs[tid]) * qn[tid] * a.scale;   // o_i = qs_i (H q_i) + (scale P Vn)_i: the output scale is folded in here and in P
-    sc[C + tid] = __expf(bC - bs[tid]) * kn[tid];    // Vd_j = ks_j Vn_j
-    sc[2 * C + tid] = __expf(bC);
-  }
-  if (warp == 0) tc::mbar_wait_warp(mma_bar, 0, abort_flag);
-  __syncthreads();
-  ok = *abort_flag == 0u;
-  tc::tc_fence_after_sync();
-  {
-    const int quarter = warp & 3, colhalf = warp >> 2;
-    const int r = quarter * 32 + lane;
-    // warps whose 32 columns all lie above their 32 rows (rows 0..31 against columns 32..63) have nothing to gate
-    const bool above = colhalf > (quarter & 1);
-    uint32_t acc[32];
-    if (!above) {
-      tc::tmem_ld32(tm + PT_GRAM + ((uint32_t)(quarter * 32) << 16) + 32 * colhalf, acc);
-      tc::tmem_ld_wait();
-    }
-    if (r < C) {  // A = strict_lower(beta_i e^{b_i-b_j} k_i.k_j); blocks above the diagonal are not stored
-      const int i = r;
-      const float bi = bs[i], fi = betas[i] * kn[i];
-      if (!above) {
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const int j0 = 32 * colhalf + 4 * j4;
-          float av[4];
-          gate4(av, acc + 4 * j4, bi, fi, bs + j0, kn + j0, i - j0);
-          if ((j0 >> 4) <= (i >> 4))
-            *reinterpret_cast<float4*>(Ab + tri(i >> 4, j0 >> 4) * BLK_FLOATS + (i & 15) * BLK_LD + (j0 & 15)) =
-                make_float4(av[0], av[1], av[2], av[3]);
-        }
-      }
-    } else {      // P = lower_incl(e^{b_i-b_j} q_i.k_j), bf16 hi + lo
-      const int i = r - C;
-      const float bi = bs[i], fi = (i < cr.len) ? qn[i] * a.scale : 0.f;
-      uint32_t ph[16], pl[16];
-      if (!above) {
-#pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          const int j0 = 32 * colhalf + 4 * j4;
-          float pv[4];
-          gate4(pv, acc + 4 * j4, bi, fi, bs + j0, kn + j0, i - j0 + 1);
-          split_pair(make_float2(pv[0], pv[1]), ph[2 * j4], pl[2 * j4]);
-          split_pair(make_float2(pv[2], pv[3]), ph[2 * j4 + 1], pl[2 * j4 + 1]);
-        }
-      } else {
-#pragma unroll
-        for (int w = 0; w < 16; ++w) { ph[w] = 0u; pl[w] = 0u; }
-      }
-      // the Q halves are dead (the Gram MMA is complete): they take the swizzled tile images of P hi and P lo, which
-      // leave with one bulk copy each
-      uint4* ih = reinterpret_cast<uint4*>(smem + PP_PHI + i * 128);
-      uint4* il = reinterpret_cast<uint4*>(smem + PP_PLO + i * 128);
-#pragma unroll
-      for (int v4 = 0; v4 < 4; ++v4) {
-        const int piece = (4 * colhalf + v4) ^ (i & 7);
-        ih[piece] = make_uint4(ph[4 * v4], ph[4 * v4 + 1], ph[4 * v4 + 2], ph[4 * v4 + 3]);
-        il[piece] = make_uint4(pl[4 * v4], pl[4 * v4 + 1], pl[4 * v4 + 2], pl[4 * v4 + 3]);
-      }
-      tc::fence_proxy_async_smem();
-    }
-  }
-  __syncthreads();
-  if (tid == 0 && ok) {
-    tc::bulk_store(out.p_hi + rec * (C * C), smem + PP_PHI, REC_P);
-    tc::bulk_store(out.p_lo + rec * (C * C), smem + PP_PLO, REC_P);
-    tc::bulk_commit();
-  }
-  // ---- T = (I + A)^-1 by 16x16 blocks.  With D = blockdiag(I + A_rr) and E = D^-1 (A - A_D) (strictly block lower,
-  // E^4 = 0):  T = (I - E + E^2 - E^3) D^-1.  Only the four small D_r^-1 need a sequential substitution.
-  if (tid < 64) {  // column k of (I + A_rr)^-1, 16 rows, one thread each
-    const int r = tid >> 4, k = tid & 15;
-    const float* Arr = Ab + tri(r, r) * BLK_FLOATS;
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float s0 = (i == k) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-      for (int j = 0; j < i; ++j) {
-        const float av = Arr[i * BLK_LD + j];
-        if (j & 1) s1 = fmaf(-av, x[j], s1); else s0 = fmaf(-av, x[j], s0);
-      }
-      x[i] = s0 + s1;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) Di[r * BLK_FLOATS + i * BLK_LD + k] = x[i];
-  } else if (tid < 128) {  // q's norms are no longer read: reuse their slot for the column factors of Tw
-    const int j = tid - 64;
-    fwv[j] = betas[j] * __expf(bs[j]) * kn[j];
-  }
-  if (tid == 0) tc::bulk_wait_read<0>();  // the P images have been read: the block scratch may overwrite them
-  __syncthreads();
-  // E_rc = D_r^-1 A_rc, r > c: six products, one warp each
-  if (warp < 6) {
-    constexpr int RR[6] = {1, 2, 2, 3, 3, 3}, CC[6] = {0, 0, 1, 0, 1, 2};
-    const int r = RR[warp], c = CC[warp];
-    float acc[2][4] = {};
-    const float* L = Di + r * BLK_FLOATS;
-    block_mma(acc, [&](int row, int col) { return L[row * BLK_LD + col]; }, Ab + tri(r, c) * BLK_FLOATS, lane);
-    block_store(Eb + (tri(r, c) - r) * BLK_FLOATS, acc, lane);  // strictly-lower block index: tri(r,c) - r
-  }
-  __syncthreads();
-  // E^2: (2,0) = E21 E10, (3,1) = E32 E21, (3,0) = E31 E10 + E32 E20
-  auto Eblk = [&](int r, int c) { return Eb + (tri(r, c) - r) * BLK_FLOATS; };
-  if (warp < 3) {
-    float acc[2][4] = {};
-    if (warp == 0) {
-      const float* L = Eblk(2, 1);
-      block_mma(acc, [&](int row, int col) { return L[row * BLK_LD + col]; }, Eblk(1, 0), lane);
-    } else if (warp == 1) {
-      const float* L = Eblk(3, 2);
-      block_mma(acc, [&](int row, int col) { return L[row * BLK_LD + col]; }, Eblk(2, 1), lane);
-    } else {
-      const float* L1 = Eblk(3, 1);
-      block_mma(acc, [&](int row, int col) { return L1[row * BLK_LD + col]; }, Eblk(1, 0), lane);
-      const float* L2 = Eblk(3, 2);
-      block_mma(acc, [&](int row, int col) { return L2[row * BLK_LD + col]; }, Eblk(2, 0), lane);
-    }
-    block_store(E2b + warp * BLK_FLOATS, acc, lane);  // order: (2,0), (3,1), (3,0)
-  }
-  __syncthreads();
-  // E^3: (3,0) = E32 E2_20
-  if (warp == 0) {
-    float acc[2][4] = {};
-    const float* L = Eblk(3, 2);
-    block_mma(acc, [&](int row, int col) { return L[row * BLK_LD + col]; }, E2b, lane);
-    block_store(E3b, acc, lane);
-  }
-  __syncthreads();
-  // T_rc = (-E + E^2 - E^3)_rc D_c^-1, r > c (written over A_rc, which is no longer needed); T_rr = D_r^-1
-  if (warp < 6) {
-    constexpr int RR[6] = {1, 2, 2, 3, 3, 3}, CC[6] = {0, 0, 1, 0, 1, 2};
-    const int r = RR[warp], c = CC[warp];
-    const float* e1 = Eblk(r, c);
-    const float* e2 = (r - c >= 2) ? E2b + ((r == 2) ? 0 : (c == 1 ? 1 : 2)) * BLK_FLOATS : nullptr;
-    const float* e3 = (r - c == 3) ? E3b : nullptr;
-    float acc[2][4] = {};
-    block_mma(acc, [&](int row, int col) {
-      float v = -e1[row * BLK_LD + col];
-      if (e2 != nullptr) v += e2[row * BLK_LD + col];
-      if (e3 != nullptr) v -= e3[row * BLK_LD + col];
-      return v;
-    }, Di + c * BLK_FLOATS, lane);
-    block_store(Ab + tri(r, c) * BLK_FLOATS, acc, lane);
-  }
-  __syncthreads();
-  // Tw = T diag(beta e^b kn) as bf16 hi + lo K-major tiles [i][j] with the 128-byte swizzle (B operand of the W MMA);
-  // Tu = T diag(beta) as bf16 hi + lo straight to scratch, in the same swizzled tile layout (the scan brings it in with
-  // a bulk copy).  A thread owns one 16-byte piece (8 columns) of two rows; a warp covers four full rows per store.
-  {
-    const int pc = tid & 7, cb = pc >> 1;
-    float fw[8], fu[8];
-    {
-      const float4 a0 = *reinterpret_cast<const float4*>(fwv + 8 * pc), a1 = *reinterpret_cast<const float4*>(fwv + 8 * pc + 4);
-      const float4 b0 = *reinterpret_cast<const float4*>(betas + 8 * pc), b1 = *reinterpret_cast<const float4*>(betas + 8 * pc + 4);
-      fw[0] = a0.x; fw[1] = a0.y; fw[2] = a0.z; fw[3] = a0.w; fw[4] = a1.x; fw[5] = a1.y; fw[6] = a1.z; fw[7] = a1.w;
-      fu[0] = b0.x; fu[1] = b0.y; fu[2] = b0.z; fu[3] = b0.w; fu[4] = b1.x; fu[5] = b1.y; fu[6] = b1.z; fu[7] = b1.w;
-    }
-    uint4* guh = reinterpret_cast<uint4*>(out.tu_hi + rec * (C * C));
-    uint4* gul = reinterpret_cast<uint4*>(out.tu_lo + rec * (C * C));
-#pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const int i = (tid >> 3) + 32 * it, rb = i >> 4;
-      float t[8];
-      if (cb <= rb) {
-        const float* src = ((rb == cb) ? Di + rb * BLK_FLOATS : Ab + tri(rb, cb) * BLK_FLOATS) + (i & 15) * BLK_LD + (pc & 1) * 8;
-        const float4 t0 = *reinterpret_cast<const float4*>(src), t1 = *reinterpret_cast<const float4*>(src + 4);
-        t[0] = t0.x; t[1] = t0.y; t[2] = t0.z; t[3] = t0.w; t[4] = t1.x; t[5] = t1.y; t[6] = t1.z; t[7] = t1.w;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) t[e] = (8 * pc + e <= i) ? t[e] : 0.f;
-      } else {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) t[e] = 0.f;
-      }
-      uint32_t wh[4], wl[4], uh[4], ul[4];
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const float2 tp = make_float2(t[2 * w], t[2 * w + 1]);
-        split_pair(__fmul2_rn(tp, make_float2(fw[2 * w], fw[2 * w + 1])), wh[w], wl[w]);
-        split_pair(__fmul2_rn(tp, make_float2(fu[2 * w], fu[2 * w + 1])), uh[w], ul[w]);
-      }
-      const uint32_t off = (uint32_t)(i * 128 + ((pc ^ (i & 7)) << 4));
-      *reinterpret_cast<uint4*>(smem + PP_TWH + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-      *reinterpret_cast<uint4*>(smem + PP_TWL + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
-      if (ok) {
-        guh[i * 8 + (pc ^ (i & 7))] = make_uint4(uh[0], uh[1], uh[2], uh[3]);  // same swizzled image as in shared memory
-        gul[i * 8 + (pc ^ (i & 7))] = make_uint4(ul[0], ul[1], ul[2], ul[3]);
-      }
-    }
-  }
-  tc::fence_proxy_async_smem();
-  __syncthreads();
-  constexpr uint32_t idesc_w = tc::idesc_f16(128, 64, 1, 1, true, false);  // A MN-major (token rows), B K-major
-  if (warp == 0) {
-    const bool leader = tc::elect_one();
-    if (ok && leader) {
-      const uint32_t kbase = tc::smem_u32(smem + PP_KQ);
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const uint32_t tw = tc::smem_u32(smem + (t ? PP_TWL : PP_TWH));
-#pragma unroll
-        for (int k = 0; k < 4; ++k)  // K halves sit 16384 bytes apart (the Q halves' slots lie between them)
-          tc::mma_ss(tm + PT_W, tc::smem_desc_sw128(kbase + k * 2048, 16384, 1024), tc::smem_desc_sw128(tw + k * 32, 16, 1024), idesc_w,
-                     (t | k) != 0 ? 1u : 0u);
-      }
-      tc::mma_commit(mma2_bar);
-    }
-    __syncwarp();
-  }
-  if (warp == 0) tc::mbar_wait_warp(mma2_bar, 0, abort_flag);
-  __syncthreads();
-  ok = ok && *abort_flag == 0u;
-  tc::tc_fence_after_sync();
-  {
-    // Each lane owns one row of W^T (a d_k index) and each warp half of its 64 tokens.  The K, Q and Tw tiles are dead
-    // now; the bf16 hi and lo rows are written over them in the 128-byte-swizzled tile layout the scan's MMA reads, so
-    // that the tile leaves with one bulk copy and arrives in the scan's shared memory with another, unchanged.
-    const int quarter = warp & 3, colhalf = warp >> 2;
-    const int r = quarter * 32 + lane;
-    uint32_t acc[32];
-    tc::tmem_ld32(tm + PT_W + ((uint32_t)(quarter * 32) << 16) + 32 * colhalf, acc);
-    tc::tmem_ld_wait();
-    uint4* ih = reinterpret_cast<uint4*>(smem + PP_WHI + r * 128);
-    uint4* il = reinterpret_cast<uint4*>(smem + PP_WLO + r * 128);
-#pragma unroll
-    for (int p4 = 0; p4 < 4; ++p4) {
-      uint32_t hi[4], lo[4];
-#pragma unroll
-      for (int w = 0; w < 4; ++w)
-        split_pair(make_float2(__uint_as_float(acc[8 * p4 + 2 * w]), __uint_as_float(acc[8 * p4 + 2 * w + 1])), hi[w], lo[w]);
-      const int piece = (4 * colhalf + p4) ^ (r & 7);
-      ih[piece] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      il[piece] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
-  }
-  tc::fence_proxy_async_smem();
-  tc::tc_fence_before_sync();
-  __syncthreads();
-  if (tid == 0 && ok) {
-    tc::bulk_store(out.w_hi + rec * (C * D), smem + PP_WHI, REC_W);
-    tc::bulk_store(out.w_lo + rec * (C * D), smem + PP_WLO, REC_W);
-    tc::bulk_commit();
-    tc::bulk_wait_read<0>();  // shared memory must stay intact until the copies have read it
-  }
-  if (warp == 2) {
-    tc::tc_fence_after_sync();
-    tc::tmem_dealloc(tm, 64);
-  }
-  if (!ok && tid == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
-}
+namespace ave {
+namespace {
 
 // ------------------------------------------------------------------------------------------------ pass 2
 // Warpgroup 0: warp 0 loader, warps 1 and 2 MMA issuers; warpgroups 1..NG: chain epilogue, each covering all 128 TMEM
@@ -1663,6 +1235,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   ScanPlan plan;
   plan.parts = L.parts;
   for (int p = 0; p <= MAX_PARTS; ++p) plan.part_begin[p] = L.part_begin[p];
+  const unsigned prep_rows = (unsigned)(a.Hk * ((a.Hv / a.Hk + 1) / 2));  // a pass-1 CTA takes up to two value heads of a key head
   const unsigned scan_grid = (unsigned)a.n_seqs * (unsigned)(2 * L.parts - 1) * (unsigned)a.Hv;
   const int part0_tokens = L.parts > 1 ? min(a.T, L.part_begin[1] * C) : a.T;  // tokens no fix-up touches (dense layout)
 
@@ -1700,7 +1273,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   if (side == nullptr) {
     // one launch per pass on the caller's stream
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
-    chunk_prep_kernel<<<dim3((unsigned)L.chunks, (unsigned)a.Hv), PREP_THREADS, PREP_SMEM, stream>>>(a, maps, chunk_start, po, plan, 0);
+    chunk_prep_kernel<<<dim3((unsigned)L.chunks, prep_rows), PREP_THREADS, PREP_SMEM, stream>>>(a, chunk_start, po, plan, 0);
     AVE_CUDA_TRY(cudaGetLastError());
     (L.parts > 1 ? chunk_scan_tc_kernel<true> : chunk_scan_tc_kernel<false>)<<<scan_grid, SCAN_THREADS, SCAN_SMEM, stream>>>(
         a, maps, chunk_start, po.w_hi, po.w_lo, po.p_hi, po.p_lo, po.tu_hi, po.tu_lo, po.scal, o_f32, qt_img, carry, m0_pack, seq_order, plan);
@@ -1727,8 +1300,8 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   for (int i = 0; i < L.segments && rc == AVE_GDN_OK; ++i) {
     plan.r0 = L.seg_begin[i]; plan.rn = L.seg_begin[i + 1] - L.seg_begin[i];
     if (plan.rn <= 0) continue;
-    chunk_prep_kernel<<<dim3((unsigned)(a.n_seqs * L.parts * plan.rn), (unsigned)a.Hv), PREP_THREADS, PREP_SMEM, side->prep>>>(
-        a, maps, chunk_start, po, plan, 1);
+    chunk_prep_kernel<<<dim3((unsigned)(a.n_seqs * L.parts * plan.rn), prep_rows), PREP_THREADS, PREP_SMEM, side->prep>>>(
+        a, chunk_start, po, plan, 1);
     if (!step(cudaGetLastError())) break;
     if (!step(cudaEventRecord(side->done[i], side->prep))) break;
     if (!step(cudaStreamWaitEvent(side->scan, side->done[i], 0))) break;
