@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB = os.path.join(HERE, "libave_gdn_b200.so")
 HOST = os.path.join(HERE, "_host.so")  # Python module: the host side of the public functions (csrc/host.cpp)
-SOURCES = ["api.cu", "decode.cu", "decode_layer.cu", "backward.cu", "rmsnorm.cu", "prefill_simt.cu", "elementwise.cu", "gemm.cu", "tmap.cu", "prefill_tc.cu"]
+SOURCES = ["api.cu", "decode.cu", "decode_layer.cu", "backward.cu", "rmsnorm.cu", "prefill_d64.cu", "elementwise.cu", "gemm.cu", "tmap.cu", "prefill_tc.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I" + INCLUDE,
               "-I" + CSRC]

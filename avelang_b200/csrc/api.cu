@@ -6,8 +6,8 @@ namespace ave {
 thread_local int g_last_cuda_error = 0;
 
 int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
-int launch_prefill_simt(const AveGdnArgs& a, cudaStream_t stream);
-size_t prefill_simt_workspace_bytes(const AveGdnArgs& a);
+int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream);
+size_t prefill_d64_workspace_bytes(const AveGdnArgs& a);
 int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain);
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain);
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain);
@@ -23,7 +23,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream);
 size_t backward_workspace_bytes(const AveGdnBwdArgs& a);
 
 static size_t prefill_ws_bytes(const AveGdnArgs& a) {
-  return a.dk == 128 ? prefill_tc_workspace_bytes(a, false) : prefill_simt_workspace_bytes(a);
+  return a.dk == 128 ? prefill_tc_workspace_bytes(a, false) : prefill_d64_workspace_bytes(a);
 }
 
 static int check_rows(const void* p, int64_t st, int64_t sh, int64_t sb, int elem_bytes) {
@@ -91,7 +91,7 @@ int ave_gdn_prefill_launch_count(const AveGdnArgs* args) {
   if (validate_gdn(args, true) != AVE_GDN_OK) return 0;
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return 0;
   if (args->dk == 128) return prefill_tc_launch_count(*args, false);
-  return (args->cu_seqlens ? 1 : 0) + 2 + (args->z ? 1 : 0);  // chunk table, two passes, gated norm
+  return 3;  // chunk tiles, chain of states, outputs (with the gated norm)
 }
 
 int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream) {
@@ -100,9 +100,9 @@ int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream) {
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return AVE_GDN_OK;
   if (args->workspace == nullptr || !aligned16(args->workspace)) return AVE_GDN_INVALID_ARGUMENT;
   if (args->workspace_bytes < prefill_ws_bytes(*args)) return AVE_GDN_WORKSPACE_TOO_SMALL;
-  // d = 128 runs on the tensor cores; d = 64 (the small CPU-reference shape) on the fp32 CUDA-core kernels
+  // d = 128 runs on the tcgen05 scan; d = 64 (the small CPU-reference shape) has a form of its own, with fp32 accuracy
   if (args->dk == 128) return launch_prefill_tc(*args, reinterpret_cast<cudaStream_t>(stream), false);
-  return launch_prefill_simt(*args, reinterpret_cast<cudaStream_t>(stream));
+  return launch_prefill_d64(*args, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int ave_gdn_decode_step(const AveGdnArgs* args, void* stream) {

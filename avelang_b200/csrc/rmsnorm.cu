@@ -150,12 +150,8 @@ int launch_gated_rmsnorm(const AveGdnNormArgs& a, cudaStream_t stream) {
   return launch_norm_t(reinterpret_cast<const __nv_bfloat16*>(a.x), a, stream);
 }
 
-// fp32 input variant used by the prefill path when the un-normalised output is staged in scratch
-int launch_gated_rmsnorm_f32in(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers, int64_t peer_off) {
-  return launch_norm_t(reinterpret_cast<const float*>(a.x), a, stream, peers, n_peers, peer_off);
-}
-
-// The same over `batches` batch rows in one launch: a.rows counts the rows of one batch row, the strides step between them.
+// fp32 input variant used by the prefill path when the un-normalised output is staged in scratch, over `batches` batch rows
+// in one launch: a.rows counts the rows of one batch row, the strides step between them.
 int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers,
                                        int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b) {
   return launch_norm_t(reinterpret_cast<const float*>(a.x), a, stream, peers, n_peers, peer_off, batches, xs_b, zs_b, ys_b);
