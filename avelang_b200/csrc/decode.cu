@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_kernel(const AveGdnArgs a) 
   const int col = (lane % C::kLanesPerRow) * 4;
   const int row0 = warp * C::kRowsPerWarp + lane / C::kLanesPerRow;
 
+  pdl_trigger();
+  pdl_wait();
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
   __nv_bfloat16* o_base = reinterpret_cast<__nv_bfloat16*>(a.o) + sp.b * a.o_stride_b + (int64_t)h * a.o_stride_h;
 
@@ -59,6 +61,7 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_kernel(const AveGdnArgs a) 
   float4 S[C::kLoads];
   if (a.initial_state != nullptr) {
     const float* src = a.initial_state + tile;
+    asm volatile("" : "+l"(src));  // keeps the streaming loads behind pdl_wait
 #pragma unroll
     for (int i = 0; i < C::kLoads; ++i)
       S[i] = __ldcs(reinterpret_cast<const float4*>(src + (row0 + i * C::kRowsPerLoad) * DV + col));
@@ -210,13 +213,17 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
   };
   auto tile_offset = [&](int t, int slot) -> int64_t { return ((int64_t)slot * a.Hv + (t % a.Hv)) * (int64_t)(DK * DV); };
 
-  int t = blockIdx.x;
-  if (t >= n_tiles) return;
-  int slot = slot_of(t);
+  pdl_trigger();
   if (threadIdx.x == 0) {
     tc::mbar_init(&full_bar, 1);
     abort_flag = 0;
     tc::fence_barrier_init();
+  }
+  pdl_wait();
+  int t = blockIdx.x;
+  if (t >= n_tiles) return;
+  int slot = slot_of(t);
+  if (threadIdx.x == 0) {
     if (slot >= 0) {
       tc::mbar_expect_tx(&full_bar, DK * DV * 4);
       tc::bulk_load(tile_s, a.initial_state + tile_offset(t, slot), DK * DV * 4, &full_bar);
@@ -363,11 +370,11 @@ int launch_decode(const AveGdnArgs& a, cudaStream_t stream) {
     }
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned persistent = (unsigned)(2 * sms);
-    gdn_decode_pool_kernel<<<grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream>>>(a, (int)grid);
+    AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel, grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream, a, (int)grid));
   } else if (a.dk == 128 && a.dv == 128) {
-    gdn_decode_kernel<128, 128><<<grid, 256, 0, stream>>>(a);
+    AVE_CUDA_TRY(launch_after(gdn_decode_kernel<128, 128>, grid, 256, 0, stream, a));
   } else if (a.dk == 64 && a.dv == 64) {
-    gdn_decode_kernel<64, 64><<<grid, 256, 0, stream>>>(a);
+    AVE_CUDA_TRY(launch_after(gdn_decode_kernel<64, 64>, grid, 256, 0, stream, a));
   } else {
     return AVE_GDN_UNSUPPORTED;
   }

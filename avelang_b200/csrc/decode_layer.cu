@@ -40,6 +40,13 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
   const __nv_bfloat16* cb = reinterpret_cast<const __nv_bfloat16*>(a.conv_bias);
   __nv_bfloat16* cstate = reinterpret_cast<__nv_bfloat16*>(a.conv_state);
 
+  pdl_trigger();
+  if (tid == 0) {
+    tc::mbar_init(&full_bar, 1);
+    abort_flag = 0;
+    tc::fence_barrier_init();
+  }
+  pdl_wait();
   if ((int)blockIdx.x >= n_units) return;
   const int n_local = ((n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * r;  // tiles this CTA walks
   auto unit_of = [&](int i) { return (int)blockIdx.x + (i / r) * (int)gridDim.x; };
@@ -70,9 +77,6 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
 
   int slot = slot_of_seq(unit_of(0) / a.Hk);
   if (tid == 0) {
-    tc::mbar_init(&full_bar, 1);
-    abort_flag = 0;
-    tc::fence_barrier_init();
     if (slot >= 0) {
       tc::mbar_expect_tx(&full_bar, DK * DV * 4);
       tc::bulk_load(tile_s, tile_ptr(slot, (unit_of(0) % a.Hk) * r), DK * DV * 4, &full_bar);
@@ -214,9 +218,9 @@ int launch_decode_layer(const AveGdnDecodeLayerArgs& a, cudaStream_t stream) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const unsigned grid = (unsigned)(units < 2 * sms ? units : 2 * sms);
   switch (a.width) {
-    case 2: gdn_decode_layer_kernel<2><<<grid, 256, DK * DV * 4, stream>>>(a, units); break;
-    case 3: gdn_decode_layer_kernel<3><<<grid, 256, DK * DV * 4, stream>>>(a, units); break;
-    case 4: gdn_decode_layer_kernel<4><<<grid, 256, DK * DV * 4, stream>>>(a, units); break;
+    case 2: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<2>, grid, 256, DK * DV * 4, stream, a, units)); break;
+    case 3: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<3>, grid, 256, DK * DV * 4, stream, a, units)); break;
+    case 4: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<4>, grid, 256, DK * DV * 4, stream, a, units)); break;
     default: return AVE_GDN_UNSUPPORTED;
   }
   AVE_CUDA_TRY(cudaGetLastError());

@@ -9,6 +9,7 @@ namespace ave {
 // the SMs can issue), so the arithmetic runs on packed fp32 pairs: one FFMA2 per tap and channel pair.
 template <int WIDTH>
 __global__ void __launch_bounds__(128) conv1d_silu_kernel(const AveConvArgs a, int tokens_per_cta) {
+  pdl_wait();
   const int cg = blockIdx.x * blockDim.x + threadIdx.x;  // channel group
   if (cg * 8 >= a.C) return;
   const int b = blockIdx.z;
@@ -102,9 +103,9 @@ int launch_conv1d_silu(const AveConvArgs& a, cudaStream_t stream) {
   const int tokens_per_cta = 64;
   dim3 grid((groups + threads - 1) / threads, (a.T + tokens_per_cta - 1) / tokens_per_cta, a.B);
   switch (a.width) {
-    case 2: conv1d_silu_kernel<2><<<grid, threads, 0, stream>>>(a, tokens_per_cta); break;
-    case 3: conv1d_silu_kernel<3><<<grid, threads, 0, stream>>>(a, tokens_per_cta); break;
-    case 4: conv1d_silu_kernel<4><<<grid, threads, 0, stream>>>(a, tokens_per_cta); break;
+    case 2: AVE_CUDA_TRY(launch_after(conv1d_silu_kernel<2>, grid, threads, 0, stream, a, tokens_per_cta)); break;
+    case 3: AVE_CUDA_TRY(launch_after(conv1d_silu_kernel<3>, grid, threads, 0, stream, a, tokens_per_cta)); break;
+    case 4: AVE_CUDA_TRY(launch_after(conv1d_silu_kernel<4>, grid, threads, 0, stream, a, tokens_per_cta)); break;
     default: return AVE_GDN_UNSUPPORTED;
   }
   AVE_CUDA_TRY(cudaGetLastError());
@@ -115,6 +116,8 @@ int launch_conv1d_silu(const AveConvArgs& a, cudaStream_t stream) {
 // is a coalesced 16-byte piece.
 template <int WIDTH>
 __global__ void __launch_bounds__(128) conv1d_update_kernel(const AveConvUpdateArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int cg = blockIdx.x * blockDim.x + threadIdx.x;
   const int n = blockIdx.y;
   if (cg * 8 >= a.C) return;
@@ -157,9 +160,9 @@ int launch_conv1d_update(const AveConvUpdateArgs& a, cudaStream_t stream) {
   if (a.n_seqs == 0 || a.C == 0) return AVE_GDN_OK;
   dim3 grid((a.C / 8 + 127) / 128, a.n_seqs);
   switch (a.width) {
-    case 2: conv1d_update_kernel<2><<<grid, 128, 0, stream>>>(a); break;
-    case 3: conv1d_update_kernel<3><<<grid, 128, 0, stream>>>(a); break;
-    case 4: conv1d_update_kernel<4><<<grid, 128, 0, stream>>>(a); break;
+    case 2: AVE_CUDA_TRY(launch_after(conv1d_update_kernel<2>, grid, 128, 0, stream, a)); break;
+    case 3: AVE_CUDA_TRY(launch_after(conv1d_update_kernel<3>, grid, 128, 0, stream, a)); break;
+    case 4: AVE_CUDA_TRY(launch_after(conv1d_update_kernel<4>, grid, 128, 0, stream, a)); break;
     default: return AVE_GDN_UNSUPPORTED;
   }
   AVE_CUDA_TRY(cudaGetLastError());
@@ -167,6 +170,8 @@ int launch_conv1d_update(const AveConvUpdateArgs& a, cudaStream_t stream) {
 }
 
 __global__ void __launch_bounds__(256) gate_beta_kernel(const AveGateArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t total = a.rows * a.Hv;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = e / a.Hv;
@@ -183,7 +188,7 @@ int launch_gate_beta(const AveGateArgs& a, cudaStream_t stream) {
   const int64_t total = a.rows * a.Hv;
   if (total == 0) return AVE_GDN_OK;
   const int64_t blocks = (total + 255) / 256;
-  gate_beta_kernel<<<(unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, stream>>>(a);
+  AVE_CUDA_TRY(launch_after(gate_beta_kernel, (unsigned)(blocks < 148 * 16 ? blocks : 148 * 16), 256, 0, stream, a));
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }

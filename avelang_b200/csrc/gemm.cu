@@ -72,6 +72,7 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -244,6 +245,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   const int rank = (int)(blockIdx.x % split), tile = (int)(blockIdx.x / split), tm = tile / nt, tn = tile % nt;
   const int per = (kb_count + split - 1) / split, kb0 = rank * per, kb1 = min(kb_count, kb0 + per);
 
+  pdl_trigger();
   if (threadIdx.x == 0) {
     for (int s = 0; s < stages; ++s) { tc::mbar_init(&full[s], 1); tc::mbar_init(&empty[s], 1); }
     tc::mbar_init(&acc_full, 1);
@@ -257,6 +259,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tmem_base = tmem_slot;
+  pdl_wait();
 
   // Both issuing warps run their loops whole and elect a lane for the instructions themselves.  A stage holds `ks` blocks
   // of 64 along K, [A][A].. [B][B].., behind one barrier: a wait, its loads or MMAs and the release cost about 700 cycles
@@ -498,22 +501,24 @@ int launch_gemm_bf16_nt_impl(const AveGemmArgs& a, cudaStream_t stream, const Ge
     uint32_t cols = 32;
     while ((int)cols < bn) cols *= 2;
     cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)sp.split; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)(((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) * sp.split));
     cfg.blockDim = dim3(GEMM_THREADS);
     cfg.dynamicSmemBytes = SKINNY_SMEM;
     cfg.stream = stream;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    cfg.attrs = at; cfg.numAttrs = 2;
     AVE_CUDA_TRY(cudaLaunchKernelEx(&cfg, gemm_skinny_kernel, tmA, tmB, reinterpret_cast<__nv_bfloat16*>(a.c), a.M, a.N, a.K, a.ldc, a.status,
                                     sp, cols));
     return AVE_GDN_OK;
   }
   const int64_t tiles = ((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn);
   const unsigned grid = (unsigned)(tiles < sms ? tiles : sms);
-  gemm_bf16_nt_kernel<<<grid, GEMM_THREADS, sc.dst != nullptr ? GEMM_SMEM_SCATTER : GEMM_SMEM, stream>>>(tmA, tmB, reinterpret_cast<__nv_bfloat16*>(a.c), a.M, a.N, a.K,
-                                                               a.ldc, a.status, bn, sc);
+  AVE_CUDA_TRY(launch_after(gemm_bf16_nt_kernel, grid, GEMM_THREADS, sc.dst != nullptr ? GEMM_SMEM_SCATTER : GEMM_SMEM, stream, tmA, tmB,
+                            reinterpret_cast<__nv_bfloat16*>(a.c), a.M, a.N, a.K, a.ldc, a.status, bn, sc));
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }

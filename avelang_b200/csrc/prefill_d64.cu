@@ -89,7 +89,7 @@ constexpr int PQ_Z1 = PQ_BLK;  // the blocks are dead when Z exists
 static_assert(PQ_Z1 + 3 * IMG <= PQ_BLK_END, "Z must fit where the blocks were");
 constexpr int PQ_SC = PQ_BLK_END, PQ_SMEM = PQ_SC + SC_FLOATS * 4;
 
-__global__ void __launch_bounds__(THREADS) d64_prep_kernel(const AveGdnArgs a, uint8_t* __restrict__ recs) {
+__global__ void __launch_bounds__(THREADS) d64_prep_kernel(const AveGdnArgs a, uint8_t* recs) {
   extern __shared__ __align__(1024) uint8_t smem[];
   float* Ab = reinterpret_cast<float*>(smem + PQ_A);
   float* Di = reinterpret_cast<float*>(smem + PQ_D);
@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(THREADS) d64_prep_kernel(const AveGdnArgs a, u
   float* bs = reinterpret_cast<float*>(smem + PQ_SC);
   float *betas = bs + CH, *qn = bs + 3 * CH, *kn = bs + 4 * CH;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  pdl_trigger();
+  pdl_wait();
   if (!offsets_ok(a, blockIdx.x == 0 && h == 0)) return;
   const Chunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
@@ -319,10 +321,12 @@ __global__ void __launch_bounds__(THREADS) d64_prep_kernel(const AveGdnArgs a, u
 constexpr int CN_T = 128, CN_ROWS = 16, CN_LD = DH + 4;
 constexpr int CN_PHI = 0, CN_GAM = DH * DH * 4, CN_STAGE = CN_GAM + CN_ROWS * DH * 4, CN_SMEM = 3 * CN_STAGE;
 
-__global__ void __launch_bounds__(CN_T) d64_chain_kernel(const AveGdnArgs a, uint8_t* __restrict__ recs) {
+__global__ void __launch_bounds__(CN_T) d64_chain_kernel(const AveGdnArgs a, uint8_t* recs) {
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(16) float Hs[2][CN_ROWS][CN_LD];
   const int tid = threadIdx.x, n = blockIdx.x, h = blockIdx.y, row0 = blockIdx.z * CN_ROWS;
+  pdl_trigger();
+  pdl_wait();
   if (!offsets_ok(a, false)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok) return;
@@ -406,9 +410,11 @@ __global__ void __launch_bounds__(CN_T) d64_chain_kernel(const AveGdnArgs a, uin
 constexpr int OT_K = 0, OT_Q = 8192, OT_V = 16384, OT_T = 24576, OT_P = OT_T + 3 * IMG, OT_H = OT_P + 3 * IMG, OT_X = OT_H + 3 * IMG,
               OT_SC = OT_X + 3 * IMG, OT_RED = OT_SC + SC_FLOATS * 4, OT_SMEM = OT_RED + 2 * CH * 4;
 
-__global__ void __launch_bounds__(THREADS) d64_out_kernel(const AveGdnArgs a, const uint8_t* __restrict__ recs) {
+__global__ void __launch_bounds__(THREADS) d64_out_kernel(const AveGdnArgs a, const uint8_t* recs) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  pdl_trigger();
+  pdl_wait();
   if (!offsets_ok(a, false)) return;
   const Chunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
@@ -561,12 +567,9 @@ int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream) {
   }
   uint8_t* recs = reinterpret_cast<uint8_t*>(a.workspace);
   const dim3 chunks((unsigned)d64_slots(a), (unsigned)a.Hv);
-  d64_prep_kernel<<<chunks, THREADS, PQ_SMEM, stream>>>(a, recs);
-  AVE_CUDA_TRY(cudaGetLastError());
-  d64_chain_kernel<<<dim3((unsigned)a.n_seqs, (unsigned)a.Hv, DH / CN_ROWS), CN_T, CN_SMEM, stream>>>(a, recs);
-  AVE_CUDA_TRY(cudaGetLastError());
-  d64_out_kernel<<<chunks, THREADS, OT_SMEM, stream>>>(a, recs);
-  AVE_CUDA_TRY(cudaGetLastError());
+  AVE_CUDA_TRY(launch_after(d64_prep_kernel, chunks, THREADS, PQ_SMEM, stream, a, recs));
+  AVE_CUDA_TRY(launch_after(d64_chain_kernel, dim3((unsigned)a.n_seqs, (unsigned)a.Hv, DH / CN_ROWS), CN_T, CN_SMEM, stream, a, recs));
+  AVE_CUDA_TRY(launch_after(d64_out_kernel, chunks, THREADS, OT_SMEM, stream, a, recs));
   return AVE_GDN_OK;
 }
 

@@ -166,10 +166,12 @@ __device__ __forceinline__ void prep_row(uint8_t* smem, int hh, int lane, bool l
 }
 
 __global__ void __launch_bounds__(PREP_THREADS, 2)
-chunk_prep_kernel(const AveGdnArgs a, const int32_t* __restrict__ chunk_start, PrepOut out, const __grid_constant__ ScanPlan plan,
+chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, const __grid_constant__ ScanPlan plan,
                   int compact_grid) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  pdl_trigger();
+  pdl_wait();
   // Whole-batch launches index every chunk of the batch; range launches use the compact grid
   // n_seqs x parts x rn so that no CTA is spent on chunks outside the range.
   int c = blockIdx.x;

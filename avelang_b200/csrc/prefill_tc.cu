@@ -63,10 +63,12 @@ __device__ __forceinline__ ChunkRef find_chunk(const AveGdnArgs& a, const int32_
 // (every CTA of the following launches tests it and leaves) and the status word gets AVE_GDN_DEV_BAD_SEQLEN.
 // Everything behind this launch waits for it, so it is all latency: a block scan by shuffles and a warp per sequence for
 // the map take 3 us where a serial sum and map took 7.5 us (one sequence) to 13 us (64 sequences, 4123 chunks).
-__global__ void chunk_table_tc_kernel(const int32_t* __restrict__ cu_seqlens, int n_seqs, int T, int32_t* __restrict__ chunk_start,
+__global__ void chunk_table_tc_kernel(const int32_t* cu_seqlens, int n_seqs, int T, int32_t* chunk_start,
                                       int max_chunks, uint32_t* __restrict__ status) {
   __shared__ int part[1024], first[1024], warp_sum_s[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, threads = blockDim.x, warps = threads >> 5;
+  pdl_trigger();
+  pdl_wait();
   const int per = (n_seqs + threads - 1) / threads;
   const int lo = min(tid * per, n_seqs), hi = min(lo + per, n_seqs);
   int s = 0, bad = 0;
@@ -213,12 +215,12 @@ __device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint3
 // state, which keeps the output warpgroup inside its register budget with 32-token pieces.
 template <bool kMulti>
 __global__ void __launch_bounds__(SCAN_THREADS, 1)
-chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, const int32_t* __restrict__ chunk_start,
-                     const __nv_bfloat16* __restrict__ w_hi_ws, const __nv_bfloat16* __restrict__ w_lo_ws,
-                     const __nv_bfloat16* __restrict__ p_hi_ws, const __nv_bfloat16* __restrict__ p_lo_ws,
-                     const __nv_bfloat16* __restrict__ tu_hi_ws, const __nv_bfloat16* __restrict__ tu_lo_ws,
-                     const float* __restrict__ scal_ws, float* __restrict__ o_f32, uint8_t* __restrict__ qt_img,
-                     float* __restrict__ carry, uint8_t* __restrict__ m0_pack, const int32_t* __restrict__ seq_order,
+chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, const int32_t* chunk_start,
+                     const __nv_bfloat16* w_hi_ws, const __nv_bfloat16* w_lo_ws,
+                     const __nv_bfloat16* p_hi_ws, const __nv_bfloat16* p_lo_ws,
+                     const __nv_bfloat16* tu_hi_ws, const __nv_bfloat16* tu_lo_ws,
+                     const float* scal_ws, float* o_f32, uint8_t* qt_img,
+                     float* carry, uint8_t* m0_pack, const int32_t* seq_order,
                      const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -245,6 +247,7 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
   // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
   // chain of part p >= 1 (see ScanPlan).
   const int chains = kMulti ? 2 * plan.parts - 1 : 1;
@@ -343,6 +346,7 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
     if (lane == 0) {
       for (int c = 0; c < n_chunks; ++c) {
         const int s = c & 1;
+        if (c == n_chunks - 1) pdl_trigger();
         const uint32_t free_par = ((uint32_t)(c >> 1) & 1u) ^ 1u;  // parity of "chunk c-2 is done with it"
         uint8_t* st = smem + s * STAGE;
         const int64_t rec = (int64_t)(c_first + c) * a.Hv + h;
@@ -715,11 +719,13 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
 constexpr int COMBINE_COLS = 8, COMBINE_PITCH = 129;
 constexpr size_t COMBINE_SMEM = (size_t)D * COMBINE_PITCH * 4;
 __global__ void __launch_bounds__(256)
-part_combine_kernel(const AveGdnArgs a, const int32_t* __restrict__ chunk_start, const float* __restrict__ carry,
-                    uint8_t* __restrict__ m0_pack, const __grid_constant__ ScanPlan plan) {
+part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry,
+                    uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ float Fs[];  // [D][COMBINE_PITCH]
   __shared__ __align__(16) float cur[2][D][COMBINE_COLS];
   const int cb = blockIdx.x, h = blockIdx.y, n = blockIdx.z, tid = threadIdx.x;
+  pdl_trigger();
+  pdl_wait();
   if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
@@ -804,8 +810,8 @@ constexpr int FIN_PITCH = 132;  // floats per staged row: 16-byte aligned rows t
 constexpr int FIN_A = 0, FIN_B = 65536, FIN_STAGE = FIN_B + PACK_BYTES, FIN_BARS = FIN_STAGE + 128 * FIN_PITCH * 4;
 constexpr size_t FIN_SMEM = FIN_BARS + 64 + 1024;
 __global__ void __launch_bounds__(FIN_THREADS, 1)
-part_finish_kernel(const AveGdnArgs a, const int32_t* __restrict__ chunk_start, const float* __restrict__ o_f32,
-                   const uint8_t* __restrict__ qt_img, const uint8_t* __restrict__ m0_pack, const __grid_constant__ ScanPlan plan) {
+part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* o_f32,
+                   const uint8_t* qt_img, const uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   float* stage = reinterpret_cast<float*>(smem + FIN_STAGE);  // [128 tokens][FIN_PITCH] product rows
@@ -817,6 +823,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* __restrict__ chunk_start, 
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = blockIdx.z / (plan.parts - 1), part = 1 + blockIdx.z % (plan.parts - 1);
+  pdl_wait();
   if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
@@ -1224,8 +1231,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     dev.attr_set = true;
   }
   if (a.cu_seqlens != nullptr) {
-    chunk_table_tc_kernel<<<1, a.n_seqs <= 256 ? 256 : 1024, 0, stream>>>(a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status);
-    AVE_CUDA_TRY(cudaGetLastError());
+    AVE_CUDA_TRY(launch_after(chunk_table_tc_kernel, 1, a.n_seqs <= 256 ? 256 : 1024, 0, stream, a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status));
   }
   float* o_f32 = (a.z != nullptr || L.parts > 1) ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
   uint8_t* qt_img = L.parts > 1 ? reinterpret_cast<uint8_t*>(ws + L.qt_img) : nullptr;
@@ -1273,11 +1279,9 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   if (side == nullptr) {
     // one launch per pass on the caller's stream
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
-    chunk_prep_kernel<<<dim3((unsigned)L.chunks, prep_rows), PREP_THREADS, PREP_SMEM, stream>>>(a, chunk_start, po, plan, 0);
-    AVE_CUDA_TRY(cudaGetLastError());
-    (L.parts > 1 ? chunk_scan_tc_kernel<true> : chunk_scan_tc_kernel<false>)<<<scan_grid, SCAN_THREADS, SCAN_SMEM, stream>>>(
-        a, maps, chunk_start, po.w_hi, po.w_lo, po.p_hi, po.p_lo, po.tu_hi, po.tu_lo, po.scal, o_f32, qt_img, carry, m0_pack, seq_order, plan);
-    AVE_CUDA_TRY(cudaGetLastError());
+    AVE_CUDA_TRY(launch_after(chunk_prep_kernel, dim3((unsigned)L.chunks, prep_rows), PREP_THREADS, PREP_SMEM, stream, a, chunk_start, po, plan, 0));
+    AVE_CUDA_TRY(launch_after(L.parts > 1 ? chunk_scan_tc_kernel<true> : chunk_scan_tc_kernel<false>, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps,
+                              chunk_start, po.w_hi, po.w_lo, po.p_hi, po.p_lo, po.tu_hi, po.tu_lo, po.scal, o_f32, qt_img, carry, m0_pack, seq_order, plan));
     if (a.z != nullptr) {
       // packed layouts: the norm covers every row (rows of later parts are rewritten by the fix-up, which runs after it)
       const int rc = norm_rows(a, o_f32, a.token_begin, a.cu_seqlens ? a.T : part0_tokens, stream);

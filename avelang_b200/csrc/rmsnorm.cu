@@ -16,12 +16,13 @@ struct NormBatch {
 // streaming helpers the kernel is bound by instruction issue before HBM, so the math runs on packed fp32 pairs and
 // tensors whose rows are evenly spaced (`flat`) skip the per-row index divisions.
 template <int D, typename XT>
-__global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* __restrict__ x, const __nv_bfloat16* __restrict__ z,
-                                                            const float* __restrict__ w, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const __nv_bfloat16* z,
+                                                            const float* w, __nv_bfloat16* y,
                                                             int64_t rows, int heads, int64_t xs_t, int64_t xs_h,
                                                             int64_t zs_t, int64_t zs_h, int64_t ys_t, int64_t ys_h,
-                                                            float eps, int gate_first, const void* const* __restrict__ peers,
+                                                            float eps, int gate_first, const void* const* peers,
                                                             int n_peers, int64_t peer_off, NormBatch nb, int flat) {
+  pdl_wait();
   constexpr int E = D / 16;  // elements per lane: 8 or 4
   constexpr int P = E / 2;   // pairs per lane
   constexpr int U = 2;       // rows in flight per half-warp
@@ -134,11 +135,11 @@ static int launch_norm_t(const XT* x, const AveGdnNormArgs& a, cudaStream_t stre
   const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(a.z);
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y);
   if (a.d == 128) {
-    gated_rmsnorm_kernel<128, XT><<<grid, 256, 0, stream>>>(x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb, flat);
+    AVE_CUDA_TRY(launch_after(gated_rmsnorm_kernel<128, XT>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
+                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb, flat));
   } else if (a.d == 64) {
-    gated_rmsnorm_kernel<64, XT><<<grid, 256, 0, stream>>>(x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, nullptr, 0, 0, nb, flat);
+    AVE_CUDA_TRY(launch_after(gated_rmsnorm_kernel<64, XT>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
+                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, (const void* const*)nullptr, 0, (int64_t)0, nb, flat));
   } else {
     return AVE_GDN_UNSUPPORTED;
   }
