@@ -137,7 +137,7 @@ struct GdnMaps {
 //           so that the missing contribution is M0(p)^T qt_t: one GEMM per part once M0(p) is known.
 //   ranges: independently, a launch covers only the chunk offsets [r0, r0 + rn) inside every part, so that pass 1 of a
 //           later range runs while pass 2 walks an earlier one; a chain's state crosses launches in the carry buffer.
-constexpr int MAX_PARTS = 8;
+constexpr int MAX_PARTS = 16;
 struct ScanPlan {
   int parts;
   int part_begin[MAX_PARTS + 1];  // part_begin[parts] = 1 << 24
@@ -713,16 +713,18 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
 // Serial combine over the parts of one (sequence, value head, 8-column slice of d_v): M0(1) = state after part 0,
 // M0(p+1) = F_p M0(p) + Psi_p in fp32 on the CUDA cores; the last one is the sequence's final state.  M0(p) for p >= 2
 // also leaves as the bf16 hi/lo operand image the fix-up kernel's MMAs read (B[d_v][k]); the image of M0(1) was written
-// by the scan itself.  The steps are serial, so each is kept short: F_p is staged in shared memory with coalesced loads
-// (row pitch 129: a thread walks its own row without bank conflicts) and the tile of the next step is already in
-// registers while the current one is multiplied.
-constexpr int COMBINE_COLS = 8, COMBINE_PITCH = 129;
-constexpr size_t COMBINE_SMEM = (size_t)D * COMBINE_PITCH * 4;
+// by the scan itself.  The steps are serial and everything behind them waits, so each is kept short: the next F lands in
+// shared memory by asynchronous copies while this one is multiplied (row pitch 132: 16-byte reads of eight rows meet eight
+// different bank groups), and a thread takes two rows, four columns and half of the contraction, which needs six 16-byte
+// reads for 32 multiply-adds.  Fifteen steps: 44 us, 55 us with one row a thread, scalar reads
+// and F staged through registers.
+constexpr int COMBINE_COLS = 8, COMBINE_PITCH = 132;
+constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 1) * COMBINE_COLS * 4;  // (a gap of one row between the halves)
+constexpr int COMBINE_STAGES = 3;
+constexpr size_t COMBINE_SMEM = COMBINE_STAGES * (size_t)COMBINE_F + 2 * COMBINE_CUR;
 __global__ void __launch_bounds__(256)
-part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry,
-                    uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
-  extern __shared__ float Fs[];  // [D][COMBINE_PITCH]
-  __shared__ __align__(16) float cur[2][D][COMBINE_COLS];
+part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int cb = blockIdx.x, h = blockIdx.y, n = blockIdx.z, tid = threadIdx.x;
   pdl_trigger();
   pdl_wait();
@@ -738,50 +740,68 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   if (active == 2 && a.final_state == nullptr) return;  // nothing to produce
   const int chains = 2 * plan.parts - 1;
   auto tile_of = [&](int chain) { return carry + (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D); };
-  {
-    const float* src = tile_of(0);
-    for (int e = tid; e < D * COMBINE_COLS; e += 256) cur[0][e / COMBINE_COLS][e % COMBINE_COLS] = src[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS];
-  }
-  // a thread fetches 16 float4 of the 128x128 tile: element 4 * (tid + 256 i), i.e. row (tid + 256 i) / 32
-  float4 pre[16], psi_pre;
-  auto fetch = [&](int p) {
-    const float4* F4 = reinterpret_cast<const float4*>(tile_of(2 * p));
+  auto cur_at = [&](int b, int k, int j) -> float& {
+    return reinterpret_cast<float*>(smem_raw + COMBINE_STAGES * COMBINE_F + b * COMBINE_CUR)[(k + (k >> 6)) * COMBINE_COLS + j];
+  };
+  const uint32_t sb = tc::smem_u32(smem_raw);
+  // this thread: rows k and k + 64, columns j0 .. j0 + 3, contraction indices d0 .. d0 + 63
+  const int dh = tid & 1, j0 = ((tid >> 1) & 1) * 4, k = tid >> 2, d0 = dh * 64;
+  auto fetch = [&](int p) {  // F_p into buffer p % 3
+    if (p >= active) { cp_commit(); return; }
+    const float* F = tile_of(2 * p);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) pre[i] = F4[tid + 256 * i];
-    psi_pre = *reinterpret_cast<const float4*>(tile_of(2 * p - 1) + (int64_t)(tid >> 1) * D + cb * COMBINE_COLS + (tid & 1) * 4);
+    for (int i = 0; i < D * D / 4 / 256; ++i) {
+      const int e = tid + 256 * i, row = e >> 5, c4 = e & 31;
+      cp16(sb + (p % COMBINE_STAGES) * COMBINE_F + row * COMBINE_PITCH * 4 + c4 * 16, F + 4 * e, true);
+    }
+    cp_commit();
+  };
+  auto psi_of = [&](int p) {
+    return p < active ? *reinterpret_cast<const float4*>(tile_of(2 * p - 1) + (int64_t)(k + 64 * dh) * D + cb * COMBINE_COLS + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   fetch(1);
+  fetch(2);
+  float4 psi_next = psi_of(1);
+  for (int e = tid; e < D * COMBINE_COLS; e += 256) cur_at(0, e / COMBINE_COLS, e % COMBINE_COLS) = tile_of(0)[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS];
   int b = 0;
   for (int p = 1; p < active; ++p) {
-    __syncthreads();  // the previous step's readers of Fs are done
+    cp_wait<1>();
+    __syncthreads();  // F_p and cur are complete; F_{p-1} has been read
+    fetch(p + 2);
+    const float4 psi = psi_next;
+    psi_next = psi_of(p + 1);
+    const float* F0 = reinterpret_cast<const float*>(smem_raw + (p % COMBINE_STAGES) * COMBINE_F) + k * COMBINE_PITCH + d0;
+    float2 x[2][2] = {};
+#pragma unroll 4
+    for (int d = 0; d < 64; d += 4) {
+      const float4 f0 = *reinterpret_cast<const float4*>(F0 + d), f1 = *reinterpret_cast<const float4*>(F0 + 64 * COMBINE_PITCH + d);
+      const float fa[4] = {f0.x, f0.y, f0.z, f0.w}, fb[4] = {f1.x, f1.y, f1.z, f1.w};
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int e = 4 * (tid + 256 * i), row = e >> 7, c0 = e & 127;
-      float* dst = Fs + row * COMBINE_PITCH + c0;
-      dst[0] = pre[i].x; dst[1] = pre[i].y; dst[2] = pre[i].z; dst[3] = pre[i].w;
-    }
-    const float4 psi = psi_pre;
-    if (p + 1 < active) fetch(p + 1);
-    __syncthreads();
-    {  // next = F_p cur + Psi_p: a thread owns one row k and four columns
-      const int k = tid >> 1, j0 = (tid & 1) * 4;
-      const float* Frow = Fs + k * COMBINE_PITCH;
-      float acc0 = psi.x, acc1 = psi.y, acc2 = psi.z, acc3 = psi.w;
-#pragma unroll 16
-      for (int d = 0; d < D; ++d) {
-        const float f = Frow[d];
-        const float4 c4 = *reinterpret_cast<const float4*>(&cur[b][d][j0]);
-        acc0 = fmaf(f, c4.x, acc0); acc1 = fmaf(f, c4.y, acc1); acc2 = fmaf(f, c4.z, acc2); acc3 = fmaf(f, c4.w, acc3);
+      for (int e = 0; e < 4; ++e) {
+        const float4 c4 = *reinterpret_cast<const float4*>(&cur_at(b, d0 + d + e, j0));
+        x[0][0] = __ffma2_rn(make_float2(fa[e], fa[e]), make_float2(c4.x, c4.y), x[0][0]);
+        x[0][1] = __ffma2_rn(make_float2(fa[e], fa[e]), make_float2(c4.z, c4.w), x[0][1]);
+        x[1][0] = __ffma2_rn(make_float2(fb[e], fb[e]), make_float2(c4.x, c4.y), x[1][0]);
+        x[1][1] = __ffma2_rn(make_float2(fb[e], fb[e]), make_float2(c4.z, c4.w), x[1][1]);
       }
-      *reinterpret_cast<float4*>(&cur[b ^ 1][k][j0]) = make_float4(acc0, acc1, acc2, acc3);
+    }
+    {  // the two halves of the contraction meet; each of the two threads finishes one of the two rows
+      float v[8] = {x[0][0].x, x[0][0].y, x[0][1].x, x[0][1].y, x[1][0].x, x[1][0].y, x[1][1].x, x[1][1].y};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float mine = dh ? v[4 + i] : v[i], other = dh ? v[i] : v[4 + i];
+        v[i] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+      }
+      *reinterpret_cast<float4*>(&cur_at(b ^ 1, k + 64 * dh, j0)) = make_float4(v[0] + psi.x, v[1] + psi.y, v[2] + psi.z, v[3] + psi.w);
     }
     b ^= 1;
+    if (p + 1 == active) break;
     __syncthreads();
-    if (p + 1 < active && tid < 128) {  // operand image of M0(p+1): B[row = d_v][k] = M0[k][d_v]; a 16-byte piece of hi and of lo
+    if (tid < 128) {  // operand image of M0(p+1): B[row = d_v][k] = M0[k][d_v]; a 16-byte piece of hi and of lo
       const int k8 = tid >> 3, v = tid & 7;
       uint32_t hi[4], lo[4];
 #pragma unroll
-      for (int w = 0; w < 4; ++w) split_pair(make_float2(cur[b][8 * k8 + 2 * w][v], cur[b][8 * k8 + 2 * w + 1][v]), hi[w], lo[w]);
+      for (int w = 0; w < 4; ++w) split_pair(make_float2(cur_at(b, 8 * k8 + 2 * w, v), cur_at(b, 8 * k8 + 2 * w + 1, v)), hi[w], lo[w]);
       uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1) + p) * a.Hv + h) * (int64_t)PACK_BYTES;
       const uint32_t off = kmajor_piece_off(cb * COMBINE_COLS + v, k8);
       *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
@@ -791,7 +811,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   __syncthreads();
   if (a.final_state != nullptr) {
     float* dst = a.final_state + ((int64_t)slot * a.Hv + h) * (int64_t)(D * D);
-    for (int e = tid; e < D * COMBINE_COLS; e += 256) dst[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS] = cur[b][e / COMBINE_COLS][e % COMBINE_COLS];
+    for (int e = tid; e < D * COMBINE_COLS; e += 256) dst[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS] = cur_at(b, e / COMBINE_COLS, e % COMBINE_COLS);
   }
 }
 
@@ -877,6 +897,23 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
     const int c0 = c_begin + 2 * pair;
     const int64_t tok0 = sp.t0 + (int64_t)c0 * C;
     const int rows = min(min(2, c_end - c0) * C, sp.len - c0 * C);
+    // the rows this half-warp will stream (hw, hw + 32, hw + 64, hw + 96) are fetched before the product is waited for
+    float4 ol[4][2];
+    uint4 zraw[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = hw + 32 * u;
+      ol[u][0] = ol[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+      zraw[u] = make_uint4(0u, 0u, 0u, 0u);
+      if (!skipped && r < rows) {
+        const float* src = o_f32 + (((int64_t)sp.b * a.T + tok0 + r) * a.Hv + h) * D + 8 * sub;
+        ol[u][0] = *reinterpret_cast<const float4*>(src);
+        ol[u][1] = *reinterpret_cast<const float4*>(src + 4);
+      }
+      if (a.z != nullptr && r < rows)
+        zraw[u] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.z) + sp.b * a.z_stride_b +
+                                                  (tok0 + r) * a.z_stride_t + (int64_t)h * a.z_stride_h + 8 * sub);
+    }
     if (!skipped) {
       if (warp == 0) {
         bool landed = it > 0 || tc::mbar_wait_warp(b_bar, 0, abort_flag);
@@ -915,28 +952,17 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
     ok = __syncthreads_and(ok ? 1 : 0) != 0;  // staged rows complete; the accumulator is free for the next product
     tc::tc_fence_after_sync();
     if (ok) {
-      // streaming pass: this half-warp takes token rows hw, hw + 32, hw + 64, hw + 96
       float2 x[4][4];
-      uint4 zraw[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int r = hw + 32 * u;
-        const bool live = r < rows;
-        if (!skipped && live) {
-          const float* ol = o_f32 + (((int64_t)sp.b * a.T + tok0 + r) * a.Hv + h) * D + 8 * sub;
-          const float4 o0 = *reinterpret_cast<const float4*>(ol), o1 = *reinterpret_cast<const float4*>(ol + 4);
-          const float4 p0 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub);
-          const float4 p1 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub + 4);
-          x[u][0] = make_float2(o0.x + p0.x, o0.y + p0.y); x[u][1] = make_float2(o0.z + p0.z, o0.w + p0.w);
-          x[u][2] = make_float2(o1.x + p1.x, o1.y + p1.y); x[u][3] = make_float2(o1.z + p1.z, o1.w + p1.w);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) x[u][i] = make_float2(0.f, 0.f);
+        float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
+        if (!skipped && r < rows) {
+          p0 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub);
+          p1 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub + 4);
         }
-        zraw[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (a.z != nullptr && live)
-          zraw[u] = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(a.z) + sp.b * a.z_stride_b +
-                                                    (tok0 + r) * a.z_stride_t + (int64_t)h * a.z_stride_h + 8 * sub);
+        x[u][0] = make_float2(ol[u][0].x + p0.x, ol[u][0].y + p0.y); x[u][1] = make_float2(ol[u][0].z + p0.z, ol[u][0].w + p0.w);
+        x[u][2] = make_float2(ol[u][1].x + p1.x, ol[u][1].y + p1.y); x[u][3] = make_float2(ol[u][1].z + p1.z, ol[u][1].w + p1.w);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
@@ -982,7 +1008,8 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
 }
 
 // ------------------------------------------------------------------------------------------------ schedule and scratch
-constexpr int SEG_FIRST_DIV = 16;   // first range = 1/16 of the longest chain's chunks
+constexpr int SEG_FIRST_DIV = 6;    // first range = 1/6 of the longest chain's chunks (64 heads, 4096 tokens: 290 us; 1/16: 328)
+constexpr int SEG_FIRST_DIV_PARTS = 4;  // with parts the chains are short and pass 1 is the critical resource
 constexpr int SEG_GROWTH_X4 = 12;   // each range 3x the one before (in quarters)
 constexpr int SEG_MAX = 8;
 constexpr int PART0_X4 = 4;         // length of part 0 in quarters of a later part's length
@@ -1028,11 +1055,11 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   if (!plain && !push && max_chunks >= 32) {
     const int64_t per_head = (NUM_SMS / (heads_total > 0 ? heads_total : 1) + 1) / 2;  // chains per head that still get an SM each: 2S - 1
     int S = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
-    while (S > 1 && max_chunks / S < 16) --S;
-    // Two parts only halve the walk and pay for it with a third as many chains again plus the fix-up of half the rows:
-    // measured break-even (32 heads, 8192 tokens: 0.46 ms either way).  From three parts on the cut wins: 4 / 8 / 16 heads
-    // at 32768 tokens run 3.0x / 2.0x / 1.3x faster than the plain chain.
-    L.parts = S >= 3 ? S : 1;
+    while (S > 1 && max_chunks / S < 8) --S;  // a part of fewer chunks costs more in combine and fix-up than it saves
+    // Two parts take three chains a head: worth it while pass 1 keeps a third of the SMs (32 heads, 8192 tokens: 399 us
+    // against 433; 48 heads, 6000 tokens: 411 against 386).  4 / 8 / 16 heads at 32768 tokens: 285 / 437 / 778 us with up to
+    // 16 parts, 391 / 514 / 861 with up to 8 and a slower combine.
+    L.parts = S >= 3 || (S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3) ? S : 1;
   }
   L.part_begin[0] = 0;
   {
@@ -1063,7 +1090,8 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
     // With the fused all-gather the gated norm of a range also pushes that range's rows to every peer over NVLink,
     // which takes about as long as the chain itself; only the last range's push is exposed, so the ranges are equal
     // and as many as the event pool allows instead of growing.
-    int len = push ? (part_len + SEG_MAX - 1) / SEG_MAX : max(1, (part_len + SEG_FIRST_DIV - 1) / SEG_FIRST_DIV);
+    const int first_div = L.parts > 1 ? SEG_FIRST_DIV_PARTS : SEG_FIRST_DIV;
+    int len = push ? (part_len + SEG_MAX - 1) / SEG_MAX : max(1, (part_len + first_div - 1) / first_div);
     L.segments = 0;
     while (L.seg_begin[L.segments] < part_len) {
       int next = L.seg_begin[L.segments] + len;
