@@ -172,6 +172,7 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   pdl_trigger();
   pdl_wait();
+  if (batch_rejected(a, chunk_start, blockIdx.x == 0 && blockIdx.y == 0)) return;
   // Whole-batch launches index every chunk of the batch; range launches use the compact grid
   // n_seqs x parts x rn so that no CTA is spent on chunks outside the range.
   int c = blockIdx.x;
@@ -179,10 +180,9 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
     const int per_seq = plan.parts * plan.rn;
     const int n = blockIdx.x / per_seq, rest = blockIdx.x % per_seq;
     const int cis = plan.part_begin[rest / plan.rn] + plan.r0 + rest % plan.rn;
-    if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;  // table rejected
-    const int per = a.cu_seqlens ? (chunk_start[n + 1] - chunk_start[n]) : (a.T + C - 1) / C;
+    const int per = ((a.cu_seqlens ? a.cu_seqlens[n + 1] - a.cu_seqlens[n] : a.T) + C - 1) / C;
     if (cis >= per || cis >= plan.part_begin[rest / plan.rn + 1]) return;
-    c = (a.cu_seqlens ? chunk_start[n] : n * per) + cis;
+    c = first_record(a, chunk_start, n) + cis;
   }
   const ChunkRef cr = find_chunk(a, chunk_start, c);  // (a compact grid only ever names chunks of this launch's range)
   if (!cr.ok) return;

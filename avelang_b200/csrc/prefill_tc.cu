@@ -38,6 +38,26 @@ struct PrepOut {
 
 struct ChunkRef { int n, b, t0, len, cis; bool ok; };  // cis: index of the chunk inside its sequence
 
+// Records are numbered by chunk.  A packed batch comes with chunk tables (see below) or, when all of its chains run at once
+// anyway, without (chunk_start == nullptr): then sequence n starts at record floor(first token / 64) + n, which leaves gaps
+// but needs no launch in front of pass 1, and the sequence of a record is found by bisection.
+__device__ __forceinline__ int first_record(const AveGdnArgs& a, const int32_t* chunk_start, int n) {
+  if (a.cu_seqlens == nullptr) return n * ((a.T + C - 1) / C);
+  return chunk_start != nullptr ? chunk_start[n] : a.cu_seqlens[n] / C + n;
+}
+// Whether the offsets of a packed batch are not monotone inside [0, T]: nothing runs then.  Called by whole warps.
+__device__ __forceinline__ bool batch_rejected(const AveGdnArgs& a, const int32_t* chunk_start, bool flag = false) {
+  if (a.cu_seqlens == nullptr) return false;
+  if (chunk_start != nullptr) return chunk_start[a.n_seqs] < 0;
+  bool bad = false;
+  for (int n = threadIdx.x & 31; n < a.n_seqs; n += 32) {
+    const int x = a.cu_seqlens[n], y = a.cu_seqlens[n + 1];
+    bad |= x < 0 || y < x || y > a.T;
+  }
+  bad = __any_sync(0xffffffffu, bad);
+  if (bad && flag && threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_BAD_SEQLEN);
+  return bad;
+}
 __device__ __forceinline__ ChunkRef find_chunk(const AveGdnArgs& a, const int32_t* chunk_start, int c) {
   ChunkRef r; r.ok = false;
   if (a.cu_seqlens == nullptr) {
@@ -48,11 +68,20 @@ __device__ __forceinline__ ChunkRef find_chunk(const AveGdnArgs& a, const int32_
     r.t0 = r.cis * C; r.len = min(C, a.T - r.t0); r.ok = true;
     return r;
   }
-  if (c >= chunk_start[a.n_seqs]) return r;
-  const int lo = chunk_start[a.n_seqs + 1 + c];  // chunk -> sequence map, stored behind the prefix table
+  int lo = 0;
+  if (chunk_start != nullptr) {
+    if (c >= chunk_start[a.n_seqs]) return r;
+    lo = chunk_start[a.n_seqs + 1 + c];  // chunk -> sequence map, stored behind the prefix table
+  } else {
+    int hi = a.n_seqs;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (a.cu_seqlens[mid] / C + mid <= c) lo = mid; else hi = mid;
+    }
+  }
   const int s0 = a.cu_seqlens[lo], s1 = a.cu_seqlens[lo + 1];
   if (s0 < 0 || s1 < s0 || s1 > a.T) return r;
-  r.n = lo; r.b = 0; r.cis = c - chunk_start[lo]; r.t0 = s0 + r.cis * C; r.len = min(C, s1 - r.t0); r.ok = r.len > 0;
+  r.n = lo; r.b = 0; r.cis = c - first_record(a, chunk_start, lo); r.t0 = s0 + r.cis * C; r.len = min(C, s1 - r.t0); r.ok = r.cis >= 0 && r.len > 0;
   return r;
 }
 
@@ -258,7 +287,7 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
   const int part = (chain + 1) >> 1;
   const bool phi = kMulti && chain > 0 && (chain & 1) == 0;
   const int hk = h / (a.Hv / a.Hk);
-  if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;  // the chunk table was rejected: nothing runs
+  if (batch_rejected(a, chunk_start)) return;
   SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
   // longer than the caller's bound: the launch schedule was sized from that bound, so the sequence is skipped (zero
   // output, no state access, like a negative slot) and flagged
@@ -313,7 +342,7 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
   if (c_lo >= c_hi) return;  // finished in an earlier launch, or not reached yet
   const bool seg_first = plan.r0 == 0;
   const bool seg_last = c_hi == part_end && !multi;
-  const int c_first = (a.cu_seqlens ? chunk_start[n] : n * ((a.T + C - 1) / C)) + c_lo;
+  const int c_first = first_record(a, chunk_start, n) + c_lo;
   sp.t0 += c_lo * C;
   sp.len = min(sp.len - c_lo * C, (c_hi - c_lo) * C);
   const int n_chunks = c_hi - c_lo;
@@ -728,7 +757,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   const int cb = blockIdx.x, h = blockIdx.y, n = blockIdx.z, tid = threadIdx.x;
   pdl_trigger();
   pdl_wait();
-  if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;
+  if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
   const int seq_chunks = (sp.len + C - 1) / C;
@@ -844,7 +873,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = blockIdx.z / (plan.parts - 1), part = 1 + blockIdx.z % (plan.parts - 1);
   pdl_wait();
-  if (a.cu_seqlens != nullptr && chunk_start[a.n_seqs] < 0) return;
+  if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
   const int seq_chunks = (sp.len + C - 1) / C;
@@ -853,7 +882,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   if ((int)blockIdx.x >= n_pairs) return;
   const int slot = a.state_indices ? a.state_indices[n] : n;
   const bool skipped = slot < 0 || slot >= a.num_slots;  // the scan skipped the sequence: its rows are zero
-  const int64_t rec0 = a.cu_seqlens ? chunk_start[n] : (int64_t)n * ((a.T + C - 1) / C);  // record of the sequence's chunk 0
+  const int64_t rec0 = first_record(a, chunk_start, n);  // record of the sequence's chunk 0
   const int stride = gridDim.x;
 
   auto load_qt = [&](int pair) {  // called by one thread
@@ -1113,15 +1142,20 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
 int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers,
                                        int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b);
 
+// More chains than SMs: the scan's launch order matters (longest first), so the tables are built.  32 heads, 203 tokens:
+// 33.1 us with them.
+static bool needs_tables(const AveGdnArgs& a) { return a.cu_seqlens != nullptr && (int64_t)a.n_seqs * a.Hv > NUM_SMS; }
+
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain) { return ws_layout(a, plain).total; }
 
 // Kernels one call enqueues, mirroring launch_prefill_tc below.
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain) {
   const WsLayout L = ws_layout(a, plain);
   if (L.chunks == 0 || a.n_seqs == 0) return 0;
+  const bool tables = needs_tables(a);
   const bool push = a.o_peers != nullptr && a.n_peers > 1;
   const int norm_launch = (push || a.B == 1) ? 1 : a.B;  // norm_rows: one launch, or one per batch row
-  int n = a.cu_seqlens != nullptr ? 1 : 0;                 // chunk table
+  int n = tables ? 1 : 0;                                  // chunk tables
   n += 2 * L.segments;                                     // pass 1 and pass 2 of every range
   if (a.z != nullptr) n += (a.cu_seqlens == nullptr ? L.segments : 1) * norm_launch;
   if (L.parts > 1) n += 2;                                 // combine and fix-up
@@ -1220,7 +1254,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   const WsLayout L = ws_layout(a, plain);
   if (L.chunks == 0 || a.n_seqs == 0) return AVE_GDN_OK;
   char* ws = reinterpret_cast<char*>(a.workspace);
-  int32_t* chunk_start = reinterpret_cast<int32_t*>(ws + L.chunk_start);
+  int32_t* chunk_start = needs_tables(a) ? reinterpret_cast<int32_t*>(ws + L.chunk_start) : nullptr;
   PrepOut po;
   po.w_hi = reinterpret_cast<__nv_bfloat16*>(ws + L.w_hi);
   po.w_lo = reinterpret_cast<__nv_bfloat16*>(ws + L.w_lo);
@@ -1258,14 +1292,14 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
     dev.attr_set = true;
   }
-  if (a.cu_seqlens != nullptr) {
+  if (chunk_start != nullptr) {
     AVE_CUDA_TRY(launch_after(chunk_table_tc_kernel, 1, a.n_seqs <= 256 ? 256 : 1024, 0, stream, a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status));
   }
   float* o_f32 = (a.z != nullptr || L.parts > 1) ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
   uint8_t* qt_img = L.parts > 1 ? reinterpret_cast<uint8_t*>(ws + L.qt_img) : nullptr;
   float* carry = reinterpret_cast<float*>(ws + L.carry);
   uint8_t* m0_pack = reinterpret_cast<uint8_t*>(ws + L.m0_pack);
-  const int32_t* seq_order = a.cu_seqlens ? chunk_start + a.n_seqs + 1 + L.chunks : nullptr;
+  const int32_t* seq_order = chunk_start != nullptr ? chunk_start + a.n_seqs + 1 + L.chunks : nullptr;
   ScanPlan plan;
   plan.parts = L.parts;
   for (int p = 0; p <= MAX_PARTS; ++p) plan.part_begin[p] = L.part_begin[p];
