@@ -353,14 +353,17 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
   const int hh = warp >> 2;
   if (hh >= nh) return;
   const int64_t rec = (int64_t)c * a.Hv + h0 + hh;
-  const bool lead = (warp & 3) == 3 && lane == 0;  // in the warp with the least work
+  // Block row R of T costs R + 1 units of work and the warps 0 and 4, 1 and 5, ... share a scheduler, so the second head
+  // hands its rows out in the opposite order
+  const int row = hh == 0 ? 3 - warp : warp - 4;
+  const bool lead = row == 0 && lane == 0;  // in the warp with the least work
   if (lead) {
     tc::bulk_store(out.p_hi + rec * (C * C), smem + PP_R + hh * 16384, REC_P);
     tc::bulk_store(out.p_lo + rec * (C * C), smem + PP_R + hh * 16384 + REC_P, REC_P);
     tc::bulk_commit();
   }
-  if ((warp & 3) < 2) {  // column k of (I + A_bb)^-1, one lane each: 4 blocks x 16 columns over two warps
-    const int b = 2 * (warp & 1) + (lane >> 4), k = lane & 15;
+  if (row >= 2) {  // column k of (I + A_bb)^-1, one lane each: 4 blocks x 16 columns over two warps
+    const int b = 2 * (row & 1) + (lane >> 4), k = lane & 15;
     float* ad = reinterpret_cast<float*>(smem + PP_F + hh * PP_F_HEAD + PF_AD) + b * 16 * AD_LD;
     float x[16];
 #pragma unroll
@@ -382,10 +385,10 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
       *reinterpret_cast<float4*>(ad + k * AD_LD + 4 * i4) = make_float4(x[4 * i4], x[4 * i4 + 1], x[4 * i4 + 2], x[4 * i4 + 3]);
   }
   head_sync(hh);
-  switch (warp & 3) {
-    case 0: prep_row<3>(smem, hh, lane, lead, out, rec); break;
-    case 1: prep_row<2>(smem, hh, lane, lead, out, rec); break;
-    case 2: prep_row<1>(smem, hh, lane, lead, out, rec); break;
+  switch (row) {
+    case 3: prep_row<3>(smem, hh, lane, lead, out, rec); break;
+    case 2: prep_row<2>(smem, hh, lane, lead, out, rec); break;
+    case 1: prep_row<1>(smem, hh, lane, lead, out, rec); break;
     default: prep_row<0>(smem, hh, lane, lead, out, rec); break;
   }
 }
