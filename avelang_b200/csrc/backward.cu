@@ -18,14 +18,14 @@
 // after chunk; bwd_reverse: the state gradients and Ut, chunk after chunk from the end (it needs nothing of bwd_forward).
 // bwd_grads: everything else, in parallel over (chunk, key head), summing over the value heads that share the key head.
 //
-// The contractions run on warp-level bf16 MMAs with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
+// The contractions run on warp-level bf16 MMAs (most of bwd_grads: on tcgen05) with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
 // every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with one fp32 operand is
 // three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which the gradient of
 // the gate needs, because it is a difference of large sums.
 // The scans hold the state transposed, H = M^T: a warp owns 16 of the 128 d_v rows for the whole sequence, every product
 // is (its rows) x (a tile all warps read), and the accumulator of one product is, in place, the left operand of the next,
 // so the warps of a chain never exchange anything and only meet where a tile buffer is refilled.
-// Two sequences of 4096 tokens, 32 value heads: 1.49 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.73)
+// Two sequences of 4096 tokens, 32 value heads: 1.33 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.57)
 // against 22.1 ms for the token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
 #include "blockalg.cuh"
 #include "common.cuh"
@@ -502,11 +502,19 @@ __global__ void __launch_bounds__(SC_T, 1) bwd_reverse_kernel(const AveGdnBwdArg
 }
 
 // ---------------------------------------------------------------------------------------------- the gradients of one chunk
-// 16 warps; a warp owns 32 tokens x 16 d_k columns of dQ and dK.  M0 and E, each element used by exactly one warp column
-// (two warps), go from global memory straight into right-operand registers; everything several warps read is a tile.
-constexpr int GR_T = 512;
-constexpr int GR_K = 0, GR_Q = 16384, GR_DO = 32768, GR_VN = 49152, GR_U = GR_VN + 3 * 16384, GR_X = GR_U + 3 * 16384,
-              GR_Y = GR_X + 3 * IMG, GR_RED = GR_Y + 3 * IMG, GR_SC = GR_RED + 8 * BCH * 20, GR_SMEM = GR_SC + SC_BYTES + 64;
+// One CTA of 16 warps per (chunk, key head).  Seven of the nine products contract over a whole tile and run on tcgen05, transposed
+// (128 d_k lanes x 64 tokens, so that the tile that differs per product is the narrow operand): dO M0^T, Ut M0^T and Vn E^T
+// over d_v, and X K, Y K, X^T Q + Y^T K over the tokens.  fp32 operands are three bf16 tiles each.  M0 and E pass through shared
+// memory 16 d_v rows at a time, split on the way in; while the tensor core works on one such step the warps fetch and split the
+// next and do the same d_v rows of X and Y (lower triangles, 16 x 8 blocks) on warp-level MMAs.
+// Two sequences of 4096 tokens, 32 value heads: 0.57 ms; all of it on warp-level MMAs, at 16 cycles each, took 0.73.
+constexpr int GR_T = 512, GR_DV = 16, GR_TERM = GR_DV * BD * 2, GR_STAGE = 6 * GR_TERM;
+constexpr int GR_K = 0, GR_Q = 16384, GR_DO = 32768, GR_VN = 49152, GR_U = GR_VN + 3 * 16384, GR_ST = GR_U + 3 * 16384,
+              GR_X = GR_ST, GR_Y = GR_X + 3 * IMG,  // X and Y take the place of the two stages once those are consumed
+              GR_RED = GR_ST + 2 * GR_STAGE, GR_UV = GR_RED + 4 * BCH * 16, GR_SC = GR_UV + 8 * BCH * 4, GR_F = GR_SC + SC_BYTES + 96,
+              GR_BAR = GR_F + 3 * BCH * 4, GR_SMEM = GR_BAR + 64;
+static_assert(GR_Y + 3 * IMG <= GR_RED && GR_SMEM <= 227 * 1024, "shared memory");
+enum { TG_Q = 0, TG_R = 64, TG_S = 128, TG_XK = 192, TG_YK = 256, TG_COL = 320, TG_DQ = 384, TG_DK = 448 };  // tensor-memory columns
 
 // fp32 [128][64] -> three bf16 tiles of 128-byte rows
 __device__ __forceinline__ void split_tile(uint8_t* dst, const float* src, int tid) {
@@ -523,17 +531,52 @@ __device__ __forceinline__ void split_tile(uint8_t* dst, const float* src, int t
     *reinterpret_cast<uint2*>(p + 32768) = make_uint2(l[0], l[1]);
   }
 }
+// four adjacent fp32 of row `row` (d_v) of a 16-row step -> the three tiles of the step, [128 d_k / 64][16 rows][128 bytes]
+__device__ __forceinline__ void split_step(uint8_t* dst, const float4& x, int row, int lane) {
+  uint32_t h[2], m[2], l[2];
+  split3(make_float2(x.x, x.y), h[0], m[0], l[0]);
+  split3(make_float2(x.z, x.w), h[1], m[1], l[1]);
+  uint8_t* p = dst + (lane >> 4) * (GR_TERM / 2) + piece<128>(row, (lane & 15) >> 1) + 8 * (lane & 1);
+  *reinterpret_cast<uint2*>(p) = make_uint2(h[0], h[1]);
+  *reinterpret_cast<uint2*>(p + GR_TERM) = make_uint2(m[0], m[1]);
+  *reinterpret_cast<uint2*>(p + 2 * GR_TERM) = make_uint2(l[0], l[1]);
+}
 __device__ __forceinline__ float quad_sum(float x) {
   x += __shfl_xor_sync(0xffffffffu, x, 1);
   return x + __shfl_xor_sync(0xffffffffu, x, 2);
 }
-// per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16
+// v[lane] of the 32 values summed over the lanes
+__device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int i = 0; i < o; ++i) {
+      const float give = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+      v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  return v[0];
+}
+// Per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16: eight tokens
+// of one d_k column per lane.
 template <bool kSum>
-__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const BwdChunk& c, int head, int tok, int col, float x, float y) {
-  if (tok >= c.len) return;
-  const int64_t row = (int64_t)c.b * a.T + c.t0 + tok;
-  if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(dst) + (row * a.Hk + head) * BD + col) = pack_bf16x2(x, y);
-  else *reinterpret_cast<float2*>(dst + (row * a.Hv + head) * BD + col) = make_float2(x, y);
+__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const BwdChunk& c, int head, int tok0, int dk, const float (&x)[8]) {
+  const int64_t row = (int64_t)c.b * a.T + c.t0 + tok0;
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) {
+    if (kSum) {  // even lanes store token i, odd lanes token i + 1, two columns each
+      const bool odd = dk & 1;
+      const float y = __shfl_xor_sync(0xffffffffu, odd ? x[i] : x[i + 1], 1);
+      const int j = i + (odd ? 1 : 0);
+      if (tok0 + j < c.len)
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(dst) + ((row + j) * a.Hk + head) * BD + (dk & ~1)) =
+            odd ? pack_bf16x2(y, x[i + 1]) : pack_bf16x2(x[i], y);
+    } else {
+      if (tok0 + i < c.len) dst[((row + i) * a.Hv + head) * BD + dk] = x[i];
+      if (tok0 + i + 1 < c.len) dst[((row + i + 1) * a.Hv + head) * BD + dk] = x[i + 1];
+    }
+  }
 }
 
 template <bool kSum>
@@ -545,77 +588,163 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
   const BwdChunk c = chunk_of_slot(a, slot);
   if (!c.ok) return;
   const uint32_t sb = tc::smem_u32(smem);
-  float* red = reinterpret_cast<float*>(smem + GR_RED);  // [8 column blocks][64 tokens][q.dq, k.row, k.col, k.state, u.v]
+  float4* red = reinterpret_cast<float4*>(smem + GR_RED);  // [4 d_k quarters][64 tokens]: q.dq, k.row, k.col, k.state
+  float* uv = reinterpret_cast<float*>(smem + GR_UV);      // [8 d_v blocks][64 tokens]: u.v
   float* bs = reinterpret_cast<float*>(smem + GR_SC);
   float* betas = bs + BCH;
-  float* dots = bs + 3 * BCH;  // [8] partial <E, M0>, then [8] the carry of the suffix sum
-  const int wm = warp & 1, wn = warp >> 1;  // token half, 16-column block
+  float* dots = bs + 3 * BCH;  // [16] partial <E, M0>; after the sums are taken, [8..11] carry the suffix sum
+  float* fac = reinterpret_cast<float*>(smem + GR_F);      // per token: factors of dO M0^T, Ut M0^T, Vn E^T
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GR_BAR);  // the two stages, and everything
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + GR_BAR + 32);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + GR_BAR + 40);
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) tc::mbar_init(&bars[i], 1);
+    *abort_flag = 0u;
+    tc::fence_barrier_init();
+  }
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
+  const int wm = warp & 1, wn = warp >> 1;  // dV: token half, 16 d_v columns
   const int64_t row0 = (int64_t)c.b * a.T + c.t0;
 
-  load_tile<BCH, 16, GR_T>(sb + GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
-  load_tile<BCH, 16, GR_T>(sb + GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
-  float dq[2][2][4], dk[2][2][4];  // [16-token tile][8-column tile], summed over the value heads
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 2; ++j) { zero(dq[i][j]); zero(dk[i][j]); }
+  auto load_half_tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
+    load_tile<BCH, 8, GR_T>(sb + at, src, stride, c.len, tid);
+    load_tile<BCH, 8, GR_T>(sb + at + 8192, src + 64, stride, c.len, tid);
+  };
+  load_half_tiles(GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t);
+  load_half_tiles(GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t);
+  uint32_t tm = 0;
+  uint32_t phase = 0;  // bit i: parity of the next completion of bars[i]
 
 #pragma unroll 1
   for (int hh = 0; hh < r; ++hh) {
     const int h = hk * r + hh;
     const int64_t rec = slot * a.Hv + h;
     if (hh > 0) __syncthreads();  // the tiles and sums of the previous head are no longer read
-    load_tile<BCH, 16, GR_T>(sb + GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t, c.len, tid);
+    load_half_tiles(GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t);
     cp_commit();
+    const float4* hp = reinterpret_cast<const float4*>(ws.m0 + rec * STATE_FLOATS) + tid;  // row warp of a step, columns 4 lane ..
+    const float4* ep = reinterpret_cast<const float4*>(ws.e + rec * STATE_FLOATS) + tid;
+    float4 hx[2], ex[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) { hx[s] = __ldcs(hp + s * GR_T); ex[s] = __ldcs(ep + s * GR_T); }
     split_tile(smem + GR_VN, ws.vn + rec * VEC_FLOATS, tid);
     split_tile(smem + GR_U, ws.u + rec * VEC_FLOATS, tid);
     if (tid < 3 * BCH) bs[tid] = reinterpret_cast<const float*>(ws.prep + rec * PREP_BYTES + PREP_SC)[tid];
     cp_wait<0>();
+    tc::tc_fence_before_sync();
     __syncthreads();
-
-    {  // X = S lower(dO Vn^T) o G and Y = -beta strict_lower(Ut Vn^T) o G: warp = (16-row tile, column tiles nq and nq + 4)
-      const int m = warp >> 2, nq = warp & 3, last = 2 * m + 1;
-      if (nq <= last) {
-        float ax[2][4], ay[2][4];
-        zero(ax[0]); zero(ax[1]); zero(ay[0]); zero(ay[1]);
-        const bool two = nq + 4 <= last;
-#pragma unroll 2
-        for (int ks = 0; ks < 8; ++ks) {
-          uint32_t o[4], uh[4], um[4], ul[4], vh[4], vm[4], vl[4];
-          ldsm4(o, sb + GR_DO + at_a<256>(16 * m, 2 * ks, lane));
-          const uint32_t ua = sb + GR_U + at_at<128>(16 * ks, 2 * m, lane);
-          ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
-          const uint32_t va = sb + GR_VN + piece<128>(16 * ks + (lane & 15), nq + 4 * (lane >> 4));
-          ldsm4t(vh, va); ldsm4t(vm, va + 16384); ldsm4t(vl, va + 32768);
+    tc::tc_fence_after_sync();
+    tm = *tmem_slot;
+    if (tid < BCH) {
+      const float eb = __expf(bs[tid]), be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
+      fac[tid] = a.scale * eb;
+      fac[BCH + tid] = -be * eb;
+      fac[2 * BCH + tid] = gate_between(bs, BCH - 1, tid);
+    }
+    // X = S lower(dO Vn^T) o G and Y = -beta strict_lower(Ut Vn^T) o G: warp = (16-row tile, column tiles nq and nq + 4)
+    const int m = warp >> 2, nq = warp & 3, last = 2 * m + 1;
+    float ax[2][4], ay[2][4], dot = 0.f;
+    zero(ax[0]); zero(ax[1]); zero(ay[0]); zero(ay[1]);
+#pragma unroll 1
+    for (int s0 = 0; s0 < 8; s0 += 2)
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            if (e == 1 && !two) break;
-            mma_bf16(ax[e], o, vh[2 * e], vh[2 * e + 1]);
-            mma_bf16(ax[e], o, vm[2 * e], vm[2 * e + 1]);
-            mma_bf16(ax[e], o, vl[2 * e], vl[2 * e + 1]);
-            mma6(ay[e], uh, um, ul, vh[2 * e], vh[2 * e + 1], vm[2 * e], vm[2 * e + 1], vl[2 * e], vl[2 * e + 1]);
-          }
+    for (int st = 0; st < 2; ++st) {
+      const int s = s0 + st;
+      uint8_t* stage = smem + GR_ST + st * GR_STAGE;
+      if (s >= 2) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
+      split_step(stage, hx[st], warp, lane);
+      split_step(stage + 3 * GR_TERM, ex[st], warp, lane);
+      dot = fmaf(hx[st].x, ex[st].x, fmaf(hx[st].y, ex[st].y, fmaf(hx[st].z, ex[st].z, fmaf(hx[st].w, ex[st].w, dot))));
+      if (s < 6) { hx[st] = __ldcs(hp + (s + 2) * GR_T); ex[st] = __ldcs(ep + (s + 2) * GR_T); }
+      tc::fence_proxy_async_smem();
+      __syncthreads();
+      if (warp == 3 && tc::elect_one()) {  // a warp without blocks of X and Y
+        constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true);
+        const uint32_t so = sb + GR_ST + st * GR_STAGE;
+        uint64_t mo[3], eo[3], u[3], v[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          mo[i] = tc::smem_desc_sw128(so + i * GR_TERM, GR_TERM / 2, 1024);
+          eo[i] = tc::smem_desc_sw128(so + (3 + i) * GR_TERM, GR_TERM / 2, 1024);
+          u[i] = tc::smem_desc_sw128(sb + GR_U + i * 16384 + s * 2048, 8192, 1024);
+          v[i] = tc::smem_desc_sw128(sb + GR_VN + i * 16384 + s * 2048, 8192, 1024);
         }
+        const uint64_t o = tc::smem_desc_sw128(sb + GR_DO + (s >> 2) * 8192 + (s & 3) * 32, 16, 1024);
+        const uint32_t acc = s > 0 ? 1u : 0u;
+        // ordered so that neighbours write different accumulators
+        tc::mma_ss(tm + TG_R, mo[0], u[0], id_mn, acc); tc::mma_ss(tm + TG_S, eo[0], v[0], id_mn, acc); tc::mma_ss(tm + TG_Q, mo[0], o, id_k, acc);
+        tc::mma_ss(tm + TG_R, mo[0], u[1], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[0], v[1], id_mn, 1u); tc::mma_ss(tm + TG_Q, mo[1], o, id_k, 1u);
+        tc::mma_ss(tm + TG_R, mo[1], u[0], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[1], v[0], id_mn, 1u); tc::mma_ss(tm + TG_Q, mo[2], o, id_k, 1u);
+        tc::mma_ss(tm + TG_R, mo[0], u[2], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[0], v[2], id_mn, 1u);
+        tc::mma_ss(tm + TG_R, mo[2], u[0], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[2], v[0], id_mn, 1u);
+        tc::mma_ss(tm + TG_R, mo[1], u[1], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[1], v[1], id_mn, 1u);
+        tc::mma_commit(&bars[st]);
+      }
+      __syncwarp();
+      if (nq <= last) {
+        uint32_t o[4], uh[4], um[4], ul[4], vh[4], vm[4], vl[4];
+        ldsm4(o, sb + GR_DO + (s >> 2) * 8192 + at_a<128>(16 * m, 2 * (s & 3), lane));
+        const uint32_t ua = sb + GR_U + at_at<128>(16 * s, 2 * m, lane);
+        ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
+        const uint32_t va = sb + GR_VN + piece<128>(16 * s + (lane & 15), nq + 4 * (lane >> 4));
+        ldsm4t(vh, va); ldsm4t(vm, va + 16384); ldsm4t(vl, va + 32768);
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
-          if (e == 1 && !two) break;
-          const int nt = nq + 4 * e;
-#pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
-            const float e0 = gate_between(bs, i, j), e1 = gate_between(bs, i, j + 1);
-            const float be = -(fabsf(betas[i]) < 1e-20f ? 1e-20f : betas[i]);
-            uint32_t xh, xm, xl;
-            uint8_t* dst = smem + GR_X + piece<128>(i, nt) + 4 * t;
-            split3(make_float2(i >= j ? a.scale * e0 * ax[e][2 * half] : 0.f, i > j ? a.scale * e1 * ax[e][2 * half + 1] : 0.f), xh, xm, xl);
-            *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
-            dst += GR_Y - GR_X;
-            split3(make_float2(i > j ? be * e0 * ay[e][2 * half] : 0.f, i > j + 1 ? be * e1 * ay[e][2 * half + 1] : 0.f), xh, xm, xl);
-            *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
-          }
+          if (e == 1 && nq + 4 > last) break;
+          mma_bf16(ax[e], o, vh[2 * e], vh[2 * e + 1]);
+          mma_bf16(ax[e], o, vm[2 * e], vm[2 * e + 1]);
+          mma_bf16(ax[e], o, vl[2 * e], vl[2 * e + 1]);
+          mma6(ay[e], uh, um, ul, vh[2 * e], vh[2 * e + 1], vm[2 * e], vm[2 * e + 1], vl[2 * e], vl[2 * e + 1]);
         }
       }
     }
+    dot = warp_sum(dot);
+    if (lane == 0) dots[warp] = dot;
+#pragma unroll
+    for (int st = 0; st < 2; ++st) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
+    // X and Y take the place of the stages; blocks above the diagonal are zero
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int nt = nq + 4 * e;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
+        float2 x = make_float2(0.f, 0.f), y = x;
+        if (nt <= last) {
+          const float e0 = gate_between(bs, i, j), e1 = gate_between(bs, i, j + 1);
+          const float be = -(fabsf(betas[i]) < 1e-20f ? 1e-20f : betas[i]);
+          x = make_float2(i >= j ? a.scale * e0 * ax[e][2 * half] : 0.f, i > j ? a.scale * e1 * ax[e][2 * half + 1] : 0.f);
+          y = make_float2(i > j ? be * e0 * ay[e][2 * half] : 0.f, i > j + 1 ? be * e1 * ay[e][2 * half + 1] : 0.f);
+        }
+        uint32_t xh, xm, xl;
+        uint8_t* dst = smem + GR_X + piece<128>(i, nt) + 4 * t;
+        split3(x, xh, xm, xl);
+        *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
+        dst += GR_Y - GR_X;
+        split3(y, xh, xm, xl);
+        *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
+      }
+    }
+    tc::fence_proxy_async_smem();
+    __syncthreads();
+    if (warp == 3 && tc::elect_one()) {
+      constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true);
+#pragma unroll 1
+      for (int ks = 0; ks < 4; ++ks) {
+        const uint64_t ka = tc::smem_desc_sw128(sb + GR_K + ks * 2048, 8192, 1024), qa = tc::smem_desc_sw128(sb + GR_Q + ks * 2048, 8192, 1024);
+        const uint32_t acc = ks > 0 ? 1u : 0u;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const uint32_t x = sb + GR_X + i * IMG, y = sb + GR_Y + i * IMG, more = i > 0 ? 1u : acc;
+          tc::mma_ss(tm + TG_XK, ka, tc::smem_desc_sw128(x + ks * 32, 16, 1024), id_k, more);
+          tc::mma_ss(tm + TG_YK, ka, tc::smem_desc_sw128(y + ks * 32, 16, 1024), id_k, more);
+          tc::mma_ss(tm + TG_COL, qa, tc::smem_desc_sw128(x + ks * 2048, 8192, 1024), id_mn, more);
+          tc::mma_ss(tm + TG_COL, ka, tc::smem_desc_sw128(y + ks * 2048, 8192, 1024), id_mn, 1u);
+        }
+      }
+      tc::mma_commit(&bars[2]);
+    }
+    __syncwarp();
     {  // dV = beta Ut and the row sums of Ut o V: this warp's 16 d_v columns and 32 tokens
 #pragma unroll
       for (int mt = 0; mt < 2; ++mt) {
@@ -640,174 +769,88 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
             }
           }
           s = quad_sum(s);
-          if (t == 0) red[(wn * BCH + tok) * 5 + 4] = s;
+          if (t == 0) uv[wn * BCH + tok] = s;
         }
       }
     }
-    // dO M0^T, Ut M0^T, Vn E^T over d_v
-    float qa[2][2][4], ra[2][2][4], sa[2][2][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-      for (int j = 0; j < 2; ++j) { zero(qa[i][j]); zero(ra[i][j]); zero(sa[i][j]); }
-    float dot = 0.f;
-    {
-      // right-operand element (k = 16 ks + 2 t (+1, +8, +9), column 16 wn + 8 nt + g)
-      const float* hp = ws.m0 + rec * STATE_FLOATS + 2 * t * BD + 16 * wn + g;
-      const float* ep = ws.e + rec * STATE_FLOATS + 2 * t * BD + 16 * wn + g;
-      float hx[8], ex[8];
-      auto fetch = [&](int ks) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int off = (16 * ks + (e & 1) + 8 * ((e >> 1) & 1)) * BD + 8 * (e >> 2);
-          hx[e] = __ldcs(hp + off);
-          ex[e] = __ldcs(ep + off);
-        }
-      };
-      fetch(0);
+    tc::mbar_wait_warp(&bars[2], phase >> 2 & 1, abort_flag);
+    phase ^= 4u;
+    tc::tc_fence_after_sync();
+    const int quarter = warp & 3, dk = 32 * quarter + lane;  // a warp reads the tensor-memory lanes of its quarter
 #pragma unroll 1
-      for (int ks = 0; ks < 8; ++ks) {
-        uint32_t hh_[4], hm[4], hl[4], eh[4], em[4], el[4];  // [column tile][b0, b1]
+    for (int pc = 0; pc < 2; ++pc) {
+      const int tok0 = 16 * (warp >> 2) + 8 * pc;
+      const uint32_t at = tm + ((uint32_t)(32 * quarter) << 16) + tok0;
+      uint32_t xq[8], xr[8], xs[8], xk[8], yk[8], xc[8];
+      tc::tmem_ld8(at + TG_Q, xq); tc::tmem_ld8(at + TG_R, xr); tc::tmem_ld8(at + TG_S, xs);
+      tc::tmem_ld8(at + TG_XK, xk); tc::tmem_ld8(at + TG_YK, yk); tc::tmem_ld8(at + TG_COL, xc);
+      tc::tmem_ld_wait();
+      float v[32], dq[8], dkv[8];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          split3(make_float2(hx[2 * e], hx[2 * e + 1]), hh_[e], hm[e], hl[e]);
-          split3(make_float2(ex[2 * e], ex[2 * e + 1]), eh[e], em[e], el[e]);
-          dot = fmaf(hx[2 * e], ex[2 * e], fmaf(hx[2 * e + 1], ex[2 * e + 1], dot));
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t off = (dk >> 6) * 8192 + piece<128>(tok0 + i, (dk & 63) >> 3) + 2 * (dk & 7);
+        const float k = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_K + off));
+        const float q = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_Q + off));
+        const float gq = fmaf(fac[tok0 + i], __uint_as_float(xq[i]), __uint_as_float(xk[i]));
+        const float row = fmaf(fac[BCH + tok0 + i], __uint_as_float(xr[i]), __uint_as_float(yk[i]));
+        const float state = fac[2 * BCH + tok0 + i] * __uint_as_float(xs[i]), col = state + __uint_as_float(xc[i]);
+        v[4 * i] = q * gq; v[4 * i + 1] = k * row; v[4 * i + 2] = k * col; v[4 * i + 3] = k * state;
+        dq[i] = gq; dkv[i] = row + col;
+      }
+      reinterpret_cast<float*>(red + quarter * BCH + tok0)[lane] = lane_sums(v, lane);
+      if (kSum && r > 1) {  // the sums over the heads so far wait in tensor memory
+        if (hh > 0) {
+          tc::tmem_ld8(at + TG_DQ, xq); tc::tmem_ld8(at + TG_DK, xr);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 8; ++i) { dq[i] += __uint_as_float(xq[i]); dkv[i] += __uint_as_float(xr[i]); }
         }
-        if (ks < 7) fetch(ks + 1);
+        if (hh < r - 1) {
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-          const int m0 = 32 * wm + 16 * mt;
-          uint32_t x[4], y[4], z[4];
-          ldsm4(x, sb + GR_DO + at_a<256>(m0, 2 * ks, lane));
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            mma_bf16(qa[mt][nt], x, hh_[2 * nt], hh_[2 * nt + 1]);
-            mma_bf16(qa[mt][nt], x, hm[2 * nt], hm[2 * nt + 1]);
-            mma_bf16(qa[mt][nt], x, hl[2 * nt], hl[2 * nt + 1]);
-          }
-          const uint32_t ua = sb + GR_U + at_at<128>(16 * ks, m0 >> 3, lane);
-          ldsm4t(x, ua); ldsm4t(y, ua + 16384); ldsm4t(z, ua + 32768);
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt)
-            mma6(ra[mt][nt], x, y, z, hh_[2 * nt], hh_[2 * nt + 1], hm[2 * nt], hm[2 * nt + 1], hl[2 * nt], hl[2 * nt + 1]);
-          const uint32_t va = ua - (GR_U - GR_VN);
-          ldsm4t(x, va); ldsm4t(y, va + 16384); ldsm4t(z, va + 32768);
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt)
-            mma6(sa[mt][nt], x, y, z, eh[2 * nt], eh[2 * nt + 1], em[2 * nt], em[2 * nt + 1], el[2 * nt], el[2 * nt + 1]);
+          for (int i = 0; i < 8; ++i) { xq[i] = __float_as_uint(dq[i]); xr[i] = __float_as_uint(dkv[i]); }
+          tc::tmem_st8(at + TG_DQ, xq); tc::tmem_st8(at + TG_DK, xr);
+          tc::tmem_st_wait();
         }
+      }
+      if (!kSum || hh == r - 1) {
+        store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok0, dk, dq);
+        store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok0, dk, dkv);
       }
     }
-    dot = warp_sum(dot);
-    if (lane == 0 && wm == 0) dots[wn] = dot;
-    __syncthreads();  // X and Y are complete
-    const float bC = bs[BCH - 1];
-#pragma unroll
-    for (int mt = 0; mt < 2; ++mt) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int tok = 32 * wm + 16 * mt + g + 8 * half;
-        const float eb = __expf(bs[tok]), fq = a.scale * eb, fd = gate_between(bs, BCH - 1, tok);
-        const float be = fabsf(betas[tok]) < 1e-20f ? 1e-20f : betas[tok], fr = -be * eb;
-        float st = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          float* q4 = qa[mt][nt] + 2 * half; float* r4 = ra[mt][nt] + 2 * half; float* s4 = sa[mt][nt] + 2 * half;
-          q4[0] *= fq; q4[1] *= fq; r4[0] *= fr; r4[1] *= fr; s4[0] *= fd; s4[1] *= fd;
-          const float2 k = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_K + piece<256>(tok, 2 * wn + nt) + 4 * t));
-          st = fmaf(k.x, s4[0], fmaf(k.y, s4[1], st));
-        }
-        st = quad_sum(st);
-        if (t == 0) red[(wn * BCH + tok) * 5 + 3] = st;
-      }
-      const int m = 2 * wm + mt;  // 16-token tile
-#pragma unroll 1
-      for (int ks = 0; ks <= m; ++ks) {  // rows of tile m need the tokens up to it
-        uint32_t kb[4], x[4], y[4], z[4];
-        ldsm4t(kb, sb + GR_K + at_bt<256>(16 * ks, 2 * wn, lane));
-        const uint32_t xa = sb + GR_X + at_a<128>(16 * m, 2 * ks, lane);
-        ldsm4(x, xa); ldsm4(y, xa + IMG); ldsm4(z, xa + 2 * IMG);
-        mma3(qa[mt][0], x, y, z, kb[0], kb[1]);
-        mma3(qa[mt][1], x, y, z, kb[2], kb[3]);
-        const uint32_t ya = xa + (GR_Y - GR_X);
-        ldsm4(x, ya); ldsm4(y, ya + IMG); ldsm4(z, ya + 2 * IMG);
-        mma3(ra[mt][0], x, y, z, kb[0], kb[1]);
-        mma3(ra[mt][1], x, y, z, kb[2], kb[3]);
-      }
-#pragma unroll 1
-      for (int ks = m; ks < 4; ++ks) {  // columns of tile m take from the tokens from it on
-        uint32_t kb[4], qb[4], x[4], y[4], z[4];
-        ldsm4t(kb, sb + GR_K + at_bt<256>(16 * ks, 2 * wn, lane));
-        ldsm4t(qb, sb + GR_Q + at_bt<256>(16 * ks, 2 * wn, lane));
-        const uint32_t xa = sb + GR_X + at_at<128>(16 * ks, 2 * m, lane);
-        ldsm4t(x, xa); ldsm4t(y, xa + IMG); ldsm4t(z, xa + 2 * IMG);
-        mma3(sa[mt][0], x, y, z, qb[0], qb[1]);
-        mma3(sa[mt][1], x, y, z, qb[2], qb[3]);
-        const uint32_t ya = xa + (GR_Y - GR_X);
-        ldsm4t(x, ya); ldsm4t(y, ya + IMG); ldsm4t(z, ya + 2 * IMG);
-        mma3(sa[mt][0], x, y, z, kb[0], kb[1]);
-        mma3(sa[mt][1], x, y, z, kb[2], kb[3]);
-      }
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int tok = 32 * wm + 16 * mt + g + 8 * half;
-        float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-          const uint32_t off = piece<256>(tok, 2 * wn + nt) + 4 * t;
-          const float2 k = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_K + off));
-          const float2 q = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(smem + GR_Q + off));
-          const float* q4 = qa[mt][nt] + 2 * half; const float* r4 = ra[mt][nt] + 2 * half; const float* s4 = sa[mt][nt] + 2 * half;
-          s0 = fmaf(q.x, q4[0], fmaf(q.y, q4[1], s0));
-          s1 = fmaf(k.x, r4[0], fmaf(k.y, r4[1], s1));
-          s2 = fmaf(k.x, s4[0], fmaf(k.y, s4[1], s2));
-          dq[mt][nt][2 * half] += q4[0]; dq[mt][nt][2 * half + 1] += q4[1];
-          dk[mt][nt][2 * half] += r4[0] + s4[0]; dk[mt][nt][2 * half + 1] += r4[1] + s4[1];
-        }
-        s0 = quad_sum(s0); s1 = quad_sum(s1); s2 = quad_sum(s2);
-        if (t == 0) {
-          float* dst = red + (wn * BCH + tok) * 5;
-          dst[0] = s0; dst[1] = s1; dst[2] = s2;
-        }
-        if (!kSum || hh == r - 1) {
-#pragma unroll
-          for (int nt = 0; nt < 2; ++nt) {
-            const int col = 16 * wn + 8 * nt + 2 * t;
-            float* q4 = dq[mt][nt] + 2 * half; float* k4 = dk[mt][nt] + 2 * half;
-            store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok, col, q4[0], q4[1]);
-            store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok, col, k4[0], k4[1]);
-            if (!kSum) q4[0] = q4[1] = k4[0] = k4[1] = 0.f;
-          }
-        }
-      }
-    }
+    tc::tc_fence_before_sync();
     __syncthreads();
     if (tid < BCH) {  // dbeta, and dg as a suffix sum of db
-      float s[5] = {};
+      float4 s = red[tid];
+      float su = 0.f, em = 0.f;
 #pragma unroll
-      for (int w = 0; w < 8; ++w)
+      for (int w = 1; w < 4; ++w) {
+        const float4 x = red[w * BCH + tid];
+        s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+      }
 #pragma unroll
-        for (int e = 0; e < 5; ++e) s[e] += red[(w * BCH + tid) * 5 + e];
+      for (int w = 0; w < 8; ++w) su += uv[w * BCH + tid];
+#pragma unroll
+      for (int w = 0; w < 16; ++w) em += dots[w];
       const float be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
       const int64_t off = (row0 + tid) * a.Hv + h;
-      if (tid < c.len) a.d_beta[off] = s[4] + s[1] / be;
-      float db = s[0] + s[1] - s[2];
+      if (tid < c.len) a.d_beta[off] = su + s.y / be;
+      float db = s.x + s.y - s.z;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const float x = __shfl_down_sync(0xffffffffu, db, o);
         if (lane + o < 32) db += x;
       }
-      const float st = warp_sum(s[3]);
-      if (lane == 0) { dots[8 + 2 * warp] = db; dots[9 + 2 * warp] = st; }
+      const float st = warp_sum(s.w);
+      float* carry = dots + 16;
+      if (lane == 0) { carry[2 * warp] = db; carry[1 + 2 * warp] = st; }
       asm volatile("bar.sync 1, 64;" ::: "memory");
-      float em = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) em += dots[w];
-      if (warp == 0) db += dots[10];
-      if (tid < c.len) a.d_g[off] = db + (dots[9] + dots[11]) + __expf(bC) * em;
+      if (warp == 0) db += carry[2];
+      if (tid < c.len) a.d_g[off] = db + (carry[1] + carry[3]) + __expf(bs[BCH - 1]) * em;
     }
   }
+  __syncthreads();
+  if (tid == 0 && *abort_flag != 0u && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+  if (warp == 1) tc::tmem_dealloc(tm, 512);
 }
 
 int64_t backward_slots(const AveGdnBwdArgs& a) { return (int64_t)a.B * a.T / BCH + a.n_seqs + 1; }
