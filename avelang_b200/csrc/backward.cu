@@ -18,14 +18,14 @@
 // after chunk; bwd_reverse: the state gradients and Ut, chunk after chunk from the end (it needs nothing of bwd_forward).
 // bwd_grads: everything else, in parallel over (chunk, key head), summing over the value heads that share the key head.
 //
-// The contractions run on warp-level bf16 MMAs (most of bwd_grads: on tcgen05) with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
+// The contractions run on warp-level bf16 MMAs (bwd_grads: on tcgen05) with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
 // every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with one fp32 operand is
 // three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which the gradient of
 // the gate needs, because it is a difference of large sums.
 // The scans hold the state transposed, H = M^T: a warp owns 16 of the 128 d_v rows for the whole sequence, every product
 // is (its rows) x (a tile all warps read), and the accumulator of one product is, in place, the left operand of the next,
 // so the warps of a chain never exchange anything and only meet where a tile buffer is refilled.
-// Two sequences of 4096 tokens, 32 value heads: 1.33 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.57)
+// Two sequences of 4096 tokens, 32 value heads: 1.20 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.44)
 // against 22.1 ms for the token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
 #include "blockalg.cuh"
 #include "common.cuh"
@@ -502,29 +502,34 @@ __global__ void __launch_bounds__(SC_T, 1) bwd_reverse_kernel(const AveGdnBwdArg
 }
 
 // ---------------------------------------------------------------------------------------------- the gradients of one chunk
-// One CTA of 16 warps per (chunk, key head).  Seven of the nine products contract over a whole tile and run on tcgen05, transposed
-// (128 d_k lanes x 64 tokens, so that the tile that differs per product is the narrow operand): dO M0^T, Ut M0^T and Vn E^T
-// over d_v, and X K, Y K, X^T Q + Y^T K over the tokens.  fp32 operands are three bf16 tiles each.  M0 and E pass through shared
-// memory 16 d_v rows at a time, split on the way in; while the tensor core works on one such step the warps fetch and split the
-// next and do the same d_v rows of X and Y (lower triangles, 16 x 8 blocks) on warp-level MMAs.
-// Two sequences of 4096 tokens, 32 value heads: 0.57 ms; all of it on warp-level MMAs, at 16 cycles each, took 0.73.
+// A persistent CTA of 16 warps walks (chunk, key head) pairs.  All products run on tcgen05: X and Y (64 x 64) and, transposed
+// (128 d_k lanes x 64 tokens, so that the tile that differs per product is the narrow operand), dO M0^T, Ut M0^T and Vn E^T over
+// d_v, and X K, Y K, X^T Q + Y^T K over the tokens.  fp32 operands are three bf16 tiles each.  M0 and E pass through shared
+// memory 16 d_v rows at a time, split on the way in, two steps deep.  One thread needs about 100 cycles per MMA of this size,
+// so four warps issue, each into accumulators of its own; the records of the next head are asked for (into L2) a head ahead.
+// Two sequences of 4096 tokens, 32 value heads: 0.44 ms (0.57 with X and Y on warp-level MMAs, one issuer, one pair per CTA;
+// 0.73 with every product on warp-level MMAs, whose pipe takes 16 cycles for each).
+constexpr int GR_CTAS = 148;  // one CTA per SM
 constexpr int GR_T = 512, GR_DV = 16, GR_TERM = GR_DV * BD * 2, GR_STAGE = 6 * GR_TERM;
 constexpr int GR_K = 0, GR_Q = 16384, GR_DO = 32768, GR_VN = 49152, GR_U = GR_VN + 3 * 16384, GR_ST = GR_U + 3 * 16384,
               GR_X = GR_ST, GR_Y = GR_X + 3 * IMG,  // X and Y take the place of the two stages once those are consumed
-              GR_RED = GR_ST + 2 * GR_STAGE, GR_UV = GR_RED + 4 * BCH * 16, GR_SC = GR_UV + 8 * BCH * 4, GR_F = GR_SC + SC_BYTES + 96,
-              GR_BAR = GR_F + 3 * BCH * 4, GR_SMEM = GR_BAR + 64;
+              GR_RED = GR_ST + 2 * GR_STAGE, GR_UV = GR_RED + 4 * BCH * 8, GR_SC = GR_UV + 8 * BCH * 4, GR_F = GR_SC + SC_BYTES + 144,
+              GR_BAR = GR_F + BCH * 16, GR_SMEM = GR_BAR + 64;
 static_assert(GR_Y + 3 * IMG <= GR_RED && GR_SMEM <= 227 * 1024, "shared memory");
 enum { TG_Q = 0, TG_R = 64, TG_S = 128, TG_XK = 192, TG_YK = 256, TG_COL = 320, TG_DQ = 384, TG_DK = 448 };  // tensor-memory columns
 
 // fp32 [128][64] -> three bf16 tiles of 128-byte rows
-__device__ __forceinline__ void split_tile(uint8_t* dst, const float* src, int tid) {
+__device__ __forceinline__ void fetch_tile(float4 (&x)[4], const float* src, int tid) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) x[i] = __ldcs(reinterpret_cast<const float4*>(src) + tid + i * GR_T);
+}
+__device__ __forceinline__ void split_tile(uint8_t* dst, const float4 (&x)[4], int tid) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int e = tid + i * GR_T, row = e >> 4, q4 = e & 15;
-    const float4 x = __ldcs(reinterpret_cast<const float4*>(src + row * BCH + 4 * q4));
     uint32_t h[2], m[2], l[2];
-    split3(make_float2(x.x, x.y), h[0], m[0], l[0]);
-    split3(make_float2(x.z, x.w), h[1], m[1], l[1]);
+    split3(make_float2(x[i].x, x[i].y), h[0], m[0], l[0]);
+    split3(make_float2(x[i].z, x[i].w), h[1], m[1], l[1]);
     uint8_t* p = dst + piece<128>(row, q4 >> 1) + 8 * (q4 & 1);
     *reinterpret_cast<uint2*>(p) = make_uint2(h[0], h[1]);
     *reinterpret_cast<uint2*>(p + 16384) = make_uint2(m[0], m[1]);
@@ -545,10 +550,10 @@ __device__ __forceinline__ float quad_sum(float x) {
   x += __shfl_xor_sync(0xffffffffu, x, 1);
   return x + __shfl_xor_sync(0xffffffffu, x, 2);
 }
-// v[lane] of the 32 values summed over the lanes
-__device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
+// v[lane & 15] of the 16 values summed over the lanes
+__device__ __forceinline__ float lane_sums(float (&v)[16], int lane) {
 #pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) {
+  for (int o = 8; o >= 1; o >>= 1) {
     const bool up = (lane & o) != 0;
 #pragma unroll
     for (int i = 0; i < o; ++i) {
@@ -556,7 +561,7 @@ __device__ __forceinline__ float lane_sums(float (&v)[32], int lane) {
       v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
     }
   }
-  return v[0];
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 16);
 }
 // Per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16: eight tokens
 // of one d_k column per lane.
@@ -580,277 +585,307 @@ __device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, co
 }
 
 template <bool kSum>
-__global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+__global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs a, BwdScratch ws, int64_t slots) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int hk = blockIdx.y, r = a.Hv / a.Hk;
-  const int64_t slot = blockIdx.x;
-  const BwdChunk c = chunk_of_slot(a, slot);
-  if (!c.ok) return;
+  const int r = a.Hv / a.Hk;
   const uint32_t sb = tc::smem_u32(smem);
-  float4* red = reinterpret_cast<float4*>(smem + GR_RED);  // [4 d_k quarters][64 tokens]: q.dq, k.row, k.col, k.state
+  float2* red = reinterpret_cast<float2*>(smem + GR_RED);  // [4 d_k quarters][64 tokens]: q.dq + k.row - k.col, k.row
   float* uv = reinterpret_cast<float*>(smem + GR_UV);      // [8 d_v blocks][64 tokens]: u.v
   float* bs = reinterpret_cast<float*>(smem + GR_SC);
   float* betas = bs + BCH;
-  float* dots = bs + 3 * BCH;  // [16] partial <E, M0>; after the sums are taken, [8..11] carry the suffix sum
-  float* fac = reinterpret_cast<float*>(smem + GR_F);      // per token: factors of dO M0^T, Ut M0^T, Vn E^T
+  float* dots = bs + 3 * BCH;  // [16] partial <E, M0> | [16] partial k.state | the carry of the suffix sum
+  float4* fac = reinterpret_cast<float4*>(smem + GR_F);    // per token: factors of dO M0^T, Ut M0^T, Vn E^T
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GR_BAR);  // the two stages, and everything
   volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + GR_BAR + 32);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + GR_BAR + 40);
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) tc::mbar_init(&bars[i], 1);
+    for (int i = 0; i < 3; ++i) tc::mbar_init(&bars[i], i < 2 ? 4 : 3);  // commits: one per issuing warp
     *abort_flag = 0u;
     tc::fence_barrier_init();
   }
   if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
   const int wm = warp & 1, wn = warp >> 1;  // dV: token half, 16 d_v columns
-  const int64_t row0 = (int64_t)c.b * a.T + c.t0;
-
-  auto load_half_tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
-    load_tile<BCH, 8, GR_T>(sb + at, src, stride, c.len, tid);
-    load_tile<BCH, 8, GR_T>(sb + at + 8192, src + 64, stride, c.len, tid);
-  };
-  load_half_tiles(GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t);
-  load_half_tiles(GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t);
   uint32_t tm = 0;
   uint32_t phase = 0;  // bit i: parity of the next completion of bars[i]
 
+  // Persistent: the CTA walks its (chunk, key head) pairs and asks for the next head's tiles while it works on one.
+  const int64_t pairs = slots * a.Hk;
 #pragma unroll 1
-  for (int hh = 0; hh < r; ++hh) {
-    const int h = hk * r + hh;
-    const int64_t rec = slot * a.Hv + h;
-    if (hh > 0) __syncthreads();  // the tiles and sums of the previous head are no longer read
-    load_half_tiles(GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t);
-    cp_commit();
-    const float4* hp = reinterpret_cast<const float4*>(ws.m0 + rec * STATE_FLOATS) + tid;  // row warp of a step, columns 4 lane ..
-    const float4* ep = reinterpret_cast<const float4*>(ws.e + rec * STATE_FLOATS) + tid;
-    float4 hx[2], ex[2];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) { hx[s] = __ldcs(hp + s * GR_T); ex[s] = __ldcs(ep + s * GR_T); }
-    split_tile(smem + GR_VN, ws.vn + rec * VEC_FLOATS, tid);
-    split_tile(smem + GR_U, ws.u + rec * VEC_FLOATS, tid);
-    if (tid < 3 * BCH) bs[tid] = reinterpret_cast<const float*>(ws.prep + rec * PREP_BYTES + PREP_SC)[tid];
-    cp_wait<0>();
-    tc::tc_fence_before_sync();
-    __syncthreads();
-    tc::tc_fence_after_sync();
-    tm = *tmem_slot;
-    if (tid < BCH) {
-      const float eb = __expf(bs[tid]), be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
-      fac[tid] = a.scale * eb;
-      fac[BCH + tid] = -be * eb;
-      fac[2 * BCH + tid] = gate_between(bs, BCH - 1, tid);
-    }
-    // X = S lower(dO Vn^T) o G and Y = -beta strict_lower(Ut Vn^T) o G: warp = (16-row tile, column tiles nq and nq + 4)
-    const int m = warp >> 2, nq = warp & 3, last = 2 * m + 1;
-    float ax[2][4], ay[2][4], dot = 0.f;
-    zero(ax[0]); zero(ax[1]); zero(ay[0]); zero(ay[1]);
+  for (int64_t p = blockIdx.x; p < pairs; p += gridDim.x) {
+    const int64_t slot = p / a.Hk;
+    const int hk = (int)(p % a.Hk);
+    const BwdChunk c = chunk_of_slot(a, slot);
+    if (!c.ok) continue;
+    const int64_t row0 = (int64_t)c.b * a.T + c.t0;
+    auto load_half_tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
+      load_tile<BCH, 8, GR_T>(sb + at, src, stride, c.len, tid);
+      load_tile<BCH, 8, GR_T>(sb + at + 8192, src + 64, stride, c.len, tid);
+    };
+    __syncthreads();  // the tiles and sums of the pair before are no longer read
+    load_half_tiles(GR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t);
+    load_half_tiles(GR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t);
+
 #pragma unroll 1
-    for (int s0 = 0; s0 < 8; s0 += 2)
+    for (int hh = 0; hh < r; ++hh) {
+      const int h = hk * r + hh;
+      const int64_t rec = slot * a.Hv + h;
+      if (hh > 0) __syncthreads();  // the tiles and sums of the previous head are no longer read
+      load_half_tiles(GR_DO, bf(a.d_o) + c.b * a.do_stride_b + (int64_t)c.t0 * a.do_stride_t + h * a.do_stride_h, a.do_stride_t);
+      cp_commit();
+      if (tid == 0) {  // the next head's records towards L2
+        const int64_t np = hh + 1 < r ? p : p + gridDim.x;
+        if (np < pairs) {
+          const int64_t nrec = (np / a.Hk) * a.Hv + (np % a.Hk) * r + (hh + 1 < r ? hh + 1 : 0);
+          tc::bulk_prefetch_l2(ws.vn + nrec * VEC_FLOATS, VEC_FLOATS * 4);
+          tc::bulk_prefetch_l2(ws.u + nrec * VEC_FLOATS, VEC_FLOATS * 4);
+          tc::bulk_prefetch_l2(ws.m0 + nrec * STATE_FLOATS, STATE_FLOATS * 4);
+          tc::bulk_prefetch_l2(ws.e + nrec * STATE_FLOATS, STATE_FLOATS * 4);
+        }
+      }
+      const float4* hp = reinterpret_cast<const float4*>(ws.m0 + rec * STATE_FLOATS) + tid;  // row warp of a step, columns 4 lane ..
+      const float4* ep = reinterpret_cast<const float4*>(ws.e + rec * STATE_FLOATS) + tid;
+      float4 hx[2], ex[2];
+      {
+        float4 vn[4], ut[4];
+        fetch_tile(vn, ws.vn + rec * VEC_FLOATS, tid);
+        fetch_tile(ut, ws.u + rec * VEC_FLOATS, tid);
 #pragma unroll
-    for (int st = 0; st < 2; ++st) {
-      const int s = s0 + st;
-      uint8_t* stage = smem + GR_ST + st * GR_STAGE;
-      if (s >= 2) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
-      split_step(stage, hx[st], warp, lane);
-      split_step(stage + 3 * GR_TERM, ex[st], warp, lane);
-      dot = fmaf(hx[st].x, ex[st].x, fmaf(hx[st].y, ex[st].y, fmaf(hx[st].z, ex[st].z, fmaf(hx[st].w, ex[st].w, dot))));
-      if (s < 6) { hx[st] = __ldcs(hp + (s + 2) * GR_T); ex[st] = __ldcs(ep + (s + 2) * GR_T); }
-      tc::fence_proxy_async_smem();
+        for (int s = 0; s < 2; ++s) { hx[s] = __ldcs(hp + s * GR_T); ex[s] = __ldcs(ep + s * GR_T); }
+        split_tile(smem + GR_VN, vn, tid);
+        split_tile(smem + GR_U, ut, tid);
+      }
+      if (tid < 3 * BCH) bs[tid] = reinterpret_cast<const float*>(ws.prep + rec * PREP_BYTES + PREP_SC)[tid];
+      cp_wait<0>();
+      tc::tc_fence_before_sync();
       __syncthreads();
-      if (warp == 3 && tc::elect_one()) {  // a warp without blocks of X and Y
-        constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true);
-        const uint32_t so = sb + GR_ST + st * GR_STAGE;
-        uint64_t mo[3], eo[3], u[3], v[3];
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          mo[i] = tc::smem_desc_sw128(so + i * GR_TERM, GR_TERM / 2, 1024);
-          eo[i] = tc::smem_desc_sw128(so + (3 + i) * GR_TERM, GR_TERM / 2, 1024);
-          u[i] = tc::smem_desc_sw128(sb + GR_U + i * 16384 + s * 2048, 8192, 1024);
-          v[i] = tc::smem_desc_sw128(sb + GR_VN + i * 16384 + s * 2048, 8192, 1024);
-        }
-        const uint64_t o = tc::smem_desc_sw128(sb + GR_DO + (s >> 2) * 8192 + (s & 3) * 32, 16, 1024);
-        const uint32_t acc = s > 0 ? 1u : 0u;
-        // ordered so that neighbours write different accumulators
-        tc::mma_ss(tm + TG_R, mo[0], u[0], id_mn, acc); tc::mma_ss(tm + TG_S, eo[0], v[0], id_mn, acc); tc::mma_ss(tm + TG_Q, mo[0], o, id_k, acc);
-        tc::mma_ss(tm + TG_R, mo[0], u[1], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[0], v[1], id_mn, 1u); tc::mma_ss(tm + TG_Q, mo[1], o, id_k, 1u);
-        tc::mma_ss(tm + TG_R, mo[1], u[0], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[1], v[0], id_mn, 1u); tc::mma_ss(tm + TG_Q, mo[2], o, id_k, 1u);
-        tc::mma_ss(tm + TG_R, mo[0], u[2], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[0], v[2], id_mn, 1u);
-        tc::mma_ss(tm + TG_R, mo[2], u[0], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[2], v[0], id_mn, 1u);
-        tc::mma_ss(tm + TG_R, mo[1], u[1], id_mn, 1u); tc::mma_ss(tm + TG_S, eo[1], v[1], id_mn, 1u);
-        tc::mma_commit(&bars[st]);
+      tc::tc_fence_after_sync();
+      tm = *tmem_slot;
+      if (tid < BCH) {
+        const float eb = __expf(bs[tid]), be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
+        fac[tid] = make_float4(a.scale * eb, -be * eb, gate_between(bs, BCH - 1, tid), 0.f);
       }
-      __syncwarp();
-      if (nq <= last) {
-        uint32_t o[4], uh[4], um[4], ul[4], vh[4], vm[4], vl[4];
-        ldsm4(o, sb + GR_DO + (s >> 2) * 8192 + at_a<128>(16 * m, 2 * (s & 3), lane));
-        const uint32_t ua = sb + GR_U + at_at<128>(16 * s, 2 * m, lane);
-        ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
-        const uint32_t va = sb + GR_VN + piece<128>(16 * s + (lane & 15), nq + 4 * (lane >> 4));
-        ldsm4t(vh, va); ldsm4t(vm, va + 16384); ldsm4t(vl, va + 32768);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          if (e == 1 && nq + 4 > last) break;
-          mma_bf16(ax[e], o, vh[2 * e], vh[2 * e + 1]);
-          mma_bf16(ax[e], o, vm[2 * e], vm[2 * e + 1]);
-          mma_bf16(ax[e], o, vl[2 * e], vl[2 * e + 1]);
-          mma6(ay[e], uh, um, ul, vh[2 * e], vh[2 * e + 1], vm[2 * e], vm[2 * e + 1], vl[2 * e], vl[2 * e + 1]);
-        }
-      }
-    }
-    dot = warp_sum(dot);
-    if (lane == 0) dots[warp] = dot;
-#pragma unroll
-    for (int st = 0; st < 2; ++st) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
-    // X and Y take the place of the stages; blocks above the diagonal are zero
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int nt = nq + 4 * e;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
-        float2 x = make_float2(0.f, 0.f), y = x;
-        if (nt <= last) {
-          const float e0 = gate_between(bs, i, j), e1 = gate_between(bs, i, j + 1);
-          const float be = -(fabsf(betas[i]) < 1e-20f ? 1e-20f : betas[i]);
-          x = make_float2(i >= j ? a.scale * e0 * ax[e][2 * half] : 0.f, i > j ? a.scale * e1 * ax[e][2 * half + 1] : 0.f);
-          y = make_float2(i > j ? be * e0 * ay[e][2 * half] : 0.f, i > j + 1 ? be * e1 * ay[e][2 * half + 1] : 0.f);
-        }
-        uint32_t xh, xm, xl;
-        uint8_t* dst = smem + GR_X + piece<128>(i, nt) + 4 * t;
-        split3(x, xh, xm, xl);
-        *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
-        dst += GR_Y - GR_X;
-        split3(y, xh, xm, xl);
-        *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
-      }
-    }
-    tc::fence_proxy_async_smem();
-    __syncthreads();
-    if (warp == 3 && tc::elect_one()) {
-      constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true);
+      float dot = 0.f;
 #pragma unroll 1
-      for (int ks = 0; ks < 4; ++ks) {
-        const uint64_t ka = tc::smem_desc_sw128(sb + GR_K + ks * 2048, 8192, 1024), qa = tc::smem_desc_sw128(sb + GR_Q + ks * 2048, 8192, 1024);
-        const uint32_t acc = ks > 0 ? 1u : 0u;
+      for (int s0 = 0; s0 < 8; s0 += 2)
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const uint32_t x = sb + GR_X + i * IMG, y = sb + GR_Y + i * IMG, more = i > 0 ? 1u : acc;
-          tc::mma_ss(tm + TG_XK, ka, tc::smem_desc_sw128(x + ks * 32, 16, 1024), id_k, more);
-          tc::mma_ss(tm + TG_YK, ka, tc::smem_desc_sw128(y + ks * 32, 16, 1024), id_k, more);
-          tc::mma_ss(tm + TG_COL, qa, tc::smem_desc_sw128(x + ks * 2048, 8192, 1024), id_mn, more);
-          tc::mma_ss(tm + TG_COL, ka, tc::smem_desc_sw128(y + ks * 2048, 8192, 1024), id_mn, 1u);
-        }
-      }
-      tc::mma_commit(&bars[2]);
-    }
-    __syncwarp();
-    {  // dV = beta Ut and the row sums of Ut o V: this warp's 16 d_v columns and 32 tokens
+      for (int st = 0; st < 2; ++st) {
+        const int s = s0 + st;
+        uint8_t* stage = smem + GR_ST + st * GR_STAGE;
+        if (s >= 2) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
+        split_step(stage, hx[st], warp, lane);
+        split_step(stage + 3 * GR_TERM, ex[st], warp, lane);
+        dot = fmaf(hx[st].x, ex[st].x, fmaf(hx[st].y, ex[st].y, fmaf(hx[st].z, ex[st].z, fmaf(hx[st].w, ex[st].w, dot))));
+        tc::fence_proxy_async_smem();  // waits for loads in flight: the next ones go out behind it
+        if (s < 6) { hx[st] = __ldcs(hp + (s + 2) * GR_T); ex[st] = __ldcs(ep + (s + 2) * GR_T); }
+        __syncthreads();
+        if (warp < 4 && tc::elect_one()) {  // four issuers; X and Y take the columns of X K and Y K, which come after them
+          constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true),
+                             id_x = tc::idesc_f16(64, 64, 1, 1, false, true), id_y = tc::idesc_f16(64, 64, 1, 1, true, true);
+          const uint32_t so = sb + GR_ST + st * GR_STAGE, acc = s > 0 ? 1u : 0u;
+          const uint64_t mo = tc::smem_desc_sw128(so, GR_TERM / 2, 1024), eo = tc::smem_desc_sw128(so + 3 * GR_TERM, GR_TERM / 2, 1024),
+                         u = tc::smem_desc_sw128(sb + GR_U + s * 2048, 8192, 1024), v = tc::smem_desc_sw128(sb + GR_VN + s * 2048, 8192, 1024),
+                         o = tc::smem_desc_sw128(sb + GR_DO + (s >> 2) * 8192 + (s & 3) * 32, 16, 1024);
+          if (warp == 3) {
 #pragma unroll
-      for (int mt = 0; mt < 2; ++mt) {
-        uint32_t uh[4], um[4], ul[4];
-        const uint32_t ua = sb + GR_U + at_at<128>(16 * wn, 4 * wm + 2 * mt, lane);
-        ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
+            for (int i = 0; i < 3; ++i) {
+              tc::mma_ss(tm + TG_Q, mo + i * (GR_TERM >> 4), o, id_k, i > 0 ? 1u : acc);
+              tc::mma_ss(tm + TG_XK, o, v + i * (16384 >> 4), id_x, i > 0 ? 1u : acc);
+            }
+          } else {
+            const uint64_t left = warp == 0 ? mo : warp == 1 ? eo : u, right = warp == 0 ? u : v;
+            const uint32_t step = (warp == 2 ? 16384 : GR_TERM) >> 4, id = warp == 2 ? id_y : id_mn, dst = tm + (warp == 0 ? TG_R : warp == 1 ? TG_S : TG_YK);
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int tok = 32 * wm + 16 * mt + g + 8 * half;
-          float s = 0.f;
-#pragma unroll
-          for (int kk = 0; kk < 2; ++kk) {
-            const int idx = half + 2 * kk, col = 16 * wn + 8 * kk + 2 * t;
-            const float2 x = bf16x2_to_float2(uh[idx]), y = bf16x2_to_float2(um[idx]), z = bf16x2_to_float2(ul[idx]);
-            const float2 ut = make_float2(x.x + (y.x + z.x), x.y + (y.y + z.y));
-            if (tok < c.len) {
-              const float2 v = bf16x2_to_float2(*reinterpret_cast<const uint32_t*>(bf(a.v) + c.b * a.v_stride_b + (int64_t)(c.t0 + tok) * a.v_stride_t + h * a.v_stride_h + col));
-              s = fmaf(ut.x, v.x, fmaf(ut.y, v.y, s));
-              const float be = betas[tok];
-              if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.d_v) + ((row0 + tok) * a.Hv + h) * BD + col) = pack_bf16x2(be * ut.x, be * ut.y);
-              else *reinterpret_cast<float2*>(a.d_v + ((row0 + tok) * a.Hv + h) * BD + col) = make_float2(be * ut.x, be * ut.y);
+            for (int i = 0; i < 6; ++i) {  // hh hm mh hl lh mm
+              constexpr int L[6] = {0, 0, 1, 0, 2, 1}, R[6] = {0, 1, 0, 2, 0, 1};
+              tc::mma_ss(dst, left + L[i] * step, right + R[i] * (16384 >> 4), id, i > 0 ? 1u : acc);
             }
           }
-          s = quad_sum(s);
-          if (t == 0) uv[wn * BCH + tok] = s;
+          tc::mma_commit(&bars[st]);
         }
+        __syncwarp();
       }
-    }
-    tc::mbar_wait_warp(&bars[2], phase >> 2 & 1, abort_flag);
-    phase ^= 4u;
-    tc::tc_fence_after_sync();
-    const int quarter = warp & 3, dk = 32 * quarter + lane;  // a warp reads the tensor-memory lanes of its quarter
-#pragma unroll 1
-    for (int pc = 0; pc < 2; ++pc) {
-      const int tok0 = 16 * (warp >> 2) + 8 * pc;
-      const uint32_t at = tm + ((uint32_t)(32 * quarter) << 16) + tok0;
-      uint32_t xq[8], xr[8], xs[8], xk[8], yk[8], xc[8];
-      tc::tmem_ld8(at + TG_Q, xq); tc::tmem_ld8(at + TG_R, xr); tc::tmem_ld8(at + TG_S, xs);
-      tc::tmem_ld8(at + TG_XK, xk); tc::tmem_ld8(at + TG_YK, yk); tc::tmem_ld8(at + TG_COL, xc);
+      dot = warp_sum(dot);
+      if (lane == 0) dots[warp] = dot;
+#pragma unroll
+      for (int st = 0; st < 2; ++st) { tc::mbar_wait_warp(&bars[st], phase >> st & 1, abort_flag); phase ^= 1u << st; }
+      // X = S lower(dO Vn^T) o G and Y = -beta strict_lower(Ut Vn^T) o G, 16 rows per quarter of the tensor-memory lanes, take the
+      // place of the stages; blocks above the diagonal are zero
+      tc::tc_fence_after_sync();
+      const int m = warp & 3, nq = warp >> 2, last = 2 * m + 1;
+      float ax[2][4], ay[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t at = tm + ((uint32_t)(32 * m) << 16) + 8 * (nq + 4 * e);
+        tc::tmem_ld_frag(at + TG_XK, ax[e]);
+        tc::tmem_ld_frag(at + TG_YK, ay[e]);
+      }
       tc::tmem_ld_wait();
-      float v[32], dq[8], dkv[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const uint32_t off = (dk >> 6) * 8192 + piece<128>(tok0 + i, (dk & 63) >> 3) + 2 * (dk & 7);
-        const float k = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_K + off));
-        const float q = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_Q + off));
-        const float gq = fmaf(fac[tok0 + i], __uint_as_float(xq[i]), __uint_as_float(xk[i]));
-        const float row = fmaf(fac[BCH + tok0 + i], __uint_as_float(xr[i]), __uint_as_float(yk[i]));
-        const float state = fac[2 * BCH + tok0 + i] * __uint_as_float(xs[i]), col = state + __uint_as_float(xc[i]);
-        v[4 * i] = q * gq; v[4 * i + 1] = k * row; v[4 * i + 2] = k * col; v[4 * i + 3] = k * state;
-        dq[i] = gq; dkv[i] = row + col;
-      }
-      reinterpret_cast<float*>(red + quarter * BCH + tok0)[lane] = lane_sums(v, lane);
-      if (kSum && r > 1) {  // the sums over the heads so far wait in tensor memory
-        if (hh > 0) {
-          tc::tmem_ld8(at + TG_DQ, xq); tc::tmem_ld8(at + TG_DK, xr);
-          tc::tmem_ld_wait();
+      for (int e = 0; e < 2; ++e) {
+        const int nt = nq + 4 * e;
 #pragma unroll
-          for (int i = 0; i < 8; ++i) { dq[i] += __uint_as_float(xq[i]); dkv[i] += __uint_as_float(xr[i]); }
-        }
-        if (hh < r - 1) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) { xq[i] = __float_as_uint(dq[i]); xr[i] = __float_as_uint(dkv[i]); }
-          tc::tmem_st8(at + TG_DQ, xq); tc::tmem_st8(at + TG_DK, xr);
-          tc::tmem_st_wait();
+        for (int half = 0; half < 2; ++half) {
+          const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
+          float2 x = make_float2(0.f, 0.f), y = x;
+          if (nt <= last) {
+            const float e0 = gate_between(bs, i, j), e1 = gate_between(bs, i, j + 1);
+            const float be = -(fabsf(betas[i]) < 1e-20f ? 1e-20f : betas[i]);
+            x = make_float2(i >= j ? a.scale * e0 * ax[e][2 * half] : 0.f, i > j ? a.scale * e1 * ax[e][2 * half + 1] : 0.f);
+            y = make_float2(i > j ? be * e0 * ay[e][2 * half] : 0.f, i > j + 1 ? be * e1 * ay[e][2 * half + 1] : 0.f);
+          }
+          uint32_t xh, xm, xl;
+          uint8_t* dst = smem + GR_X + piece<128>(i, nt) + 4 * t;
+          split3(x, xh, xm, xl);
+          *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
+          dst += GR_Y - GR_X;
+          split3(y, xh, xm, xl);
+          *reinterpret_cast<uint32_t*>(dst) = xh; *reinterpret_cast<uint32_t*>(dst + IMG) = xm; *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = xl;
         }
       }
-      if (!kSum || hh == r - 1) {
-        store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok0, dk, dq);
-        store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok0, dk, dkv);
+      tc::fence_proxy_async_smem();
+      uint32_t vv[2][2][2];  // this warp's part of V (see dV below)
+#pragma unroll
+      for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+#pragma unroll
+          for (int kk = 0; kk < 2; ++kk) {
+            const int tok = 32 * wm + 16 * mt + g + 8 * half;
+            vv[mt][half][kk] = tok < c.len ? __ldg(reinterpret_cast<const uint32_t*>(bf(a.v) + c.b * a.v_stride_b + (int64_t)(c.t0 + tok) * a.v_stride_t + h * a.v_stride_h + 16 * wn + 8 * kk + 2 * t)) : 0u;
+          }
+      tc::tc_fence_before_sync();
+      __syncthreads();
+      if (warp < 3 && tc::elect_one()) {  // X K, Y K, X^T Q + Y^T K
+        tc::tc_fence_after_sync();
+        constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true);
+        const uint64_t ka = tc::smem_desc_sw128(sb + GR_K, 8192, 1024), qa = tc::smem_desc_sw128(sb + GR_Q, 8192, 1024);
+        const uint64_t x = tc::smem_desc_sw128(sb + GR_X, 8192, 1024), y = tc::smem_desc_sw128(sb + GR_Y, 8192, 1024);
+#pragma unroll 1
+        for (int ks = 0; ks < 4; ++ks) {
+          const uint32_t acc = ks > 0 ? 1u : 0u;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const uint32_t more = i > 0 ? 1u : acc, term = i * (IMG >> 4), rows = ks * (2048 >> 4);
+            if (warp == 0) tc::mma_ss(tm + TG_XK, ka + rows, x + term + ks * 2, id_k, more);
+            if (warp == 1) tc::mma_ss(tm + TG_YK, ka + rows, y + term + ks * 2, id_k, more);
+            if (warp == 2) {
+              tc::mma_ss(tm + TG_COL, qa + rows, x + term + rows, id_mn, more);
+              tc::mma_ss(tm + TG_COL, ka + rows, y + term + rows, id_mn, 1u);
+            }
+          }
+        }
+        tc::mma_commit(&bars[2]);
       }
-    }
-    tc::tc_fence_before_sync();
-    __syncthreads();
-    if (tid < BCH) {  // dbeta, and dg as a suffix sum of db
-      float4 s = red[tid];
-      float su = 0.f, em = 0.f;
+      __syncwarp();
+      {  // dV = beta Ut and the row sums of Ut o V: this warp's 16 d_v columns and 32 tokens
 #pragma unroll
-      for (int w = 1; w < 4; ++w) {
-        const float4 x = red[w * BCH + tid];
-        s.x += x.x; s.y += x.y; s.z += x.z; s.w += x.w;
+        for (int mt = 0; mt < 2; ++mt) {
+          uint32_t uh[4], um[4], ul[4];
+          const uint32_t ua = sb + GR_U + at_at<128>(16 * wn, 4 * wm + 2 * mt, lane);
+          ldsm4t(uh, ua); ldsm4t(um, ua + 16384); ldsm4t(ul, ua + 32768);
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            const int tok = 32 * wm + 16 * mt + g + 8 * half;
+            float s = 0.f;
+#pragma unroll
+            for (int kk = 0; kk < 2; ++kk) {
+              const int idx = half + 2 * kk, col = 16 * wn + 8 * kk + 2 * t;
+              const float2 x = bf16x2_to_float2(uh[idx]), y = bf16x2_to_float2(um[idx]), z = bf16x2_to_float2(ul[idx]);
+              const float2 ut = make_float2(x.x + (y.x + z.x), x.y + (y.y + z.y));
+              if (tok < c.len) {
+                const float2 v = bf16x2_to_float2(vv[mt][half][kk]);
+                s = fmaf(ut.x, v.x, fmaf(ut.y, v.y, s));
+                const float be = betas[tok];
+                if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.d_v) + ((row0 + tok) * a.Hv + h) * BD + col) = pack_bf16x2(be * ut.x, be * ut.y);
+                else *reinterpret_cast<float2*>(a.d_v + ((row0 + tok) * a.Hv + h) * BD + col) = make_float2(be * ut.x, be * ut.y);
+              }
+            }
+            s = quad_sum(s);
+            if (t == 0) uv[wn * BCH + tok] = s;
+          }
+        }
       }
+      tc::mbar_wait_warp(&bars[2], phase >> 2 & 1, abort_flag);
+      phase ^= 4u;
+      tc::tc_fence_after_sync();
+      const int quarter = warp & 3, dk = 32 * quarter + lane;  // a warp reads the tensor-memory lanes of its quarter
+      float states = 0.f;
+#pragma unroll 1
+      for (int pc = 0; pc < 2; ++pc) {
+        const int tok0 = 16 * (warp >> 2) + 8 * pc;
+        const uint32_t at = tm + ((uint32_t)(32 * quarter) << 16) + tok0;
+        uint32_t xq[8], xr[8], xs[8], xk[8], yk[8], xc[8];
+        tc::tmem_ld8(at + TG_Q, xq); tc::tmem_ld8(at + TG_R, xr); tc::tmem_ld8(at + TG_S, xs);
+        tc::tmem_ld8(at + TG_XK, xk); tc::tmem_ld8(at + TG_YK, yk); tc::tmem_ld8(at + TG_COL, xc);
+        tc::tmem_ld_wait();
+        float v[16], dq[8], dkv[8];
 #pragma unroll
-      for (int w = 0; w < 8; ++w) su += uv[w * BCH + tid];
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t off = (dk >> 6) * 8192 + piece<128>(tok0 + i, (dk & 63) >> 3) + 2 * (dk & 7);
+          const float k = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_K + off));
+          const float q = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(smem + GR_Q + off));
+          const float4 f = fac[tok0 + i];
+          const float gq = fmaf(f.x, __uint_as_float(xq[i]), __uint_as_float(xk[i]));
+          const float row = fmaf(f.y, __uint_as_float(xr[i]), __uint_as_float(yk[i]));
+          const float state = f.z * __uint_as_float(xs[i]), col = state + __uint_as_float(xc[i]);
+          v[2 * i] = fmaf(q, gq, k * (row - col)); v[2 * i + 1] = k * row;
+          states = fmaf(k, state, states);
+          dq[i] = gq; dkv[i] = row + col;
+        }
+        const float sums = lane_sums(v, lane);
+        if (lane < 16) reinterpret_cast<float*>(red + quarter * BCH + tok0)[lane] = sums;
+        if (kSum && r > 1) {  // the sums over the heads so far wait in tensor memory
+          if (hh > 0) {
+            tc::tmem_ld8(at + TG_DQ, xq); tc::tmem_ld8(at + TG_DK, xr);
+            tc::tmem_ld_wait();
 #pragma unroll
-      for (int w = 0; w < 16; ++w) em += dots[w];
-      const float be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
-      const int64_t off = (row0 + tid) * a.Hv + h;
-      if (tid < c.len) a.d_beta[off] = su + s.y / be;
-      float db = s.x + s.y - s.z;
+            for (int i = 0; i < 8; ++i) { dq[i] += __uint_as_float(xq[i]); dkv[i] += __uint_as_float(xr[i]); }
+          }
+          if (hh < r - 1) {
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const float x = __shfl_down_sync(0xffffffffu, db, o);
-        if (lane + o < 32) db += x;
+            for (int i = 0; i < 8; ++i) { xq[i] = __float_as_uint(dq[i]); xr[i] = __float_as_uint(dkv[i]); }
+            tc::tmem_st8(at + TG_DQ, xq); tc::tmem_st8(at + TG_DK, xr);
+            tc::tmem_st_wait();
+          }
+        }
+        if (!kSum || hh == r - 1) {
+          store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok0, dk, dq);
+          store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok0, dk, dkv);
+        }
       }
-      const float st = warp_sum(s.w);
-      float* carry = dots + 16;
-      if (lane == 0) { carry[2 * warp] = db; carry[1 + 2 * warp] = st; }
-      asm volatile("bar.sync 1, 64;" ::: "memory");
-      if (warp == 0) db += carry[2];
-      if (tid < c.len) a.d_g[off] = db + (carry[1] + carry[3]) + __expf(bs[BCH - 1]) * em;
+      states = warp_sum(states);
+      if (lane == 0) dots[16 + warp] = states;
+      tc::tc_fence_before_sync();
+      __syncthreads();
+      if (tid < BCH) {  // dbeta, and dg as a suffix sum of db
+        float2 s = red[tid];
+        float su = 0.f, em = 0.f, st = 0.f;
+#pragma unroll
+        for (int w = 1; w < 4; ++w) { s.x += red[w * BCH + tid].x; s.y += red[w * BCH + tid].y; }
+#pragma unroll
+        for (int w = 0; w < 8; ++w) su += uv[w * BCH + tid];
+#pragma unroll
+        for (int w = 0; w < 16; ++w) { em += dots[w]; st += dots[16 + w]; }
+        const float be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
+        const int64_t off = (row0 + tid) * a.Hv + h;
+        if (tid < c.len) a.d_beta[off] = su + s.y / be;
+        float db = s.x;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const float x = __shfl_down_sync(0xffffffffu, db, o);
+          if (lane + o < 32) db += x;
+        }
+        if (tid == 32) dots[32] = db;
+        asm volatile("bar.sync 1, 64;" ::: "memory");
+        if (warp == 0) db += dots[32];
+        if (tid < c.len) a.d_g[off] = db + st + __expf(bs[BCH - 1]) * em;
+      }
     }
   }
   __syncthreads();
   if (tid == 0 && *abort_flag != 0u && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
-  if (warp == 1) tc::tmem_dealloc(tm, 512);
+  if (warp == 1) tc::tmem_dealloc(*tmem_slot, 512);
 }
 
 int64_t backward_slots(const AveGdnBwdArgs& a) { return (int64_t)a.B * a.T / BCH + a.n_seqs + 1; }
@@ -902,7 +937,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
   bwd_reverse_kernel<<<2 * units, SC_T, 2 * RV_STAGE, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
   const bool sum = (a.flags & AVE_GDN_FLAG_BWD_SUMMED) != 0;
-  (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<dim3(slots, (unsigned)a.Hk), GR_T, GR_SMEM, stream>>>(a, ws);
+  (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<(unsigned)min((int64_t)GR_CTAS, (int64_t)slots * a.Hk), GR_T, GR_SMEM, stream>>>(a, ws, slots);
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }
