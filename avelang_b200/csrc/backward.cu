@@ -14,19 +14,16 @@
 //     db_i    = q_i.dq_i + k_i.row_i - k_i.col_i,  and  dg_t = sum_{i >= t} db_i + sum_j k_j.(D_j (Vn E^T)_j) + e^{b_C} <E, M0>
 //           (b_i rides on q_i and on the row side of k_i with a plus sign, on the column side of k_i with a minus sign).
 //
-// Four launches.  bwd_prep: T, P and b of every (chunk, value head), in parallel.  bwd_forward: the states and Vn, chunk
-// after chunk; bwd_reverse: the state gradients and Ut, chunk after chunk from the end (it needs nothing of bwd_forward).
+// Three launches.  bwd_prep: T, P and b of every (chunk, value head), in parallel.  bwd_scans: the states and Vn, chunk after
+// chunk, and beside them the state gradients and Ut, chunk after chunk from the end (neither needs anything of the other).
 // bwd_grads: everything else, in parallel over (chunk, key head), summing over the value heads that share the key head.
 //
-// The contractions run on warp-level bf16 MMAs (bwd_grads: on tcgen05) with fp32 accumulation.  q, k, v and dO are bf16 and enter as they are;
-// every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with one fp32 operand is
-// three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which the gradient of
-// the gate needs, because it is a difference of large sums.
-// The scans hold the state transposed, H = M^T: a warp owns 16 of the 128 d_v rows for the whole sequence, every product
-// is (its rows) x (a tile all warps read), and the accumulator of one product is, in place, the left operand of the next,
-// so the warps of a chain never exchange anything and only meet where a tile buffer is refilled.
-// Two sequences of 4096 tokens, 32 value heads: 1.20 ms (prep 0.12, forward scan 0.27, reverse scan 0.38, gradients 0.44)
-// against 22.1 ms for the token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
+// The contractions run on bf16 MMAs (bwd_prep: warp-level, the others: tcgen05) with fp32 accumulation.  q, k, v and dO are bf16
+// and enter as they are; every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with
+// one fp32 operand is three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which
+// the gradient of the gate needs, because it is a difference of large sums.
+// Two sequences of 4096 tokens, 32 value heads: 0.90 ms (prep 0.12, scans 0.34, gradients 0.44) against 22.1 ms for the
+// token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
 #include "blockalg.cuh"
 #include "common.cuh"
 #include "tc.cuh"
@@ -42,8 +39,8 @@ constexpr int STATE_FLOATS = BD * BD, VEC_FLOATS = BD * BCH;
 
 struct BwdScratch {
   uint8_t* prep;   // [slots][Hv][PREP_BYTES]; the tiles are stored as the swizzled shared-memory images the scans read
-  float *m0, *e;   // [slots][Hv][d_v][d_k]: H = M0^T and E^T of every chunk
-  float *vn, *u;   // [slots][Hv][d_v][64 tokens]: Vn^T and Ut^T
+  float *m0, *e;   // [slots][Hv][d_k / 8][d_v][8]: H = M0^T and E^T of every chunk
+  float *vn, *u;   // [slots][Hv][64 tokens / 8][d_v][8]: Vn^T and Ut^T
 };
 
 // Chunk j of sequence n has record slot floor(first token of n / 64) + n + j: unique, needs no table, and the sequence of a
@@ -234,271 +231,280 @@ __global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a,
 }
 
 // ---------------------------------------------------------------------------------------------- the two scans
-// One CTA of four warps per (sequence, value head, half of d_v): a warp owns 16 rows of the transposed state.
-constexpr int SC_T = 128;
-constexpr int FW_K = 0, FW_V = 16384, FW_TI = FW_V + 8192, FW_SC = FW_TI + 3 * IMG, FW_STAGE = FW_SC + SC_BYTES;
-constexpr int RV_K = 0, RV_Q = 16384, RV_DO = 32768, RV_TI = RV_DO + 8192, RV_PI = RV_TI + 3 * IMG, RV_SC = RV_PI + 3 * IMG,
-              RV_STAGE = RV_SC + SC_BYTES;
+// One CTA of 16 warps per (sequence, value head) and direction, in one launch.  The state stays transposed, S = H or E, d_v on the
+// 128 tensor-memory lanes: a thread keeps 32 of a row's 128 elements in fp32 registers, and S, the left operand of the first
+// product, X and (reverse) dO^T live in tensor memory as three bf16 terms each.  A chunk is three dependent products,
+//     x = S K^T,   y = (f(x, V or dO P)) T or T^T,   S += (f(y)) K   (reverse: and the scaled dO)^T Q,
+// with a pass of all threads over the result behind each; the product of the pass's tile is issued by two threads, into
+// accumulators (or column halves) of their own.  The chain is bound by these hand-offs, about 1 k cycles each beside 0.8 k of
+// MMAs.  Tiles of the next chunk land meanwhile.  Two sequences of 4096 tokens, 32 value heads: 0.34 ms; on warp-level MMAs, whose
+// pipe was full (504 and 756 of them a warp and chunk, 16 cycles each), the two scans took 0.27 + 0.38 ms one after the other.
+constexpr int SC_T = 512;
+constexpr int SC_K = 0, FW_V = 16384, FW_TI = 32768, FW_SC = FW_TI + 3 * IMG, FW_STAGE = FW_SC + 1024;
+constexpr int RV_Q = 16384, RV_DO = 32768, RV_TI = 49152, RV_PI = RV_TI + 3 * IMG, RV_SC = RV_PI + 3 * IMG, RV_STAGE = RV_SC + 1024;
+constexpr int SC_FAC = 2 * RV_STAGE, SC_BAR = SC_FAC + BCH * 16, SC_SMEM = SC_BAR + 64;
+static_assert(FW_STAGE % 1024 == 0 && RV_STAGE % 1024 == 0 && SC_SMEM <= 227 * 1024, "shared memory");
+// tensor-memory columns.  State terms: [half of d_k][term][32]; the increment's accumulator takes the first 64 of each half.
+constexpr uint32_t TS_S = 0, TS_HALF = 96, TS_X = 192, TS_DO = 288, TS_ACC = 384, TS_ACC2 = 448;
 
-struct ScanUnit { SeqSpan sp; int n, h, hk, row0; int64_t slot0, tile; };
-__device__ __forceinline__ ScanUnit scan_unit(const AveGdnBwdArgs& a, int block, int warp) {
-  ScanUnit u;
-  const int unit = block >> 1;
-  u.n = unit / a.Hv; u.h = unit % a.Hv; u.hk = u.h / (a.Hv / a.Hk);
-  u.row0 = (block & 1) * 64 + warp * 16;
-  u.sp = seq_span(a.cu_seqlens, u.n, a.T, a.status);
-  u.slot0 = u.sp.ok ? first_slot(a, u.n) : 0;
-  u.tile = ((int64_t)u.n * a.Hv + u.h) * STATE_FLOATS;
-  return u;
+// The fp32 records of a chunk, [d_v][N]: eight elements of a row are one 32-byte unit, units in the order [N / 8][d_v], so that
+// the scans (a lane is a row) and bwd_grads (a lane is half a unit) both move whole lines.
+__device__ __forceinline__ void store_unit(float* rec, int unit, int row, const float* v) {
+  float* p = rec + (unit * BD + row) * 8;
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]),
+               "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
 }
-// rows row0 + g (+ 8), columns 8 nt + 2 t (+ 1) of the transposed state <-> a key-major [d_k][d_v] state in memory
-__device__ __forceinline__ void load_state(float (&H)[16][4], const float* src, int row0, int lane) {
-  const int g = lane >> 2, t = lane & 3;
+// N fp32 values -> three terms, N / 2 tensor-memory columns each, `step` columns apart
+template <int N>
+__device__ __forceinline__ void store_terms(uint32_t at, uint32_t step, const float (&x)[N]) {
+  uint32_t h[N / 2], m[N / 2], l[N / 2];
 #pragma unroll
-  for (int nt = 0; nt < 16; ++nt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) H[nt][e] = src != nullptr ? src[(int64_t)(8 * nt + 2 * t + (e & 1)) * BD + row0 + g + 8 * (e >> 1)] : 0.f;
-}
-__device__ __forceinline__ void store_rows(float* dst, const float (&H)[16][4], int lane) {  // dst: first of this warp's rows, [d_v][d_k]
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int nt = 0; nt < 16; ++nt) {
-    *reinterpret_cast<float2*>(dst + g * BD + 8 * nt + 2 * t) = make_float2(H[nt][0], H[nt][1]);
-    *reinterpret_cast<float2*>(dst + (g + 8) * BD + 8 * nt + 2 * t) = make_float2(H[nt][2], H[nt][3]);
-  }
-}
-__device__ __forceinline__ void store_vec(float* dst, const float (&v)[8][4], int lane) {  // [d_v][64 tokens]
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    *reinterpret_cast<float2*>(dst + g * BCH + 8 * nt + 2 * t) = make_float2(v[nt][0], v[nt][1]);
-    *reinterpret_cast<float2*>(dst + (g + 8) * BCH + 8 * nt + 2 * t) = make_float2(v[nt][2], v[nt][3]);
-  }
-}
-// acc[16 rows][64 tokens] = H K^T, K a [64][128] tile
-__device__ __forceinline__ void state_times_kt(float (&acc)[8][4], const float (&H)[16][4], uint32_t k_tile, int lane) {
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) zero(acc[nt]);
-#pragma unroll
-  for (int ks = 0; ks < 8; ++ks) {
-    uint32_t ah[4], am[4], al[4];
-    split_acc(H[2 * ks], H[2 * ks + 1], ah, am, al);
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {
-      uint32_t b[4];
-      ldsm4(b, k_tile + at_b<256>(16 * np, 2 * ks, lane));
-      mma3(acc[2 * np], ah, am, al, b[0], b[1]);
-      mma3(acc[2 * np + 1], ah, am, al, b[2], b[3]);
-    }
-  }
-}
-// H[16 rows][128] += X[16 rows][64 tokens] K, K a [64][128] tile
-__device__ __forceinline__ void add_times_k(float (&H)[16][4], const float (&X)[8][4], uint32_t k_tile, int lane) {
-#pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    uint32_t ah[4], am[4], al[4];
-    split_acc(X[2 * ks], X[2 * ks + 1], ah, am, al);
-#pragma unroll
-    for (int np = 0; np < 8; ++np) {
-      uint32_t b[4];
-      ldsm4t(b, k_tile + at_bt<256>(16 * ks, 2 * np, lane));
-      mma3(H[2 * np], ah, am, al, b[0], b[1]);
-      mma3(H[2 * np + 1], ah, am, al, b[2], b[3]);
-    }
-  }
+  for (int i = 0; i < N / 2; ++i) split3(make_float2(x[2 * i], x[2 * i + 1]), h[i], m[i], l[i]);
+  tc::tmem_st_n(at, h);
+  tc::tmem_st_n(at + step, m);
+  tc::tmem_st_n(at + 2 * step, l);
 }
 
-__global__ void __launch_bounds__(SC_T, 2) bwd_forward_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, t = lane & 3;
-  const ScanUnit u = scan_unit(a, blockIdx.x, warp);
-  if (!u.sp.ok || u.sp.len == 0) return;
-  const int n_chunks = (u.sp.len + BCH - 1) / BCH;
-  const __nv_bfloat16* kp = bf(a.k) + u.sp.b * a.k_stride_b + (int64_t)u.sp.t0 * a.k_stride_t + u.hk * a.k_stride_h;
-  const __nv_bfloat16* vp = bf(a.v) + u.sp.b * a.v_stride_b + (int64_t)u.sp.t0 * a.v_stride_t + u.h * a.v_stride_h + (blockIdx.x & 1) * 64;
-  const uint32_t sb = tc::smem_u32(smem);
-  auto load = [&](int c) {
-    const uint32_t st = sb + (c & 1) * FW_STAGE;
-    const int len = min(BCH, u.sp.len - c * BCH);
-    const uint8_t* rec = ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES;
-    load_tile<BCH, 16, SC_T>(st + FW_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
-    load_tile<BCH, 8, SC_T>(st + FW_V, vp + (int64_t)c * BCH * a.v_stride_t, a.v_stride_t, len, tid);
-    load_flat<3 * IMG, SC_T>(st + FW_TI, rec, tid);
-    load_flat<SC_BYTES, SC_T>(st + FW_SC, rec + PREP_SC, tid);
-  };
-  load(0);
-  cp_commit();
-  float H[16][4];
-  load_state(H, a.initial_state ? a.initial_state + u.tile : nullptr, u.row0, lane);
-  for (int c = 0; c < n_chunks; ++c) {
-    if (c + 1 < n_chunks) load(c + 1);
-    cp_commit();
-    cp_wait<1>();
-    __syncthreads();
-    const uint32_t st = sb + (c & 1) * FW_STAGE;
-    const float* bs = reinterpret_cast<const float*>(smem + (c & 1) * FW_STAGE + FW_SC);
-    const float* betas = bs + BCH;
-    const int64_t rec = (u.slot0 + c) * a.Hv + u.h;
-    store_rows(ws.m0 + rec * STATE_FLOATS + (int64_t)u.row0 * BD, H, lane);
-    float x[8][4], vn[8][4];
-    state_times_kt(x, H, st + FW_K, lane);
-#pragma unroll
-    for (int np = 0; np < 4; ++np) {  // X^T = beta (V^T - e^b (K M0)^T)
-      uint32_t v[4];
-      ldsm4t(v, st + FW_V + piece<128>(16 * np + (lane & 7) + ((lane >> 4) << 3), (u.row0 & 63) / 8 + ((lane >> 3) & 1)));
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int nt = 2 * np + e;
-        const float2 b = *reinterpret_cast<const float2*>(bs + 8 * nt + 2 * t), be = *reinterpret_cast<const float2*>(betas + 8 * nt + 2 * t);
-        const float e0 = __expf(b.x), e1 = __expf(b.y);
-        const float2 v0 = bf16x2_to_float2(v[2 * e]), v1 = bf16x2_to_float2(v[2 * e + 1]);
-        x[nt][0] = be.x * (v0.x - e0 * x[nt][0]); x[nt][1] = be.y * (v0.y - e1 * x[nt][1]);
-        x[nt][2] = be.x * (v1.x - e0 * x[nt][2]); x[nt][3] = be.y * (v1.y - e1 * x[nt][3]);
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) zero(vn[nt]);
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {  // Vn^T = X^T T^T
-      uint32_t ah[4], am[4], al[4];
-      split_acc(x[2 * ks], x[2 * ks + 1], ah, am, al);
-#pragma unroll
-      for (int np = ks; np < 4; ++np) {
-        uint32_t th[4], tm[4], tl[4];
-        const uint32_t at = st + FW_TI + at_b<128>(16 * np, 2 * ks, lane);
-        ldsm4(th, at); ldsm4(tm, at + IMG); ldsm4(tl, at + 2 * IMG);
-        mma6(vn[2 * np], ah, am, al, th[0], th[1], tm[0], tm[1], tl[0], tl[1]);
-        mma6(vn[2 * np + 1], ah, am, al, th[2], th[3], tm[2], tm[3], tl[2], tl[3]);
-      }
-    }
-    store_vec(ws.vn + rec * VEC_FLOATS + u.row0 * BCH, vn, lane);
-    if (c + 1 == n_chunks) break;
-    const float bC = bs[BCH - 1], decay = __expf(bC);
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const float d0 = gate_between(bs, BCH - 1, 8 * nt + 2 * t), d1 = gate_between(bs, BCH - 1, 8 * nt + 2 * t + 1);
-      vn[nt][0] *= d0; vn[nt][1] *= d1; vn[nt][2] *= d0; vn[nt][3] *= d1;
-    }
-#pragma unroll
-    for (int nt = 0; nt < 16; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) H[nt][e] *= decay;
-    add_times_k(H, vn, st + FW_K, lane);
-    __syncthreads();  // every warp is done with this stage before it is refilled
-  }
-}
-
-__global__ void __launch_bounds__(SC_T, 1) bwd_reverse_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const ScanUnit u = scan_unit(a, blockIdx.x, warp);
-  if (!u.sp.ok) return;
-  if (u.sp.len == 0) {  // empty sequence: the state gradient passes through
-    if (a.d_initial_state != nullptr)
-      for (int e = tid + (blockIdx.x & 1) * (STATE_FLOATS / 2); e < ((int)(blockIdx.x & 1) + 1) * (STATE_FLOATS / 2); e += SC_T)
-        a.d_initial_state[u.tile + e] = a.d_final_state ? a.d_final_state[u.tile + e] : 0.f;
+template <bool kRev>
+__device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratch& ws, int unit, uint8_t* smem) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n = unit / a.Hv, h = unit % a.Hv, hk = h / (a.Hv / a.Hk);
+  const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
+  if (!sp.ok) return;
+  const int64_t tile = (int64_t)unit * STATE_FLOATS;
+  if (sp.len == 0) {  // empty sequence: the state gradient passes through
+    if (kRev && a.d_initial_state != nullptr)
+      for (int e = tid; e < STATE_FLOATS; e += SC_T) a.d_initial_state[tile + e] = a.d_final_state ? a.d_final_state[tile + e] : 0.f;
     return;
   }
-  const int n_chunks = (u.sp.len + BCH - 1) / BCH;
-  const __nv_bfloat16* kp = bf(a.k) + u.sp.b * a.k_stride_b + (int64_t)u.sp.t0 * a.k_stride_t + u.hk * a.k_stride_h;
-  const __nv_bfloat16* qp = bf(a.q) + u.sp.b * a.q_stride_b + (int64_t)u.sp.t0 * a.q_stride_t + u.hk * a.q_stride_h;
-  const __nv_bfloat16* dop = bf(a.d_o) + u.sp.b * a.do_stride_b + (int64_t)u.sp.t0 * a.do_stride_t + u.h * a.do_stride_h + (blockIdx.x & 1) * 64;
+  constexpr int STAGE = kRev ? RV_STAGE : FW_STAGE, TI = kRev ? RV_TI : FW_TI, SC = kRev ? RV_SC : FW_SC, ROWS = kRev ? RV_DO : FW_V;
+  const int64_t slot0 = first_slot(a, n);
+  const int n_chunks = (sp.len + BCH - 1) / BCH;
+  const __nv_bfloat16* kp = bf(a.k) + sp.b * a.k_stride_b + (int64_t)sp.t0 * a.k_stride_t + hk * a.k_stride_h;
+  const __nv_bfloat16* qp = bf(a.q) + sp.b * a.q_stride_b + (int64_t)sp.t0 * a.q_stride_t + hk * a.q_stride_h;
+  const __nv_bfloat16* vp = bf(a.v) + sp.b * a.v_stride_b + (int64_t)sp.t0 * a.v_stride_t + h * a.v_stride_h;
+  const __nv_bfloat16* dop = bf(a.d_o) + sp.b * a.do_stride_b + (int64_t)sp.t0 * a.do_stride_t + h * a.do_stride_h;
   const uint32_t sb = tc::smem_u32(smem);
+  float4* fac = reinterpret_cast<float4*>(smem + SC_FAC);       // per token: forward beta, e^b, D; reverse D, S e^b, -beta e^b
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SC_BAR);  // one per product
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + SC_BAR + 32);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SC_BAR + 40);
   auto load = [&](int c) {
-    const uint32_t st = sb + (c & 1) * RV_STAGE;
-    const int len = min(BCH, u.sp.len - c * BCH);
-    load_tile<BCH, 16, SC_T>(st + RV_K, kp + (int64_t)c * BCH * a.k_stride_t, a.k_stride_t, len, tid);
-    load_tile<BCH, 16, SC_T>(st + RV_Q, qp + (int64_t)c * BCH * a.q_stride_t, a.q_stride_t, len, tid);
-    load_tile<BCH, 8, SC_T>(st + RV_DO, dop + (int64_t)c * BCH * a.do_stride_t, a.do_stride_t, len, tid);
-    load_flat<PREP_BYTES, SC_T>(st + RV_TI, ws.prep + ((u.slot0 + c) * a.Hv + u.h) * PREP_BYTES, tid);
-  };
-  load(n_chunks - 1);
-  cp_commit();
-  float E[16][4];
-  load_state(E, a.d_final_state ? a.d_final_state + u.tile : nullptr, u.row0, lane);
-  for (int c = n_chunks - 1; c >= 0; --c) {
-    if (c > 0) load(c - 1);
-    cp_commit();
-    cp_wait<1>();
-    __syncthreads();
-    const uint32_t st = sb + (c & 1) * RV_STAGE;
-    const float* bs = reinterpret_cast<const float*>(smem + (c & 1) * RV_STAGE + RV_SC);
-    const float* betas = bs + BCH;
-    const int64_t rec = (u.slot0 + c) * a.Hv + u.h;
-    store_rows(ws.e + rec * STATE_FLOATS + (int64_t)u.row0 * BD, E, lane);
-    const float bC = bs[BCH - 1], decay = __expf(bC);
-    float x[8][4], ut[8][4];
-    state_times_kt(x, E, st + RV_K, lane);
-    // x = dVn^T = D (E^T K^T) + S (dO^T P)
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const float d0 = gate_between(bs, BCH - 1, 8 * nt + 2 * t), d1 = gate_between(bs, BCH - 1, 8 * nt + 2 * t + 1);
-      x[nt][0] *= d0; x[nt][1] *= d1; x[nt][2] *= d0; x[nt][3] *= d1;
-      zero(ut[nt]);
+    const uint32_t st = sb + (c & 1) * STAGE;
+    const int len = min(BCH, sp.len - c * BCH);
+    auto tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
+      load_tile<BCH, 8, SC_T>(st + at, src + (int64_t)c * BCH * stride, stride, len, tid);
+      load_tile<BCH, 8, SC_T>(st + at + 8192, src + (int64_t)c * BCH * stride + 64, stride, len, tid);
+    };
+    const uint8_t* rec = ws.prep + ((slot0 + c) * a.Hv + h) * PREP_BYTES;
+    tiles(SC_K, kp, a.k_stride_t);
+    if constexpr (kRev) {
+      tiles(RV_Q, qp, a.q_stride_t);
+      tiles(RV_DO, dop, a.do_stride_t);
+      load_flat<PREP_BYTES, SC_T>(st + RV_TI, rec, tid);
+    } else {
+      tiles(FW_V, vp, a.v_stride_t);
+      load_flat<3 * IMG, SC_T>(st + FW_TI, rec, tid);
+      load_flat<SC_BYTES, SC_T>(st + FW_SC, rec + PREP_SC, tid);
     }
-    uint32_t doa[4][4];  // dO^T, this warp's rows x 64 tokens
+    cp_commit();
+  };
+  load(kRev ? n_chunks - 1 : 0);
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) tc::mbar_init(&bars[i], 2);  // commits of the two issuers
+    *abort_flag = 0u;
+    tc::fence_barrier_init();
+  }
+  if (warp == 2) tc::tmem_alloc(tmem_slot, 512);
+  // this thread: row `row` of d_v; 16 tokens from 16 grp; 32 columns of d_k from 32 grp
+  const int grp = warp >> 2, quarter = warp & 3, row = 32 * quarter + lane;
+  float S[32];
+  {
+    const float* src = kRev ? a.d_final_state : a.initial_state;
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks) ldsm4t(doa[ks], st + RV_DO + at_at<128>(16 * ks, (u.row0 & 63) / 8, lane));
+    for (int i = 0; i < 32; ++i) S[i] = src != nullptr ? src[tile + (int64_t)(32 * grp + i) * BD + row] : 0.f;
+  }
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tm = *tmem_slot, lanes = tm + ((uint32_t)(32 * quarter) << 16);
+  const uint32_t s_cols = lanes + TS_S + (grp >> 1) * TS_HALF;
+  store_terms<32>(s_cols + 16 * (grp & 1), 32, S);
+#pragma unroll 1
+  for (int it = 0; it < n_chunks; ++it) {
+    const int c = kRev ? n_chunks - 1 - it : it;
+    const uint32_t st = sb + (c & 1) * STAGE, phase = it & 1;
+    uint8_t* stage = smem + (c & 1) * STAGE;
+    const float* bs = reinterpret_cast<const float*>(stage + SC);
+    const int64_t rec = (slot0 + c) * a.Hv + h;
+    const int len = min(BCH, sp.len - c * BCH);
+    const bool last = it + 1 == n_chunks, update = kRev ? !last || a.d_initial_state != nullptr : !last;
+    tc::tmem_st_wait();
+    cp_wait<0>();
+    tc::fence_proxy_async_smem();
+    tc::tc_fence_before_sync();
+    __syncthreads();
+    if (warp < 2 && tc::elect_one()) {  // S K^T; forward: its terms over two accumulators; reverse: beside dO^T P
+      tc::tc_fence_after_sync();
+      constexpr uint32_t id = tc::idesc_f16(128, 64, 1, 1, false, false), id_p = tc::idesc_f16(128, 64, 1, 1, true, true);
+      const uint64_t kd = tc::smem_desc_sw128(st + SC_K, 16, 1024);
+      auto step = [&](int i, int ks, uint32_t acc, bool more) {
+        tc::mma_ts(tm + acc, tm + TS_S + (ks >> 2) * TS_HALF + 32 * i + 8 * (ks & 3), kd + (uint64_t)(((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), id, more ? 1u : 0u);
+      };
+      if (kRev && warp == 1) {
+        const uint64_t od = tc::smem_desc_sw128(st + RV_DO, 8192, 1024), pd = tc::smem_desc_sw128(st + RV_PI, 8192, 1024);
 #pragma unroll
-    for (int ks = 0; ks < 4; ++ks)
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int np = 0; np <= ks; ++np) {
-        const uint32_t at = st + RV_PI + at_bt<128>(16 * ks, 2 * np, lane);
+          for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tm + TS_ACC2, od + ks * (2048 >> 4), pd + (i * IMG + ks * 2048 >> 4), id_p, (i | ks) != 0 ? 1u : 0u);
+      } else if (kRev) {
 #pragma unroll
-        for (int term = 0; term < 3; ++term) {
-          uint32_t b[4];
-          ldsm4t(b, at + term * IMG);
-          mma_bf16(ut[2 * np], doa[ks], b[0], b[1]);
-          mma_bf16(ut[2 * np + 1], doa[ks], b[2], b[3]);
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int ks = 0; ks < 8; ++ks) step(i, ks, TS_ACC, (i | ks) != 0);
+      } else {
+#pragma unroll
+        for (int ks = 0; ks < 8; ++ks) step(warp == 0 ? 0 : 2, ks, warp == 0 ? TS_ACC : TS_ACC2, ks != 0);
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) step(1, warp == 0 ? ks : 4 + ks, warp == 0 ? TS_ACC : TS_ACC2, true);
+      }
+      tc::mma_commit(&bars[0]);
+    }
+    __syncwarp();
+    if (!last) load(kRev ? c - 1 : c + 1);
+    if (tid < BCH) {
+      const float eb = __expf(bs[tid]), be = bs[BCH + tid], D = gate_between(bs, BCH - 1, tid);
+      fac[tid] = kRev ? make_float4(D, tid < len ? a.scale * eb : 0.f, -be * eb, 0.f) : make_float4(be, eb, D, 0.f);
+    }
+    {
+      float* dst = (kRev ? ws.e : ws.m0) + rec * STATE_FLOATS;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) store_unit(dst, 4 * grp + i, row, S + 8 * i);
+    }
+    const float decay = __expf(bs[BCH - 1]);
+    float rows[16];  // V^T or dO^T
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      rows[i] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(stage + ROWS + (row >> 6) * 8192 + piece<128>(16 * grp + i, (row & 63) >> 3) + 2 * (row & 7)));
+    __syncthreads();  // the factors are complete
+    if constexpr (kRev) {
+      if (update) {
+        float x[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) x[i] = fac[16 * grp + i].y * rows[i];
+        store_terms<16>(lanes + TS_DO + 8 * grp, 32, x);
+      }
+    }
+    tc::mbar_wait_warp(&bars[0], phase, abort_flag);
+    tc::tc_fence_after_sync();
+    {
+      uint32_t u[16], w[16];
+      tc::tmem_ld16(lanes + TS_ACC + 16 * grp, u);
+      tc::tmem_ld16(lanes + TS_ACC2 + 16 * grp, w);
+      tc::tmem_ld_wait();
+      float x[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const float4 f = fac[16 * grp + i];
+        if (kRev) x[i] = fmaf(a.scale, __uint_as_float(w[i]), f.x * __uint_as_float(u[i]));       // D (E^T K^T) + S (dO^T P)
+        else x[i] = f.x * (rows[i] - f.y * (__uint_as_float(u[i]) + __uint_as_float(w[i])));       // beta (V^T - e^b (K M0)^T)
+      }
+      store_terms<16>(lanes + TS_X + 8 * grp, 32, x);
+    }
+    tc::tmem_st_wait();
+    tc::tc_fence_before_sync();
+    __syncthreads();
+    if (warp < 2 && tc::elect_one()) {  // X T^T or X T, the six term products over two accumulators
+      tc::tc_fence_after_sync();
+      constexpr int L[2][3] = {{0, 0, 1}, {0, 2, 1}}, R[2][3] = {{0, 1, 0}, {2, 0, 1}};  // hh hm mh | hl lh mm
+      const uint32_t acc = tm + (warp == 0 ? TS_ACC : TS_ACC2);
+      const uint64_t td = tc::smem_desc_sw128(st + TI, kRev ? 8192 : 16, 1024);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) {
+        const uint32_t l = tm + TS_X + 32 * (warp == 0 ? L[0][j] : L[1][j]);
+        const uint64_t r = td + (uint64_t)((warp == 0 ? R[0][j] : R[1][j]) * (IMG >> 4));
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          if constexpr (kRev) tc::mma_ts(acc, l + 8 * ks, r + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), (j | ks) != 0 ? 1u : 0u);
+          else  // tokens from 16 ks on: T is lower triangular
+            tc::mma_ts(acc + 16 * ks, l + 8 * ks, r + ks * ((2048 + 32) >> 4), tc::idesc_f16(128, 64 - 16 * ks, 1, 1, false, false), (j | ks) != 0 ? 1u : 0u);
         }
       }
+      tc::mma_commit(&bars[1]);
+      if (kRev && update) {  // (S e^b dO)^T Q, this issuer's half of d_k, opens the increment
+        const uint64_t qd = tc::smem_desc_sw128(st + RV_Q + warp * 8192, 8192, 1024);
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) x[nt][e] = fmaf(a.scale, ut[nt][e], x[nt][e]);
-      zero(ut[nt]);
-    }
-#pragma unroll
-    for (int ks = 0; ks < 4; ++ks) {  // Ut^T = dVn^T T
-      uint32_t ah[4], am[4], al[4];
-      split_acc(x[2 * ks], x[2 * ks + 1], ah, am, al);
-#pragma unroll
-      for (int np = 0; np <= ks; ++np) {
-        uint32_t th[4], tm[4], tl[4];
-        const uint32_t at = st + RV_TI + at_bt<128>(16 * ks, 2 * np, lane);
-        ldsm4t(th, at); ldsm4t(tm, at + IMG); ldsm4t(tl, at + 2 * IMG);
-        mma6(ut[2 * np], ah, am, al, th[0], th[1], tm[0], tm[1], tl[0], tl[1]);
-        mma6(ut[2 * np + 1], ah, am, al, th[2], th[3], tm[2], tm[3], tl[2], tl[3]);
+          for (int ks = 0; ks < 4; ++ks)
+            tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_DO + 32 * i + 8 * ks, qd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), (i | ks) != 0 ? 1u : 0u);
       }
     }
-    store_vec(ws.u + rec * VEC_FLOATS + u.row0 * BCH, ut, lane);
-    if (c == 0 && a.d_initial_state == nullptr) break;
-    // E <- e^{b_C} E + (S e^b dO)^T Q - (beta e^b Ut)^T K
+    __syncwarp();
+    tc::mbar_wait_warp(&bars[1], phase, abort_flag);
+    tc::tc_fence_after_sync();
+    {
+      uint32_t u[16], w[16];
+      tc::tmem_ld16(lanes + TS_ACC + 16 * grp, u);
+      tc::tmem_ld16(lanes + TS_ACC2 + 16 * grp, w);
+      tc::tmem_ld_wait();
+      float y[16];
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt)
+      for (int i = 0; i < 16; ++i) y[i] = __uint_as_float(u[i]) + __uint_as_float(w[i]);
+      float* dst = (kRev ? ws.u : ws.vn) + rec * VEC_FLOATS;
+      store_unit(dst, 2 * grp, row, y);
+      store_unit(dst, 2 * grp + 1, row, y + 8);
+      if (update) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) E[nt][e] *= decay;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      const float2 b = *reinterpret_cast<const float2*>(bs + 8 * nt + 2 * t), be = *reinterpret_cast<const float2*>(betas + 8 * nt + 2 * t);
-      const float f0 = __expf(b.x), f1 = __expf(b.y);
-      const float2 o0 = bf16x2_to_float2(doa[nt >> 1][2 * (nt & 1)]), o1 = bf16x2_to_float2(doa[nt >> 1][2 * (nt & 1) + 1]);
-      const float s0 = a.scale * f0, s1 = a.scale * f1;
-      x[nt][0] = s0 * o0.x; x[nt][1] = s1 * o0.y; x[nt][2] = s0 * o1.x; x[nt][3] = s1 * o1.y;
-      const float u0 = -be.x * f0, u1 = -be.y * f1;
-      ut[nt][0] *= u0; ut[nt][1] *= u1; ut[nt][2] *= u0; ut[nt][3] *= u1;
+        for (int i = 0; i < 16; ++i) y[i] *= fac[16 * grp + i].z;
+        store_terms<16>(lanes + TS_X + 8 * grp, 32, y);
+      }
     }
-    add_times_k(E, x, st + RV_Q, lane);
-    add_times_k(E, ut, st + RV_K, lane);
+    if (!update) break;
+    tc::tmem_st_wait();
+    tc::tc_fence_before_sync();
     __syncthreads();
-  }
-  if (a.d_initial_state != nullptr) {
-    float* dst = a.d_initial_state + u.tile;
+    if (warp < 2 && tc::elect_one()) {  // the increment: X K, this issuer's half of d_k
+      tc::tc_fence_after_sync();
+      const uint64_t kd = tc::smem_desc_sw128(st + SC_K + warp * 8192, 8192, 1024);
 #pragma unroll
-    for (int nt = 0; nt < 16; ++nt)
+      for (int i = 0; i < 3; ++i)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) dst[(int64_t)(8 * nt + 2 * t + (e & 1)) * BD + u.row0 + g + 8 * (e >> 1)] = E[nt][e];
+        for (int ks = 0; ks < 4; ++ks)
+          tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_X + 32 * i + 8 * ks, kd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), kRev || (i | ks) != 0 ? 1u : 0u);
+      tc::mma_commit(&bars[2]);
+    }
+    __syncwarp();
+    tc::mbar_wait_warp(&bars[2], phase, abort_flag);
+    tc::tc_fence_after_sync();
+    {
+      uint32_t d[32];
+      tc::tmem_ld32(s_cols + 32 * (grp & 1), d);
+      tc::tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 32; ++i) S[i] = fmaf(decay, S[i], __uint_as_float(d[i]));
+      // the two warps of this half and quarter have both read the accumulator: the new terms take its columns
+      tc::tc_fence_before_sync();
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + 4 * (grp >> 1) + quarter) : "memory");
+      tc::tc_fence_after_sync();
+      if (!last) store_terms<32>(s_cols + 16 * (grp & 1), 32, S);
+    }
   }
+  if (kRev && a.d_initial_state != nullptr) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) a.d_initial_state[tile + (int64_t)(32 * grp + i) * BD + row] = S[i];
+  }
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  if (tid == 0 && *abort_flag != 0u && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+  if (warp == 2) tc::tmem_dealloc(tm, 512);
+}
+__global__ void __launch_bounds__(SC_T, 1) bwd_scans_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const int units = a.n_seqs * a.Hv;
+  if ((int)blockIdx.x < units) bwd_scan<true>(a, ws, blockIdx.x, smem);
+  else bwd_scan<false>(a, ws, blockIdx.x - units, smem);
 }
 
 // ---------------------------------------------------------------------------------------------- the gradients of one chunk
@@ -526,22 +532,22 @@ __device__ __forceinline__ void fetch_tile(float4 (&x)[4], const float* src, int
 __device__ __forceinline__ void split_tile(uint8_t* dst, const float4 (&x)[4], int tid) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int e = tid + i * GR_T, row = e >> 4, q4 = e & 15;
+    const int e = tid + i * GR_T, unit = e >> 8, row = (e >> 1) & (BD - 1);
     uint32_t h[2], m[2], l[2];
     split3(make_float2(x[i].x, x[i].y), h[0], m[0], l[0]);
     split3(make_float2(x[i].z, x[i].w), h[1], m[1], l[1]);
-    uint8_t* p = dst + piece<128>(row, q4 >> 1) + 8 * (q4 & 1);
+    uint8_t* p = dst + piece<128>(row, unit) + 8 * (e & 1);
     *reinterpret_cast<uint2*>(p) = make_uint2(h[0], h[1]);
     *reinterpret_cast<uint2*>(p + 16384) = make_uint2(m[0], m[1]);
     *reinterpret_cast<uint2*>(p + 32768) = make_uint2(l[0], l[1]);
   }
 }
-// four adjacent fp32 of row `row` (d_v) of a 16-row step -> the three tiles of the step, [128 d_k / 64][16 rows][128 bytes]
-__device__ __forceinline__ void split_step(uint8_t* dst, const float4& x, int row, int lane) {
+// half a unit of a 16-row step (d_v), unit = warp, row = lane / 2 -> the three tiles of the step, [128 d_k / 64][16 rows][128 bytes]
+__device__ __forceinline__ void split_step(uint8_t* dst, const float4& x, int warp, int lane) {
   uint32_t h[2], m[2], l[2];
   split3(make_float2(x.x, x.y), h[0], m[0], l[0]);
   split3(make_float2(x.z, x.w), h[1], m[1], l[1]);
-  uint8_t* p = dst + (lane >> 4) * (GR_TERM / 2) + piece<128>(row, (lane & 15) >> 1) + 8 * (lane & 1);
+  uint8_t* p = dst + (warp >> 3) * (GR_TERM / 2) + piece<128>(lane >> 1, warp & 7) + 8 * (lane & 1);
   *reinterpret_cast<uint2*>(p) = make_uint2(h[0], h[1]);
   *reinterpret_cast<uint2*>(p + GR_TERM) = make_uint2(m[0], m[1]);
   *reinterpret_cast<uint2*>(p + 2 * GR_TERM) = make_uint2(l[0], l[1]);
@@ -643,15 +649,17 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
           tc::bulk_prefetch_l2(ws.e + nrec * STATE_FLOATS, STATE_FLOATS * 4);
         }
       }
-      const float4* hp = reinterpret_cast<const float4*>(ws.m0 + rec * STATE_FLOATS) + tid;  // row warp of a step, columns 4 lane ..
-      const float4* ep = reinterpret_cast<const float4*>(ws.e + rec * STATE_FLOATS) + tid;
+      constexpr int STEP = 2 * GR_DV;  // float4s from one step of d_v rows to the next
+      const int first = (warp * BD + (lane >> 1)) * 2 + (lane & 1);
+      const float4* hp = reinterpret_cast<const float4*>(ws.m0 + rec * STATE_FLOATS) + first;
+      const float4* ep = reinterpret_cast<const float4*>(ws.e + rec * STATE_FLOATS) + first;
       float4 hx[2], ex[2];
       {
         float4 vn[4], ut[4];
         fetch_tile(vn, ws.vn + rec * VEC_FLOATS, tid);
         fetch_tile(ut, ws.u + rec * VEC_FLOATS, tid);
 #pragma unroll
-        for (int s = 0; s < 2; ++s) { hx[s] = __ldcs(hp + s * GR_T); ex[s] = __ldcs(ep + s * GR_T); }
+        for (int s = 0; s < 2; ++s) { hx[s] = __ldcs(hp + s * STEP); ex[s] = __ldcs(ep + s * STEP); }
         split_tile(smem + GR_VN, vn, tid);
         split_tile(smem + GR_U, ut, tid);
       }
@@ -677,7 +685,7 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
         split_step(stage + 3 * GR_TERM, ex[st], warp, lane);
         dot = fmaf(hx[st].x, ex[st].x, fmaf(hx[st].y, ex[st].y, fmaf(hx[st].z, ex[st].z, fmaf(hx[st].w, ex[st].w, dot))));
         tc::fence_proxy_async_smem();  // waits for loads in flight: the next ones go out behind it
-        if (s < 6) { hx[st] = __ldcs(hp + (s + 2) * GR_T); ex[st] = __ldcs(ep + (s + 2) * GR_T); }
+        if (s < 6) { hx[st] = __ldcs(hp + (s + 2) * STEP); ex[st] = __ldcs(ep + (s + 2) * STEP); }
         __syncthreads();
         if (warp < 4 && tc::elect_one()) {  // four issuers; X and Y take the columns of X K and Y K, which come after them
           constexpr uint32_t id_k = tc::idesc_f16(128, 64, 1, 1, true, false), id_mn = tc::idesc_f16(128, 64, 1, 1, true, true),
@@ -922,8 +930,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
   if (dev < 0 || dev >= 64) return AVE_GDN_UNSUPPORTED;
   if (!attr_set_dev[dev]) {
     AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * FW_STAGE));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_reverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * RV_STAGE));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_scans_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SC_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_grads_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_grads_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
     attr_set_dev[dev] = true;  // repeating the calls from another thread is harmless
@@ -932,9 +939,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
   const unsigned slots = (unsigned)backward_slots(a);
   bwd_prep_kernel<<<dim3(slots, (unsigned)a.Hv), PREP_T, PR_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
-  bwd_forward_kernel<<<2 * units, SC_T, 2 * FW_STAGE, stream>>>(a, ws);
-  AVE_CUDA_TRY(cudaGetLastError());
-  bwd_reverse_kernel<<<2 * units, SC_T, 2 * RV_STAGE, stream>>>(a, ws);
+  bwd_scans_kernel<<<2 * units, SC_T, SC_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
   const bool sum = (a.flags & AVE_GDN_FLAG_BWD_SUMMED) != 0;
   (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<(unsigned)min((int64_t)GR_CTAS, (int64_t)slots * a.Hk), GR_T, GR_SMEM, stream>>>(a, ws, slots);
