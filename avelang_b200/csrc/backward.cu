@@ -287,9 +287,9 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
   const __nv_bfloat16* dop = bf(a.d_o) + sp.b * a.do_stride_b + (int64_t)sp.t0 * a.do_stride_t + h * a.do_stride_h;
   const uint32_t sb = tc::smem_u32(smem);
   float4* fac = reinterpret_cast<float4*>(smem + SC_FAC);       // per token: forward beta, e^b, D; reverse D, S e^b, -beta e^b
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SC_BAR);  // one per product
-  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + SC_BAR + 32);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SC_BAR + 40);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SC_BAR);  // one per product, then one per stage
+  volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + SC_BAR + 48);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SC_BAR + 56);
   auto load = [&](int c) {
     const uint32_t st = sb + (c & 1) * STAGE;
     const int len = min(BCH, sp.len - c * BCH);
@@ -297,25 +297,32 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
       load_tile<BCH, 8, SC_T>(st + at, src + (int64_t)c * BCH * stride, stride, len, tid);
       load_tile<BCH, 8, SC_T>(st + at + 8192, src + (int64_t)c * BCH * stride + 64, stride, len, tid);
     };
-    const uint8_t* rec = ws.prep + ((slot0 + c) * a.Hv + h) * PREP_BYTES;
     tiles(SC_K, kp, a.k_stride_t);
     if constexpr (kRev) {
       tiles(RV_Q, qp, a.q_stride_t);
       tiles(RV_DO, dop, a.do_stride_t);
-      load_flat<PREP_BYTES, SC_T>(st + RV_TI, rec, tid);
     } else {
       tiles(FW_V, vp, a.v_stride_t);
-      load_flat<3 * IMG, SC_T>(st + FW_TI, rec, tid);
-      load_flat<SC_BYTES, SC_T>(st + FW_SC, rec + PREP_SC, tid);
     }
     cp_commit();
+    if (tid == 0) {
+      const uint8_t* rec = ws.prep + ((slot0 + c) * a.Hv + h) * PREP_BYTES;
+      uint8_t* dst = smem + (c & 1) * STAGE;
+      tc::mbar_expect_tx(&bars[3 + (c & 1)], kRev ? PREP_BYTES : 3 * IMG + SC_BYTES);
+      if constexpr (kRev) {
+        tc::bulk_load(dst + RV_TI, rec, PREP_BYTES, &bars[3 + (c & 1)]);
+      } else {
+        tc::bulk_load(dst + FW_TI, rec, 3 * IMG, &bars[3 + (c & 1)]);
+        tc::bulk_load(dst + FW_SC, rec + PREP_SC, SC_BYTES, &bars[3 + (c & 1)]);
+      }
+    }
   };
-  load(kRev ? n_chunks - 1 : 0);
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) tc::mbar_init(&bars[i], 2);  // commits of the two issuers
+    for (int i = 0; i < 5; ++i) tc::mbar_init(&bars[i], i < 3 ? 2 : 1);  // commits of the two issuers; the records of the two stages
     *abort_flag = 0u;
     tc::fence_barrier_init();
   }
+  load(kRev ? n_chunks - 1 : 0);
   if (warp == 2) tc::tmem_alloc(tmem_slot, 512);
   // this thread: row `row` of d_v; 16 tokens from 16 grp; 32 columns of d_k from 32 grp
   const int grp = warp >> 2, quarter = warp & 3, row = 32 * quarter + lane;
@@ -325,15 +332,32 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
 #pragma unroll
     for (int i = 0; i < 32; ++i) S[i] = src != nullptr ? src[tile + (int64_t)(32 * grp + i) * BD + row] : 0.f;
   }
+  // all of a chunk's tiles are there for the MMAs (behind the next barrier).  The fence waits for this thread's outstanding
+  // accesses to global memory, so it stands where few are.
+  auto landed = [&](int c, uint32_t n_th) {
+    cp_wait<0>();
+    tc::fence_proxy_async_smem();
+    tc::mbar_wait_warp(&bars[3 + (c & 1)], n_th >> 1 & 1, abort_flag);  // the stage's (n_th / 2)-th use
+  };
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
+  landed(kRev ? n_chunks - 1 : 0, 0);
   const uint32_t tm = *tmem_slot, lanes = tm + ((uint32_t)(32 * quarter) << 16);
   const uint32_t s_cols = lanes + TS_S + (grp >> 1) * TS_HALF;
+  auto issue_do_p = [&](int c) {  // dO^T P of a chunk
+    const uint32_t st = sb + (c & 1) * STAGE;
+    const uint64_t od = tc::smem_desc_sw128(st + RV_DO, 8192, 1024), pd = tc::smem_desc_sw128(st + RV_PI, 8192, 1024);
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int ks = 0; ks < 4; ++ks)
+        tc::mma_ss(tm + TS_ACC2, od + ks * (2048 >> 4), pd + ((i * IMG + ks * 2048) >> 4), tc::idesc_f16(128, 64, 1, 1, true, true), (i | ks) != 0 ? 1u : 0u);
+  };
   store_terms<32>(s_cols + 16 * (grp & 1), 32, S);
 #pragma unroll 1
   for (int it = 0; it < n_chunks; ++it) {
-    const int c = kRev ? n_chunks - 1 - it : it;
+    const int c = kRev ? n_chunks - 1 - it : it, c_next = kRev ? c - 1 : c + 1;
     const uint32_t st = sb + (c & 1) * STAGE, phase = it & 1;
     uint8_t* stage = smem + (c & 1) * STAGE;
     const float* bs = reinterpret_cast<const float*>(stage + SC);
@@ -341,28 +365,24 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
     const int len = min(BCH, sp.len - c * BCH);
     const bool last = it + 1 == n_chunks, update = kRev ? !last || a.d_initial_state != nullptr : !last;
     tc::tmem_st_wait();
-    cp_wait<0>();
-    tc::fence_proxy_async_smem();
     tc::tc_fence_before_sync();
     __syncthreads();
     if (warp < 2 && tc::elect_one()) {  // S K^T; forward: its terms over two accumulators; reverse: beside dO^T P
       tc::tc_fence_after_sync();
-      constexpr uint32_t id = tc::idesc_f16(128, 64, 1, 1, false, false), id_p = tc::idesc_f16(128, 64, 1, 1, true, true);
+      constexpr uint32_t id = tc::idesc_f16(128, 64, 1, 1, false, false);
       const uint64_t kd = tc::smem_desc_sw128(st + SC_K, 16, 1024);
       auto step = [&](int i, int ks, uint32_t acc, bool more) {
         tc::mma_ts(tm + acc, tm + TS_S + (ks >> 2) * TS_HALF + 32 * i + 8 * (ks & 3), kd + (uint64_t)(((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), id, more ? 1u : 0u);
       };
-      if (kRev && warp == 1) {
-        const uint64_t od = tc::smem_desc_sw128(st + RV_DO, 8192, 1024), pd = tc::smem_desc_sw128(st + RV_PI, 8192, 1024);
+      if constexpr (kRev) {
+        if (warp == 1) {
+          if (it == 0) issue_do_p(c);  // later ones: behind the increment of the chunk before
+        } else {
 #pragma unroll
-        for (int i = 0; i < 3; ++i)
+          for (int i = 0; i < 3; ++i)
 #pragma unroll
-          for (int ks = 0; ks < 4; ++ks) tc::mma_ss(tm + TS_ACC2, od + ks * (2048 >> 4), pd + (i * IMG + ks * 2048 >> 4), id_p, (i | ks) != 0 ? 1u : 0u);
-      } else if (kRev) {
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int ks = 0; ks < 8; ++ks) step(i, ks, TS_ACC, (i | ks) != 0);
+            for (int ks = 0; ks < 8; ++ks) step(i, ks, TS_ACC, (i | ks) != 0);
+        }
       } else {
 #pragma unroll
         for (int ks = 0; ks < 8; ++ks) step(warp == 0 ? 0 : 2, ks, warp == 0 ? TS_ACC : TS_ACC2, ks != 0);
@@ -372,15 +392,10 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
       tc::mma_commit(&bars[0]);
     }
     __syncwarp();
-    if (!last) load(kRev ? c - 1 : c + 1);
-    if (tid < BCH) {
-      const float eb = __expf(bs[tid]), be = bs[BCH + tid], D = gate_between(bs, BCH - 1, tid);
-      fac[tid] = kRev ? make_float4(D, tid < len ? a.scale * eb : 0.f, -be * eb, 0.f) : make_float4(be, eb, D, 0.f);
-    }
-    {
-      float* dst = (kRev ? ws.e : ws.m0) + rec * STATE_FLOATS;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) store_unit(dst, 4 * grp + i, row, S + 8 * i);
+    if (tid >= SC_T - BCH) {
+      const int i = tid - (SC_T - BCH);
+      const float eb = __expf(bs[i]), be = bs[BCH + i], D = gate_between(bs, BCH - 1, i);
+      fac[i] = kRev ? make_float4(D, i < len ? a.scale * eb : 0.f, -be * eb, 0.f) : make_float4(be, eb, D, 0.f);
     }
     const float decay = __expf(bs[BCH - 1]);
     float rows[16];  // V^T or dO^T
@@ -396,6 +411,8 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
         store_terms<16>(lanes + TS_DO + 8 * grp, 32, x);
       }
     }
+    float* s_rec = (kRev ? ws.e : ws.m0) + rec * STATE_FLOATS;
+    if (!last) load(c_next);
     tc::mbar_wait_warp(&bars[0], phase, abort_flag);
     tc::tc_fence_after_sync();
     {
@@ -426,8 +443,10 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
         const uint64_t r = td + (uint64_t)((warp == 0 ? R[0][j] : R[1][j]) * (IMG >> 4));
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
-          if constexpr (kRev) tc::mma_ts(acc, l + 8 * ks, r + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), (j | ks) != 0 ? 1u : 0u);
-          else  // tokens from 16 ks on: T is lower triangular
+          // T is lower triangular: tokens up to 16 kr + 15 (the first step, kr = 3, covers all), or from 16 ks on
+          const int kr = 3 - ks;
+          if constexpr (kRev) tc::mma_ts(acc, l + 8 * kr, r + kr * (2048 >> 4), tc::idesc_f16(128, 16 * (kr + 1), 1, 1, false, true), (j | ks) != 0 ? 1u : 0u);
+          else
             tc::mma_ts(acc + 16 * ks, l + 8 * ks, r + ks * ((2048 + 32) >> 4), tc::idesc_f16(128, 64 - 16 * ks, 1, 1, false, false), (j | ks) != 0 ? 1u : 0u);
         }
       }
@@ -442,6 +461,8 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
       }
     }
     __syncwarp();
+    store_unit(s_rec, 4 * grp, row, S);
+    store_unit(s_rec, 4 * grp + 1, row, S + 8);
     tc::mbar_wait_warp(&bars[1], phase, abort_flag);
     tc::tc_fence_after_sync();
     {
@@ -453,29 +474,34 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
 #pragma unroll
       for (int i = 0; i < 16; ++i) y[i] = __uint_as_float(u[i]) + __uint_as_float(w[i]);
       float* dst = (kRev ? ws.u : ws.vn) + rec * VEC_FLOATS;
+      if (update) {
+        float f[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) f[i] = y[i] * fac[16 * grp + i].z;
+        store_terms<16>(lanes + TS_X + 8 * grp, 32, f);
+        tc::tmem_st_wait();
+        if (!last) landed(c_next, it + 1);
+        tc::tc_fence_before_sync();
+        __syncthreads();
+        if (warp < 2 && tc::elect_one()) {  // the increment: X K, this issuer's half of d_k
+          tc::tc_fence_after_sync();
+          const uint64_t kd = tc::smem_desc_sw128(st + SC_K + warp * 8192, 8192, 1024);
+#pragma unroll
+          for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int ks = 0; ks < 4; ++ks)
+              tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_X + 32 * i + 8 * ks, kd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), kRev || (i | ks) != 0 ? 1u : 0u);
+          tc::mma_commit(&bars[2]);
+          if (kRev && warp == 1 && !last) issue_do_p(c_next);
+        }
+        __syncwarp();
+      }
       store_unit(dst, 2 * grp, row, y);
       store_unit(dst, 2 * grp + 1, row, y + 8);
-      if (update) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) y[i] *= fac[16 * grp + i].z;
-        store_terms<16>(lanes + TS_X + 8 * grp, 32, y);
-      }
+      store_unit(s_rec, 4 * grp + 2, row, S + 16);
+      store_unit(s_rec, 4 * grp + 3, row, S + 24);
     }
     if (!update) break;
-    tc::tmem_st_wait();
-    tc::tc_fence_before_sync();
-    __syncthreads();
-    if (warp < 2 && tc::elect_one()) {  // the increment: X K, this issuer's half of d_k
-      tc::tc_fence_after_sync();
-      const uint64_t kd = tc::smem_desc_sw128(st + SC_K + warp * 8192, 8192, 1024);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_X + 32 * i + 8 * ks, kd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), kRev || (i | ks) != 0 ? 1u : 0u);
-      tc::mma_commit(&bars[2]);
-    }
-    __syncwarp();
     tc::mbar_wait_warp(&bars[2], phase, abort_flag);
     tc::tc_fence_after_sync();
     {
