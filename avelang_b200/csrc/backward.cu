@@ -239,10 +239,10 @@ __global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a,
 // accumulators (or column halves) of their own.  The chain is bound by these hand-offs, about 1 k cycles each beside 0.8 k of
 // MMAs.  Tiles of the next chunk land meanwhile.  Two sequences of 4096 tokens, 32 value heads: 0.34 ms; on warp-level MMAs, whose
 // pipe was full (504 and 756 of them a warp and chunk, 16 cycles each), the two scans took 0.27 + 0.38 ms one after the other.
-constexpr int SC_T = 512;
+constexpr int SC_T = 512, SC_LT = 256;  // the first SC_LT threads copy tiles; warps 10 and 13 issue the first products
 constexpr int SC_K = 0, FW_V = 16384, FW_TI = 32768, FW_SC = FW_TI + 3 * IMG, FW_STAGE = FW_SC + 1024;
 constexpr int RV_Q = 16384, RV_DO = 32768, RV_TI = 49152, RV_PI = RV_TI + 3 * IMG, RV_SC = RV_PI + 3 * IMG, RV_STAGE = RV_SC + 1024;
-constexpr int SC_FAC = 2 * RV_STAGE, SC_BAR = SC_FAC + BCH * 16, SC_SMEM = SC_BAR + 64;
+constexpr int SC_FAC = 2 * RV_STAGE, SC_BAR = SC_FAC + 2 * BCH * 16, SC_SMEM = SC_BAR + 64;
 static_assert(FW_STAGE % 1024 == 0 && RV_STAGE % 1024 == 0 && SC_SMEM <= 227 * 1024, "shared memory");
 // tensor-memory columns.  State terms: [half of d_k][term][32]; the increment's accumulator takes the first 64 of each half.
 constexpr uint32_t TS_S = 0, TS_HALF = 96, TS_X = 192, TS_DO = 288, TS_ACC = 384, TS_ACC2 = 448;
@@ -286,25 +286,27 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
   const __nv_bfloat16* vp = bf(a.v) + sp.b * a.v_stride_b + (int64_t)sp.t0 * a.v_stride_t + h * a.v_stride_h;
   const __nv_bfloat16* dop = bf(a.d_o) + sp.b * a.do_stride_b + (int64_t)sp.t0 * a.do_stride_t + h * a.do_stride_h;
   const uint32_t sb = tc::smem_u32(smem);
-  float4* fac = reinterpret_cast<float4*>(smem + SC_FAC);       // per token: forward beta, e^b, D; reverse D, S e^b, -beta e^b
+  float4* fac_of = reinterpret_cast<float4*>(smem + SC_FAC);    // per stage and token: forward beta, e^b, D; reverse D, S e^b, -beta e^b
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SC_BAR);  // one per product, then one per stage
   volatile uint32_t* abort_flag = reinterpret_cast<uint32_t*>(smem + SC_BAR + 48);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + SC_BAR + 56);
   auto load = [&](int c) {
     const uint32_t st = sb + (c & 1) * STAGE;
     const int len = min(BCH, sp.len - c * BCH);
-    auto tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
-      load_tile<BCH, 8, SC_T>(st + at, src + (int64_t)c * BCH * stride, stride, len, tid);
-      load_tile<BCH, 8, SC_T>(st + at + 8192, src + (int64_t)c * BCH * stride + 64, stride, len, tid);
-    };
-    tiles(SC_K, kp, a.k_stride_t);
-    if constexpr (kRev) {
-      tiles(RV_Q, qp, a.q_stride_t);
-      tiles(RV_DO, dop, a.do_stride_t);
-    } else {
-      tiles(FW_V, vp, a.v_stride_t);
+    if (tid < SC_LT) {
+      auto tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
+        load_tile<BCH, 8, SC_LT>(st + at, src + (int64_t)c * BCH * stride, stride, len, tid);
+        load_tile<BCH, 8, SC_LT>(st + at + 8192, src + (int64_t)c * BCH * stride + 64, stride, len, tid);
+      };
+      tiles(SC_K, kp, a.k_stride_t);
+      if constexpr (kRev) {
+        tiles(RV_Q, qp, a.q_stride_t);
+        tiles(RV_DO, dop, a.do_stride_t);
+      } else {
+        tiles(FW_V, vp, a.v_stride_t);
+      }
+      cp_commit();
     }
-    cp_commit();
     if (tid == 0) {
       const uint8_t* rec = ws.prep + ((slot0 + c) * a.Hv + h) * PREP_BYTES;
       uint8_t* dst = smem + (c & 1) * STAGE;
@@ -338,6 +340,12 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
     cp_wait<0>();
     tc::fence_proxy_async_smem();
     tc::mbar_wait_warp(&bars[3 + (c & 1)], n_th >> 1 & 1, abort_flag);  // the stage's (n_th / 2)-th use
+    if (tid >= SC_T - BCH) {
+      const int i = tid - (SC_T - BCH);
+      const float* bs = reinterpret_cast<const float*>(smem + (c & 1) * STAGE + SC);
+      const float eb = __expf(bs[i]), be = bs[BCH + i], D = gate_between(bs, BCH - 1, i);
+      fac_of[(c & 1) * BCH + i] = kRev ? make_float4(D, i < sp.len - c * BCH ? a.scale * eb : 0.f, -be * eb, 0.f) : make_float4(be, eb, D, 0.f);
+    }
   };
   tc::tc_fence_before_sync();
   __syncthreads();
@@ -345,7 +353,8 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
   landed(kRev ? n_chunks - 1 : 0, 0);
   const uint32_t tm = *tmem_slot, lanes = tm + ((uint32_t)(32 * quarter) << 16);
   const uint32_t s_cols = lanes + TS_S + (grp >> 1) * TS_HALF;
-  auto issue_do_p = [&](int c) {  // dO^T P of a chunk
+  auto issue_do_p = [&](int c) {  // dO^T P of a chunk, ahead of it
+    tc::tc_fence_after_sync();
     const uint32_t st = sb + (c & 1) * STAGE;
     const uint64_t od = tc::smem_desc_sw128(st + RV_DO, 8192, 1024), pd = tc::smem_desc_sw128(st + RV_PI, 8192, 1024);
 #pragma unroll
@@ -353,8 +362,14 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks)
         tc::mma_ss(tm + TS_ACC2, od + ks * (2048 >> 4), pd + ((i * IMG + ks * 2048) >> 4), tc::idesc_f16(128, 64, 1, 1, true, true), (i | ks) != 0 ? 1u : 0u);
+    tc::mma_commit(&bars[0]);  // counts for the chunk's first product
   };
   store_terms<32>(s_cols + 16 * (grp & 1), 32, S);
+  if constexpr (kRev) {
+    __syncthreads();
+    if (warp == 10 && tc::elect_one()) issue_do_p(n_chunks - 1);
+    __syncwarp();
+  }
 #pragma unroll 1
   for (int it = 0; it < n_chunks; ++it) {
     const int c = kRev ? n_chunks - 1 - it : it, c_next = kRev ? c - 1 : c + 1;
@@ -362,12 +377,12 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
     uint8_t* stage = smem + (c & 1) * STAGE;
     const float* bs = reinterpret_cast<const float*>(stage + SC);
     const int64_t rec = (slot0 + c) * a.Hv + h;
-    const int len = min(BCH, sp.len - c * BCH);
+    const float4* fac = fac_of + (c & 1) * BCH;
     const bool last = it + 1 == n_chunks, update = kRev ? !last || a.d_initial_state != nullptr : !last;
     tc::tmem_st_wait();
     tc::tc_fence_before_sync();
     __syncthreads();
-    if (warp < 2 && tc::elect_one()) {  // S K^T; forward: its terms over two accumulators; reverse: beside dO^T P
+    if ((warp == 13 || (!kRev && warp == 10)) && tc::elect_one()) {  // S K^T; forward: its terms over two accumulators
       tc::tc_fence_after_sync();
       constexpr uint32_t id = tc::idesc_f16(128, 64, 1, 1, false, false);
       const uint64_t kd = tc::smem_desc_sw128(st + SC_K, 16, 1024);
@@ -375,34 +390,25 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
         tc::mma_ts(tm + acc, tm + TS_S + (ks >> 2) * TS_HALF + 32 * i + 8 * (ks & 3), kd + (uint64_t)(((ks >> 2) * 8192 + (ks & 3) * 32) >> 4), id, more ? 1u : 0u);
       };
       if constexpr (kRev) {
-        if (warp == 1) {
-          if (it == 0) issue_do_p(c);  // later ones: behind the increment of the chunk before
-        } else {
 #pragma unroll
-          for (int i = 0; i < 3; ++i)
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks) step(i, ks, TS_ACC, (i | ks) != 0);
-        }
+          for (int ks = 0; ks < 8; ++ks) step(i, ks, TS_ACC, (i | ks) != 0);
       } else {
+        const bool first = warp == 13;
 #pragma unroll
-        for (int ks = 0; ks < 8; ++ks) step(warp == 0 ? 0 : 2, ks, warp == 0 ? TS_ACC : TS_ACC2, ks != 0);
+        for (int ks = 0; ks < 8; ++ks) step(first ? 0 : 2, ks, first ? TS_ACC : TS_ACC2, ks != 0);
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) step(1, warp == 0 ? ks : 4 + ks, warp == 0 ? TS_ACC : TS_ACC2, true);
+        for (int ks = 0; ks < 4; ++ks) step(1, first ? ks : 4 + ks, first ? TS_ACC : TS_ACC2, true);
       }
       tc::mma_commit(&bars[0]);
     }
     __syncwarp();
-    if (tid >= SC_T - BCH) {
-      const int i = tid - (SC_T - BCH);
-      const float eb = __expf(bs[i]), be = bs[BCH + i], D = gate_between(bs, BCH - 1, i);
-      fac[i] = kRev ? make_float4(D, i < len ? a.scale * eb : 0.f, -be * eb, 0.f) : make_float4(be, eb, D, 0.f);
-    }
     const float decay = __expf(bs[BCH - 1]);
     float rows[16];  // V^T or dO^T
 #pragma unroll
     for (int i = 0; i < 16; ++i)
       rows[i] = __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(stage + ROWS + (row >> 6) * 8192 + piece<128>(16 * grp + i, (row & 63) >> 3) + 2 * (row & 7)));
-    __syncthreads();  // the factors are complete
     if constexpr (kRev) {
       if (update) {
         float x[16];
@@ -492,8 +498,8 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
             for (int ks = 0; ks < 4; ++ks)
               tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_X + 32 * i + 8 * ks, kd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), kRev || (i | ks) != 0 ? 1u : 0u);
           tc::mma_commit(&bars[2]);
-          if (kRev && warp == 1 && !last) issue_do_p(c_next);
         }
+        if (kRev && !last && warp == 10 && tc::elect_one()) issue_do_p(c_next);
         __syncwarp();
       }
       store_unit(dst, 2 * grp, row, y);
