@@ -22,7 +22,7 @@
 // and enter as they are; every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with
 // one fp32 operand is three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which
 // the gradient of the gate needs, because it is a difference of large sums.
-// Two sequences of 4096 tokens, 32 value heads: 0.90 ms (prep 0.12, scans 0.34, gradients 0.44) against 22.1 ms for the
+// Two sequences of 4096 tokens, 32 value heads: 0.86 ms (prep 0.12, scans 0.30, gradients 0.44) against 22.1 ms for the
 // token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
 #include "blockalg.cuh"
 #include "common.cuh"
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a,
 //     x = S K^T,   y = (f(x, V or dO P)) T or T^T,   S += (f(y)) K   (reverse: and the scaled dO)^T Q,
 // with a pass of all threads over the result behind each; the product of the pass's tile is issued by two threads, into
 // accumulators (or column halves) of their own.  The chain is bound by these hand-offs, about 1 k cycles each beside 0.8 k of
-// MMAs.  Tiles of the next chunk land meanwhile.  Two sequences of 4096 tokens, 32 value heads: 0.34 ms; on warp-level MMAs, whose
+// MMAs.  Tiles of the next chunk land meanwhile.  Two sequences of 4096 tokens, 32 value heads: 0.30 ms; on warp-level MMAs, whose
 // pipe was full (504 and 756 of them a warp and chunk, 16 cycles each), the two scans took 0.27 + 0.38 ms one after the other.
 constexpr int SC_T = 512, SC_LT = 256;  // the first SC_LT threads copy tiles; warps 10 and 13 issue the first products
 constexpr int SC_K = 0, FW_V = 16384, FW_TI = 32768, FW_SC = FW_TI + 3 * IMG, FW_STAGE = FW_SC + 1024;
@@ -499,7 +499,6 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
               tc::mma_ts(tm + TS_S + warp * TS_HALF, tm + TS_X + 32 * i + 8 * ks, kd + ks * (2048 >> 4), tc::idesc_f16(128, 64, 1, 1, false, true), kRev || (i | ks) != 0 ? 1u : 0u);
           tc::mma_commit(&bars[2]);
         }
-        if (kRev && !last && warp == 10 && tc::elect_one()) issue_do_p(c_next);
         __syncwarp();
       }
       store_unit(dst, 2 * grp, row, y);
@@ -510,6 +509,8 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
     if (!update) break;
     tc::mbar_wait_warp(&bars[2], phase, abort_flag);
     tc::tc_fence_after_sync();
+    if (kRev && !last && warp == 10 && tc::elect_one()) issue_do_p(c_next);  // the tensor core idles during the pass below
+    __syncwarp();
     {
       uint32_t d[32];
       tc::tmem_ld32(s_cols + 32 * (grp & 1), d);
