@@ -22,12 +22,11 @@
 // and enter as they are; every fp32 operand enters as three bf16 terms x = h + m + l (24 significant bits), so a product with
 // one fp32 operand is three MMAs and one with two is six (h h, h m, m h, h l, l h, m m): the accuracy of fp32 arithmetic, which
 // the gradient of the gate needs, because it is a difference of large sums.
-// Two sequences of 4096 tokens, 32 value heads: 0.86 ms (prep 0.12, scans 0.30, gradients 0.44) against 22.1 ms for the
+// Two sequences of 4096 tokens, 32 value heads: 0.82 ms (prep 0.08, scans 0.30, gradients 0.44) against 22.1 ms for the
 // token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
-#include "blockalg.cuh"
 #include "common.cuh"
 #include "tc.cuh"
-#include "warpmma.cuh"
+#include "wyblocks.cuh"
 
 namespace ave {
 namespace {
@@ -69,32 +68,57 @@ __device__ __forceinline__ float gate_between(const float* sc, int i, int j) {
 }
 
 // ---------------------------------------------------------------------------------------------- T, P and b of every chunk
+// One CTA of eight warps per (chunk, key head, up to two of its value heads); the Gram products are shared by the two.  Bound by the
+// latency of its dependent steps, like the forward pass's preparation, whose block algebra it uses: warps 0..3 form the
+// fragments of A, 4..7 those of P, then a warp per row of blocks forms T.  P and T leave through the same shared memory, by
+// bulk copies.  4096 (chunk, value head) units: 78 us against 116 for one head per CTA with the block products spread
+// over CTA barriers.
 constexpr int PREP_T = 256;
-constexpr int PR_K = 0, PR_Q = 16384, PR_A = 32768, PR_D = PR_A + 10 * BLK_FLOATS * 4, PR_E = PR_D + 4 * BLK_FLOATS * 4,
-              PR_SC = PR_E + 10 * BLK_FLOATS * 4, PR_SMEM = PR_SC + SC_BYTES;
+constexpr int PR_K = 0, PR_Q = 16384, PR_OUT = 0, PR_OUT_HEAD = 3 * IMG, PR_F = 2 * PR_OUT_HEAD, PR_F_HEAD = 16384, PR_SC = PR_F + 2 * PR_F_HEAD,
+              PR_SMEM = PR_SC + 2 * SC_BYTES;
+static_assert(PR_Q + 16384 <= PR_F && WY_BYTES <= PR_F_HEAD, "shared memory");
 
-__global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
+template <int R>
+__device__ __forceinline__ void bwd_prep_row(uint8_t* smem, int hh, int lane, bool lead, uint8_t* rec) {
+  float T[R + 1][2][4];
+  wy_row<R>(T, smem + PR_F + hh * PR_F_HEAD, lane);
+  if (lead) tc::bulk_wait_read<0>();  // P has been read out of the head's region
+  head_sync(hh);
+  const uint32_t region = tc::smem_u32(smem + PR_OUT + hh * PR_OUT_HEAD);
+#pragma unroll
+  for (int c = 0; c <= R; ++c) {
+    uint32_t h[4], m[4], l[4];
+    split_acc(T[c][0], T[c][1], h, m, l);
+    const uint32_t at = region + at_a<128>(16 * R, 2 * c, lane);
+    stsm4(at, h[0], h[1], h[2], h[3]);
+    stsm4(at + IMG, m[0], m[1], m[2], m[3]);
+    stsm4(at + 2 * IMG, l[0], l[1], l[2], l[3]);
+  }
+  tc::fence_proxy_async_smem();
+  head_sync(hh);
+  if (lead) {
+    tc::bulk_store(rec, smem + PR_OUT + hh * PR_OUT_HEAD, PR_OUT_HEAD);
+    tc::bulk_commit();
+    tc::bulk_wait_read<0>();  // shared memory must stay intact until the copy has read it
+  }
+}
+
+__global__ void __launch_bounds__(PREP_T, 2) bwd_prep_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  float* Ab = reinterpret_cast<float*>(smem + PR_A);
-  float* Di = reinterpret_cast<float*>(smem + PR_D);
-  float* Eb = reinterpret_cast<float*>(smem + PR_E);
-  float* E2b = Eb + 6 * BLK_FLOATS;
-  float* E3b = E2b + 3 * BLK_FLOATS;
-  float* bs = reinterpret_cast<float*>(smem + PR_SC);
-  float* betas = bs + BCH;
-  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const BwdChunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
-  const int hk = h / (a.Hv / a.Hk);
-  uint8_t* rec = ws.prep + ((int64_t)blockIdx.x * a.Hv + h) * PREP_BYTES;
+  const int r = a.Hv / a.Hk, pairs = (r + 1) / 2;
+  const int hk = blockIdx.y / pairs, h0 = hk * r + 2 * (blockIdx.y % pairs), nh = min(2, hk * r + r - h0);
+  uint8_t* rec0 = ws.prep + ((int64_t)blockIdx.x * a.Hv + h0) * PREP_BYTES;
   const uint32_t sb = tc::smem_u32(smem);
   load_tile<BCH, 16, PREP_T>(sb + PR_K, bf(a.k) + c.b * a.k_stride_b + (int64_t)c.t0 * a.k_stride_t + hk * a.k_stride_h, a.k_stride_t, c.len, tid);
   load_tile<BCH, 16, PREP_T>(sb + PR_Q, bf(a.q) + c.b * a.q_stride_b + (int64_t)c.t0 * a.q_stride_t + hk * a.q_stride_h, a.q_stride_t, c.len, tid);
   cp_commit();
-  if (warp == 0) {  // inclusive scan of the gates; beyond the end of the sequence b stays and beta is 0
+  if (warp < nh) {  // inclusive scan of the gates; beyond the end of the sequence b stays and beta is 0
     // b reaches hundreds while e^{b_i - b_j} of near tokens matters: it is summed in double and kept as two floats, so that
     // the differences are as exact as the gates themselves
-    const int64_t off = c.b * a.g_stride_b + (int64_t)c.t0 * a.g_stride_t + h;
+    const int64_t off = c.b * a.g_stride_b + (int64_t)c.t0 * a.g_stride_t + h0 + warp;
     double v0 = lane < c.len ? a.g[off + lane * a.g_stride_t] : 0.f, v1 = lane + 32 < c.len ? a.g[off + (lane + 32) * a.g_stride_t] : 0.f;
     const float be0 = lane < c.len ? a.beta[off + lane * a.g_stride_t] : 0.f, be1 = lane + 32 < c.len ? a.beta[off + (lane + 32) * a.g_stride_t] : 0.f;
 #pragma unroll
@@ -103,130 +127,110 @@ __global__ void __launch_bounds__(PREP_T) bwd_prep_kernel(const AveGdnBwdArgs a,
       if (lane >= o) { v0 += t0; v1 += t1; }
     }
     v1 += __shfl_sync(0xffffffffu, v0, 31);
-    float* sc = reinterpret_cast<float*>(rec + PREP_SC);
-    const float h0 = (float)v0, h1 = (float)v1, l0 = (float)(v0 - h0), l1 = (float)(v1 - h1);
-    bs[lane] = sc[lane] = h0; bs[lane + 32] = sc[lane + 32] = h1;
-    betas[lane] = sc[BCH + lane] = be0; betas[lane + 32] = sc[BCH + lane + 32] = be1;
+    float* sc = reinterpret_cast<float*>(rec0 + warp * PREP_BYTES + PREP_SC);
+    float* bs = reinterpret_cast<float*>(smem + PR_SC + warp * SC_BYTES);
+    const float x0 = (float)v0, x1 = (float)v1, l0 = (float)(v0 - x0), l1 = (float)(v1 - x1);
+    bs[lane] = sc[lane] = x0; bs[lane + 32] = sc[lane + 32] = x1;
+    bs[BCH + lane] = sc[BCH + lane] = be0; bs[BCH + lane + 32] = sc[BCH + lane + 32] = be1;
     bs[2 * BCH + lane] = sc[2 * BCH + lane] = l0; bs[2 * BCH + lane + 32] = sc[2 * BCH + lane + 32] = l1;
   }
   cp_wait<0>();
   __syncthreads();
-  {  // warps 0..3: rows 16m.. of K K^T -> A;  warps 4..7: rows 16m.. of Q K^T -> P.  Blocks above the diagonal are skipped.
-    const int m = warp & 3, g = lane >> 2, t = lane & 3;
-    const bool is_p = warp >= 4;
-    float acc[8][4];
+  // Warps 0..3: rows of K block m against the blocks from it on (A transposed); warps 4..7: rows of Q block m against the K blocks
+  // up to it.  acc[2 x] and acc[2 x + 1]: the x-th of those blocks.
+  const int m = warp & 3;
+  const bool is_p = warp >= 4;
+  const int first = is_p ? 0 : m, count = is_p ? m + 1 : 4 - m;
+  float acc[8][4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) zero(acc[i]);
+  for (int i = 0; i < 8; ++i) zero(acc[i]);
 #pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      uint32_t af[4];
-      ldsm4(af, sb + (is_p ? PR_Q : PR_K) + at_a<256>(16 * m, 2 * ks, lane));
+  for (int ks = 0; ks < 8; ++ks) {
+    uint32_t af[4];
+    ldsm4(af, sb + (is_p ? PR_Q : PR_K) + at_a<256>(16 * m, 2 * ks, lane));
 #pragma unroll
-      for (int np = 0; np < 4; ++np) {
-        if (np > m) break;
-        uint32_t b[4];
-        ldsm4(b, sb + PR_K + at_b<256>(16 * np, 2 * ks, lane));
-        mma_bf16(acc[2 * np], af, b[0], b[1]);
-        mma_bf16(acc[2 * np + 1], af, b[2], b[3]);
-      }
+    for (int x = 0; x < 4; ++x) {
+      if (x >= count) break;
+      uint32_t b[4];
+      ldsm4(b, sb + PR_K + at_b<256>(16 * (first + x), 2 * ks, lane));
+      mma_bf16(acc[2 * x], af, b[0], b[1]);
+      mma_bf16(acc[2 * x + 1], af, b[2], b[3]);
     }
+  }
+  __syncthreads();  // K and Q make room for P, later T; their blocks above the diagonal are zero
+  for (int e = tid; e < nh * 3 * 6 * 32; e += PREP_T) {
+    const int blk = (e >> 5) % 6, brow = (blk < 3 ? 0 : blk < 5 ? 1 : 2), bcol = (blk < 3 ? blk + 1 : blk < 5 ? blk - 1 : 3);
+    *reinterpret_cast<uint4*>(smem + PR_OUT + ((e >> 5) / 6) * IMG + piece<128>(16 * brow + ((e & 31) >> 1), 2 * bcol + (e & 1))) = make_uint4(0u, 0u, 0u, 0u);
+  }
+#pragma unroll 1
+  for (int hh = 0; hh < nh; ++hh) {
+    const float* bs = reinterpret_cast<const float*>(smem + PR_SC + hh * SC_BYTES);
+    uint8_t* frag = smem + PR_F + hh * PR_F_HEAD;
+    if (!is_p) {  // element (row j = 16 m + g + 8 hf, column i = 16 s + 8 nt + 2 t + e) of the transposed A
+      float* ad = reinterpret_cast<float*>(frag + WY_DIAG) + m * 16 * AD_LD;
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
+      for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int i = 16 * m + g + 8 * half, j = 8 * nt + 2 * t;
-        const float x0 = gate_between(bs, i, j) * acc[nt][2 * half], x1 = gate_between(bs, i, j + 1) * acc[nt][2 * half + 1];
-        if (is_p) {
-          uint32_t ph, pm, pl;
-          split3(make_float2(i >= j ? x0 : 0.f, i > j ? x1 : 0.f), ph, pm, pl);
-          uint8_t* dst = rec + PREP_P + piece<128>(i, nt) + 4 * t;
-          *reinterpret_cast<uint32_t*>(dst) = ph;
-          *reinterpret_cast<uint32_t*>(dst + IMG) = pm;
-          *reinterpret_cast<uint32_t*>(dst + 2 * IMG) = pl;
-        } else if (nt <= 2 * m + 1) {
-          const float be = betas[i];
-          *reinterpret_cast<float2*>(Ab + tri(m, nt >> 1) * BLK_FLOATS + (i & 15) * BLK_LD + (j & 15)) =
-              make_float2(i > j ? be * x0 : 0.f, i > j + 1 ? be * x1 : 0.f);
+        for (int e = 0; e < 4; ++e) {
+          const int j = g + 8 * (e >> 1), i = 8 * nt + 2 * t + (e & 1);
+          const float x = bs[BCH + 16 * m + i] * gate_between(bs, 16 * m + i, 16 * m + j) * acc[nt][e];
+          ad[i * AD_LD + j] = i > j ? x : 0.f;
         }
+#pragma unroll
+      for (int x = 1; x < 4; ++x) {
+        if (x >= count) break;
+        const int s = m + x;
+        uint32_t ah[4], am[4], al[4];
+#pragma unroll
+        for (int idx = 0; idx < 4; ++idx) {  // (column tile idx & 1, row half idx >> 1)
+          const int i = 16 * s + 8 * (idx & 1) + 2 * t, j = 16 * m + g + 8 * (idx >> 1);
+          const float* p = acc[2 * x + (idx & 1)] + 2 * (idx >> 1);
+          split3(make_float2(bs[BCH + i] * gate_between(bs, i, j) * p[0], bs[BCH + i + 1] * gate_between(bs, i + 1, j) * p[1]), ah[idx], am[idx], al[idx]);
+        }
+        uint4* f = reinterpret_cast<uint4*>(frag + (s * (s - 1) / 2 + m) * WY_BLOCK) + lane;
+        f[0] = make_uint4(ah[0], ah[1], ah[2], ah[3]);
+        f[32] = make_uint4(am[0], am[1], am[2], am[3]);
+        f[64] = make_uint4(al[0], al[1], al[2], al[3]);
+      }
+    } else {  // element (row i = 16 m + g + 8 hf, column j = 16 x + 8 nt + 2 t + e) of P
+      const uint32_t region = sb + PR_OUT + hh * PR_OUT_HEAD;
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        if (x >= count) break;
+        uint32_t ph[4], pm[4], pl[4];
+#pragma unroll
+        for (int idx = 0; idx < 4; ++idx) {  // (column tile idx >> 1, row half idx & 1)
+          const int i = 16 * m + g + 8 * (idx & 1), j = 16 * x + 8 * (idx >> 1) + 2 * t;
+          const float* p = acc[2 * x + (idx >> 1)] + 2 * (idx & 1);
+          const float y0 = gate_between(bs, i, j) * p[0], y1 = gate_between(bs, i, j + 1) * p[1];
+          split3(make_float2(i >= j ? y0 : 0.f, i > j ? y1 : 0.f), ph[idx], pm[idx], pl[idx]);
+        }
+        const uint32_t at = region + at_a<128>(16 * m, 2 * x, lane);
+        stsm4(at, ph[0], ph[1], ph[2], ph[3]);
+        stsm4(at + IMG, pm[0], pm[1], pm[2], pm[3]);
+        stsm4(at + 2 * IMG, pl[0], pl[1], pl[2], pl[3]);
       }
     }
   }
+  tc::fence_proxy_async_smem();
   __syncthreads();
-  // T = (I + A)^-1 by 16x16 blocks, as in the forward pass: D = blockdiag(I + A_rr), E = D^-1 (A - A_D),
-  // T = (I - E + E^2 - E^3) D^-1
-  if (tid < 64) {
-    const int r = tid >> 4, k = tid & 15;
-    const float* Arr = Ab + tri(r, r) * BLK_FLOATS;
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float s0 = (i == k) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-      for (int j = 0; j < i; ++j) {
-        const float av = Arr[i * BLK_LD + j];
-        if (j & 1) s1 = fmaf(-av, x[j], s1); else s0 = fmaf(-av, x[j], s0);
-      }
-      x[i] = s0 + s1;
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) Di[r * BLK_FLOATS + i * BLK_LD + k] = x[i];
+  const int hh = warp >> 2;
+  if (hh >= nh) return;
+  uint8_t* rec = rec0 + hh * PREP_BYTES;
+  // rows cost R + 1 units of work and warps 0 and 4, 1 and 5, ... share a scheduler: opposite orders
+  const int row = hh == 0 ? 3 - warp : warp - 4;
+  const bool lead = row == 0 && lane == 0;  // in the warp with the least work
+  if (lead) {
+    tc::bulk_store(rec + PREP_P, smem + PR_OUT + hh * PR_OUT_HEAD, PR_OUT_HEAD);
+    tc::bulk_commit();
   }
-  __syncthreads();
-  constexpr int RR[6] = {1, 2, 2, 3, 3, 3}, CC[6] = {0, 0, 1, 0, 1, 2};
-  auto Eblk = [&](int r, int cc) { return Eb + (tri(r, cc) - r) * BLK_FLOATS; };
-  auto plain = [](const float* L) { return [L](int row, int col) { return L[row * BLK_LD + col]; }; };
-  if (warp < 6) {
-    const int r = RR[warp], cc = CC[warp];
-    float acc[2][4] = {};
-    block_mma(acc, plain(Di + r * BLK_FLOATS), Ab + tri(r, cc) * BLK_FLOATS, lane);
-    block_store(Eblk(r, cc), acc, lane);
-  }
-  __syncthreads();
-  if (warp < 3) {  // E^2: (2,0), (3,1), (3,0)
-    float acc[2][4] = {};
-    if (warp == 0) block_mma(acc, plain(Eblk(2, 1)), Eblk(1, 0), lane);
-    else if (warp == 1) block_mma(acc, plain(Eblk(3, 2)), Eblk(2, 1), lane);
-    else { block_mma(acc, plain(Eblk(3, 1)), Eblk(1, 0), lane); block_mma(acc, plain(Eblk(3, 2)), Eblk(2, 0), lane); }
-    block_store(E2b + warp * BLK_FLOATS, acc, lane);
-  }
-  __syncthreads();
-  if (warp == 0) {
-    float acc[2][4] = {};
-    block_mma(acc, plain(Eblk(3, 2)), E2b, lane);
-    block_store(E3b, acc, lane);
-  }
-  __syncthreads();
-  if (warp < 6) {
-    const int r = RR[warp], cc = CC[warp];
-    const float* e1 = Eblk(r, cc);
-    const float* e2 = (r - cc >= 2) ? E2b + ((r == 2) ? 0 : (cc == 1 ? 1 : 2)) * BLK_FLOATS : nullptr;
-    const float* e3 = (r - cc == 3) ? E3b : nullptr;
-    float acc[2][4] = {};
-    block_mma(acc, [&](int row, int col) {
-      float v = -e1[row * BLK_LD + col];
-      if (e2 != nullptr) v += e2[row * BLK_LD + col];
-      if (e3 != nullptr) v -= e3[row * BLK_LD + col];
-      return v;
-    }, Di + cc * BLK_FLOATS, lane);
-    block_store(Ab + tri(r, cc) * BLK_FLOATS, acc, lane);
-  }
-  __syncthreads();
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const int i = (tid >> 3) + 32 * it, rb = i >> 4, pc = tid & 7, cb = pc >> 1;
-    uint32_t th[4] = {}, tm[4] = {}, tl[4] = {};
-    if (cb <= rb) {
-      const float* src = ((rb == cb) ? Di + rb * BLK_FLOATS : Ab + tri(rb, cb) * BLK_FLOATS) + (i & 15) * BLK_LD + (pc & 1) * 8;
-#pragma unroll
-      for (int w = 0; w < 4; ++w) {
-        const int j = 8 * pc + 2 * w;
-        split3(make_float2(j <= i ? src[2 * w] : 0.f, j + 1 <= i ? src[2 * w + 1] : 0.f), th[w], tm[w], tl[w]);
-      }
-    }
-    uint8_t* dst = rec + piece<128>(i, pc);
-    *reinterpret_cast<uint4*>(dst) = make_uint4(th[0], th[1], th[2], th[3]);
-    *reinterpret_cast<uint4*>(dst + IMG) = make_uint4(tm[0], tm[1], tm[2], tm[3]);
-    *reinterpret_cast<uint4*>(dst + 2 * IMG) = make_uint4(tl[0], tl[1], tl[2], tl[3]);
+  if (row >= 2) wy_invert(smem + PR_F + hh * PR_F_HEAD, row & 1, lane);
+  head_sync(hh);
+  switch (row) {
+    case 3: bwd_prep_row<3>(smem, hh, lane, lead, rec); break;
+    case 2: bwd_prep_row<2>(smem, hh, lane, lead, rec); break;
+    case 1: bwd_prep_row<1>(smem, hh, lane, lead, rec); break;
+    default: bwd_prep_row<0>(smem, hh, lane, lead, rec); break;
   }
 }
 
@@ -970,7 +974,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
   }
   const BwdScratch ws = scratch_layout(a, nullptr);
   const unsigned slots = (unsigned)backward_slots(a);
-  bwd_prep_kernel<<<dim3(slots, (unsigned)a.Hv), PREP_T, PR_SMEM, stream>>>(a, ws);
+  bwd_prep_kernel<<<dim3(slots, (unsigned)(a.Hk * ((a.Hv / a.Hk + 1) / 2))), PREP_T, PR_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
   bwd_scans_kernel<<<2 * units, SC_T, SC_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());

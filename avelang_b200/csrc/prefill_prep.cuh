@@ -17,17 +17,15 @@
 // 132 k (chunk, head) units of a packed batch: 3.02 ms, 7.8 k warp instructions a unit; the form that took one head per CTA
 // through tcgen05 products and CTA barriers needed 12.4 k instructions and 3.84 ms.
 #pragma once
-#include "warpmma.cuh"
+#include "wyblocks.cuh"
 
 namespace ave {
 namespace {
 
 constexpr int PREP_THREADS = 256;
-constexpr int AD_LD = 20;                                     // row pitch (floats) of a 16x16 fp32 block
 constexpr int PP_K = 0, PP_R = 16384;                         // K tile; per head a 16 KB region (head 0's holds the Q tile first)
 constexpr int PP_F = PP_R + 2 * 16384, PP_F_HEAD = 16384;     // per head: off-diagonal A fragments | diagonal blocks; later W^T
-constexpr int PF_AD = 6 * 3 * 512;
-static_assert(PF_AD + 4 * 16 * AD_LD * 4 <= PP_F_HEAD, "fragments and diagonal blocks must fit");
+static_assert(WY_BYTES <= PP_F_HEAD, "fragments and diagonal blocks must fit");
 constexpr int PP_V = PP_F + 2 * PP_F_HEAD;                    // per head: vectors of 64 floats
 enum { V_B, V_BETA, V_RA, V_RP, V_DA, V_DP, V_FW, V_W1, V_W2, V_W3, V_COUNT };
 constexpr int PP_N = PP_V + 2 * V_COUNT * C * 4;              // row norms of k | q
@@ -39,55 +37,15 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 constexpr float LOG2E = 1.4426950408889634f;
-// the four warps of one head
-__device__ __forceinline__ void head_sync(int hh) {
-  __syncwarp();
-  asm volatile("bar.sync %0, 128;" ::"r"(1 + hh) : "memory");
-}
-
 // Row R of 16x16 blocks of T, and with it rows / columns 16 R .. 16 R + 15 of Tu and W^T.  Called by one warp per R; the
 // four warps of the head meet at named barriers.  `lead` (one lane of the head's warps) moves finished tiles out.
 template <int R>
 __device__ __forceinline__ void prep_row(uint8_t* smem, int hh, int lane, bool lead, const PrepOut& out, int64_t rec) {
   const int g = lane >> 2, t = lane & 3;
   uint8_t* frag = smem + PP_F + hh * PP_F_HEAD;
-  const float* Dt = reinterpret_cast<const float*>(frag + PF_AD);  // D_c transposed: [c][column][row]
   const float* vec = reinterpret_cast<const float*>(smem + PP_V) + hh * V_COUNT * C;
   float T[R + 1][2][4];
-#pragma unroll
-  for (int nt = 0; nt < 2; ++nt)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) T[R][nt][e] = Dt[R * 16 * AD_LD + (8 * nt + 2 * t + (e & 1)) * AD_LD + g + 8 * (e >> 1)];
-  if constexpr (R > 0) {
-    uint32_t th[R][4], tm[R][4], tl[R][4];  // T_rs as left operand, [R - s]
-    split_acc(T[R][0], T[R][1], th[0], tm[0], tl[0]);
-#pragma unroll
-    for (int c = R - 1; c >= 0; --c) {
-      float y[2][4];
-      zero(y[0]); zero(y[1]);
-#pragma unroll
-      for (int s = c + 1; s <= R; ++s) {
-        const uint4* f = reinterpret_cast<const uint4*>(frag + (s * (s - 1) / 2 + c) * 1536) + lane;
-        const uint4 ah = f[0], am = f[32], al = f[64];
-        mma6(y[0], th[R - s], tm[R - s], tl[R - s], ah.x, ah.y, am.x, am.y, al.x, al.y);
-        mma6(y[1], th[R - s], tm[R - s], tl[R - s], ah.z, ah.w, am.z, am.w, al.z, al.w);
-      }
-      uint32_t yh[4], ym[4], yl[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) { y[0][e] = -y[0][e]; y[1][e] = -y[1][e]; }
-      split_acc(y[0], y[1], yh, ym, yl);
-      zero(T[c][0]); zero(T[c][1]);
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-        const float* d = Dt + c * 16 * AD_LD + (8 * nt + g) * AD_LD + 2 * t;
-        uint32_t dh[2], dm[2], dl[2];
-        split3(*reinterpret_cast<const float2*>(d), dh[0], dm[0], dl[0]);
-        split3(*reinterpret_cast<const float2*>(d + 8), dh[1], dm[1], dl[1]);
-        mma6(T[c][nt], yh, ym, yl, dh[0], dh[1], dm[0], dm[1], dl[0], dl[1]);
-      }
-      if (c > 0) split_acc(T[c][0], T[c][1], th[R - c], tm[R - c], tl[R - c]);
-    }
-  }
+  wy_row<R>(T, frag, lane);
   if (lead) tc::bulk_wait_read<0>();  // the P tiles have been read out of the head's region
   head_sync(hh);                      // and nobody needs the fragments any more
   const uint32_t region = tc::smem_u32(smem + PP_R + hh * 16384);
@@ -286,7 +244,7 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
     const float* vec = vecs + hh * V_COUNT * C;
     const float* bs = vec + V_B * C;
     if (!is_p) {  // element (row j = 16 m + g + 8 hf, column i = 16 s + 8 nt + 2 t + e) of the transposed A
-      float* ad = reinterpret_cast<float*>(smem + PP_F + hh * PP_F_HEAD + PF_AD) + m * 16 * AD_LD;
+      float* ad = reinterpret_cast<float*>(smem + PP_F + hh * PP_F_HEAD + WY_DIAG) + m * 16 * AD_LD;
 #pragma unroll
       for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
@@ -307,7 +265,7 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
         };
         gate(0, acc[2 * x], r0, w0); gate(1, acc[2 * x + 1], r1, w0);
         gate(2, acc[2 * x] + 2, r0, w1); gate(3, acc[2 * x + 1] + 2, r1, w1);
-        uint4* f = reinterpret_cast<uint4*>(smem + PP_F + hh * PP_F_HEAD + (s * (s - 1) / 2 + m) * 1536) + lane;
+        uint4* f = reinterpret_cast<uint4*>(smem + PP_F + hh * PP_F_HEAD + (s * (s - 1) / 2 + m) * WY_BLOCK) + lane;
         f[0] = make_uint4(ah[0], ah[1], ah[2], ah[3]);
         f[32] = make_uint4(am[0], am[1], am[2], am[3]);
         f[64] = make_uint4(al[0], al[1], al[2], al[3]);
@@ -362,28 +320,7 @@ chunk_prep_kernel(const AveGdnArgs a, const int32_t* chunk_start, PrepOut out, c
     tc::bulk_store(out.p_lo + rec * (C * C), smem + PP_R + hh * 16384 + REC_P, REC_P);
     tc::bulk_commit();
   }
-  if (row >= 2) {  // column k of (I + A_bb)^-1, one lane each: 4 blocks x 16 columns over two warps
-    const int b = 2 * (row & 1) + (lane >> 4), k = lane & 15;
-    float* ad = reinterpret_cast<float*>(smem + PP_F + hh * PP_F_HEAD + PF_AD) + b * 16 * AD_LD;
-    float x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      float s0 = (i == k) ? 1.f : 0.f, s1 = 0.f;
-#pragma unroll
-      for (int j4 = 0; j4 < (i + 3) / 4; ++j4) {
-        const float4 av = *reinterpret_cast<const float4*>(ad + i * AD_LD + 4 * j4);
-        s0 = fmaf(-av.x, x[4 * j4], s0);
-        if (4 * j4 + 1 < i) s1 = fmaf(-av.y, x[4 * j4 + 1], s1);
-        if (4 * j4 + 2 < i) s0 = fmaf(-av.z, x[4 * j4 + 2], s0);
-        if (4 * j4 + 3 < i) s1 = fmaf(-av.w, x[4 * j4 + 3], s1);
-      }
-      x[i] = s0 + s1;
-    }
-    __syncwarp();  // every lane has read the block: its inverse, transposed, takes its place
-#pragma unroll
-    for (int i4 = 0; i4 < 4; ++i4)
-      *reinterpret_cast<float4*>(ad + k * AD_LD + 4 * i4) = make_float4(x[4 * i4], x[4 * i4 + 1], x[4 * i4 + 2], x[4 * i4 + 3]);
-  }
+  if (row >= 2) wy_invert(smem + PP_F + hh * PP_F_HEAD, row & 1, lane);
   head_sync(hh);
   switch (row) {
     case 3: prep_row<3>(smem, hh, lane, lead, out, rec); break;
