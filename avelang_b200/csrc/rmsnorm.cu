@@ -14,14 +14,14 @@ struct NormBatch {
 // D = 128: a half-warp per row, eight elements (16 bytes of bf16, 32 of fp32) per lane, two rows in flight per
 // half-warp; D = 64: same with four elements per lane.  Rows are (batch, token, head) in that order.  Like the other
 // streaming helpers the kernel is bound by instruction issue before HBM, so the math runs on packed fp32 pairs and
-// tensors whose rows are evenly spaced (`flat`) skip the per-row index divisions.
-template <int D, typename XT>
+// tensors whose rows are evenly spaced (kFlat) skip the per-row index divisions.
+template <int D, typename XT, bool kFlat>
 __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const __nv_bfloat16* z,
                                                             const float* w, __nv_bfloat16* y,
                                                             int64_t rows, int heads, int64_t xs_t, int64_t xs_h,
                                                             int64_t zs_t, int64_t zs_h, int64_t ys_t, int64_t ys_h,
                                                             float eps, int gate_first, const void* const* peers,
-                                                            int n_peers, int64_t peer_off, NormBatch nb, int flat) {
+                                                            int n_peers, int64_t peer_off, NormBatch nb) {
   pdl_wait();
   constexpr int E = D / 16;  // elements per lane: 8 or 4
   constexpr int P = E / 2;   // pairs per lane
@@ -35,9 +35,14 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const _
   // (batch, token, head) of the next row, kept by stepping: divisions in the loop would cost a quarter of its instructions
   // (131072 tokens x 32 rows of fp32, gate and result bf16: 0.83 -> 0.75 ms, 0.90 of the copy rate).
   // 32-bit: the launcher checks the row count.
-  const uint32_t tokens = ((uint32_t)nb.rows_per_batch + (uint32_t)heads - 1u) / (uint32_t)heads, step = (uint32_t)n_hw, dt = step / (uint32_t)heads, dh = step - dt * (uint32_t)heads;
-  uint32_t t = (uint32_t)hw_global / (uint32_t)heads, h = (uint32_t)hw_global - t * (uint32_t)heads, b = t / tokens;
-  t -= b * tokens;
+  [[maybe_unused]] uint32_t tokens = 1, dt = 0, dh = 0, t = 0, h = 0, b = 0;
+  if constexpr (!kFlat) {
+    const uint32_t hd = (uint32_t)heads, step = (uint32_t)n_hw, r = (uint32_t)hw_global;
+    tokens = ((uint32_t)nb.rows_per_batch + hd - 1u) / hd;
+    dt = step / hd; dh = step - dt * hd;
+    t = r / hd; h = r - t * hd;
+    b = t / tokens; t -= b * tokens;
+  }
   for (int64_t r0 = hw_global; r0 < rows; r0 += U * n_hw) {
     float2 xv[U][P], zv[U][P];
     int64_t yoff[U];
@@ -53,7 +58,7 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const _
         continue;
       }
       int64_t xo, zo;
-      if (flat) {  // row r sits r head-strides from the base in all three tensors
+      if constexpr (kFlat) {  // row r sits r head-strides from the base in all three tensors
         xo = r * xs_h; zo = r * zs_h; yoff[u] = r * ys_h + sub * E;
       } else {
         xo = (int64_t)b * nb.xs_b + (int64_t)t * xs_t + h * xs_h;
@@ -135,15 +140,15 @@ static int launch_norm_t(const XT* x, const AveGdnNormArgs& a, cudaStream_t stre
   const int gate_first = (a.flags & AVE_GDN_FLAG_GATE_FIRST) ? 1 : 0;
   // evenly spaced rows: token stride = heads x head stride in every tensor, and batch rows follow one another the same way
   const bool even = a.x_stride_t == a.heads * a.x_stride_h && a.z_stride_t == a.heads * a.z_stride_h && a.y_stride_t == a.heads * a.y_stride_h;
-  const int flat = (even && (batches == 1 || (xs_b == a.rows * a.x_stride_h && zs_b == a.rows * a.z_stride_h && ys_b == a.rows * a.y_stride_h))) ? 1 : 0;
+  const bool flat = even && (batches == 1 || (xs_b == a.rows * a.x_stride_h && zs_b == a.rows * a.z_stride_h && ys_b == a.rows * a.y_stride_h));
   const __nv_bfloat16* z = reinterpret_cast<const __nv_bfloat16*>(a.z);
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y);
   if (a.d == 128) {
-    AVE_CUDA_TRY(launch_after(gated_rmsnorm_kernel<128, XT>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb, flat));
+    AVE_CUDA_TRY(launch_after(flat ? gated_rmsnorm_kernel<128, XT, true> : gated_rmsnorm_kernel<128, XT, false>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
+                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb));
   } else if (a.d == 64) {
-    AVE_CUDA_TRY(launch_after(gated_rmsnorm_kernel<64, XT>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, (const void* const*)nullptr, 0, (int64_t)0, nb, flat));
+    AVE_CUDA_TRY(launch_after(flat ? gated_rmsnorm_kernel<64, XT, true> : gated_rmsnorm_kernel<64, XT, false>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
+                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, (const void* const*)nullptr, 0, (int64_t)0, nb));
   } else {
     return AVE_GDN_UNSUPPORTED;
   }
