@@ -747,10 +747,12 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
 // different bank groups), and a thread takes two rows, four columns and half of the contraction, which needs six 16-byte
 // reads for 32 multiply-adds.  Fifteen steps: 44 us, 55 us with one row a thread, scalar reads
 // and F staged through registers.
-constexpr int COMBINE_COLS = 8, COMBINE_PITCH = 132;
-constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 1) * COMBINE_COLS * 4;  // (a gap of one row between the halves)
+constexpr int COMBINE_PITCH = 132;
+constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 4) * 8 * 4;  // (a gap of one row between the shares of the contraction)
 constexpr int COMBINE_STAGES = 3;
 constexpr size_t COMBINE_SMEM = COMBINE_STAGES * (size_t)COMBINE_F + 2 * COMBINE_CUR;
+// COLS columns a CTA: 8, or 4 while that still is one wave (its step is shorter, but F passes through twice as many SMs).
+template <int COLS>
 __global__ void __launch_bounds__(256)
 part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -769,12 +771,13 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   if (active == 2 && a.final_state == nullptr) return;  // nothing to produce
   const int chains = 2 * plan.parts - 1;
   auto tile_of = [&](int chain) { return carry + (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D); };
+  constexpr int SPLIT = 16 / COLS, SHARE = D / SPLIT;  // threads that share a contraction, and its length for each
   auto cur_at = [&](int b, int k, int j) -> float& {
-    return reinterpret_cast<float*>(smem_raw + COMBINE_STAGES * COMBINE_F + b * COMBINE_CUR)[(k + (k >> 6)) * COMBINE_COLS + j];
+    return reinterpret_cast<float*>(smem_raw + COMBINE_STAGES * COMBINE_F + b * COMBINE_CUR)[(k + k / SHARE) * COLS + j];
   };
   const uint32_t sb = tc::smem_u32(smem_raw);
-  // this thread: rows k and k + 64, columns j0 .. j0 + 3, contraction indices d0 .. d0 + 63
-  const int dh = tid & 1, j0 = ((tid >> 1) & 1) * 4, k = tid >> 2, d0 = dh * 64;
+  // this thread: rows k and k + 64, columns j0 .. j0 + 3, contraction indices d0 .. d0 + SHARE - 1
+  const int dh = tid & 1, j0 = COLS == 8 ? ((tid >> 1) & 1) * 4 : 0, k = tid >> 2, d0 = (tid & (SPLIT - 1)) * SHARE;
   auto fetch = [&](int p) {  // F_p into buffer p % 3
     if (p >= active) { cp_commit(); return; }
     const float* F = tile_of(2 * p);
@@ -786,12 +789,12 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
     cp_commit();
   };
   auto psi_of = [&](int p) {
-    return p < active ? *reinterpret_cast<const float4*>(tile_of(2 * p - 1) + (int64_t)(k + 64 * dh) * D + cb * COMBINE_COLS + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return p < active ? *reinterpret_cast<const float4*>(tile_of(2 * p - 1) + (int64_t)(k + 64 * dh) * D + cb * COLS + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   fetch(1);
   fetch(2);
   float4 psi_next = psi_of(1);
-  for (int e = tid; e < D * COMBINE_COLS; e += 256) cur_at(0, e / COMBINE_COLS, e % COMBINE_COLS) = tile_of(0)[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS];
+  for (int e = tid; e < D * COLS; e += 256) cur_at(0, e / COLS, e % COLS) = tile_of(0)[(e / COLS) * D + cb * COLS + e % COLS];
   int b = 0;
   for (int p = 1; p < active; ++p) {
     cp_wait<1>();
@@ -802,7 +805,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
     const float* F0 = reinterpret_cast<const float*>(smem_raw + (p % COMBINE_STAGES) * COMBINE_F) + k * COMBINE_PITCH + d0;
     float2 x[2][2] = {};
 #pragma unroll 4
-    for (int d = 0; d < 64; d += 4) {
+    for (int d = 0; d < SHARE; d += 4) {
       const float4 f0 = *reinterpret_cast<const float4*>(F0 + d), f1 = *reinterpret_cast<const float4*>(F0 + 64 * COMBINE_PITCH + d);
       const float fa[4] = {f0.x, f0.y, f0.z, f0.w}, fb[4] = {f1.x, f1.y, f1.z, f1.w};
 #pragma unroll
@@ -814,25 +817,26 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
         x[1][1] = __ffma2_rn(make_float2(fb[e], fb[e]), make_float2(c4.z, c4.w), x[1][1]);
       }
     }
-    {  // the two halves of the contraction meet; each of the two threads finishes one of the two rows
+    {  // the shares of the contraction meet; an even and an odd thread finish one of the two rows each
       float v[8] = {x[0][0].x, x[0][0].y, x[0][1].x, x[0][1].y, x[1][0].x, x[1][0].y, x[1][1].x, x[1][1].y};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float mine = dh ? v[4 + i] : v[i], other = dh ? v[i] : v[4 + i];
         v[i] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
+        if (SPLIT == 4) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2);
       }
-      *reinterpret_cast<float4*>(&cur_at(b ^ 1, k + 64 * dh, j0)) = make_float4(v[0] + psi.x, v[1] + psi.y, v[2] + psi.z, v[3] + psi.w);
+      if (SPLIT == 2 || (tid & 2) == 0) *reinterpret_cast<float4*>(&cur_at(b ^ 1, k + 64 * dh, j0)) = make_float4(v[0] + psi.x, v[1] + psi.y, v[2] + psi.z, v[3] + psi.w);
     }
     b ^= 1;
     if (p + 1 == active) break;
     __syncthreads();
-    if (tid < 128) {  // operand image of M0(p+1): B[row = d_v][k] = M0[k][d_v]; a 16-byte piece of hi and of lo
-      const int k8 = tid >> 3, v = tid & 7;
+    if (tid < 16 * COLS) {  // operand image of M0(p+1): B[row = d_v][k] = M0[k][d_v]; a 16-byte piece of hi and of lo
+      const int k8 = tid / COLS, v = tid % COLS;
       uint32_t hi[4], lo[4];
 #pragma unroll
       for (int w = 0; w < 4; ++w) split_pair(make_float2(cur_at(b, 8 * k8 + 2 * w, v), cur_at(b, 8 * k8 + 2 * w + 1, v)), hi[w], lo[w]);
       uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1) + p) * a.Hv + h) * (int64_t)PACK_BYTES;
-      const uint32_t off = kmajor_piece_off(cb * COMBINE_COLS + v, k8);
+      const uint32_t off = kmajor_piece_off(cb * COLS + v, k8);
       *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
       *reinterpret_cast<uint4*>(img + D * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
     }
@@ -840,7 +844,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   __syncthreads();
   if (a.final_state != nullptr) {
     float* dst = a.final_state + ((int64_t)slot * a.Hv + h) * (int64_t)(D * D);
-    for (int e = tid; e < D * COMBINE_COLS; e += 256) dst[(e / COMBINE_COLS) * D + cb * COMBINE_COLS + e % COMBINE_COLS] = cur_at(b, e / COMBINE_COLS, e % COMBINE_COLS);
+    for (int e = tid; e < D * COLS; e += 256) dst[(e / COLS) * D + cb * COLS + e % COLS] = cur_at(b, e / COLS, e % COLS);
   }
 }
 
@@ -1289,7 +1293,8 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIN_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
     dev.attr_set = true;
   }
   if (chunk_start != nullptr) {
@@ -1313,16 +1318,18 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   auto finish_parts = [&](cudaStream_t s, cudaStream_t side_stream, cudaEvent_t scanned, cudaEvent_t combined) -> int {
     if (L.parts <= 1) return AVE_GDN_OK;
     plan.r0 = 0; plan.rn = 1 << 24;
-    const dim3 cgrid(D / COMBINE_COLS, (unsigned)a.Hv, (unsigned)a.n_seqs);
+    const int cols = (int64_t)a.n_seqs * a.Hv * (D / 4) <= NUM_SMS ? 4 : 8;
+    const auto combine = cols == 4 ? part_combine_kernel<4> : part_combine_kernel<8>;
+    const dim3 cgrid((unsigned)(D / cols), (unsigned)a.Hv, (unsigned)a.n_seqs);
     const bool beside = L.parts == 2 && side_stream != nullptr;
     if (beside) {
       AVE_CUDA_TRY(cudaEventRecord(scanned, s));
       AVE_CUDA_TRY(cudaStreamWaitEvent(side_stream, scanned, 0));
-      part_combine_kernel<<<cgrid, 256, COMBINE_SMEM, side_stream>>>(a, chunk_start, carry, m0_pack, plan);
+      combine<<<cgrid, 256, COMBINE_SMEM, side_stream>>>(a, chunk_start, carry, m0_pack, plan);
       AVE_CUDA_TRY(cudaGetLastError());
       AVE_CUDA_TRY(cudaEventRecord(combined, side_stream));
     } else {
-      part_combine_kernel<<<cgrid, 256, COMBINE_SMEM, s>>>(a, chunk_start, carry, m0_pack, plan);
+      combine<<<cgrid, 256, COMBINE_SMEM, s>>>(a, chunk_start, carry, m0_pack, plan);
       AVE_CUDA_TRY(cudaGetLastError());
     }
     int part_len = 0;  // the longest of the later parts
