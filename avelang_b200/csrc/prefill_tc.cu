@@ -752,6 +752,8 @@ constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 4) * 8 * 4; 
 constexpr int COMBINE_STAGES = 3;
 constexpr size_t COMBINE_SMEM = COMBINE_STAGES * (size_t)COMBINE_F + 2 * COMBINE_CUR;
 // COLS columns a CTA: 8, or 4 while that still is one wave (its step is shorter, but F passes through twice as many SMs).
+// Bound by shared-memory reads and the issue of the copies, 2 us a step: 15 steps for 4 heads 30 us (42 us when the lanes of a
+// quarter warp read one row at four offsets of 128 bytes, 8 wavefronts a load).
 template <int COLS>
 __global__ void __launch_bounds__(256)
 part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
@@ -777,7 +779,8 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   };
   const uint32_t sb = tc::smem_u32(smem_raw);
   // this thread: rows k and k + 64, columns j0 .. j0 + 3, contraction indices d0 .. d0 + SHARE - 1
-  const int dh = tid & 1, j0 = COLS == 8 ? ((tid >> 1) & 1) * 4 : 0, k = tid >> 2, d0 = (tid & (SPLIT - 1)) * SHARE;
+  // (the lanes of a quarter warp, which a 16-byte shared load serves together, read eight rows, so no two meet in a bank)
+  const int part = (tid >> 3) & 3, dh = part & 1, j0 = COLS == 8 ? (part >> 1) * 4 : 0, k = (tid >> 5) * 8 + (tid & 7), d0 = (part & (SPLIT - 1)) * SHARE;
   auto fetch = [&](int p) {  // F_p into buffer p % 3
     if (p >= active) { cp_commit(); return; }
     const float* F = tile_of(2 * p);
@@ -817,15 +820,15 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
         x[1][1] = __ffma2_rn(make_float2(fb[e], fb[e]), make_float2(c4.z, c4.w), x[1][1]);
       }
     }
-    {  // the shares of the contraction meet; an even and an odd thread finish one of the two rows each
+    {  // the shares of the contraction meet; two of them finish one of the two rows each
       float v[8] = {x[0][0].x, x[0][0].y, x[0][1].x, x[0][1].y, x[1][0].x, x[1][0].y, x[1][1].x, x[1][1].y};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float mine = dh ? v[4 + i] : v[i], other = dh ? v[i] : v[4 + i];
-        v[i] = mine + __shfl_xor_sync(0xffffffffu, other, 1);
-        if (SPLIT == 4) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 2);
+        v[i] = mine + __shfl_xor_sync(0xffffffffu, other, 8);
+        if (SPLIT == 4) v[i] += __shfl_xor_sync(0xffffffffu, v[i], 16);
       }
-      if (SPLIT == 2 || (tid & 2) == 0) *reinterpret_cast<float4*>(&cur_at(b ^ 1, k + 64 * dh, j0)) = make_float4(v[0] + psi.x, v[1] + psi.y, v[2] + psi.z, v[3] + psi.w);
+      if (SPLIT == 2 || part < 2) *reinterpret_cast<float4*>(&cur_at(b ^ 1, k + 64 * dh, j0)) = make_float4(v[0] + psi.x, v[1] + psi.y, v[2] + psi.z, v[3] + psi.w);
     }
     b ^= 1;
     if (p + 1 == active) break;
