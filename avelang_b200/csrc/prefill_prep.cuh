@@ -41,7 +41,7 @@ constexpr float LOG2E = 1.4426950408889634f;
 // four warps of the head meet at named barriers.  `lead` (one lane of the head's warps) moves finished tiles out.
 template <int R>
 __device__ __forceinline__ void prep_row(uint8_t* smem, int hh, int lane, bool lead, const PrepOut& out, int64_t rec) {
-  const int g = lane >> 2, t = lane & 3;
+  const int t = lane & 3;
   uint8_t* frag = smem + PP_F + hh * PP_F_HEAD;
   const float* vec = reinterpret_cast<const float*>(smem + PP_V) + hh * V_COUNT * C;
   float T[R + 1][2][4];
