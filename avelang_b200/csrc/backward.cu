@@ -25,6 +25,7 @@
 // Two sequences of 4096 tokens, 32 value heads: 0.82 ms (prep 0.08, scans 0.30, gradients 0.44) against 22.1 ms for the
 // token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
 #include "common.cuh"
+#include "recslots.cuh"
 #include "tc.cuh"
 #include "wyblocks.cuh"
 
@@ -41,31 +42,6 @@ struct BwdScratch {
   float *m0, *e;   // [slots][Hv][d_k / 8][d_v][8]: H = M0^T and E^T of every chunk
   float *vn, *u;   // [slots][Hv][64 tokens / 8][d_v][8]: Vn^T and Ut^T
 };
-
-// Chunk j of sequence n has record slot floor(first token of n / 64) + n + j: unique, needs no table, and the sequence of a
-// slot is found by bisection because the first slots of the sequences increase strictly.
-struct BwdChunk { int n, b, t0, len; bool ok; };
-__device__ __forceinline__ int64_t first_slot(const AveGdnBwdArgs& a, int n) {
-  return (a.cu_seqlens ? (int64_t)a.cu_seqlens[n] : (int64_t)n * a.T) / BCH + n;
-}
-__device__ __forceinline__ BwdChunk chunk_of_slot(const AveGdnBwdArgs& a, int64_t slot) {
-  int lo = 0, hi = a.n_seqs;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first_slot(a, mid) <= slot) lo = mid; else hi = mid;
-  }
-  BwdChunk c{lo, 0, 0, 0, false};
-  const SeqSpan sp = seq_span(a.cu_seqlens, lo, a.T, nullptr);
-  const int64_t j = slot - first_slot(a, lo);
-  if (!sp.ok || j < 0 || j * BCH >= sp.len) return c;
-  c.b = sp.b; c.t0 = sp.t0 + (int)j * BCH; c.len = min(BCH, sp.len - (int)j * BCH); c.ok = true;
-  return c;
-}
-
-// e^{b_i - b_j} for i >= j (at most 1 elsewhere); sc: b[64] | beta[64] | low part of b[64]
-__device__ __forceinline__ float gate_between(const float* sc, int i, int j) {
-  return __expf(fminf((sc[i] - sc[j]) + (sc[2 * BCH + i] - sc[2 * BCH + j]), 0.f));
-}
 
 // ---------------------------------------------------------------------------------------------- T, P and b of every chunk
 // One CTA of eight warps per (chunk, key head, up to two of its value heads); the Gram products are shared by the two.  Bound by the
@@ -106,7 +82,8 @@ __device__ __forceinline__ void bwd_prep_row(uint8_t* smem, int hh, int lane, bo
 __global__ void __launch_bounds__(PREP_T, 2) bwd_prep_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const BwdChunk c = chunk_of_slot(a, blockIdx.x);
+  if (!offsets_ok(a, blockIdx.x == 0 && blockIdx.y == 0)) return;
+  const SlotChunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
   const int r = a.Hv / a.Hk, pairs = (r + 1) / 2;
   const int hk = blockIdx.y / pairs, h0 = hk * r + 2 * (blockIdx.y % pairs), nh = min(2, hk * r + r - h0);
@@ -274,8 +251,7 @@ template <bool kRev>
 __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratch& ws, int unit, uint8_t* smem) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = unit / a.Hv, h = unit % a.Hv, hk = h / (a.Hv / a.Hk);
-  const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
-  if (!sp.ok) return;
+  const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   const int64_t tile = (int64_t)unit * STATE_FLOATS;
   if (sp.len == 0) {  // empty sequence: the state gradient passes through
     if (kRev && a.d_initial_state != nullptr)
@@ -539,6 +515,7 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
 }
 __global__ void __launch_bounds__(SC_T, 1) bwd_scans_kernel(const AveGdnBwdArgs a, BwdScratch ws) {
   extern __shared__ __align__(1024) uint8_t smem[];
+  if (!offsets_ok(a, false)) return;
   const int units = a.n_seqs * a.Hv;
   if ((int)blockIdx.x < units) bwd_scan<true>(a, ws, blockIdx.x, smem);
   else bwd_scan<false>(a, ws, blockIdx.x - units, smem);
@@ -609,7 +586,7 @@ __device__ __forceinline__ float lane_sums(float (&v)[16], int lane) {
 // Per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16: eight tokens
 // of one d_k column per lane.
 template <bool kSum>
-__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const BwdChunk& c, int head, int tok0, int dk, const float (&x)[8]) {
+__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const SlotChunk& c, int head, int tok0, int dk, const float (&x)[8]) {
   const int64_t row = (int64_t)c.b * a.T + c.t0 + tok0;
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
@@ -631,6 +608,7 @@ template <bool kSum>
 __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs a, BwdScratch ws, int64_t slots) {
   extern __shared__ __align__(1024) uint8_t smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  if (!offsets_ok(a, false)) return;
   const int r = a.Hv / a.Hk;
   const uint32_t sb = tc::smem_u32(smem);
   float2* red = reinterpret_cast<float2*>(smem + GR_RED);  // [4 d_k quarters][64 tokens]: q.dq + k.row - k.col, k.row
@@ -658,7 +636,7 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
   for (int64_t p = blockIdx.x; p < pairs; p += gridDim.x) {
     const int64_t slot = p / a.Hk;
     const int hk = (int)(p % a.Hk);
-    const BwdChunk c = chunk_of_slot(a, slot);
+    const SlotChunk c = chunk_of_slot(a, slot);
     if (!c.ok) continue;
     const int64_t row0 = (int64_t)c.b * a.T + c.t0;
     auto load_half_tiles = [&](int at, const __nv_bfloat16* src, int64_t stride) {  // [64 tokens][128] as two tiles of 128-byte rows
@@ -933,10 +911,8 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
   if (warp == 1) tc::tmem_dealloc(*tmem_slot, 512);
 }
 
-int64_t backward_slots(const AveGdnBwdArgs& a) { return (int64_t)a.B * a.T / BCH + a.n_seqs + 1; }
-
 BwdScratch scratch_layout(const AveGdnBwdArgs& a, size_t* total) {
-  const size_t recs = (size_t)backward_slots(a) * a.Hv;
+  const size_t recs = (size_t)record_slots(a) * a.Hv;
   uint8_t* p = reinterpret_cast<uint8_t*>(a.workspace);
   BwdScratch ws;
   size_t off = 0;
@@ -973,7 +949,7 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
     attr_set_dev[dev] = true;  // repeating the calls from another thread is harmless
   }
   const BwdScratch ws = scratch_layout(a, nullptr);
-  const unsigned slots = (unsigned)backward_slots(a);
+  const unsigned slots = (unsigned)record_slots(a);
   bwd_prep_kernel<<<dim3(slots, (unsigned)(a.Hk * ((a.Hv / a.Hk + 1) / 2))), PREP_T, PR_SMEM, stream>>>(a, ws);
   AVE_CUDA_TRY(cudaGetLastError());
   bwd_scans_kernel<<<2 * units, SC_T, SC_SMEM, stream>>>(a, ws);

@@ -13,6 +13,7 @@
 // four heads.
 #include "blockalg.cuh"
 #include "common.cuh"
+#include "recslots.cuh"
 #include "tc.cuh"
 #include "warpmma.cuh"
 
@@ -24,40 +25,6 @@ constexpr int CH = 64, DH = 64, IMG = CH * CH * 2, THREADS = 256;
 constexpr int R_T = 0, R_P = 3 * IMG, R_PHI = 6 * IMG, R_GAM = R_PHI + DH * DH * 4, R_H = R_GAM + DH * DH * 4, R_SC = R_H + DH * DH * 4,
               SC_FLOATS = 5 * CH, REC_BYTES = R_SC + SC_FLOATS * 4;  // T h m l | P h m l | Phi | Gam | H | b, beta, low b, |q|^-1, |k|^-1
 
-// Chunk j of sequence n has record slot floor(first token of n / 64) + n + j (unique, no table needed).
-struct Chunk { int n, b, t0, len; bool ok; };
-__device__ __forceinline__ int64_t first_slot(const AveGdnArgs& a, int n) {
-  return (a.cu_seqlens ? (int64_t)a.cu_seqlens[n] : (int64_t)n * a.T) / CH + n;
-}
-__device__ __forceinline__ Chunk chunk_of_slot(const AveGdnArgs& a, int64_t slot) {
-  int lo = 0, hi = a.n_seqs;
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (first_slot(a, mid) <= slot) lo = mid; else hi = mid;
-  }
-  Chunk c{lo, 0, 0, 0, false};
-  const SeqSpan sp = seq_span(a.cu_seqlens, lo, a.T, nullptr);
-  const int64_t j = slot - first_slot(a, lo);
-  if (!sp.ok || j < 0 || j * CH >= sp.len) return c;
-  c.b = sp.b; c.t0 = sp.t0 + (int)j * CH; c.len = min(CH, sp.len - (int)j * CH); c.ok = true;
-  return c;
-}
-// A packed batch whose offsets are not monotone inside [0, T] is skipped as a whole.  Called by the whole CTA.
-__device__ __forceinline__ bool offsets_ok(const AveGdnArgs& a, bool flag) {
-  if (a.cu_seqlens == nullptr) return true;
-  int bad = 0;
-  for (int n = threadIdx.x; n < a.n_seqs; n += blockDim.x) {
-    const int x = a.cu_seqlens[n], y = a.cu_seqlens[n + 1];
-    bad |= (x < 0 || y < x || y > a.T) ? 1 : 0;
-  }
-  bad = __syncthreads_or(bad);
-  if (bad && flag && threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_BAD_SEQLEN);
-  return bad == 0;
-}
-// e^{b_i - b_j} for i >= j (at most 1 elsewhere); b is kept as two floats so that near differences are exact
-__device__ __forceinline__ float gate_between(const float* sc, int i, int j) {
-  return __expf(fminf((sc[i] - sc[j]) + (sc[2 * CH + i] - sc[2 * CH + j]), 0.f));
-}
 // three bf16 terms of a pair -> images at `at`, `at` + IMG, `at` + 2 IMG
 __device__ __forceinline__ void put3(uint8_t* at, float x, float y) {
   uint32_t h, m, l;
@@ -102,7 +69,7 @@ __global__ void __launch_bounds__(THREADS) d64_prep_kernel(const AveGdnArgs a, u
   pdl_trigger();
   pdl_wait();
   if (!offsets_ok(a, blockIdx.x == 0 && h == 0)) return;
-  const Chunk c = chunk_of_slot(a, blockIdx.x);
+  const SlotChunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
   const int hk = h / (a.Hv / a.Hk);
   uint8_t* rec = recs + ((int64_t)blockIdx.x * a.Hv + h) * REC_BYTES;
@@ -416,7 +383,7 @@ __global__ void __launch_bounds__(THREADS) d64_out_kernel(const AveGdnArgs a, co
   pdl_trigger();
   pdl_wait();
   if (!offsets_ok(a, false)) return;
-  const Chunk c = chunk_of_slot(a, blockIdx.x);
+  const SlotChunk c = chunk_of_slot(a, blockIdx.x);
   if (!c.ok) return;
   const int hk = h / (a.Hv / a.Hk);
   const uint8_t* rec = recs + ((int64_t)blockIdx.x * a.Hv + h) * REC_BYTES;
@@ -548,11 +515,9 @@ __global__ void __launch_bounds__(THREADS) d64_out_kernel(const AveGdnArgs a, co
   }
 }
 
-int64_t d64_slots(const AveGdnArgs& a) { return (int64_t)a.B * a.T / CH + a.n_seqs + 1; }
-
 }  // namespace
 
-size_t prefill_d64_workspace_bytes(const AveGdnArgs& a) { return (size_t)d64_slots(a) * a.Hv * REC_BYTES; }
+size_t prefill_d64_workspace_bytes(const AveGdnArgs& a) { return (size_t)record_slots(a) * a.Hv * REC_BYTES; }
 
 int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream) {
   if (a.n_seqs == 0) return AVE_GDN_OK;
@@ -566,7 +531,7 @@ int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream) {
     attr_set_dev[dev & 63] = true;  // repeating the calls from another thread is harmless
   }
   uint8_t* recs = reinterpret_cast<uint8_t*>(a.workspace);
-  const dim3 chunks((unsigned)d64_slots(a), (unsigned)a.Hv);
+  const dim3 chunks((unsigned)record_slots(a), (unsigned)a.Hv);
   AVE_CUDA_TRY(launch_after(d64_prep_kernel, chunks, THREADS, PQ_SMEM, stream, a, recs));
   AVE_CUDA_TRY(launch_after(d64_chain_kernel, dim3((unsigned)a.n_seqs, (unsigned)a.Hv, DH / CN_ROWS), CN_T, CN_SMEM, stream, a, recs));
   AVE_CUDA_TRY(launch_after(d64_out_kernel, chunks, THREADS, OT_SMEM, stream, a, recs));

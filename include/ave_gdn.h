@@ -53,9 +53,10 @@ typedef enum AveGdnStatus {
 
 /* bits OR-ed into the device status word */
 #define AVE_GDN_DEV_BAD_SLOT 1u      /* state index >= num_slots: that sequence was skipped */
-#define AVE_GDN_DEV_BAD_SEQLEN 2u    /* cu_seqlens not monotone inside [0, T]: the whole batch was skipped (its outputs are
-                                        undefined); or a sequence longer than max_seqlen: that sequence was skipped like
-                                        one with a negative slot (zero output, state untouched) */
+#define AVE_GDN_DEV_BAD_SEQLEN 2u    /* cu_seqlens not monotone inside [0, T]: the whole batch of a prefill or backward call was
+                                        skipped (its outputs are undefined), the decode step skips such a sequence alone; or a
+                                        sequence longer than max_seqlen: that sequence was skipped like one with a negative
+                                        slot (zero output, state untouched) */
 #define AVE_GDN_DEV_WAIT_EXPIRED 4u  /* a bounded wait inside a kernel gave up */
 
 /* flags */
