@@ -11,6 +11,9 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/core/InferenceMode.h>
+#include <c10/cuda/CUDACachingAllocator.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <dlfcn.h>
@@ -159,19 +162,108 @@ const Tensor& status_word(const at::Device& dev) {
   const int idx = dev.has_index() ? dev.index() : c10::cuda::current_device();
   std::lock_guard<std::mutex> lock(g_mu);
   Tensor& w = status_words()[idx];
+  const c10::InferenceMode ordinary(false);  // a word made in inference mode could not be reset outside it
   if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, idx)));
   return w;
 }
-// Scratch grown on demand and reused, one per (device, stream): calls in one stream are ordered.
-void* workspace(const Tensor& like, cudaStream_t stream, size_t nbytes, uint64_t* size) {
-  static auto* pool = new std::map<std::pair<int, cudaStream_t>, Tensor>();
-  std::lock_guard<std::mutex> lock(g_mu);
-  Tensor& w = (*pool)[{like.get_device(), stream}];
-  if (!w.defined() || (size_t)w.numel() < nbytes)
-    w = at::empty({(int64_t)(nbytes > 0 ? nbytes : 1)}, at::TensorOptions().dtype(at::kByte).device(like.device()));
-  *size = (uint64_t)w.numel();
-  return w.data_ptr();
+// Scratch.  A call owns its block from the moment it asks for one until all that uses it is enqueued, and then leaves it for the
+// next call on the same stream: two host threads on one stream never work on one block, and since the stream orders the
+// calls, a block left behind may still be in use on the GPU.  While the stream is being captured the block comes from the
+// graph's own memory and is not kept, so a replay finds what it was captured with whatever ran in between.  Kept blocks are
+// bounded in number and bytes, the least recently used going first, and go back to torch's allocator when that runs short.
+constexpr size_t KEPT_BLOCKS = 8;             // a device
+constexpr int64_t KEPT_BYTES = 12ll << 30;    // a device; the largest prefill measured (262144 tokens, 32 heads) takes 9
+class ScratchPool {
+ public:
+  Tensor take(int device, cudaStream_t stream, int64_t bytes) {
+    Tensor t;
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      const auto it = blocks_.find({device, stream});
+      if (it != blocks_.end()) {
+        t = std::move(it->second.t);
+        blocks_.erase(it);
+      }
+    }
+    if (t.defined() && t.numel() < bytes) t.reset();  // (before the larger one is asked for)
+    if (!t.defined()) t = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, device)));
+    return t;
+  }
+  void give(int device, cudaStream_t stream, Tensor t) {
+    std::vector<Tensor> out;  // outlives the lock: freeing a block may call release()
+    out.push_back(std::move(t));
+    if (out[0].numel() > KEPT_BYTES) return;
+    std::lock_guard<std::mutex> lock(mu_);
+    Block& own = blocks_[{device, stream}];
+    if (!own.t.defined() || own.t.numel() < out[0].numel()) std::swap(own.t, out[0]);  // (another thread may have left a larger one)
+    own.used = ++clock_;
+    for (;;) {
+      size_t count = 0;
+      int64_t bytes = 0;
+      auto oldest = blocks_.end();
+      for (auto it = blocks_.begin(); it != blocks_.end(); ++it) {
+        if (it->first.first != device) continue;
+        ++count;
+        bytes += it->second.t.numel();
+        if (oldest == blocks_.end() || it->second.used < oldest->second.used) oldest = it;
+      }
+      if (count <= KEPT_BLOCKS && bytes <= KEPT_BYTES) break;
+      out.push_back(std::move(oldest->second.t));
+      blocks_.erase(oldest);
+    }
+  }
+  bool release(int device) {  // whether there was anything to give back
+    std::vector<Tensor> out;
+    std::lock_guard<std::mutex> lock(mu_);
+    for (auto it = blocks_.begin(); it != blocks_.end();) {
+      if (it->first.first != device) { ++it; continue; }
+      out.push_back(std::move(it->second.t));
+      it = blocks_.erase(it);
+    }
+    return !out.empty();
+  }
+
+ private:
+  struct Block {
+    Tensor t;
+    uint64_t used = 0;
+  };
+  std::mutex mu_;
+  std::map<std::pair<int, cudaStream_t>, Block> blocks_;
+  uint64_t clock_ = 0;
+};
+ScratchPool& scratch_pool() {
+  static auto* pool = new ScratchPool();  // never destroyed: the CUDA context may be gone at exit
+  return *pool;
 }
+// Called by torch's allocator, before it gives up, on the thread that asked it for memory (with that thread's device current).
+class ReleaseScratch : public c10::FreeMemoryCallback {
+ public:
+  bool Execute() override { return scratch_pool().release(c10::cuda::current_device()); }
+};
+
+class Scratch {  // one call's block
+ public:
+  Scratch(const Tensor& like, cudaStream_t stream, size_t bytes)
+      : device_(like.get_device()), stream_(stream),
+        captured_(c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+    const int64_t n = bytes > 0 ? (int64_t)bytes : 1;
+    t_ = captured_ ? at::empty({n}, at::TensorOptions().dtype(at::kByte).device(like.device())) : scratch_pool().take(device_, stream, n);
+  }
+  ~Scratch() {
+    if (!captured_) scratch_pool().give(device_, stream_, std::move(t_));
+  }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+  void* data() const { return t_.data_ptr(); }
+  uint64_t size() const { return (uint64_t)t_.numel(); }
+
+ private:
+  int device_;
+  cudaStream_t stream_;
+  bool captured_;
+  Tensor t_;
+};
 struct Launch {  // device of the tensors made current, its current stream, no GIL while the library enqueues
   c10::cuda::OptionalCUDAGuard guard;
   cudaStream_t stream;
@@ -305,7 +397,8 @@ AveGdnArgs fill_args(const Tensor& q, const Tensor& k, const Tensor& v, const Te
 
 void enqueue_prefill(AveGdnArgs& a, const Tensor& q) {
   Launch launch(q);
-  a.workspace = workspace(q, launch.stream, api.prefill_workspace_bytes(&a), &a.workspace_bytes);
+  const Scratch ws(q, launch.stream, api.prefill_workspace_bytes(&a));
+  a.workspace = ws.data(); a.workspace_bytes = ws.size();
   check(launch([&] { return api.chunk_prefill(&a, launch.stream); }), "chunk_gated_delta_rule");
 }
 void enqueue_decode(AveGdnArgs& a, const Tensor& q) {
@@ -658,7 +751,8 @@ AveGdnBwdArgs bwd_args(const Tensor& q, const Tensor& k, const Tensor& v, const 
 }
 void enqueue_backward(AveGdnBwdArgs& a, const Tensor& q) {
   Launch launch(q);
-  a.workspace = workspace(q, launch.stream, api.backward_workspace_bytes(&a), &a.workspace_bytes);
+  const Scratch ws(q, launch.stream, api.backward_workspace_bytes(&a));
+  a.workspace = ws.data(); a.workspace_bytes = ws.size();
   check(launch([&] { return api.recurrent_backward(&a, launch.stream); }), "gated_delta_rule_backward");
 }
 
@@ -835,4 +929,7 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, null
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__host() {
+  c10::FreeCudaMemoryCallbacksRegistry()->Register(text("avelang_gdn_scratch ", &scratch_pool()), [] { return std::make_unique<ReleaseScratch>(); }, "");
+  return PyModule_Create(&module);
+}
