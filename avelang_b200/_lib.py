@@ -13,7 +13,7 @@ P, U32, I32, I64, U64, F32 = (ctypes.c_void_p, ctypes.c_uint32, ctypes.c_int32, 
 
 OK, INVALID_ARGUMENT, UNSUPPORTED, MISALIGNED, CUDA_ERROR, WORKSPACE_TOO_SMALL = range(6)
 DEV_BAD_SLOT, DEV_BAD_SEQLEN, DEV_WAIT_EXPIRED = 1, 2, 4
-FLAG_QK_L2NORM, FLAG_GATE_FIRST = 1, 2
+FLAG_QK_L2NORM, FLAG_GATE_FIRST, FLAG_BWD_SUMMED = 1, 2, 4
 NOALLOC_SCRATCH_BYTES = 64 << 20
 ABI_VERSION = 4
 

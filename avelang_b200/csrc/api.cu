@@ -20,7 +20,7 @@ int launch_gemm_bf16_nt_scatter(const AveGemmReduceArgs& a, cudaStream_t stream)
 int launch_gemm_reduce_push(const AveGemmReduceArgs& a, cudaStream_t stream);
 int launch_decode_layer(const AveGdnDecodeLayerArgs& a, cudaStream_t stream);
 int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream);
-size_t backward_workspace_bytes(const AveGdnBwdArgs& a);
+size_t backward_workspace_bytes(const AveGdnBwdArgs& a, int key_heads);
 
 static size_t prefill_ws_bytes(const AveGdnArgs& a) {
   return a.dk == 128 ? prefill_tc_workspace_bytes(a, false) : prefill_d64_workspace_bytes(a);
@@ -168,7 +168,7 @@ static int validate_bwd(const AveGdnBwdArgs* a) {
 
 size_t ave_gdn_backward_workspace_bytes(const AveGdnBwdArgs* a) {
   if (validate_bwd(a) != AVE_GDN_OK) return 0;
-  return backward_workspace_bytes(*a);
+  return backward_workspace_bytes(*a, a->Hk);
 }
 
 int ave_gdn_recurrent_backward(const AveGdnBwdArgs* a, void* stream) {
@@ -176,7 +176,7 @@ int ave_gdn_recurrent_backward(const AveGdnBwdArgs* a, void* stream) {
   if (rc != AVE_GDN_OK) return rc;
   if ((int64_t)a->B * a->T == 0 || a->n_seqs == 0) return AVE_GDN_OK;
   if (a->workspace == nullptr || !aligned16(a->workspace)) return AVE_GDN_INVALID_ARGUMENT;
-  if (a->workspace_bytes < backward_workspace_bytes(*a)) return AVE_GDN_WORKSPACE_TOO_SMALL;
+  if (a->workspace_bytes < backward_workspace_bytes(*a, 1)) return AVE_GDN_WORKSPACE_TOO_SMALL;
   return launch_backward(*a, reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -24,6 +24,8 @@
 // the gradient of the gate needs, because it is a difference of large sums.
 // Two sequences of 4096 tokens, 32 value heads: 0.82 ms (prep 0.08, scans 0.30, gradients 0.44) against 22.1 ms for the
 // token-by-token reverse sweep this replaced (a 64 KiB tile written and read per token).
+#include <type_traits>
+
 #include "common.cuh"
 #include "recslots.cuh"
 #include "tc.cuh"
@@ -37,10 +39,15 @@ constexpr int IMG = BCH * BCH * 2;              // one bf16 [64][64] tile
 constexpr int PREP_P = 3 * IMG, PREP_SC = 6 * IMG, SC_BYTES = 3 * BCH * 4, PREP_BYTES = PREP_SC + SC_BYTES;  // T h m l | P h m l | b | beta | b's low part
 constexpr int STATE_FLOATS = BD * BD, VEC_FLOATS = BD * BCH;
 
+// 246528 bytes a (slot, value head).  The key heads are independent of one another, so a call with less scratch than all of
+// them need takes them in several passes over the same scratch, one after the other.  A pass is a call on its own heads: Hk
+// and Hv of its argument block are theirs, and its pointers start at their first; hk_all and hv_all are the heads of the
+// whole call, the pitch of the states and of the results.
 struct BwdScratch {
   uint8_t* prep;   // [slots][Hv][PREP_BYTES]; the tiles are stored as the swizzled shared-memory images the scans read
   float *m0, *e;   // [slots][Hv][d_k / 8][d_v][8]: H = M0^T and E^T of every chunk
   float *vn, *u;   // [slots][Hv][64 tokens / 8][d_v][8]: Vn^T and Ut^T
+  int hk_all, hv_all;
 };
 
 // ---------------------------------------------------------------------------------------------- T, P and b of every chunk
@@ -252,7 +259,7 @@ __device__ __forceinline__ void bwd_scan(const AveGdnBwdArgs& a, const BwdScratc
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = unit / a.Hv, h = unit % a.Hv, hk = h / (a.Hv / a.Hk);
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
-  const int64_t tile = (int64_t)unit * STATE_FLOATS;
+  const int64_t tile = ((int64_t)n * ws.hv_all + h) * STATE_FLOATS;
   if (sp.len == 0) {  // empty sequence: the state gradient passes through
     if (kRev && a.d_initial_state != nullptr)
       for (int e = tid; e < STATE_FLOATS; e += SC_T) a.d_initial_state[tile + e] = a.d_final_state ? a.d_final_state[tile + e] : 0.f;
@@ -586,7 +593,7 @@ __device__ __forceinline__ float lane_sums(float (&v)[16], int lane) {
 // Per-head gradients kept in fp32 (the C entry point), or summed over the heads of a key head and rounded to bf16: eight tokens
 // of one d_k column per lane.
 template <bool kSum>
-__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, const SlotChunk& c, int head, int tok0, int dk, const float (&x)[8]) {
+__device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, const BwdScratch& ws, float* dst, const SlotChunk& c, int head, int tok0, int dk, const float (&x)[8]) {
   const int64_t row = (int64_t)c.b * a.T + c.t0 + tok0;
 #pragma unroll
   for (int i = 0; i < 8; i += 2) {
@@ -595,11 +602,11 @@ __device__ __forceinline__ void store_dqk(const AveGdnBwdArgs& a, float* dst, co
       const float y = __shfl_xor_sync(0xffffffffu, odd ? x[i] : x[i + 1], 1);
       const int j = i + (odd ? 1 : 0);
       if (tok0 + j < c.len)
-        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(dst) + ((row + j) * a.Hk + head) * BD + (dk & ~1)) =
+        *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(dst) + ((row + j) * ws.hk_all + head) * BD + (dk & ~1)) =
             odd ? pack_bf16x2(y, x[i + 1]) : pack_bf16x2(x[i], y);
     } else {
-      if (tok0 + i < c.len) dst[((row + i) * a.Hv + head) * BD + dk] = x[i];
-      if (tok0 + i + 1 < c.len) dst[((row + i + 1) * a.Hv + head) * BD + dk] = x[i + 1];
+      if (tok0 + i < c.len) dst[((row + i) * ws.hv_all + head) * BD + dk] = x[i];
+      if (tok0 + i + 1 < c.len) dst[((row + i + 1) * ws.hv_all + head) * BD + dk] = x[i + 1];
     }
   }
 }
@@ -820,8 +827,8 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
                 const float2 v = bf16x2_to_float2(vv[mt][half][kk]);
                 s = fmaf(ut.x, v.x, fmaf(ut.y, v.y, s));
                 const float be = betas[tok];
-                if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.d_v) + ((row0 + tok) * a.Hv + h) * BD + col) = pack_bf16x2(be * ut.x, be * ut.y);
-                else *reinterpret_cast<float2*>(a.d_v + ((row0 + tok) * a.Hv + h) * BD + col) = make_float2(be * ut.x, be * ut.y);
+                if (kSum) *reinterpret_cast<uint32_t*>(reinterpret_cast<__nv_bfloat16*>(a.d_v) + ((row0 + tok) * ws.hv_all + h) * BD + col) = pack_bf16x2(be * ut.x, be * ut.y);
+                else *reinterpret_cast<float2*>(a.d_v + ((row0 + tok) * ws.hv_all + h) * BD + col) = make_float2(be * ut.x, be * ut.y);
               }
             }
             s = quad_sum(s);
@@ -873,8 +880,8 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
           }
         }
         if (!kSum || hh == r - 1) {
-          store_dqk<kSum>(a, a.d_q, c, kSum ? hk : h, tok0, dk, dq);
-          store_dqk<kSum>(a, a.d_k, c, kSum ? hk : h, tok0, dk, dkv);
+          store_dqk<kSum>(a, ws, a.d_q, c, kSum ? hk : h, tok0, dk, dq);
+          store_dqk<kSum>(a, ws, a.d_k, c, kSum ? hk : h, tok0, dk, dkv);
         }
       }
       states = warp_sum(states);
@@ -891,7 +898,7 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
 #pragma unroll
         for (int w = 0; w < 16; ++w) { em += dots[w]; st += dots[16 + w]; }
         const float be = fabsf(betas[tid]) < 1e-20f ? 1e-20f : betas[tid];
-        const int64_t off = (row0 + tid) * a.Hv + h;
+        const int64_t off = (row0 + tid) * ws.hv_all + h;
         if (tid < c.len) a.d_beta[off] = su + s.y / be;
         float db = s.x;
 #pragma unroll
@@ -911,32 +918,52 @@ __global__ void __launch_bounds__(GR_T, 1) bwd_grads_kernel(const AveGdnBwdArgs 
   if (warp == 1) tc::tmem_dealloc(*tmem_slot, 512);
 }
 
-BwdScratch scratch_layout(const AveGdnBwdArgs& a, size_t* total) {
-  const size_t recs = (size_t)record_slots(a) * a.Hv;
-  uint8_t* p = reinterpret_cast<uint8_t*>(a.workspace);
+// Scratch of a pass over nk key heads.
+BwdScratch scratch_layout(const AveGdnBwdArgs& a, int nk, size_t* total) {
   BwdScratch ws;
+  ws.hk_all = a.Hk; ws.hv_all = a.Hv;
+  const size_t recs = (size_t)record_slots(a) * nk * (a.Hv / a.Hk);
+  uint8_t* p = reinterpret_cast<uint8_t*>(a.workspace);
   size_t off = 0;
-  auto take = [&](size_t bytes) { uint8_t* q = p + off; off += (bytes + 255) & ~(size_t)255; return q; };
-  ws.prep = take(recs * PREP_BYTES);
-  ws.m0 = reinterpret_cast<float*>(take(recs * STATE_FLOATS * 4));
-  ws.e = reinterpret_cast<float*>(take(recs * STATE_FLOATS * 4));
-  ws.vn = reinterpret_cast<float*>(take(recs * VEC_FLOATS * 4));
-  ws.u = reinterpret_cast<float*>(take(recs * VEC_FLOATS * 4));
+  auto take = [&](size_t bytes) { uint8_t* q = p + off; off += (recs * bytes + 255) & ~(size_t)255; return q; };
+  ws.prep = take(PREP_BYTES);
+  ws.m0 = reinterpret_cast<float*>(take(STATE_FLOATS * 4));
+  ws.e = reinterpret_cast<float*>(take(STATE_FLOATS * 4));
+  ws.vn = reinterpret_cast<float*>(take(VEC_FLOATS * 4));
+  ws.u = reinterpret_cast<float*>(take(VEC_FLOATS * 4));
   if (total != nullptr) *total = off;
   return ws;
 }
 
+// The argument block of a pass over the nk key heads from hk0 on.
+AveGdnBwdArgs pass_args(const AveGdnBwdArgs& a, int hk0, int nk) {
+  const int r = a.Hv / a.Hk, h0 = hk0 * r;
+  const bool sum = (a.flags & AVE_GDN_FLAG_BWD_SUMMED) != 0;
+  AveGdnBwdArgs p = a;
+  auto skip = [](auto& ptr, int64_t bytes) { if (ptr != nullptr) ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(reinterpret_cast<uintptr_t>(ptr) + bytes); };
+  p.Hk = nk; p.Hv = nk * r;
+  skip(p.q, hk0 * a.q_stride_h * 2); skip(p.k, hk0 * a.k_stride_h * 2);
+  skip(p.v, h0 * a.v_stride_h * 2); skip(p.d_o, h0 * a.do_stride_h * 2);
+  skip(p.g, (int64_t)h0 * 4); skip(p.beta, (int64_t)h0 * 4);
+  for (auto* s : {&p.initial_state, &p.d_final_state}) skip(*s, (int64_t)h0 * STATE_FLOATS * 4);
+  skip(p.d_initial_state, (int64_t)h0 * STATE_FLOATS * 4);
+  for (auto* d : {&p.d_q, &p.d_k}) skip(*d, (int64_t)(sum ? hk0 * 2 : h0 * 4) * BD);
+  skip(p.d_v, (int64_t)h0 * BD * (sum ? 2 : 4));
+  skip(p.d_g, (int64_t)h0 * 4); skip(p.d_beta, (int64_t)h0 * 4);
+  return p;
+}
+
 }  // namespace
 
-size_t backward_workspace_bytes(const AveGdnBwdArgs& a) {
+// Bytes for a pass over nk of the a.Hk key heads.
+size_t backward_workspace_bytes(const AveGdnBwdArgs& a, int nk) {
   size_t total = 0;
-  scratch_layout(a, &total);
+  scratch_layout(a, nk, &total);
   return total;
 }
 
 int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
-  const int units = a.n_seqs * a.Hv;
-  if (units == 0 || a.T == 0) return AVE_GDN_OK;
+  if (a.n_seqs * a.Hv == 0 || a.T == 0) return AVE_GDN_OK;
   static bool attr_set_dev[64] = {};
   int dev = 0;
   AVE_CUDA_TRY(cudaGetDevice(&dev));
@@ -948,15 +975,20 @@ int launch_backward(const AveGdnBwdArgs& a, cudaStream_t stream) {
     AVE_CUDA_TRY(cudaFuncSetAttribute(bwd_grads_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GR_SMEM));
     attr_set_dev[dev] = true;  // repeating the calls from another thread is harmless
   }
-  const BwdScratch ws = scratch_layout(a, nullptr);
+  int passes = 1, nk = a.Hk;  // as few passes as the scratch allows, of equal size
+  while (nk > 1 && backward_workspace_bytes(a, nk) > a.workspace_bytes) nk = (a.Hk + passes) / (passes + 1), ++passes;
   const unsigned slots = (unsigned)record_slots(a);
-  bwd_prep_kernel<<<dim3(slots, (unsigned)(a.Hk * ((a.Hv / a.Hk + 1) / 2))), PREP_T, PR_SMEM, stream>>>(a, ws);
-  AVE_CUDA_TRY(cudaGetLastError());
-  bwd_scans_kernel<<<2 * units, SC_T, SC_SMEM, stream>>>(a, ws);
-  AVE_CUDA_TRY(cudaGetLastError());
   const bool sum = (a.flags & AVE_GDN_FLAG_BWD_SUMMED) != 0;
-  (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<(unsigned)min((int64_t)GR_CTAS, (int64_t)slots * a.Hk), GR_T, GR_SMEM, stream>>>(a, ws, slots);
-  AVE_CUDA_TRY(cudaGetLastError());
+  for (int hk0 = 0; hk0 < a.Hk; hk0 += nk) {
+    const AveGdnBwdArgs p = pass_args(a, hk0, min(nk, a.Hk - hk0));
+    const BwdScratch ws = scratch_layout(a, p.Hk, nullptr);
+    bwd_prep_kernel<<<dim3(slots, (unsigned)(p.Hk * ((p.Hv / p.Hk + 1) / 2))), PREP_T, PR_SMEM, stream>>>(p, ws);
+    AVE_CUDA_TRY(cudaGetLastError());
+    bwd_scans_kernel<<<2 * p.n_seqs * p.Hv, SC_T, SC_SMEM, stream>>>(p, ws);
+    AVE_CUDA_TRY(cudaGetLastError());
+    (sum ? bwd_grads_kernel<true> : bwd_grads_kernel<false>)<<<(unsigned)min((int64_t)GR_CTAS, (int64_t)slots * p.Hk), GR_T, GR_SMEM, stream>>>(p, ws, slots);
+    AVE_CUDA_TRY(cudaGetLastError());
+  }
   return AVE_GDN_OK;
 }
 

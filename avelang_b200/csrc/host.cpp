@@ -22,6 +22,7 @@
 
 #include <map>
 #include <mutex>
+#include <optional>
 #include <sstream>
 #include <string>
 #include <utility>
@@ -751,8 +752,21 @@ AveGdnBwdArgs bwd_args(const Tensor& q, const Tensor& k, const Tensor& v, const 
 }
 void enqueue_backward(AveGdnBwdArgs& a, const Tensor& q) {
   Launch launch(q);
-  const Scratch ws(q, launch.stream, api.backward_workspace_bytes(&a));
-  a.workspace = ws.data(); a.workspace_bytes = ws.size();
+  // Scratch for all key heads at once; where that does not fit, for half of them, a quarter, ...: the call then takes as many
+  // passes.  (Two sequences of 4096 tokens, 32 value heads: 0.82 ms
+  // in one pass of 1.03 GB, 1.12 in two, 1.78 in four: half the heads leave half the SMs to the scans.)
+  std::optional<Scratch> ws;
+  for (int heads = a.Hk;; heads = (heads + 1) / 2) {
+    AveGdnBwdArgs part = a;
+    part.Hk = heads; part.Hv = a.Hk > 0 ? heads * (a.Hv / a.Hk) : a.Hv;
+    try {
+      ws.emplace(q, launch.stream, api.backward_workspace_bytes(&part));
+      break;
+    } catch (const c10::OutOfMemoryError&) {
+      if (heads <= 1) throw;
+    }
+  }
+  a.workspace = ws->data(); a.workspace_bytes = ws->size();
   check(launch([&] { return api.recurrent_backward(&a, launch.stream); }), "gated_delta_rule_backward");
 }
 

@@ -263,7 +263,10 @@ int ave_gdn_decode_layer_step(const AveGdnDecodeLayerArgs* args, void* stream);
  * dq, dk [B,T,Hv,dk] PER VALUE HEAD (the caller sums the value heads that share a key head), dv [B,T,Hv,dv],
  * dg, dbeta [B,T,Hv], and optionally d_initial_state [n_seqs,Hv,dk,dv]; all contiguous.  With AVE_GDN_FLAG_BWD_SUMMED
  * d_q and d_k point to bf16 [B,T,Hk,dk] (the value heads of a key head summed in fp32) and d_v to bf16 [B,T,Hv,dv].
- * Chunked like the forward pass, with fp32-level accuracy; the states and their gradients of all chunks live in `workspace`. */
+ * Chunked like the forward pass, with fp32-level accuracy; the states and their gradients of all chunks live in `workspace`:
+ * ave_gdn_backward_workspace_bytes() is 246528 bytes for every (record, value head), with floor(B*T/64) + n_seqs + 1 records
+ * (131072 tokens x 32 heads: 16.2 GB).  With less, down to what one key head needs (ask with Hk = 1 and Hv = the value heads of
+ * a key head), the call takes the key heads in as many passes as it must, with the same results. */
 typedef struct AveGdnBwdArgs {
   uint32_t struct_size;
   uint32_t flags;
@@ -283,7 +286,7 @@ typedef struct AveGdnBwdArgs {
   float* d_beta;                  /* fp32 [B,T,Hv] */
   float* d_initial_state;         /* optional */
   uint32_t* status;
-  void* workspace;                /* >= ave_gdn_backward_workspace_bytes() */
+  void* workspace;                /* ave_gdn_backward_workspace_bytes(), or less (see above) */
   uint64_t workspace_bytes;
   int32_t B, T, Hk, Hv, dk, dv, n_seqs, reserved0;
   int64_t q_stride_b, q_stride_t, q_stride_h;
