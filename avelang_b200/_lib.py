@@ -151,6 +151,15 @@ class _Host:
 host = _Host()
 
 
+def register_operators() -> None:
+    """Registers the CUDA implementations of ``torch.ops.avelang_gdn.*`` (they come with the native host side).  Where something
+    is not built yet, the first public call says so."""
+    try:
+        host.bind
+    except (ImportError, OSError, ValueError):
+        pass
+
+
 def check(rc: int, what: str) -> None:
     """Map a status code to the reference's exception convention: argument problems raise ValueError
     (python/avelang_kernels/amdgpu_gemm.py:463-486), device/runtime problems RuntimeError

@@ -1,16 +1,19 @@
-// Host side of the public functions (module avelang_b200._host): argument checks, output allocation, scratch and the call
-// into libave_gdn_b200.so, in C++.  A decode step of a few sequences runs for 5 to 30 us on the GPU; with the checks and
-// the argument block filled from Python (attribute by attribute through ctypes, behind a dispatcher round trip) a call cost
-// 45 to 75 us of host time and the GPU idled between steps.  Here a call costs a few microseconds (back-to-back steps on one
-// sequence of 32 heads: 51.0 -> 6.1 us; 37 sequences with the gated norm: 57.6 -> 32.8 us, now bound by the kernel).
+// Host side of the library (module avelang_b200._host), in C++: the operators torch.ops.avelang_gdn.* and the public functions.
 //
-// The functions take the positional arguments their Python wrappers pass (METH_FASTCALL: no tuple, no keyword parsing),
-// raise ValueError with the wording of the Python API for bad arguments, enqueue on torch's current stream of the tensors'
-// device and return without synchronising.
+// An operator's CUDA kernel fills the C argument block and calls into libave_gdn_b200.so on torch's current stream.  A public
+// function takes the positional arguments its Python wrapper passes (METH_FASTCALL: no tuple, no keyword parsing), checks
+// them, raises ValueError with the wording of the Python API, allocates what it returns and calls the operator through the
+// dispatcher, so dispatch modes, tensor subclasses and the profiler see every call.
+//
+// A decode step of a few sequences runs for 5 to 30 us on the GPU; with the checks and the argument block filled from Python
+// (attribute by attribute through ctypes, behind a boxed dispatcher round trip) a call cost 45 to 75 us of host time and the
+// GPU idled between steps.  Here a call costs a few microseconds (back-to-back steps on one sequence of 32 heads:
+// 51.0 -> 5.0 us; 37 sequences with the gated norm: 57.6 -> 30.1 us, now bound by the kernel).
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/core/dispatch/Dispatcher.h>
 #include <c10/core/InferenceMode.h>
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
@@ -19,8 +22,11 @@
 #include <dlfcn.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
+#include <torch/library.h>
 
+#include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <optional>
 #include <sstream>
@@ -35,18 +41,17 @@ namespace {
 using at::Tensor;
 
 // ---------------------------------------------------------------------------------------------- errors
-struct BadArgument {
-  std::string what;
-};
 template <class... Parts>
 std::string text(const Parts&... parts) {
   std::ostringstream s;
   (void)std::initializer_list<int>{(s << parts, 0)...};
   return s.str();
 }
-#define REQ(cond, ...)                                     \
-  do {                                                     \
-    if (__builtin_expect(!(cond), 0)) throw BadArgument{text(__VA_ARGS__)}; \
+// argument problems raise ValueError, from a public function and from an operator alike
+#define BAD_ARGUMENT(...) throw c10::ValueError({__func__, __FILE__, static_cast<uint32_t>(__LINE__)}, text(__VA_ARGS__))
+#define REQ(cond, ...)                                            \
+  do {                                                            \
+    if (__builtin_expect(!(cond), 0)) BAD_ARGUMENT(__VA_ARGS__);  \
   } while (0)
 
 std::string shape_of(at::IntArrayRef s) {  // as Python prints a tuple
@@ -93,12 +98,11 @@ struct Api {
 void check(int rc, const char* what) {
   if (__builtin_expect(rc == AVE_GDN_OK, 1)) return;
   const std::string msg = text(what, ": ", api.status_string(rc));
-  if (rc == AVE_GDN_CUDA_ERROR) {
-    PyErr_SetString(PyExc_RuntimeError, text(msg, " (cudaError ", api.last_cuda_error(), ")").c_str());
-    throw python_error();
-  }
-  throw BadArgument{msg};
+  if (rc == AVE_GDN_CUDA_ERROR) throw c10::Error({__func__, __FILE__, static_cast<uint32_t>(__LINE__)}, text(msg, " (cudaError ", api.last_cuda_error(), ")"));
+  BAD_ARGUMENT(msg);
 }
+// an operator reached before the Python layer has loaded the library
+void loaded() { TORCH_CHECK(api.chunk_prefill != nullptr, "libave_gdn_b200.so is not loaded: run `python -m avelang_b200.build`; there is no fallback implementation"); }
 
 // ---------------------------------------------------------------------------------------------- arguments
 const Tensor* opt_tensor(PyObject* o, const char* name) {
@@ -151,21 +155,23 @@ Tensor empty(at::IntArrayRef shape, at::ScalarType dt, const Tensor& like) {
   return at::empty(shape, like.options().dtype(dt).requires_grad(false));
 }
 // fp32, contiguous; the tensor itself when it is both already
-Tensor f32(const Tensor& t) { return t.detach().to(at::kFloat).contiguous(); }
+Tensor f32(const Tensor& t) { return (t.requires_grad() ? t.detach() : t).to(at::kFloat).contiguous(); }
 
 // ---------------------------------------------------------------------------------------------- scratch and status word
-std::mutex g_mu;
-std::map<int, Tensor>& status_words() {
-  static auto* m = new std::map<int, Tensor>();  // never destroyed: the CUDA context may be gone at exit
-  return *m;
-}
-const Tensor& status_word(const at::Device& dev) {
+const Tensor& status_word(const at::Device& dev) {  // one a device, never destroyed: the CUDA context may be gone at exit
+  static std::atomic<Tensor*> words[C10_COMPILE_TIME_MAX_GPUS];
+  static std::mutex mu;
   const int idx = dev.has_index() ? dev.index() : c10::cuda::current_device();
-  std::lock_guard<std::mutex> lock(g_mu);
-  Tensor& w = status_words()[idx];
-  const c10::InferenceMode ordinary(false);  // a word made in inference mode could not be reset outside it
-  if (!w.defined()) w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, idx)));
-  return w;
+  std::atomic<Tensor*>& w = words[idx];
+  Tensor* t = w.load(std::memory_order_acquire);
+  if (t == nullptr) {
+    const c10::InferenceMode ordinary(false);  // a word made in inference mode could not be reset outside it
+    auto made = std::make_unique<Tensor>(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::Device(at::kCUDA, idx))));
+    std::lock_guard<std::mutex> lock(mu);
+    t = w.load(std::memory_order_acquire);
+    if (t == nullptr) w.store(t = made.release(), std::memory_order_release);
+  }
+  return *t;
 }
 // Scratch.  A call owns its block from the moment it asks for one until all that uses it is enqueued, and then leaves it for the
 // next call on the same stream: two host threads on one stream never work on one block, and since the stream orders the
@@ -274,6 +280,7 @@ struct Launch {  // device of the tensors made current, its current stream, no G
   }
   template <class F>
   int operator()(F f) {
+    if (PyGILState_Check() == 0) return f();  // an operator called without it
     PyThreadState* ts = PyEval_SaveThread();
     const int rc = f();
     PyEval_RestoreThread(ts);
@@ -344,8 +351,8 @@ Tensor prep_norm_weight(const Tensor* w, const Tensor* z, const Shape& s, const 
   return f32(*w);
 }
 
-// final states to write (undefined when none are wanted) and the number of slots of the state arrays
-std::pair<Tensor, int64_t> prep_states(const Tensor* s0, const Tensor* idx, const Shape& s, const Tensor& like, bool want_final,
+// final states to write (undefined when none are wanted)
+Tensor prep_states(const Tensor* s0, const Tensor* idx, const Shape& s, const Tensor& like, bool want_final,
                                        bool inplace) {
   int64_t slots = s.n;
   if (s0 != nullptr) {
@@ -367,7 +374,7 @@ std::pair<Tensor, int64_t> prep_states(const Tensor* s0, const Tensor* idx, cons
     if (idx != nullptr) final = inplace ? *s0 : s0->clone();
     else final = empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, like);
   }
-  return {final, slots};
+  return final;
 }
 
 #define STRIDES4(dst, name, t) \
@@ -396,6 +403,20 @@ AveGdnArgs fill_args(const Tensor& q, const Tensor& k, const Tensor& v, const Te
   return a;
 }
 
+// ---------------------------------------------------------------------------------------------- operators
+// The CUDA kernels of torch.ops.avelang_gdn.* (schemas: torch_ops.py).  They take tensors the caller has laid out; the library
+// checks what they pass on.
+using OptTensor = std::optional<Tensor>;
+const Tensor* some(const Tensor& t) { return t.defined() ? &t : nullptr; }
+const Tensor* some(const OptTensor& t) { return t.has_value() && t->defined() ? &*t : nullptr; }
+OptTensor opt(const Tensor* t) { return t != nullptr ? OptTensor(*t) : OptTensor(); }
+OptTensor opt(const Tensor& t) { return opt(some(t)); }
+int64_t n_sequences(const Tensor& q, const Tensor* cu) { return cu != nullptr ? cu->numel() - 1 : q.size(0); }
+int64_t n_slots(const Tensor* s0, const Tensor* final, int64_t n) {
+  const Tensor* pool = final != nullptr ? final : s0;
+  return pool != nullptr ? pool->size(0) : n;
+}
+
 void enqueue_prefill(AveGdnArgs& a, const Tensor& q) {
   Launch launch(q);
   const Scratch ws(q, launch.stream, api.prefill_workspace_bytes(&a));
@@ -407,100 +428,132 @@ void enqueue_decode(AveGdnArgs& a, const Tensor& q) {
   check(launch([&] { return api.decode_step(&a, launch.stream); }), "fused_recurrent_gated_delta_rule");
 }
 
-double scale_or(PyObject* o, int64_t dk) { return o == Py_None ? 1.0 / std::sqrt((double)dk) : number(o); }
-const Tensor* some(const Tensor& t) { return t.defined() ? &t : nullptr; }
-
-// ---------------------------------------------------------------------------------------------- public functions
-// prefill(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm, cu_seqlens, z, norm_weight, norm_eps,
-//         state_indices, inplace_state, chunk_size, out, out_peers, max_seqlen) -> (o, final or None)
-PyObject* prefill(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
-  const Tensor *s0 = opt_tensor(p[6], "initial_state"), *cu = opt_tensor(p[9], "cu_seqlens"), *z = opt_tensor(p[10], "z"),
-               *w = opt_tensor(p[11], "norm_weight"), *idx = opt_tensor(p[13], "state_indices"), *out = opt_tensor(p[16], "out"),
-               *peers = opt_tensor(p[17], "out_peers");
-  const Shape s = check_common(q, k, v, g, beta, z, cu);
-  const int64_t chunk = integer(p[15]);
-  REQ(chunk == 64, "chunk_size must be 64, got ", chunk, ".");
-  int64_t bound = 0;
-  if (p[18] != Py_None) {
-    const int64_t m = integer(p[18]);
-    REQ(m >= 0, "max_seqlen must be non-negative, got ", m, ".");
-    if (cu != nullptr) bound = std::min(m, s.T);
-  }
-  const Tensor o = prep_out(out, v);
-  const Tensor nw = prep_norm_weight(w, z, s, q.device());
-  const auto [final, slots] = prep_states(s0, idx, s, q, truth(p[7]), truth(p[14]));
-  if (peers != nullptr) {
-    REQ(z != nullptr, "out_peers needs z (the stores are fused into the gated norm)");
-    REQ(peers->scalar_type() == at::kLong && peers->dim() == 1 && peers->device() == q.device() && peers->is_contiguous(),
-        "out_peers must be a contiguous 1-D int64 tensor on ", q.device());
-  }
-  AveGdnArgs a = fill_args(q, k, v, g, beta, z, some(nw), number(p[12]), o, scale_or(p[5], s.dk), s0, some(final), cu, idx, slots, s.n, truth(p[8]));
-  a.max_seqlen = (int32_t)bound;
+void op_prefill(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& out, double scale,
+                const OptTensor& initial_state, const OptTensor& final_state, const OptTensor& cu_seqlens, const OptTensor& state_indices,
+                const OptTensor& z, const OptTensor& norm_weight, double norm_eps, bool l2norm, int64_t max_seqlen, const OptTensor& out_peers) {
+  loaded();
+  const Tensor *s0 = some(initial_state), *sf = some(final_state), *cu = some(cu_seqlens), *peers = some(out_peers);
+  const int64_t n = n_sequences(q, cu);
+  AveGdnArgs a = fill_args(q, k, v, g, beta, some(z), some(norm_weight), norm_eps, out, scale, s0, sf, cu, some(state_indices),
+                           n_slots(s0, sf, n), n, l2norm);
+  a.max_seqlen = (int32_t)max_seqlen;
   if (peers != nullptr) { a.o_peers = reinterpret_cast<const void* const*>(peers->data_ptr()); a.n_peers = (int32_t)peers->numel(); }
   enqueue_prefill(a, q);
-  return wrap_pair(o, final);
 }
 
-// decode(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm, cu_seqlens, state_indices, inplace_state, z,
-//        norm_weight, norm_eps, out) -> (o, final or None)
-PyObject* decode(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
-  const Tensor *s0 = opt_tensor(p[6], "initial_state"), *cu = opt_tensor(p[9], "cu_seqlens"), *idx = opt_tensor(p[10], "state_indices"),
-               *z = opt_tensor(p[12], "z"), *w = opt_tensor(p[13], "norm_weight"), *out = opt_tensor(p[15], "out");
-  const Shape s = check_common(q, k, v, g, beta, z, cu);
-  const Tensor o = prep_out(out, v);
-  const Tensor nw = prep_norm_weight(w, z, s, q.device());
-  const auto [final, slots] = prep_states(s0, idx, s, q, truth(p[7]), truth(p[11]));
-  AveGdnArgs a = fill_args(q, k, v, g, beta, z, some(nw), number(p[14]), o, scale_or(p[5], s.dk), s0, some(final), cu, idx, slots, s.n, truth(p[8]));
+void op_decode(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& out, double scale,
+               const OptTensor& initial_state, const OptTensor& final_state, const OptTensor& cu_seqlens, const OptTensor& state_indices,
+               const OptTensor& z, const OptTensor& norm_weight, double norm_eps, bool l2norm) {
+  loaded();
+  const Tensor *s0 = some(initial_state), *sf = some(final_state), *cu = some(cu_seqlens);
+  const int64_t n = n_sequences(q, cu);
+  AveGdnArgs a = fill_args(q, k, v, g, beta, some(z), some(norm_weight), norm_eps, out, scale, s0, sf, cu, some(state_indices),
+                           n_slots(s0, sf, n), n, l2norm);
   enqueue_decode(a, q);
-  return wrap_pair(o, final);
 }
 
-// mixed(q, k, v, g, beta, cu_seqlens, n_decode, state_pool, state_indices, scale, l2norm, z, norm_weight, norm_eps, out) -> o
-PyObject* mixed(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
-  const Tensor *cu = opt_tensor(p[5], "cu_seqlens"), *pool = opt_tensor(p[7], "state_pool"), *idx = opt_tensor(p[8], "state_indices"),
-               *z = opt_tensor(p[11], "z"), *w = opt_tensor(p[12], "norm_weight"), *out = opt_tensor(p[14], "out");
-  const Shape s = check_common(q, k, v, g, beta, z, cu);
-  REQ(cu != nullptr && s.B == 1, "mixed_prefill_decode_step takes a packed batch: B == 1 with cu_seqlens");
-  const int64_t nd = integer(p[6]);
-  REQ(nd >= 0 && nd <= s.n && nd <= s.T, "n_decode must lie in [0, ", std::min(s.n, s.T), "], got ", nd, ".");
-  REQ(pool != nullptr && idx != nullptr, "mixed_prefill_decode_step needs state_pool and state_indices");
-  const Tensor o = prep_out(out, v);
-  const Tensor nw = prep_norm_weight(w, z, s, q.device());
-  const auto [final, slots] = prep_states(pool, idx, s, q, true, true);
-  AveGdnArgs a = fill_args(q, k, v, g, beta, z, some(nw), number(p[13]), o, scale_or(p[9], s.dk), pool, &*pool, cu, idx, slots, s.n, truth(p[10]));
-  if (nd > 0) {  // one single-token sequence per row: the token stride becomes the batch stride
+void op_mixed(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& out, double scale,
+              const Tensor& state_pool, const Tensor& cu_seqlens, const Tensor& state_indices, int64_t n_decode, const OptTensor& z,
+              const OptTensor& norm_weight, double norm_eps, bool l2norm) {
+  loaded();
+  const int64_t n = cu_seqlens.numel() - 1;
+  REQ(n_decode >= 0 && n_decode <= n && n_decode <= q.size(1), "n_decode must lie in [0, ", std::min(n, q.size(1)), "], got ", n_decode, ".");
+  AveGdnArgs a = fill_args(q, k, v, g, beta, some(z), some(norm_weight), norm_eps, out, scale, &state_pool, &state_pool, &cu_seqlens, &state_indices,
+                           state_pool.size(0), n, l2norm);
+  if (n_decode > 0) {  // one single-token sequence per row: the token stride becomes the batch stride
     AveGdnArgs d = a;
-    d.B = d.n_seqs = (int32_t)nd;
+    d.B = d.n_seqs = (int32_t)n_decode;
     d.T = 1;
     d.cu_seqlens = nullptr;
     d.q_stride_b = a.q_stride_t; d.k_stride_b = a.k_stride_t; d.v_stride_b = a.v_stride_t; d.z_stride_b = a.z_stride_t;
     d.o_stride_b = a.o_stride_t; d.g_stride_b = a.g_stride_t;
     enqueue_decode(d, q);
   }
-  if (nd < s.n) {
-    a.cu_seqlens += nd;  // offsets stay absolute: the tables use differences, the tokens are addressed from the packed base
-    a.state_indices += nd;
-    a.n_seqs = (int32_t)(s.n - nd);
-    a.token_begin = (int32_t)nd;
+  if (n_decode < n) {
+    a.cu_seqlens += n_decode;  // offsets stay absolute: the tables use differences, the tokens are addressed from the packed base
+    a.state_indices += n_decode;
+    a.n_seqs = (int32_t)(n - n_decode);
+    a.token_begin = (int32_t)n_decode;
     enqueue_prefill(a, q);
   }
-  return wrap(o);
 }
 
-// decode_layer(proj, conv_weight, conv_state, A_log, dt_bias, state_pool, state_indices, Hk, Hv, conv_bias, norm_weight,
-//              norm_eps, scale, gate_first, out) -> o
-PyObject* decode_layer(PyObject* const* p) {
+// [rows, H, d] views
+void op_rmsnorm(const Tensor& x, const Tensor& z, const OptTensor& weight, double eps, bool gate_first, const Tensor& out) {
+  loaded();
+  AveGdnNormArgs a{};
+  a.struct_size = sizeof(a);
+  a.flags = gate_first ? AVE_GDN_FLAG_GATE_FIRST : 0;
+  a.x = x.data_ptr(); a.z = z.data_ptr(); a.y = out.data_ptr();
+  a.weight = ptr_as<float>(some(weight));
+  a.rows = x.size(0) * x.size(1); a.heads = (int32_t)x.size(1); a.d = (int32_t)x.size(2);
+  a.x_stride_t = x.stride(0); a.x_stride_h = x.stride(1);
+  a.z_stride_t = z.stride(0); a.z_stride_h = z.stride(1);
+  a.y_stride_t = out.stride(0); a.y_stride_h = out.stride(1);
+  a.eps = (float)eps;
+  Launch launch(x);
+  check(launch([&] { return api.gated_rmsnorm(&a, launch.stream); }), "gated_rmsnorm");
+}
+
+void op_conv(const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& cu_seqlens, const Tensor& out) {
+  loaded();
+  const Tensor* cu = some(cu_seqlens);
+  REQ(out.data_ptr() != x.data_ptr() || x.numel() == 0, "out must not alias x (later tokens read earlier inputs)");
+  AveConvArgs a{};
+  a.struct_size = sizeof(a);
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.y = out.data_ptr(); a.bias = ptr(some(bias));
+  a.B = (int32_t)x.size(0); a.T = (int32_t)x.size(1); a.C = (int32_t)x.size(2); a.width = (int32_t)w.size(1);
+  if (cu != nullptr) { a.cu_seqlens = reinterpret_cast<const int32_t*>(cu->data_ptr()); a.n_seqs = (int32_t)cu->numel() - 1; }
+  a.x_stride_b = x.stride(0); a.x_stride_t = x.stride(1); a.y_stride_b = out.stride(0); a.y_stride_t = out.stride(1);
+  Launch launch(x);
+  check(launch([&] { return api.conv1d_silu(&a, launch.stream); }), "causal_conv1d_silu");
+}
+
+void op_conv_update(const Tensor& x, const Tensor& conv_state, const Tensor& w, const OptTensor& bias, const OptTensor& state_indices, const Tensor& out) {
+  loaded();
+  AveConvUpdateArgs a{};
+  a.struct_size = sizeof(a);
+  a.x = x.data_ptr(); a.w = w.data_ptr(); a.y = out.data_ptr(); a.conv_state = conv_state.data_ptr(); a.bias = ptr(some(bias));
+  a.state_indices = ptr_as<int32_t>(some(state_indices));
+  a.n_seqs = (int32_t)x.size(0); a.C = (int32_t)x.size(1); a.width = (int32_t)w.size(1); a.num_slots = (int32_t)conv_state.size(0);
+  a.x_stride = x.stride(0); a.y_stride = out.stride(0);
+  a.status = reinterpret_cast<uint32_t*>(status_word(x.device()).data_ptr());
+  Launch launch(x);
+  check(launch([&] { return api.conv1d_update(&a, launch.stream); }), "causal_conv1d_update");
+}
+
+// a, b: [rows, Hv] views
+void op_gate(const Tensor& a, const Tensor& b, const Tensor& A_log, const Tensor& dt_bias, const Tensor& g, const Tensor& beta) {
+  loaded();
+  AveGateArgs s{};
+  s.struct_size = sizeof(s);
+  s.a = a.data_ptr(); s.b = b.data_ptr(); s.A_log = ptr_as<float>(&A_log); s.dt_bias = ptr_as<float>(&dt_bias);
+  s.g = ptr_as<float>(&g); s.beta = ptr_as<float>(&beta);
+  s.rows = a.size(0); s.Hv = (int32_t)a.size(1);
+  s.a_stride_row = a.stride(0); s.b_stride_row = b.stride(0);
+  Launch launch(a);
+  check(launch([&] { return api.gate_beta(&s, launch.stream); }), "gate_beta");
+}
+
+void op_gemm(const Tensor& A, const Tensor& B, const Tensor& out) {
+  loaded();
+  AveGemmArgs a{};
+  a.struct_size = sizeof(a);
+  a.a = A.data_ptr(); a.b = B.data_ptr(); a.c = out.data_ptr();
+  a.M = A.size(0); a.N = B.size(0); a.K = A.size(1);
+  a.lda = A.stride(0); a.ldb = B.stride(0); a.ldc = out.stride(0);
+  a.status = reinterpret_cast<uint32_t*>(status_word(A.device()).data_ptr());
+  Launch launch(A);
+  check(launch([&] { return api.gemm_bf16_nt(&a, launch.stream); }), "gemm_pipeline_transposed_b");
+}
+
+// The checks of a decode layer step, for the operator and the public function.
+void check_layer(const Tensor& proj, const Tensor& cw, const Tensor* cb, const Tensor& cs, const Tensor& A_log, const Tensor& dt_bias,
+                 const Tensor* w, const Tensor& pool, const Tensor* idx, int64_t Hk, int64_t Hv) {
   constexpr int64_t d = 128;
-  const Tensor &proj = tensor(p[0], "proj"), &cw = tensor(p[1], "conv_weight"), &cs = tensor(p[2], "conv_state"),
-               &pool = tensor(p[5], "state_pool");
-  const Tensor *idx = opt_tensor(p[6], "state_indices"), *cb = opt_tensor(p[9], "conv_bias"), *w = opt_tensor(p[10], "norm_weight"),
-               *out = opt_tensor(p[14], "out");
   REQ(proj.scalar_type() == at::kBFloat16 && proj.dim() == 2 && proj.is_cuda() && proj.stride(1) == 1,
       "proj must be a bf16 CUDA tensor [N, columns]");
-  const int64_t N = proj.size(0), Hk = integer(p[7]), Hv = integer(p[8]);
+  const int64_t N = proj.size(0);
   REQ(Hk > 0 && Hv > 0 && Hv % Hk == 0, "value heads (", Hv, ") must be a multiple of key heads (", Hk, ").");
   const int64_t Cn = 2 * Hk * d + Hv * d, cols = 2 * Hk * d + 2 * Hv * d + 2 * Hv;
   REQ(proj.size(1) >= cols, "proj must have at least ", cols, " columns, got ", proj.size(1), ".");
@@ -520,52 +573,181 @@ PyObject* decode_layer(PyObject* const* p) {
         "state_indices must be a contiguous int32 tensor (", N, ",) on ", proj.device());
   else
     REQ(pool.size(0) >= N, "the pools need one slot per sequence when state_indices is not given");
-  const Tensor A_log = f32(tensor(p[3], "A_log")), dt_bias = f32(tensor(p[4], "dt_bias"));
   REQ(A_log.numel() == Hv && dt_bias.numel() == Hv && A_log.device() == proj.device(), "A_log and dt_bias must have ", Hv, " elements on ",
       proj.device());
-  Tensor nw, bias;
-  if (w != nullptr) {
-    REQ(w->numel() == d && w->device() == proj.device(), "norm_weight must have ", d, " elements on ", proj.device());
-    nw = f32(*w);
-  }
-  if (cb != nullptr) {
+  if (w != nullptr) REQ(w->numel() == d && w->device() == proj.device(), "norm_weight must have ", d, " elements on ", proj.device());
+  if (cb != nullptr)
     REQ(cb->scalar_type() == at::kBFloat16 && cb->numel() == Cn && cb->device() == proj.device(), "conv_bias must be bf16 [", Cn, "]");
-    bias = cb->contiguous();
-  }
-  const Tensor o = out != nullptr ? *out : empty({N, Hv, d}, at::kBFloat16, proj);
-  REQ(o.dim() == 3 && o.size(0) == N && o.size(1) == Hv && o.size(2) == d && o.scalar_type() == at::kBFloat16 &&
-          o.device() == proj.device() && o.stride(2) == 1 && o.stride(1) == d,
+}
+
+void op_decode_layer(const Tensor& proj, const Tensor& conv_w, const OptTensor& conv_bias, const Tensor& conv_state, const Tensor& A_log_in,
+                     const Tensor& dt_bias_in, const OptTensor& norm_weight, const Tensor& state_pool, const OptTensor& state_indices,
+                     const Tensor& out, int64_t Hk, int64_t Hv, double scale, double norm_eps, bool gate_first) {
+  loaded();
+  constexpr int64_t d = 128;
+  const Tensor *cb = some(conv_bias), *w = some(norm_weight), *idx = some(state_indices);
+  check_layer(proj, conv_w, cb, conv_state, A_log_in, dt_bias_in, w, state_pool, idx, Hk, Hv);
+  const int64_t N = proj.size(0);
+  REQ(out.dim() == 3 && out.size(0) == N && out.size(1) == Hv && out.size(2) == d && out.scalar_type() == at::kBFloat16 &&
+          out.device() == proj.device() && out.stride(2) == 1 && out.stride(1) == d,
       "out must be a bf16 tensor (", N, ", ", Hv, ", ", d, ") with contiguous rows on ", proj.device());
-  const Tensor cwc = cw.contiguous();
+  const Tensor A_log = f32(A_log_in), dt_bias = f32(dt_bias_in), cw = conv_w.contiguous();
+  const Tensor nw = w != nullptr ? f32(*w) : Tensor(), bias = cb != nullptr ? cb->contiguous() : Tensor();
   AveGdnDecodeLayerArgs a{};
   a.struct_size = sizeof(a);
-  a.flags = truth(p[13]) ? AVE_GDN_FLAG_GATE_FIRST : 0;
-  a.proj = proj.data_ptr(); a.conv_w = cwc.data_ptr(); a.conv_bias = ptr(some(bias)); a.conv_state = cs.data_ptr();
+  a.flags = gate_first ? AVE_GDN_FLAG_GATE_FIRST : 0;
+  a.proj = proj.data_ptr(); a.conv_w = cw.data_ptr(); a.conv_bias = ptr(some(bias)); a.conv_state = conv_state.data_ptr();
   a.A_log = ptr_as<float>(&A_log); a.dt_bias = ptr_as<float>(&dt_bias); a.norm_weight = ptr_as<float>(some(nw));
-  a.state_pool = ptr_as<float>(&pool); a.state_indices = ptr_as<int32_t>(idx); a.o = o.data_ptr();
+  a.state_pool = ptr_as<float>(&state_pool); a.state_indices = ptr_as<int32_t>(idx); a.o = out.data_ptr();
   a.status = reinterpret_cast<uint32_t*>(status_word(proj.device()).data_ptr());
-  a.n_seqs = (int32_t)N; a.Hk = (int32_t)Hk; a.Hv = (int32_t)Hv; a.dk = a.dv = (int32_t)d; a.width = (int32_t)W;
-  a.num_slots = (int32_t)pool.size(0);
-  a.proj_stride = proj.stride(0); a.o_stride = o.stride(0);
-  a.norm_eps = (float)number(p[11]); a.scale = (float)scale_or(p[12], d);
+  a.n_seqs = (int32_t)N; a.Hk = (int32_t)Hk; a.Hv = (int32_t)Hv; a.dk = a.dv = (int32_t)d; a.width = (int32_t)cw.size(1);
+  a.num_slots = (int32_t)state_pool.size(0);
+  a.proj_stride = proj.stride(0); a.o_stride = out.stride(0);
+  a.norm_eps = (float)norm_eps; a.scale = (float)scale;
   Launch launch(proj);
   check(launch([&] { return api.decode_layer_step(&a, launch.stream); }), "decode_layer_step");
+}
+
+// dq, dk and dv: fp32 per value head, or all bf16 with dq and dk summed over the value heads of a key head; contiguous
+void op_backward(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& d_o, double scale,
+                 const OptTensor& initial_state, const OptTensor& d_final_state, const OptTensor& cu_seqlens, const Tensor& dq, const Tensor& dk,
+                 const Tensor& dv, const Tensor& dg, const Tensor& dbeta, const OptTensor& d_initial_state) {
+  loaded();
+  const bool summed = dq.scalar_type() == at::kBFloat16;
+  const at::ScalarType dt = summed ? at::kBFloat16 : at::kFloat;
+  REQ(dq.scalar_type() == dt && dk.scalar_type() == dt && dv.scalar_type() == dt, "dq, dk and dv must be all fp32 or all bf16");
+  const Tensor *s0 = some(initial_state), *ds = some(d_final_state), *cu = some(cu_seqlens), *ds0 = some(d_initial_state);
+  AveGdnBwdArgs a{};
+  a.struct_size = sizeof(a);
+  a.flags = summed ? AVE_GDN_FLAG_BWD_SUMMED : 0;
+  a.q = ptr(&q); a.k = ptr(&k); a.v = ptr(&v); a.g = ptr_as<float>(&g); a.beta = ptr_as<float>(&beta); a.d_o = ptr(&d_o);
+  a.initial_state = ptr_as<float>(s0); a.d_final_state = ptr_as<float>(ds); a.cu_seqlens = ptr_as<int32_t>(cu);
+  a.d_q = ptr_as<float>(&dq); a.d_k = ptr_as<float>(&dk); a.d_v = ptr_as<float>(&dv);
+  a.d_g = ptr_as<float>(&dg); a.d_beta = ptr_as<float>(&dbeta); a.d_initial_state = ptr_as<float>(ds0);
+  a.status = reinterpret_cast<uint32_t*>(status_word(q.device()).data_ptr());
+  a.B = (int32_t)q.size(0); a.T = (int32_t)q.size(1); a.Hk = (int32_t)q.size(2); a.Hv = (int32_t)v.size(2);
+  a.dk = (int32_t)q.size(3); a.dv = (int32_t)v.size(3);
+  a.n_seqs = (int32_t)(cu != nullptr ? cu->numel() - 1 : q.size(0));
+  STRIDES4(a, q, q); STRIDES4(a, k, k); STRIDES4(a, v, v); STRIDES4(a, do, d_o);
+  a.g_stride_b = g.stride(0); a.g_stride_t = g.stride(1); a.scale = (float)scale;
+  Launch launch(q);
+  // Scratch for all key heads at once; where that does not fit, for half of them, a quarter, ...: the call then takes as many
+  // passes.  (Two sequences of 4096 tokens, 32 value heads: 0.82 ms in one pass of 1.03 GB, 1.12 in two, 1.78 in four: with half
+  // the heads the scans use half the SMs.)
+  std::optional<Scratch> ws;
+  for (int heads = a.Hk;; heads = (heads + 1) / 2) {
+    AveGdnBwdArgs part = a;
+    part.Hk = heads; part.Hv = a.Hk > 0 ? heads * (a.Hv / a.Hk) : a.Hv;
+    try {
+      ws.emplace(q, launch.stream, api.backward_workspace_bytes(&part));
+      break;
+    } catch (const c10::OutOfMemoryError&) {
+      if (heads <= 1) throw;
+    }
+  }
+  a.workspace = ws->data(); a.workspace_bytes = ws->size();
+  check(launch([&] { return api.recurrent_backward(&a, launch.stream); }), "gated_delta_rule_backward");
+}
+
+#define OPERATORS(X)                                                                                                        \
+  X("chunk_prefill", op_prefill) X("decode_step", op_decode) X("mixed_step", op_mixed) X("decode_layer_step", op_decode_layer) \
+  X("gated_rmsnorm", op_rmsnorm) X("conv1d_silu", op_conv) X("conv1d_update", op_conv_update) X("gate_beta", op_gate)          \
+  X("gemm_bf16_nt", op_gemm) X("recurrent_backward", op_backward)
+TORCH_LIBRARY_IMPL(avelang_gdn, CUDA, m) {
+#define CUDA_KERNEL(name, f) m.impl(name, f);
+  OPERATORS(CUDA_KERNEL)
+}
+// The operators return nothing and write into what they are given, so torch's stand-in for a missing autograd kernel, which
+// goes through a boxed call (0.4 us), has nothing to do for them.
+TORCH_LIBRARY_IMPL(avelang_gdn, Autograd, m) {
+#define NO_AUTOGRAD(name, f) m.impl(name, torch::CppFunction::makeFallthrough());
+  OPERATORS(NO_AUTOGRAD)
+}
+
+double scale_or(PyObject* o, int64_t dk) { return o == Py_None ? 1.0 / std::sqrt((double)dk) : number(o); }
+
+// ---------------------------------------------------------------------------------------------- public functions
+// The operator F, through the dispatcher.
+template <auto F, class... Args>
+void call(const char* name, Args&&... args) {
+  static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow(name, "").typed<std::remove_pointer_t<decltype(F)>>();
+  op.call(std::forward<Args>(args)...);
+}
+
+// prefill(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm, cu_seqlens, z, norm_weight, norm_eps,
+//         state_indices, inplace_state, chunk_size, out, out_peers, max_seqlen) -> (o, final or None)
+PyObject* prefill(PyObject* const* p) {
+  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
+  const Tensor *s0 = opt_tensor(p[6], "initial_state"), *cu = opt_tensor(p[9], "cu_seqlens"), *z = opt_tensor(p[10], "z"),
+               *w = opt_tensor(p[11], "norm_weight"), *idx = opt_tensor(p[13], "state_indices"), *out = opt_tensor(p[16], "out"),
+               *peers = opt_tensor(p[17], "out_peers");
+  const Shape s = check_common(q, k, v, g, beta, z, cu);
+  const int64_t chunk = integer(p[15]);
+  REQ(chunk == 64, "chunk_size must be 64, got ", chunk, ".");
+  int64_t bound = 0;
+  if (p[18] != Py_None) {
+    const int64_t m = integer(p[18]);
+    REQ(m >= 0, "max_seqlen must be non-negative, got ", m, ".");
+    if (cu != nullptr) bound = std::min(m, s.T);
+  }
+  const Tensor o = prep_out(out, v);
+  const Tensor nw = prep_norm_weight(w, z, s, q.device());
+  const Tensor final = prep_states(s0, idx, s, q, truth(p[7]), truth(p[14]));
+  if (peers != nullptr) {
+    REQ(z != nullptr, "out_peers needs z (the stores are fused into the gated norm)");
+    REQ(peers->scalar_type() == at::kLong && peers->dim() == 1 && peers->device() == q.device() && peers->is_contiguous(),
+        "out_peers must be a contiguous 1-D int64 tensor on ", q.device());
+  }
+  call<op_prefill>("avelang_gdn::chunk_prefill", q, k, v, g, beta, o, scale_or(p[5], s.dk), opt(s0), opt(final), opt(cu), opt(idx), opt(z), opt(nw),
+                   number(p[12]), truth(p[8]), bound, opt(peers));
+  return wrap_pair(o, final);
+}
+
+// decode(q, k, v, g, beta, scale, initial_state, output_final_state, l2norm, cu_seqlens, state_indices, inplace_state, z,
+//        norm_weight, norm_eps, out) -> (o, final or None)
+PyObject* decode(PyObject* const* p) {
+  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
+  const Tensor *s0 = opt_tensor(p[6], "initial_state"), *cu = opt_tensor(p[9], "cu_seqlens"), *idx = opt_tensor(p[10], "state_indices"),
+               *z = opt_tensor(p[12], "z"), *w = opt_tensor(p[13], "norm_weight"), *out = opt_tensor(p[15], "out");
+  const Shape s = check_common(q, k, v, g, beta, z, cu);
+  const Tensor o = prep_out(out, v);
+  const Tensor nw = prep_norm_weight(w, z, s, q.device());
+  const Tensor final = prep_states(s0, idx, s, q, truth(p[7]), truth(p[11]));
+  call<op_decode>("avelang_gdn::decode_step", q, k, v, g, beta, o, scale_or(p[5], s.dk), opt(s0), opt(final), opt(cu), opt(idx), opt(z), opt(nw),
+                  number(p[14]), truth(p[8]));
+  return wrap_pair(o, final);
+}
+
+// mixed(q, k, v, g, beta, cu_seqlens, n_decode, state_pool, state_indices, scale, l2norm, z, norm_weight, norm_eps, out) -> o
+PyObject* mixed(PyObject* const* p) {
+  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta");
+  const Tensor *cu = opt_tensor(p[5], "cu_seqlens"), *pool = opt_tensor(p[7], "state_pool"), *idx = opt_tensor(p[8], "state_indices"),
+               *z = opt_tensor(p[11], "z"), *w = opt_tensor(p[12], "norm_weight"), *out = opt_tensor(p[14], "out");
+  const Shape s = check_common(q, k, v, g, beta, z, cu);
+  REQ(cu != nullptr && s.B == 1, "mixed_prefill_decode_step takes a packed batch: B == 1 with cu_seqlens");
+  const int64_t nd = integer(p[6]);
+  REQ(nd >= 0 && nd <= s.n && nd <= s.T, "n_decode must lie in [0, ", std::min(s.n, s.T), "], got ", nd, ".");
+  REQ(pool != nullptr && idx != nullptr, "mixed_prefill_decode_step needs state_pool and state_indices");
+  const Tensor o = prep_out(out, v);
+  const Tensor nw = prep_norm_weight(w, z, s, q.device());
+  prep_states(pool, idx, s, q, true, true);  // its checks
+  call<op_mixed>("avelang_gdn::mixed_step", q, k, v, g, beta, o, scale_or(p[9], s.dk), *pool, *cu, *idx, nd, opt(z), opt(nw), number(p[13]), truth(p[10]));
   return wrap(o);
 }
 
-void enqueue_rmsnorm(const Tensor& x, const Tensor& z, const Tensor* w, double eps, bool gate_first, const Tensor& y) {
-  AveGdnNormArgs a{};
-  a.struct_size = sizeof(a);
-  a.flags = gate_first ? AVE_GDN_FLAG_GATE_FIRST : 0;
-  a.x = x.data_ptr(); a.z = z.data_ptr(); a.y = y.data_ptr();
-  a.weight = ptr_as<float>(w);
-  a.rows = x.size(0) * x.size(1); a.heads = (int32_t)x.size(1); a.d = (int32_t)x.size(2);
-  a.x_stride_t = x.stride(0); a.x_stride_h = x.stride(1);
-  a.z_stride_t = z.stride(0); a.z_stride_h = z.stride(1);
-  a.y_stride_t = y.stride(0); a.y_stride_h = y.stride(1);
-  a.eps = (float)eps;
-  Launch launch(x);
-  check(launch([&] { return api.gated_rmsnorm(&a, launch.stream); }), "gated_rmsnorm");
+// decode_layer(proj, conv_weight, conv_state, A_log, dt_bias, state_pool, state_indices, Hk, Hv, conv_bias, norm_weight,
+//              norm_eps, scale, gate_first, out) -> o
+PyObject* decode_layer(PyObject* const* p) {
+  const Tensor &proj = tensor(p[0], "proj"), &cw = tensor(p[1], "conv_weight"), &cs = tensor(p[2], "conv_state"), &A_log = tensor(p[3], "A_log"),
+               &dt_bias = tensor(p[4], "dt_bias"), &pool = tensor(p[5], "state_pool");
+  const Tensor *idx = opt_tensor(p[6], "state_indices"), *cb = opt_tensor(p[9], "conv_bias"), *w = opt_tensor(p[10], "norm_weight"),
+               *out = opt_tensor(p[14], "out");
+  const int64_t Hk = integer(p[7]), Hv = integer(p[8]);
+  check_layer(proj, cw, cb, cs, A_log, dt_bias, w, pool, idx, Hk, Hv);
+  const Tensor o = out != nullptr ? *out : empty({proj.size(0), Hv, 128}, at::kBFloat16, proj);
+  call<op_decode_layer>("avelang_gdn::decode_layer_step", proj, cw, opt(cb), cs, A_log, dt_bias, opt(w), pool, opt(idx), o, Hk, Hv, scale_or(p[12], 128),
+                        number(p[11]), truth(p[13]));
+  return wrap(o);
 }
 
 // rmsnorm(x, z, weight, eps, gate_first, out) -> out
@@ -584,26 +766,15 @@ PyObject* rmsnorm(PyObject* const* p) {
       shape_of(x.sizes()), " on ", x.device());
   const auto rows = [&](const Tensor& t) { return t.dim() == 3 ? t : t.reshape({-1, H, d}); };
   const Tensor x3 = rows(x), z3 = rows(z), y3 = rows(y);
-  REQ(y3.data_ptr() == y.data_ptr(), "out must be viewable as [rows, H, d] without a copy");
+  REQ(y3.is_alias_of(y), "out must be viewable as [rows, H, d] without a copy");
   REQ(x3.stride(2) == 1 && z3.stride(2) == 1 && y3.stride(2) == 1, "tensors must be contiguous in their last dimension");
   Tensor nw;
   if (w != nullptr) {
     REQ(w->numel() == d && w->device() == x.device(), "weight must have ", d, " elements on ", x.device());
     nw = f32(*w);
   }
-  enqueue_rmsnorm(x3, z3, some(nw), number(p[3]), truth(p[4]), y3);
+  call<op_rmsnorm>("avelang_gdn::gated_rmsnorm", x3, z3, opt(nw), number(p[3]), truth(p[4]), y3);
   return wrap(y);
-}
-
-void enqueue_conv(const Tensor& x, const Tensor& w, const Tensor* bias, const Tensor* cu, const Tensor& y) {
-  AveConvArgs a{};
-  a.struct_size = sizeof(a);
-  a.x = x.data_ptr(); a.w = w.data_ptr(); a.y = y.data_ptr(); a.bias = ptr(bias);
-  a.B = (int32_t)x.size(0); a.T = (int32_t)x.size(1); a.C = (int32_t)x.size(2); a.width = (int32_t)w.size(1);
-  if (cu != nullptr) { a.cu_seqlens = reinterpret_cast<const int32_t*>(cu->data_ptr()); a.n_seqs = (int32_t)cu->numel() - 1; }
-  a.x_stride_b = x.stride(0); a.x_stride_t = x.stride(1); a.y_stride_b = y.stride(0); a.y_stride_t = y.stride(1);
-  Launch launch(x);
-  check(launch([&] { return api.conv1d_silu(&a, launch.stream); }), "causal_conv1d_silu");
 }
 
 // conv(x, weight, bias, cu_seqlens, out) -> out
@@ -626,24 +797,12 @@ PyObject* conv(PyObject* const* p) {
   const Tensor y = out != nullptr ? *out : empty(x.sizes(), at::kBFloat16, x);
   REQ(y.sizes() == x.sizes() && y.scalar_type() == at::kBFloat16 && y.device() == x.device() && y.stride(2) == 1,
       "out must be a bf16 tensor of shape ", shape_of(x.sizes()), " on ", x.device());
-  REQ(y.data_ptr() != x.data_ptr() || x.numel() == 0, "out must not alias x (later tokens read earlier inputs)");
+  REQ(!y.is_alias_of(x) || y.storage_offset() != x.storage_offset() || x.numel() == 0, "out must not alias x (later tokens read earlier inputs)");
   if (cu != nullptr)
     REQ(x.size(0) == 1 && cu->scalar_type() == at::kInt && cu->device() == x.device() && cu->is_contiguous(),
         "cu_seqlens must be a contiguous int32 tensor on the device of x, with B == 1");
-  enqueue_conv(x, wc, some(bc), cu, y);
+  call<op_conv>("avelang_gdn::conv1d_silu", x, wc, opt(bc), opt(cu), y);
   return wrap(y);
-}
-
-void enqueue_conv_update(const Tensor& x, const Tensor& cs, const Tensor& w, const Tensor* bias, const Tensor* idx, const Tensor& y) {
-  AveConvUpdateArgs a{};
-  a.struct_size = sizeof(a);
-  a.x = x.data_ptr(); a.w = w.data_ptr(); a.y = y.data_ptr(); a.conv_state = cs.data_ptr(); a.bias = ptr(bias);
-  a.state_indices = ptr_as<int32_t>(idx);
-  a.n_seqs = (int32_t)x.size(0); a.C = (int32_t)x.size(1); a.width = (int32_t)w.size(1); a.num_slots = (int32_t)cs.size(0);
-  a.x_stride = x.stride(0); a.y_stride = y.stride(0);
-  a.status = reinterpret_cast<uint32_t*>(status_word(x.device()).data_ptr());
-  Launch launch(x);
-  check(launch([&] { return api.conv1d_update(&a, launch.stream); }), "causal_conv1d_update");
 }
 
 // conv_update(x, conv_state, weight, bias, state_indices, out) -> out
@@ -668,19 +827,8 @@ PyObject* conv_update(PyObject* const* p) {
   REQ(y.sizes() == x.sizes() && y.scalar_type() == at::kBFloat16 && y.device() == x.device() && y.stride(1) == 1,
       "out must be a bf16 tensor of shape ", shape_of(x.sizes()), " on ", x.device());
   const Tensor bc = bias != nullptr ? bias->contiguous() : Tensor();
-  enqueue_conv_update(x, cs, wc, some(bc), idx, y);
+  call<op_conv_update>("avelang_gdn::conv1d_update", x, cs, wc, opt(bc), opt(idx), y);
   return wrap(y);
-}
-
-void enqueue_gate(const Tensor& a2, const Tensor& b2, const Tensor& A_log, const Tensor& dt_bias, const Tensor& g, const Tensor& beta) {
-  AveGateArgs s{};
-  s.struct_size = sizeof(s);
-  s.a = a2.data_ptr(); s.b = b2.data_ptr(); s.A_log = ptr_as<float>(&A_log); s.dt_bias = ptr_as<float>(&dt_bias);
-  s.g = ptr_as<float>(&g); s.beta = ptr_as<float>(&beta);
-  s.rows = a2.size(0); s.Hv = (int32_t)a2.size(1);
-  s.a_stride_row = a2.stride(0); s.b_stride_row = b2.stride(0);
-  Launch launch(a2);
-  check(launch([&] { return api.gate_beta(&s, launch.stream); }), "gate_beta");
 }
 
 // gate(a, b, A_log, dt_bias) -> (g, beta)
@@ -690,23 +838,12 @@ PyObject* gate(PyObject* const* p) {
   REQ(a.dim() >= 1 && a.sizes() == b.sizes() && a.stride(-1) == 1 && b.stride(-1) == 1, "a and b must share a shape [..., Hv]");
   const int64_t Hv = a.size(-1);
   const Tensor a2 = a.dim() != 2 ? a.reshape({-1, Hv}) : a, b2 = b.dim() != 2 ? b.reshape({-1, Hv}) : b;
-  REQ(a2.data_ptr() == a.data_ptr() && b2.data_ptr() == b.data_ptr(), "a and b must be viewable as [rows, Hv]");
+  REQ(a2.is_alias_of(a) && b2.is_alias_of(b), "a and b must be viewable as [rows, Hv]");
   const Tensor A_log = f32(tensor(p[2], "A_log")), dt_bias = f32(tensor(p[3], "dt_bias"));
   REQ(A_log.numel() == Hv && dt_bias.numel() == Hv && A_log.device() == a.device(), "A_log and dt_bias must have ", Hv, " elements");
   const Tensor g = empty(a.sizes(), at::kFloat, a), beta = empty(a.sizes(), at::kFloat, a);
-  enqueue_gate(a2, b2, A_log, dt_bias, g, beta);
+  call<op_gate>("avelang_gdn::gate_beta", a2, b2, A_log, dt_bias, g, beta);
   return wrap_pair(g, beta);
-}
-
-void enqueue_gemm(const Tensor& A, const Tensor& B, const Tensor& out) {
-  AveGemmArgs a{};
-  a.struct_size = sizeof(a);
-  a.a = A.data_ptr(); a.b = B.data_ptr(); a.c = out.data_ptr();
-  a.M = A.size(0); a.N = B.size(0); a.K = A.size(1);
-  a.lda = A.stride(0); a.ldb = B.stride(0); a.ldc = out.stride(0);
-  a.status = reinterpret_cast<uint32_t*>(status_word(A.device()).data_ptr());
-  Launch launch(A);
-  check(launch([&] { return api.gemm_bf16_nt(&a, launch.stream); }), "gemm_pipeline_transposed_b");
 }
 
 // gemm(A, B, out) -> out
@@ -728,46 +865,8 @@ PyObject* gemm(PyObject* const* p) {
     REQ(out->stride(1) == 1, "out must be contiguous in its last dimension.");
   }
   const Tensor c = out != nullptr ? *out : empty({m, n}, at::kBFloat16, A);
-  enqueue_gemm(A, B, c);
+  call<op_gemm>("avelang_gdn::gemm_bf16_nt", A, B, c);
   return wrap(c);
-}
-
-AveGdnBwdArgs bwd_args(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, const Tensor& d_o,
-                       double scale, const Tensor* s0, const Tensor* ds, const Tensor* cu, const Tensor& dq, const Tensor& dk,
-                       const Tensor& dv, const Tensor& dg, const Tensor& dbeta, const Tensor* ds0, uint32_t flags) {
-  AveGdnBwdArgs a{};
-  a.struct_size = sizeof(a);
-  a.flags = flags;
-  a.q = ptr(&q); a.k = ptr(&k); a.v = ptr(&v); a.g = ptr_as<float>(&g); a.beta = ptr_as<float>(&beta); a.d_o = ptr(&d_o);
-  a.initial_state = ptr_as<float>(s0); a.d_final_state = ptr_as<float>(ds); a.cu_seqlens = ptr_as<int32_t>(cu);
-  a.d_q = ptr_as<float>(&dq); a.d_k = ptr_as<float>(&dk); a.d_v = ptr_as<float>(&dv);
-  a.d_g = ptr_as<float>(&dg); a.d_beta = ptr_as<float>(&dbeta); a.d_initial_state = ptr_as<float>(ds0);
-  a.status = reinterpret_cast<uint32_t*>(status_word(q.device()).data_ptr());
-  a.B = (int32_t)q.size(0); a.T = (int32_t)q.size(1); a.Hk = (int32_t)q.size(2); a.Hv = (int32_t)v.size(2);
-  a.dk = (int32_t)q.size(3); a.dv = (int32_t)v.size(3);
-  a.n_seqs = (int32_t)(cu != nullptr ? cu->numel() - 1 : q.size(0));
-  STRIDES4(a, q, q); STRIDES4(a, k, k); STRIDES4(a, v, v); STRIDES4(a, do, d_o);
-  a.g_stride_b = g.stride(0); a.g_stride_t = g.stride(1); a.scale = (float)scale;
-  return a;
-}
-void enqueue_backward(AveGdnBwdArgs& a, const Tensor& q) {
-  Launch launch(q);
-  // Scratch for all key heads at once; where that does not fit, for half of them, a quarter, ...: the call then takes as many
-  // passes.  (Two sequences of 4096 tokens, 32 value heads: 0.82 ms
-  // in one pass of 1.03 GB, 1.12 in two, 1.78 in four: half the heads leave half the SMs to the scans.)
-  std::optional<Scratch> ws;
-  for (int heads = a.Hk;; heads = (heads + 1) / 2) {
-    AveGdnBwdArgs part = a;
-    part.Hk = heads; part.Hv = a.Hk > 0 ? heads * (a.Hv / a.Hk) : a.Hv;
-    try {
-      ws.emplace(q, launch.stream, api.backward_workspace_bytes(&part));
-      break;
-    } catch (const c10::OutOfMemoryError&) {
-      if (heads <= 1) throw;
-    }
-  }
-  a.workspace = ws->data(); a.workspace_bytes = ws->size();
-  check(launch([&] { return api.recurrent_backward(&a, launch.stream); }), "gated_delta_rule_backward");
 }
 
 // backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens) -> (dq, dk, dv, dg, dbeta, ds0 or None)
@@ -788,8 +887,7 @@ PyObject* backward(PyObject* const* p) {
   const Tensor dq = empty(q.sizes(), at::kBFloat16, q), dk = empty(q.sizes(), at::kBFloat16, q), dv = empty(v.sizes(), at::kBFloat16, v);
   const Tensor dg = empty(g.sizes(), at::kFloat, q), dbeta = empty(g.sizes(), at::kFloat, q);
   const Tensor ds0 = s0 != nullptr ? empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, q) : Tensor();
-  AveGdnBwdArgs a = bwd_args(q, k, v, g, beta, d_o, scale_or(p[6], s.dk), s0, ds, cu, dq, dk, dv, dg, dbeta, some(ds0), AVE_GDN_FLAG_BWD_SUMMED);
-  enqueue_backward(a, q);
+  call<op_backward>("avelang_gdn::recurrent_backward", q, k, v, g, beta, d_o, scale_or(p[6], s.dk), opt(s0), opt(ds), opt(cu), dq, dk, dv, dg, dbeta, opt(ds0));
   PyObject* r = PyTuple_New(6);
   if (r == nullptr) throw python_error();
   const Tensor* out[] = {&dq, &dk, &dv, &dg, &dbeta, &ds0};
@@ -800,76 +898,7 @@ PyObject* backward(PyObject* const* p) {
   return r;
 }
 
-// ---------------------------------------------------------------------------------------------- torch.ops.avelang_gdn.*
-// The operators take tensors the caller has laid out; the library checks what they pass on.
-int64_t n_sequences(const Tensor& q, const Tensor* cu) { return cu != nullptr ? cu->numel() - 1 : q.size(0); }
-int64_t n_slots(const Tensor* s0, const Tensor* final, int64_t n) {
-  const Tensor* pool = final != nullptr ? final : s0;
-  return pool != nullptr ? pool->size(0) : n;
-}
 PyObject* none() { Py_RETURN_NONE; }
-
-// op_prefill(q, k, v, g, beta, out, scale, initial_state, final_state, cu_seqlens, state_indices, z, norm_weight, norm_eps,
-//            qk_l2norm, max_seqlen, out_peers)
-PyObject* op_prefill(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta"),
-               &o = tensor(p[5], "out");
-  const Tensor *s0 = opt_tensor(p[7], "initial_state"), *sf = opt_tensor(p[8], "final_state"), *cu = opt_tensor(p[9], "cu_seqlens"),
-               *idx = opt_tensor(p[10], "state_indices"), *z = opt_tensor(p[11], "z"), *w = opt_tensor(p[12], "norm_weight"),
-               *peers = opt_tensor(p[16], "out_peers");
-  const int64_t n = n_sequences(q, cu);
-  AveGdnArgs a = fill_args(q, k, v, g, beta, z, w, number(p[13]), o, number(p[6]), s0, sf, cu, idx, n_slots(s0, sf, n), n, truth(p[14]));
-  a.max_seqlen = (int32_t)integer(p[15]);
-  if (peers != nullptr) { a.o_peers = reinterpret_cast<const void* const*>(peers->data_ptr()); a.n_peers = (int32_t)peers->numel(); }
-  enqueue_prefill(a, q);
-  return none();
-}
-// op_decode(q, k, v, g, beta, out, scale, initial_state, final_state, cu_seqlens, state_indices, z, norm_weight, norm_eps, qk_l2norm)
-PyObject* op_decode(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q"), &k = tensor(p[1], "k"), &v = tensor(p[2], "v"), &g = tensor(p[3], "g"), &beta = tensor(p[4], "beta"),
-               &o = tensor(p[5], "out");
-  const Tensor *s0 = opt_tensor(p[7], "initial_state"), *sf = opt_tensor(p[8], "final_state"), *cu = opt_tensor(p[9], "cu_seqlens"),
-               *idx = opt_tensor(p[10], "state_indices"), *z = opt_tensor(p[11], "z"), *w = opt_tensor(p[12], "norm_weight");
-  const int64_t n = n_sequences(q, cu);
-  AveGdnArgs a = fill_args(q, k, v, g, beta, z, w, number(p[13]), o, number(p[6]), s0, sf, cu, idx, n_slots(s0, sf, n), n, truth(p[14]));
-  enqueue_decode(a, q);
-  return none();
-}
-// op_rmsnorm(x, z, weight, eps, gate_first, out): [rows, H, d] views
-PyObject* op_rmsnorm(PyObject* const* p) {
-  enqueue_rmsnorm(tensor(p[0], "x"), tensor(p[1], "z"), opt_tensor(p[2], "weight"), number(p[3]), truth(p[4]), tensor(p[5], "out"));
-  return none();
-}
-PyObject* op_conv(PyObject* const* p) {
-  enqueue_conv(tensor(p[0], "x"), tensor(p[1], "weight"), opt_tensor(p[2], "bias"), opt_tensor(p[3], "cu_seqlens"), tensor(p[4], "out"));
-  return none();
-}
-PyObject* op_conv_update(PyObject* const* p) {
-  enqueue_conv_update(tensor(p[0], "x"), tensor(p[1], "conv_state"), tensor(p[2], "weight"), opt_tensor(p[3], "bias"),
-                      opt_tensor(p[4], "state_indices"), tensor(p[5], "out"));
-  return none();
-}
-PyObject* op_gate(PyObject* const* p) {
-  enqueue_gate(tensor(p[0], "a"), tensor(p[1], "b"), tensor(p[2], "A_log"), tensor(p[3], "dt_bias"), tensor(p[4], "g"), tensor(p[5], "beta"));
-  return none();
-}
-PyObject* op_gemm(PyObject* const* p) {
-  enqueue_gemm(tensor(p[0], "A"), tensor(p[1], "B"), tensor(p[2], "out"));
-  return none();
-}
-
-// op_backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens, dq, dk, dv, dg, dbeta, d_initial_state): dq, dk
-// and dv in fp32 per value head, contiguous
-PyObject* op_backward(PyObject* const* p) {
-  const Tensor &q = tensor(p[0], "q");
-  AveGdnBwdArgs a = bwd_args(q, tensor(p[1], "k"), tensor(p[2], "v"), tensor(p[3], "g"), tensor(p[4], "beta"), tensor(p[5], "d_o"), number(p[6]),
-                             opt_tensor(p[7], "initial_state"), opt_tensor(p[8], "d_final_state"), opt_tensor(p[9], "cu_seqlens"),
-                             tensor(p[10], "dq"), tensor(p[11], "dk"), tensor(p[12], "dv"), tensor(p[13], "dg"), tensor(p[14], "dbeta"),
-                             opt_tensor(p[15], "d_initial_state"), 0);
-  enqueue_backward(a, q);
-  return none();
-}
-
 // status_word(device_index) -> the device status word; workspace-independent
 PyObject* py_status_word(PyObject* const* p) { return wrap(status_word(at::Device(at::kCUDA, (c10::DeviceIndex)integer(p[0])))); }
 
@@ -907,12 +936,7 @@ PyObject* entry(PyObject*, PyObject* const* args, Py_ssize_t n) {
     PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", N, n);
     return nullptr;
   }
-  try {
-    return F(args);
-  } catch (const BadArgument& e) {
-    PyErr_SetString(PyExc_ValueError, e.what.c_str());
-    return nullptr;
-  }
+  return F(args);
   END_HANDLE_TH_ERRORS
 }
 #define ENTRY(name, fn, n) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&entry<fn, n>)), METH_FASTCALL, nullptr}
@@ -930,14 +954,6 @@ PyMethodDef methods[] = {
     ENTRY("gate", gate, 4),
     ENTRY("gemm", gemm, 3),
     ENTRY("backward", backward, 10),
-    ENTRY("op_backward", op_backward, 16),
-    ENTRY("op_prefill", op_prefill, 17),
-    ENTRY("op_decode", op_decode, 15),
-    ENTRY("op_rmsnorm", op_rmsnorm, 6),
-    ENTRY("op_conv", op_conv, 5),
-    ENTRY("op_conv_update", op_conv_update, 6),
-    ENTRY("op_gate", op_gate, 6),
-    ENTRY("op_gemm", op_gemm, 3),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -21,12 +21,13 @@ import ctypes
 
 import torch
 
-from . import _lib, torch_ops
+from . import _lib, torch_ops  # noqa: F401  (torch_ops declares the operators the native functions call)
 
 __all__ = ["chunk_gated_delta_rule", "fused_recurrent_gated_delta_rule", "mixed_prefill_decode_step", "gated_rmsnorm",
            "causal_conv1d_silu", "causal_conv1d_update", "gate_beta", "decode_layer_step", "gated_delta_rule_backward", "GatedDeltaRuleFunction", "prefill_launch_count", "read_status"]
 
-_native = _lib.host  # checks, allocation and launch of every public function (csrc/host.cpp)
+_native = _lib.host  # checks and allocation of every public function, and the operators behind them (csrc/host.cpp)
+_lib.register_operators()
 
 
 def _status_word(device: torch.device) -> torch.Tensor:
@@ -67,12 +68,6 @@ def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, out
                            norm_weight, norm_eps, state_indices, inplace_state, chunk_size, out, out_peers, max_seqlen)
 
 
-@torch_ops.implement("chunk_prefill")
-def _chunk_prefill(*args):
-    """torch.ops.avelang_gdn.chunk_prefill -> ave_gdn_chunk_prefill on the current stream."""
-    _native.op_prefill(*args)
-
-
 def prefill_launch_count(q, k, v, *, z=None, cu_seqlens=None, max_seqlen=None, push=False) -> int:
     """Number of kernels one ``chunk_gated_delta_rule`` call on tensors of these shapes enqueues (``push``: with the
     fused all-gather).  Asked from the library, which derives it from the same schedule it launches."""
@@ -109,12 +104,6 @@ def fused_recurrent_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state
                           state_indices, inplace_state, z, norm_weight, norm_eps, out)
 
 
-@torch_ops.implement("decode_step")
-def _decode_step(*args):
-    """torch.ops.avelang_gdn.decode_step -> ave_gdn_decode_step on the current stream."""
-    _native.op_decode(*args)
-
-
 def mixed_prefill_decode_step(q, k, v, g, beta, cu_seqlens, n_decode, state_pool, state_indices, scale=None,
                               use_qk_l2norm_in_kernel=False, *, z=None, norm_weight=None, norm_eps=1e-6, out=None):
     """One continuous-batching step over a packed batch (``B == 1``) ordered decode-first: sequences ``[0, n_decode)``
@@ -135,13 +124,6 @@ def gated_delta_rule_backward(q, k, v, g, beta, d_o, scale=None, initial_state=N
     value heads sharing a key head are summed), dv in the dtype of v, dg, dbeta fp32, ``d_initial_state`` fp32 or None
     when no initial state was given.  Chunked like the forward pass (64 tokens), every fp32 operand carried to 24 bits."""
     return _native.backward(q, k, v, g, beta, d_o, scale, initial_state, d_final_state, cu_seqlens)
-
-
-@torch_ops.implement("recurrent_backward")
-def _recurrent_backward(*args):
-    """torch.ops.avelang_gdn.recurrent_backward -> ave_gdn_recurrent_backward on the current stream (dq, dk, dv in fp32 per
-    value head)."""
-    _native.op_backward(*args)
 
 
 class GatedDeltaRuleFunction(torch.autograd.Function):
@@ -177,24 +159,10 @@ def decode_layer_step(proj, conv_weight, conv_state, A_log, dt_bias, state_pool,
                                 norm_eps, scale, gate_first, out)
 
 
-@torch_ops.implement("decode_layer_step")
-def _decode_layer_step(proj, conv_w, conv_bias, conv_state, A_log, dt_bias, norm_weight, state_pool, state_indices, out, Hk, Hv,
-                       scale, norm_eps, gate_first):
-    """torch.ops.avelang_gdn.decode_layer_step -> ave_gdn_decode_layer_step on the current stream."""
-    _native.decode_layer(proj, conv_w, conv_state, A_log, dt_bias, state_pool, state_indices, Hk, Hv, conv_bias, norm_weight, norm_eps,
-                         scale, gate_first, out)
-
-
 def gated_rmsnorm(x, z, weight=None, eps=1e-6, *, gate_first=False, out=None):
     """``y = weight * x * rsqrt(mean(x^2) + eps) * silu(z)`` over the last dimension (64 or 128), bf16 in/out,
     fp32 math.  ``x``/``z``/``out``: ``[..., H, d]`` with a contiguous last dimension."""
     return _native.rmsnorm(x, z, weight, eps, gate_first, out)
-
-
-@torch_ops.implement("gated_rmsnorm")
-def _gated_rmsnorm(*args):
-    """torch.ops.avelang_gdn.gated_rmsnorm -> ave_gdn_gated_rmsnorm; tensors are [rows, H, d] views."""
-    _native.op_rmsnorm(*args)
 
 
 def causal_conv1d_silu(x, weight, bias=None, cu_seqlens=None, *, out=None):
@@ -205,12 +173,6 @@ def causal_conv1d_silu(x, weight, bias=None, cu_seqlens=None, *, out=None):
     return _native.conv(x, weight, bias, cu_seqlens, out)
 
 
-@torch_ops.implement("conv1d_silu")
-def _conv1d_silu(*args):
-    """torch.ops.avelang_gdn.conv1d_silu -> ave_gdn_conv1d_silu."""
-    _native.op_conv(*args)
-
-
 def causal_conv1d_update(x, conv_state, weight, bias=None, state_indices=None, *, out=None):
     """Decode-time step of ``causal_conv1d_silu``: ``x`` bf16 ``[N, C]`` (one new token per sequence), ``conv_state`` bf16
     ``[slots, W-1, C]`` holding each sequence's last W-1 inputs (oldest first), updated in place; optional int32
@@ -219,19 +181,7 @@ def causal_conv1d_update(x, conv_state, weight, bias=None, state_indices=None, *
     return _native.conv_update(x, conv_state, weight, bias, state_indices, out)
 
 
-@torch_ops.implement("conv1d_update")
-def _conv1d_update(*args):
-    """torch.ops.avelang_gdn.conv1d_update -> ave_gdn_conv1d_update (history updated in place)."""
-    _native.op_conv_update(*args)
-
-
 def gate_beta(a_in, b_in, A_log, dt_bias):
     """``g = -exp(A_log) * softplus(a + dt_bias)`` and ``beta = sigmoid(b)`` in fp32.  ``a_in``, ``b_in``: bf16
     ``[..., Hv]`` (last dimension contiguous, one common row stride); ``A_log``, ``dt_bias``: ``[Hv]``."""
     return _native.gate(a_in, b_in, A_log, dt_bias)
-
-
-@torch_ops.implement("gate_beta")
-def _gate_beta(*args):
-    """torch.ops.avelang_gdn.gate_beta -> ave_gdn_gate_beta; a, b are [rows, Hv] views."""
-    _native.op_gate(*args)

@@ -19,12 +19,6 @@ def gemm_pipeline_transposed_b(A: torch.Tensor, B: torch.Tensor, out: torch.Tens
     return gdn._native.gemm(A, B, out)
 
 
-@torch_ops.implement("gemm_bf16_nt")
-def _gemm_bf16_nt(*args):
-    """torch.ops.avelang_gdn.gemm_bf16_nt -> ave_gemm_bf16_nt on the current stream."""
-    gdn._native.op_gemm(*args)
-
-
 # ---------------------------------------------------------------- row-parallel linear with the cross-rank sum fused in
 def _reduce_args(stage, stage_peers, out_peers, rank, M, N, ldc, rows_per_owner):
     r = _lib.GemmReduceArgs()

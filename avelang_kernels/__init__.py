@@ -12,8 +12,9 @@ themselves (one implementation under two import paths); importing them registers
 operators through which every entry point reaches the C library."""
 import sys
 
-from avelang_b200 import gdn, gemm
+from avelang_b200 import _lib, gdn, gemm
 
+_lib.register_operators()
 sys.modules[__name__ + ".gdn"] = gdn
 sys.modules[__name__ + ".gemm"] = gemm
 
