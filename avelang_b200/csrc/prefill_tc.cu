@@ -1045,7 +1045,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
 
 // ------------------------------------------------------------------------------------------------ schedule and scratch
 constexpr int SEG_FIRST_DIV = 6;    // first range = 1/6 of the longest chain's chunks (64 heads, 4096 tokens: 290 us; 1/16: 328)
-constexpr int SEG_FIRST_DIV_PARTS = 4;  // with parts the chains are short and pass 1 is the critical resource
+constexpr int SEG_FIRST_DIV_PARTS = 4;  // with parts the chains are short (4 heads, 32768 tokens: 267 us against 277 with a sixth)
 constexpr int SEG_GROWTH_X4 = 12;   // each range 3x the one before (in quarters)
 constexpr int SEG_MAX = 8;
 constexpr int PART0_X4 = 4;         // length of part 0 in quarters of a later part's length
@@ -1085,17 +1085,20 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   // Parts: with few long chains most SMs idle while every chain walks its chunks one after the other.  Cutting the
   // sequences into S parts that run at the same time shortens the walk S-fold at the price of a second (transition)
   // chain per later part and one GEMM-shaped fix-up; S is the largest count whose 2S-1 chains per head still get an SM
-  // each.  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
+  // each, up to 16 (4 heads, 8192 / 16384 / 32768 tokens: 123 / 174 / 267 us, with at most 8 parts 128 / 194 / 314).  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
   // beside it.
   L.parts = 1;
   if (!plain && !push && max_chunks >= 32) {
     const int64_t per_head = (NUM_SMS / (heads_total > 0 ? heads_total : 1) + 1) / 2;  // chains per head that still get an SM each: 2S - 1
     int S = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
     while (S > 1 && max_chunks / S < 8) --S;  // a part of fewer chunks costs more in combine and fix-up than it saves
-    // Two parts take three chains a head: worth it while pass 1 keeps a third of the SMs (32 heads, 8192 tokens: 399 us
-    // against 433; 48 heads, 6000 tokens: 411 against 386).  4 / 8 / 16 heads at 32768 tokens: 285 / 437 / 778 us with up to
-    // 16 parts, 391 / 514 / 861 with up to 8 and a slower combine.
-    L.parts = S >= 3 || (S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3) ? S : 1;
+    // Two parts take three chains a head.  They pay while pass 1 keeps a third of the SMs and the chains are long enough for the
+    // fix-up, which with a gate also holds the later part's norms back.  32 chains, two parts against one, with a gate:
+    // 5120 tokens 275 us against 269, 7168 354 / 369, 8192 394 / 406, 32768 1438 / 1488; without: 3072 175 / 172,
+    // 4096 208 / 211, 8192 361 / 392, 32768 1225 / 1480.  More chains, with a gate: 36 at 8192 tokens 422 / 433 but at 16384
+    // 809 / 795, 40 461 / 438 and 873 / 822, 48 527 / 465 and 1006 / 900.
+    const bool two = S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64);
+    L.parts = S >= 3 || two ? S : 1;
   }
   L.part_begin[0] = 0;
   {
