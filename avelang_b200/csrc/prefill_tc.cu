@@ -759,8 +759,6 @@ __global__ void __launch_bounds__(256)
 part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int cb = blockIdx.x, h = blockIdx.y, n = blockIdx.z, tid = threadIdx.x;
-  pdl_trigger();
-  pdl_wait();
   if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
@@ -879,7 +877,6 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n = blockIdx.z / (plan.parts - 1), part = 1 + blockIdx.z % (plan.parts - 1);
-  pdl_wait();
   if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;

@@ -51,12 +51,6 @@ __device__ __forceinline__ void split_acc(const float (&c0)[4], const float (&c1
   split3(make_float2(c1[0], c1[1]), h[2], m[2], l[2]);
   split3(make_float2(c1[2], c1[3]), h[3], m[3], l[3]);
 }
-// d += (h + m + l) * b with b exact
-__device__ __forceinline__ void mma3(float (&d)[4], const uint32_t (&h)[4], const uint32_t (&m)[4], const uint32_t (&l)[4], uint32_t b0, uint32_t b1) {
-  mma_bf16(d, h, b0, b1);
-  mma_bf16(d, m, b0, b1);
-  mma_bf16(d, l, b0, b1);
-}
 // d += (ah + am + al) (bh + bm + bl), the terms below 2^-24 left out
 __device__ __forceinline__ void mma6(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&am)[4], const uint32_t (&al)[4],
                                      uint32_t bh0, uint32_t bh1, uint32_t bm0, uint32_t bm1, uint32_t bl0, uint32_t bl1) {
