@@ -13,8 +13,9 @@
 // accumulators scaled by beta e^b are the right operands of W^T.  fp32 operands enter as three bf16 terms (24 bits), the
 // last product as two, like the tiles themselves.  Off the diagonal blocks the gate factors into
 // e^{b_i - b_s} e^{b_s - b_j} with b_s the first gate of i's block (both exponents are <= 0), so 64 + 96 exponentials
-// serve all but the diagonal blocks.
-// 132 k (chunk, head) units of a packed batch: 3.02 ms, 7.8 k warp instructions a unit; the form that took one head per CTA
+// serve all but the diagonal blocks.  (Those take e^{b_i - b_j} element by element and drop the half above the diagonal, where
+// the exponent is positive.)
+// 132 k (chunk, head) units of a packed batch: 2.85 ms, 8.0 k warp instructions a unit; the form that took one head per CTA
 // through tcgen05 products and CTA barriers needed 12.4 k instructions and 3.84 ms.
 #pragma once
 #include "wyblocks.cuh"

@@ -745,15 +745,15 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
 // by the scan itself.  The steps are serial and everything behind them waits, so each is kept short: the next F lands in
 // shared memory by asynchronous copies while this one is multiplied (row pitch 132: 16-byte reads of eight rows meet eight
 // different bank groups), and a thread takes two rows, four columns and half of the contraction, which needs six 16-byte
-// reads for 32 multiply-adds.  Fifteen steps: 44 us, 55 us with one row a thread, scalar reads
-// and F staged through registers.
+// reads for 32 multiply-adds.
 constexpr int COMBINE_PITCH = 132;
 constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 4) * 8 * 4;  // (a gap of one row between the shares of the contraction)
 constexpr int COMBINE_STAGES = 3;
 constexpr size_t COMBINE_SMEM = COMBINE_STAGES * (size_t)COMBINE_F + 2 * COMBINE_CUR;
 // COLS columns a CTA: 8, or 4 while that still is one wave (its step is shorter, but F passes through twice as many SMs).
 // Bound by shared-memory reads and the issue of the copies, 2 us a step: 15 steps for 4 heads 30 us (42 us when the lanes of a
-// quarter warp read one row at four offsets of 128 bytes, 8 wavefronts a load).
+// quarter warp read one row at four offsets of 128 bytes, 8 wavefronts a load; 55 us with one row a thread, scalar reads and F
+// staged through registers).
 template <int COLS>
 __global__ void __launch_bounds__(256)
 part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {

@@ -36,7 +36,8 @@ def _status_word(device: torch.device) -> torch.Tensor:
 
 def read_status(device=None, reset: bool = True) -> int:
     """Device status word accumulated by earlier calls (synchronises).  Bits: 1 = a state index beyond the
-    pool, 2 = malformed cu_seqlens, 4 = a bounded device wait gave up.  The affected sequences were skipped."""
+    pool, 2 = malformed cu_seqlens, 4 = a bounded device wait gave up.  The affected sequences were skipped (with a
+    malformed cu_seqlens the whole batch of a prefill or backward call)."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     w = _status_word(device)
     val = int(w.item())

@@ -193,7 +193,7 @@ def bench_prefill(args, rank, world):
     cap = torch.cuda.Stream()
     cap.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(cap):
-        step()  # this stream's scratch exists before the capture
+        step()  # what a first call sets up exists before the capture
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph, stream=cap):
             step()
@@ -348,8 +348,8 @@ def bench_decode(steps=1000, warmup=20):
 
 
 def bench_backward(steps=2):
-    """The backward pass on the headline shape (B=1, T=8192, 32 value heads): the correct-first reverse sweep, timed so
-    that its distance from the forward pass is on record."""
+    """The backward pass (chunked, three launches) on the headline shape (B=1, T=8192, 32 value heads), timed so that its
+    distance from the forward pass is on record."""
     from avelang_b200 import gdn, synth
     g = synth.config1().to("cuda")
     d_o = torch.randn_like(g.v)
@@ -621,18 +621,7 @@ def bench_helpers(args):
 
     out = {"metric": "gdn_helper_kernels", "peaks": peaks, "gemm": [], "streaming": []}
     gen = torch.Generator(device="cuda").manual_seed(0)
-    for (m, n, k, what) in ((131072, 1544, 2048, "in-projection of one rank of eight"), (131072, 12352, 2048, "in-projection, one GPU"),
-                            (8192, 8192, 8192, "square")):
-        A = torch.randn(m, k, device="cuda", generator=gen).bfloat16()
-        B = (0.02 * torch.randn(n, k, device="cuda", generator=gen)).bfloat16()
-        C = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
-        ours = timed(lambda: gemm.gemm_pipeline_transposed_b(A, B, out=C))
-        ref = timed(lambda: torch.matmul(A, B.T, out=C))
-        fl = 2.0 * m * n * k
-        out["gemm"].append({"shape": [m, n, k], "what": what, "ms": ours, "tflops": fl / ours / 1e9, "cublas_ms": ref,
-                            "cublas_tflops": fl / ref / 1e9, "frac_of_cublas": ref / ours,
-                            "frac_of_measured_peak": fl / ours / 1e9 / peaks["bf16_tflops_sustained"]})
-        del A, B, C
+    # the streaming kernels first: behind seconds of GEMMs the clock is down and they read 15 to 20 % slower
     Bt, T, Cn = 4, 32768, 8192
     x = torch.randn(Bt, T, Cn, device="cuda", generator=gen).bfloat16()
     w = (torch.randn(Cn, 4, device="cuda", generator=gen) / 2).bfloat16()
@@ -657,6 +646,18 @@ def bench_helpers(args):
     by = rows * H * (2 + 2 + 4 + 4)
     out["streaming"].append({"kernel": "gate_beta_kernel", "shape": [rows, H], "ms": ms, "GBps": by / ms / 1e6,
                              "frac_of_measured_hbm": by / ms / 1e6 / peaks["hbm_gbs"], "bytes": by})
+    for (m, n, k, what) in ((131072, 1544, 2048, "in-projection of one rank of eight"), (131072, 12352, 2048, "in-projection, one GPU"),
+                            (8192, 8192, 8192, "square")):
+        A = torch.randn(m, k, device="cuda", generator=gen).bfloat16()
+        B = (0.02 * torch.randn(n, k, device="cuda", generator=gen)).bfloat16()
+        C = torch.empty(m, n, dtype=torch.bfloat16, device="cuda")
+        ours = timed(lambda: gemm.gemm_pipeline_transposed_b(A, B, out=C))
+        ref = timed(lambda: torch.matmul(A, B.T, out=C))
+        fl = 2.0 * m * n * k
+        out["gemm"].append({"shape": [m, n, k], "what": what, "ms": ours, "tflops": fl / ours / 1e9, "cublas_ms": ref,
+                            "cublas_tflops": fl / ref / 1e9, "frac_of_cublas": ref / ours,
+                            "frac_of_measured_peak": fl / ours / 1e9 / peaks["bf16_tflops_sustained"]})
+        del A, B, C
     print(json.dumps(out))
 
 
@@ -673,6 +674,21 @@ def profile_case(name: str):
         inp = synth.config1(T=2048).to("cuda")
         for _ in range(2):
             gdn.chunk_gated_delta_rule(inp.q, inp.k, inp.v, inp.g, inp.beta, output_final_state=True, z=inp.z)
+    elif name == "prefill8k":
+        inp = synth.config1().to("cuda")  # the headline shape: 0.3 GB of inputs, 0.5 GB of scratch
+        for _ in range(3):
+            gdn.chunk_gated_delta_rule(inp.q, inp.k, inp.v, inp.g, inp.beta, output_final_state=True, z=inp.z)
+    elif name == "d64":
+        inp = synth.make_inputs(1, 256, 4, 4, 64, 64, seed=0).to("cuda")  # the CPU-reference shape
+        for _ in range(3):
+            gdn.chunk_gated_delta_rule(inp.q, inp.k, inp.v, inp.g, inp.beta, output_final_state=True)
+    elif name == "proj64":
+        # the two projections of a decode layer step of 64 sequences (K split over clusters); weights rotate through more than L2
+        from avelang_b200 import gemm
+        for k, n, copies in ((2048, 2 * HK * D + 2 * HV * D + 2 * HV, 4), (HV * D, 2048, 10)):
+            A = torch.randn(64, k, device="cuda").bfloat16()
+            for W in [(0.02 * torch.randn(n, k, device="cuda")).bfloat16() for _ in range(copies)]:
+                gemm.gemm_pipeline_transposed_b(A, W)
     elif name == "varlen32k":
         # throughput regime in the small: 64 packed sequences, about 550 chunks x 32 heads, 1.5 GB of scratch
         inp = synth.config3(total=32768, lo=128, hi=2048).to("cuda")
@@ -720,7 +736,7 @@ def main():
     ap.add_argument("--workload", default="prefill", choices=["prefill", "varlen", "block", "helpers"],
                     help="prefill (default, the headline line), varlen (head-sharded packed prefill), block, or helpers "
                          "(GEMM, conv1d, norm and gate kernels timed alone on one GPU)")
-    ap.add_argument("--profile-case", default=None, choices=["decode", "prefill2048", "varlen32k", "parts8k", "gemm1544", "conv", "norm"],
+    ap.add_argument("--profile-case", default=None, choices=["decode", "prefill2048", "prefill8k", "varlen32k", "parts8k", "d64", "proj64", "gemm1544", "conv", "norm"],
                     help="run a small fixed case for a profiler capture and exit")
     args = ap.parse_args()
     if args.profile_case:
@@ -763,8 +779,8 @@ def main():
             "clocks": clocks}
     achieved = flops / (ms * 1e-3) / 1e12
     line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
-                        "frac": achieved / peaks["bf16_tflops"], "traffic": 469_767_936,
-                        "traffic_source": "profiles/prefill_config1_launch_list.md: DRAM bytes read + written by the four "
+                        "frac": achieved / peaks["bf16_tflops"], "traffic": 555_651_840,
+                        "traffic_source": "profiles/prefill_config1_launch_list.md: DRAM bytes read + written by the two "
                                           "chunk_scan launches of one step (the dominant kernel), ncu with its "
                                           "cache flush between kernels; algorithmic bytes of the step are in hbm_view",
                         "peak_source": peaks["source"] + " (burst)",

@@ -22,7 +22,8 @@
  *    per-device mutex (its schedule forks onto library-owned helper streams through events, and the record/wait pairs
  *    of two callers must not interleave); a small pool of helper-stream sets per device, picked by the caller's stream,
  *    lets prefills on different streams overlap on the GPU.  Calls that overlap on the GPU need their own scratch and
- *    outputs.
+ *    outputs, and calls from several threads their own scratch on one stream too: the launches of two backward passes, or
+ *    of two prefills with dk = 64, may interleave.
  *  - Data-dependent faults (a slot index outside the pool, a bounded device wait that ran out) cannot be
  *    seen by the host without a sync: the kernels skip the offending unit and OR a bit into the optional
  *    device word `status` (see AVE_GDN_DEV_*).

@@ -51,7 +51,7 @@ def test_value_heads_per_key_head(built_lib, checker, ratio):
 @pytest.mark.parametrize("ratio", [1, 2])
 def test_several_pairs_a_cta(built_lib, checker, ratio):
     """Twelve ragged sequences x 16 key heads: 500 pairs and more, three or four to a CTA.  Every sequence must come out as it does
-    alone, where no CTA has a second pair; the first, a middle and the last one are held against the checker."""
+    alone, where no CTA has a second pair; the first, a middle and the last one are held against the oracle."""
     from avelang_b200 import gdn
     O, _ = checker
     Hk, lens = 16, [130, 64, 1, 200, 65, 127, 190, 128, 63, 129, 256, 70]
