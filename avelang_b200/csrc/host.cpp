@@ -372,6 +372,7 @@ Tensor prep_states(const Tensor* s0, const Tensor* idx, const Shape& s, const Te
   Tensor final;
   if (want_final) {
     if (idx != nullptr) final = inplace ? *s0 : s0->clone();
+    else if (s.T == 0) final = s0 != nullptr ? s0->clone() : at::zeros({s.n, s.Hv, s.dk, s.dv}, like.options().dtype(at::kFloat));  // no kernel runs
     else final = empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, like);
   }
   return final;
@@ -886,7 +887,12 @@ PyObject* backward(PyObject* const* p) {
           name, " must be a contiguous fp32 tensor (", s.n, ", ", s.Hv, ", ", s.dk, ", ", s.dv, ") on ", q.device());
   const Tensor dq = empty(q.sizes(), at::kBFloat16, q), dk = empty(q.sizes(), at::kBFloat16, q), dv = empty(v.sizes(), at::kBFloat16, v);
   const Tensor dg = empty(g.sizes(), at::kFloat, q), dbeta = empty(g.sizes(), at::kFloat, q);
-  const Tensor ds0 = s0 != nullptr ? empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, q) : Tensor();
+  Tensor ds0;
+  if (s0 != nullptr) {
+    ds0 = empty({s.n, s.Hv, s.dk, s.dv}, at::kFloat, q);
+    if (s.T == 0 && ds != nullptr) ds0.copy_(*ds);  // no kernel runs: the gradient of the states passes through
+    else if (s.T == 0) ds0.zero_();
+  }
   call<op_backward>("avelang_gdn::recurrent_backward", q, k, v, g, beta, d_o, scale_or(p[6], s.dk), opt(s0), opt(ds), opt(cu), dq, dk, dv, dg, dbeta, opt(ds0));
   PyObject* r = PyTuple_New(6);
   if (r == nullptr) throw python_error();
