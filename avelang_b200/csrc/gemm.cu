@@ -44,7 +44,7 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
                     __nv_bfloat16* __restrict__ C, int64_t M, int64_t N, int64_t K, int64_t ldc, uint32_t* status, int bn,
                     const GemmScatter sc) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = tc::align1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
   uint64_t* full = bars;                 // [STAGES]
   uint64_t* empty = bars + STAGES;       // [STAGES]
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, __nv_bfloat16* __restrict__ C,
                    int64_t M, int64_t N, int64_t K, int64_t ldc, uint32_t* status, const SkinnyPlan plan, uint32_t tmem_cols) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = tc::align1024(smem_raw);
   __shared__ uint64_t full[SKINNY_STAGES], empty[SKINNY_STAGES], acc_full;
   __shared__ uint32_t tmem_slot;
   __shared__ volatile uint32_t abort_flag;

@@ -252,7 +252,7 @@ chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, c
                      float* carry, uint8_t* m0_pack, const int32_t* seq_order,
                      const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = tc::align1024(smem_raw);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
   uint64_t* full = bars;          // [2] W, Q, K and V tiles of the stage landed
   uint64_t* pfull = bars + 2;     // [2] P tiles and the scale vectors of the stage landed
@@ -867,7 +867,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1)
 part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* o_f32,
                    const uint8_t* qt_img, const uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* smem = tc::align1024(smem_raw);
   float* stage = reinterpret_cast<float*>(smem + FIN_STAGE);  // [128 tokens][FIN_PITCH] product rows
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FIN_BARS);
   uint64_t* b_bar = bars;
