@@ -1,0 +1,557 @@
+// Pass 2 of the chunked prefill: one CTA per chain walks its chunks with the state on chip, transposed (H = M^T, rows = d_v = TMEM
+// lanes) so that every MMA has M = 128:
+//     X^T  = kx H K^T                     (A = H hi/lo from TMEM, B = K tile, K-major)
+//     Vn^T = V^T Tu^T - X^T Tu^T          (A = V tile MN-major / X hi/lo from TMEM, B = Tu hi/lo, packed triangles)
+//     O^T  = qs H Q^T + Vn^T P^T          (A = H or Vn hi/lo from TMEM, B = Q or P hi/lo)
+//     H   <- decay H + Vd^T K             (A = Vd hi/lo from TMEM, B = K, MN-major), Vd_j = ks_j Vn_j
+// with kx_j = e^{b_j}, qs_i = scale e^{b_i}, ks_j = e^{b_C - b_j}, decay = e^{b_C}.  The fp32 state lives in the chain-epilogue threads'
+// registers; its bf16 hi/lo image is rewritten to TMEM every chunk.  Pass 1 could also hand over W = Tu diag(kx) K, which
+// makes Vn = U - H W one product: a hand-off less in a step, but W is twice as many bytes as everything else in a record and a third
+// of pass 1.  K itself is exact in bf16, so H K^T takes 16 MMAs where H W^T takes 24.  (262144 packed tokens x 32 heads: 5.75 ms with W,
+// 3.73 without; 8192 tokens 370 us / 344; 4 heads x 32768 254 / 215; 1024 63.4 / 60.6.)
+// A step takes 4.55 k cycles alone and with every SM streaming, of which the tensor pipe is busy 2.4 k: H K^T 0.85 k, X 0.65 k, its
+// product 0.65 k, Vd 0.4 k, the increment 1.1 k, the new state 0.7 k, each of them about a third hand-over (commit or arrival, wake-up,
+// first load).  The conversions are bound by the instructions of a scheduler (a pair of values into two bf16 terms takes 7 cycles of it).
+// O2 waits for the increment: side by side they shared the pipe and the increment came 200 cycles later; H K^T in columns of its own lets
+// O2 end beside the next step (5.0 -> 4.55 k cycles together).  Measured and dropped: the state a chunk behind the chain by
+// S(c+1) = decay H(c) K(c+1)^T + Vd(c) (K(c+1) K(c)^T)^T, with three splits of 16 epilogue warps (3.08, 3.52 and 4.48 ms where this
+// form then took 2.73: 11 to 15 k instructions a chunk, and the code of 20 warps misses the instruction cache); the gated norm in
+// the output warps (layer of 8192 tokens 344 -> 374 us with eight of them, 422 with four).
+#pragma once
+
+namespace ave {
+namespace {
+
+// Warpgroup 0: warp 0 loader, warps 1 and 2 MMA issuers; warpgroups 1..NG: chain epilogue, each covering all 128 TMEM
+// lanes and 1/NG of the columns; the last warpgroup: output.  (Four epilogue groups at 80 registers were measured: no
+// faster, the epilogue is bound by the instructions issued per scheduler, not by the work per thread.)
+constexpr int NG = 2;
+constexpr int SCAN_THREADS = 32 * (4 + 4 * NG + 4);
+constexpr int REGS_LAUNCH = 128;
+constexpr int REGS_CTRL = 72, REGS_CHAIN = 168, REGS_OUT = 104;
+static_assert(NG == 2, "the register split below is for two epilogue groups");
+static_assert(REGS_CTRL + NG * REGS_CHAIN + REGS_OUT <= (NG + 2) * REGS_LAUNCH, "register redistribution exceeds the launch allocation");
+static_assert(SCAN_THREADS * REGS_LAUNCH <= 65536, "launch allocation exceeds the register file");
+constexpr int HC = D / NG;   // columns of H (d_k) per chain-epilogue group
+constexpr int VC = C / NG;   // columns of Vn (tokens) per group
+constexpr size_t SCAN_SMEM_MAX = 232448;
+// A stage of the ring: the Q, K and V tiles of a chunk and its record
+constexpr int CS_Q = 0, CS_K = 16384, CS_V = 32768, CS_REC = 49152, CS_STAGE = CS_REC + REC_BYTES, CS_STAGES = 3;
+constexpr int CS_BARS = CS_STAGES * CS_STAGE;
+constexpr size_t SCAN_SMEM = CS_BARS + 256 + 1024;
+static_assert(CS_STAGE % 1024 == 0, "swizzled tiles need 1024-byte alignment");
+static_assert(SCAN_SMEM <= SCAN_SMEM_MAX, "shared memory of an SM");
+// TMEM columns: hi and lo image of H, accumulator of Vn (then the images of Vd), images of Vn, outputs, state increment.  H K^T
+// and the images of X take columns of the increment, which they are never alive beside.
+constexpr uint32_t TC_HHI = 0, TC_HLO = 64, TC_VN = 128, TC_VI = 192, TC_O1 = 256, TC_O2 = 320, TC_DH = 384, TC_X = TC_DH;
+// The bf16 hi and lo images of an accumulator of 64 tokens reuse its columns.  Each chain-epilogue group packs its VC tokens
+// into its own VC columns (hi in the first half, lo in the second), so a warp overwrites only columns it has itself
+// read and the groups need no barrier between reading the accumulator and writing the images.
+__host__ __device__ constexpr uint32_t img_col(uint32_t base, int k, bool lo) {  // 16-token step k
+  return base + (uint32_t)(VC * ((16 * k) / VC) + ((16 * k) % VC) / 2 + (lo ? VC / 2 : 0));
+}
+// The issue loops stay rolled: a warp issues an MMA every 20 to 60 cycles at best, and the code of all roles together has to stay small.
+// D[:, 16 k ..] (+)= +-A[:, 16 k .. 16 k + 15] Tri[16 k .., 16 k .. 16 k + 15]^T over the four 16-token steps of a packed lower triangle, for
+// (A hi, Tri hi), (A lo, Tri hi), (A hi, Tri lo); `first` overwrites D: step 0 covers all of its columns.  A: bf16 image in TMEM.
+template <bool kNeg>
+__device__ __forceinline__ void issue_tri(uint32_t d_tmem, uint32_t a_base, uint32_t tri, bool first) {
+#pragma unroll 1
+  for (int t = 0; t < 3; ++t) {
+    const uint32_t a_img = a_base + (t == 1 ? VC / 2 : 0), b = tri + (t == 2 ? REC_TRI : 0);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      tc::mma_ts(d_tmem + 16 * k, img_col(a_img, k, false), tc::smem_desc_plain(b + tri_step(k), 128, 256),
+                 tc::idesc_f16(128, 64 - 16 * k, 1, 1, false, false, kNeg, false), (first && (t | k) == 0) ? 0u : 1u);
+  }
+}
+// D = H B^T over the 128 features, H as hi and lo image, B a K-major [64][128] tile
+__device__ __forceinline__ void issue_state(uint32_t d_tmem, uint32_t tm, uint32_t tile) {
+  constexpr uint32_t id_n64 = tc::idesc_f16(128, 64, 1, 1, false, false);
+#pragma unroll 1
+  for (int i = 0; i < 4; ++i) {  // hi, lo x features 0 .. 63, 64 .. 127
+    const uint64_t b = tc::smem_desc_sw128(tile + (i & 1) * 8192, 16, 1024);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) tc::mma_ts(d_tmem, tm + TC_HHI + 32 * i + 8 * k, b + (uint64_t)(2 * k), id_n64, (i | k) != 0 ? 1u : 0u);
+  }
+}
+
+// kMulti: built with the parallel-parts machinery (ScanPlan::parts > 1).
+template <bool kMulti>
+__global__ void __launch_bounds__(SCAN_THREADS, 1)
+chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, const int32_t* chunk_start,
+                     const uint8_t* recs, float* o_f32, uint8_t* qt_img,
+                     float* carry, uint8_t* m0_pack, const int32_t* seq_order,
+                     const __grid_constant__ ScanPlan plan) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = tc::align1024(smem_raw);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + CS_BARS);
+  uint64_t* full = bars;          // [3] tiles and record of the stage landed
+  uint64_t* empty = bars + 3;     // [3] everything that reads the stage is complete
+  uint64_t* h_ready = bars + 6;   // bf16 image of the state is in TMEM
+  uint64_t* kh_full = bars + 7;   // H K^T accumulated
+  uint64_t* x_ready = bars + 8;   // X hi+lo written back to TMEM
+  uint64_t* vn_full = bars + 9;   // Vn = Tu (V - X) accumulated
+  uint64_t* vd_ready = bars + 10; // Vd hi+lo written to TMEM (the state update needs nothing else)
+  uint64_t* vn_ready = bars + 11; // Vn hi+lo written to TMEM
+  uint64_t* dh_full = bars + 12;  // state increment accumulated
+  uint64_t* o_full = bars + 13;   // both output accumulators complete
+  uint64_t* o1_empty = bars + 14; // O1 accumulator drained (the output warps take it first, whole, so O1 of the next chunk can run early)
+  uint64_t* o2_empty = bars + 15; // O2 accumulator drained
+  uint64_t* o1_done = bars + 16;  // O1 complete: the bf16 image of H may be overwritten
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  volatile uint32_t* abort_flag = tmem_slot + 1;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_wait();
+  // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
+  // chain of part p >= 1 (see ScanPlan).
+  const int chains = kMulti ? 2 * plan.parts - 1 : 1;
+  const int h = blockIdx.x % a.Hv;
+  const int unit = blockIdx.x / a.Hv;
+  const int chain = kMulti ? unit % chains : 0;
+  const int n = seq_order ? seq_order[unit / chains] : unit / chains;  // varlen: longest sequences first
+  const int part = (chain + 1) >> 1;
+  const bool phi = kMulti && chain > 0 && (chain & 1) == 0;
+  const int hk = h / (a.Hv / a.Hk);
+  if (batch_rejected(a, chunk_start)) return;
+  SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
+  // longer than the caller's bound: the launch schedule was sized from that bound, so the sequence is skipped (zero
+  // output, no state access, like a negative slot) and flagged
+  const bool too_long = a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen;
+  if (too_long && a.status != nullptr && threadIdx.x == 0) atomicOr(a.status, AVE_GDN_DEV_BAD_SEQLEN);
+  if (!sp.ok || sp.len == 0) {
+    if (plan.r0 > 0 || chain > 0) return;
+    // zero-length sequence: the final state is the initial state
+    if (sp.ok && a.final_state != nullptr && a.final_state != a.initial_state) {
+      const int slot0 = a.state_indices ? a.state_indices[n] : n;
+      if (slot0 >= 0 && slot0 < a.num_slots) {
+        const int64_t tile0 = ((int64_t)slot0 * a.Hv + h) * (int64_t)(D * D);
+        for (int e = threadIdx.x; e < D * D; e += SCAN_THREADS)
+          a.final_state[tile0 + e] = a.initial_state ? a.initial_state[tile0 + e] : 0.f;
+      }
+    }
+    return;
+  }
+  const int seq_chunks = (sp.len + C - 1) / C;
+  // a sequence that ends inside part 0 is one plain chain: outputs and the final state leave directly
+  const bool multi = kMulti && plan.parts > 1 && seq_chunks > plan.part_begin[1] && !too_long;
+  if (chain > 0 && (!multi || plan.part_begin[part] >= seq_chunks)) return;
+  int slot = n;
+  if (a.state_indices != nullptr) {
+    slot = a.state_indices[n];
+    if (slot >= a.num_slots) {
+      if (a.status != nullptr && threadIdx.x == 0) atomicOr(a.status, AVE_GDN_DEV_BAD_SLOT);
+      slot = -1;
+    }
+  }
+  if (too_long) slot = -1;
+  __nv_bfloat16* og = reinterpret_cast<__nv_bfloat16*>(a.o) + sp.b * a.o_stride_b + (int64_t)h * a.o_stride_h;
+  // where this chain's per-token rows go: the local rows of later parts wait in fp32 scratch for the fix-up, and so do those of a
+  // gated call for the norm; the transition chain's rows leave as the bf16 hi/lo operand images the fix-up's MMAs read;
+  // all others are the result
+  float* const out_f32 = (!phi && (a.z != nullptr || part > 0)) ? o_f32 : nullptr;
+  if (slot < 0) {  // skipped sequence: zero output, no state access (chain 0 clears the whole sequence once)
+    if (chain > 0 || plan.r0 > 0) return;
+    float* zf = a.z != nullptr ? o_f32 : nullptr;
+    for (int e = threadIdx.x; e < sp.len * D; e += SCAN_THREADS) {
+      const int64_t tok = sp.t0 + e / D;
+      if (zf != nullptr) zf[(((int64_t)sp.b * a.T + tok) * a.Hv + h) * D + e % D] = 0.f;
+      else og[tok * a.o_stride_t + e % D] = __float2bfloat16(0.f);
+    }
+    return;
+  }
+  // This launch covers chunks [c_lo, c_hi) of the chain's part; the state enters from / leaves to the carry buffer
+  // unless this is the first / last launch of a plain chain.
+  const int part_end = min(plan.part_begin[part + 1], seq_chunks);
+  const int c_lo = plan.part_begin[part] + plan.r0;
+  const int c_hi = min(c_lo + plan.rn, part_end);
+  if (c_lo >= c_hi) return;  // finished in an earlier launch, or not reached yet
+  const bool seg_first = plan.r0 == 0;
+  const bool seg_last = c_hi == part_end && !multi;
+  const int c_first = first_record(a, chunk_start, n) + c_lo;
+  sp.t0 += c_lo * C;
+  sp.len = min(sp.len - c_lo * C, (c_hi - c_lo) * C);
+  const int n_chunks = c_hi - c_lo;
+  const int64_t carry_tile = (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D);
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
+    tc::mbar_init(h_ready, 4 * NG); tc::mbar_init(x_ready, 4 * NG); tc::mbar_init(vd_ready, 4 * NG); tc::mbar_init(vn_ready, 4 * NG);
+    for (uint64_t* b : {kh_full, vn_full, dh_full, o_full, o1_done}) tc::mbar_init(b, 1);
+    tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
+    *abort_flag = 0;
+    tc::fence_barrier_init();
+  }
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  tc::tc_fence_after_sync();
+  const uint32_t tm = *tmem_slot;
+
+  if (warp < 4) {
+  tc::reg_set<REGS_CTRL, REGS_LAUNCH>();
+  if (warp == 0) {
+    // ------------------------------------------------------------------ loader: a stage is {Q, K, V, record}, three of them
+    if (lane == 0) {
+      int s = 0;
+      uint32_t ph = 1;  // parity of "chunk c - 3 is done with the stage"; the first round waits for nothing
+      for (int c = 0; c < n_chunks; ++c) {
+        if (c == n_chunks - 1) pdl_trigger();
+        if (c >= CS_STAGES && !tc::mbar_wait(&empty[s], ph, abort_flag)) break;
+        uint8_t* st = smem + s * CS_STAGE;
+        const int tok = sp.t0 + c * C;
+        tc::mbar_expect_tx(&full[s], phi ? CS_STAGE - 16384u : (uint32_t)CS_STAGE);  // the transition chain has no V
+        tc::tma_load_4d(st + CS_K, &maps.k, &full[s], 0, hk, tok, sp.b);
+        tc::tma_load_4d(st + CS_K + 8192, &maps.k, &full[s], 64, hk, tok, sp.b);
+        tc::bulk_load(st + CS_REC, recs + ((int64_t)(c_first + c) * a.Hv + h) * REC_BYTES, REC_BYTES, &full[s]);
+        if (!phi) {
+          tc::tma_load_4d(st + CS_V, &maps.v, &full[s], 0, h, tok, sp.b);
+          tc::tma_load_4d(st + CS_V + 8192, &maps.v, &full[s], 64, h, tok, sp.b);
+        }
+        tc::tma_load_4d(st + CS_Q, &maps.q, &full[s], 0, hk, tok, sp.b);
+        tc::tma_load_4d(st + CS_Q + 8192, &maps.q, &full[s], 64, hk, tok, sp.b);
+        if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ chain MMA issuer (whole warp runs the loop, one
+    // elected lane issues): the MMAs the recurrence waits for.  One thread needs 20 to 60 cycles per MMA instruction, so
+    // the instructions of a chunk are shared between two warps; this one keeps the state-dependent ones short:
+    //   U^T(c+1) -> [state published] H K^T(c) -> [X written] Vn^T(c) -> [Vd written] dH(c)
+    constexpr uint32_t id_dh = tc::idesc_f16(128, 128, 1, 1, false, true);                // B MN-major
+    // U^T = V^T (Tu_hi + Tu_lo)^T opens the Vn^T accumulator of a chunk.  It does not depend on the state, so it is
+    // issued a chunk ahead, right behind the previous chunk's state-increment MMAs (which read the Vd images in the
+    // same columns and, issued earlier by this thread, complete first): the tensor pipe runs it while the chain
+    // epilogue re-packs H.
+    auto issue_u = [&](uint32_t sb) {
+      if (phi) return;  // v = 0: U^T = 0, the first Vn MMA overwrites the accumulator instead
+      if (tc::elect_one()) {
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)  // 16 tokens per step: V rows 2048 bytes apart, feature halves 8192 bytes apart
+            tc::mma_ss(tm + TC_VN + 16 * k, tc::smem_desc_sw128(sb + CS_V + k * 2048, 8192, 1024),
+                       tc::smem_desc_plain(sb + CS_REC + REC_TU + t * REC_TRI + tri_step(k), 128, 256),
+                       tc::idesc_f16(128, 64 - 16 * k, 1, 1, true, false), (t | k) != 0 ? 1u : 0u);
+      }
+      __syncwarp();
+    };
+    int s = 0, s_next = 1;
+    uint32_t ph_next = 0;
+    const uint32_t smem0 = tc::smem_u32(smem);
+    bool issuing = n_chunks > 0 && tc::mbar_wait_warp(&full[0], 0u, abort_flag);
+    if (issuing) { tc::tc_fence_after_sync(); issue_u(smem0); }
+    for (int c = 0; c < n_chunks && issuing; ++c) {
+      const uint32_t cp = (uint32_t)c & 1u;
+      const uint32_t sb = smem0 + s * CS_STAGE;  // the stage has landed: this warp waited for it a chunk ago
+      if (!tc::mbar_wait_warp(h_ready, cp, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      if (tc::elect_one()) {
+        issue_state(tm + TC_X, tm, sb + CS_K);
+        tc::mma_commit(kh_full);
+        // the MMAs of the chunk before are complete with these, and the epilogue, which has published a state, is through with its scale vectors
+        if (c > 0) tc::mma_commit(&empty[s == 0 ? CS_STAGES - 1 : s - 1]);
+      }
+      __syncwarp();
+      if (!tc::mbar_wait_warp(x_ready, cp, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      if (tc::elect_one()) {
+        issue_tri<true>(tm + TC_VN, tm + TC_X, sb + CS_REC + REC_TU, phi);  // Vn^T -= X Tu^T
+        tc::mma_commit(vn_full);
+      }
+      __syncwarp();
+      if (!tc::mbar_wait_warp(vd_ready, cp, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      if (tc::elect_one()) {
+        // dH = (Vd_hi + Vd_lo) contracted with K over the chunk's tokens (K tile read MN-major: 16 token rows per step)
+        const uint64_t k_desc = tc::smem_desc_sw128(sb + CS_K, 8192, 1024);
+#pragma unroll 1
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            tc::mma_ts(tm + TC_DH, img_col(tm + TC_VN + t * (VC / 2), k, false), k_desc + (uint64_t)(128 * k), id_dh, (t | k) != 0 ? 1u : 0u);
+        tc::mma_commit(dh_full);
+      }
+      __syncwarp();
+      if (c + 1 < n_chunks) {
+        if (!tc::mbar_wait_warp(&full[s_next], ph_next, abort_flag)) break;
+        tc::tc_fence_after_sync();
+        issue_u(smem0 + s_next * CS_STAGE);
+        s = s_next;
+        if (++s_next == CS_STAGES) { s_next = 0; ph_next ^= 1u; }
+      }
+    }
+  } else if (warp == 2) {
+    // ------------------------------------------------------------------ output MMA issuer: O1 = H Q^T once H K^T is
+    // complete (so that it runs behind it, while the chain epilogue converts X), O2 = Vn P^T once Vn hi/lo are back
+    int s = 0;
+    uint32_t ph = 0;
+    for (int c = 0; c < n_chunks; ++c) {
+      const uint32_t cp = (uint32_t)c & 1u;
+      const uint32_t sb = tc::smem_u32(smem) + s * CS_STAGE;
+      if (!tc::mbar_wait3(kh_full, cp, o1_empty, cp ^ 1u, &full[s], ph, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      if (tc::elect_one()) {
+        issue_state(tm + TC_O1, tm, sb + CS_Q);  // the chain epilogue waits for its completion before it overwrites the bf16 image of H
+        tc::mma_commit(o1_done);
+      }
+      __syncwarp();
+      // behind the state increment, which the recurrence waits for: side by side they would share the tensor pipe
+      if (!tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, dh_full, cp, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      if (tc::elect_one()) {
+        issue_tri<false>(tm + TC_O2, tm + TC_VI, sb + CS_REC + REC_PT, true);  // O2 = Vn P^T
+        tc::mma_commit(o_full);
+        tc::mma_commit(&empty[s]);
+      }
+      __syncwarp();
+      if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
+    }
+  }
+  } else if (warp < 4 + 4 * NG) {
+    tc::reg_set<REGS_CHAIN, REGS_LAUNCH>();
+    // ------------------------------------------------------------------ chain epilogue: Vn/Vd conversion and state update
+    const int grp = (warp - 4) >> 2;    // column group
+    const int quarter = warp & 3;       // TMEM lane quarter this warp may touch
+    const int d = quarter * 32 + lane;  // row of H (d_v index)
+    const uint32_t lane_addr = tm + ((uint32_t)(quarter * 32) << 16);
+    const int64_t tile = ((int64_t)slot * a.Hv + h) * (int64_t)(D * D);
+    bool alive = true;
+
+    float2 Hreg[HC / 2];  // H[d][HC*grp + 2w .. +1] = M[HC*grp + 2w .. +1][d]
+    // first launch of a chain: part 0 starts from the caller's state, a later part's local chain from zero and its
+    // transition chain from the identity
+    const float* state_in = !seg_first ? carry + carry_tile : (part == 0 && a.initial_state ? a.initial_state + tile : nullptr);
+    float* state_out = seg_last ? (a.final_state ? a.final_state + tile : nullptr) : carry + carry_tile;
+    if (phi && seg_first) {
+#pragma unroll
+      for (int w = 0; w < HC / 2; ++w)
+        Hreg[w] = make_float2(HC * grp + 2 * w == d ? 1.f : 0.f, HC * grp + 2 * w + 1 == d ? 1.f : 0.f);
+    } else if (state_in != nullptr) {
+#pragma unroll
+      for (int w = 0; w < HC / 2; ++w)
+        Hreg[w] = make_float2(state_in[(int64_t)(HC * grp + 2 * w) * D + d], state_in[(int64_t)(HC * grp + 2 * w + 1) * D + d]);
+    } else {
+#pragma unroll
+      for (int w = 0; w < HC / 2; ++w) Hreg[w] = make_float2(0.f, 0.f);
+    }
+    auto publish_h = [&]() {
+#pragma unroll
+      for (int part16 = 0; part16 < HC / 32; ++part16) {  // 16 packed words (32 columns of H) at a time
+        uint32_t hi[16], lo[16];
+#pragma unroll
+        for (int w = 0; w < 16; ++w) split_pair(Hreg[16 * part16 + w], hi[w], lo[w]);
+        tc::tmem_st16(lane_addr + TC_HHI + (HC / 2) * grp + 16 * part16, hi);
+        tc::tmem_st16(lane_addr + TC_HLO + (HC / 2) * grp + 16 * part16, lo);
+      }
+      tc::tmem_st_wait();
+      tc::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(h_ready);
+    };
+    publish_h();
+
+    int s = 0;
+    uint32_t ph = 0;
+    for (int c = 0; c < n_chunks && alive; ++c) {
+      const uint32_t cp = (uint32_t)c & 1u;
+      const float* scal = reinterpret_cast<const float*>(smem + s * CS_STAGE + CS_REC + REC_SCAL);
+      if (!tc::mbar_wait2(&full[s], ph, kh_full, cp, abort_flag)) { alive = false; break; }  // (the scale vectors come with the stage)
+      if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
+      tc::tc_fence_after_sync();
+      {  // X_j = kx_j H k_j
+        uint32_t acc[VC], xh[VC / 2], xl[VC / 2];
+        tc::tmem_ld_n<VC>(lane_addr + TC_X + VC * grp, acc);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int w = 0; w < VC / 2; ++w) {
+          const float2 kx = *reinterpret_cast<const float2*>(scal + 2 * C + VC * grp + 2 * w);
+          split_pair(__fmul2_rn(make_float2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1])), kx), xh[w], xl[w]);
+        }
+        tc::tmem_st_n<VC / 2>(lane_addr + TC_X + VC * grp, xh);  // into this warp's own accumulator columns
+        tc::tmem_st_n<VC / 2>(lane_addr + TC_X + VC * grp + VC / 2, xl);
+        tc::tmem_st_wait();
+        tc::tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(x_ready);
+      }
+      if (!tc::mbar_wait_warp(vn_full, cp, abort_flag)) { alive = false; break; }
+      tc::tc_fence_after_sync();
+      {
+        uint32_t acc[VC];
+        tc::tmem_ld_n<VC>(lane_addr + TC_VN + VC * grp, acc);
+        float2 v[VC / 2];
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int w = 0; w < VC / 2; ++w) v[w] = make_float2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1]));
+        {  // Vd first: its columns alias nothing, and the state update waits only for it
+          uint32_t dh[VC / 2], dl[VC / 2];
+#pragma unroll
+          for (int w = 0; w < VC / 2; ++w) {
+            const float2 ks = *reinterpret_cast<const float2*>(scal + C + VC * grp + 2 * w);
+            split_pair(__fmul2_rn(v[w], ks), dh[w], dl[w]);
+          }
+          tc::tmem_st_n<VC / 2>(lane_addr + TC_VN + VC * grp, dh);  // into this warp's own accumulator columns
+          tc::tmem_st_n<VC / 2>(lane_addr + TC_VN + VC * grp + VC / 2, dl);
+          tc::tmem_st_wait();
+          tc::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(vd_ready);
+        }
+        // the Vn images of the chunk before have been read (long ago: its O2 ran beside its state's conversion)
+        if (!tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) { alive = false; break; }
+        {
+          uint32_t vh[VC / 2], vl[VC / 2];
+#pragma unroll
+          for (int w = 0; w < VC / 2; ++w) split_pair(v[w], vh[w], vl[w]);
+          tc::tmem_st_n<VC / 2>(lane_addr + TC_VI + VC * grp, vh);
+          tc::tmem_st_n<VC / 2>(lane_addr + TC_VI + VC * grp + VC / 2, vl);
+          tc::tmem_st_wait();
+          tc::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(vn_ready);
+        }
+      }
+      if (!tc::mbar_wait2(dh_full, cp, o1_done, cp, abort_flag)) { alive = false; break; }
+      tc::tc_fence_after_sync();
+      {
+        const float decay = scal[3 * C];
+#pragma unroll
+        for (int part32 = 0; part32 < HC / 32; ++part32) {
+          uint32_t dh[32];
+          tc::tmem_ld32(lane_addr + TC_DH + HC * grp + 32 * part32, dh);
+          tc::tmem_ld_wait();
+#pragma unroll
+          for (int w = 0; w < 16; ++w)
+            Hreg[16 * part32 + w] = __ffma2_rn(make_float2(decay, decay), Hreg[16 * part32 + w],
+                                               make_float2(__uint_as_float(dh[2 * w]), __uint_as_float(dh[2 * w + 1])));
+        }
+        publish_h();
+      }
+    }
+    if (alive && state_out != nullptr) {
+#pragma unroll
+      for (int w = 0; w < HC / 2; ++w) {
+        state_out[(int64_t)(HC * grp + 2 * w) * D + d] = Hreg[w].x;
+        state_out[(int64_t)(HC * grp + 2 * w + 1) * D + d] = Hreg[w].y;
+      }
+    }
+    if (alive && multi && chain == 0 && c_hi == part_end) {
+      // the state that enters part 1, as the fix-up's B operand image (row = d_v, K = d_k): this thread's row, HC / 8 pieces
+      uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1)) * a.Hv + h) * (int64_t)PACK_BYTES;
+#pragma unroll
+      for (int j = 0; j < HC / 8; ++j) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) split_pair(Hreg[4 * j + w], hi[w], lo[w]);
+        const uint32_t off = kmajor_piece_off(d, (HC / 8) * grp + j);
+        *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(img + D * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+    }
+  } else {
+    tc::reg_set<REGS_OUT, REGS_LAUNCH>();
+    // ------------------------------------------------------------------ output warps: o = qs_i O1 + O2, a d_v row per thread.  Rows of
+    // tokens are formed in shared memory, in the place of the chunk's Q and K tiles (all MMAs that read them are complete with O2), so
+    // that each warp's 32 features leave in 16-byte pieces (a quarter of the store instructions of one element per lane).
+    const int wq = warp & 3, d = wq * 32 + lane;
+    const uint32_t lane_addr = tm + ((uint32_t)(wq * 32) << 16);
+    int s = 0;
+    for (int c = 0; c < n_chunks; ++c) {
+      const uint32_t cp = (uint32_t)c & 1u;
+      const float* scal = reinterpret_cast<const float*>(smem + s * CS_STAGE + CS_REC + REC_SCAL);
+      float* stage = reinterpret_cast<float*>(smem + s * CS_STAGE);  // [64 tokens][128 features]
+      // 16-byte piece p of token t: neighbouring pieces trade places, so that lanes two pieces, or a token, apart meet different banks
+      auto piece16 = [&](int t, int p) { return stage + t * D + 4 * (p ^ (((p >> 3) ^ t) & 1)); };
+      const int len = min(C, sp.len - c * C);
+      const int64_t tok0 = sp.t0 + c * C;
+      // o_full is committed by the MMA warp after it saw this chunk's stage (tiles and scale vectors) land, so it also
+      // orders the scale vectors; waiting on the stage barrier here would alias phases once this warp lags a chunk
+      if (!tc::mbar_wait_warp(o_full, cp, abort_flag)) break;
+      tc::tc_fence_after_sync();
+      // O1 is taken whole and released at once: O1 of the next chunk is the first thing the tensor pipe runs while the
+      // chain epilogue converts X, and must not wait for the stores below.
+      uint32_t o1[C];
+      tc::tmem_ld32(lane_addr + TC_O1, reinterpret_cast<uint32_t(&)[32]>(o1[0]));
+      tc::tmem_ld32(lane_addr + TC_O1 + 32, reinterpret_cast<uint32_t(&)[32]>(o1[32]));
+      tc::tmem_ld_wait();
+      tc::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(o1_empty);
+      // O2 follows in pieces and is folded into the registers that hold O1
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        uint32_t o2[16];
+        tc::tmem_ld16(lane_addr + TC_O2 + 16 * p, o2);
+        tc::tmem_ld_wait();
+        if (p == 3) {
+          tc::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(o2_empty);
+        }
+#pragma unroll
+        for (int j4 = 0; j4 < 4; ++j4) {
+          const int j = 16 * p + 4 * j4;
+          const float4 qs = *reinterpret_cast<const float4*>(scal + j);
+          const float2 r0 = __ffma2_rn(make_float2(qs.x, qs.y), make_float2(__uint_as_float(o1[j]), __uint_as_float(o1[j + 1])),
+                                       make_float2(__uint_as_float(o2[4 * j4]), __uint_as_float(o2[4 * j4 + 1])));
+          const float2 r1 = __ffma2_rn(make_float2(qs.z, qs.w), make_float2(__uint_as_float(o1[j + 2]), __uint_as_float(o1[j + 3])),
+                                       make_float2(__uint_as_float(o2[4 * j4 + 2]), __uint_as_float(o2[4 * j4 + 3])));
+          o1[j] = __float_as_uint(r0.x); o1[j + 1] = __float_as_uint(r0.y); o1[j + 2] = __float_as_uint(r1.x); o1[j + 3] = __float_as_uint(r1.y);
+        }
+      }
+      if (kMulti && phi) {
+        // qt^T of this chunk as bf16 hi and lo images [128 d_k rows][64 tokens] with the 128-byte swizzle: the fix-up
+        // reads them, unchanged, as the MN-major A operand of its MMA.  This thread owns row d.
+        uint8_t* img = qt_img + ((int64_t)(c_first + c) * a.Hv + h) * (int64_t)QT_BYTES + d * 128;
+#pragma unroll
+        for (int e8 = 0; e8 < C / 8; ++e8) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) split_pair(make_float2(__uint_as_float(o1[8 * e8 + 2 * w]), __uint_as_float(o1[8 * e8 + 2 * w + 1])), hi[w], lo[w]);
+          const uint32_t off = (uint32_t)((e8 ^ (d & 7)) << 4);
+          *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<uint4*>(img + C * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < C; ++t) piece16(t, d >> 2)[d & 3] = __uint_as_float(o1[t]);
+        __syncwarp();
+        if (out_f32 != nullptr) {
+          float* dst = out_f32 + (((int64_t)sp.b * a.T + tok0) * a.Hv + h) * D + 32 * wq + 4 * (lane & 7);
+#pragma unroll 4
+          for (int i = 0; i < 16; ++i) {
+            const int t = 4 * i + (lane >> 3);
+            const float4 v = *reinterpret_cast<const float4*>(piece16(t, 8 * wq + (lane & 7)));
+            if (t < len) *reinterpret_cast<float4*>(dst + (int64_t)t * a.Hv * D) = v;
+          }
+        } else {
+          const int p = 8 * wq + 2 * (lane & 3);
+#pragma unroll 4
+          for (int i = 0; i < 8; ++i) {
+            const int t = 8 * i + (lane >> 2);
+            const float4 v = *reinterpret_cast<const float4*>(piece16(t, p)), w = *reinterpret_cast<const float4*>(piece16(t, p + 1));
+            if (t < len)
+              *reinterpret_cast<uint4*>(og + (tok0 + t) * a.o_stride_t + 4 * p) = make_uint4(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w), pack_bf16x2(w.x, w.y), pack_bf16x2(w.z, w.w));
+          }
+        }
+        tc::fence_proxy_async_smem();  // the next tiles of this stage come by asynchronous copies
+      }
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&empty[s]);
+      if (++s == CS_STAGES) s = 0;
+    }
+  }
+
+  tc::tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag != 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+  if (warp == 1) {
+    tc::tc_fence_after_sync();
+    tc::tmem_dealloc(tm, 512);
+  }
+}
+
+
+}  // namespace
+}  // namespace ave

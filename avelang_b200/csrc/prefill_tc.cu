@@ -1,19 +1,9 @@
 // Chunked gated-delta-rule prefill on the tensor cores (d_k = d_v = 128, chunk 64).
 //
-// Pass 1, chunk_prep (prefill_prep.cuh; parallel over chunks): in-chunk cumulative gate b, T = (I+A)^-1 with
-//   A = strict_lower(beta_i e^{b_i-b_j} k_i.k_j), P = scale * lower_incl(e^{b_i-b_j} q_i.k_j), W^T = K^T (T diag(beta e^b))^T.
-//   W^T, P and Tu = T diag(beta) leave as bf16 hi+lo pairs (the tensor cores then see 16 significant bits), each as the
-//   swizzled shared-memory image of its tile so that a bulk copy moves it out here and in again in pass 2, plus per-token
-//   scale vectors.
-// Pass 2, chunk_scan (one CTA per (sequence, value head)): the recurrence over chunks with the state kept
-//   on chip, transposed (H = M^T, rows = d_v = TMEM lanes) so that every MMA has M = 128:
-//     Vn^T = V^T Tu^T - H W^T             (A = V tile MN-major / H hi/lo from TMEM, B = Tu hi/lo, W^T hi/lo MN-major)
-//     O^T  = qs-scaled H Q^T + Vn^T P^T   (A = H or Vn hi/lo from TMEM, B = Q or P hi/lo, K-major)
-//     H   <- e^{b_C} H + Vd^T K           (A = Vd hi/lo from TMEM, B = K, MN-major), Vd_j = e^{b_C-b_j} Vn_j
-//   The fp32 master copy of H lives in the chain-epilogue threads' registers; its bf16 hi/lo image is rewritten to
-//   TMEM every chunk.  Four warpgroups with redistributed register budgets: control (warp 0 = TMA loader, warp 1 issues
-//   the MMAs the recurrence waits for, warp 2 the output MMAs), two chain-epilogue groups (each covers all 128 TMEM
-//   lanes and half of the columns), one output group.
+// Pass 1, chunk_tiles (prefill_tiles.cuh; parallel over chunks): in-chunk cumulative gate b, T = (I+A)^-1 with
+//   A = strict_lower(beta_i e^{b_i-b_j} k_i.k_j), P = scale * lower_incl(e^{b_i-b_j} q_i.k_j).  P and Tu = T diag(beta) leave as
+//   bf16 hi+lo pairs (the tensor cores then see 16 significant bits), lower triangles only, plus per-token scale vectors.
+// Pass 2, chunk_scan (prefill_scan.cuh; one CTA per (sequence, value head)): the recurrence over chunks with the state kept on chip.
 //   With a gate tensor z the un-normalised output goes to fp32 scratch and a gated-RMSNorm launch finishes it
 //   (optionally storing each row into every GPU's buffer: the fused all-gather).
 // All waits are bounded; on give-up the CTA drains, frees its tensor memory and sets a status bit.
@@ -27,14 +17,11 @@ namespace {
 
 constexpr int C = 64;     // chunk
 constexpr int D = 128;    // d_k = d_v
-constexpr int REC_W = C * D * 2;       // one bf16 [64][128] tile
-constexpr int REC_P = C * C * 2;       // one bf16 [64][64] tile
-constexpr int SCAL_FLOATS = 3 * C;     // qs[64] ks[64] decay(+pad)
-
-struct PrepOut {
-  __nv_bfloat16 *w_hi, *w_lo, *p_hi, *p_lo, *tu_hi, *tu_lo;
-  float *scal;
-};
+// A record: what pass 1 leaves per (chunk, value head) for the scan.  Tu and P are lower triangles of 16x16 blocks as bf16 hi
+// and lo, packed by 16-token steps of the contraction: step c holds rows 16 c .. 63, eight of them after eight, each as two 8x8 core
+// matrices of 128 bytes.  qs[64] | ks[64] | kx[64] | decay[64] in fp32 behind them.
+constexpr int REC_TRI = 5120, REC_TU = 0, REC_PT = 2 * REC_TRI, REC_SCAL = 4 * REC_TRI, REC_BYTES = REC_SCAL + 4 * C * 4;
+__host__ __device__ constexpr int tri_step(int c) { return 2048 * c - 256 * c * (c - 1); }  // byte offset of step c
 
 struct ChunkRef { int n, b, t0, len, cis; bool ok; };  // cis: index of the chunk inside its sequence
 
@@ -183,557 +170,11 @@ __device__ __forceinline__ uint32_t kmajor_piece_off(int row, int k8) {
 }  // namespace
 }  // namespace ave
 
-#include "prefill_prep.cuh"  // pass 1
+#include "prefill_tiles.cuh"  // pass 1
+#include "prefill_scan.cuh"   // pass 2
 
 namespace ave {
 namespace {
-
-// ------------------------------------------------------------------------------------------------ pass 2
-// Warpgroup 0: warp 0 loader, warps 1 and 2 MMA issuers; warpgroups 1..NG: chain epilogue, each covering all 128 TMEM
-// lanes and 1/NG of the columns; the last warpgroup: output.  (Four epilogue groups at 80 registers were measured: no
-// faster, the epilogue is bound by the instructions issued per scheduler, not by the work per thread.)
-constexpr int NG = 2;
-constexpr int SCAN_THREADS = 32 * (4 + 4 * NG + 4);
-constexpr int REGS_LAUNCH = 128;
-constexpr int REGS_CTRL = 72, REGS_CHAIN = 168, REGS_OUT = 104;
-static_assert(NG == 2, "the register split below is for two epilogue groups");
-static_assert(REGS_CTRL + NG * REGS_CHAIN + REGS_OUT <= (NG + 2) * REGS_LAUNCH, "register redistribution exceeds the launch allocation");
-static_assert(SCAN_THREADS * REGS_LAUNCH <= 65536, "launch allocation exceeds the register file");
-constexpr int HC = D / NG;   // columns of H (d_k) per chain-epilogue group
-constexpr int VC = C / NG;   // columns of Vn (tokens) per group
-constexpr int ST_WHI = 0, ST_WLO = 16384, ST_Q = 32768, ST_K = 49152, ST_PHI = 65536, ST_PLO = 73728, ST_V = 81920;
-constexpr int STAGE = 98304;                         // multiple of 1024
-constexpr int SCAL_BYTES = SCAL_FLOATS * 4;
-constexpr uint32_t TILES_TX = STAGE - 2 * REC_P;  // W hi, W lo, Q, K, V
-constexpr int OFF_SCAL = 2 * STAGE;                  // 4 x [qs | ks | decay]: a deeper ring than the tile stages, because
-                                                     // the output warps read qs up to a chunk after the stage is recycled
-constexpr int OFF_VT = OFF_SCAL + 4 * SCAL_BYTES;    // single buffer: Tu hi | Tu lo (they come from scratch that pass 1 has
-                                                     // just written; the V tile, an input read with a long-latency strided
-                                                     // pattern, rides in the stage ring a chunk ahead)
-constexpr int VT_TUH = 0, VT_TUL = 8192, VT_BYTES = 16384;
-static_assert(OFF_VT % 1024 == 0, "swizzled tiles need 1024-byte alignment");
-constexpr int OFF_BARS = OFF_VT + VT_BYTES;
-constexpr size_t SCAN_SMEM = OFF_BARS + 256 + 1024;
-// TMEM columns
-constexpr uint32_t TM_HHI = 0, TM_HLO = 64, TM_VN = 128, TM_VNHI = 192, TM_VNLO = 224, TM_O1 = 256, TM_O2 = 320, TM_DH = 384;
-// The bf16 hi and lo images of Vd reuse the Vn accumulator's columns.  Each chain-epilogue group packs its VC tokens
-// into its own VC columns (hi in the first half, lo in the second), so a warp overwrites only columns it has itself
-// read and the groups need no barrier between reading the accumulator and writing the images.  Their only reader is
-// the state-increment MMA, issued by the same thread that next writes the accumulator (U^T of the following chunk),
-// so program order protects them.  (The images of Vn, read by the other issuer's O2, have columns of their own.)
-// 16-token K step k of the Vd image starts at:
-__host__ __device__ constexpr uint32_t vd_img_col(int k, bool lo) {
-  return TM_VN + (uint32_t)(VC * ((16 * k) / VC) + ((16 * k) % VC) / 2 + (lo ? VC / 2 : 0));
-}
-
-// Issues `ksteps` MMAs D (+)= A[tmem] * B[smem] over consecutive 16-wide K steps.  A advances 8 TMEM columns per
-// step; B advances b_step bytes per step and jumps b_half extra after four steps (second 64-wide K half of a
-// K-major tile; 0 when there is none).
-__device__ __forceinline__ void issue_ts(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_smem, uint32_t b_step, uint32_t b_half,
-                                         uint32_t lbo, uint32_t idesc, int ksteps, bool accumulate) {
-  const uint64_t desc = tc::smem_desc_sw128(b_smem, lbo, 1024);
-#pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    if (k < ksteps)
-      tc::mma_ts(d_tmem, a_tmem + 8 * k, desc + (uint64_t)((k * b_step + ((k > 3) ? b_half : 0u)) >> 4), idesc,
-                 (accumulate || k != 0) ? 1u : 0u);
-  }
-}
-
-// kMulti: built with the parallel-parts machinery (ScanPlan::parts > 1).  The plain instantiation carries none of its
-// state, which keeps the output warpgroup inside its register budget with 32-token pieces.
-template <bool kMulti>
-__global__ void __launch_bounds__(SCAN_THREADS, 1)
-chunk_scan_tc_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, const int32_t* chunk_start,
-                     const __nv_bfloat16* w_hi_ws, const __nv_bfloat16* w_lo_ws,
-                     const __nv_bfloat16* p_hi_ws, const __nv_bfloat16* p_lo_ws,
-                     const __nv_bfloat16* tu_hi_ws, const __nv_bfloat16* tu_lo_ws,
-                     const float* scal_ws, float* o_f32, uint8_t* qt_img,
-                     float* carry, uint8_t* m0_pack, const int32_t* seq_order,
-                     const __grid_constant__ ScanPlan plan) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = tc::align1024(smem_raw);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
-  uint64_t* full = bars;          // [2] W, Q, K and V tiles of the stage landed
-  uint64_t* pfull = bars + 2;     // [2] P tiles and the scale vectors of the stage landed
-  uint64_t* h_ready = bars + 4;   // bf16 image of the state is in TMEM
-  uint64_t* vn_full = bars + 5;   // -(H W^T) accumulated
-  uint64_t* vn_ready = bars + 6;  // Vn / Vd hi+lo written back to TMEM
-  uint64_t* dh_full = bars + 7;   // state increment accumulated
-  uint64_t* o_full = bars + 8;    // both output accumulators complete
-  uint64_t* o1_empty = bars + 9;  // O1 accumulator drained (the output warps take it first, whole, so O1 of the next chunk can run early)
-  uint64_t* o2_empty = bars + 12; // O2 accumulator drained
-  uint64_t* o1_done = bars + 13;  // O1 complete: the bf16 image of H may be overwritten
-  uint64_t* u_full = bars + 10;   // Tu tiles landed
-  uint64_t* u_empty = bars + 11;  // the U^T MMAs that read them are complete
-  uint64_t* vd_ready = bars + 14; // Vd hi+lo written to TMEM (the state update needs nothing else)
-  // a stage is given back tile by tile, as soon as the last MMA that reads the tile is complete
-  uint64_t* w_empty = bars + 16;  // [2] after the Vn MMAs
-  uint64_t* q_empty = bars + 18;  // [2] after O1
-  uint64_t* k_empty = bars + 20;  // [2] after the state increment
-  uint64_t* p_empty = bars + 22;  // [2] after O2
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
-  volatile uint32_t* abort_flag = tmem_slot + 1;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_wait();
-  // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
-  // chain of part p >= 1 (see ScanPlan).
-  const int chains = kMulti ? 2 * plan.parts - 1 : 1;
-  const int h = blockIdx.x % a.Hv;
-  const int unit = blockIdx.x / a.Hv;
-  const int chain = kMulti ? unit % chains : 0;
-  const int n = seq_order ? seq_order[unit / chains] : unit / chains;  // varlen: longest sequences first
-  const int part = (chain + 1) >> 1;
-  const bool phi = kMulti && chain > 0 && (chain & 1) == 0;
-  const int hk = h / (a.Hv / a.Hk);
-  if (batch_rejected(a, chunk_start)) return;
-  SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, a.status);
-  // longer than the caller's bound: the launch schedule was sized from that bound, so the sequence is skipped (zero
-  // output, no state access, like a negative slot) and flagged
-  const bool too_long = a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen;
-  if (too_long && a.status != nullptr && threadIdx.x == 0) atomicOr(a.status, AVE_GDN_DEV_BAD_SEQLEN);
-  if (!sp.ok || sp.len == 0) {
-    if (plan.r0 > 0 || chain > 0) return;
-    // zero-length sequence: the final state is the initial state
-    if (sp.ok && a.final_state != nullptr && a.final_state != a.initial_state) {
-      const int slot0 = a.state_indices ? a.state_indices[n] : n;
-      if (slot0 >= 0 && slot0 < a.num_slots) {
-        const int64_t tile0 = ((int64_t)slot0 * a.Hv + h) * (int64_t)(D * D);
-        for (int e = threadIdx.x; e < D * D; e += SCAN_THREADS)
-          a.final_state[tile0 + e] = a.initial_state ? a.initial_state[tile0 + e] : 0.f;
-      }
-    }
-    return;
-  }
-  const int seq_chunks = (sp.len + C - 1) / C;
-  // a sequence that ends inside part 0 is one plain chain: outputs and the final state leave directly
-  const bool multi = kMulti && plan.parts > 1 && seq_chunks > plan.part_begin[1] && !too_long;
-  if (chain > 0 && (!multi || plan.part_begin[part] >= seq_chunks)) return;
-  int slot = n;
-  if (a.state_indices != nullptr) {
-    slot = a.state_indices[n];
-    if (slot >= a.num_slots) {
-      if (a.status != nullptr && threadIdx.x == 0) atomicOr(a.status, AVE_GDN_DEV_BAD_SLOT);
-      slot = -1;
-    }
-  }
-  if (too_long) slot = -1;
-  __nv_bfloat16* og = reinterpret_cast<__nv_bfloat16*>(a.o) + sp.b * a.o_stride_b + (int64_t)h * a.o_stride_h;
-  // where this chain's per-token rows go: the local rows of later parts wait in fp32 scratch for the fix-up; part 0
-  // writes fp32 scratch only when a gated norm follows, else the result itself; the transition chain's rows leave as
-  // the bf16 hi/lo operand images the fix-up's MMAs read (see the output warps)
-  float* const out_f32 = (!phi && (a.z != nullptr || part > 0)) ? o_f32 : nullptr;
-  if (slot < 0) {  // skipped sequence: zero output, no state access (chain 0 clears the whole sequence once)
-    if (chain > 0 || plan.r0 > 0) return;
-    float* zf = a.z != nullptr ? o_f32 : nullptr;
-    for (int e = threadIdx.x; e < sp.len * D; e += SCAN_THREADS) {
-      const int64_t tok = sp.t0 + e / D;
-      if (zf != nullptr) zf[(((int64_t)sp.b * a.T + tok) * a.Hv + h) * D + e % D] = 0.f;
-      else og[tok * a.o_stride_t + e % D] = __float2bfloat16(0.f);
-    }
-    return;
-  }
-  // This launch covers chunks [c_lo, c_hi) of the chain's part; the state enters from / leaves to the carry buffer
-  // unless this is the first / last launch of a plain chain.
-  const int part_end = min(plan.part_begin[part + 1], seq_chunks);
-  const int c_lo = plan.part_begin[part] + plan.r0;
-  const int c_hi = min(c_lo + plan.rn, part_end);
-  if (c_lo >= c_hi) return;  // finished in an earlier launch, or not reached yet
-  const bool seg_first = plan.r0 == 0;
-  const bool seg_last = c_hi == part_end && !multi;
-  const int c_first = first_record(a, chunk_start, n) + c_lo;
-  sp.t0 += c_lo * C;
-  sp.len = min(sp.len - c_lo * C, (c_hi - c_lo) * C);
-  const int n_chunks = c_hi - c_lo;
-  const int64_t carry_tile = (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D);
-
-  if (threadIdx.x == 0) {
-    tc::mbar_init(&full[0], 1); tc::mbar_init(&full[1], 1);
-    tc::mbar_init(&pfull[0], 1); tc::mbar_init(&pfull[1], 1);
-    for (int i = 0; i < 2; ++i) { tc::mbar_init(&w_empty[i], 1); tc::mbar_init(&q_empty[i], 1); tc::mbar_init(&k_empty[i], 1); tc::mbar_init(&p_empty[i], 1); }
-    tc::mbar_init(h_ready, 4 * NG); tc::mbar_init(vn_full, 1); tc::mbar_init(vn_ready, 4 * NG);
-    tc::mbar_init(dh_full, 1); tc::mbar_init(o_full, 1); tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4); tc::mbar_init(o1_done, 1);
-    tc::mbar_init(u_full, 1); tc::mbar_init(u_empty, 1);
-    tc::mbar_init(vd_ready, 4 * NG);
-    *abort_flag = 0;
-    tc::fence_barrier_init();
-  }
-  if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
-  tc::tc_fence_before_sync();
-  __syncthreads();
-  tc::tc_fence_after_sync();
-  const uint32_t tm = *tmem_slot;
-
-  if (warp < 4) {
-  tc::reg_set<REGS_CTRL, REGS_LAUNCH>();
-  if (warp == 0) {
-    // ------------------------------------------------------------------ loader
-    // Two stages of {W hi, W lo, Q, K, P hi, P lo, V}.  A tile of chunk c+2 is fetched as soon as the last MMA that
-    // reads the same tile of chunk c is complete (W after the Vn MMAs, early in the chunk's period; P last), so most of a
-    // stage lands more than a period before it is needed instead of a fraction of one.
-    if (lane == 0) {
-      for (int c = 0; c < n_chunks; ++c) {
-        const int s = c & 1;
-        if (c == n_chunks - 1) pdl_trigger();
-        const uint32_t free_par = ((uint32_t)(c >> 1) & 1u) ^ 1u;  // parity of "chunk c-2 is done with it"
-        uint8_t* st = smem + s * STAGE;
-        const int64_t rec = (int64_t)(c_first + c) * a.Hv + h;
-        const int tok = sp.t0 + c * C;
-        // The Vn MMAs of chunk c-2 are complete: so are its U^T MMAs, issued before them (W and V slots are free), and
-        // the MMA warp has long passed its wait for the stage's previous phase, so the barrier can be armed again.
-        if (!tc::mbar_wait(&w_empty[s], free_par, abort_flag)) break;
-        tc::mbar_expect_tx(&full[s], phi ? TILES_TX - 16384u : TILES_TX);  // the transition chain has no V
-        if (!phi) {
-          tc::tma_load_4d(st + ST_V, &maps.v, &full[s], 0, h, tok, sp.b);
-          tc::tma_load_4d(st + ST_V + 8192, &maps.v, &full[s], 64, h, tok, sp.b);
-        }
-        tc::bulk_load(st + ST_WHI, w_hi_ws + rec * (C * D), REC_W, &full[s]);  // W^T tile images: 128 d_k rows of 64 tokens
-        tc::bulk_load(st + ST_WLO, w_lo_ws + rec * (C * D), REC_W, &full[s]);
-        if (!tc::mbar_wait(&q_empty[s], free_par, abort_flag)) break;
-        tc::tma_load_4d(st + ST_Q, &maps.q, &full[s], 0, hk, tok, sp.b);
-        tc::tma_load_4d(st + ST_Q + 8192, &maps.q, &full[s], 64, hk, tok, sp.b);
-        if (!tc::mbar_wait(&k_empty[s], free_par, abort_flag)) break;
-        tc::tma_load_4d(st + ST_K, &maps.k, &full[s], 0, hk, tok, sp.b);
-        tc::tma_load_4d(st + ST_K + 8192, &maps.k, &full[s], 64, hk, tok, sp.b);
-        // P and the scale vectors last.  The scale-vector ring is four deep: the output warps read qs of chunk c-4 until
-        // they release its accumulators, which O1 of chunk c-2, and so this wait, comes after.
-        if (!tc::mbar_wait(&p_empty[s], free_par, abort_flag)) break;
-        tc::mbar_expect_tx(&pfull[s], 2 * REC_P + SCAL_BYTES);
-        tc::bulk_load(st + ST_PHI, p_hi_ws + rec * (C * C), REC_P, &pfull[s]);
-        tc::bulk_load(st + ST_PLO, p_lo_ws + rec * (C * C), REC_P, &pfull[s]);
-        tc::bulk_load(smem + OFF_SCAL + (c & 3) * SCAL_BYTES, scal_ws + rec * SCAL_FLOATS, SCAL_BYTES, &pfull[s]);
-        if (phi) continue;
-        // Tu of chunk c replaces that of chunk c-1 once the U^T MMAs of chunk c-1 have read it
-        if (!tc::mbar_wait(u_empty, ((uint32_t)c & 1u) ^ 1u, abort_flag)) break;
-        uint8_t* vt = smem + OFF_VT;
-        tc::mbar_expect_tx(u_full, VT_BYTES);
-        tc::bulk_load(vt + VT_TUH, tu_hi_ws + rec * (C * C), REC_P, u_full);
-        tc::bulk_load(vt + VT_TUL, tu_lo_ws + rec * (C * C), REC_P, u_full);
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ chain MMA issuer (whole warp runs the loop, one
-    // elected lane issues): the MMAs the recurrence waits for.  One thread needs 20 to 60 cycles per MMA instruction, so
-    // the 68 instructions of a chunk are shared between two warps; this one keeps the state-dependent ones short:
-    //   U^T(c+1) -> [state published] Vn^T(c) -> [Vd written] dH(c)
-    constexpr uint32_t id_vn = tc::idesc_f16(128, 64, 1, 1, false, true, true, false);    // negated A, B = W^T read MN-major
-    constexpr uint32_t id_dh = tc::idesc_f16(128, 128, 1, 1, false, true);                // B MN-major
-    constexpr uint32_t id_u = tc::idesc_f16(128, 64, 1, 1, true, false);                  // A = V tile read MN-major
-    const uint32_t vtb = tc::smem_u32(smem + OFF_VT);
-    // U^T = V^T (Tu_hi + Tu_lo)^T opens the Vn^T accumulator of a chunk.  It does not depend on the state, so it is
-    // issued a chunk ahead, right behind the previous chunk's state-increment MMAs (which read the Vd images in the
-    // same columns and, issued earlier by this thread, complete first): the tensor pipe runs it while the chain
-    // epilogue re-packs H.
-    auto issue_u = [&](int c) {
-      if (phi) return;  // v = 0: U^T = 0, the first Vn MMA overwrites the accumulator instead
-      const uint32_t vb = tc::smem_u32(smem + (c & 1) * STAGE + ST_V);
-      if (tc::elect_one()) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)  // 16 tokens per step: V rows 2048 bytes apart, feature halves 8192 bytes apart
-            tc::mma_ss(tm + TM_VN, tc::smem_desc_sw128(vb + k * 2048, 8192, 1024),
-                       tc::smem_desc_sw128(vtb + (t ? VT_TUL : VT_TUH) + k * 32, 16, 1024), id_u, (t | k) != 0 ? 1u : 0u);
-        tc::mma_commit(u_empty);
-      }
-      __syncwarp();
-    };
-    bool issuing = n_chunks > 0 && tc::mbar_wait_warp(&full[0], 0u, abort_flag) && (phi || tc::mbar_wait_warp(u_full, 0u, abort_flag));
-    if (issuing) { tc::tc_fence_after_sync(); issue_u(0); }
-    for (int c = 0; c < n_chunks && issuing; ++c) {
-      const int s = c & 1;
-      const uint32_t cp = (uint32_t)c & 1u;
-      const uint32_t sb = tc::smem_u32(smem + s * STAGE);  // W, K have landed: this warp waited for the stage a chunk ago
-      if (!tc::mbar_wait_warp(h_ready, cp, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        // Vn^T += -(Hhi Whi^T + Hhi Wlo^T + Hlo Whi^T); W^T is one [128 d_k][64 token] tile, 16 d_k rows per step
-        issue_ts(tm + TM_VN, tm + TM_HHI, sb + ST_WHI, 2048, 0, 16, id_vn, 8, !phi);
-        issue_ts(tm + TM_VN, tm + TM_HHI, sb + ST_WLO, 2048, 0, 16, id_vn, 8, true);
-        issue_ts(tm + TM_VN, tm + TM_HLO, sb + ST_WHI, 2048, 0, 16, id_vn, 8, true);
-        tc::mma_commit(vn_full);
-        tc::mma_commit(&w_empty[s]);
-      }
-      __syncwarp();
-      if (!tc::mbar_wait_warp(vd_ready, cp, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        // dH = (Vd_hi + Vd_lo) contracted with K over the chunk's tokens (K tile read MN-major: 16 token rows per step)
-        const uint64_t k_desc = tc::smem_desc_sw128(sb + ST_K, 8192, 1024);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tc::mma_ts(tm + TM_DH, tm + vd_img_col(k, false), k_desc + (uint64_t)(128 * k), id_dh, k != 0 ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) tc::mma_ts(tm + TM_DH, tm + vd_img_col(k, true), k_desc + (uint64_t)(128 * k), id_dh, 1u);
-        tc::mma_commit(dh_full);
-        tc::mma_commit(&k_empty[s]);
-      }
-      __syncwarp();
-      if (c + 1 < n_chunks) {
-        // the next chunk's tiles, polled together so that the latencies of phases that are already complete overlap
-        uint64_t* b_f = &full[(c + 1) & 1];
-        const uint32_t p_f = (uint32_t)((c + 1) >> 1) & 1u;
-        if (!(phi ? tc::mbar_wait_warp(b_f, p_f, abort_flag) : tc::mbar_wait2(b_f, p_f, u_full, (uint32_t)(c + 1) & 1u, abort_flag))) break;
-        tc::tc_fence_after_sync();
-        issue_u(c + 1);
-      }
-    }
-  } else if (warp == 2) {
-    // ------------------------------------------------------------------ output MMA issuer: O1 = H Q^T once the Vn MMAs are
-    // complete (so that it runs behind them, while the chain epilogue converts Vn), O2 = Vn P^T once Vn hi/lo are back
-    constexpr uint32_t id_n64 = tc::idesc_f16(128, 64, 1, 1, false, false);
-    for (int c = 0; c < n_chunks; ++c) {
-      const int s = c & 1;
-      const uint32_t cp = (uint32_t)c & 1u, u = (uint32_t)(c >> 1);
-      const uint32_t sb = tc::smem_u32(smem + s * STAGE);
-      if (!tc::mbar_wait3(vn_full, cp, o1_empty, cp ^ 1u, &full[s], u & 1u, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        // O1 = (Hhi + Hlo) Q^T; the chain epilogue waits for its completion before it overwrites the bf16 image of H
-        issue_ts(tm + TM_O1, tm + TM_HHI, sb + ST_Q, 32, 8192 - 128, 16, id_n64, 8, false);
-        issue_ts(tm + TM_O1, tm + TM_HLO, sb + ST_Q, 32, 8192 - 128, 16, id_n64, 8, true);
-        tc::mma_commit(o1_done);
-        tc::mma_commit(&q_empty[s]);
-      }
-      __syncwarp();
-      if (!tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, &pfull[s], u & 1u, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        // O2 = Vn_hi Phi^T + Vn_lo Phi^T + Vn_hi Plo^T
-        issue_ts(tm + TM_O2, tm + TM_VNHI, sb + ST_PHI, 32, 0, 16, id_n64, 4, false);
-        issue_ts(tm + TM_O2, tm + TM_VNLO, sb + ST_PHI, 32, 0, 16, id_n64, 4, true);
-        issue_ts(tm + TM_O2, tm + TM_VNHI, sb + ST_PLO, 32, 0, 16, id_n64, 4, true);
-        tc::mma_commit(o_full);
-        tc::mma_commit(&p_empty[s]);
-      }
-      __syncwarp();
-    }
-  }
-  } else if (warp < 4 + 4 * NG) {
-    tc::reg_set<REGS_CHAIN, REGS_LAUNCH>();
-    // ------------------------------------------------------------------ chain epilogue: Vn/Vd conversion and state update
-    const int grp = (warp - 4) >> 2;    // column group
-    const int quarter = warp & 3;       // TMEM lane quarter this warp may touch
-    const int d = quarter * 32 + lane;  // row of H (d_v index)
-    const uint32_t lane_addr = tm + ((uint32_t)(quarter * 32) << 16);
-    const int64_t tile = ((int64_t)slot * a.Hv + h) * (int64_t)(D * D);
-    bool alive = true;
-
-    float2 Hreg[HC / 2];  // H[d][HC*grp + 2w .. +1] = M[HC*grp + 2w .. +1][d]
-    // first launch of a chain: part 0 starts from the caller's state, a later part's local chain from zero and its
-    // transition chain from the identity
-    const float* state_in = !seg_first ? carry + carry_tile : (part == 0 && a.initial_state ? a.initial_state + tile : nullptr);
-    float* state_out = seg_last ? (a.final_state ? a.final_state + tile : nullptr) : carry + carry_tile;
-    if (phi && seg_first) {
-#pragma unroll
-      for (int w = 0; w < HC / 2; ++w)
-        Hreg[w] = make_float2(HC * grp + 2 * w == d ? 1.f : 0.f, HC * grp + 2 * w + 1 == d ? 1.f : 0.f);
-    } else if (state_in != nullptr) {
-#pragma unroll
-      for (int w = 0; w < HC / 2; ++w)
-        Hreg[w] = make_float2(state_in[(int64_t)(HC * grp + 2 * w) * D + d], state_in[(int64_t)(HC * grp + 2 * w + 1) * D + d]);
-    } else {
-#pragma unroll
-      for (int w = 0; w < HC / 2; ++w) Hreg[w] = make_float2(0.f, 0.f);
-    }
-    auto publish_h = [&]() {
-#pragma unroll
-      for (int part16 = 0; part16 < HC / 32; ++part16) {  // 16 packed words (32 columns of H) at a time
-        uint32_t hi[16], lo[16];
-#pragma unroll
-        for (int w = 0; w < 16; ++w) split_pair(Hreg[16 * part16 + w], hi[w], lo[w]);
-        tc::tmem_st16(lane_addr + TM_HHI + (HC / 2) * grp + 16 * part16, hi);
-        tc::tmem_st16(lane_addr + TM_HLO + (HC / 2) * grp + 16 * part16, lo);
-      }
-      tc::tmem_st_wait();
-      tc::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(h_ready);
-    };
-    publish_h();
-
-    for (int c = 0; c < n_chunks && alive; ++c) {
-      const int s = c & 1;
-      const uint32_t cp = (uint32_t)c & 1u, u = (uint32_t)(c >> 1);
-      const float* scal = reinterpret_cast<const float*>(smem + OFF_SCAL + (c & 3) * SCAL_BYTES);
-      if (!tc::mbar_wait_warp(&pfull[s], u & 1u, abort_flag)) { alive = false; break; }  // the scale vectors
-      if (!tc::mbar_wait_warp(vn_full, cp, abort_flag)) { alive = false; break; }
-      tc::tc_fence_after_sync();
-      {
-        uint32_t acc[VC];
-        tc::tmem_ld_n<VC>(lane_addr + TM_VN + VC * grp, acc);
-        float2 v[VC / 2];
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int w = 0; w < VC / 2; ++w) v[w] = make_float2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1]));
-        {  // Vd first: its columns alias nothing, and the state update waits only for it
-          uint32_t dh[VC / 2], dl[VC / 2];
-#pragma unroll
-          for (int w = 0; w < VC / 2; ++w) {
-            const float2 ks = *reinterpret_cast<const float2*>(scal + C + VC * grp + 2 * w);
-            split_pair(__fmul2_rn(v[w], ks), dh[w], dl[w]);
-          }
-          tc::tmem_st_n<VC / 2>(lane_addr + TM_VN + VC * grp, dh);  // into this warp's own accumulator columns
-          tc::tmem_st_n<VC / 2>(lane_addr + TM_VN + VC * grp + VC / 2, dl);
-          tc::tmem_st_wait();
-          tc::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(vd_ready);
-        }
-        // the Vn images have columns of their own, free once O2 of the previous chunk is complete (long ago)
-        if (!tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) { alive = false; break; }
-        {
-          uint32_t vh[VC / 2], vl[VC / 2];
-#pragma unroll
-          for (int w = 0; w < VC / 2; ++w) split_pair(v[w], vh[w], vl[w]);
-          tc::tmem_st_n<VC / 2>(lane_addr + TM_VNHI + (VC / 2) * grp, vh);
-          tc::tmem_st_n<VC / 2>(lane_addr + TM_VNLO + (VC / 2) * grp, vl);
-          tc::tmem_st_wait();
-          tc::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(vn_ready);
-        }
-      }
-      if (!tc::mbar_wait2(dh_full, cp, o1_done, cp, abort_flag)) { alive = false; break; }
-      tc::tc_fence_after_sync();
-      {
-        const float decay = scal[2 * C];
-#pragma unroll
-        for (int part32 = 0; part32 < HC / 32; ++part32) {
-          uint32_t dh[32];
-          tc::tmem_ld32(lane_addr + TM_DH + HC * grp + 32 * part32, dh);
-          tc::tmem_ld_wait();
-#pragma unroll
-          for (int w = 0; w < 16; ++w)
-            Hreg[16 * part32 + w] = __ffma2_rn(make_float2(decay, decay), Hreg[16 * part32 + w],
-                                               make_float2(__uint_as_float(dh[2 * w]), __uint_as_float(dh[2 * w + 1])));
-        }
-        publish_h();
-      }
-    }
-    if (alive && state_out != nullptr) {
-#pragma unroll
-      for (int w = 0; w < HC / 2; ++w) {
-        state_out[(int64_t)(HC * grp + 2 * w) * D + d] = Hreg[w].x;
-        state_out[(int64_t)(HC * grp + 2 * w + 1) * D + d] = Hreg[w].y;
-      }
-    }
-    if (alive && multi && chain == 0 && c_hi == part_end) {
-      // the state that enters part 1, as the fix-up's B operand image (row = d_v, K = d_k): this thread's row, HC / 8 pieces
-      uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1)) * a.Hv + h) * (int64_t)PACK_BYTES;
-#pragma unroll
-      for (int j = 0; j < HC / 8; ++j) {
-        uint32_t hi[4], lo[4];
-#pragma unroll
-        for (int w = 0; w < 4; ++w) split_pair(Hreg[4 * j + w], hi[w], lo[w]);
-        const uint32_t off = kmajor_piece_off(d, (HC / 8) * grp + j);
-        *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-        *reinterpret_cast<uint4*>(img + D * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-      }
-    }
-  } else {
-    tc::reg_set<REGS_OUT, REGS_LAUNCH>();
-    // ------------------------------------------------------------------ output warps: o = scale (qs_i O1 + O2), straight
-    // from registers: thread = d_v row, one store per token (a warp covers 32 adjacent features of one token).  When a
-    // gated norm follows, the un-normalised output is kept in fp32 scratch for the norm kernel; otherwise it is the result.
-    const int quarter = warp & 3;
-    const int d = quarter * 32 + lane;
-    const uint32_t lane_addr = tm + ((uint32_t)(quarter * 32) << 16);
-    float* of = out_f32 ? out_f32 + ((int64_t)sp.b * a.T * a.Hv + h) * D + d : nullptr;
-    bool alive = true;
-    for (int c = 0; c < n_chunks && alive; ++c) {
-      const uint32_t cp = (uint32_t)c & 1u;
-      const float* scal = reinterpret_cast<const float*>(smem + OFF_SCAL + (c & 3) * SCAL_BYTES);
-      const int len = min(C, sp.len - c * C);
-      const int64_t tok0 = sp.t0 + c * C;
-      // o_full is committed by the MMA warp after it saw this chunk's stage (tiles and scale vectors) land, so it also
-      // orders the scale vectors; waiting on the stage barrier here would alias phases once this warp lags a chunk
-      if (!tc::mbar_wait_warp(o_full, cp, abort_flag)) { alive = false; break; }
-      tc::tc_fence_after_sync();
-      float* pf = of ? of + tok0 * ((int64_t)a.Hv * D) : nullptr;
-      __nv_bfloat16* pb = og + tok0 * a.o_stride_t + d;
-      const int64_t fstep = (int64_t)a.Hv * D, bstep = a.o_stride_t;
-      // O1 is taken whole and released at once: O1 of the next chunk is the first thing the tensor pipe runs while the
-      // chain epilogue converts Vn, and must not wait for the stores below.
-      uint32_t o1[C];
-      tc::tmem_ld32(lane_addr + TM_O1, reinterpret_cast<uint32_t(&)[32]>(o1[0]));
-      tc::tmem_ld32(lane_addr + TM_O1 + 32, reinterpret_cast<uint32_t(&)[32]>(o1[32]));
-      tc::tmem_ld_wait();
-      tc::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(o1_empty);
-      // O2 follows in pieces and is folded into the registers that hold O1 (o = qs O1 + O2), so both accumulators are
-      // free before the first store: how fast the stores drain no longer decides when the next chunk's output MMAs may run.
-      constexpr int PW = 16;  // tokens per piece
-#pragma unroll
-      for (int piece = 0; piece < C / PW; ++piece) {
-        uint32_t o2[PW];
-        tc::tmem_ld16(lane_addr + TM_O2 + PW * piece, o2);
-        tc::tmem_ld_wait();
-        if (piece == C / PW - 1) {  // the accumulator is in registers: the next chunk's MMAs may overwrite it
-          tc::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) tc::mbar_arrive(o2_empty);
-        }
-#pragma unroll
-        for (int j4 = 0; j4 < PW / 4; ++j4) {
-          const int j = PW * piece + 4 * j4;
-          const float4 qs = *reinterpret_cast<const float4*>(scal + j);
-          const float2 r0 = __ffma2_rn(make_float2(qs.x, qs.y), make_float2(__uint_as_float(o1[j]), __uint_as_float(o1[j + 1])),
-                                       make_float2(__uint_as_float(o2[4 * j4]), __uint_as_float(o2[4 * j4 + 1])));
-          const float2 r1 = __ffma2_rn(make_float2(qs.z, qs.w), make_float2(__uint_as_float(o1[j + 2]), __uint_as_float(o1[j + 3])),
-                                       make_float2(__uint_as_float(o2[4 * j4 + 2]), __uint_as_float(o2[4 * j4 + 3])));
-          o1[j] = __float_as_uint(r0.x); o1[j + 1] = __float_as_uint(r0.y); o1[j + 2] = __float_as_uint(r1.x); o1[j + 3] = __float_as_uint(r1.y);
-        }
-      }
-#pragma unroll
-      for (int piece = 0; piece < C / PW; ++piece) {
-        float ov[PW];
-#pragma unroll
-        for (int j = 0; j < PW; ++j) ov[j] = __uint_as_float(o1[PW * piece + j]);
-        const int n_here = min(PW, len - PW * piece);  // tokens of this piece that exist
-        if (phi) {
-          // qt^T of this chunk as bf16 hi and lo images [128 d_k rows][64 tokens] with the 128-byte swizzle: the fix-up
-          // reads them, unchanged, as the MN-major A operand of its MMA.  This thread owns row d: two 16-byte pieces.
-          uint8_t* img = qt_img + ((int64_t)(c_first + c) * a.Hv + h) * (int64_t)QT_BYTES + d * 128;
-#pragma unroll
-          for (int e8 = 0; e8 < PW / 8; ++e8) {
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int w = 0; w < 4; ++w) split_pair(make_float2(ov[8 * e8 + 2 * w], ov[8 * e8 + 2 * w + 1]), hi[w], lo[w]);
-            const uint32_t off = (uint32_t)((((PW / 8) * piece + e8) ^ (d & 7)) << 4);
-            *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(img + C * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-          }
-        } else if (pf != nullptr) {
-          if (n_here == PW) {
-#pragma unroll
-            for (int j = 0; j < PW; ++j) { *pf = ov[j]; pf += fstep; }
-          } else {
-#pragma unroll
-            for (int j = 0; j < PW; ++j) { if (j < n_here) *pf = ov[j]; pf += fstep; }
-          }
-        } else {
-          if (n_here == PW) {
-#pragma unroll
-            for (int j = 0; j < PW; ++j) { *pb = __float2bfloat16(ov[j]); pb += bstep; }
-          } else {
-#pragma unroll
-            for (int j = 0; j < PW; ++j) { if (j < n_here) *pb = __float2bfloat16(ov[j]); pb += bstep; }
-          }
-        }
-      }
-    }
-  }
-
-  tc::tc_fence_before_sync();
-  __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag != 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
-  if (warp == 1) {
-    tc::tc_fence_after_sync();
-    tc::tmem_dealloc(tm, 512);
-  }
-}
 
 // ------------------------------------------------------------------------------------------------ parts: combine and fix-up
 // Once every chain of a multi-part sequence has run, the carry buffer holds, per (sequence, value head): chain 0 = the
@@ -1041,21 +482,19 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
 }
 
 // ------------------------------------------------------------------------------------------------ schedule and scratch
-constexpr int SEG_FIRST_DIV = 6;    // first range = 1/6 of the longest chain's chunks (64 heads, 4096 tokens: 290 us; 1/16: 328)
-constexpr int SEG_FIRST_DIV_PARTS = 4;  // with parts the chains are short (4 heads, 32768 tokens: 267 us against 277 with a sixth)
-constexpr int SEG_GROWTH_X4 = 12;   // each range 3x the one before (in quarters)
 constexpr int SEG_MAX = 8;
 constexpr int PART0_X4 = 4;         // length of part 0 in quarters of a later part's length
+constexpr int REC_PLANNED = 66304;  // a record's share where the scratch stays the size that callers have planned with: with parts, and in the fixed array
 constexpr int NUM_SMS = 148;        // B200; the schedule is a pure function of the arguments, so that the workspace
                                     // query and the launch agree without a device being current
 struct WsLayout {
-  size_t chunk_start, w_hi, w_lo, p_hi, p_lo, tu_hi, tu_lo, scal, o_f32, qt_img, carry, m0_pack, total;
+  size_t chunk_start, recs, o_f32, qt_img, carry, m0_pack, total;
   int64_t chunks;
   int max_chunks;      // bound of the longest sequence, in chunks
   int parts;           // see ScanPlan
   int part_begin[MAX_PARTS + 1];
   int segments;        // chunk ranges handled by separate launches
-  int seg_begin[9];    // range i covers chunk offsets [seg_begin[i], seg_begin[i+1]) inside every part
+  int seg_begin[9];    // range i covers chunk offsets [seg_begin[i], seg_begin[i+1])
 };
 
 // `plain`: one part, one range, everything on the caller's stream (the schedule of the fixed-scratch entry point).
@@ -1064,15 +503,6 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   L.chunks = a.cu_seqlens ? (int64_t)a.T / C + a.n_seqs : (int64_t)a.B * ((a.T + C - 1) / C);
   const size_t recs = (size_t)L.chunks * a.Hv;
   auto up = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
-  size_t off = 0;
-  L.chunk_start = off; off = up(off + (2 * (size_t)a.n_seqs + 1 + (size_t)L.chunks) * 4);  // prefix table, chunk -> sequence map, scan order
-  L.w_hi = off; off = up(off + recs * REC_W);
-  L.w_lo = off; off = up(off + recs * REC_W);
-  L.p_hi = off; off = up(off + recs * REC_P);
-  L.p_lo = off; off = up(off + recs * REC_P);
-  L.tu_hi = off; off = up(off + recs * REC_P);
-  L.tu_lo = off; off = up(off + recs * REC_P);
-  L.scal = off; off = up(off + recs * (size_t)(SCAL_FLOATS * 4));
   // The longest chain is known for dense batches and for packed ones that come with the max_seqlen bound; otherwise only
   // its bound T is.
   const int max_chunks = ((a.cu_seqlens != nullptr && a.max_seqlen > 0 ? min(a.max_seqlen, a.T) : a.T) + C - 1) / C;
@@ -1082,18 +512,15 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   // Parts: with few long chains most SMs idle while every chain walks its chunks one after the other.  Cutting the
   // sequences into S parts that run at the same time shortens the walk S-fold at the price of a second (transition)
   // chain per later part and one GEMM-shaped fix-up; S is the largest count whose 2S-1 chains per head still get an SM
-  // each, up to 16 (4 heads, 8192 / 16384 / 32768 tokens: 123 / 174 / 267 us, with at most 8 parts 128 / 194 / 314).  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
+  // each, up to 16.  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
   // beside it.
   L.parts = 1;
   if (!plain && !push && max_chunks >= 32) {
     const int64_t per_head = (NUM_SMS / (heads_total > 0 ? heads_total : 1) + 1) / 2;  // chains per head that still get an SM each: 2S - 1
     int S = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
     while (S > 1 && max_chunks / S < 8) --S;  // a part of fewer chunks costs more in combine and fix-up than it saves
-    // Two parts take three chains a head.  They pay while pass 1 keeps a third of the SMs and the chains are long enough for the
-    // fix-up, which with a gate also holds the later part's norms back.  32 chains, two parts against one, with a gate:
-    // 5120 tokens 275 us against 269, 7168 354 / 369, 8192 394 / 406, 32768 1438 / 1488; without: 3072 175 / 172,
-    // 4096 208 / 211, 8192 361 / 392, 32768 1225 / 1480.  More chains, with a gate: 36 at 8192 tokens 422 / 433 but at 16384
-    // 809 / 795, 40 461 / 438 and 873 / 822, 48 527 / 465 and 1006 / 900.
+    // Two parts take three chains a head.  They pay while these leave a third of the SMs and the chains are long enough for the
+    // fix-up, which with a gate also holds the later part's norms back.
     const bool two = S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64);
     L.parts = S >= 3 || two ? S : 1;
   }
@@ -1105,37 +532,29 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
     const int first = L.parts > 1 ? max(2, (max_chunks - (L.parts - 1) * len + 1) & ~1) : 0;
     for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < L.parts ? first + (p - 1) * len : (1 << 24);
   }
-  int part_len = 0;  // the longest part, in chunks
-  for (int p = 0; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], max_chunks) - L.part_begin[p]);
-  L.o_f32 = off;
-  if (a.z != nullptr || L.parts > 1) off = up(off + (size_t)a.B * a.T * a.Hv * D * 4);  // rows waiting for the norm / the fix-up
-  L.qt_img = off;
-  if (L.parts > 1) off = up(off + recs * (size_t)QT_BYTES);                             // the transition chains' rows (operand images)
-  // Ranges: few long chains (fewer scan CTAs than half the SMs, or parts): pass 1 of range i+1 runs on the idle SMs
-  // while pass 2 of range i walks its chains.  The state crosses ranges through the carry buffer.  (Also switching them
-  // on for packed batches whose longest chain exceeds 1.5 times an SM's share of all chunk-heads was measured on an
-  // eighth of the heads of the 256K-token batch, 256 chains: 1.38 ms against 1.15 ms without ranges.)
-  const bool chain_bound = heads_total <= 74;
+  // Ranges: with the fused all-gather a launch of its own norms the rows and pushes them to every peer over NVLink, which takes about
+  // as long as a chain itself; with few long chains that runs beside the chains of the next range, and only the last range's push is
+  // exposed, so the ranges are equal and as many as the event pool allows.  (Without peers ranges do not pay any more: pass 1 of
+  // the whole batch takes less than the two launches and the state's way through the carry buffer, about 10 us a range.  One
+  // launch against two ranges or more: 2 x 4096 tokens x 32 heads 228 us / 244, 32768 x 4 218 / 239, 8192 x 16 196 / 217.)
   L.seg_begin[0] = 0;
-  if (plain || !(chain_bound && max_chunks >= 32)) {
-    L.segments = 1;
-    L.seg_begin[1] = 1 << 24;  // every chunk (times 64 still fits an int)
-  } else {
-    // A short first range (its pass 1 is the only one nothing overlaps), then ranges that grow geometrically: pass 1
-    // of a range must fit inside pass 2 of the range before it.
-    // With the fused all-gather the gated norm of a range also pushes that range's rows to every peer over NVLink,
-    // which takes about as long as the chain itself; only the last range's push is exposed, so the ranges are equal
-    // and as many as the event pool allows instead of growing.
-    const int first_div = L.parts > 1 ? SEG_FIRST_DIV_PARTS : SEG_FIRST_DIV;
-    int len = push ? (part_len + SEG_MAX - 1) / SEG_MAX : max(1, (part_len + first_div - 1) / first_div);
+  L.segments = 1;
+  L.seg_begin[1] = 1 << 24;  // every chunk (times 64 still fits an int)
+  if (!plain && push && heads_total <= 74 && max_chunks >= 32) {
+    const int len = (max_chunks + SEG_MAX - 1) / SEG_MAX;
     L.segments = 0;
-    while (L.seg_begin[L.segments] < part_len) {
-      int next = L.seg_begin[L.segments] + len;
-      if (L.segments == SEG_MAX - 1 || next >= part_len) next = part_len;
-      L.seg_begin[++L.segments] = next;
-      if (!push) len = max(len + 1, len * SEG_GROWTH_X4 / 4);
+    while (L.seg_begin[L.segments] < max_chunks) {
+      L.seg_begin[L.segments + 1] = L.segments == SEG_MAX - 1 ? max_chunks : min(max_chunks, L.seg_begin[L.segments] + len);
+      ++L.segments;
     }
   }
+  size_t off = 0;
+  L.chunk_start = off; off = up(off + (2 * (size_t)a.n_seqs + 1 + (size_t)L.chunks) * 4);  // prefix table, chunk -> sequence map, scan order
+  L.recs = off; off = up(off + recs * (size_t)(plain || L.parts > 1 ? REC_PLANNED : REC_BYTES));
+  L.o_f32 = off;
+  if (L.parts > 1 || a.z != nullptr) off = up(off + (size_t)a.B * a.T * a.Hv * D * 4);  // rows waiting for the fix-up / the norm
+  L.qt_img = off;
+  if (L.parts > 1) off = up(off + recs * (size_t)QT_BYTES);                             // the transition chains' rows (operand images)
   L.carry = off;
   if (L.segments > 1 || L.parts > 1) off = up(off + (size_t)a.n_seqs * (2 * L.parts - 1) * a.Hv * D * D * 4);
   L.m0_pack = off;
@@ -1161,15 +580,14 @@ int prefill_tc_launch_count(const AveGdnArgs& a, bool plain) {
   if (L.chunks == 0 || a.n_seqs == 0) return 0;
   const bool tables = needs_tables(a);
   const bool push = a.o_peers != nullptr && a.n_peers > 1;
-  const int norm_launch = (push || a.B == 1) ? 1 : a.B;  // norm_rows: one launch, or one per batch row
   int n = tables ? 1 : 0;                                  // chunk tables
   n += 2 * L.segments;                                     // pass 1 and pass 2 of every range
-  if (a.z != nullptr) n += (a.cu_seqlens == nullptr ? L.segments : 1) * norm_launch;
+  if (a.z != nullptr) n += (a.cu_seqlens == nullptr ? L.segments : 1) * (push || a.B == 1 ? 1 : a.B);  // norm_rows: one launch, or one per batch row
   if (L.parts > 1) n += 2;                                 // combine and fix-up
   return n;
 }
 
-// Helper streams and events for the range-overlapped schedule.  Pass 2 runs on a high-priority stream so that, when a
+// Helper streams and events for the ranges.  Pass 2 runs on a high-priority stream so that, when a
 // range's pass 1 completes and both its pass 2 and the next range's pass 1 become runnable, the few whole-SM pass-2
 // CTAs are placed first.  Each device owns a small pool of such sets; a call takes the set its stream hashes to, so
 // calls on different streams usually overlap instead of queueing behind one another's helper streams.  A device's sets
@@ -1178,7 +596,7 @@ int prefill_tc_launch_count(const AveGdnArgs& a, bool plain) {
 // the time of the call).
 struct SideSet {
   cudaStream_t prep = nullptr, scan = nullptr, norm = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr, join_norm = nullptr, chains_done = nullptr, combined = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr, join_norm = nullptr;
   cudaEvent_t done[SEG_MAX] = {}, scanned[SEG_MAX] = {};
   bool ready = false;
 };
@@ -1194,7 +612,7 @@ static void destroy_side_set(SideSet& s) {
   if (s.prep) cudaStreamDestroy(s.prep);
   if (s.scan) cudaStreamDestroy(s.scan);
   if (s.norm) cudaStreamDestroy(s.norm);
-  for (cudaEvent_t e : {s.fork, s.join, s.join_norm, s.chains_done, s.combined}) if (e) cudaEventDestroy(e);
+  for (cudaEvent_t e : {s.fork, s.join, s.join_norm}) if (e) cudaEventDestroy(e);
   for (int i = 0; i < SEG_MAX; ++i) { if (s.done[i]) cudaEventDestroy(s.done[i]); if (s.scanned[i]) cudaEventDestroy(s.scanned[i]); }
   s = SideSet{};
 }
@@ -1211,8 +629,6 @@ static SideSet* side_set(DeviceSide& dev, cudaStream_t stream) {
   ok = ok && cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming) == cudaSuccess;
   ok = ok && cudaEventCreateWithFlags(&s.join_norm, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&s.chains_done, cudaEventDisableTiming) == cudaSuccess;
-  ok = ok && cudaEventCreateWithFlags(&s.combined, cudaEventDisableTiming) == cudaSuccess;
   for (int i = 0; i < SEG_MAX; ++i) {
     ok = ok && cudaEventCreateWithFlags(&s.done[i], cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&s.scanned[i], cudaEventDisableTiming) == cudaSuccess;
@@ -1223,7 +639,7 @@ static SideSet* side_set(DeviceSide& dev, cudaStream_t stream) {
   return &slot;
 }
 
-// Gated RMSNorm over the fp32 output for tokens [t_begin, t_end) of every batch row, one launch.
+// Gated RMSNorm over the fp32 output for tokens [t_begin, t_end) of every batch row.
 static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, cudaStream_t stream) {
   if (t_end <= t_begin) return AVE_GDN_OK;
   AveGdnNormArgs nb{};
@@ -1262,14 +678,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   if (L.chunks == 0 || a.n_seqs == 0) return AVE_GDN_OK;
   char* ws = reinterpret_cast<char*>(a.workspace);
   int32_t* chunk_start = needs_tables(a) ? reinterpret_cast<int32_t*>(ws + L.chunk_start) : nullptr;
-  PrepOut po;
-  po.w_hi = reinterpret_cast<__nv_bfloat16*>(ws + L.w_hi);
-  po.w_lo = reinterpret_cast<__nv_bfloat16*>(ws + L.w_lo);
-  po.p_hi = reinterpret_cast<__nv_bfloat16*>(ws + L.p_hi);
-  po.p_lo = reinterpret_cast<__nv_bfloat16*>(ws + L.p_lo);
-  po.tu_hi = reinterpret_cast<__nv_bfloat16*>(ws + L.tu_hi);
-  po.tu_lo = reinterpret_cast<__nv_bfloat16*>(ws + L.tu_lo);
-  po.scal = reinterpret_cast<float*>(ws + L.scal);
+  uint8_t* recs = reinterpret_cast<uint8_t*>(ws + L.recs);
 
   GdnMaps maps;
   {
@@ -1292,9 +701,9 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   DeviceSide& dev = g_side[dev_id];
   std::lock_guard<std::mutex> guard(dev.mu);
   if (!dev.attr_set) {
-    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PREP_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILES_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
@@ -1303,7 +712,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   if (chunk_start != nullptr) {
     AVE_CUDA_TRY(launch_after(chunk_table_tc_kernel, 1, a.n_seqs <= 256 ? 256 : 1024, 0, stream, a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status));
   }
-  float* o_f32 = (a.z != nullptr || L.parts > 1) ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
+  float* o_f32 = L.parts > 1 || a.z != nullptr ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
   uint8_t* qt_img = L.parts > 1 ? reinterpret_cast<uint8_t*>(ws + L.qt_img) : nullptr;
   float* carry = reinterpret_cast<float*>(ws + L.carry);
   uint8_t* m0_pack = reinterpret_cast<uint8_t*>(ws + L.m0_pack);
@@ -1311,59 +720,41 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   ScanPlan plan;
   plan.parts = L.parts;
   for (int p = 0; p <= MAX_PARTS; ++p) plan.part_begin[p] = L.part_begin[p];
-  const unsigned prep_rows = (unsigned)(a.Hk * ((a.Hv / a.Hk + 1) / 2));  // a pass-1 CTA takes up to two value heads of a key head
+  const int64_t tile_rows = (int64_t)a.Hk * ((a.Hv / a.Hk + 1) / 2);  // a unit of pass 1 takes up to two value heads of a key head
+  auto tiles_grid = [&](int64_t chunks) { return dim3((unsigned)min(chunks * tile_rows, (int64_t)(2 * NUM_SMS))); };  // persistent, two CTAs an SM
   const unsigned scan_grid = (unsigned)a.n_seqs * (unsigned)(2 * L.parts - 1) * (unsigned)a.Hv;
-  const int part0_tokens = L.parts > 1 ? min(a.T, L.part_begin[1] * C) : a.T;  // tokens no fix-up touches (dense layout)
-
-  // combine + fix-up of the later parts, after every chain has finished (parts > 1 only).  The image of M0(1) comes from
-  // the scan, so with two parts the fix-up needs nothing from the combine, which then only produces the final states
-  // and runs on `side_stream` (when given) beside the fix-up.
-  auto finish_parts = [&](cudaStream_t s, cudaStream_t side_stream, cudaEvent_t scanned, cudaEvent_t combined) -> int {
-    if (L.parts <= 1) return AVE_GDN_OK;
-    plan.r0 = 0; plan.rn = 1 << 24;
-    const int cols = (int64_t)a.n_seqs * a.Hv * (D / 4) <= NUM_SMS ? 4 : 8;
-    const auto combine = cols == 4 ? part_combine_kernel<4> : part_combine_kernel<8>;
-    const dim3 cgrid((unsigned)(D / cols), (unsigned)a.Hv, (unsigned)a.n_seqs);
-    const bool beside = L.parts == 2 && side_stream != nullptr;
-    if (beside) {
-      AVE_CUDA_TRY(cudaEventRecord(scanned, s));
-      AVE_CUDA_TRY(cudaStreamWaitEvent(side_stream, scanned, 0));
-      combine<<<cgrid, 256, COMBINE_SMEM, side_stream>>>(a, chunk_start, carry, m0_pack, plan);
-      AVE_CUDA_TRY(cudaGetLastError());
-      AVE_CUDA_TRY(cudaEventRecord(combined, side_stream));
-    } else {
-      combine<<<cgrid, 256, COMBINE_SMEM, s>>>(a, chunk_start, carry, m0_pack, plan);
-      AVE_CUDA_TRY(cudaGetLastError());
-    }
-    int part_len = 0;  // the longest of the later parts
-    for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
-    const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
-    int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of the SMs
-    split = max(1, min(split, (part_len + 1) / 2));
-    part_finish_kernel<<<dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, s>>>(
-        a, chunk_start, o_f32, qt_img, m0_pack, plan);
-    AVE_CUDA_TRY(cudaGetLastError());
-    if (beside) AVE_CUDA_TRY(cudaStreamWaitEvent(s, combined, 0));
-    return AVE_GDN_OK;
-  };
+  const auto scan = L.parts > 1 ? chunk_scan_kernel<true> : chunk_scan_kernel<false>;
 
   SideSet* side = L.segments > 1 ? side_set(dev, stream) : nullptr;
   if (side == nullptr) {
     // one launch per pass on the caller's stream
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
-    AVE_CUDA_TRY(launch_after(chunk_prep_kernel, dim3((unsigned)L.chunks, prep_rows), PREP_THREADS, PREP_SMEM, stream, a, chunk_start, po, plan, 0));
-    AVE_CUDA_TRY(launch_after(L.parts > 1 ? chunk_scan_tc_kernel<true> : chunk_scan_tc_kernel<false>, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps,
-                              chunk_start, po.w_hi, po.w_lo, po.p_hi, po.p_lo, po.tu_hi, po.tu_lo, po.scal, o_f32, qt_img, carry, m0_pack, seq_order, plan));
+    AVE_CUDA_TRY(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
+    AVE_CUDA_TRY(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));
     if (a.z != nullptr) {
-      // packed layouts: the norm covers every row (rows of later parts are rewritten by the fix-up, which runs after it)
-      const int rc = norm_rows(a, o_f32, a.token_begin, a.cu_seqlens ? a.T : part0_tokens, stream);
+      // dense layouts: the tokens no fix-up touches; packed ones: every row (those of later parts are rewritten by the fix-up behind it)
+      const int rc = norm_rows(a, o_f32, a.token_begin, a.cu_seqlens == nullptr && L.parts > 1 ? min(a.T, L.part_begin[1] * C) : a.T, stream);
       if (rc != AVE_GDN_OK) return rc;
     }
-    return finish_parts(stream, nullptr, nullptr, nullptr);
+    if (L.parts <= 1) return AVE_GDN_OK;
+    // combine and fix-up of the later parts
+    const int cols = (int64_t)a.n_seqs * a.Hv * (D / 4) <= NUM_SMS ? 4 : 8;
+    const auto combine = cols == 4 ? part_combine_kernel<4> : part_combine_kernel<8>;
+    combine<<<dim3((unsigned)(D / cols), (unsigned)a.Hv, (unsigned)a.n_seqs), 256, COMBINE_SMEM, stream>>>(a, chunk_start, carry, m0_pack, plan);
+    AVE_CUDA_TRY(cudaGetLastError());
+    int part_len = 0;  // the longest of the later parts
+    for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
+    const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
+    int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of the SMs
+    split = max(1, min(split, (part_len + 1) / 2));
+    part_finish_kernel<<<dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream>>>(
+        a, chunk_start, o_f32, qt_img, m0_pack, plan);
+    AVE_CUDA_TRY(cudaGetLastError());
+    return AVE_GDN_OK;
   }
 
   // Pass 1 of all ranges back to back on one helper stream, pass 2 of range i on a second once pass 1 of range i is
-  // done, and (dense layouts) the gated norm of part 0's rows of range i on a third once pass 2 of range i is done; all
+  // done, and (dense layouts) the gated norm of range i on a third once pass 2 of range i is done; all
   // fork from the caller's stream and join back into it through events.  After an error the joins are still enqueued,
   // so that a surrounding stream capture stays well formed.
   const bool norm_per_range = a.z != nullptr && a.cu_seqlens == nullptr;
@@ -1376,25 +767,20 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   for (int i = 0; i < L.segments && rc == AVE_GDN_OK; ++i) {
     plan.r0 = L.seg_begin[i]; plan.rn = L.seg_begin[i + 1] - L.seg_begin[i];
     if (plan.rn <= 0) continue;
-    chunk_prep_kernel<<<dim3((unsigned)(a.n_seqs * L.parts * plan.rn), prep_rows), PREP_THREADS, PREP_SMEM, side->prep>>>(
-        a, chunk_start, po, plan, 1);
+    chunk_tiles_kernel<<<tiles_grid((int64_t)a.n_seqs * plan.rn), TILES_THREADS, TILES_SMEM, side->prep>>>(a, chunk_start, recs, plan, a.n_seqs * plan.rn, 1);
     if (!step(cudaGetLastError())) break;
     if (!step(cudaEventRecord(side->done[i], side->prep))) break;
     if (!step(cudaStreamWaitEvent(side->scan, side->done[i], 0))) break;
-    (L.parts > 1 ? chunk_scan_tc_kernel<true> : chunk_scan_tc_kernel<false>)<<<scan_grid, SCAN_THREADS, SCAN_SMEM, side->scan>>>(
-        a, maps, chunk_start, po.w_hi, po.w_lo, po.p_hi, po.p_lo, po.tu_hi, po.tu_lo, po.scal, o_f32, qt_img, carry, m0_pack, seq_order, plan);
+    scan<<<scan_grid, SCAN_THREADS, SCAN_SMEM, side->scan>>>(a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan);
     if (!step(cudaGetLastError())) break;
     if (norm_per_range) {
       if (!step(cudaEventRecord(side->scanned[i], side->scan))) break;
       if (!step(cudaStreamWaitEvent(side->norm, side->scanned[i], 0))) break;
-      const int nrc = norm_rows(a, o_f32, min(part0_tokens, plan.r0 * C), min(part0_tokens, (plan.r0 + plan.rn) * C), side->norm);
+      const int nrc = norm_rows(a, o_f32, min(a.T, plan.r0 * C), min(a.T, (plan.r0 + plan.rn) * C), side->norm);
       if (nrc != AVE_GDN_OK && rc == AVE_GDN_OK) rc = nrc;
     }
   }
-  if (rc == AVE_GDN_OK) {
-    if (a.z != nullptr && !norm_per_range) rc = norm_rows(a, o_f32, a.token_begin, a.T, side->scan);  // packed layout: after the last scan
-    if (rc == AVE_GDN_OK) rc = finish_parts(side->scan, side->prep, side->chains_done, side->combined);
-  }
+  if (rc == AVE_GDN_OK && a.z != nullptr && !norm_per_range) rc = norm_rows(a, o_f32, a.token_begin, a.T, side->scan);  // packed layout: after the last scan
   step(cudaEventRecord(side->join, side->scan));
   step(cudaStreamWaitEvent(stream, side->join, 0));
   step(cudaEventRecord(side->join_norm, norm_per_range ? side->norm : side->prep));

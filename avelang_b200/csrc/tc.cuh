@@ -179,6 +179,16 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo
   d |= (uint64_t)2 << 61;  // 128-byte swizzle
   return d;
 }
+// K-major operand without swizzle: 8x8 core matrices of 128 contiguous bytes (row after row), `lbo` bytes from one to the next
+// along K and `sbo` bytes along M or N.
+__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3fffu);
+  d |= (uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16;
+  d |= (uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32;
+  d |= (uint64_t)1 << 46;  // descriptor version of this architecture
+  return d;
+}
 // 32-bit instruction descriptor for kind::f16 with fp32 accumulate.  fmt: 0 = f16, 1 = bf16.
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int a_fmt, int b_fmt, bool a_mn_major, bool b_mn_major,
                                                  bool a_neg = false, bool b_neg = false) {

@@ -17,10 +17,8 @@ __device__ __forceinline__ void head_sync(int hh) {
   asm volatile("bar.sync %0, 128;" ::"r"(1 + hh) : "memory");
 }
 
-// The diagonal blocks 2 part and 2 part + 1 in place: (I + A_bb)^-1, transposed.  One warp each, a lane per column.
-__device__ __forceinline__ void wy_invert(uint8_t* frag, int part, int lane) {
-  const int b = 2 * part + (lane >> 4), k = lane & 15;
-  float* ad = reinterpret_cast<float*>(frag + WY_DIAG) + b * 16 * AD_LD;
+// A diagonal block in place: (I + A_bb)^-1, transposed.  A lane per column k; lanes that are not `owner` repeat another's work.
+__device__ __forceinline__ void wy_invert_block(float* ad, int k, bool owner) {
   float x[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
@@ -36,9 +34,14 @@ __device__ __forceinline__ void wy_invert(uint8_t* frag, int part, int lane) {
     x[i] = s0 + s1;
   }
   __syncwarp();  // every lane has read the block: its inverse, transposed, takes its place
+  if (owner)
 #pragma unroll
-  for (int i4 = 0; i4 < 4; ++i4)
-    *reinterpret_cast<float4*>(ad + k * AD_LD + 4 * i4) = make_float4(x[4 * i4], x[4 * i4 + 1], x[4 * i4 + 2], x[4 * i4 + 3]);
+    for (int i4 = 0; i4 < 4; ++i4)
+      *reinterpret_cast<float4*>(ad + k * AD_LD + 4 * i4) = make_float4(x[4 * i4], x[4 * i4 + 1], x[4 * i4 + 2], x[4 * i4 + 3]);
+}
+// The diagonal blocks 2 part and 2 part + 1, by one warp.
+__device__ __forceinline__ void wy_invert(uint8_t* frag, int part, int lane) {
+  wy_invert_block(reinterpret_cast<float*>(frag + WY_DIAG) + (2 * part + (lane >> 4)) * 16 * AD_LD, lane & 15, true);
 }
 // Row R of 16x16 blocks of T: T_rc = -(sum_{c < s <= r} T_rs A_sc) D_c, D_c = (I + A_cc)^-1; every block stays in accumulators.
 template <int R>
