@@ -189,15 +189,16 @@ namespace {
 // reads for 32 multiply-adds.
 constexpr int COMBINE_PITCH = 132;
 constexpr int COMBINE_F = D * COMBINE_PITCH * 4, COMBINE_CUR = (D + 4) * 8 * 4;  // (a gap of one row between the shares of the contraction)
-constexpr int COMBINE_STAGES = 3;
-constexpr size_t COMBINE_SMEM = COMBINE_STAGES * (size_t)COMBINE_F + 2 * COMBINE_CUR;
+constexpr size_t combine_smem(int stages) { return stages * (size_t)COMBINE_F + 2 * COMBINE_CUR; }
 // COLS columns a CTA: 8, or 4 while that still is one wave (its step is shorter, but F passes through twice as many SMs).
 // Bound by shared-memory reads and the issue of the copies, 2 us a step: 15 steps for 4 heads 30 us (42 us when the lanes of a
 // quarter warp read one row at four offsets of 128 bytes, 8 wavefronts a load; 55 us with one row a thread, scalar reads and F
-// staged through registers).
-template <int COLS>
+// staged through registers).  STAGES of the ring: three, or one where two parts leave a single step, so that three CTAs share an SM
+// (32 heads: 24 us with three stages and 3.5 waves).
+template <int COLS, int STAGES>
 __global__ void __launch_bounds__(256)
 part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* carry, uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
+  pdl_wait();
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int cb = blockIdx.x, h = blockIdx.y, n = blockIdx.z, tid = threadIdx.x;
   if (batch_rejected(a, chunk_start)) return;
@@ -214,7 +215,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   auto tile_of = [&](int chain) { return carry + (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D); };
   constexpr int SPLIT = 16 / COLS, SHARE = D / SPLIT;  // threads that share a contraction, and its length for each
   auto cur_at = [&](int b, int k, int j) -> float& {
-    return reinterpret_cast<float*>(smem_raw + COMBINE_STAGES * COMBINE_F + b * COMBINE_CUR)[(k + k / SHARE) * COLS + j];
+    return reinterpret_cast<float*>(smem_raw + STAGES * COMBINE_F + b * COMBINE_CUR)[(k + k / SHARE) * COLS + j];
   };
   const uint32_t sb = tc::smem_u32(smem_raw);
   // this thread: rows k and k + 64, columns j0 .. j0 + 3, contraction indices d0 .. d0 + SHARE - 1
@@ -226,7 +227,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
 #pragma unroll
     for (int i = 0; i < D * D / 4 / 256; ++i) {
       const int e = tid + 256 * i, row = e >> 5, c4 = e & 31;
-      cp16(sb + (p % COMBINE_STAGES) * COMBINE_F + row * COMBINE_PITCH * 4 + c4 * 16, F + 4 * e, true);
+      cp16(sb + (p % STAGES) * COMBINE_F + row * COMBINE_PITCH * 4 + c4 * 16, F + 4 * e, true);
     }
     cp_commit();
   };
@@ -234,17 +235,17 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
     return p < active ? *reinterpret_cast<const float4*>(tile_of(2 * p - 1) + (int64_t)(k + 64 * dh) * D + cb * COLS + j0) : make_float4(0.f, 0.f, 0.f, 0.f);
   };
   fetch(1);
-  fetch(2);
+  if (STAGES > 1) fetch(2);
   float4 psi_next = psi_of(1);
   for (int e = tid; e < D * COLS; e += 256) cur_at(0, e / COLS, e % COLS) = tile_of(0)[(e / COLS) * D + cb * COLS + e % COLS];
   int b = 0;
   for (int p = 1; p < active; ++p) {
-    cp_wait<1>();
+    cp_wait<(STAGES > 1 ? 1 : 0)>();
     __syncthreads();  // F_p and cur are complete; F_{p-1} has been read
-    fetch(p + 2);
+    if (STAGES > 1) fetch(p + 2);
     const float4 psi = psi_next;
     psi_next = psi_of(p + 1);
-    const float* F0 = reinterpret_cast<const float*>(smem_raw + (p % COMBINE_STAGES) * COMBINE_F) + k * COMBINE_PITCH + d0;
+    const float* F0 = reinterpret_cast<const float*>(smem_raw + (p % STAGES) * COMBINE_F) + k * COMBINE_PITCH + d0;
     float2 x[2][2] = {};
 #pragma unroll 4
     for (int d = 0; d < SHARE; d += 4) {
@@ -308,6 +309,7 @@ __global__ void __launch_bounds__(FIN_THREADS, 1)
 part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* o_f32,
                    const uint8_t* qt_img, const uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
+  pdl_wait();
   uint8_t* smem = tc::align1024(smem_raw);
   float* stage = reinterpret_cast<float*>(smem + FIN_STAGE);  // [128 tokens][FIN_PITCH] product rows
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FIN_BARS);
@@ -705,8 +707,9 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(chunk_scan_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_SMEM));
     AVE_CUDA_TRY(cudaFuncSetAttribute(part_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FIN_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)COMBINE_SMEM));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<4, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)combine_smem(3)));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<8, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)combine_smem(3)));
+    AVE_CUDA_TRY(cudaFuncSetAttribute(part_combine_kernel<8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)combine_smem(1)));
     dev.attr_set = true;
   }
   if (chunk_start != nullptr) {
@@ -731,26 +734,41 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
     AVE_CUDA_TRY(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
     AVE_CUDA_TRY(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));
+    if (L.parts <= 1) return a.z != nullptr ? norm_rows(a, o_f32, a.token_begin, a.T, stream) : AVE_GDN_OK;
+    // Parts: the combine and the fix-up of the later ones.  Dense layouts: the gated norm of the tokens no fix-up touches runs beside them,
+    // forked to a helper stream and joined back (the combine is all latency); packed layouts: the norm covers every row, and the fix-up
+    // behind it rewrites those of later parts.
+    const bool beside = a.z != nullptr && a.cu_seqlens == nullptr;
+    side = beside ? side_set(dev, stream) : nullptr;
+    int rc = AVE_GDN_OK;
     if (a.z != nullptr) {
-      // dense layouts: the tokens no fix-up touches; packed ones: every row (those of later parts are rewritten by the fix-up behind it)
-      const int rc = norm_rows(a, o_f32, a.token_begin, a.cu_seqlens == nullptr && L.parts > 1 ? min(a.T, L.part_begin[1] * C) : a.T, stream);
-      if (rc != AVE_GDN_OK) return rc;
+      const int end = beside ? min(a.T, L.part_begin[1] * C) : a.T;
+      if (side != nullptr) {
+        AVE_CUDA_TRY(cudaEventRecord(side->fork, stream));
+        AVE_CUDA_TRY(cudaStreamWaitEvent(side->norm, side->fork, 0));
+        rc = norm_rows(a, o_f32, 0, end, side->norm);
+      } else {
+        rc = norm_rows(a, o_f32, a.token_begin, end, stream);
+      }
     }
-    if (L.parts <= 1) return AVE_GDN_OK;
-    // combine and fix-up of the later parts
-    const int cols = (int64_t)a.n_seqs * a.Hv * (D / 4) <= NUM_SMS ? 4 : 8;
-    const auto combine = cols == 4 ? part_combine_kernel<4> : part_combine_kernel<8>;
-    combine<<<dim3((unsigned)(D / cols), (unsigned)a.Hv, (unsigned)a.n_seqs), 256, COMBINE_SMEM, stream>>>(a, chunk_start, carry, m0_pack, plan);
-    AVE_CUDA_TRY(cudaGetLastError());
-    int part_len = 0;  // the longest of the later parts
-    for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
-    const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
-    int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of the SMs
-    split = max(1, min(split, (part_len + 1) / 2));
-    part_finish_kernel<<<dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream>>>(
-        a, chunk_start, o_f32, qt_img, m0_pack, plan);
-    AVE_CUDA_TRY(cudaGetLastError());
-    return AVE_GDN_OK;
+    auto step = [&](cudaError_t e) { if (e != cudaSuccess && rc == AVE_GDN_OK) rc = cuda_fail(e); };
+    if (rc == AVE_GDN_OK) {
+      const int cols = (int64_t)a.n_seqs * a.Hv * (D / 4) <= NUM_SMS ? 4 : 8, stages = cols == 8 && L.parts == 2 ? 1 : 3;
+      const auto combine = cols == 4 ? part_combine_kernel<4, 3> : stages == 1 ? part_combine_kernel<8, 1> : part_combine_kernel<8, 3>;
+      step(launch_after(combine, dim3((unsigned)(D / cols), (unsigned)a.Hv, (unsigned)a.n_seqs), 256, combine_smem(stages), stream, a, chunk_start, carry, m0_pack, plan));
+      int part_len = 0;  // the longest of the later parts
+      for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
+      const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
+      int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of the SMs
+      split = max(1, min(split, (part_len + 1) / 2));
+      step(launch_after(part_finish_kernel, dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream,
+                        a, chunk_start, o_f32, qt_img, m0_pack, plan));
+    }
+    if (side != nullptr) {
+      step(cudaEventRecord(side->join_norm, side->norm));
+      step(cudaStreamWaitEvent(stream, side->join_norm, 0));
+    }
+    return rc;
   }
 
   // Pass 1 of all ranges back to back on one helper stream, pass 2 of range i on a second once pass 1 of range i is
