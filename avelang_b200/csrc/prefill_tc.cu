@@ -291,30 +291,32 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
   }
 }
 
-// Fix-up of the parts after the first.  For 128 tokens (two chunks of one part) of one value head,
-//   o = o_local + qt M0(part)        (qt = the transition chain's rows, [128 tokens][128 d_k])
-// is one 128x128x128 product on tcgen05 with both operands as bf16 hi+lo pairs (hi hi + hi lo + lo hi): A = the qt^T
-// images the scan wrote (MN-major, brought in by bulk copies), B = the image of M0(part).  The accumulator (a thread
-// per token row) is staged through shared memory so that everything that touches global memory runs in the layout of
+// Fix-up of the parts after the first.  For a chunk of 64 tokens of one value head,
+//   o = o_local + qt M0(part)        (qt = the transition chain's rows, [64 tokens][128 d_k])
+// is one product on tcgen05, transposed like the scan's (128 d_v lanes x 64 tokens), with both operands as bf16 hi+lo pairs (hi hi +
+// hi lo + lo hi): A = the image of M0(part), B = the qt^T images the scan wrote (MN-major, brought in by bulk copies).  The
+// accumulator is staged in the place of B, so that everything that touches global memory runs in the layout of
 // the streaming norm kernel: a half-warp per token row, 8 adjacent features per lane, 16- and 32-byte accesses, the
 // RMS over d_v as four shuffles.  (Reading o_local and z straight from the accumulator's layout, a row or a column per
 // thread, measured three to four times slower: 2- or 4-byte accesses and tens of instructions per element.)
-// A CTA serves one (sequence, part, head) and walks every `gridDim.x`-th pair of chunks with the M0 image resident; the
-// images of the next pair are in flight while the current pair's rows are streamed.
-constexpr int FIN_THREADS = 512;
-constexpr int FIN_PITCH = 132;  // floats per staged row: 16-byte aligned rows that spread over the banks
-constexpr int FIN_A = 0, FIN_B = 65536, FIN_STAGE = FIN_B + PACK_BYTES, FIN_BARS = FIN_STAGE + 128 * FIN_PITCH * 4;
+// A CTA serves one (sequence, part, head) and walks every `gridDim.x`-th chunk with the M0 image resident.  Bound by memory traffic
+// (96 KB a chunk with a gate) and by the serial steps of a chunk, which two CTAs per SM overlap: 8192
+// tokens x 32 heads 51 us (55 with pairs of chunks, one CTA an SM), 5 TB/s while it streams; a whole call 323 -> 318.
+constexpr int FIN_THREADS = 256;
+constexpr int FIN_Q = 0, FIN_M0 = QT_BYTES, FIN_BARS = FIN_M0 + PACK_BYTES;
 constexpr size_t FIN_SMEM = FIN_BARS + 64 + 1024;
-__global__ void __launch_bounds__(FIN_THREADS, 1)
+static_assert(C * D * 4 <= QT_BYTES, "the rows are staged in the place of the qt images");
+__global__ void __launch_bounds__(FIN_THREADS, 2)
 part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* o_f32,
                    const uint8_t* qt_img, const uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
   pdl_wait();
   uint8_t* smem = tc::align1024(smem_raw);
-  float* stage = reinterpret_cast<float*>(smem + FIN_STAGE);  // [128 tokens][FIN_PITCH] product rows
+  float* stage = reinterpret_cast<float*>(smem + FIN_Q);  // [64 tokens][128] product rows, neighbouring 16-byte pieces swapped by token
+  auto piece16 = [&](int t, int p) { return stage + t * D + 4 * (p ^ (((p >> 3) ^ t) & 1)); };
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FIN_BARS);
-  uint64_t* b_bar = bars;
-  uint64_t* a_full = bars + 1;
+  uint64_t* m0_full = bars;
+  uint64_t* q_full = bars + 1;
   uint64_t* mma_bar = bars + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -324,43 +326,35 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
   const int seq_chunks = (sp.len + C - 1) / C;
-  const int c_begin = plan.part_begin[part], c_end = min(plan.part_begin[part + 1], seq_chunks);
-  const int n_pairs = (c_end - c_begin + 1) / 2;  // part boundaries are even, so a pair never straddles two parts
-  if ((int)blockIdx.x >= n_pairs) return;
+  const int c_end = min(plan.part_begin[part + 1], seq_chunks), c_begin = plan.part_begin[part] + (int)blockIdx.x, stride = gridDim.x;
+  if (c_begin >= c_end) return;
   const int slot = a.state_indices ? a.state_indices[n] : n;
   const bool skipped = slot < 0 || slot >= a.num_slots;  // the scan skipped the sequence: its rows are zero
   const int64_t rec0 = first_record(a, chunk_start, n);  // record of the sequence's chunk 0
-  const int stride = gridDim.x;
 
-  auto load_qt = [&](int pair) {  // called by one thread
-    const int c0 = c_begin + 2 * pair, cnt = min(2, c_end - c0);
-    tc::mbar_expect_tx(a_full, (uint32_t)(cnt * QT_BYTES));
-    for (int i = 0; i < cnt; ++i) {
-      const uint8_t* img = qt_img + ((rec0 + c0 + i) * a.Hv + h) * (int64_t)QT_BYTES;
-      tc::bulk_load(smem + FIN_A + i * 16384, img, 16384, a_full);                   // hi: [chunk 0 | chunk 1]
-      tc::bulk_load(smem + FIN_A + 32768 + i * 16384, img + 16384, 16384, a_full);   // lo: [chunk 0 | chunk 1]
-    }
+  auto load_qt = [&](int c) {  // called by one thread
+    tc::mbar_expect_tx(q_full, QT_BYTES);
+    tc::bulk_load(smem + FIN_Q, qt_img + ((rec0 + c) * a.Hv + h) * (int64_t)QT_BYTES, QT_BYTES, q_full);
   };
   if (tid == 0) {
-    tc::mbar_init(b_bar, 1);
-    tc::mbar_init(a_full, 1);
+    tc::mbar_init(m0_full, 1);
+    tc::mbar_init(q_full, 1);
     tc::mbar_init(mma_bar, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
     if (!skipped) {
       const uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1) + (part - 1)) * a.Hv + h) * (int64_t)PACK_BYTES;
-      tc::mbar_expect_tx(b_bar, PACK_BYTES);
-      tc::bulk_load(smem + FIN_B, img, PACK_BYTES, b_bar);
-      load_qt(blockIdx.x);
+      tc::mbar_expect_tx(m0_full, PACK_BYTES);
+      tc::bulk_load(smem + FIN_M0, img, PACK_BYTES, m0_full);
+      load_qt(c_begin);
     }
   }
-  if (warp == 1) tc::tmem_alloc(tmem_slot, 128);
+  if (warp == 1) tc::tmem_alloc(tmem_slot, 64);
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tm = *tmem_slot;
-  const int quarter = warp & 3, colq = warp >> 2;  // accumulator: TMEM lane quarter (token rows) and column quarter of this warp
-  const int hw = tid >> 4, sub = tid & 15;          // streaming pass: half-warp index (32 of them) and lane inside it
+  const int hw = tid >> 4, sub = tid & 15;  // streaming pass: half-warp index (16 of them) and lane inside it
   const bool gate_first = (a.flags & AVE_GDN_FLAG_GATE_FIRST) != 0;
   float2 wv[4];
 #pragma unroll
@@ -369,16 +363,15 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   bool ok = true;
 
   int it = 0;
-  for (int pair = blockIdx.x; pair < n_pairs && ok; pair += stride, ++it) {
-    const int c0 = c_begin + 2 * pair;
-    const int64_t tok0 = sp.t0 + (int64_t)c0 * C;
-    const int rows = min(min(2, c_end - c0) * C, sp.len - c0 * C);
-    // the rows this half-warp will stream (hw, hw + 32, hw + 64, hw + 96) are fetched before the product is waited for
+  for (int c = c_begin; c < c_end && ok; c += stride, ++it) {
+    const int64_t tok0 = sp.t0 + (int64_t)c * C;
+    const int rows = min(C, sp.len - c * C);
+    // the rows this half-warp will stream (hw, hw + 16, hw + 32, hw + 48) are fetched before the product is waited for
     float4 ol[4][2];
     uint4 zraw[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      const int r = hw + 32 * u;
+      const int r = hw + 16 * u;
       ol[u][0] = ol[u][1] = make_float4(0.f, 0.f, 0.f, 0.f);
       zraw[u] = make_uint4(0u, 0u, 0u, 0u);
       if (!skipped && r < rows) {
@@ -392,19 +385,19 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
     }
     if (!skipped) {
       if (warp == 0) {
-        bool landed = it > 0 || tc::mbar_wait_warp(b_bar, 0, abort_flag);
-        landed = landed && tc::mbar_wait_warp(a_full, (uint32_t)it & 1u, abort_flag);
+        bool landed = it > 0 || tc::mbar_wait_warp(m0_full, 0, abort_flag);
+        landed = landed && tc::mbar_wait_warp(q_full, (uint32_t)it & 1u, abort_flag);
         tc::tc_fence_after_sync();
         if (landed && tc::elect_one()) {
-          constexpr uint32_t idesc = tc::idesc_f16(128, 128, 1, 1, true, false);  // A MN-major (token rows), B K-major
-          const uint32_t sa = tc::smem_u32(smem + FIN_A), sb = tc::smem_u32(smem + FIN_B);
-#pragma unroll
+          constexpr uint32_t idesc = tc::idesc_f16(128, 64, 1, 1, false, true);  // A K-major, B MN-major (token rows)
+          const uint32_t sq = tc::smem_u32(smem + FIN_Q), sm = tc::smem_u32(smem + FIN_M0);
+#pragma unroll 1
           for (int t = 0; t < 3; ++t) {  // hi hi, hi lo, lo hi
-            const uint32_t ab = sa + (t == 2 ? 32768u : 0u), bb = sb + (t == 1 ? 32768u : 0u);
+            const uint32_t qb = sq + (t == 1 ? QT_BYTES / 2 : 0), mb = sm + (t == 2 ? PACK_BYTES / 2 : 0);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)  // 16 d_k rows of qt^T per step: 2048 bytes; the two chunks' images lie 16384 bytes apart
-              tc::mma_ss(tm, tc::smem_desc_sw128(ab + k * 2048, 16384, 1024),
-                         tc::smem_desc_sw128(bb + (uint32_t)((k >> 2) * 16384 + (k & 3) * 32), 16, 1024), idesc, (t | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < 8; ++k)  // 16 d_k rows of qt^T per step: 2048 bytes
+              tc::mma_ss(tm, tc::smem_desc_sw128(mb + (uint32_t)((k >> 2) * 16384 + (k & 3) * 32), 16, 1024),
+                         tc::smem_desc_sw128(qb + k * 2048, 16, 1024), idesc, (t | k) != 0 ? 1u : 0u);
           }
           tc::mma_commit(mma_bar);
         }
@@ -412,46 +405,38 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
       }
       ok = tc::mbar_wait(mma_bar, (uint32_t)it & 1u, abort_flag);
       tc::tc_fence_after_sync();
-      // the images have been read: the next pair's take their place while this pair is finished
-      if (ok && tid == 0 && pair + stride < n_pairs) load_qt(pair + stride);
-      if (ok) {  // accumulator row -> staged row (this warp: 32 token rows x 32 columns)
+      if (ok) {  // accumulator (a d_v row per thread, 32 tokens) -> staged token rows
+        const int d = (warp & 3) * 32 + lane, first = 32 * (warp >> 2);
         uint32_t acc[32];
-        tc::tmem_ld32(tm + ((uint32_t)(quarter * 32) << 16) + 32 * colq, acc);
+        tc::tmem_ld32(tm + ((uint32_t)((warp & 3) * 32) << 16) + first, acc);
         tc::tmem_ld_wait();
-        float* dstrow = stage + (quarter * 32 + lane) * FIN_PITCH + 32 * colq;
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          *reinterpret_cast<uint4*>(dstrow + 4 * i) = make_uint4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+        for (int t = 0; t < 32; ++t) piece16(first + t, d >> 2)[d & 3] = __uint_as_float(acc[t]);
       }
     }
     tc::tc_fence_before_sync();
     ok = __syncthreads_and(ok ? 1 : 0) != 0;  // staged rows complete; the accumulator is free for the next product
     tc::tc_fence_after_sync();
     if (ok) {
-      float2 x[4][4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const int r = hw + 32 * u;
+        const int r = hw + 16 * u;
         float4 p0 = make_float4(0.f, 0.f, 0.f, 0.f), p1 = p0;
         if (!skipped && r < rows) {
-          p0 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub);
-          p1 = *reinterpret_cast<const float4*>(stage + r * FIN_PITCH + 8 * sub + 4);
+          p0 = *reinterpret_cast<const float4*>(piece16(r, 2 * sub));
+          p1 = *reinterpret_cast<const float4*>(piece16(r, 2 * sub + 1));
         }
-        x[u][0] = make_float2(ol[u][0].x + p0.x, ol[u][0].y + p0.y); x[u][1] = make_float2(ol[u][0].z + p0.z, ol[u][0].w + p0.w);
-        x[u][2] = make_float2(ol[u][1].x + p1.x, ol[u][1].y + p1.y); x[u][3] = make_float2(ol[u][1].z + p1.z, ol[u][1].w + p1.w);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int r = hw + 32 * u;
+        float2 x[4] = {make_float2(ol[u][0].x + p0.x, ol[u][0].y + p0.y), make_float2(ol[u][0].z + p0.z, ol[u][0].w + p0.w),
+                       make_float2(ol[u][1].x + p1.x, ol[u][1].y + p1.y), make_float2(ol[u][1].z + p1.z, ol[u][1].w + p1.w)};
         uint32_t packed[4];
         if (a.z != nullptr) {
-          float2 gate[4] = {silu2(bf16x2_to_float2(zraw[u].x)), silu2(bf16x2_to_float2(zraw[u].y)),
-                            silu2(bf16x2_to_float2(zraw[u].z)), silu2(bf16x2_to_float2(zraw[u].w))};
+          const float2 gate[4] = {silu2(bf16x2_to_float2(zraw[u].x)), silu2(bf16x2_to_float2(zraw[u].y)),
+                                  silu2(bf16x2_to_float2(zraw[u].z)), silu2(bf16x2_to_float2(zraw[u].w))};
           float2 ss2 = make_float2(0.f, 0.f);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            if (gate_first) x[u][i] = __fmul2_rn(x[u][i], gate[i]);
-            ss2 = __ffma2_rn(x[u][i], x[u][i], ss2);
+            if (gate_first) x[i] = __fmul2_rn(x[i], gate[i]);
+            ss2 = __ffma2_rn(x[i], x[i], ss2);
           }
           float ss = ss2.x + ss2.y;
 #pragma unroll
@@ -459,27 +444,29 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
           const float rinv = rsqrtf(ss * (1.0f / D) + a.norm_eps);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            float2 y2 = __fmul2_rn(__fmul2_rn(x[u][i], make_float2(rinv, rinv)), wv[i]);
+            float2 y2 = __fmul2_rn(__fmul2_rn(x[i], make_float2(rinv, rinv)), wv[i]);
             if (!gate_first) y2 = __fmul2_rn(y2, gate[i]);
             packed[i] = pack_bf16x2(y2.x, y2.y);
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) packed[i] = pack_bf16x2(x[u][i].x, x[u][i].y);
+          for (int i = 0; i < 4; ++i) packed[i] = pack_bf16x2(x[i].x, x[i].y);
         }
         if (r < rows)
           *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(a.o) + sp.b * a.o_stride_b + (tok0 + r) * a.o_stride_t +
                                     (int64_t)h * a.o_stride_h + 8 * sub) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
       }
     }
-    __syncthreads();  // the staged rows have been read: the next pair may overwrite them
+    tc::fence_proxy_async_smem();
+    __syncthreads();  // the staged rows have been read: the next chunk's images may take their place
+    if (ok && tid == 0 && !skipped && c + stride < c_end) load_qt(c + stride);
   }
   tc::tc_fence_before_sync();
   __syncthreads();
   if (*abort_flag != 0u && tid == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
   if (warp == 1) {
     tc::tc_fence_after_sync();
-    tc::tmem_dealloc(tm, 128);
+    tc::tmem_dealloc(tm, 64);
   }
 }
 
@@ -529,7 +516,7 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   L.part_begin[0] = 0;
   {
     // Part 0 runs one chain and needs no fix-up, a later part runs two chains and its rows wait for the fix-up, so
-    // part 0 is made PART0_X4 / 4 times as long as the others; lengths are even (the fix-up works on pairs of chunks).
+    // part 0 is made PART0_X4 / 4 times as long as the others; lengths are even.
     const int len = max(2, (4 * max_chunks / (4 * (L.parts - 1) + PART0_X4) + 1) & ~1);
     const int first = L.parts > 1 ? max(2, (max_chunks - (L.parts - 1) * len + 1) & ~1) : 0;
     for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < L.parts ? first + (p - 1) * len : (1 << 24);
@@ -759,8 +746,8 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
       int part_len = 0;  // the longest of the later parts
       for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
       const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
-      int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of the SMs
-      split = max(1, min(split, (part_len + 1) / 2));
+      int split = (int)(2 * NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of two an SM
+      split = max(1, min(split, part_len));
       step(launch_after(part_finish_kernel, dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream,
                         a, chunk_start, o_f32, qt_img, m0_pack, plan));
     }
