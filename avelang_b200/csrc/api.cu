@@ -6,9 +6,10 @@ namespace ave {
 thread_local int g_last_cuda_error = 0;
 
 int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
+bool decode_beside_ok(const AveGdnArgs& a);
 int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream);
 size_t prefill_d64_workspace_bytes(const AveGdnArgs& a);
-int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain);
+int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, const AveGdnArgs* decode);
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain);
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain);
 int launch_gated_rmsnorm(const AveGdnNormArgs& a, cudaStream_t stream);
@@ -101,7 +102,7 @@ int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream) {
   if (args->workspace == nullptr || !aligned16(args->workspace)) return AVE_GDN_INVALID_ARGUMENT;
   if (args->workspace_bytes < prefill_ws_bytes(*args)) return AVE_GDN_WORKSPACE_TOO_SMALL;
   // d = 128 runs on the tcgen05 scan; d = 64 (the small CPU-reference shape) has a form of its own, with fp32 accuracy
-  if (args->dk == 128) return launch_prefill_tc(*args, reinterpret_cast<cudaStream_t>(stream), false);
+  if (args->dk == 128) return launch_prefill_tc(*args, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
   return launch_prefill_d64(*args, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -110,6 +111,20 @@ int ave_gdn_decode_step(const AveGdnArgs* args, void* stream) {
   if (rc != AVE_GDN_OK) return rc;
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return AVE_GDN_OK;
   return launch_decode(*args, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int ave_gdn_mixed_step(const AveGdnArgs* decode, const AveGdnArgs* prefill, void* stream) {
+  int rc = validate_gdn(decode, false);
+  if (rc == AVE_GDN_OK) rc = validate_gdn(prefill, true);
+  if (rc != AVE_GDN_OK) return rc;
+  const bool none = (int64_t)prefill->B * prefill->T == 0 || prefill->n_seqs == 0;
+  if (none || prefill->dk != 128 || prefill->n_peers > 1 || !decode_beside_ok(*decode)) {
+    rc = ave_gdn_decode_step(decode, stream);
+    return rc != AVE_GDN_OK ? rc : ave_gdn_chunk_prefill(prefill, stream);
+  }
+  if (prefill->workspace == nullptr || !aligned16(prefill->workspace)) return AVE_GDN_INVALID_ARGUMENT;
+  if (prefill->workspace_bytes < prefill_ws_bytes(*prefill)) return AVE_GDN_WORKSPACE_TOO_SMALL;
+  return launch_prefill_tc(*prefill, reinterpret_cast<cudaStream_t>(stream), false, decode);
 }
 
 int ave_gdn_gated_rmsnorm(const AveGdnNormArgs* a, void* stream) {

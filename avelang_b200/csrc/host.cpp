@@ -82,6 +82,7 @@ struct Api {
   decltype(&ave_gdn_chunk_prefill) chunk_prefill = nullptr;
   decltype(&ave_gdn_prefill_workspace_bytes) prefill_workspace_bytes = nullptr;
   decltype(&ave_gdn_decode_step) decode_step = nullptr;
+  decltype(&ave_gdn_mixed_step) mixed_step = nullptr;
   decltype(&ave_gdn_gated_rmsnorm) gated_rmsnorm = nullptr;
   decltype(&ave_gemm_bf16_nt) gemm_bf16_nt = nullptr;
   decltype(&ave_gdn_conv1d_silu) conv1d_silu = nullptr;
@@ -418,10 +419,11 @@ int64_t n_slots(const Tensor* s0, const Tensor* final, int64_t n) {
   return pool != nullptr ? pool->size(0) : n;
 }
 
-void enqueue_prefill(AveGdnArgs& a, const Tensor& q) {
+void enqueue_prefill(AveGdnArgs& a, const Tensor& q, const AveGdnArgs* decode = nullptr) {  // with the single-token part of a mixed step
   Launch launch(q);
   const Scratch ws(q, launch.stream, api.prefill_workspace_bytes(&a));
   a.workspace = ws.data(); a.workspace_bytes = ws.size();
+  if (decode != nullptr) return check(launch([&] { return api.mixed_step(decode, &a, launch.stream); }), "mixed_prefill_decode_step");
   check(launch([&] { return api.chunk_prefill(&a, launch.stream); }), "chunk_gated_delta_rule");
 }
 void enqueue_decode(AveGdnArgs& a, const Tensor& q) {
@@ -461,21 +463,21 @@ void op_mixed(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g
   REQ(n_decode >= 0 && n_decode <= n && n_decode <= q.size(1), "n_decode must lie in [0, ", std::min(n, q.size(1)), "], got ", n_decode, ".");
   AveGdnArgs a = fill_args(q, k, v, g, beta, some(z), some(norm_weight), norm_eps, out, scale, &state_pool, &state_pool, &cu_seqlens, &state_indices,
                            state_pool.size(0), n, l2norm);
+  AveGdnArgs d = a;
   if (n_decode > 0) {  // one single-token sequence per row: the token stride becomes the batch stride
-    AveGdnArgs d = a;
     d.B = d.n_seqs = (int32_t)n_decode;
     d.T = 1;
     d.cu_seqlens = nullptr;
     d.q_stride_b = a.q_stride_t; d.k_stride_b = a.k_stride_t; d.v_stride_b = a.v_stride_t; d.z_stride_b = a.z_stride_t;
     d.o_stride_b = a.o_stride_t; d.g_stride_b = a.g_stride_t;
-    enqueue_decode(d, q);
+    if (n_decode == n) return enqueue_decode(d, q);
   }
   if (n_decode < n) {
     a.cu_seqlens += n_decode;  // offsets stay absolute: the tables use differences, the tokens are addressed from the packed base
     a.state_indices += n_decode;
     a.n_seqs = (int32_t)(n - n_decode);
     a.token_begin = (int32_t)n_decode;
-    enqueue_prefill(a, q);
+    enqueue_prefill(a, q, n_decode > 0 ? &d : nullptr);
   }
 }
 
@@ -920,6 +922,7 @@ PyObject* bind(PyObject* const* p) {
   RESOLVE(chunk_prefill, ave_gdn_chunk_prefill);
   RESOLVE(prefill_workspace_bytes, ave_gdn_prefill_workspace_bytes);
   RESOLVE(decode_step, ave_gdn_decode_step);
+  RESOLVE(mixed_step, ave_gdn_mixed_step);
   RESOLVE(gated_rmsnorm, ave_gdn_gated_rmsnorm);
   RESOLVE(gemm_bf16_nt, ave_gemm_bf16_nt);
   RESOLVE(conv1d_silu, ave_gdn_conv1d_silu);

@@ -158,6 +158,7 @@ struct ScanPlan {
   int parts;
   int part_begin[MAX_PARTS + 1];  // part_begin[parts] = 1 << 24
   int r0, rn;
+  bool decode_behind;  // the single-token sequences of a mixed step are launched behind pass 2 and may start beside it
 };
 constexpr int PACK_BYTES = 2 * 128 * 128 * 2;  // bf16 hi image | lo image of one [128][128] operand
 constexpr int QT_BYTES = 2 * 128 * 64 * 2;     // bf16 hi image | lo image of one chunk's qt^T [128 d_k][64 tokens]
@@ -554,8 +555,10 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
 
 }  // namespace
 
+int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
+int launch_decode_beside(const AveGdnArgs& a, cudaStream_t stream);
 int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers,
-                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b);
+                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b, bool beside);
 
 // More chains than SMs: the walk of the longest chains decides, so the tables are built, which sort the sequences for the scan.
 // 32 heads, one sequence of 203 tokens: 33.9 us with the tables, 31.3 without.
@@ -629,7 +632,7 @@ static SideSet* side_set(DeviceSide& dev, cudaStream_t stream) {
 }
 
 // Gated RMSNorm over the fp32 output for tokens [t_begin, t_end) of every batch row.
-static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, cudaStream_t stream) {
+static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, cudaStream_t stream, bool beside = false) {
   if (t_end <= t_begin) return AVE_GDN_OK;
   AveGdnNormArgs nb{};
   nb.struct_size = sizeof(nb);
@@ -648,23 +651,23 @@ static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, 
   const int64_t xs_b = (int64_t)a.T * a.Hv * D;
   if (push || a.B == 1)
     return launch_gated_rmsnorm_f32in_batched(nb, stream, a.o_peers, a.n_peers, (int64_t)t_begin * a.o_stride_t, a.B, xs_b,
-                                              a.z_stride_b, a.o_stride_b);
+                                              a.z_stride_b, a.o_stride_b, beside);
   for (int b = 0; b < a.B; ++b) {
     AveGdnNormArgs one = nb;
     one.x = reinterpret_cast<const float*>(nb.x) + b * xs_b;
     one.z = reinterpret_cast<const __nv_bfloat16*>(nb.z) + b * a.z_stride_b;
     one.y = reinterpret_cast<__nv_bfloat16*>(nb.y) + b * a.o_stride_b;
     const int rc = launch_gated_rmsnorm_f32in_batched(one, stream, a.o_peers, a.n_peers,
-                                                      (int64_t)b * a.o_stride_b + (int64_t)t_begin * a.o_stride_t, 1, 0, 0, 0);
+                                                      (int64_t)b * a.o_stride_b + (int64_t)t_begin * a.o_stride_t, 1, 0, 0, 0, false);
     if (rc != AVE_GDN_OK) return rc;
   }
   return AVE_GDN_OK;
 }
 
-// Enqueues one prefill.  Thread-safe: the enqueue sequence of a call runs under the device's mutex (see SideSet).
-int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
+// Enqueues one prefill, and the single-token part of a mixed step with it (`decode`).  Thread-safe: the enqueue sequence of a call runs under the device's mutex (see SideSet).
+int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, const AveGdnArgs* decode) {
   const WsLayout L = ws_layout(a, plain);
-  if (L.chunks == 0 || a.n_seqs == 0) return AVE_GDN_OK;
+  if (L.chunks == 0 || a.n_seqs == 0) return decode != nullptr ? launch_decode(*decode, stream) : AVE_GDN_OK;
   char* ws = reinterpret_cast<char*>(a.workspace);
   int32_t* chunk_start = needs_tables(a) ? reinterpret_cast<int32_t*>(ws + L.chunk_start) : nullptr;
   uint8_t* recs = reinterpret_cast<uint8_t*>(ws + L.recs);
@@ -709,6 +712,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
   const int32_t* seq_order = chunk_start != nullptr ? chunk_start + a.n_seqs + 1 + L.chunks : nullptr;
   ScanPlan plan;
   plan.parts = L.parts;
+  plan.decode_behind = decode != nullptr;
   for (int p = 0; p <= MAX_PARTS; ++p) plan.part_begin[p] = L.part_begin[p];
   const int64_t tile_rows = (int64_t)a.Hk * ((a.Hv / a.Hk + 1) / 2);  // a unit of pass 1 takes up to two value heads of a key head
   auto tiles_grid = [&](int64_t chunks) { return dim3((unsigned)min(chunks * tile_rows, (int64_t)(2 * NUM_SMS))); };  // persistent, two CTAs an SM
@@ -721,7 +725,11 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
     AVE_CUDA_TRY(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
     AVE_CUDA_TRY(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));
-    if (L.parts <= 1) return a.z != nullptr ? norm_rows(a, o_f32, a.token_begin, a.T, stream) : AVE_GDN_OK;
+    if (decode != nullptr) {  // a mixed step: its single tokens run beside pass 2, the gated norm beside the end of both
+      const int drc = launch_decode_beside(*decode, stream);
+      if (drc != AVE_GDN_OK) return drc;
+    }
+    if (L.parts <= 1) return a.z != nullptr ? norm_rows(a, o_f32, a.token_begin, a.T, stream, decode != nullptr) : AVE_GDN_OK;
     // Parts: the combine and the fix-up of the later ones.  Dense layouts: the gated norm of the tokens no fix-up touches runs beside them,
     // forked to a helper stream and joined back (the combine is all latency); packed layouts: the norm covers every row, and the fix-up
     // behind it rewrites those of later parts.
@@ -735,7 +743,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain) {
         AVE_CUDA_TRY(cudaStreamWaitEvent(side->norm, side->fork, 0));
         rc = norm_rows(a, o_f32, 0, end, side->norm);
       } else {
-        rc = norm_rows(a, o_f32, a.token_begin, end, stream);
+        rc = norm_rows(a, o_f32, a.token_begin, end, stream, decode != nullptr);
       }
     }
     auto step = [&](cudaError_t e) { if (e != cudaSuccess && rc == AVE_GDN_OK) rc = cuda_fail(e); };
@@ -836,5 +844,5 @@ extern "C" int ave_gdn_chunk_prefill_noalloc(const AveGdnArgs* args, void* strea
   local.workspace = scratch;
   local.workspace_bytes = kStaticScratchBytes;
   // every scratch record a launch reads is written earlier in the same launch sequence, so nothing needs clearing
-  return launch_prefill_tc(local, reinterpret_cast<cudaStream_t>(stream), true);
+  return launch_prefill_tc(local, reinterpret_cast<cudaStream_t>(stream), true, nullptr);
 }

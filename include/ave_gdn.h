@@ -135,6 +135,11 @@ int ave_gdn_chunk_prefill_noalloc(const AveGdnArgs* args, void* stream);
  * continuous-batching decode step (state streamed once in, once out, updated in place). */
 int ave_gdn_decode_step(const AveGdnArgs* args, void* stream);
 
+/* ave_gdn_decode_step(decode) and ave_gdn_chunk_prefill(prefill) as one call on one stream, for a batch in which some
+ * sequences take a single token and the others prefill.  Neither may read what the other writes (their state slots and
+ * output rows are distinct): with dk = dv = 128 the two run beside one another. */
+int ave_gdn_mixed_step(const AveGdnArgs* decode, const AveGdnArgs* prefill, void* stream);
+
 /* y = w * x * rsqrt(mean(x^2) + eps) * silu(z) over rows of `d` elements. */
 typedef struct AveGdnNormArgs {
   uint32_t struct_size;
