@@ -98,6 +98,9 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   uint64_t* o1_empty = bars + 14; // O1 accumulator drained (the output warps take it first, whole, so O1 of the next chunk can run early)
   uint64_t* o2_empty = bars + 15; // O2 accumulator drained
   uint64_t* o1_done = bars + 16;  // O1 complete: the bf16 image of H may be overwritten
+  // A wait sees only the parity of a barrier's phase, so no barrier may complete twice before each of its waiters has seen the first
+  // time.  Most are ordered by the arrivals they need.  dh_full is waited for by warp 2 as well, which no increment needs: so warp 1 issues an
+  // increment only behind o_full of the chunk before, which warp 2 commits when it has seen dh_full of that chunk.
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -261,6 +264,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
         tc::mma_commit(vn_full);
       }
       __syncwarp();
+      if (!tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) break;  // warp 2 has seen dh_full of the chunk before (and O2 is long complete)
       if (!tc::mbar_wait_warp(vd_ready, cp, abort_flag)) break;
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
