@@ -101,7 +101,8 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   // A wait sees only the parity of a barrier's phase, so no barrier may complete twice before each of its waiters has seen the first
   // time.  Most are ordered by the arrivals they need.  dh_full is waited for by warp 2 as well, which no increment needs: so warp 1 issues an
   // increment only behind o_full of the chunk before, which warp 2 commits when it has seen dh_full of that chunk.
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* tail_full = bars + 17;  // tiles and record of a ragged last chunk landed: warp 3 clears what lies behind the sequence, then completes `full`
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -181,7 +182,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   if (threadIdx.x == 0) {
     for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
     tc::mbar_init(h_ready, 4 * NG); tc::mbar_init(x_ready, 4 * NG); tc::mbar_init(vd_ready, 4 * NG); tc::mbar_init(vn_ready, 4 * NG);
-    for (uint64_t* b : {kh_full, vn_full, dh_full, o_full, o1_done}) tc::mbar_init(b, 1);
+    for (uint64_t* b : {kh_full, vn_full, dh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
     tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
     *abort_flag = 0;
     tc::fence_barrier_init();
@@ -191,6 +192,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   __syncthreads();
   tc::tc_fence_after_sync();
   const uint32_t tm = *tmem_slot;
+  const bool ragged = a.cu_seqlens != nullptr && sp.len < n_chunks * C;
 
   if (warp < 4) {
   tc::reg_set<REGS_CTRL, REGS_LAUNCH>();
@@ -199,23 +201,28 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 1;  // parity of "chunk c - 3 is done with the stage"; the first round waits for nothing
-      for (int c = 0; c < n_chunks; ++c) {
+      auto load = [&](int c, uint64_t* when_full) {
         if (c == n_chunks - 1) pdl_trigger();
-        if (c >= CS_STAGES && !tc::mbar_wait(&empty[s], ph, abort_flag)) break;
+        if (c >= CS_STAGES && !tc::mbar_wait(&empty[s], ph, abort_flag)) return false;
         uint8_t* st = smem + s * CS_STAGE;
         const int tok = sp.t0 + c * C;
-        tc::mbar_expect_tx(&full[s], phi ? CS_STAGE - 16384u : (uint32_t)CS_STAGE);  // the transition chain has no V
-        tc::tma_load_4d(st + CS_K, &maps.k, &full[s], 0, hk, tok, sp.b);
-        tc::tma_load_4d(st + CS_K + 8192, &maps.k, &full[s], 64, hk, tok, sp.b);
-        tc::bulk_load(st + CS_REC, recs + ((int64_t)(c_first + c) * a.Hv + h) * REC_BYTES, REC_BYTES, &full[s]);
+        tc::mbar_expect_tx(when_full, phi ? CS_STAGE - 16384u : (uint32_t)CS_STAGE);  // the transition chain has no V
+        tc::tma_load_4d(st + CS_K, &maps.k, when_full, 0, hk, tok, sp.b);
+        tc::tma_load_4d(st + CS_K + 8192, &maps.k, when_full, 64, hk, tok, sp.b);
+        tc::bulk_load(st + CS_REC, recs + ((int64_t)(c_first + c) * a.Hv + h) * REC_BYTES, REC_BYTES, when_full);
         if (!phi) {
-          tc::tma_load_4d(st + CS_V, &maps.v, &full[s], 0, h, tok, sp.b);
-          tc::tma_load_4d(st + CS_V + 8192, &maps.v, &full[s], 64, h, tok, sp.b);
+          tc::tma_load_4d(st + CS_V, &maps.v, when_full, 0, h, tok, sp.b);
+          tc::tma_load_4d(st + CS_V + 8192, &maps.v, when_full, 64, h, tok, sp.b);
         }
-        tc::tma_load_4d(st + CS_Q, &maps.q, &full[s], 0, hk, tok, sp.b);
-        tc::tma_load_4d(st + CS_Q + 8192, &maps.q, &full[s], 64, hk, tok, sp.b);
+        tc::tma_load_4d(st + CS_Q, &maps.q, when_full, 0, hk, tok, sp.b);
+        tc::tma_load_4d(st + CS_Q + 8192, &maps.q, when_full, 64, hk, tok, sp.b);
         if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
-      }
+        return true;
+      };
+      const int whole = ragged ? n_chunks - 1 : n_chunks;
+      bool ok = true;
+      for (int c = 0; c < whole && ok; ++c) ok = load(c, &full[s]);
+      if (ragged && ok) load(whole, tail_full);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ chain MMA issuer (whole warp runs the loop, one
@@ -311,6 +318,24 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       }
       __syncwarp();
       if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
+    }
+  } else if (__builtin_expect(ragged, 0)) {
+    // ------------------------------------------------------------------ warp 3: the tiles of a packed sequence's last chunk go on with the rows
+    // of whatever lies behind it.  Their factors are zero, but a product is not where such a row holds a NaN or an infinity, so K and V are
+    // cleared there (Q only reaches columns that are not stored; behind the end of a dense batch row the copy itself fills with zeros).
+    // By a warp that has nothing else to do, up to two chunks before the tiles are read: 203 tokens 29.4 us, 29.2 without; by warp 1 in
+    // front of U 29.9, and with the contractions over tokens cut at the last token instead, a branch around each MMA, 30.1 (8192 tokens 320, 316, 318 and 326).
+    if (tc::mbar_wait_warp(tail_full, 0u, abort_flag)) {
+      const int last = (n_chunks - 1) % CS_STAGES;
+      uint4* st = reinterpret_cast<uint4*>(smem + last * CS_STAGE + CS_K);
+      // 16-byte pieces of the halves (64 features) of K and of V; whole rows, so the swizzle does not matter.  (Not unrolled: the code
+      // runs once and is fetched while it runs.)
+#pragma unroll 1
+      for (int i = 8 * (sp.len - (n_chunks - 1) * C) + lane; i < 8 * C; i += 32)
+        st[i] = st[i + 512] = st[i + 1024] = st[i + 1536] = make_uint4(0u, 0u, 0u, 0u);
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&full[last]);
     }
   }
   } else if (warp < 4 + 4 * NG) {

@@ -10,10 +10,11 @@ SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))
 STAGES = 3
 COUNT = {"empty": 3}  # arrivals a phase: the two issuers and the output warps (a group of warps counts as one); 1 elsewhere
 ROLES = {  # marker of the role's code -> its steps: `wait` barriers, `put` for an arrival, `commit` for one that comes when the MMAs are complete
-    "loader:": ["wait empty", "commit full"],
+    "loader:": ["wait empty", "commit when_full"],  # `full`, or `tail_full` for the last chunk of a sequence that ends inside it
     "chain MMA issuer": ["wait full", "wait h_ready", "commit kh_full", "commit empty", "wait x_ready", "commit vn_full", "wait o_full",
                          "wait vd_ready", "commit dh_full", "wait full"],
     "output MMA issuer": ["wait kh_full o1_empty full", "commit o1_done", "wait vn_ready o2_empty dh_full", "commit o_full", "commit empty"],
+    "warp 3:": ["wait tail_full", "put full"],
     "chain epilogue:": ["put h_ready", "wait full kh_full", "put x_ready", "wait vn_full", "put vd_ready", "wait o_full", "put vn_ready", "wait dh_full o1_done"],
     "output warps:": ["wait o_full", "put o1_empty", "put o2_empty", "put empty"],
 }
@@ -27,20 +28,20 @@ def _source_steps():
         code = re.sub(r"//[^\n]*", "", text[begin:at[i + 1][0] if i + 1 < len(at) else None].split("\n", 1)[1])
         found = []
         for call, args in re.findall(r"tc::(mbar_wait(?:_warp|2|3)?|mbar_arrive|mma_commit|mbar_expect_tx)\(((?:[^()]|\([^()]*\))*)\)", code):
-            names = re.findall(r"&?\b([a-z0-9_]*(?:full|empty|ready|done))\b", args)
+            names = re.findall(r"\b([a-z0-9_]*(?:full|empty|ready|done))\b", args)
             found.append({"w": "wait", "a": "put", "x": "commit"}["x" if call in ("mma_commit", "mbar_expect_tx") else call[5]] + " " + " ".join(names))
         steps[mark] = found
     return steps
 
 
-def _programs(chunks, ordered=True):
+def _programs(chunks, ordered=True, ragged=True):
     """One list of steps a role: (kind, [(barrier, phase)]), a wait naming the phase that has to be complete."""
     full, empty = (lambda c: f"full{c % STAGES}"), (lambda c: f"empty{c % STAGES}")
     loader, chain, out_mma, epi, out = [], [("wait", [(full(0), 0)])], [], [("put", "h_ready")], []
     for c in range(chunks):
         if c >= STAGES:
             loader.append(("wait", [(empty(c), c // STAGES - 1)]))
-        loader.append(("commit", full(c)))
+        loader.append(("commit", full(c) if c + 1 < chunks or not ragged else "tail_full"))
         chain += [("wait", [("h_ready", c)]), ("commit", "kh_full")] + ([("commit", empty(c - 1))] if c else [])
         chain += [("wait", [("x_ready", c)]), ("commit", "vn_full")] + ([("wait", [("o_full", c - 1)])] if ordered else [])
         chain += [("wait", [("vd_ready", c)]), ("commit", "dh_full")]
@@ -52,7 +53,8 @@ def _programs(chunks, ordered=True):
         epi += [("wait", [("vn_full", c)]), ("put", "vd_ready"), ("wait", [("o_full", c - 1)]), ("put", "vn_ready")]
         epi += [("wait", [("dh_full", c), ("o1_done", c)]), ("put", "h_ready")]
         out += [("wait", [("o_full", c)]), ("put", "o1_empty"), ("put", "o2_empty"), ("put", empty(c))]
-    return [loader, chain, out_mma, epi, out]
+    clear = [("wait", [("tail_full", 0)]), ("put", full(chunks - 1))] if ragged else []
+    return [loader, chain, out_mma, epi, out, clear]
 
 
 def _stuck(programs):
@@ -105,8 +107,9 @@ def test_the_lists_are_the_kernels():
 
 
 @pytest.mark.parametrize("chunks", [1, 2, 3, 4, 5])
-def test_no_order_leaves_a_role_waiting(chunks):
-    assert not _stuck(_programs(chunks))
+@pytest.mark.parametrize("ragged", [False, True])
+def test_no_order_leaves_a_role_waiting(chunks, ragged):
+    assert not _stuck(_programs(chunks, ragged=ragged))
 
 
 def test_the_walk_finds_a_wait_that_nothing_orders():
