@@ -71,8 +71,6 @@ __device__ __forceinline__ float2 bf16x2_to_float2(uint32_t raw) {
 // calls pdl_wait before it touches global memory, which returns when everything before it is complete and visible; in a
 // kernel launched the ordinary way both do nothing.  Data of earlier kernels must not be read through pointers declared
 // `const __restrict__` (the compiler may take such loads to be invariant and move them above the wait).
-// (Two kernels of a mixed step start without a wait, because what they read was complete before the trigger they hang on, and wait at
-// their end instead, so that a wait for them still covers everything before them: gdn_decode_pool_kernel and the norm behind it.)
 // Early triggers only where the kernels that may follow find no room beside this one: CTAs that wait beside a long kernel
 // cost it time (a 5 ms GEMM ran 9 % longer under waiting convolution CTAs).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

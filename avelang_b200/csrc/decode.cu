@@ -186,13 +186,6 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_kernel(const AveGdnArgs a) 
 // Single-token step over a slot pool (T == 1), persistent form: each CTA walks tiles blockIdx.x, +gridDim.x, ...
 // While one 64 KiB tile is being reduced, updated and streamed out of registers, the next one is already landing
 // in shared memory through one bulk copy, so loads stay in flight across the compute and store phases.
-// kBeside: the grid behind pass 2 of a prefill in a mixed step.  It starts when every CTA of pass 2 is on an SM and takes the SMs
-// that those leave or never had (pass 2 holds one SM a chain and is bound by latency; this one is bound by memory).  Pass 2 triggers after
-// its own wait, so all that came before pass 2 is complete; the fence drops what this SM's L1 may hold of it.  The last CTA has
-// no tile: it waits for pass 2 and only then lets the grid behind start (which may use pass 2's results without a wait) and this
-// one end, so that a wait for this grid covers pass 2 as well.  61 sequences beside three prompts of 1500 tokens, 32 heads: 119.5 us
-// with the decode in front, 95.1 beside (norm beside the tail of the decode included); 200 beside one of 100: 171.7, 161.7.
-template <bool kBeside>
 __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArgs a, int n_tiles) {
   constexpr int DK = 128, DV = 128;
   using C = DecodeCfg<DK, DV>;
@@ -220,22 +213,16 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
   };
   auto tile_offset = [&](int t, int slot) -> int64_t { return ((int64_t)slot * a.Hv + (t % a.Hv)) * (int64_t)(DK * DV); };
 
-  if (kBeside && blockIdx.x == gridDim.x - 1) {  // no tile: holds back what follows until everything before this grid is complete
-    pdl_wait();
-    pdl_trigger();
-    return;
-  }
   pdl_trigger();
   if (threadIdx.x == 0) {
     tc::mbar_init(&full_bar, 1);
     abort_flag = 0;
     tc::fence_barrier_init();
   }
-  if constexpr (kBeside) __threadfence();
-  else pdl_wait();
+  pdl_wait();
   int t = blockIdx.x;
   if (t >= n_tiles) return;
-  const int stride = kBeside ? (int)gridDim.x - 1 : (int)gridDim.x;
+  const int stride = (int)gridDim.x;
   int slot = slot_of(t);
   if (threadIdx.x == 0) {
     if (slot >= 0) {
@@ -375,8 +362,7 @@ static cudaError_t pool_kernel_attr() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || set[dev & 63]) return e;
-  if ((e = cudaFuncSetAttribute(gdn_decode_pool_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(gdn_decode_pool_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4)) != cudaSuccess) return e;
+  if ((e = cudaFuncSetAttribute(gdn_decode_pool_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 128 * 4)) != cudaSuccess) return e;
   set[dev & 63] = true;
   return e;
 }
@@ -388,15 +374,16 @@ static bool pool_form(const AveGdnArgs& a) {
 
 bool decode_beside_ok(const AveGdnArgs& a) { return pool_form(a) && a.n_seqs > 0; }
 
-// Behind pass 2 of a prefill only (see kBeside)
+// The single tokens of a mixed step, on a stream of their own beside pass 2 of the prefill
 int launch_decode_beside(const AveGdnArgs& a, cudaStream_t stream) {
   AVE_CUDA_TRY(pool_kernel_attr());
   const int tiles = a.n_seqs * a.Hv;
-  // Tiles a CTA: few, because CTAs start as SMs fall free and the last ones alone are the tail (seven, the persistent form's number
-  // at 61 x 32 tiles: 112 us, two 102, one 103, before the norm ran beside the tail); four where there are more than eight a slot
-  // (128 x 32 tiles 154.7 us, with two 156.9, with one 162.7).
+  // Tiles a CTA: few, because CTAs start as SMs fall free and the last ones alone are the tail (a whole step with 61 x 32 tiles: seven, the
+  // persistent form's number, 104.7 us, four 94.4, two 95.4, one 97.2; 20 x 32 tiles: 58.0, 51.4, 44.4, 43.8); four where there are more
+  // than eight a slot (200 x 32 tiles and 100 tokens: seven 168.6, four 161.7, one 167.6).
   const int per = tiles >= 8 * 2 * 148 ? 4 : 2;
-  AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel<true>, (unsigned)((tiles + per - 1) / per + 1), 256, 128 * 128 * 4, stream, a, tiles));
+  gdn_decode_pool_kernel<<<(unsigned)((tiles + per - 1) / per), 256, 128 * 128 * 4, stream>>>(a, tiles);
+  AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }
 
@@ -409,7 +396,7 @@ int launch_decode(const AveGdnArgs& a, cudaStream_t stream) {
     AVE_CUDA_TRY(pool_kernel_attr());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned persistent = (unsigned)(2 * sms);
-    AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel<false>, grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream, a, (int)grid));
+    AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel, grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream, a, (int)grid));
   } else if (a.dk == 128 && a.dv == 128) {
     AVE_CUDA_TRY(launch_after(gdn_decode_kernel<128, 128>, grid, 256, 0, stream, a));
   } else if (a.dk == 64 && a.dv == 64) {

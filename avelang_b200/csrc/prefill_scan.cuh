@@ -107,7 +107,6 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   pdl_wait();
-  if (plan.decode_behind) pdl_trigger();
   // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
   // chain of part p >= 1 (see ScanPlan).
   const int chains = kMulti ? 2 * plan.parts - 1 : 1;

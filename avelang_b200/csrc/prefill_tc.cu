@@ -158,7 +158,6 @@ struct ScanPlan {
   int parts;
   int part_begin[MAX_PARTS + 1];  // part_begin[parts] = 1 << 24
   int r0, rn;
-  bool decode_behind;  // the single-token sequences of a mixed step are launched behind pass 2 and may start beside it
 };
 constexpr int PACK_BYTES = 2 * 128 * 128 * 2;  // bf16 hi image | lo image of one [128][128] operand
 constexpr int QT_BYTES = 2 * 128 * 64 * 2;     // bf16 hi image | lo image of one chunk's qt^T [128 d_k][64 tokens]
@@ -558,7 +557,7 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
 int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
 int launch_decode_beside(const AveGdnArgs& a, cudaStream_t stream);
 int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers,
-                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b, bool beside);
+                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b);
 
 // More chains than SMs: the walk of the longest chains decides, so the tables are built, which sort the sequences for the scan.
 // 32 heads, one sequence of 203 tokens: 33.9 us with the tables, 31.3 without.
@@ -632,7 +631,7 @@ static SideSet* side_set(DeviceSide& dev, cudaStream_t stream) {
 }
 
 // Gated RMSNorm over the fp32 output for tokens [t_begin, t_end) of every batch row.
-static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, cudaStream_t stream, bool beside = false) {
+static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, cudaStream_t stream) {
   if (t_end <= t_begin) return AVE_GDN_OK;
   AveGdnNormArgs nb{};
   nb.struct_size = sizeof(nb);
@@ -651,14 +650,14 @@ static int norm_rows(const AveGdnArgs& a, float* o_f32, int t_begin, int t_end, 
   const int64_t xs_b = (int64_t)a.T * a.Hv * D;
   if (push || a.B == 1)
     return launch_gated_rmsnorm_f32in_batched(nb, stream, a.o_peers, a.n_peers, (int64_t)t_begin * a.o_stride_t, a.B, xs_b,
-                                              a.z_stride_b, a.o_stride_b, beside);
+                                              a.z_stride_b, a.o_stride_b);
   for (int b = 0; b < a.B; ++b) {
     AveGdnNormArgs one = nb;
     one.x = reinterpret_cast<const float*>(nb.x) + b * xs_b;
     one.z = reinterpret_cast<const __nv_bfloat16*>(nb.z) + b * a.z_stride_b;
     one.y = reinterpret_cast<__nv_bfloat16*>(nb.y) + b * a.o_stride_b;
     const int rc = launch_gated_rmsnorm_f32in_batched(one, stream, a.o_peers, a.n_peers,
-                                                      (int64_t)b * a.o_stride_b + (int64_t)t_begin * a.o_stride_t, 1, 0, 0, 0, false);
+                                                      (int64_t)b * a.o_stride_b + (int64_t)t_begin * a.o_stride_t, 1, 0, 0, 0);
     if (rc != AVE_GDN_OK) return rc;
   }
   return AVE_GDN_OK;
@@ -712,38 +711,29 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
   const int32_t* seq_order = chunk_start != nullptr ? chunk_start + a.n_seqs + 1 + L.chunks : nullptr;
   ScanPlan plan;
   plan.parts = L.parts;
-  plan.decode_behind = decode != nullptr;
   for (int p = 0; p <= MAX_PARTS; ++p) plan.part_begin[p] = L.part_begin[p];
   const int64_t tile_rows = (int64_t)a.Hk * ((a.Hv / a.Hk + 1) / 2);  // a unit of pass 1 takes up to two value heads of a key head
   auto tiles_grid = [&](int64_t chunks) { return dim3((unsigned)min(chunks * tile_rows, (int64_t)(2 * NUM_SMS))); };  // persistent, two CTAs an SM
   const unsigned scan_grid = (unsigned)a.n_seqs * (unsigned)(2 * L.parts - 1) * (unsigned)a.Hv;
   const auto scan = L.parts > 1 ? chunk_scan_kernel<true> : chunk_scan_kernel<false>;
 
-  SideSet* side = L.segments > 1 ? side_set(dev, stream) : nullptr;
-  if (side == nullptr) {
-    // one launch per pass on the caller's stream
-    plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
-    AVE_CUDA_TRY(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
-    AVE_CUDA_TRY(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));
-    if (decode != nullptr) {  // a mixed step: its single tokens run beside pass 2, the gated norm beside the end of both
-      const int drc = launch_decode_beside(*decode, stream);
-      if (drc != AVE_GDN_OK) return drc;
-    }
-    if (L.parts <= 1) return a.z != nullptr ? norm_rows(a, o_f32, a.token_begin, a.T, stream, decode != nullptr) : AVE_GDN_OK;
+  // What follows pass 2 on the caller's stream
+  auto finish = [&]() -> int {
+    if (L.parts <= 1) return a.z != nullptr ? norm_rows(a, o_f32, a.token_begin, a.T, stream) : AVE_GDN_OK;
     // Parts: the combine and the fix-up of the later ones.  Dense layouts: the gated norm of the tokens no fix-up touches runs beside them,
     // forked to a helper stream and joined back (the combine is all latency); packed layouts: the norm covers every row, and the fix-up
     // behind it rewrites those of later parts.
-    const bool beside = a.z != nullptr && a.cu_seqlens == nullptr;
-    side = beside ? side_set(dev, stream) : nullptr;
+    const bool forked = a.z != nullptr && a.cu_seqlens == nullptr;
+    SideSet* side = forked ? side_set(dev, stream) : nullptr;
     int rc = AVE_GDN_OK;
     if (a.z != nullptr) {
-      const int end = beside ? min(a.T, L.part_begin[1] * C) : a.T;
+      const int end = forked ? min(a.T, L.part_begin[1] * C) : a.T;
       if (side != nullptr) {
         AVE_CUDA_TRY(cudaEventRecord(side->fork, stream));
         AVE_CUDA_TRY(cudaStreamWaitEvent(side->norm, side->fork, 0));
         rc = norm_rows(a, o_f32, 0, end, side->norm);
       } else {
-        rc = norm_rows(a, o_f32, a.token_begin, end, stream, decode != nullptr);
+        rc = norm_rows(a, o_f32, a.token_begin, end, stream);
       }
     }
     auto step = [&](cudaError_t e) { if (e != cudaSuccess && rc == AVE_GDN_OK) rc = cuda_fail(e); };
@@ -762,6 +752,35 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
     if (side != nullptr) {
       step(cudaEventRecord(side->join_norm, side->norm));
       step(cudaStreamWaitEvent(stream, side->join_norm, 0));
+    }
+    return rc;
+  };
+
+  SideSet* side = L.segments > 1 ? side_set(dev, stream) : nullptr;
+  if (side == nullptr) {
+    // One launch per pass on the caller's stream.  The single tokens of a mixed step run beside pass 2, on a helper stream: pass 2 holds one SM a
+    // chain and is bound by latency, they are bound by memory and take the SMs that its chains leave or never had.  They fork behind
+    // pass 1, so that pass 2, which is launched dependent on it, has its SMs first; the gated norm follows pass 2 and runs beside the rest of them.
+    // 61 sequences beside three prompts of 1500 tokens, 32 heads: one part behind the other 128 us, 95.3 so (92.9 replayed from a graph); 200
+    // beside one of 100: 176, 162; 128 beside 2048 tokens 218, 145.  (With an event that completes when pass 2's CTAs have started, the
+    // runtime held the single tokens back until pass 2 was complete: 128.)
+    plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
+    SideSet* beside = decode != nullptr ? side_set(dev, stream) : nullptr;
+    if (decode != nullptr && beside == nullptr) {
+      const int drc = launch_decode(*decode, stream);
+      if (drc != AVE_GDN_OK) return drc;
+    }
+    int rc = AVE_GDN_OK;
+    auto step = [&](cudaError_t e) { if (e != cudaSuccess && rc == AVE_GDN_OK) rc = cuda_fail(e); return rc == AVE_GDN_OK; };
+    step(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
+    const bool forked = beside != nullptr && step(cudaEventRecord(beside->fork, stream)) && step(cudaStreamWaitEvent(beside->prep, beside->fork, 0));
+    if (rc == AVE_GDN_OK)
+      step(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));
+    if (rc == AVE_GDN_OK && forked) rc = launch_decode_beside(*decode, beside->prep);
+    if (rc == AVE_GDN_OK) rc = finish();
+    if (forked) {  // after an error too, so that a surrounding stream capture stays well formed
+      step(cudaEventRecord(beside->join, beside->prep));
+      step(cudaStreamWaitEvent(stream, beside->join, 0));
     }
     return rc;
   }

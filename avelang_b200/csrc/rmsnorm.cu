@@ -21,10 +21,8 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const _
                                                             int64_t rows, int heads, int64_t xs_t, int64_t xs_h,
                                                             int64_t zs_t, int64_t zs_h, int64_t ys_t, int64_t ys_h,
                                                             float eps, int gate_first, const void* const* peers,
-                                                            int n_peers, int64_t peer_off, NormBatch nb, int beside) {
-  // beside: x is complete before this grid starts, and the grid in front may still be running (see gdn_decode_pool_kernel)
-  if (beside) __threadfence();
-  else pdl_wait();
+                                                            int n_peers, int64_t peer_off, NormBatch nb) {
+  pdl_wait();
   constexpr int E = D / 16;  // elements per lane: 8 or 4
   constexpr int P = E / 2;   // pairs per lane
   constexpr int U = 2;       // rows in flight per half-warp
@@ -128,12 +126,11 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_kernel(const XT* x, const _
       }
     }
   }
-  if (beside && blockIdx.x == gridDim.x - 1) pdl_wait();  // complete only once the grid in front is
 }
 
 template <typename XT>
 static int launch_norm_t(const XT* x, const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers = nullptr, int n_peers = 0,
-                         int64_t peer_off = 0, int batches = 1, int64_t xs_b = 0, int64_t zs_b = 0, int64_t ys_b = 0, bool beside = false) {
+                         int64_t peer_off = 0, int batches = 1, int64_t xs_b = 0, int64_t zs_b = 0, int64_t ys_b = 0) {
   if (a.rows == 0 || batches == 0) return AVE_GDN_OK;
   const NormBatch nb{a.rows, xs_b, zs_b, ys_b};
   const int64_t rows = a.rows * batches;
@@ -148,10 +145,10 @@ static int launch_norm_t(const XT* x, const AveGdnNormArgs& a, cudaStream_t stre
   __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y);
   if (a.d == 128) {
     AVE_CUDA_TRY(launch_after(flat ? gated_rmsnorm_kernel<128, XT, true> : gated_rmsnorm_kernel<128, XT, false>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb, (int)beside));
+                                                            a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, peers, n_peers, peer_off, nb));
   } else if (a.d == 64) {
     AVE_CUDA_TRY(launch_after(flat ? gated_rmsnorm_kernel<64, XT, true> : gated_rmsnorm_kernel<64, XT, false>, grid, 256, 0, stream, x, z, a.weight, y, rows, a.heads, a.x_stride_t, a.x_stride_h,
-                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, (const void* const*)nullptr, 0, (int64_t)0, nb, (int)beside));
+                                                           a.z_stride_t, a.z_stride_h, a.y_stride_t, a.y_stride_h, a.eps, gate_first, (const void* const*)nullptr, 0, (int64_t)0, nb));
   } else {
     return AVE_GDN_UNSUPPORTED;
   }
@@ -166,8 +163,8 @@ int launch_gated_rmsnorm(const AveGdnNormArgs& a, cudaStream_t stream) {
 // fp32 input variant used by the prefill path when the un-normalised output is staged in scratch, over `batches` batch rows
 // in one launch: a.rows counts the rows of one batch row, the strides step between them.
 int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t stream, const void* const* peers, int n_peers,
-                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b, bool beside) {
-  return launch_norm_t(reinterpret_cast<const float*>(a.x), a, stream, peers, n_peers, peer_off, batches, xs_b, zs_b, ys_b, beside);
+                                       int64_t peer_off, int batches, int64_t xs_b, int64_t zs_b, int64_t ys_b) {
+  return launch_norm_t(reinterpret_cast<const float*>(a.x), a, stream, peers, n_peers, peer_off, batches, xs_b, zs_b, ys_b);
 }
 
 }  // namespace ave
