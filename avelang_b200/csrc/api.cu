@@ -6,7 +6,7 @@ namespace ave {
 thread_local int g_last_cuda_error = 0;
 
 int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
-bool decode_beside_ok(const AveGdnArgs& a);
+bool decode_beside_ok(const AveGdnArgs& a, const AveGdnArgs& prefill);
 int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream);
 size_t prefill_d64_workspace_bytes(const AveGdnArgs& a);
 int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, const AveGdnArgs* decode);
@@ -118,7 +118,7 @@ int ave_gdn_mixed_step(const AveGdnArgs* decode, const AveGdnArgs* prefill, void
   if (rc == AVE_GDN_OK) rc = validate_gdn(prefill, true);
   if (rc != AVE_GDN_OK) return rc;
   const bool none = (int64_t)prefill->B * prefill->T == 0 || prefill->n_seqs == 0;
-  if (none || prefill->dk != 128 || prefill->n_peers > 1 || !decode_beside_ok(*decode)) {
+  if (none || prefill->n_peers > 1 || !decode_beside_ok(*decode, *prefill)) {
     rc = ave_gdn_decode_step(decode, stream);
     return rc != AVE_GDN_OK ? rc : ave_gdn_chunk_prefill(prefill, stream);
   }

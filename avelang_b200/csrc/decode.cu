@@ -6,35 +6,16 @@
 // is applied in registers before the tile is streamed back to the same slot.  One read and one
 // write of the state per token; for T > 1 the tile stays in registers across the tokens.
 #include "common.cuh"
+#include "recurrent.cuh"
 #include "tc.cuh"
 
 namespace ave {
 
 template <int DK, int DV>
-struct DecodeCfg {
-  static constexpr int kThreads = 256;
-  static constexpr int kWarps = 8;
-  static constexpr int kLanesPerRow = DV / 4;             // one float4 per lane
-  static constexpr int kRowsPerLoad = 32 / kLanesPerRow;  // rows covered by one warp-wide load
-  static constexpr int kRowsPerWarp = DK / kWarps;
-  static constexpr int kLoads = kRowsPerWarp / kRowsPerLoad;
-  static_assert(DV % 4 == 0 && kLanesPerRow <= 32 && 32 % kLanesPerRow == 0, "dv layout");
-  static_assert(DK % kWarps == 0 && kRowsPerWarp % kRowsPerLoad == 0, "dk layout");
-};
-
-template <int DK, int DV>
 __global__ void __launch_bounds__(256, 2) gdn_decode_kernel(const AveGdnArgs a) {
-  using C = DecodeCfg<DK, DV>;
-  __shared__ __align__(16) float k_s[DK];
-  __shared__ __align__(16) float q_s[DK];
-  __shared__ __align__(16) float red[2][C::kWarps][DV];
-
+  __shared__ __align__(16) DecodeSmem<DK, DV> sm;
   const int n = blockIdx.x / a.Hv;
   const int h = blockIdx.x % a.Hv;
-  const int hk = h / (a.Hv / a.Hk);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int col = (lane % C::kLanesPerRow) * 4;
-  const int row0 = warp * C::kRowsPerWarp + lane / C::kLanesPerRow;
 
   pdl_trigger();
   pdl_wait();
@@ -57,136 +38,15 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_kernel(const AveGdnArgs a) 
     return;
   }
 
-  const int64_t tile = ((int64_t)slot * a.Hv + h) * (int64_t)(DK * DV);
-  float4 S[C::kLoads];
-  if (a.initial_state != nullptr) {
-    const float* src = a.initial_state + tile;
-    asm volatile("" : "+l"(src));  // keeps the streaming loads behind pdl_wait
-#pragma unroll
-    for (int i = 0; i < C::kLoads; ++i)
-      S[i] = __ldcs(reinterpret_cast<const float4*>(src + (row0 + i * C::kRowsPerLoad) * DV + col));
-  } else {
-#pragma unroll
-    for (int i = 0; i < C::kLoads; ++i) S[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-
-  const __nv_bfloat16* q_base = reinterpret_cast<const __nv_bfloat16*>(a.q) + sp.b * a.q_stride_b + (int64_t)hk * a.q_stride_h;
-  const __nv_bfloat16* k_base = reinterpret_cast<const __nv_bfloat16*>(a.k) + sp.b * a.k_stride_b + (int64_t)hk * a.k_stride_h;
-  const __nv_bfloat16* v_base = reinterpret_cast<const __nv_bfloat16*>(a.v) + sp.b * a.v_stride_b + (int64_t)h * a.v_stride_h;
-  const __nv_bfloat16* z_base = a.z ? reinterpret_cast<const __nv_bfloat16*>(a.z) + sp.b * a.z_stride_b + (int64_t)h * a.z_stride_h : nullptr;
-  const float* g_base = a.g + sp.b * a.g_stride_b + h;
-  const float* beta_base = a.beta + sp.b * a.g_stride_b + h;
-  const bool l2 = (a.flags & AVE_GDN_FLAG_QK_L2NORM) != 0;
-
-  for (int t = 0; t < sp.len; ++t) {
-    const int64_t tok = sp.t0 + t;
-    if (t > 0) __syncthreads();  // k_s/q_s/red of the previous token are no longer read
-    if (threadIdx.x < DK) {
-      k_s[threadIdx.x] = bf2f(k_base[tok * a.k_stride_t + threadIdx.x]);
-    } else if (threadIdx.x < 2 * DK) {
-      q_s[threadIdx.x - DK] = bf2f(q_base[tok * a.q_stride_t + threadIdx.x - DK]);
-    }
-    float v4[4];
-    unpack_bf16x4(*reinterpret_cast<const uint2*>(v_base + tok * a.v_stride_t + col), v4);
-    const float alpha = __expf(g_base[tok * a.g_stride_t]);
-    const float beta = beta_base[tok * a.g_stride_t];
-    __syncthreads();
-
-    // every warp derives k.q and the two norms redundantly from shared memory (no extra barrier)
-    float kq = 0.f, kk = 0.f, qq = 0.f;
-#pragma unroll
-    for (int i = lane; i < DK; i += 32) {
-      const float kv = k_s[i], qv = q_s[i];
-      kq += kv * qv; kk += kv * kv; qq += qv * qv;
-    }
-    kq = warp_sum(kq);
-    float kn = 1.f, qn = 1.f;
-    if (l2) {
-      kn = rsqrtf(warp_sum(kk) + 1e-6f);
-      qn = rsqrtf(warp_sum(qq) + 1e-6f);
-      kq *= kn * qn;
-    }
-
-    float r[4] = {0.f, 0.f, 0.f, 0.f}, p[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int i = 0; i < C::kLoads; ++i) {
-      const int row = row0 + i * C::kRowsPerLoad;
-      const float kr = k_s[row] * kn, qr = q_s[row] * qn;
-      r[0] += S[i].x * kr; r[1] += S[i].y * kr; r[2] += S[i].z * kr; r[3] += S[i].w * kr;
-      p[0] += S[i].x * qr; p[1] += S[i].y * qr; p[2] += S[i].z * qr; p[3] += S[i].w * qr;
-    }
-    if (C::kRowsPerLoad > 1) {  // lanes that share columns but hold different rows
-#pragma unroll
-      for (int off = C::kLanesPerRow; off < 32; off <<= 1) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          r[c] += __shfl_xor_sync(0xffffffffu, r[c], off);
-          p[c] += __shfl_xor_sync(0xffffffffu, p[c], off);
-        }
-      }
-    }
-    if (lane < C::kLanesPerRow) {
-      *reinterpret_cast<float4*>(&red[0][warp][col]) = make_float4(r[0], r[1], r[2], r[3]);
-      *reinterpret_cast<float4*>(&red[1][warp][col]) = make_float4(p[0], p[1], p[2], p[3]);
-    }
-    __syncthreads();
-    float4 rs = make_float4(0.f, 0.f, 0.f, 0.f), ps = rs;
-#pragma unroll
-    for (int w = 0; w < C::kWarps; ++w) {
-      const float4 x = *reinterpret_cast<const float4*>(&red[0][w][col]);
-      const float4 y = *reinterpret_cast<const float4*>(&red[1][w][col]);
-      rs.x += x.x; rs.y += x.y; rs.z += x.z; rs.w += x.w;
-      ps.x += y.x; ps.y += y.y; ps.z += y.z; ps.w += y.w;
-    }
-    float u[4], o[4];
-    u[0] = beta * (v4[0] - alpha * rs.x); u[1] = beta * (v4[1] - alpha * rs.y);
-    u[2] = beta * (v4[2] - alpha * rs.z); u[3] = beta * (v4[3] - alpha * rs.w);
-    o[0] = a.scale * (alpha * ps.x + u[0] * kq); o[1] = a.scale * (alpha * ps.y + u[1] * kq);
-    o[2] = a.scale * (alpha * ps.z + u[2] * kq); o[3] = a.scale * (alpha * ps.w + u[3] * kq);
-#pragma unroll
-    for (int i = 0; i < C::kLoads; ++i) {
-      const float kr = k_s[row0 + i * C::kRowsPerLoad] * kn;
-      S[i].x = alpha * S[i].x + kr * u[0]; S[i].y = alpha * S[i].y + kr * u[1];
-      S[i].z = alpha * S[i].z + kr * u[2]; S[i].w = alpha * S[i].w + kr * u[3];
-    }
-    if (warp == 0) {  // warp 0's first kLanesPerRow lanes cover every column once
-      if (z_base != nullptr) {
-        float zz[4];
-        unpack_bf16x4(*reinterpret_cast<const uint2*>(z_base + tok * a.z_stride_t + col), zz);
-        const bool gate_first = (a.flags & AVE_GDN_FLAG_GATE_FIRST) != 0;
-        if (gate_first) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) o[c] *= silu(zz[c]);
-        }
-        float ss = o[0] * o[0] + o[1] * o[1] + o[2] * o[2] + o[3] * o[3];
-        if (lane >= C::kLanesPerRow) ss = 0.f;
-        ss = warp_sum(ss);
-        const float rinv = rsqrtf(ss * (1.0f / DV) + a.norm_eps);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float w = a.norm_weight ? a.norm_weight[col + c] : 1.0f;
-          o[c] = o[c] * rinv * w * (gate_first ? 1.0f : silu(zz[c]));
-        }
-      }
-      if (lane < C::kLanesPerRow) {
-        uint2 packed = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
-        *reinterpret_cast<uint2*>(o_base + tok * a.o_stride_t + col) = packed;
-      }
-    }
-  }
-
-  if (a.final_state != nullptr) {
-    float* dst = a.final_state + tile;
-#pragma unroll
-    for (int i = 0; i < C::kLoads; ++i)
-      __stcs(reinterpret_cast<float4*>(dst + (row0 + i * C::kRowsPerLoad) * DV + col), S[i]);
-  }
+  recurrent_tokens<DK, DV>(a, sp, h, slot, sm, threadIdx.x, [] { __syncthreads(); });
 }
 
 // Single-token step over a slot pool (T == 1), persistent form: each CTA walks tiles blockIdx.x, +gridDim.x, ...
 // While one 64 KiB tile is being reduced, updated and streamed out of registers, the next one is already landing
 // in shared memory through one bulk copy, so loads stay in flight across the compute and store phases.
-__global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArgs a, int n_tiles) {
+// In a mixed step this grid runs beside the chains of the prompts, whose slots are `prompt_slots` (null: sequence n has slot n): a sequence that
+// shares its slot with one of them has been served in front of them (gdn_shared_slots_kernel).
+__global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArgs a, int n_tiles, const int32_t* prompt_slots, int n_prompts) {
   constexpr int DK = 128, DV = 128;
   using C = DecodeCfg<DK, DV>;
   extern __shared__ __align__(128) uint8_t dyn_smem[];
@@ -203,8 +63,7 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
   const bool l2 = (a.flags & AVE_GDN_FLAG_QK_L2NORM) != 0;
 
   auto slot_of = [&](int t) -> int {  // < 0: the tile is skipped
-    const int n = t / a.Hv;
-    int slot = a.state_indices ? a.state_indices[n] : n;
+    int slot = state_slot(a, t / a.Hv);
     if (slot >= a.num_slots) {
       if (a.status != nullptr && threadIdx.x == 0) atomicOr(a.status, AVE_GDN_DEV_BAD_SLOT);
       slot = -1;
@@ -222,6 +81,15 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
   pdl_wait();
   int t = blockIdx.x;
   if (t >= n_tiles) return;
+  // slots of the first 32 prompts, one a lane.  Compared late, when a tile's results are there: 200 sequences beside one prompt 162.6 us, 161.8
+  // without, 164.6 when the tile has landed, 168 in front of its load.
+  int prompt_slot = -1;
+  if (lane < n_prompts) prompt_slot = prompt_slots != nullptr ? prompt_slots[lane] : lane;
+  auto served = [&](int slot) {
+    bool named = prompt_slot == slot;
+    for (int i = 32 + lane; i < n_prompts; i += 32) named |= (prompt_slots != nullptr ? prompt_slots[i] : i) == slot;
+    return __any_sync(0xffffffffu, named) != 0;
+  };
   const int stride = (int)gridDim.x;
   int slot = slot_of(t);
   if (threadIdx.x == 0) {
@@ -324,6 +192,11 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
     u[2] = beta * (v4[2] - alpha * rs.z); u[3] = beta * (v4[3] - alpha * rs.w);
     o[0] = a.scale * (alpha * ps.x + u[0] * kq); o[1] = a.scale * (alpha * ps.y + u[1] * kq);
     o[2] = a.scale * (alpha * ps.z + u[2] * kq); o[3] = a.scale * (alpha * ps.w + u[3] * kq);
+    if (n_prompts > 0 && served(slot)) {
+      slot = slot_next;
+      cur = nxt;
+      continue;
+    }
     float* dst = a.final_state + tile_offset(t, slot);
 #pragma unroll
     for (int i = 0; i < C::kLoads; ++i) {
@@ -357,6 +230,28 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
   }
 }
 
+// The sequences of a mixed step that the grid above leaves out: their tokens come before the prompt that names the same slot, so they are
+// taken in front of the prompts' passes, by a CTA for each (prompt, value head): the first of the prompts where several name the slot.  Nothing is
+// shared as a rule, and this is one look at the slots, all latency: 61 sequences beside three prompts of 1500 tokens 95.6 us without it, 97.8 with
+// it; 20 beside three of 400 44.7, 46.9.  (The look inside pass 1 cost 4 us, inside pass 2, beside the single tokens' traffic, 5; on the helper
+// stream with an event in front of pass 2 the single tokens had the SMs first: 144.  An early trigger of pass 1: no gain.)
+__global__ void __launch_bounds__(256, 2) gdn_shared_slots_kernel(const AveGdnArgs a, const int32_t* prompt_slots, int n_prompts) {
+  __shared__ __align__(16) DecodeSmem<128, 128> sm;
+  const int n = blockIdx.x / a.Hv, h = blockIdx.x % a.Hv;
+  auto prompt_slot = [&](int i) { return prompt_slots != nullptr ? prompt_slots[i] : i; };
+  pdl_wait();
+  const int slot = prompt_slot(n);
+  bool named = false, earlier = false;
+  for (int i = threadIdx.x; i < a.n_seqs; i += 256) named |= state_slot(a, i) == slot;
+  for (int i = threadIdx.x; i < n; i += 256) earlier |= prompt_slot(i) == slot;
+  if (slot < 0 || slot >= a.num_slots || !__syncthreads_or(named) || __syncthreads_or(earlier)) return;
+  for (int i = 0; i < a.n_seqs; ++i) {
+    if (state_slot(a, i) != slot) continue;
+    recurrent_tokens<128, 128>(a, SeqSpan{i, 0, 1, true}, h, slot, sm, threadIdx.x, [] { __syncthreads(); });
+    __syncthreads();
+  }
+}
+
 static cudaError_t pool_kernel_attr() {
   static bool set[64] = {};
   int dev = 0;
@@ -372,17 +267,26 @@ static bool pool_form(const AveGdnArgs& a) {
   return a.dk == 128 && a.dv == 128 && a.T == 1 && a.cu_seqlens == nullptr && a.initial_state != nullptr && a.final_state != nullptr;
 }
 
-bool decode_beside_ok(const AveGdnArgs& a) { return pool_form(a) && a.n_seqs > 0; }
+// Beside a prefill: both update the same state pool in place, so that a sequence of each may share a slot (the single token comes first)
+bool decode_beside_ok(const AveGdnArgs& a, const AveGdnArgs& prefill) {
+  return pool_form(a) && a.n_seqs > 0 && a.initial_state == a.final_state && prefill.initial_state == a.initial_state &&
+         prefill.final_state == a.final_state && prefill.num_slots == a.num_slots && prefill.Hv == a.Hv && prefill.dk == 128;
+}
+
+int launch_shared_slots(const AveGdnArgs& a, const AveGdnArgs& prefill, cudaStream_t stream) {
+  AVE_CUDA_TRY(launch_after(gdn_shared_slots_kernel, (unsigned)prefill.n_seqs * (unsigned)a.Hv, 256, 0, stream, a, prefill.state_indices, prefill.n_seqs));
+  return AVE_GDN_OK;
+}
 
 // The single tokens of a mixed step, on a stream of their own beside pass 2 of the prefill
-int launch_decode_beside(const AveGdnArgs& a, cudaStream_t stream) {
+int launch_decode_beside(const AveGdnArgs& a, const AveGdnArgs& prefill, cudaStream_t stream) {
   AVE_CUDA_TRY(pool_kernel_attr());
   const int tiles = a.n_seqs * a.Hv;
   // Tiles a CTA: few, because CTAs start as SMs fall free and the last ones alone are the tail (a whole step with 61 x 32 tiles: seven, the
   // persistent form's number, 104.7 us, four 94.4, two 95.4, one 97.2; 20 x 32 tiles: 58.0, 51.4, 44.4, 43.8); four where there are more
   // than eight a slot (200 x 32 tiles and 100 tokens: seven 168.6, four 161.7, one 167.6).
   const int per = tiles >= 8 * 2 * 148 ? 4 : 2;
-  gdn_decode_pool_kernel<<<(unsigned)((tiles + per - 1) / per), 256, 128 * 128 * 4, stream>>>(a, tiles);
+  gdn_decode_pool_kernel<<<(unsigned)((tiles + per - 1) / per), 256, 128 * 128 * 4, stream>>>(a, tiles, prefill.state_indices, prefill.n_seqs);
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }
@@ -396,7 +300,7 @@ int launch_decode(const AveGdnArgs& a, cudaStream_t stream) {
     AVE_CUDA_TRY(pool_kernel_attr());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const unsigned persistent = (unsigned)(2 * sms);
-    AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel, grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream, a, (int)grid));
+    AVE_CUDA_TRY(launch_after(gdn_decode_pool_kernel, grid < persistent ? grid : persistent, 256, 128 * 128 * 4, stream, a, (int)grid, (const int32_t*)nullptr, 0));
   } else if (a.dk == 128 && a.dv == 128) {
     AVE_CUDA_TRY(launch_after(gdn_decode_kernel<128, 128>, grid, 256, 0, stream, a));
   } else if (a.dk == 64 && a.dv == 64) {

@@ -112,8 +112,9 @@ def mixed_prefill_decode_step(q, k, v, g, beta, cu_seqlens, n_decode, state_pool
     (or chunked-prefill continuation) sequences of any length and take the chunked kernel.  Every sequence reads its
     state from, and writes it back to, slot ``state_indices[n]`` of ``state_pool`` in place (a fresh sequence starts
     from a zeroed slot).  ``cu_seqlens`` describes the whole packed batch; its first ``n_decode + 1`` entries must be
-    ``0, 1, ..., n_decode`` (not checked: that would need a device synchronisation).  Everything goes to the current stream;
-    the two parts run beside one another, so the slots of a step are distinct.  Returns ``o`` ``[1, T, Hv, dv]``."""
+    ``0, 1, ..., n_decode`` (not checked: that would need a device synchronisation).  Everything goes to the current stream
+    (the two parts run beside one another on the GPU).  Where a prompt names the slot of a single-token sequence, the single token comes
+    first; single-token sequences, and prompts, that share a slot among themselves have no order.  Returns ``o`` ``[1, T, Hv, dv]``."""
     return _native.mixed(q, k, v, g, beta, cu_seqlens, n_decode, state_pool, state_indices, scale, use_qk_l2norm_in_kernel, z,
                          norm_weight, norm_eps, out)
 

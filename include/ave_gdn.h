@@ -136,8 +136,9 @@ int ave_gdn_chunk_prefill_noalloc(const AveGdnArgs* args, void* stream);
 int ave_gdn_decode_step(const AveGdnArgs* args, void* stream);
 
 /* ave_gdn_decode_step(decode) and ave_gdn_chunk_prefill(prefill) as one call on one stream, for a batch in which some
- * sequences take a single token and the others prefill.  Neither may read what the other writes (their state slots and
- * output rows are distinct): with dk = dv = 128 the two run beside one another. */
+ * sequences take a single token and the others prefill.  The results are those of the two calls one after the other.  With
+ * dk = dv = 128 and one pool of states updated in place by both, the two run beside one another; a single-token sequence and a
+ * prompt may name the same slot, and the token comes first.  Their output rows are distinct. */
 int ave_gdn_mixed_step(const AveGdnArgs* decode, const AveGdnArgs* prefill, void* stream);
 
 /* y = w * x * rsqrt(mean(x^2) + eps) * silu(z) over rows of `d` elements. */
