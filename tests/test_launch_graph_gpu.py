@@ -34,6 +34,17 @@ def _waits(call):
     return waits
 
 
+# two parts: the scan has written all that the fix-up needs; three: the combine forms the state that enters the third
+@pytest.mark.parametrize("B, heads, T, two", [(1, 32, 64 * 112, True), (2, 16, 64 * 112, True), (1, 28, 64 * 40, False)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_the_fix_up_of_two_parts_waits_for_the_scan_alone(built_lib, B, heads, T, two, gated):
+    from avelang_b200 import gdn
+    inp = synth.make_inputs(B, T, heads // 2, heads, 128, 128, seed=T, with_z=gated, n_states=B).to("cuda")
+    waits = _waits(lambda: gdn.chunk_gated_delta_rule(inp.q, inp.k, inp.v, inp.g, inp.beta, output_final_state=True, z=inp.z))
+    assert waits["part_finish"] == ({"chunk_scan"} if two else {"part_combine"})
+    assert waits["part_combine"] == {"chunk_scan"} and waits.get("gated_rmsnorm", set()) <= {"chunk_scan", "gated_rmsnorm"}  # (a launch a batch row)
+
+
 @pytest.mark.parametrize("lens", [(200, 100), (3000,)])  # whole chains; parts
 def test_single_tokens_run_beside_the_scan_and_nothing_waits_through_them(built_lib, lens):
     from avelang_b200 import gdn
