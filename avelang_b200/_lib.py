@@ -88,6 +88,7 @@ SYMBOLS = {
     "ave_gdn_chunk_prefill": (ctypes.c_int, [ctypes.POINTER(GdnArgs), P]),
     "ave_gdn_prefill_workspace_bytes": (ctypes.c_size_t, [ctypes.POINTER(GdnArgs)]),
     "ave_gdn_prefill_launch_count": (ctypes.c_int, [ctypes.POINTER(GdnArgs)]),
+    "ave_gdn_prefill_parts": (ctypes.c_int, [ctypes.POINTER(GdnArgs)]),
     "ave_gdn_chunk_prefill_noalloc": (ctypes.c_int, [ctypes.POINTER(GdnArgs), P]),
     "ave_gdn_mixed_step": (ctypes.c_int, [ctypes.POINTER(GdnArgs), ctypes.POINTER(GdnArgs), P]),
     "ave_gdn_decode_step": (ctypes.c_int, [ctypes.POINTER(GdnArgs), P]),

@@ -12,6 +12,7 @@ size_t prefill_d64_workspace_bytes(const AveGdnArgs& a);
 int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, const AveGdnArgs* decode);
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain);
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain);
+int prefill_tc_parts(const AveGdnArgs& a);
 int launch_gated_rmsnorm(const AveGdnNormArgs& a, cudaStream_t stream);
 int launch_conv1d_silu(const AveConvArgs& a, cudaStream_t stream);
 int launch_gate_beta(const AveGateArgs& a, cudaStream_t stream);
@@ -93,6 +94,11 @@ int ave_gdn_prefill_launch_count(const AveGdnArgs* args) {
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return 0;
   if (args->dk == 128) return prefill_tc_launch_count(*args, false);
   return 3;  // chunk tiles, chain of states, outputs (with the gated norm)
+}
+
+int ave_gdn_prefill_parts(const AveGdnArgs* args) {
+  if (validate_gdn(args, true) != AVE_GDN_OK) return 0;
+  return args->dk == 128 ? prefill_tc_parts(*args) : 1;
 }
 
 int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream) {

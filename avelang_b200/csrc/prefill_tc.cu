@@ -473,7 +473,6 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
 // ------------------------------------------------------------------------------------------------ schedule and scratch
 constexpr int SEG_MAX = 8;
 constexpr int PART0_X4 = 4;         // length of part 0 in quarters of a later part's length
-constexpr int REC_PLANNED = 66304;  // a record's share where the scratch stays the size that callers have planned with: with parts, and in the fixed array
 constexpr int NUM_SMS = 148;        // B200; the schedule is a pure function of the arguments, so that the workspace
                                     // query and the launch agree without a device being current
 struct WsLayout {
@@ -539,7 +538,7 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   }
   size_t off = 0;
   L.chunk_start = off; off = up(off + (2 * (size_t)a.n_seqs + 1 + (size_t)L.chunks) * 4);  // prefix table, chunk -> sequence map, scan order
-  L.recs = off; off = up(off + recs * (size_t)(plain || L.parts > 1 ? REC_PLANNED : REC_BYTES));
+  L.recs = off; off = up(off + recs * (size_t)REC_BYTES);
   L.o_f32 = off;
   if (L.parts > 1 || a.z != nullptr) off = up(off + (size_t)a.B * a.T * a.Hv * D * 4);  // rows waiting for the fix-up / the norm
   L.qt_img = off;
@@ -565,6 +564,8 @@ int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t str
 static bool needs_tables(const AveGdnArgs& a) { return a.cu_seqlens != nullptr && (int64_t)a.n_seqs * a.Hv > NUM_SMS; }
 
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain) { return ws_layout(a, plain).total; }
+
+int prefill_tc_parts(const AveGdnArgs& a) { return ws_layout(a, false).parts; }
 
 // Kernels one call enqueues, mirroring launch_prefill_tc below.
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain) {
@@ -852,8 +853,11 @@ extern "C" int ave_gdn_chunk_prefill_noalloc(const AveGdnArgs* args, void* strea
   if (rc != AVE_GDN_OK) return rc;
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return AVE_GDN_OK;
   if (args->dk != 128 || args->dv != 128) return AVE_GDN_UNSUPPORTED;
-  // the plain schedule: one launch per pass on the caller's stream, no helper streams or events, the least scratch
-  if (prefill_tc_workspace_bytes(*args, true) > kStaticScratchBytes) return AVE_GDN_WORKSPACE_TOO_SMALL;
+  // The plain schedule: one launch per pass on the caller's stream, no helper streams or events, the least scratch.  A request is judged by
+  // the records' size that the documented limits were given for; what a call uses of the array is less.
+  constexpr size_t kJudgedRecord = 66304;
+  const size_t records = (size_t)(args->cu_seqlens ? (int64_t)args->T / C + args->n_seqs : (int64_t)args->B * ((args->T + C - 1) / C)) * args->Hv;
+  if (prefill_tc_workspace_bytes(*args, true) + records * (kJudgedRecord - REC_BYTES) > kStaticScratchBytes) return AVE_GDN_WORKSPACE_TOO_SMALL;
   static std::mutex mu;
   static void* scratch_of_device[64] = {};
   int dev = 0;

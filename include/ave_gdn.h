@@ -116,6 +116,9 @@ size_t ave_gdn_prefill_workspace_bytes(const AveGdnArgs* args);
 /* Number of kernels one ave_gdn_chunk_prefill call with these arguments enqueues (a pure function of the shapes and of
  * which optional tensors are present; no device needed).  0 for invalid arguments. */
 int ave_gdn_prefill_launch_count(const AveGdnArgs* args);
+/* Number of parts the schedule cuts a sequence of the longest length into, which are scanned at the same time (1: whole
+ * chains); like the launch count a pure function of the arguments.  0 for invalid arguments. */
+int ave_gdn_prefill_parts(const AveGdnArgs* args);
 
 /* Same computation as ave_gdn_chunk_prefill for callers that may not allocate device memory (a serving runtime
  * that has handed all of HBM to its paged pools, a plug-in callback limited to pre-registered buffers, a path where

@@ -1,5 +1,4 @@
-"""The prefill's schedule is a function of the shapes alone, so the edges of its rules are tested without a GPU, by the scratch it asks
-for: a record is 66304 bytes, and parallel parts keep 32 KiB of operand images beside each."""
+"""The prefill's schedule is a function of the shapes alone, so the edges of its rules are tested without a GPU, and so is the scratch it asks for."""
 import ctypes
 
 import pytest
@@ -7,18 +6,32 @@ import pytest
 from avelang_b200 import _lib
 
 
-def _parts(B, T, heads, gated):
+def _args(B, T, heads, gated):
     a = _lib.GdnArgs()
     a.struct_size = ctypes.sizeof(_lib.GdnArgs)
     for n in ("q", "k", "v", "g", "beta", "o"):
         setattr(a, n, 0x1000)  # never read: only shapes and the presence of a gate enter
     a.z = 0x1000 if gated else None
     a.B, a.T, a.Hk, a.Hv, a.dk, a.dv, a.n_seqs, a.num_slots, a.chunk = B, T, heads // 2, heads, 128, 128, B, B, 64
-    chunks = B * ((T + 63) // 64) * heads
-    scratch = _lib.load().ave_gdn_prefill_workspace_bytes(ctypes.byref(a))
-    rows = B * T * heads * 128 * 4  # un-normalised rows wait in fp32 where there is a gate, or parts
-    left = scratch - chunks * 66304 - (rows if gated else 0)
-    return left > chunks * 32768
+    return ctypes.byref(a)
+
+
+def _parts(B, T, heads, gated):
+    parts = _lib.load().ave_gdn_prefill_parts(_args(B, T, heads, gated))
+    assert parts >= 1
+    return parts > 1
+
+
+# per (chunk, value head): a record, 32 KiB of operand images of the transition chains with parts, and 32 KiB of fp32 rows that wait for the
+# norm or the fix-up; with parts 64 KiB for each chain's state and for the image of each state that enters a part.  Two per cent for tables and alignment
+@pytest.mark.parametrize("B, T, heads, gated", [(1, 8192, 32, True), (1, 8192, 32, False), (1, 32768, 4, True), (2, 1000, 32, False), (1, 64 * 40, 28, True)])
+def test_scratch_is_what_the_schedule_uses(built_lib, B, T, heads, gated):
+    args = _args(B, T, heads, gated)
+    parts, chunks = _lib.load().ave_gdn_prefill_parts(args), B * ((T + 63) // 64) * heads
+    need = chunks * 21504 + (B * T * heads * 512 if gated or parts > 1 else 0)
+    if parts > 1:
+        need += chunks * 32768 + B * heads * 65536 * (2 * parts - 1 + parts - 1)
+    assert need <= _lib.load().ave_gdn_prefill_workspace_bytes(args) <= 1.02 * need + 65536
 
 
 # the length of the longest chain, in 64-token chunks, at which two parts begin, with a gate and without
