@@ -101,7 +101,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   // A wait sees only the parity of a barrier's phase, so no barrier may complete twice before each of its waiters has seen the first
   // time.  Most are ordered by the arrivals they need.  dh_full is waited for by warp 2 as well, which no increment needs: so warp 1 issues an
   // increment only behind o_full of the chunk before, which warp 2 commits when it has seen dh_full of that chunk.
-  uint64_t* tail_full = bars + 17;  // tiles and record of a ragged last chunk landed: warp 3 clears what lies behind the sequence, then completes `full`
+  uint64_t* tail_full = bars + 17;  // tiles and record of a ragged last chunk landed: warp 0 clears what lies behind the sequence, then completes `full`
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
@@ -223,6 +223,24 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       for (int c = 0; c < whole && ok; ++c) ok = load(c, &full[s]);
       if (ragged && ok) load(whole, tail_full);
     }
+    // The tiles of a packed sequence's last chunk go on with the rows of whatever lies behind it.  Their factors are zero, but a product is
+    // not where such a row holds a NaN or an infinity, so K and V are cleared there, by the whole warp, which has nothing else to do, up to two chunks
+    // before they are read.  (Q only reaches columns that are not stored; behind the end of a dense batch row the copy itself fills with zeros.)
+    // 203 tokens: 29.4 us, 29.2 without; by warp 1 in front of U 29.9, and with the contractions over tokens cut at the last token instead, a
+    // branch around each MMA, 30.1 (8192 tokens 318, 316, 318 and 326; by warp 3 320).
+    __syncwarp();
+    if (ragged && tc::mbar_wait_warp(tail_full, 0u, abort_flag)) {
+      const int last = (n_chunks - 1) % CS_STAGES;
+      uint4* st = reinterpret_cast<uint4*>(smem + last * CS_STAGE + CS_K);
+      // 16-byte pieces of the halves (64 features) of K and of V; whole rows, so the swizzle does not matter.  (Not unrolled: the code
+      // runs once and is fetched while it runs.)
+#pragma unroll 1
+      for (int i = 8 * (sp.len - (n_chunks - 1) * C) + lane; i < 8 * C; i += 32)
+        st[i] = st[i + 512] = st[i + 1024] = st[i + 1536] = make_uint4(0u, 0u, 0u, 0u);
+      tc::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&full[last]);
+    }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ chain MMA issuer (whole warp runs the loop, one
     // elected lane issues): the MMAs the recurrence waits for.  One thread needs 20 to 60 cycles per MMA instruction, so
@@ -317,24 +335,6 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       }
       __syncwarp();
       if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
-    }
-  } else if (__builtin_expect(ragged, 0)) {
-    // ------------------------------------------------------------------ warp 3: the tiles of a packed sequence's last chunk go on with the rows
-    // of whatever lies behind it.  Their factors are zero, but a product is not where such a row holds a NaN or an infinity, so K and V are
-    // cleared there (Q only reaches columns that are not stored; behind the end of a dense batch row the copy itself fills with zeros).
-    // By a warp that has nothing else to do, up to two chunks before the tiles are read: 203 tokens 29.4 us, 29.2 without; by warp 1 in
-    // front of U 29.9, and with the contractions over tokens cut at the last token instead, a branch around each MMA, 30.1 (8192 tokens 320, 316, 318 and 326).
-    if (tc::mbar_wait_warp(tail_full, 0u, abort_flag)) {
-      const int last = (n_chunks - 1) % CS_STAGES;
-      uint4* st = reinterpret_cast<uint4*>(smem + last * CS_STAGE + CS_K);
-      // 16-byte pieces of the halves (64 features) of K and of V; whole rows, so the swizzle does not matter.  (Not unrolled: the code
-      // runs once and is fetched while it runs.)
-#pragma unroll 1
-      for (int i = 8 * (sp.len - (n_chunks - 1) * C) + lane; i < 8 * C; i += 32)
-        st[i] = st[i + 512] = st[i + 1024] = st[i + 1536] = make_uint4(0u, 0u, 0u, 0u);
-      tc::fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&full[last]);
     }
   }
   } else if (warp < 4 + 4 * NG) {

@@ -502,13 +502,18 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   // chain per later part and one GEMM-shaped fix-up; S is the largest count whose 2S-1 chains per head still get an SM
   // each, up to 16.  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
   // beside it.
+  // As measured (one sequence, gated, us by the number of parts): the largest count is the best or within 3 % of it from 6144 tokens on (4 heads x
+  // 32768 8: 280, 12: 240, 16: 212; 16 x 8192 3: 216, 4: 195, 5: 189; 24 x 8192 2: 289, 3: 247, 4: 320); with many heads and 2048 tokens two would do
+  // better (20 heads 2: 86, 4: 94; 28 heads 2: 95, 3: 109).
   L.parts = 1;
   if (!plain && !push && max_chunks >= 32) {
     const int64_t per_head = (NUM_SMS / (heads_total > 0 ? heads_total : 1) + 1) / 2;  // chains per head that still get an SM each: 2S - 1
     int S = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
     while (S > 1 && max_chunks / S < 8) --S;  // a part of fewer chunks costs more in combine and fix-up than it saves
-    // Two parts take three chains a head.  They pay while these leave a third of the SMs and the chains are long enough for the
-    // fix-up, which with a gate also holds the later part's norms back.
+    // Two parts take three chains a head.  They are taken while these leave a third of the SMs and the chains are long enough for the
+    // fix-up, which with a gate also holds the later part's norms back.  Both lines are those of slower forms of pass 1, the combine and the fix-up, and
+    // still on the safe side: two parts win at them and would win beyond (32 heads gated, whole / two: 2048 tokens 116 / 101 us, 6144 321 / 247, 8192 419 / 315;
+    // without a gate 2048 102 / 91, 4096 191 / 154; 34 heads x 8192 gated 427 / 325, 40 heads x 32768 1692 / 1271).
     const bool two = S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64);
     L.parts = S >= 3 || two ? S : 1;
   }

@@ -10,11 +10,10 @@ SOURCE = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))
 STAGES = 3
 COUNT = {"empty": 3}  # arrivals a phase: the two issuers and the output warps (a group of warps counts as one); 1 elsewhere
 ROLES = {  # marker of the role's code -> its steps: `wait` barriers, `put` for an arrival, `commit` for one that comes when the MMAs are complete
-    "loader:": ["wait empty", "commit when_full"],  # `full`, or `tail_full` for the last chunk of a sequence that ends inside it
+    "loader:": ["wait empty", "commit when_full", "wait tail_full", "put full"],  # when_full: `tail_full` for the last chunk of a sequence that ends inside it
     "chain MMA issuer": ["wait full", "wait h_ready", "commit kh_full", "commit empty", "wait x_ready", "commit vn_full", "wait o_full",
                          "wait vd_ready", "commit dh_full", "wait full"],
     "output MMA issuer": ["wait kh_full o1_empty full", "commit o1_done", "wait vn_ready o2_empty dh_full", "commit o_full", "commit empty"],
-    "warp 3:": ["wait tail_full", "put full"],
     "chain epilogue:": ["put h_ready", "wait full kh_full", "put x_ready", "wait vn_full", "put vd_ready", "wait o_full", "put vn_ready", "wait dh_full o1_done"],
     "output warps:": ["wait o_full", "put o1_empty", "put o2_empty", "put empty"],
 }
@@ -53,8 +52,8 @@ def _programs(chunks, ordered=True, ragged=True):
         epi += [("wait", [("vn_full", c)]), ("put", "vd_ready"), ("wait", [("o_full", c - 1)]), ("put", "vn_ready")]
         epi += [("wait", [("dh_full", c), ("o1_done", c)]), ("put", "h_ready")]
         out += [("wait", [("o_full", c)]), ("put", "o1_empty"), ("put", "o2_empty"), ("put", empty(c))]
-    clear = [("wait", [("tail_full", 0)]), ("put", full(chunks - 1))] if ragged else []
-    return [loader, chain, out_mma, epi, out, clear]
+    loader += [("wait", [("tail_full", 0)]), ("put", full(chunks - 1))] if ragged else []
+    return [loader, chain, out_mma, epi, out]
 
 
 def _stuck(programs):
