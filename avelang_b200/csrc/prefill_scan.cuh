@@ -8,12 +8,12 @@
 // registers; its bf16 hi/lo image is rewritten to TMEM every chunk.  Pass 1 could also hand over W = Tu diag(kx) K, which
 // makes Vn = U - H W one product: a hand-off less in a step, but W is twice as many bytes as everything else in a record and a third
 // of pass 1.  K itself is exact in bf16, so H K^T takes 16 MMAs where H W^T takes 24.  (262144 packed tokens x 32 heads: 5.75 ms with W,
-// 3.73 without; 8192 tokens 370 us / 344; 4 heads x 32768 254 / 215; 1024 63.4 / 60.6.)
+// 3.73 without, both after a rest, back to back the power cap makes it 4.1 to 4.3; 8192 tokens 370 us / 344; 4 heads x 32768 254 / 215; 1024 63.4 / 60.6.)
 // A step takes 4.55 k cycles alone and with every SM streaming, of which the tensor pipe is busy 2.4 k: H K^T 0.85 k, X 0.65 k, its
 // product 0.65 k, Vd 0.4 k, the increment 1.1 k, the new state 0.7 k, each of them about a third hand-over (commit or arrival, wake-up,
 // first load).  The conversions are bound by the instructions of a scheduler (a pair of values into two bf16 terms takes 7 cycles of it).
-// O2 waits for the increment: side by side they shared the pipe and the increment came 200 cycles later; H K^T in columns of its own lets
-// O2 end beside the next step (5.0 -> 4.55 k cycles together).  Measured and dropped: the state a chunk behind the chain by
+// O2 waits for the increment: side by side they shared the pipe and the increment came 200 cycles later; H K^T in the increment's columns and not
+// in O2's lets O2 end beside the next step (5.0 -> 4.55 k cycles together).  Measured and dropped: the state a chunk behind the chain by
 // S(c+1) = decay H(c) K(c+1)^T + Vd(c) (K(c+1) K(c)^T)^T, with three splits of 16 epilogue warps (3.08, 3.52 and 4.48 ms where this
 // form then took 2.73: 11 to 15 k instructions a chunk, and the code of 20 warps misses the instruction cache); the gated norm in
 // the output warps (layer of 8192 tokens 344 -> 374 us with eight of them, 422 with four).

@@ -61,9 +61,9 @@ def chunk_gated_delta_rule(q, k, v, g, beta, scale=None, initial_state=None, out
     norm kernel itself (a fused all-gather over NVLink) instead of into ``out``; the caller must put a barrier between
     this call and any reader of those buffers.
 
-    ``max_seqlen`` (with ``cu_seqlens``): an upper bound of the longest sequence, known to the host.  With it the chunk
-    ranges of the overlapped schedule (used for batches of few long sequences) are sized from the real chain length
-    instead of the packed total; results are the same with or without it.  A sequence longer than the bound is skipped and flagged in the status word, like a
+    ``max_seqlen`` (with ``cu_seqlens``): an upper bound of the longest sequence, known to the host.  With it the
+    parallel parts that a batch of few long sequences is cut into are sized from the real chain length
+    instead of the packed total; results agree to rounding with and without it.  A sequence longer than the bound is skipped and flagged in the status word, like a
     malformed ``cu_seqlens`` entry."""
     return _native.prefill(q, k, v, g, beta, scale, initial_state, output_final_state, use_qk_l2norm_in_kernel, cu_seqlens, z,
                            norm_weight, norm_eps, state_indices, inplace_state, chunk_size, out, out_peers, max_seqlen)

@@ -29,7 +29,7 @@ def test_decode_step_replays_from_a_graph(built_lib):
 
 
 def test_prefill_replays_from_a_graph(built_lib):
-    """One long sequence: the call forks onto the library's helper streams (range-overlapped schedule) and joins back,
+    """One long sequence: the call forks onto the library's helper streams (parallel parts) and joins back,
     which a capture has to follow."""
     from avelang_b200 import gdn
     inp = synth.make_inputs(1, 2048 + 37, 2, 4, 128, 128, seed=5, with_z=True).to("cuda")

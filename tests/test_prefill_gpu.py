@@ -267,7 +267,7 @@ def test_prefill_rejects_a_non_monotone_offset_table(gdn):
 
 
 def test_prefill_two_host_threads_two_streams(gdn, checker):
-    """Two host threads enqueue range-overlapped prefills on their own streams at the same time (the schedule forks onto
+    """Two host threads enqueue prefills in parallel parts on their own streams at the same time (the schedule forks onto
     helper streams through events): both results match the checker."""
     import threading
     O, C = checker
@@ -326,9 +326,8 @@ def test_mixed_prefill_decode_step(gdn, checker):
 
 
 def test_prefill_varlen_max_seqlen_hint(gdn, checker):
-    """With the longest sequence known, the chunk ranges of a packed batch of few long chains (16 sequences x 4 heads)
-    are sized from it; results are bit-identical to the schedule sized from the packed total, and a sequence longer
-    than the stated bound is skipped and flagged."""
+    """A packed batch of whole chains (16 sequences x 4 heads) gives the same bits with the longest sequence known, and a sequence longer
+    than the stated bound is skipped and flagged.  (Parts, whose lengths follow the bound: test_prefill_parts_gpu.py.)"""
     O, C = checker
     inp = synth.config3(n_seqs=16, total=32768, lo=128, hi=8192, Hk=2, Hv=4)
     lens = inp.extras["lengths"]

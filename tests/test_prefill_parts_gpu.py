@@ -41,3 +41,24 @@ def test_value_heads_per_key_head(built_lib, checker, ratio, T):
     for h in range(2 * ratio):
         check_o(O, o[:, :, h], y_ref[:, :, h])
         check_s(O, s[:, h], s_ref[:, h])
+
+
+# the longest sequence unknown (the parts are sized from the packed total), known, and bounded from above
+@pytest.mark.parametrize("bound", [None, 3000, 4100])
+@pytest.mark.parametrize("with_z", [False, True])
+def test_parts_of_a_packed_batch(built_lib, checker, bound, with_z):
+    from avelang_b200 import gdn
+    O, C = checker
+    lens = (700, 3000, 64, 1, 2500)
+    cu = torch.tensor([sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32)
+    inp = synth.make_inputs(1, sum(lens), 2, 4, 128, 128, seed=107, with_z=with_z, n_states=len(lens), gate_scale=0.05)
+    g = dev(inp)
+    o, s = gdn.chunk_gated_delta_rule(g.q, g.k, g.v, g.g, g.beta, initial_state=g.initial_state, output_final_state=True, cu_seqlens=cu.cuda(), z=g.z,
+                                      max_seqlen=bound)
+    assert gdn.read_status() == 0
+    o_ref, s_ref = C.recurrent(inp.q, inp.k, inp.v, inp.g, inp.beta, inp.scale, inp.initial_state, cu)
+    if with_z:
+        o_ref = O.gated_rmsnorm(o_ref, inp.z)
+    for n in range(len(lens)):
+        check_o(O, o[:, cu[n]:cu[n + 1]], o_ref[:, cu[n]:cu[n + 1]])
+        check_s(O, s[n], s_ref[n])

@@ -49,7 +49,7 @@ def test_noalloc_prefill_matches_regular_entry_point(built_lib):
 
 def test_noalloc_prefill_long_sequence_against_checker(built_lib, checker):
     """One sequence of 2048 tokens x 4 heads with a gate tensor (about 13 MB of the fixed array): the regular entry point
-    cuts such a batch into overlapped launches and parallel parts, the fixed-scratch one runs it as one plain chain on
+    cuts such a batch into parallel parts, the fixed-scratch one runs it as one plain chain on
     the caller's stream, so the two agree within the parity tolerances rather than bit for bit, and both agree with the
     fp64 checker."""
     O, C = checker
