@@ -231,22 +231,27 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_pool_kernel(const AveGdnArg
 }
 
 // The sequences of a mixed step that the grid above leaves out: their tokens come before the prompt that names the same slot, so they are
-// taken in front of the prompts' passes, by a CTA for each (prompt, value head): the first of the prompts where several name the slot.  Nothing is
-// shared as a rule, and this is one look at the slots, all latency: 61 sequences beside three prompts of 1500 tokens 95.6 us without it, 97.8 with
-// it; 20 beside three of 400 44.7, 46.9.  (The look inside pass 1 cost 4 us, inside pass 2, beside the single tokens' traffic, 5; on the helper
-// stream with an event in front of pass 2 the single tokens had the SMs first: 144.  An early trigger of pass 1: no gain.)
+// taken in front of the prompts' chains, by a CTA for each value head, one after the other.  Nothing is shared as a rule, and this is one look at the
+// slots, all latency, behind pass 1: 61 sequences beside three prompts of 1500 tokens 95.6 us without it, 96.3 with it; 20 beside three of 400 44.7,
+// 46.0.  (In front of pass 1, a CTA for each prompt and head, 97.6 and 46.7; inside pass 1 4 us more, inside pass 2, beside the single tokens'
+// traffic, 5; on the helper stream with an event in front of pass 2 the single tokens had the SMs first: 144.  An early trigger: 97.3 and 47.9.)
 __global__ void __launch_bounds__(256, 2) gdn_shared_slots_kernel(const AveGdnArgs a, const int32_t* prompt_slots, int n_prompts) {
   __shared__ __align__(16) DecodeSmem<128, 128> sm;
-  const int n = blockIdx.x / a.Hv, h = blockIdx.x % a.Hv;
+  const int h = blockIdx.x;
   auto prompt_slot = [&](int i) { return prompt_slots != nullptr ? prompt_slots[i] : i; };
   pdl_wait();
-  const int slot = prompt_slot(n);
-  bool named = false, earlier = false;
-  for (int i = threadIdx.x; i < a.n_seqs; i += 256) named |= state_slot(a, i) == slot;
-  for (int i = threadIdx.x; i < n; i += 256) earlier |= prompt_slot(i) == slot;
-  if (slot < 0 || slot >= a.num_slots || !__syncthreads_or(named) || __syncthreads_or(earlier)) return;
+  bool named = false;
+  for (int i = threadIdx.x; i < a.n_seqs; i += 256) {
+    const int slot = state_slot(a, i);
+    if (slot >= 0 && slot < a.num_slots)
+      for (int n = 0; n < n_prompts; ++n) named |= prompt_slot(n) == slot;
+  }
+  if (!__syncthreads_or(named)) return;
   for (int i = 0; i < a.n_seqs; ++i) {
-    if (state_slot(a, i) != slot) continue;
+    const int slot = state_slot(a, i);
+    bool shared = false;
+    for (int n = threadIdx.x; n < n_prompts; n += 256) shared |= prompt_slot(n) == slot;
+    if (slot < 0 || slot >= a.num_slots || !__syncthreads_or(shared)) continue;
     recurrent_tokens<128, 128>(a, SeqSpan{i, 0, 1, true}, h, slot, sm, threadIdx.x, [] { __syncthreads(); });
     __syncthreads();
   }
@@ -274,7 +279,7 @@ bool decode_beside_ok(const AveGdnArgs& a, const AveGdnArgs& prefill) {
 }
 
 int launch_shared_slots(const AveGdnArgs& a, const AveGdnArgs& prefill, cudaStream_t stream) {
-  AVE_CUDA_TRY(launch_after(gdn_shared_slots_kernel, (unsigned)prefill.n_seqs * (unsigned)a.Hv, 256, 0, stream, a, prefill.state_indices, prefill.n_seqs));
+  AVE_CUDA_TRY(launch_after(gdn_shared_slots_kernel, (unsigned)a.Hv, 256, 0, stream, a, prefill.state_indices, prefill.n_seqs));
   return AVE_GDN_OK;
 }
 

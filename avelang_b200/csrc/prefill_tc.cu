@@ -775,9 +775,9 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
     // One launch per pass on the caller's stream.  The single tokens of a mixed step run beside pass 2, on a helper stream: pass 2 holds one SM a
     // chain and is bound by latency, they are bound by memory and take the SMs that its chains leave or never had.  They fork behind
     // pass 1, so that pass 2, which is launched dependent on it, has its SMs first; the gated norm follows pass 2 and runs beside the rest of them.
-    // Those that share a slot with a prompt come in front of it all.
-    // 61 sequences beside three prompts of 1500 tokens, 32 heads: one part behind the other 128 us, 97.8 so; 200
-    // beside one of 100: 176, 165; 128 beside 2048 tokens 218, 147.  (With an event that completes when pass 2's CTAs have started, the
+    // Those that share a slot with a prompt come in front of pass 2.
+    // 61 sequences beside three prompts of 1500 tokens, 32 heads: one part behind the other 128 us, 96.3 so; 200
+    // beside one of 100: 176, 165; 128 beside 2048 tokens 218, 150.  (With an event that completes when pass 2's CTAs have started, the
     // runtime held the single tokens back until pass 2 was complete: 128.)
     plan.r0 = 0; plan.rn = 1 << 24;  // every chunk (times 64 still fits an int)
     SideSet* beside = decode != nullptr ? side_set(dev, stream) : nullptr;
@@ -787,8 +787,8 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
     }
     int rc = AVE_GDN_OK;
     auto step = [&](cudaError_t e) { if (e != cudaSuccess && rc == AVE_GDN_OK) rc = cuda_fail(e); return rc == AVE_GDN_OK; };
-    if (beside != nullptr) rc = launch_shared_slots(*decode, a, stream);
     if (rc == AVE_GDN_OK) step(launch_after(chunk_tiles_kernel, tiles_grid(L.chunks), TILES_THREADS, TILES_SMEM, stream, a, chunk_start, recs, plan, (int)L.chunks, 0));
+    if (rc == AVE_GDN_OK && beside != nullptr) rc = launch_shared_slots(*decode, a, stream);
     const bool forked = rc == AVE_GDN_OK && beside != nullptr && step(cudaEventRecord(beside->fork, stream)) && step(cudaStreamWaitEvent(beside->prep, beside->fork, 0));
     if (rc == AVE_GDN_OK)
       step(launch_after(scan, scan_grid, SCAN_THREADS, SCAN_SMEM, stream, a, maps, chunk_start, recs, o_f32, qt_img, carry, m0_pack, seq_order, plan));

@@ -53,6 +53,6 @@ def test_single_tokens_run_beside_the_scan_and_nothing_waits_through_them(built_
     cu = torch.tensor([0] + list(range(1, n + 1)) + [n + sum(lens[:i + 1]) for i in range(len(lens))], dtype=torch.int32, device="cuda")
     slots = torch.arange(seqs, dtype=torch.int32, device="cuda")
     waits = _waits(lambda: gdn.mixed_prefill_decode_step(inp.q, inp.k, inp.v, inp.g, inp.beta, cu, n, inp.initial_state, slots, z=inp.z))
-    assert waits["gdn_decode_pool"] == {"chunk_tiles"} and waits["chunk_tiles"] == {"gdn_shared_slots"}
-    assert waits["chunk_scan"] == {"chunk_tiles"} and waits["gated_rmsnorm"] == {"chunk_scan"}  # the norm reads the scan's rows: an edge of its own
+    assert waits["gdn_shared_slots"] == {"chunk_tiles"} and waits["gdn_decode_pool"] == {"gdn_shared_slots"}
+    assert waits["chunk_scan"] == {"gdn_shared_slots"} and waits["gated_rmsnorm"] == {"chunk_scan"}  # the norm reads the scan's rows: an edge of its own
     assert not any("gdn_decode_pool" in w for w in waits.values())
