@@ -762,9 +762,10 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
     if (rc == AVE_GDN_OK && !combine_beside) combine(stream);
     if (rc == AVE_GDN_OK) fix_up();
     cudaStream_t aside = norm_beside ? side->prep : combine_beside ? side->norm : nullptr;  // (in a mixed step, a packed layout, `prep` has the single tokens)
-    const bool forked = combine_beside && step(cudaStreamWaitEvent(aside, side->fork, 0));
+    const bool forked = combine_beside && rc == AVE_GDN_OK && step(cudaStreamWaitEvent(aside, side->fork, 0));
     if (forked) combine(aside);
     if (combine_beside && rc == AVE_GDN_OK) norm_of_part0();
+    // (the joins after an error too, so that a surrounding stream capture stays well formed)
     if (forked) { step(cudaEventRecord(side->done[0], aside)); step(cudaStreamWaitEvent(stream, side->done[0], 0)); }
     if (on_norm) { step(cudaEventRecord(side->join_norm, side->norm)); step(cudaStreamWaitEvent(stream, side->join_norm, 0)); }
     return rc;
