@@ -9,11 +9,19 @@
 // makes Vn = U - H W one product: a hand-off less in a step, but W is twice as many bytes as everything else in a record and a third
 // of pass 1.  K itself is exact in bf16, so H K^T takes 16 MMAs where H W^T takes 24.  (262144 packed tokens x 32 heads: 5.75 ms with W,
 // 3.73 without, both after a rest, back to back the power cap makes it 4.1 to 4.3; 8192 tokens 370 us / 344; 4 heads x 32768 254 / 215; 1024 63.4 / 60.6.)
-// A step takes 4.55 k cycles alone and with every SM streaming, of which the tensor pipe is busy 2.4 k: H K^T 0.85 k, X 0.65 k, its
-// product 0.65 k, Vd 0.4 k, the increment 1.1 k, the new state 0.7 k, each of them about a third hand-over (commit or arrival, wake-up,
-// first load).  The conversions are bound by the instructions of a scheduler (a pair of values into two bf16 terms takes 7 cycles of it).
+// A step takes 3.9 to 4.2 k cycles, of which the tensor pipe is busy 2.4 k: H K^T 0.85 k, X 0.55 k, its product 0.45 k, Vd 0.35 k, the increment
+// 0.7 k, the new state 0.7 k, each of them about a third hand-over (arrival or commit, wake-up, first load).  What it took to get there from 4.55 k
+// (8192 tokens x 32 heads 313 -> 260 us, 4 heads x 32768 212 -> 186, 262144 packed tokens 4.17 -> 3.75 ms, all with everything around the scan):
+//   - the code of all roles fits the 32 KB of the SM's instruction cache.  It was 44 KB (rolled waits, outputs in a rolled loop, descriptors from
+//     constants and roles that the compiler knows to be uniform took it down), every step fetched 150 lines of 128 bytes from the cache that the SMs of a GPC
+//     share, and chains ran up to a third slower where more of a GPC's SMs held one;
+//   - the two groups of epilogue warps hand over by halves: a group's tokens of X and Vd, and features of the state, have barriers of their own, so
+//     that the products begin with one half while the other is converted, and an increment's first features are taken while the rest is formed;
+//   - arrivals that the chain waits for are hardware barriers (30 cycles, an mbarrier 85 to 250);
+//   - outputs leave by asynchronous copies: the transition chains' steps were a fifth longer when 32 lines were written an instruction.
+// The conversions are bound by the instructions of a scheduler (a pair of values into two bf16 terms takes 7 cycles of it).
 // O2 waits for the increment: side by side they shared the pipe and the increment came 200 cycles later; H K^T in the increment's columns and not
-// in O2's lets O2 end beside the next step (5.0 -> 4.55 k cycles together).  Measured and dropped: the state a chunk behind the chain by
+// in O2's lets O2 end beside the next step.  Measured and dropped: the state a chunk behind the chain by
 // S(c+1) = decay H(c) K(c+1)^T + Vd(c) (K(c+1) K(c)^T)^T, with three splits of 16 epilogue warps (3.08, 3.52 and 4.48 ms where this
 // form then took 2.73: 11 to 15 k instructions a chunk, and the code of 20 warps misses the instruction cache); the gated norm in
 // the output warps (layer of 8192 tokens 344 -> 374 us with eight of them, 422 with four).
@@ -44,35 +52,33 @@ static_assert(SCAN_SMEM <= SCAN_SMEM_MAX, "shared memory of an SM");
 // TMEM columns: hi and lo image of H, accumulator of Vn (then the images of Vd), images of Vn, outputs, state increment.  H K^T
 // and the images of X take columns of the increment, which they are never alive beside.
 constexpr uint32_t TC_HHI = 0, TC_HLO = 64, TC_VN = 128, TC_VI = 192, TC_O1 = 256, TC_O2 = 320, TC_DH = 384, TC_X = TC_DH;
-// The bf16 hi and lo images of an accumulator of 64 tokens reuse its columns.  Each chain-epilogue group packs its VC tokens
-// into its own VC columns (hi in the first half, lo in the second), so a warp overwrites only columns it has itself
-// read and the groups need no barrier between reading the accumulator and writing the images.
-__host__ __device__ constexpr uint32_t img_col(uint32_t base, int k, bool lo) {  // 16-token step k
-  return base + (uint32_t)(VC * ((16 * k) / VC) + ((16 * k) % VC) / 2 + (lo ? VC / 2 : 0));
+// The bf16 hi and lo images of an accumulator of 64 tokens reuse its columns, 16 tokens by 16 tokens (hi in the first eight columns, lo in the others), so
+// a warp overwrites only columns it has itself read and needs no barrier between reading the accumulator and writing the images.
+__host__ __device__ constexpr uint32_t img_col(uint32_t base, int k, bool lo) { return base + (uint32_t)(16 * k + (lo ? 8 : 0)); }  // 16-token step k
+
+// The products.  `at` is the shared address / 16 of the stage, everything else a constant: with descriptors formed address by address in rolled loops a
+// warp issued an MMA every 30 to 70 cycles, and the triangles' products, 8 to 32 cycles each, waited for it.
+// D[:, 16 k ..] (+)= +-A[:, 16 k .. 16 k + 15] Tri[16 k .., 16 k .. 16 k + 15]^T over the 16-token steps k0 <= k < k1 of the packed lower triangle at `tri` in
+// the stage, for (A hi, Tri hi), (A lo, Tri hi), (A hi, Tri lo); `first` overwrites D: step 0 covers all of its columns.  A: bf16 image in TMEM.
+template <bool kNeg, int k0, int k1, int tri>
+__device__ __forceinline__ void issue_tri(uint32_t d_tmem, uint32_t a_base, uint32_t at, bool first) {
+#pragma unroll
+  for (int t = 0; t < 3; ++t)
+#pragma unroll
+    for (int k = k0; k < k1; ++k)
+      tc::mma_ts(d_tmem + 16 * k, img_col(a_base, k, t == 1),
+                 tc::smem_desc(at + tc::desc_lo(tri + (t == 2 ? REC_TRI : 0) + tri_step(k), 128), tc::desc_hi(256, false)),
+                 tc::idesc_f16(128, 64 - 16 * k, 1, 1, false, false, kNeg, false), (t | k) == 0 && first ? 0u : 1u);
 }
-// The issue loops stay rolled: a warp issues an MMA every 20 to 60 cycles at best, and the code of all roles together has to stay small.
-// D[:, 16 k ..] (+)= +-A[:, 16 k .. 16 k + 15] Tri[16 k .., 16 k .. 16 k + 15]^T over the four 16-token steps of a packed lower triangle, for
-// (A hi, Tri hi), (A lo, Tri hi), (A hi, Tri lo); `first` overwrites D: step 0 covers all of its columns.  A: bf16 image in TMEM.
-template <bool kNeg>
-__device__ __forceinline__ void issue_tri(uint32_t d_tmem, uint32_t a_base, uint32_t tri, bool first) {
-#pragma unroll 1
-  for (int t = 0; t < 3; ++t) {
-    const uint32_t a_img = a_base + (t == 1 ? VC / 2 : 0), b = tri + (t == 2 ? REC_TRI : 0);
+// D (+)= H B^T over the 64 features of group g, H as hi and lo image, B the K-major [64][128] tile at `tile` in the stage; group 0 overwrites D
+template <int tile, int g>
+__device__ __forceinline__ void issue_state(uint32_t d_tmem, uint32_t tm, uint32_t at) {
+#pragma unroll
+  for (int t = 0; t < 2; ++t)
 #pragma unroll
     for (int k = 0; k < 4; ++k)
-      tc::mma_ts(d_tmem + 16 * k, img_col(a_img, k, false), tc::smem_desc_plain(b + tri_step(k), 128, 256),
-                 tc::idesc_f16(128, 64 - 16 * k, 1, 1, false, false, kNeg, false), (first && (t | k) == 0) ? 0u : 1u);
-  }
-}
-// D = H B^T over the 128 features, H as hi and lo image, B a K-major [64][128] tile
-__device__ __forceinline__ void issue_state(uint32_t d_tmem, uint32_t tm, uint32_t tile) {
-  constexpr uint32_t id_n64 = tc::idesc_f16(128, 64, 1, 1, false, false);
-#pragma unroll 1
-  for (int i = 0; i < 4; ++i) {  // hi, lo x features 0 .. 63, 64 .. 127
-    const uint64_t b = tc::smem_desc_sw128(tile + (i & 1) * 8192, 16, 1024);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) tc::mma_ts(d_tmem, tm + TC_HHI + 32 * i + 8 * k, b + (uint64_t)(2 * k), id_n64, (i | k) != 0 ? 1u : 0u);
-  }
+      tc::mma_ts(d_tmem, tm + (t ? TC_HLO : TC_HHI) + 32 * g + 8 * k, tc::smem_desc(at + tc::desc_lo(tile + 8192 * g + 32 * k, 16), tc::desc_hi(1024, true)),
+                 tc::idesc_f16(128, 64, 1, 1, false, false), (g | t | k) != 0 ? 1u : 0u);
 }
 
 // kMulti: built with the parallel-parts machinery (ScanPlan::parts > 1).
@@ -87,25 +93,28 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + CS_BARS);
   uint64_t* full = bars;          // [3] tiles and record of the stage landed
   uint64_t* empty = bars + 3;     // [3] everything that reads the stage is complete
-  uint64_t* h_ready = bars + 6;   // bf16 image of the state is in TMEM
-  uint64_t* kh_full = bars + 7;   // H K^T accumulated
-  uint64_t* x_ready = bars + 8;   // X hi+lo written back to TMEM
-  uint64_t* vn_full = bars + 9;   // Vn = Tu (V - X) accumulated
-  uint64_t* vd_ready = bars + 10; // Vd hi+lo written to TMEM (the state update needs nothing else)
+  uint64_t* vn_full = bars + 6;   // [2] Vn = Tu (V - X) accumulated, for the tokens of each chain-epilogue group
+  uint64_t* dh_full = bars + 8;   // [2] state increment accumulated, for the features of each group
+  uint64_t* kh_full = bars + 10;  // H K^T accumulated
   uint64_t* vn_ready = bars + 11; // Vn hi+lo written to TMEM
-  uint64_t* dh_full = bars + 12;  // state increment accumulated
-  uint64_t* o_full = bars + 13;   // both output accumulators complete
-  uint64_t* o1_empty = bars + 14; // O1 accumulator drained (the output warps take it first, whole, so O1 of the next chunk can run early)
-  uint64_t* o2_empty = bars + 15; // O2 accumulator drained
-  uint64_t* o1_done = bars + 16;  // O1 complete: the bf16 image of H may be overwritten
+  uint64_t* o_full = bars + 12;   // both output accumulators complete
+  uint64_t* o1_empty = bars + 13; // O1 accumulator drained (the output warps take it first, whole, so O1 of the next chunk can run early)
+  uint64_t* o2_empty = bars + 14; // O2 accumulator drained
+  uint64_t* o1_done = bars + 15;  // O1 complete: the bf16 image of H may be overwritten
+  // From a chain-epilogue group to the chain's issuer: bf16 image of its features of the state, X hi+lo and Vd hi+lo of its tokens are in TMEM.  The chain
+  // waits for these, so they are hardware barriers; both roles take part chunk by chunk to the end, whatever became of their other waits.
+  auto h_ready = [](int g) { return tc::NamedBar{1u + g, 32 * (4 + 1)}; };
+  auto x_ready = [](int g) { return tc::NamedBar{1u + NG + g, 32 * (4 + 1)}; };
+  auto vd_ready = [](int g) { return tc::NamedBar{1u + 2 * NG + g, 32 * (4 + 1)}; };
   // A wait sees only the parity of a barrier's phase, so no barrier may complete twice before each of its waiters has seen the first
   // time.  Most are ordered by the arrivals they need.  dh_full is waited for by warp 2 as well, which no increment needs: so warp 1 issues an
   // increment only behind o_full of the chunk before, which warp 2 commits when it has seen dh_full of that chunk.
-  uint64_t* tail_full = bars + 17;  // tiles and record of a ragged last chunk landed: warp 0 clears what lies behind the sequence, then completes `full`
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
+  uint64_t* tail_full = bars + 16;  // tiles and record of a ragged last chunk landed: warp 0 clears what lies behind the sequence, then completes `full`
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (a shuffle, so that the compiler knows a role's code to be uniform: an MMA takes 6 instructions then, and 18 with descriptors in vector registers)
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   pdl_wait();
   // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
   // chain of part p >= 1 (see ScanPlan).
@@ -180,8 +189,9 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
-    tc::mbar_init(h_ready, 4 * NG); tc::mbar_init(x_ready, 4 * NG); tc::mbar_init(vd_ready, 4 * NG); tc::mbar_init(vn_ready, 4 * NG);
-    for (uint64_t* b : {kh_full, vn_full, dh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
+    for (int i = 0; i < NG; ++i) { tc::mbar_init(&vn_full[i], 1); tc::mbar_init(&dh_full[i], 1); }
+    tc::mbar_init(vn_ready, 4 * NG);
+    for (uint64_t* b : {kh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
     tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
     *abort_flag = 0;
     tc::fence_barrier_init();
@@ -190,7 +200,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
-  const uint32_t tm = *tmem_slot;
+  constexpr uint32_t tm = 0;  // all 512 columns are this CTA's, so the first is column 0
   const bool ragged = a.cu_seqlens != nullptr && sp.len < n_chunks * C;
 
   if (warp < 4) {
@@ -246,66 +256,98 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     // elected lane issues): the MMAs the recurrence waits for.  One thread needs 20 to 60 cycles per MMA instruction, so
     // the instructions of a chunk are shared between two warps; this one keeps the state-dependent ones short:
     //   U^T(c+1) -> [state published] H K^T(c) -> [X written] Vn^T(c) -> [Vd written] dH(c)
-    constexpr uint32_t id_dh = tc::idesc_f16(128, 128, 1, 1, false, true);                // B MN-major
+    constexpr uint32_t id_dh = tc::idesc_f16(128, 128, 1, 1, false, true), id_dh_half = tc::idesc_f16(128, 64, 1, 1, false, true);  // B MN-major
     // U^T = V^T (Tu_hi + Tu_lo)^T opens the Vn^T accumulator of a chunk.  It does not depend on the state, so it is
     // issued a chunk ahead, right behind the previous chunk's state-increment MMAs (which read the Vd images in the
     // same columns and, issued earlier by this thread, complete first): the tensor pipe runs it while the chain
     // epilogue re-packs H.
-    auto issue_u = [&](uint32_t sb) {
+    auto issue_u = [&](uint32_t at) {
       if (phi) return;  // v = 0: U^T = 0, the first Vn MMA overwrites the accumulator instead
       if (tc::elect_one()) {
-#pragma unroll 1
+#pragma unroll
         for (int t = 0; t < 2; ++t)
 #pragma unroll
           for (int k = 0; k < 4; ++k)  // 16 tokens per step: V rows 2048 bytes apart, feature halves 8192 bytes apart
-            tc::mma_ss(tm + TC_VN + 16 * k, tc::smem_desc_sw128(sb + CS_V + k * 2048, 8192, 1024),
-                       tc::smem_desc_plain(sb + CS_REC + REC_TU + t * REC_TRI + tri_step(k), 128, 256),
+            tc::mma_ss(tm + TC_VN + 16 * k, tc::smem_desc(at + tc::desc_lo(CS_V + k * 2048, 8192), tc::desc_hi(1024, true)),
+                       tc::smem_desc(at + tc::desc_lo(CS_REC + REC_TU + t * REC_TRI + tri_step(k), 128), tc::desc_hi(256, false)),
                        tc::idesc_f16(128, 64 - 16 * k, 1, 1, true, false), (t | k) != 0 ? 1u : 0u);
       }
       __syncwarp();
     };
     int s = 0, s_next = 1;
     uint32_t ph_next = 0;
-    const uint32_t smem0 = tc::smem_u32(smem);
-    bool issuing = n_chunks > 0 && tc::mbar_wait_warp(&full[0], 0u, abort_flag);
-    if (issuing) { tc::tc_fence_after_sync(); issue_u(smem0); }
-    for (int c = 0; c < n_chunks && issuing; ++c) {
-      const uint32_t cp = (uint32_t)c & 1u;
-      const uint32_t sb = smem0 + s * CS_STAGE;  // the stage has landed: this warp waited for it a chunk ago
-      if (!tc::mbar_wait_warp(h_ready, cp, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        issue_state(tm + TC_X, tm, sb + CS_K);
-        tc::mma_commit(kh_full);
-        // the MMAs of the chunk before are complete with these, and the epilogue, which has published a state, is through with its scale vectors
-        if (c > 0) tc::mma_commit(&empty[s == 0 ? CS_STAGES - 1 : s - 1]);
-      }
-      __syncwarp();
-      if (!tc::mbar_wait_warp(x_ready, cp, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        issue_tri<true>(tm + TC_VN, tm + TC_X, sb + CS_REC + REC_TU, phi);  // Vn^T -= X Tu^T
-        tc::mma_commit(vn_full);
-      }
-      __syncwarp();
-      if (!tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) break;  // warp 2 has seen dh_full of the chunk before (and O2 is long complete)
-      if (!tc::mbar_wait_warp(vd_ready, cp, abort_flag)) break;
-      tc::tc_fence_after_sync();
-      if (tc::elect_one()) {
-        // dH = (Vd_hi + Vd_lo) contracted with K over the chunk's tokens (K tile read MN-major: 16 token rows per step)
-        const uint64_t k_desc = tc::smem_desc_sw128(sb + CS_K, 8192, 1024);
-#pragma unroll 1
-        for (int t = 0; t < 2; ++t)
+    const uint32_t smem0 = tc::smem_u32(smem) >> 4;
+    tc::mbar_wait_warp(&full[0], 0u, abort_flag);
+    tc::tc_fence_after_sync();
+    issue_u(smem0);
+    // What the chain waits for, step by step.  A bounded wait that expires raises the flag and this role goes on, with products that nobody will use.
+    auto state_product = [&](int c, uint32_t at, int s) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            tc::mma_ts(tm + TC_DH, img_col(tm + TC_VN + t * (VC / 2), k, false), k_desc + (uint64_t)(128 * k), id_dh, (t | k) != 0 ? 1u : 0u);
-        tc::mma_commit(dh_full);
-      }
-      __syncwarp();
-      if (c + 1 < n_chunks) {
-        if (!tc::mbar_wait_warp(&full[s_next], ph_next, abort_flag)) break;
+      for (int g = 0; g < NG; ++g) {
+        tc::mbar_wait_warp(h_ready(g), (uint32_t)c & 1u, abort_flag);
         tc::tc_fence_after_sync();
-        issue_u(smem0 + s_next * CS_STAGE);
+        if (tc::elect_one()) {
+          if (g == 0) issue_state<CS_K, 0>(tm + TC_X, tm, at);
+          else issue_state<CS_K, 1>(tm + TC_X, tm, at);
+          if (g == NG - 1) {
+            tc::mma_commit(kh_full);
+            // the MMAs of the chunk before are complete with these, and the epilogue, which has published a state, is through with its scale vectors
+            if (c > 0) tc::mma_commit(&empty[s == 0 ? CS_STAGES - 1 : s - 1]);
+          }
+        }
+        __syncwarp();
+      }
+    };
+    auto new_values = [&](int c, uint32_t at) {  // Vn^T -= X Tu^T; the tokens of a group need those before them only
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        tc::mbar_wait_warp(x_ready(g), (uint32_t)c & 1u, abort_flag);
+        tc::tc_fence_after_sync();
+        if (tc::elect_one()) {
+          if (g == 0) issue_tri<true, 0, 2, CS_REC + REC_TU>(tm + TC_VN, tm + TC_X, at, phi);
+          else issue_tri<true, 2, 4, CS_REC + REC_TU>(tm + TC_VN, tm + TC_X, at, phi);
+          tc::mma_commit(&vn_full[g]);
+        }
+        __syncwarp();
+      }
+    };
+    auto outputs_before = [&](int c) {  // warp 2 has seen dh_full of the chunk before (and O2 is long complete)
+      tc::mbar_wait_warp(o_full, (uint32_t)(c + 1) & 1u, abort_flag);
+    };
+    auto increment = [&](int c, uint32_t at) {
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        tc::mbar_wait_warp(vd_ready(g), (uint32_t)c & 1u, abort_flag);
+        tc::tc_fence_after_sync();
+        if (tc::elect_one()) {
+          // dH = (Vd_hi + Vd_lo) contracted with K over the group's tokens (K tile read MN-major: 16 token rows per step); the last
+          // tokens for half of the features at a time, so that one group takes its half while the other's is formed
+#pragma unroll
+          for (int f = 0; f <= g; ++f) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i)  // hi, lo x two steps
+              tc::mma_ts(tm + TC_DH + 64 * f, img_col(tm + TC_VN, 2 * g + (i & 1), i >> 1),
+                         tc::smem_desc(at + tc::desc_lo(CS_K + 8192 * f + 2048 * (2 * g + (i & 1)), 8192), tc::desc_hi(1024, true)),
+                         g == 0 ? id_dh : id_dh_half, (g | i) != 0 ? 1u : 0u);
+            if (g == NG - 1) tc::mma_commit(&dh_full[f]);
+          }
+        }
+        __syncwarp();
+      }
+    };
+    auto values_of = [&](int stage, uint32_t parity) {
+      tc::mbar_wait_warp(&full[stage], parity, abort_flag);
+      tc::tc_fence_after_sync();
+      issue_u(smem0 + stage * (CS_STAGE >> 4));
+    };
+    for (int c = 0; c < n_chunks; ++c) {  // (to the end also when a wait has expired)
+      const uint32_t at = smem0 + s * (CS_STAGE >> 4);  // the stage has landed: this warp waited for it a chunk ago
+      state_product(c, at, s);
+      outputs_before(c);  // (for the increment, but here the wait is hidden behind the conversion of X; a wait for what is complete takes 130 to 250 cycles)
+      new_values(c, at);
+      increment(c, at);
+      if (c + 1 < n_chunks) {
+        values_of(s_next, ph_next);
         s = s_next;
         if (++s_next == CS_STAGES) { s_next = 0; ph_next ^= 1u; }
       }
@@ -313,23 +355,25 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   } else if (warp == 2) {
     // ------------------------------------------------------------------ output MMA issuer: O1 = H Q^T once H K^T is
     // complete (so that it runs behind it, while the chain epilogue converts X), O2 = Vn P^T once Vn hi/lo are back
+    const uint32_t smem0 = tc::smem_u32(smem) >> 4;
     int s = 0;
     uint32_t ph = 0;
     for (int c = 0; c < n_chunks; ++c) {
       const uint32_t cp = (uint32_t)c & 1u;
-      const uint32_t sb = tc::smem_u32(smem) + s * CS_STAGE;
-      if (!tc::mbar_wait3(kh_full, cp, o1_empty, cp ^ 1u, &full[s], ph, abort_flag)) break;
+      const uint32_t at = smem0 + s * (CS_STAGE >> 4);
+      tc::mbar_wait3(kh_full, cp, o1_empty, cp ^ 1u, &full[s], ph, abort_flag);
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
-        issue_state(tm + TC_O1, tm, sb + CS_Q);  // the chain epilogue waits for its completion before it overwrites the bf16 image of H
+        issue_state<CS_Q, 0>(tm + TC_O1, tm, at);
+        issue_state<CS_Q, 1>(tm + TC_O1, tm, at);  // the chain epilogue waits for its completion before it overwrites the bf16 image of H
         tc::mma_commit(o1_done);
       }
       __syncwarp();
       // behind the state increment, which the recurrence waits for: side by side they would share the tensor pipe
-      if (!tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, dh_full, cp, abort_flag)) break;
+      tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, &dh_full[1], cp, abort_flag);
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
-        issue_tri<false>(tm + TC_O2, tm + TC_VI, sb + CS_REC + REC_PT, true);  // O2 = Vn P^T
+        issue_tri<false, 0, 4, CS_REC + REC_PT>(tm + TC_O2, tm + TC_VI, at, true);  // O2 = Vn P^T
         tc::mma_commit(o_full);
         tc::mma_commit(&empty[s]);
       }
@@ -376,35 +420,39 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       tc::tmem_st_wait();
       tc::tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) tc::mbar_arrive(h_ready);
+      tc::mbar_arrive(h_ready(grp));
     };
     publish_h();
 
     int s = 0;
     uint32_t ph = 0;
-    for (int c = 0; c < n_chunks && alive; ++c) {
+    for (int c = 0; c < n_chunks; ++c) {  // (to the end also when a wait has expired: the chain's issuer counts on the arrivals)
       const uint32_t cp = (uint32_t)c & 1u;
       const float* scal = reinterpret_cast<const float*>(smem + s * CS_STAGE + CS_REC + REC_SCAL);
-      if (!tc::mbar_wait2(&full[s], ph, kh_full, cp, abort_flag)) { alive = false; break; }  // (the scale vectors come with the stage)
+      alive = tc::mbar_wait2(&full[s], ph, kh_full, cp, abort_flag) && alive;  // (the scale vectors come with the stage)
       if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
       tc::tc_fence_after_sync();
       {  // X_j = kx_j H k_j
-        uint32_t acc[VC], xh[VC / 2], xl[VC / 2];
-        tc::tmem_ld_n<VC>(lane_addr + TC_X + VC * grp, acc);
-        tc::tmem_ld_wait();
+#pragma unroll 1
+        for (int k = 0; k < VC / 16; ++k) {
+          uint32_t acc[16], xh[8], xl[8];
+          tc::tmem_ld16(lane_addr + TC_X + VC * grp + 16 * k, acc);
+          tc::tmem_ld_wait();
 #pragma unroll
-        for (int w = 0; w < VC / 2; ++w) {
-          const float2 kx = *reinterpret_cast<const float2*>(scal + 2 * C + VC * grp + 2 * w);
-          split_pair(__fmul2_rn(make_float2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1])), kx), xh[w], xl[w]);
+          for (int w = 0; w < 8; w += 2) {
+            const float4 kx = *reinterpret_cast<const float4*>(scal + 2 * C + VC * grp + 16 * k + 2 * w);
+            split_pair(__fmul2_rn(make_float2(__uint_as_float(acc[2 * w]), __uint_as_float(acc[2 * w + 1])), make_float2(kx.x, kx.y)), xh[w], xl[w]);
+            split_pair(__fmul2_rn(make_float2(__uint_as_float(acc[2 * w + 2]), __uint_as_float(acc[2 * w + 3])), make_float2(kx.z, kx.w)), xh[w + 1], xl[w + 1]);
+          }
+          tc::tmem_st8(lane_addr + TC_X + VC * grp + 16 * k, xh);  // into this warp's own accumulator columns
+          tc::tmem_st8(lane_addr + TC_X + VC * grp + 16 * k + 8, xl);
         }
-        tc::tmem_st_n<VC / 2>(lane_addr + TC_X + VC * grp, xh);  // into this warp's own accumulator columns
-        tc::tmem_st_n<VC / 2>(lane_addr + TC_X + VC * grp + VC / 2, xl);
         tc::tmem_st_wait();
         tc::tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(x_ready);
+        tc::mbar_arrive(x_ready(grp));
       }
-      if (!tc::mbar_wait_warp(vn_full, cp, abort_flag)) { alive = false; break; }
+      alive = tc::mbar_wait_warp(&vn_full[grp], cp, abort_flag) && alive;
       tc::tc_fence_after_sync();
       {
         uint32_t acc[VC];
@@ -416,32 +464,39 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
         {  // Vd first: its columns alias nothing, and the state update waits only for it
           uint32_t dh[VC / 2], dl[VC / 2];
 #pragma unroll
-          for (int w = 0; w < VC / 2; ++w) {
-            const float2 ks = *reinterpret_cast<const float2*>(scal + C + VC * grp + 2 * w);
-            split_pair(__fmul2_rn(v[w], ks), dh[w], dl[w]);
+          for (int w = 0; w < VC / 2; w += 2) {
+            const float4 ks = *reinterpret_cast<const float4*>(scal + C + VC * grp + 2 * w);
+            split_pair(__fmul2_rn(v[w], make_float2(ks.x, ks.y)), dh[w], dl[w]);
+            split_pair(__fmul2_rn(v[w + 1], make_float2(ks.z, ks.w)), dh[w + 1], dl[w + 1]);
           }
-          tc::tmem_st_n<VC / 2>(lane_addr + TC_VN + VC * grp, dh);  // into this warp's own accumulator columns
-          tc::tmem_st_n<VC / 2>(lane_addr + TC_VN + VC * grp + VC / 2, dl);
+#pragma unroll
+          for (int k = 0; k < VC / 16; ++k) {  // into this warp's own accumulator columns
+            tc::tmem_st8(lane_addr + TC_VN + VC * grp + 16 * k, reinterpret_cast<const uint32_t(&)[8]>(dh[8 * k]));
+            tc::tmem_st8(lane_addr + TC_VN + VC * grp + 16 * k + 8, reinterpret_cast<const uint32_t(&)[8]>(dl[8 * k]));
+          }
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(vd_ready);
+          tc::mbar_arrive(vd_ready(grp));
         }
         // the Vn images of the chunk before have been read (long ago: its O2 ran beside its state's conversion)
-        if (!tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) { alive = false; break; }
+        alive = tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag) && alive;
         {
           uint32_t vh[VC / 2], vl[VC / 2];
 #pragma unroll
           for (int w = 0; w < VC / 2; ++w) split_pair(v[w], vh[w], vl[w]);
-          tc::tmem_st_n<VC / 2>(lane_addr + TC_VI + VC * grp, vh);
-          tc::tmem_st_n<VC / 2>(lane_addr + TC_VI + VC * grp + VC / 2, vl);
+#pragma unroll
+          for (int k = 0; k < VC / 16; ++k) {  // beside them
+            tc::tmem_st8(lane_addr + TC_VI + VC * grp + 16 * k, reinterpret_cast<const uint32_t(&)[8]>(vh[8 * k]));
+            tc::tmem_st8(lane_addr + TC_VI + VC * grp + 16 * k + 8, reinterpret_cast<const uint32_t(&)[8]>(vl[8 * k]));
+          }
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
           __syncwarp();
           if (lane == 0) tc::mbar_arrive(vn_ready);
         }
       }
-      if (!tc::mbar_wait2(dh_full, cp, o1_done, cp, abort_flag)) { alive = false; break; }
+      alive = tc::mbar_wait2(&dh_full[grp], cp, o1_done, cp, abort_flag) && alive;
       tc::tc_fence_after_sync();
       {
         const float decay = scal[3 * C];
@@ -455,7 +510,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
             Hreg[16 * part32 + w] = __ffma2_rn(make_float2(decay, decay), Hreg[16 * part32 + w],
                                                make_float2(__uint_as_float(dh[2 * w]), __uint_as_float(dh[2 * w + 1])));
         }
-        publish_h();
+        if (c + 1 < n_chunks) publish_h();  // (as often as the issuer waits)
       }
     }
     if (alive && state_out != nullptr) {
@@ -480,96 +535,112 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     }
   } else {
     tc::reg_set<REGS_OUT, REGS_LAUNCH>();
-    // ------------------------------------------------------------------ output warps: o = qs_i O1 + O2, a d_v row per thread.  Rows of
-    // tokens are formed in shared memory, in the place of the chunk's Q and K tiles (all MMAs that read them are complete with O2), so
-    // that each warp's 32 features leave in 16-byte pieces (a quarter of the store instructions of one element per lane).
-    const int wq = warp & 3, d = wq * 32 + lane;
+    // ------------------------------------------------------------------ output warps: o = qs_i O1 + O2, 32 features a warp, as accumulator
+    // fragments of warp-level MMAs, which matrix stores transpose on their way into shared memory.  The tiles are formed there, in the place of the chunk's Q
+    // and K (all MMAs that read them are complete with O2), 8 KB a warp, and leave by one asynchronous copy each: these warps run beside the
+    // conversions that the chain waits for.  (With a row of d_v a thread, scalar stores, and 16-byte loads and stores on the way out, a chunk took them 2.0 to
+    // 2.8 k cycles and the transition chains' steps were a fifth longer than the others': their rows went to 32 lines an instruction.)
+    const int wq = warp & 3, gr = lane >> 2, t2 = 2 * (lane & 3), r8 = lane & 7, m4 = lane >> 3;
     const uint32_t lane_addr = tm + ((uint32_t)(wq * 32) << 16);
     int s = 0;
     for (int c = 0; c < n_chunks; ++c) {
       const uint32_t cp = (uint32_t)c & 1u;
       const float* scal = reinterpret_cast<const float*>(smem + s * CS_STAGE + CS_REC + REC_SCAL);
-      float* stage = reinterpret_cast<float*>(smem + s * CS_STAGE);  // [64 tokens][128 features]
-      // 16-byte piece p of token t: neighbouring pieces trade places, so that lanes two pieces, or a token, apart meet different banks
-      auto piece16 = [&](int t, int p) { return stage + t * D + 4 * (p ^ (((p >> 3) ^ t) & 1)); };
+      uint8_t* stage = smem + s * CS_STAGE + wq * 8192;
+      const uint32_t stage_s = tc::smem_u32(stage);
       const int len = min(C, sp.len - c * C);
       const int64_t tok0 = sp.t0 + c * C;
       // o_full is committed by the MMA warp after it saw this chunk's stage (tiles and scale vectors) land, so it also
       // orders the scale vectors; waiting on the stage barrier here would alias phases once this warp lags a chunk
       if (!tc::mbar_wait_warp(o_full, cp, abort_flag)) break;
       tc::tc_fence_after_sync();
-      // O1 is taken whole and released at once: O1 of the next chunk is the first thing the tensor pipe runs while the
-      // chain epilogue converts X, and must not wait for the stores below.
-      uint32_t o1[C];
-      tc::tmem_ld32(lane_addr + TC_O1, reinterpret_cast<uint32_t(&)[32]>(o1[0]));
-      tc::tmem_ld32(lane_addr + TC_O1 + 32, reinterpret_cast<uint32_t(&)[32]>(o1[32]));
-      tc::tmem_ld_wait();
-      tc::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(o1_empty);
-      // O2 follows in pieces and is folded into the registers that hold O1
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        uint32_t o2[16];
-        tc::tmem_ld16(lane_addr + TC_O2 + 16 * p, o2);
+      const bool whole = !(ragged && c == n_chunks - 1);  // (behind the end of a dense batch row the copies write nothing)
+      // 16 features at a time, in a loop that stays rolled: the code of all roles together has to stay small
+#pragma unroll 1
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t o[32], o2[32];  // [4 g + 2 rr + e]: feature 32 wq + 16 hf + 8 rr + gr, token 8 g + t2 + e
+        tc::tmem_ld_frags(lane_addr + ((uint32_t)hf << 20) + TC_O1, o);
+        tc::tmem_ld_frags(lane_addr + ((uint32_t)hf << 20) + TC_O2, o2);
         tc::tmem_ld_wait();
-        if (p == 3) {
+        if (hf == 1) {
           tc::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(o2_empty);
+          if (lane == 0) { tc::mbar_arrive(o1_empty); tc::mbar_arrive(o2_empty); }
         }
+        auto pair = [&](int g, int rr) { return make_float2(__uint_as_float(o[4 * g + 2 * rr]), __uint_as_float(o[4 * g + 2 * rr + 1])); };
 #pragma unroll
-        for (int j4 = 0; j4 < 4; ++j4) {
-          const int j = 16 * p + 4 * j4;
-          const float4 qs = *reinterpret_cast<const float4*>(scal + j);
-          const float2 r0 = __ffma2_rn(make_float2(qs.x, qs.y), make_float2(__uint_as_float(o1[j]), __uint_as_float(o1[j + 1])),
-                                       make_float2(__uint_as_float(o2[4 * j4]), __uint_as_float(o2[4 * j4 + 1])));
-          const float2 r1 = __ffma2_rn(make_float2(qs.z, qs.w), make_float2(__uint_as_float(o1[j + 2]), __uint_as_float(o1[j + 3])),
-                                       make_float2(__uint_as_float(o2[4 * j4 + 2]), __uint_as_float(o2[4 * j4 + 3])));
-          o1[j] = __float_as_uint(r0.x); o1[j + 1] = __float_as_uint(r0.y); o1[j + 2] = __float_as_uint(r1.x); o1[j + 3] = __float_as_uint(r1.y);
+        for (int g = 0; g < C / 8; ++g) {
+          const float2 qs = *reinterpret_cast<const float2*>(scal + 8 * g + t2);
+#pragma unroll
+          for (int rr = 0; rr < 2; ++rr) {
+            uint32_t* x = &o[4 * g + 2 * rr];
+            const float2 y = __ffma2_rn(qs, pair(g, rr), make_float2(__uint_as_float(o2[4 * g + 2 * rr]), __uint_as_float(o2[4 * g + 2 * rr + 1])));
+            x[0] = __float_as_uint(y.x); x[1] = __float_as_uint(y.y);
+          }
+        }
+        if (kMulti && phi) {
+          // qt^T of this chunk as bf16 hi and lo images [128 d_k rows][64 tokens] with the 128-byte swizzle: the fix-up
+          // reads them, unchanged, as the MN-major A operand of its MMA.  32 rows a warp, 4 KB of each image.
+          const uint32_t at = stage_s + (uint32_t)((16 * hf + 8 * (m4 & 1) + r8) * 128);
+#pragma unroll
+          for (int g = 0; g < C / 8; g += 2) {
+            uint32_t hi[4], lo[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) split_pair(pair(g + (m >> 1), m & 1), hi[m], lo[m]);
+            const uint32_t off = (uint32_t)(((g + (m4 >> 1)) ^ r8) << 4);
+            stsm4(at + off, hi[0], hi[1], hi[2], hi[3]);
+            stsm4(at + off + 4096, lo[0], lo[1], lo[2], lo[3]);
+          }
+        } else if (out_f32 != nullptr) {  // [64 tokens][32 features] of 4 bytes, 128-byte swizzle
+          const int c0 = (4 * hf) ^ (gr >> 2) ^ t2;
+#pragma unroll
+          for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+              float* at = reinterpret_cast<float*>(stage + (t2 + e) * 128 + (((2 * rr) ^ c0 ^ e) << 4)) + (gr & 3);
+#pragma unroll
+              for (int g = 0; g < C / 8; ++g) at[256 * g] = __uint_as_float(o[4 * g + 2 * rr + e]);
+            }
+        } else {  // [64 tokens][32 features] of 2 bytes, 64-byte swizzle
+          const uint32_t at = stage_s + (uint32_t)((8 * (m4 >> 1) + r8) * 64 + (((2 * hf + (m4 & 1)) ^ (r8 >> 1)) << 4));
+#pragma unroll
+          for (int g = 0; g < C / 8; g += 2) {
+            uint32_t x[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) { const float2 y = pair(g + (m >> 1), m & 1); x[m] = pack_bf16x2(y.x, y.y); }
+            stsm4t(at + 512 * g, x[0], x[1], x[2], x[3]);
+          }
         }
       }
+      tc::fence_proxy_async_smem();
+      __syncwarp();
       if (kMulti && phi) {
-        // qt^T of this chunk as bf16 hi and lo images [128 d_k rows][64 tokens] with the 128-byte swizzle: the fix-up
-        // reads them, unchanged, as the MN-major A operand of its MMA.  This thread owns row d.
-        uint8_t* img = qt_img + ((int64_t)(c_first + c) * a.Hv + h) * (int64_t)QT_BYTES + d * 128;
-#pragma unroll
-        for (int e8 = 0; e8 < C / 8; ++e8) {
-          uint32_t hi[4], lo[4];
-#pragma unroll
-          for (int w = 0; w < 4; ++w) split_pair(make_float2(__uint_as_float(o1[8 * e8 + 2 * w]), __uint_as_float(o1[8 * e8 + 2 * w + 1])), hi[w], lo[w]);
-          const uint32_t off = (uint32_t)((e8 ^ (d & 7)) << 4);
-          *reinterpret_cast<uint4*>(img + off) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-          *reinterpret_cast<uint4*>(img + C * D * 2 + off) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+        if (lane == 0) {
+          uint8_t* img = qt_img + ((int64_t)(c_first + c) * a.Hv + h) * (int64_t)QT_BYTES + wq * 4096;
+          tc::bulk_store(img, stage, 4096);
+          tc::bulk_store(img + C * D * 2, stage + 4096, 4096);
         }
+      } else if (whole && (out_f32 != nullptr || maps.o_ok)) {
+        if (lane == 0) tc::tma_store_4d(out_f32 != nullptr ? &maps.o32 : &maps.o, stage, 32 * wq, h, (int)tok0, sp.b);
+      } else if (out_f32 != nullptr) {
+        float* dst = out_f32 + (((int64_t)sp.b * a.T + tok0) * a.Hv + h) * D + 32 * wq + 4 * r8;
+#pragma unroll 1
+        for (int t = m4; t < len; t += 4) *reinterpret_cast<float4*>(dst + (int64_t)t * a.Hv * D) = *reinterpret_cast<const float4*>(stage + t * 128 + ((r8 ^ (t & 7)) << 4));
       } else {
-#pragma unroll
-        for (int t = 0; t < C; ++t) piece16(t, d >> 2)[d & 3] = __uint_as_float(o1[t]);
-        __syncwarp();
-        if (out_f32 != nullptr) {
-          float* dst = out_f32 + (((int64_t)sp.b * a.T + tok0) * a.Hv + h) * D + 32 * wq + 4 * (lane & 7);
-#pragma unroll 4
-          for (int i = 0; i < 16; ++i) {
-            const int t = 4 * i + (lane >> 3);
-            const float4 v = *reinterpret_cast<const float4*>(piece16(t, 8 * wq + (lane & 7)));
-            if (t < len) *reinterpret_cast<float4*>(dst + (int64_t)t * a.Hv * D) = v;
-          }
-        } else {
-          const int p = 8 * wq + 2 * (lane & 3);
-#pragma unroll 4
-          for (int i = 0; i < 8; ++i) {
-            const int t = 8 * i + (lane >> 2);
-            const float4 v = *reinterpret_cast<const float4*>(piece16(t, p)), w = *reinterpret_cast<const float4*>(piece16(t, p + 1));
-            if (t < len)
-              *reinterpret_cast<uint4*>(og + (tok0 + t) * a.o_stride_t + 4 * p) = make_uint4(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w), pack_bf16x2(w.x, w.y), pack_bf16x2(w.z, w.w));
-          }
-        }
-        tc::fence_proxy_async_smem();  // the next tiles of this stage come by asynchronous copies
+        __nv_bfloat16* dst = og + tok0 * a.o_stride_t + 32 * wq + 8 * (lane & 3);
+#pragma unroll 1
+        for (int t = lane >> 2; t < len; t += 8) *reinterpret_cast<uint4*>(dst + t * a.o_stride_t) = *reinterpret_cast<const uint4*>(stage + t * 64 + (((lane & 3) ^ ((t >> 1) & 3)) << 4));
+        tc::fence_proxy_async_smem();
+      }
+      if (lane == 0) {  // the next tiles of this stage come when it has been read
+        tc::bulk_commit();
+        tc::bulk_wait_read<0>();
       }
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&empty[s]);
       if (++s == CS_STAGES) s = 0;
     }
+    if (lane == 0) tc::bulk_wait_all();
   }
 
   tc::tc_fence_before_sync();

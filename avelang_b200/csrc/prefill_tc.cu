@@ -142,6 +142,8 @@ __global__ void chunk_table_tc_kernel(const int32_t* cu_seqlens, int n_seqs, int
 
 struct GdnMaps {
   CUtensorMap q, k, v;
+  CUtensorMap o, o32;  // 32 features of 64 tokens: the result, and the rows that wait in fp32 scratch
+  bool o_ok;           // the result's layout can be described by a map
 };
 
 // How one launch cuts the chunks of every sequence.
@@ -712,6 +714,22 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
     AVE_CUDA_TRY(launch_after(chunk_table_tc_kernel, 1, a.n_seqs <= 256 ? 256 : 1024, 0, stream, a.cu_seqlens, a.n_seqs, a.T, chunk_start, (int)L.chunks, a.status));
   }
   float* o_f32 = L.parts > 1 || a.z != nullptr ? reinterpret_cast<float*>(ws + L.o_f32) : nullptr;
+  {
+    const uint32_t box[4] = {32, 1, 64, 1};
+    const uint64_t dims[4] = {D, (uint64_t)a.Hv, (uint64_t)a.T, (uint64_t)a.B};
+    maps.o_ok = false;
+    if (a.z == nullptr) {
+      const uint64_t so[4] = {2, (uint64_t)a.o_stride_h * 2, (uint64_t)a.o_stride_t * 2, (uint64_t)(a.B > 1 ? a.o_stride_b : a.o_stride_t * a.T) * 2};
+      const int last_error = g_last_cuda_error;
+      maps.o_ok = make_tmap(&maps.o, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a.o, 4, dims, so, box, CU_TENSOR_MAP_SWIZZLE_64B) == AVE_GDN_OK;
+      if (!maps.o_ok) g_last_cuda_error = last_error;  // (no fault: 16-byte stores then)
+    }
+    if (o_f32 != nullptr) {
+      const uint64_t row = (uint64_t)a.Hv * D * 4, s32[4] = {4, D * 4, row, row * a.T};
+      const int rc = make_tmap(&maps.o32, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, o_f32, 4, dims, s32, box, CU_TENSOR_MAP_SWIZZLE_128B);
+      if (rc != AVE_GDN_OK) return rc;
+    }
+  }
   uint8_t* qt_img = L.parts > 1 ? reinterpret_cast<uint8_t*>(ws + L.qt_img) : nullptr;
   float* carry = reinterpret_cast<float*>(ws + L.carry);
   uint8_t* m0_pack = reinterpret_cast<uint8_t*>(ws + L.m0_pack);

@@ -36,42 +36,41 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after ~kWaitLimit polls or as soon as another role has raised *abort_flag.
+// Bounded wait: gives up after kWaitLimit polls that found the phase incomplete, or as soon as another role has raised *abort_flag.
 // Returns false on give-up (the caller raises the flag, records a status bit and leaves its loop).
+// The loops stay rolled, here and below: unrolled, a wait took 64 instructions and one for three phases 200, and a kernel of many roles no longer fitted the
+// SM's 32 KB of instruction cache (the prefill's scan 44 KB of loops; 8192 tokens x 32 heads 297 -> 260 us).
 constexpr uint32_t kWaitLimit = 1u << 24;
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 63u && *abort_flag != 0u) return false;
-  }
-  *abort_flag = 1u;
-  return false;
+  uint32_t left = kWaitLimit;
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity))
+    if (*abort_flag != 0u || --left == 0u) { *abort_flag = 1u; return false; }
+  return true;
 }
 
 // Bounded waits for two or three phases at once.  The polls are independent, so the latencies of phases that are
 // already complete overlap instead of adding up.
 __device__ __forceinline__ bool mbar_wait2(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, volatile uint32_t* abort_flag) {
-  bool d0 = false, d1 = false;
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
-    const bool n0 = d0 || mbar_try_wait(b0, p0), n1 = d1 || mbar_try_wait(b1, p1);
-    d0 = n0; d1 = n1;
-    if (d0 && d1) return true;
-    if ((it & 63u) == 63u && *abort_flag != 0u) return false;
+  uint32_t left = kWaitLimit;
+  bool d0 = false, d1 = false;  // seen complete, once and for all
+#pragma unroll 1
+  for (;;) {
+    d0 |= mbar_try_wait(b0, p0); d1 |= mbar_try_wait(b1, p1);
+    if (d0 & d1) return true;
+    if (*abort_flag != 0u || --left == 0u) { *abort_flag = 1u; return false; }
   }
-  *abort_flag = 1u;
-  return false;
 }
 __device__ __forceinline__ bool mbar_wait3(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, uint64_t* b2, uint32_t p2,
                                            volatile uint32_t* abort_flag) {
+  uint32_t left = kWaitLimit;
   bool d0 = false, d1 = false, d2 = false;
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
-    const bool n0 = d0 || mbar_try_wait(b0, p0), n1 = d1 || mbar_try_wait(b1, p1), n2 = d2 || mbar_try_wait(b2, p2);
-    d0 = n0; d1 = n1; d2 = n2;
-    if (d0 && d1 && d2) return true;
-    if ((it & 63u) == 63u && *abort_flag != 0u) return false;
+#pragma unroll 1
+  for (;;) {
+    d0 |= mbar_try_wait(b0, p0); d1 |= mbar_try_wait(b1, p1); d2 |= mbar_try_wait(b2, p2);
+    if (d0 & d1 & d2) return true;
+    if (*abort_flag != 0u || --left == 0u) { *abort_flag = 1u; return false; }
   }
-  *abort_flag = 1u;
-  return false;
 }
 
 // Bounded wait called by all 32 lanes of a converged warp.  Every lane polls: letting lane 0 poll alone and
@@ -80,6 +79,14 @@ __device__ __forceinline__ bool mbar_wait3(uint64_t* b0, uint32_t p0, uint64_t* 
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
   return mbar_wait(bar, parity, abort_flag);
 }
+
+// A hardware barrier as a hand-off: `threads` of them arrive or wait, whole warps, and those that wait go on when all are there.  30 cycles from the
+// last arrival to the first instruction behind the wait, an mbarrier 85 to 100 (alone on an SM; more beside others' shared-memory traffic).
+// A wait on it is not bounded, so it is only for roles that arrive as often as they are waited for whatever happens, bounded waits of theirs
+// that expire included.  The parity is not needed: nobody may arrive again before the waiting warps have gone on.
+struct NamedBar { uint32_t id, threads; };
+__device__ __forceinline__ void mbar_arrive(NamedBar b) { asm volatile("bar.arrive %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory"); }
+__device__ __forceinline__ void mbar_wait_warp(NamedBar b, uint32_t, volatile uint32_t*) { asm volatile("bar.sync %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory"); }
 
 // One lane of a converged warp; the enclosing control flow stays warp-uniform, which lets the compiler keep
 // descriptors in uniform registers for the MMA issue.
@@ -138,7 +145,14 @@ __device__ __forceinline__ void bulk_store(void* dst, const void* src, uint32_t 
                "r"(smem_u32(src)), "r"(bytes)
                : "memory");
 }
+// tiled copy shared -> global, tracked the same way; what lies outside the tensor is not written
+__device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* src, int x, int y, int z, int w) {
+  asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%2, %3, %4, %5}], [%1];" ::"l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(src)),
+               "r"(x), "r"(y), "r"(z), "r"(w)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 
@@ -189,6 +203,11 @@ __device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo
   d |= (uint64_t)1 << 46;  // descriptor version of this architecture
   return d;
 }
+// The two words of such a descriptor for a tile that lies `off` bytes behind one whose address / 16 is known: the low word is that plus
+// desc_lo, the high word is desc_hi, both constants.  (An address put together, shifted and masked for every MMA costs more than a small MMA.)
+__host__ __device__ constexpr uint32_t desc_lo(int off, int lbo_bytes) { return (uint32_t)(off >> 4) | (uint32_t)(lbo_bytes >> 4) << 16; }
+__host__ __device__ constexpr uint32_t desc_hi(int sbo_bytes, bool swizzled) { return (uint32_t)(sbo_bytes >> 4) | 1u << 14 | (swizzled ? 2u << 29 : 0u); }
+__device__ __forceinline__ uint64_t smem_desc(uint32_t lo, uint32_t hi) { return (uint64_t)hi << 32 | lo; }
 // 32-bit instruction descriptor for kind::f16 with fp32 accumulate.  fmt: 0 = f16, 1 = bf16.
 __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int a_fmt, int b_fmt, bool a_mn_major, bool b_mn_major,
                                                  bool a_neg = false, bool b_neg = false) {
@@ -246,6 +265,26 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
 // 16 lanes x 8 columns in the accumulator layout of the warp-level m16n8 MMAs
 __device__ __forceinline__ void tmem_ld_frag(uint32_t taddr, float (&r)[4]) {
   asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0,%1,%2,%3}, [%4];" : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]) : "r"(taddr) : "memory");
+}
+// the same for eight and four adjacent groups of 8 columns, four registers a group
+__device__ __forceinline__ void tmem_ld_frags(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
+        "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld_frags(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
