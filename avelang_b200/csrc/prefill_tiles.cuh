@@ -132,7 +132,7 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
                    int n_chunks, int compact_grid) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = tc::align1024(smem_raw);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // (uniform to the compiler)
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TL_BARS);
   uint64_t* desc_full = bars;      // [2] the unit's description is in shared memory
   uint64_t* vec_full = bars + 2;   // [2] its token factors are
@@ -272,13 +272,13 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
       float kn[2] = {1.f, 1.f}, qn[2] = {1.f, 1.f};
       if (l2norm) {
         if (!tc::mbar_wait_warp(tile_full, (uint32_t)k & 1u, abort_flag)) break;
-#pragma unroll
+#pragma unroll 1
         for (int e = 0; e < 2; ++e) {
           const int i = lane + 32 * e;
           const uint8_t* k_row = smem + TL_TILE + (i >> 3) * 2048 + (i & 7) * 128;
           const uint8_t* q_row = smem + TL_TILE + ((i >> 3) ^ 6) * 2048 + 1024 + (i & 7) * 128;
           float2 sk = make_float2(0.f, 0.f), sq = sk;
-#pragma unroll 4
+#pragma unroll 2
           for (int p = 0; p < 16; ++p) {  // the swizzle permutes pieces inside a row, a sum needs no decode
             const int at = (p >> 3) * TL_HALF + (((p + lane) & 7) << 4);
             const uint4 kr = *reinterpret_cast<const uint4*>(k_row + at), qr = *reinterpret_cast<const uint4*>(q_row + at);
@@ -289,13 +289,14 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
               sk = __ffma2_rn(kf, kf, sk); sq = __ffma2_rn(qf, qf, sq);
             }
           }
-          kn[e] = rsqrtf(sk.x + sk.y + 1e-6f); qn[e] = rsqrtf(sq.x + sq.y + 1e-6f);
+          const float rk = rsqrtf(sk.x + sk.y + 1e-6f), rq = rsqrtf(sq.x + sq.y + 1e-6f);
+          if (e == 0) { kn[0] = rk; qn[0] = rq; } else { kn[1] = rk; qn[1] = rq; }
         }
         tc::mbar_arrive(norm_done);
       }
-#pragma unroll
+#pragma unroll 1
       for (int hh = 0; hh < 2; ++hh) {
-        const float v0 = g[hh][0], v1 = g[hh][1];
+        const float v0 = hh ? g[1][0] : g[0][0], v1 = hh ? g[1][1] : g[0][1], be0 = hh ? be[1][0] : be[0][0], be1 = hh ? be[1][1] : be[0][1];
         const float bs1 = __shfl_sync(0xffffffffu, v0, 16), bs2 = __shfl_sync(0xffffffffu, v1, 0), bs3 = __shfl_sync(0xffffffffu, v1, 16);
         const float bC = __shfl_sync(0xffffffffu, v1, 31);
         float* vec = reinterpret_cast<float*>(smem + TL_VEC) + (2 * buf + hh) * TV_FLOATS;
@@ -304,7 +305,7 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int i = lane + 32 * e;
-          const float x = g[hh][e], beta = be[hh][e], q = i < len ? qn[e] * a.scale : 0.f, bk = beta * kn[e];
+          const float x = e ? v1 : v0, beta = e ? be1 : be0, q = i < len ? qn[e] * a.scale : 0.f, bk = beta * kn[e];
           const float u0 = ex2_approx((x - __shfl_sync(0xffffffffu, x, lane & 16)) * LOG2E);
           vec[TV_B * C + i] = x; vec[TV_BETA * C + i] = beta;
           vec[TV_RA * C + i] = -bk * u0; vec[TV_RP * C + i] = q * u0;
