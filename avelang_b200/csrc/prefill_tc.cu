@@ -301,61 +301,65 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
 // the streaming norm kernel: a half-warp per token row, 8 adjacent features per lane, 16- and 32-byte accesses, the
 // RMS over d_v as four shuffles.  (Reading o_local and z straight from the accumulator's layout, a row or a column per
 // thread, measured three to four times slower: 2- or 4-byte accesses and tens of instructions per element.)
-// A CTA serves one (sequence, part, head) and walks every `gridDim.x`-th chunk with the M0 image resident.  Bound by memory traffic
-// (96 KB a chunk with a gate) and by the serial steps of a chunk, which two CTAs per SM overlap: 8192
-// tokens x 32 heads 51 us (55 with pairs of chunks, one CTA an SM), 5 TB/s while it streams; a whole call 323 -> 318.
-constexpr int FIN_THREADS = 256;
-constexpr int FIN_Q = 0, FIN_M0 = QT_BYTES, FIN_BARS = FIN_M0 + PACK_BYTES;
+// A CTA serves one (sequence, part, head) with the M0 image resident.  Its two groups of eight warps walk the chunks independently, the last ones
+// first: what the scan wrote last is still in L2.  A group has images, staged rows, accumulator and barriers of its own, and asks for the next chunk's images as
+// soon as its product has read these, so that they arrive under the staging and the norm.  Bound by memory traffic (96 KB a chunk with a gate) and
+// by the serial steps of a chunk, which the groups overlap.  A whole call, 8192 tokens x 32 heads / 32768 x 4 heads: two CTAs an SM of one group each, whose
+// images were in the place of the staged rows, 259.9 / 185.0 us, the last chunks first 258.6 / 183.5, two groups 253.6 / 171.8 (256.8 / 179.0 with
+// the next chunk's rows prefetched into L2 as well).
+constexpr int FIN_GROUP = 256, FIN_THREADS = 2 * FIN_GROUP;
+constexpr int FIN_M0 = 0, FIN_Q = PACK_BYTES, FIN_ST = QT_BYTES, FIN_GROUP_BYTES = QT_BYTES + C * D * 4, FIN_BARS = FIN_Q + 2 * FIN_GROUP_BYTES;
 constexpr size_t FIN_SMEM = FIN_BARS + 64 + 1024;
-static_assert(C * D * 4 <= QT_BYTES, "the rows are staged in the place of the qt images");
-__global__ void __launch_bounds__(FIN_THREADS, 2)
+__global__ void __launch_bounds__(FIN_THREADS, 1)
 part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* o_f32,
                    const uint8_t* qt_img, const uint8_t* m0_pack, const __grid_constant__ ScanPlan plan) {
   extern __shared__ uint8_t smem_raw[];
   pdl_wait();
   uint8_t* smem = tc::align1024(smem_raw);
-  float* stage = reinterpret_cast<float*>(smem + FIN_Q);  // [64 tokens][128] product rows, neighbouring 16-byte pieces swapped by token
+  const int grp = __shfl_sync(0xffffffffu, (int)(threadIdx.x / FIN_GROUP), 0);
+  uint8_t* mine = smem + FIN_Q + grp * FIN_GROUP_BYTES;
+  float* stage = reinterpret_cast<float*>(mine + FIN_ST);  // [64 tokens][128] product rows, neighbouring 16-byte pieces swapped by token
   auto piece16 = [&](int t, int p) { return stage + t * D + 4 * (p ^ (((p >> 3) ^ t) & 1)); };
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + FIN_BARS);
   uint64_t* m0_full = bars;
-  uint64_t* q_full = bars + 1;
-  uint64_t* mma_bar = bars + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 3);
+  uint64_t* q_full = bars + 1 + grp;
+  uint64_t* mma_bar = bars + 3 + grp;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 5);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  const int h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.y, tid = threadIdx.x % FIN_GROUP, warp = tid >> 5, lane = tid & 31;  // within the group
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(FIN_GROUP) : "memory"); };
   const int n = blockIdx.z / (plan.parts - 1), part = 1 + blockIdx.z % (plan.parts - 1);
   if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
   if (!sp.ok || (a.cu_seqlens != nullptr && a.max_seqlen > 0 && sp.len > a.max_seqlen)) return;
   const int seq_chunks = (sp.len + C - 1) / C;
-  const int c_end = min(plan.part_begin[part + 1], seq_chunks), c_begin = plan.part_begin[part] + (int)blockIdx.x, stride = gridDim.x;
-  if (c_begin >= c_end) return;
+  const int c_end = min(plan.part_begin[part + 1], seq_chunks), c_begin = plan.part_begin[part] + 2 * (int)blockIdx.x + grp, stride = 2 * gridDim.x;
+  if (c_begin - grp >= c_end) return;
+  auto from_end = [&](int i) { return plan.part_begin[part] + c_end - 1 - i; };
   const int slot = a.state_indices ? a.state_indices[n] : n;
   const bool skipped = slot < 0 || slot >= a.num_slots;  // the scan skipped the sequence: its rows are zero
   const int64_t rec0 = first_record(a, chunk_start, n);  // record of the sequence's chunk 0
 
   auto load_qt = [&](int c) {  // called by one thread
     tc::mbar_expect_tx(q_full, QT_BYTES);
-    tc::bulk_load(smem + FIN_Q, qt_img + ((rec0 + c) * a.Hv + h) * (int64_t)QT_BYTES, QT_BYTES, q_full);
+    tc::bulk_load(mine, qt_img + ((rec0 + c) * a.Hv + h) * (int64_t)QT_BYTES, QT_BYTES, q_full);
   };
-  if (tid == 0) {
-    tc::mbar_init(m0_full, 1);
-    tc::mbar_init(q_full, 1);
-    tc::mbar_init(mma_bar, 1);
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 5; ++i) tc::mbar_init(bars + i, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
     if (!skipped) {
       const uint8_t* img = m0_pack + (((int64_t)n * (plan.parts - 1) + (part - 1)) * a.Hv + h) * (int64_t)PACK_BYTES;
       tc::mbar_expect_tx(m0_full, PACK_BYTES);
       tc::bulk_load(smem + FIN_M0, img, PACK_BYTES, m0_full);
-      load_qt(c_begin);
     }
   }
-  if (warp == 1) tc::tmem_alloc(tmem_slot, 64);
+  if (grp == 0 && warp == 1) tc::tmem_alloc(tmem_slot, 128);
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
-  const uint32_t tm = *tmem_slot;
+  if (tid == 0 && !skipped && c_begin < c_end) load_qt(from_end(c_begin));
+  const uint32_t tm = *tmem_slot + 64 * grp;
   const int hw = tid >> 4, sub = tid & 15;  // streaming pass: half-warp index (16 of them) and lane inside it
   const bool gate_first = (a.flags & AVE_GDN_FLAG_GATE_FIRST) != 0;
   float2 wv[4];
@@ -365,7 +369,8 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   bool ok = true;
 
   int it = 0;
-  for (int c = c_begin; c < c_end && ok; c += stride, ++it) {
+  for (int i = c_begin; i < c_end; i += stride, ++it) {
+    const int c = from_end(i);
     const int64_t tok0 = sp.t0 + (int64_t)c * C;
     const int rows = min(C, sp.len - c * C);
     // the rows this half-warp will stream (hw, hw + 16, hw + 32, hw + 48) are fetched before the product is waited for
@@ -392,7 +397,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
         tc::tc_fence_after_sync();
         if (landed && tc::elect_one()) {
           constexpr uint32_t idesc = tc::idesc_f16(128, 64, 1, 1, false, true);  // A K-major, B MN-major (token rows)
-          const uint32_t sq = tc::smem_u32(smem + FIN_Q), sm = tc::smem_u32(smem + FIN_M0);
+          const uint32_t sq = tc::smem_u32(mine), sm = tc::smem_u32(smem + FIN_M0);
 #pragma unroll 1
           for (int t = 0; t < 3; ++t) {  // hi hi, hi lo, lo hi
             const uint32_t qb = sq + (t == 1 ? QT_BYTES / 2 : 0), mb = sm + (t == 2 ? PACK_BYTES / 2 : 0);
@@ -405,8 +410,9 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
         }
         __syncwarp();
       }
-      ok = tc::mbar_wait(mma_bar, (uint32_t)it & 1u, abort_flag);
+      ok = tc::mbar_wait(mma_bar, (uint32_t)it & 1u, abort_flag) && ok;
       tc::tc_fence_after_sync();
+      if (tid == 0 && i + stride < c_end) load_qt(c - stride);  // the product has read the images
       if (ok) {  // accumulator (a d_v row per thread, 32 tokens) -> staged token rows
         const int d = (warp & 3) * 32 + lane, first = 32 * (warp >> 2);
         uint32_t acc[32];
@@ -417,7 +423,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
       }
     }
     tc::tc_fence_before_sync();
-    ok = __syncthreads_and(ok ? 1 : 0) != 0;  // staged rows complete; the accumulator is free for the next product
+    group_sync();  // staged rows complete; the accumulator is free for the next product
     tc::tc_fence_after_sync();
     if (ok) {
 #pragma unroll
@@ -459,16 +465,14 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
                                     (int64_t)h * a.o_stride_h + 8 * sub) = make_uint4(packed[0], packed[1], packed[2], packed[3]);
       }
     }
-    tc::fence_proxy_async_smem();
-    __syncthreads();  // the staged rows have been read: the next chunk's images may take their place
-    if (ok && tid == 0 && !skipped && c + stride < c_end) load_qt(c + stride);
+    group_sync();  // the staged rows have been read
   }
   tc::tc_fence_before_sync();
   __syncthreads();
-  if (*abort_flag != 0u && tid == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
-  if (warp == 1) {
+  if (*abort_flag != 0u && threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+  if (grp == 0 && warp == 1) {
     tc::tc_fence_after_sync();
-    tc::tmem_dealloc(tm, 64);
+    tc::tmem_dealloc(tm, 128);
   }
 }
 
@@ -763,8 +767,8 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
       int part_len = 0;  // the longest of the later parts
       for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
       const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
-      int split = (int)(2 * NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head): about one wave of two an SM
-      split = max(1, min(split, part_len));
+      int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));
+      split = max(1, min(split, (part_len + 1) / 2));
       step(launch_after(part_finish_kernel, dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream,
                         a, chunk_start, o_f32, qt_img, m0_pack, plan));
     };
