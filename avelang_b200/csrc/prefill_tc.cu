@@ -503,34 +503,43 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   L.max_chunks = max_chunks;
   const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
   const bool push = a.o_peers != nullptr && a.n_peers > 1;
-  // Parts: with few long chains most SMs idle while every chain walks its chunks one after the other.  Cutting the
-  // sequences into S parts that run at the same time shortens the walk S-fold at the price of a second (transition)
-  // chain per later part and one GEMM-shaped fix-up; S is the largest count whose 2S-1 chains per head still get an SM
-  // each, up to 16.  Not with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of
-  // beside it.
-  // As measured (one sequence, gated, us by the number of parts): the largest count is the best or within 3 % of it from 6144 tokens on (4 heads x
-  // 32768 8: 280, 12: 240, 16: 212; 16 x 8192 3: 216, 4: 195, 5: 189; 24 x 8192 2: 289, 3: 247, 4: 320); with many heads and 2048 tokens two would do
-  // better (20 heads 2: 86, 4: 94; 28 heads 2: 95, 3: 109).
+  // Parts: with few chains most SMs idle while every chain walks its chunks one after the other.  Cutting the sequences into S parts that run at
+  // the same time shortens the walk S-fold at the price of a second (transition) chain per later part, a combine and one GEMM-shaped fix-up.  Not
+  // with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of beside it.
+  // Part 0 runs one chain and needs no fix-up, a later part runs two chains and its rows wait for the fix-up, so part 0 is made PART0_X4 / 4
+  // times as long as the others; lengths are even.
+  auto length = [&](int S) { return max(2, (4 * max_chunks / (4 * (S - 1) + PART0_X4) + 1) & ~1); };
+  auto first_length = [&](int S) { return S > 1 ? max(2, (max_chunks - (S - 1) * length(S) + 1) & ~1) : 0; };
+  // What a call with S parts takes beside what it takes anyway, in ns: its longest chain's steps, which get longer with the SMs that hold chains, their
+  // start, the fix-up, and what goes with any.  Fitted to 1156 measurements (4 to 96 chains of 8 to 256 chunks, whole and in 2 to 16 parts, with a gate and
+  // without; 3.4 % off on the mean, as good with either).
+  auto cost = [&](int S) {
+    const int64_t chains = heads_total * (2 * S - 1), steps = S > 1 ? max(length(S), first_length(S)) : max_chunks;
+    return steps * (1870 + 34 * chains / 10) + 122 * chains + (S == 1 ? 0 : S == 2 ? 10500 : 13000 + 460 * (S - 1)) +
+           (S > 1 ? 147 * heads_total * max(0, max_chunks - first_length(S)) / 10 : 0) + 10100 + 3 * heads_total * max_chunks;
+  };
   L.parts = 1;
-  if (!plain && !push && max_chunks >= 32) {
-    const int64_t per_head = (NUM_SMS / (heads_total > 0 ? heads_total : 1) + 1) / 2;  // chains per head that still get an SM each: 2S - 1
-    int S = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
-    while (S > 1 && max_chunks / S < 8) --S;  // a part of fewer chunks costs more in combine and fix-up than it saves
-    // Two parts take three chains a head.  They are taken while these leave a third of the SMs and the chains are long enough for the
-    // fix-up, which with a gate also holds the later part's norms back.  Both lines are those of slower forms of pass 1, the combine and the fix-up, and
-    // still on the safe side: two parts win at them and would win beyond (32 heads gated, whole / two: 2048 tokens 116 / 101 us, 6144 321 / 247, 8192 419 / 315;
-    // without a gate 2048 102 / 91, 4096 191 / 154; 34 heads x 8192 gated 427 / 325, 40 heads x 32768 1692 / 1271).
-    const bool two = S == 2 && 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64);
-    L.parts = S >= 3 || two ? S : 1;
+  if (!plain && !push && heads_total > 0 && max_chunks >= 12) {
+    const int64_t per_head = (NUM_SMS / heads_total + 1) / 2;  // chains per head that still get an SM each: 2S - 1
+    int most = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
+    while (most > 1 && max_chunks / most < 2) --most;
+    int S = most;
+    for (int i = most - 1; i >= 3; --i) if (cost(i) < cost(S)) S = i;
+    if (max_chunks < 32) {  // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
+      if (most >= 2 && cost(2) < cost(S)) S = 2;
+      L.parts = S >= 2 && heads_total <= 16 && 20 * cost(S) < 19 * cost(1) ? S : 1;
+    } else if (S >= 3) {  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
+      L.parts = 20 * cost(2) < 19 * cost(S) ? 2 : S;
+    } else if (S == 2) {
+      // Two parts take three chains a head.  They are taken while these leave a third of the SMs and the chains are long enough for the
+      // fix-up, which with a gate also holds the later part's norms back.  Both lines are those of slower forms of pass 1, the combine and the fix-up, and
+      // on the safe side: two parts win at them and would win beyond (32 heads gated, whole / two: 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199;
+      // without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
+      L.parts = 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64) ? 2 : 1;
+    }
   }
   L.part_begin[0] = 0;
-  {
-    // Part 0 runs one chain and needs no fix-up, a later part runs two chains and its rows wait for the fix-up, so
-    // part 0 is made PART0_X4 / 4 times as long as the others; lengths are even.
-    const int len = max(2, (4 * max_chunks / (4 * (L.parts - 1) + PART0_X4) + 1) & ~1);
-    const int first = L.parts > 1 ? max(2, (max_chunks - (L.parts - 1) * len + 1) & ~1) : 0;
-    for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < L.parts ? first + (p - 1) * len : (1 << 24);
-  }
+  for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < L.parts ? first_length(L.parts) + (p - 1) * length(L.parts) : (1 << 24);
   // Ranges: with the fused all-gather a launch of its own norms the rows and pushes them to every peer over NVLink, which takes about
   // as long as a chain itself; with few long chains that runs beside the chains of the next range, and only the last range's push is
   // exposed, so the ranges are equal and as many as the event pool allows.  (Without peers ranges do not pay any more: pass 1 of

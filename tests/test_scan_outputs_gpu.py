@@ -52,3 +52,17 @@ def test_rows_of_parts_behind_a_sequence_stay(gdn, checker, lens):
     check_o(O, out, o_ref)
     check_s(O, s, s_ref)
     assert bool((whole[:, T:] == 7.0).all()) and bool((whole[:, :, 4:] == 7.0).all())
+
+
+@pytest.mark.parametrize("B,T,Hv", [(1, 1024, 4), (1, 1529, 16), (2, 1990, 8), (1, 2048, 24), (1, 6144, 8)])  # four, two, four, two and eight parts
+@pytest.mark.parametrize("gated", [False, True])
+def test_short_chains_in_parts(gdn, checker, B, T, Hv, gated):
+    O, C = checker
+    inp = synth.make_inputs(B, T, Hv // 2, Hv, 128, 128, seed=T, with_z=gated, n_states=B, gate_scale=0.02)
+    g = dev(inp)
+    o, s = gdn.chunk_gated_delta_rule(g.q, g.k, g.v, g.g, g.beta, initial_state=g.initial_state, output_final_state=True, z=g.z if gated else None)
+    o_ref, s_ref = C.recurrent(inp.q, inp.k, inp.v, inp.g, inp.beta, inp.scale, inp.initial_state)
+    if gated:
+        o_ref = O.gated_rmsnorm(o_ref, inp.z)
+    check_o(O, o, o_ref)
+    check_s(O, s, s_ref)
