@@ -433,7 +433,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
       tc::tc_fence_after_sync();
       {  // X_j = kx_j H k_j
-#pragma unroll 1
+#pragma unroll
         for (int k = 0; k < VC / 16; ++k) {
           uint32_t acc[16], xh[8], xl[8];
           tc::tmem_ld16(lane_addr + TC_X + VC * grp + 16 * k, acc);
@@ -555,27 +555,39 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       if (!tc::mbar_wait_warp(o_full, cp, abort_flag)) break;
       tc::tc_fence_after_sync();
       const bool whole = !(ragged && c == n_chunks - 1);  // (behind the end of a dense batch row the copies write nothing)
+      // O1 is taken whole and released at once: O1 of the next chunk is the first thing the tensor pipe runs while the chain epilogue converts X, and X's
+      // product must not wait for it.  o[4 g + 2 rr + e]: feature 32 wq + 16 hf + 8 rr + gr, token 8 g + t2 + e.
+      uint32_t o[32], o_next[32];
+      tc::tmem_ld_frags(lane_addr + TC_O1, o);
+      tc::tmem_ld_frags(lane_addr + (16u << 16) + TC_O1, o_next);
+      tc::tmem_ld_wait();
+      tc::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(o1_empty);
       // 16 features at a time, in a loop that stays rolled: the code of all roles together has to stay small
 #pragma unroll 1
       for (int hf = 0; hf < 2; ++hf) {
-        uint32_t o[32], o2[32];  // [4 g + 2 rr + e]: feature 32 wq + 16 hf + 8 rr + gr, token 8 g + t2 + e
-        tc::tmem_ld_frags(lane_addr + ((uint32_t)hf << 20) + TC_O1, o);
-        tc::tmem_ld_frags(lane_addr + ((uint32_t)hf << 20) + TC_O2, o2);
-        tc::tmem_ld_wait();
-        if (hf == 1) {
-          tc::tc_fence_before_sync();
-          __syncwarp();
-          if (lane == 0) { tc::mbar_arrive(o1_empty); tc::mbar_arrive(o2_empty); }
-        }
         auto pair = [&](int g, int rr) { return make_float2(__uint_as_float(o[4 * g + 2 * rr]), __uint_as_float(o[4 * g + 2 * rr + 1])); };
 #pragma unroll
-        for (int g = 0; g < C / 8; ++g) {
-          const float2 qs = *reinterpret_cast<const float2*>(scal + 8 * g + t2);
+        for (int g0 = 0; g0 < C / 8; g0 += 4) {
+          uint32_t o2[16];
+          tc::tmem_ld_frags(lane_addr + ((uint32_t)hf << 20) + TC_O2 + 8 * g0, o2);
+          tc::tmem_ld_wait();
+          if (g0 == 4 && hf == 1) {
+            tc::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(o2_empty);
+          }
 #pragma unroll
-          for (int rr = 0; rr < 2; ++rr) {
-            uint32_t* x = &o[4 * g + 2 * rr];
-            const float2 y = __ffma2_rn(qs, pair(g, rr), make_float2(__uint_as_float(o2[4 * g + 2 * rr]), __uint_as_float(o2[4 * g + 2 * rr + 1])));
-            x[0] = __float_as_uint(y.x); x[1] = __float_as_uint(y.y);
+          for (int g = g0; g < g0 + 4; ++g) {
+            const float2 qs = *reinterpret_cast<const float2*>(scal + 8 * g + t2);
+#pragma unroll
+            for (int rr = 0; rr < 2; ++rr) {
+              uint32_t* x = &o[4 * g + 2 * rr];
+              const uint32_t* x2 = &o2[4 * (g - g0) + 2 * rr];
+              const float2 y = __ffma2_rn(qs, pair(g, rr), make_float2(__uint_as_float(x2[0]), __uint_as_float(x2[1])));
+              x[0] = __float_as_uint(y.x); x[1] = __float_as_uint(y.y);
+            }
           }
         }
         if (kMulti && phi) {
@@ -611,6 +623,8 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
             stsm4t(at + 512 * g, x[0], x[1], x[2], x[3]);
           }
         }
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = o_next[i];
       }
       tc::fence_proxy_async_smem();
       __syncwarp();
