@@ -6,9 +6,13 @@
 //   -> gated RMSNorm with z
 // so that a decode layer is two launches (the projection GEMM and this kernel) instead of five.  The state streaming
 // is that of the slot-pool decode kernel: persistent CTAs, the next 64 KiB tile lands in shared memory through a bulk
-// copy while the current one is reduced, updated and streamed out of registers.  A CTA takes a (sequence, key head) at
-// a time and walks the value heads that share it back to back: q and k are convolved and their history shifted once,
-// by the one CTA that reads them, which is what makes the in-place history update free of races.
+// copy while the current one is reduced, updated and streamed out of registers.  A unit is a (sequence, key head); a CTA walks the value
+// heads that share it back to back: q and k are convolved and their history shifted once, by the one CTA that reads them, which is what
+// makes the in-place history update free of races.  CTAs come in clusters of two, which take units in turn; where a cluster's number of units is
+// odd, the two share the last one, half of its value heads each: both read the q and k history, and one shifts it behind a cluster
+// barrier.  The busiest CTA then has 7 tiles where 64 sequences x 16 key heads left it 8 of 6.9 on the mean, and one sequence is twice as many CTAs.
+// A layer with both projections, 32 value heads: 64 sequences 85.0 -> 82.4 us, 1: 32.2 -> 30.4, 9: 37.0 -> 34.5, 20: 51.5 -> 48.2, 100: 116.3 ->
+// 113.4; where the units come out even nothing changes (37: 58.6 and 58.8, 256: 230).
 // Rounding points are those of the separate kernels (convolution outputs are rounded to bf16, g and beta stay fp32), so
 // the fused step leaves the states and histories that conv1d_update + gate_beta + decode_step leave, bit for bit.
 #include "common.cuh"
@@ -47,9 +51,14 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
     tc::fence_barrier_init();
   }
   pdl_wait();
-  if ((int)blockIdx.x >= n_units) return;
-  const int n_local = ((n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x) * r;  // tiles this CTA walks
-  auto unit_of = [&](int i) { return (int)blockIdx.x + (i / r) * (int)gridDim.x; };
+  // this cluster's units: cluster, cluster + clusters, ...; CTA `rank` takes every second of them, and its part of the last of an odd number
+  const int clusters = gridDim.x >> 1, cluster = blockIdx.x >> 1, rank = blockIdx.x & 1;
+  const int n_mine = (n_units - cluster + clusters - 1) / clusters, own = (n_mine >> 1) * r, half = (r + 1) >> 1;  // (own: tiles of whole units)
+  const bool shared = (n_mine & 1) != 0 && r > 1;  // the last unit is walked by both
+  const int n_local = own + ((n_mine & 1) == 0 ? 0 : r == 1 ? (rank == 0 ? 1 : 0) : rank == 0 ? half : r - half);
+  if (n_local == 0) return;
+  auto unit_of = [&](int i) { return cluster + (i < own ? 2 * (i / r) + rank : n_mine - 1) * clusters; };
+  auto head_of = [&](int i) { return i < own ? i % r : i - own + rank * half; };  // among the value heads of the unit
   auto slot_of_seq = [&](int n) -> int {  // < 0: the sequence is skipped
     int slot = a.state_indices ? a.state_indices[n] : n;
     if (slot >= a.num_slots) {
@@ -61,7 +70,7 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
   auto tile_ptr = [&](int slot, int h) { return a.state_pool + ((int64_t)slot * a.Hv + h) * (int64_t)(DK * DV); };
   // one channel of the convolution for sequence n: history of slot `slot` plus the new input; the history is shifted
   // in place by this (the only) thread that reads the channel.  Same arithmetic order as the standalone update kernel.
-  auto conv_channel = [&](int n, int slot, int ch) -> float {
+  auto conv_channel = [&](int n, int slot, int ch, bool both) -> float {  // both: the other CTA of the cluster reads the channel as well, and rank 0 shifts
     __nv_bfloat16* st = cstate + (int64_t)slot * (WIDTH - 1) * Cn + ch;
     __nv_bfloat16 x[WIDTH];
 #pragma unroll
@@ -70,8 +79,11 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
     float acc = cb ? bf2f(cb[ch]) : 0.f;
 #pragma unroll
     for (int j = 0; j < WIDTH; ++j) acc = fmaf(bf2f(cw[(int64_t)ch * WIDTH + j]), bf2f(x[j]), acc);
+    if (both) tc::cluster_sync();
+    if (!both || rank == 0) {
 #pragma unroll
-    for (int j = 0; j < WIDTH - 1; ++j) st[(int64_t)j * Cn] = x[j + 1];
+      for (int j = 0; j < WIDTH - 1; ++j) st[(int64_t)j * Cn] = x[j + 1];
+    }
     return bf2f(__float2bfloat16(silu(acc)));  // the separate kernels store the convolution output as bf16
   };
 
@@ -79,27 +91,28 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
   if (tid == 0) {
     if (slot >= 0) {
       tc::mbar_expect_tx(&full_bar, DK * DV * 4);
-      tc::bulk_load(tile_s, tile_ptr(slot, (unit_of(0) % a.Hk) * r), DK * DV * 4, &full_bar);
+      tc::bulk_load(tile_s, tile_ptr(slot, (unit_of(0) % a.Hk) * r + head_of(0)), DK * DV * 4, &full_bar);
     }
   }
   __syncthreads();
   uint32_t phase = 0;
 
   for (int i = 0; i < n_local; ++i) {
-    const int u = unit_of(i), n = u / a.Hk, hk = u % a.Hk, j = i % r, h = hk * r + j;
+    const int u = unit_of(i), n = u / a.Hk, hk = u % a.Hk, j = head_of(i), h = hk * r + j;
+    const bool first = i < own ? j == 0 : i == own;  // of this unit's tiles here
     int slot_next = -1, h_next = 0;
     if (i + 1 < n_local) {
       const int u2 = unit_of(i + 1);
       slot_next = (u2 == u) ? slot : slot_of_seq(u2 / a.Hk);
-      h_next = (u2 % a.Hk) * r + (i + 1) % r;
+      h_next = (u2 % a.Hk) * r + head_of(i + 1);
     }
     __nv_bfloat16* o_ptr = reinterpret_cast<__nv_bfloat16*>(a.o) + (int64_t)n * a.o_stride + h * DV;
 
     // this token's small inputs, computed while the tile is still landing
     float kq_elem = 0.f, v_elem = 0.f, g = 0.f, beta = 0.f;
     if (slot >= 0) {
-      if (j == 0) kq_elem = conv_channel(n, slot, tid < DK ? off_k + hk * DK + tid : hk * DK + (tid - DK));
-      if (tid < DV) v_elem = conv_channel(n, slot, off_v + h * DV + tid);
+      if (first) kq_elem = conv_channel(n, slot, tid < DK ? off_k + hk * DK + tid : hk * DK + (tid - DK), shared && i >= own);
+      if (tid < DV) v_elem = conv_channel(n, slot, off_v + h * DV + tid, false);
       const float av = bf2f(proj[(int64_t)n * a.proj_stride + off_a + h]) + a.dt_bias[h];
       const float bv = bf2f(proj[(int64_t)n * a.proj_stride + off_b + h]);
       const float sp = av > 20.f ? av : log1pf(expf(av));  // softplus
@@ -129,7 +142,7 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
       slot = slot_next;
       continue;
     }
-    if (j == 0) {
+    if (first) {
       if (tid < DK) k_s[tid] = kq_elem;
       else q_s[tid - DK] = kq_elem;
     }
@@ -216,13 +229,17 @@ int launch_decode_layer(const AveGdnDecodeLayerArgs& a, cudaStream_t stream) {
     attr_set_dev[dev] = true;  // repeating the three calls from another thread is harmless
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned grid = (unsigned)(units < 2 * sms ? units : 2 * sms);
-  switch (a.width) {
-    case 2: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<2>, grid, 256, DK * DV * 4, stream, a, units)); break;
-    case 3: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<3>, grid, 256, DK * DV * 4, stream, a, units)); break;
-    case 4: AVE_CUDA_TRY(launch_after(gdn_decode_layer_kernel<4>, grid, 256, DK * DV * 4, stream, a, units)); break;
-    default: return AVE_GDN_UNSUPPORTED;
-  }
+  if (a.width < 2 || a.width > 4) return AVE_GDN_UNSUPPORTED;
+  const auto kernel = a.width == 2 ? gdn_decode_layer_kernel<2> : a.width == 3 ? gdn_decode_layer_kernel<3> : gdn_decode_layer_kernel<4>;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)(2 * (units < sms ? units : sms))); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = DK * DV * 4; cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 2;
+  AVE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a, units));
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }
