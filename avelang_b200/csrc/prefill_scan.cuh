@@ -19,6 +19,7 @@
 //     that the products begin with one half while the other is converted, and an increment's first features are taken while the rest is formed;
 //   - arrivals that the chain waits for are hardware barriers (30 cycles, an mbarrier 85 to 250);
 //   - outputs leave by asynchronous copies: the transition chains' steps were a fifth longer when 32 lines were written an instruction.
+// Later: O1 taken whole before the rows are formed (drained 1.0 to 1.25 k cycles into a step it held X's product back): 253.5 -> 249.3 us.
 // The conversions are bound by the instructions of a scheduler (a pair of values into two bf16 terms takes 7 cycles of it).
 // O2 waits for the increment: side by side they shared the pipe and the increment came 200 cycles later; H K^T in the increment's columns and not
 // in O2's lets O2 end beside the next step.  Measured and dropped: the state a chunk behind the chain by

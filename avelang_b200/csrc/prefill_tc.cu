@@ -776,7 +776,7 @@ int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, cons
       int part_len = 0;  // the longest of the later parts
       for (int p = 1; p < L.parts; ++p) part_len = max(part_len, min(L.part_begin[p + 1], L.max_chunks) - L.part_begin[p]);
       const int64_t groups = (int64_t)a.n_seqs * (L.parts - 1) * a.Hv;
-      int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));
+      int split = (int)(NUM_SMS / (groups > 0 ? groups : 1));  // CTAs per (sequence, part, head), two chunks at a time each: about one wave
       split = max(1, min(split, (part_len + 1) / 2));
       step(launch_after(part_finish_kernel, dim3((unsigned)split, (unsigned)a.Hv, (unsigned)(a.n_seqs * (L.parts - 1))), FIN_THREADS, FIN_SMEM, stream,
                         a, chunk_start, o_f32, qt_img, m0_pack, plan));
