@@ -13,7 +13,7 @@
 // 0.7 k, the new state 0.7 k, each of them about a third hand-over (arrival or commit, wake-up, first load).  What it took to get there from 4.55 k
 // (8192 tokens x 32 heads 313 -> 260 us, 4 heads x 32768 212 -> 186, 262144 packed tokens 4.17 -> 3.75 ms, all with everything around the scan):
 //   - the code of all roles fits the 32 KB of the SM's instruction cache.  It was 44 KB (rolled waits, outputs in a rolled loop, descriptors from
-//     constants and roles that the compiler knows to be uniform took it down), every step fetched 150 lines of 128 bytes from the cache that the SMs of a GPC
+//     constants and roles that the compiler knows to be uniform took it down), every step fetched 116 lines of 128 bytes, 40 now, from the cache that the SMs of a GPC
 //     share, and chains ran up to a third slower where more of a GPC's SMs held one;
 //   - the two groups of epilogue warps hand over by halves: a group's tokens of X and Vd, and features of the state, have barriers of their own, so
 //     that the products begin with one half while the other is converted, and an increment's first features are taken while the rest is formed;
@@ -116,6 +116,19 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
 
   // (a shuffle, so that the compiler knows a role's code to be uniform: an MMA takes 6 instructions then, and 18 with descriptors in vector registers)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  // what reads nothing that a launch before wrote comes in front of the wait for it
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
+    for (int i = 0; i < NG; ++i) { tc::mbar_init(&vn_full[i], 1); tc::mbar_init(&dh_full[i], 1); }
+    tc::mbar_init(vn_ready, 4 * NG);
+    for (uint64_t* b : {kh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
+    tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
+    *abort_flag = 0;
+    tc::fence_barrier_init();
+  }
+  if (warp == 2 && lane == 0) {
+    tc::prefetch_tmap(&maps.q); tc::prefetch_tmap(&maps.k); tc::prefetch_tmap(&maps.v);
+  }
   pdl_wait();
   // One CTA per (sequence, chain, value head).  Chain 0 is part 0; chains 2p-1 and 2p are the local and the transition
   // chain of part p >= 1 (see ScanPlan).
@@ -188,15 +201,6 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   const int n_chunks = c_hi - c_lo;
   const int64_t carry_tile = (((int64_t)n * chains + chain) * a.Hv + h) * (int64_t)(D * D);
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
-    for (int i = 0; i < NG; ++i) { tc::mbar_init(&vn_full[i], 1); tc::mbar_init(&dh_full[i], 1); }
-    tc::mbar_init(vn_ready, 4 * NG);
-    for (uint64_t* b : {kh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
-    tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
-    *abort_flag = 0;
-    tc::fence_barrier_init();
-  }
   if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before_sync();
   __syncthreads();

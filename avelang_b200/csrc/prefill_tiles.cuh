@@ -145,8 +145,6 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
   volatile uint32_t* abort_flag = tmem_slot + 1;
   pdl_trigger();
-  pdl_wait();
-  if (batch_rejected(a, chunk_start, blockIdx.x == 0)) return;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&desc_full[i], 1); tc::mbar_init(&vec_full[i], 32); tc::mbar_init(&gram_full[i], 1); tc::mbar_init(&unit_done[i], 8);
@@ -156,6 +154,8 @@ chunk_tiles_kernel(const AveGdnArgs a, const int32_t* chunk_start, uint8_t* recs
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
+  pdl_wait();
+  if (batch_rejected(a, chunk_start, blockIdx.x == 0)) return;
   if (warp == 8) tc::tmem_alloc(tmem_slot, 128);
   tc::tc_fence_before_sync();
   __syncthreads();

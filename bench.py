@@ -779,7 +779,7 @@ def main():
             "clocks": clocks}
     achieved = flops / (ms * 1e-3) / 1e12
     line["roofline"] = {"bound": "tensor", "achieved": achieved, "peak": peaks["bf16_tflops"], "unit": "TFLOP/s",
-                        "frac": achieved / peaks["bf16_tflops"], "traffic": 381_561_600,
+                        "frac": achieved / peaks["bf16_tflops"], "traffic": 383_056_128,
                         "traffic_source": "profiles/prefill_config1_launch_list.md: DRAM bytes read + written by the "
                                           "chunk_scan launch of one step (the dominant kernel), ncu with its "
                                           "cache flush between kernels; algorithmic bytes of the step are in hbm_view",
