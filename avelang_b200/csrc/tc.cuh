@@ -193,17 +193,8 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t saddr, uint32_t lbo
   d |= (uint64_t)2 << 61;  // 128-byte swizzle
   return d;
 }
-// K-major operand without swizzle: 8x8 core matrices of 128 contiguous bytes (row after row), `lbo` bytes from one to the next
-// along K and `sbo` bytes along M or N.
-__device__ __forceinline__ uint64_t smem_desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr >> 4) & 0x3fffu);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3fffu) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3fffu) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version of this architecture
-  return d;
-}
-// The two words of such a descriptor for a tile that lies `off` bytes behind one whose address / 16 is known: the low word is that plus
+// The two words of such a descriptor, or of one without swizzle (K-major: 8x8 core matrices of 128 contiguous bytes, `lbo` bytes from one to the next along
+// K and `sbo` along M or N), for a tile that lies `off` bytes behind one whose address / 16 is known: the low word is that plus
 // desc_lo, the high word is desc_hi, both constants.  (An address put together, shifted and masked for every MMA costs more than a small MMA.)
 __host__ __device__ constexpr uint32_t desc_lo(int off, int lbo_bytes) { return (uint32_t)(off >> 4) | (uint32_t)(lbo_bytes >> 4) << 16; }
 __host__ __device__ constexpr uint32_t desc_hi(int sbo_bytes, bool swizzled) { return (uint32_t)(sbo_bytes >> 4) | 1u << 14 | (swizzled ? 2u << 29 : 0u); }
