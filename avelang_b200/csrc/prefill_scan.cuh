@@ -103,15 +103,22 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   uint64_t* o2_empty = bars + 14; // O2 accumulator drained
   uint64_t* o1_done = bars + 15;  // O1 complete: the bf16 image of H may be overwritten
   // From a chain-epilogue group to the chain's issuer: bf16 image of its features of the state, X hi+lo and Vd hi+lo of its tokens are in TMEM.  The chain
-  // waits for these, so they are hardware barriers; both roles take part chunk by chunk to the end, whatever became of their other waits.
-  auto h_ready = [](int g) { return tc::NamedBar{1u + g, 32 * (4 + 1)}; };
-  auto x_ready = [](int g) { return tc::NamedBar{1u + NG + g, 32 * (4 + 1)}; };
-  auto vd_ready = [](int g) { return tc::NamedBar{1u + 2 * NG + g, 32 * (4 + 1)}; };
+  // waits for these, so they are hardware barriers, and their waits have no limit of their own.  A warp that arrives does not wait, so it may only come
+  // back to a barrier when the issuer has gone through: its waits for what the issuer commits behind the barrier see to that as long as they end with the phase
+  // complete (`alive`, one answer for a warp).  After a wait that has expired a warp meets the issuer in every hand-over instead of passing it, and an issuer
+  // whose own wait has expired goes through the hand-overs that are left without a product or a commit: both sides take part 3 NG times a chunk.
+  constexpr int HAND_OVERS = 3 * NG;  // of a chunk, in the issuer's order
+  auto hand_over = [](int i) { return tc::NamedBar{1u + i, 32 * (4 + 1)}; };
+  auto h_ready = [&](int g) { return hand_over(g); };
+  auto x_ready = [&](int g) { return hand_over(NG + g); };
+  auto vd_ready = [&](int g) { return hand_over(2 * NG + g); };
+  auto all = [](bool done) { return __all_sync(0xffffffffu, done) != 0; };
   // A wait sees only the parity of a barrier's phase, so no barrier may complete twice before each of its waiters has seen the first
   // time.  Most are ordered by the arrivals they need.  dh_full is waited for by warp 2 as well, which no increment needs: so warp 1 issues an
   // increment only behind o_full of the chunk before, which warp 2 commits when it has seen dh_full of that chunk.
   uint64_t* tail_full = bars + 16;  // tiles and record of a ragged last chunk landed: warp 0 clears what lies behind the sequence, then completes `full`
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* mma_end = bars + 17;    // [2] the MMAs of warps 1 and 2 complete, when a wait has expired
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   // (a shuffle, so that the compiler knows a role's code to be uniform: an MMA takes 6 instructions then, and 18 with descriptors in vector registers)
@@ -119,7 +126,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   // what reads nothing that a launch before wrote comes in front of the wait for it
   if (threadIdx.x == 0) {
     for (int i = 0; i < CS_STAGES; ++i) { tc::mbar_init(&full[i], 1); tc::mbar_init(&empty[i], 6); }
-    for (int i = 0; i < NG; ++i) { tc::mbar_init(&vn_full[i], 1); tc::mbar_init(&dh_full[i], 1); }
+    for (int i = 0; i < NG; ++i) { tc::mbar_init(&vn_full[i], 1); tc::mbar_init(&dh_full[i], 1); tc::mbar_init(&mma_end[i], 1); }
     tc::mbar_init(vn_ready, 4 * NG);
     for (uint64_t* b : {kh_full, o_full, o1_done, tail_full}) tc::mbar_init(b, 1);
     tc::mbar_init(o1_empty, 4); tc::mbar_init(o2_empty, 4);
@@ -212,6 +219,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   tc::reg_set<REGS_CTRL, REGS_LAUNCH>();
   if (warp == 0) {
     // ------------------------------------------------------------------ loader: a stage is {Q, K, V, record}, three of them
+    int issued = 0;  // chunks asked for
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 1;  // parity of "chunk c - 3 is done with the stage"; the first round waits for nothing
@@ -230,6 +238,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
         }
         tc::tma_load_4d(st + CS_Q, &maps.q, when_full, 0, hk, tok, sp.b);
         tc::tma_load_4d(st + CS_Q + 8192, &maps.q, when_full, 64, hk, tok, sp.b);
+        ++issued;
         if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
         return true;
       };
@@ -244,7 +253,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     // 203 tokens: 29.4 us, 29.2 without; by warp 1 in front of U 29.9, and with the contractions over tokens cut at the last token instead, a
     // branch around each MMA, 30.1 (8192 tokens 318, 316, 318 and 326; by warp 3 320).
     __syncwarp();
-    if (ragged && tc::mbar_wait_warp(tail_full, 0u, abort_flag)) {
+    if (ragged && all(tc::mbar_wait_warp(tail_full, 0u, abort_flag))) {
       const int last = (n_chunks - 1) % CS_STAGES;
       uint4* st = reinterpret_cast<uint4*>(smem + last * CS_STAGE + CS_K);
       // 16-byte pieces of the halves (64 features) of K and of V; whole rows, so the swizzle does not matter.  (Not unrolled: the code
@@ -255,6 +264,13 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       tc::fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&full[last]);
+    }
+    if (lane == 0) {  // nothing is on its way into the shared memory of a CTA that ends, whatever became of those who wait for it
+#pragma unroll 1
+      for (int c = max(0, issued - CS_STAGES); c < issued; ++c) {
+        const bool tail = ragged && c == n_chunks - 1;
+        tc::drain(tail ? tail_full : &full[c % CS_STAGES], tail ? 0u : (uint32_t)(c / CS_STAGES) & 1u);
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ chain MMA issuer (whole warp runs the loop, one
@@ -282,10 +298,12 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     int s = 0, s_next = 1;
     uint32_t ph_next = 0;
     const uint32_t smem0 = tc::smem_u32(smem) >> 4;
-    tc::mbar_wait_warp(&full[0], 0u, abort_flag);
+    int met = HAND_OVERS * n_chunks;  // hand-overs behind which this role leaves its loop
+    const bool landed = all(tc::mbar_wait_warp(&full[0], 0u, abort_flag));
+    if (!landed) met = 0;
     tc::tc_fence_after_sync();
-    issue_u(smem0);
-    // What the chain waits for, step by step.  A bounded wait that expires raises the flag and this role goes on, with products that nobody will use.
+    if (landed) issue_u(smem0);
+    // what the chain waits for, step by step
     auto state_product = [&](int c, uint32_t at, int s) {
 #pragma unroll
       for (int g = 0; g < NG; ++g) {
@@ -317,7 +335,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       }
     };
     auto outputs_before = [&](int c) {  // warp 2 has seen dh_full of the chunk before (and O2 is long complete)
-      tc::mbar_wait_warp(o_full, (uint32_t)(c + 1) & 1u, abort_flag);
+      return all(tc::mbar_wait_warp(o_full, (uint32_t)(c + 1) & 1u, abort_flag));
     };
     auto increment = [&](int c, uint32_t at) {
 #pragma unroll
@@ -341,22 +359,26 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       }
     };
     auto values_of = [&](int stage, uint32_t parity) {
-      tc::mbar_wait_warp(&full[stage], parity, abort_flag);
+      if (!all(tc::mbar_wait_warp(&full[stage], parity, abort_flag))) return false;
       tc::tc_fence_after_sync();
       issue_u(smem0 + stage * (CS_STAGE >> 4));
+      return true;
     };
-    for (int c = 0; c < n_chunks; ++c) {  // (to the end also when a wait has expired)
+    for (int c = 0; c < n_chunks && landed; ++c) {
       const uint32_t at = smem0 + s * (CS_STAGE >> 4);  // the stage has landed: this warp waited for it a chunk ago
       state_product(c, at, s);
-      outputs_before(c);  // (for the increment, but here the wait is hidden behind the conversion of X; a wait for what is complete takes 130 to 250 cycles)
+      // (for the increment, but here the wait is hidden behind the conversion of X; a wait for what is complete takes 130 to 250 cycles)
+      if (!outputs_before(c)) { met = HAND_OVERS * c + NG; break; }
       new_values(c, at);
       increment(c, at);
       if (c + 1 < n_chunks) {
-        values_of(s_next, ph_next);
+        if (!values_of(s_next, ph_next)) { met = HAND_OVERS * (c + 1); break; }
         s = s_next;
         if (++s_next == CS_STAGES) { s_next = 0; ph_next ^= 1u; }
       }
     }
+#pragma unroll 1
+    for (; met < HAND_OVERS * n_chunks; ++met) tc::named_sync(hand_over(met % HAND_OVERS));
   } else if (warp == 2) {
     // ------------------------------------------------------------------ output MMA issuer: O1 = H Q^T once H K^T is
     // complete (so that it runs behind it, while the chain epilogue converts X), O2 = Vn P^T once Vn hi/lo are back
@@ -366,7 +388,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     for (int c = 0; c < n_chunks; ++c) {
       const uint32_t cp = (uint32_t)c & 1u;
       const uint32_t at = smem0 + s * (CS_STAGE >> 4);
-      tc::mbar_wait3(kh_full, cp, o1_empty, cp ^ 1u, &full[s], ph, abort_flag);
+      if (!all(tc::mbar_wait3(kh_full, cp, o1_empty, cp ^ 1u, &full[s], ph, abort_flag))) break;
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
         issue_state<CS_Q, 0>(tm + TC_O1, tm, at);
@@ -375,7 +397,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       }
       __syncwarp();
       // behind the state increment, which the recurrence waits for: side by side they would share the tensor pipe
-      tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, &dh_full[1], cp, abort_flag);
+      if (!all(tc::mbar_wait3(vn_ready, cp, o2_empty, cp ^ 1u, &dh_full[1], cp, abort_flag))) break;
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
         issue_tri<false, 0, 4, CS_REC + REC_PT>(tm + TC_O2, tm + TC_VI, at, true);  // O2 = Vn P^T
@@ -394,7 +416,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
     const int d = quarter * 32 + lane;  // row of H (d_v index)
     const uint32_t lane_addr = tm + ((uint32_t)(quarter * 32) << 16);
     const int64_t tile = ((int64_t)slot * a.Hv + h) * (int64_t)(D * D);
-    bool alive = true;
+    bool alive = true;  // every wait so far has ended with its phase complete
 
     float2 Hreg[HC / 2];  // H[d][HC*grp + 2w .. +1] = M[HC*grp + 2w .. +1][d]
     // first launch of a chain: part 0 starts from the caller's state, a later part's local chain from zero and its
@@ -425,16 +447,16 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       tc::tmem_st_wait();
       tc::tc_fence_before_sync();
       __syncwarp();
-      tc::mbar_arrive(h_ready(grp));
+      tc::mbar_arrive(h_ready(grp), alive);
     };
     publish_h();
 
     int s = 0;
     uint32_t ph = 0;
-    for (int c = 0; c < n_chunks; ++c) {  // (to the end also when a wait has expired: the chain's issuer counts on the arrivals)
+    for (int c = 0; c < n_chunks; ++c) {  // (to the end also when a wait has expired: the chain's issuer counts on the hand-overs)
       const uint32_t cp = (uint32_t)c & 1u;
       const float* scal = reinterpret_cast<const float*>(smem + s * CS_STAGE + CS_REC + REC_SCAL);
-      alive = tc::mbar_wait2(&full[s], ph, kh_full, cp, abort_flag) && alive;  // (the scale vectors come with the stage)
+      alive = all(tc::mbar_wait2(&full[s], ph, kh_full, cp, abort_flag)) && alive;  // (the scale vectors come with the stage)
       if (++s == CS_STAGES) { s = 0; ph ^= 1u; }
       tc::tc_fence_after_sync();
       {  // X_j = kx_j H k_j
@@ -455,9 +477,9 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
         tc::tmem_st_wait();
         tc::tc_fence_before_sync();
         __syncwarp();
-        tc::mbar_arrive(x_ready(grp));
+        tc::mbar_arrive(x_ready(grp), alive);
       }
-      alive = tc::mbar_wait_warp(&vn_full[grp], cp, abort_flag) && alive;
+      alive = all(tc::mbar_wait_warp(&vn_full[grp], cp, abort_flag)) && alive;
       tc::tc_fence_after_sync();
       {
         uint32_t acc[VC];
@@ -482,10 +504,10 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
           __syncwarp();
-          tc::mbar_arrive(vd_ready(grp));
+          tc::mbar_arrive(vd_ready(grp), alive);
         }
         // the Vn images of the chunk before have been read (long ago: its O2 ran beside its state's conversion)
-        alive = tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag) && alive;
+        alive = all(tc::mbar_wait_warp(o_full, cp ^ 1u, abort_flag)) && alive;
         {
           uint32_t vh[VC / 2], vl[VC / 2];
 #pragma unroll
@@ -498,10 +520,10 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
           tc::tmem_st_wait();
           tc::tc_fence_before_sync();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(vn_ready);
+          if (lane == 0 && alive) tc::mbar_arrive(vn_ready);
         }
       }
-      alive = tc::mbar_wait2(&dh_full[grp], cp, o1_done, cp, abort_flag) && alive;
+      alive = all(tc::mbar_wait2(&dh_full[grp], cp, o1_done, cp, abort_flag)) && alive;
       tc::tc_fence_after_sync();
       {
         const float decay = scal[3 * C];
@@ -557,7 +579,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
       const int64_t tok0 = sp.t0 + c * C;
       // o_full is committed by the MMA warp after it saw this chunk's stage (tiles and scale vectors) land, so it also
       // orders the scale vectors; waiting on the stage barrier here would alias phases once this warp lags a chunk
-      if (!tc::mbar_wait_warp(o_full, cp, abort_flag)) break;
+      if (!all(tc::mbar_wait_warp(o_full, cp, abort_flag))) break;
       tc::tc_fence_after_sync();
       const bool whole = !(ragged && c == n_chunks - 1);  // (behind the end of a dense batch row the copies write nothing)
       // O1 is taken whole and released at once: O1 of the next chunk is the first thing the tensor pipe runs while the chain epilogue converts X, and X's
@@ -664,7 +686,12 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
 
   tc::tc_fence_before_sync();
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag != 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+  if (*abort_flag != 0u) {  // (the roles have ended: it stays as it is)
+    if (threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, AVE_GDN_DEV_WAIT_EXPIRED);
+    if (warp == 1 || warp == 2) tc::drain_mmas(&mma_end[warp - 1]);
+    tc::tc_fence_before_sync();
+    __syncthreads();
+  }
   if (warp == 1) {
     tc::tc_fence_after_sync();
     tc::tmem_dealloc(tm, 512);

@@ -82,11 +82,24 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 
 // A hardware barrier as a hand-off: `threads` of them arrive or wait, whole warps, and those that wait go on when all are there.  30 cycles from the
 // last arrival to the first instruction behind the wait, an mbarrier 85 to 100 (alone on an SM; more beside others' shared-memory traffic).
-// A wait on it is not bounded, so it is only for roles that arrive as often as they are waited for whatever happens, bounded waits of theirs
-// that expire included.  The parity is not needed: nobody may arrive again before the waiting warps have gone on.
+// A wait on it is not bounded, so it is only for roles that come to it as often as they are waited for whatever happens, bounded waits of theirs
+// that expire included.  And nobody may arrive again before the waiting warps have gone on (the barrier counts threads and knows no parity: it
+// would complete without them), so a warp may arrive only where its own waits see to that; one whose wait has expired (`alive` false, the same for the
+// whole warp) waits with the others.
 struct NamedBar { uint32_t id, threads; };
-__device__ __forceinline__ void mbar_arrive(NamedBar b) { asm volatile("bar.arrive %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory"); }
-__device__ __forceinline__ void mbar_wait_warp(NamedBar b, uint32_t, volatile uint32_t*) { asm volatile("bar.sync %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory"); }
+__device__ __forceinline__ void named_sync(NamedBar b) { asm volatile("bar.sync %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory"); }
+__device__ __forceinline__ void mbar_arrive(NamedBar b, bool alive) {
+  if (alive) asm volatile("bar.arrive %0, %1;" ::"r"(b.id), "r"(b.threads) : "memory");
+  else named_sync(b);
+}
+__device__ __forceinline__ void mbar_wait_warp(NamedBar b, uint32_t, volatile uint32_t*) { named_sync(b); }
+
+// In front of a CTA's end, for a phase that copies or MMAs of its own complete: waited for whatever the flag says, again with a limit.
+__device__ __forceinline__ void drain(uint64_t* bar, uint32_t parity) {
+  uint32_t left = kWaitLimit;
+#pragma unroll 1
+  while (!mbar_try_wait(bar, parity) && --left != 0u) {}
+}
 
 // One lane of a converged warp; the enclosing control flow stays warp-uniform, which lets the compiler keep
 // descriptors in uniform registers for the MMA issue.
@@ -224,6 +237,12 @@ __device__ __forceinline__ void mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_
 // mbarrier arrives once every tcgen05 operation issued so far by this thread has completed
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// the same for all MMAs of this warp, whose elected lane has issued them; `bar` is used by nothing else
+__device__ __forceinline__ void drain_mmas(uint64_t* bar) {
+  if (elect_one()) mma_commit(bar);
+  __syncwarp();
+  drain(bar, 0u);
 }
 
 // ---------------------------------------------------------------- TMEM <-> registers (warp-collective; a warp reaches
