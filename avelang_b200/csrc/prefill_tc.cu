@@ -297,7 +297,7 @@ part_combine_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float*
 //   o = o_local + qt M0(part)        (qt = the transition chain's rows, [64 tokens][128 d_k])
 // is one product on tcgen05, transposed like the scan's (128 d_v lanes x 64 tokens), with both operands as bf16 hi+lo pairs (hi hi +
 // hi lo + lo hi): A = the image of M0(part), B = the qt^T images the scan wrote (MN-major, brought in by bulk copies).  The
-// accumulator is staged in the place of B, so that everything that touches global memory runs in the layout of
+// accumulator is staged in shared memory, so that everything that touches global memory runs in the layout of
 // the streaming norm kernel: a half-warp per token row, 8 adjacent features per lane, 16- and 32-byte accesses, the
 // RMS over d_v as four shuffles.  (Reading o_local and z straight from the accumulator's layout, a row or a column per
 // thread, measured three to four times slower: 2- or 4-byte accesses and tens of instructions per element.)
@@ -328,6 +328,12 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   volatile uint32_t* abort_flag = tmem_slot + 1;
   const int h = blockIdx.y, tid = threadIdx.x % FIN_GROUP, warp = tid >> 5, lane = tid & 31;  // within the group
   auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(FIN_GROUP) : "memory"); };
+  auto group_all = [&](bool x) {  // the same, with one answer for the whole group
+    int all;
+    asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n bar.red.and.pred q, %2, %3, p;\n selp.s32 %0, 1, 0, q;\n}"
+                 : "=r"(all) : "r"((int)x), "r"(1 + grp), "n"(FIN_GROUP) : "memory");
+    return all != 0;
+  };
   const int n = blockIdx.z / (plan.parts - 1), part = 1 + blockIdx.z % (plan.parts - 1);
   if (batch_rejected(a, chunk_start)) return;
   const SeqSpan sp = seq_span(a.cu_seqlens, n, a.T, nullptr);
@@ -358,7 +364,8 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
   tc::tc_fence_before_sync();
   __syncthreads();
   tc::tc_fence_after_sync();
-  if (tid == 0 && !skipped && c_begin < c_end) load_qt(from_end(c_begin));
+  int asked = 0;  // images that this group's first thread has asked for
+  if (tid == 0 && !skipped && c_begin < c_end) { load_qt(from_end(c_begin)); ++asked; }
   const uint32_t tm = *tmem_slot + 64 * grp;
   const int hw = tid >> 4, sub = tid & 15;  // streaming pass: half-warp index (16 of them) and lane inside it
   const bool gate_first = (a.flags & AVE_GDN_FLAG_GATE_FIRST) != 0;
@@ -366,10 +373,11 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     wv[i] = a.norm_weight ? make_float2(a.norm_weight[8 * sub + 2 * i], a.norm_weight[8 * sub + 2 * i + 1]) : make_float2(1.f, 1.f);
-  bool ok = true;
+  // A wait that has expired ends the group's walk: no rows from a product that is not there, no further images.
+  bool ok = true, landed = true;  // ok: the same for the whole group between its meetings
 
   int it = 0;
-  for (int i = c_begin; i < c_end; i += stride, ++it) {
+  for (int i = c_begin; i < c_end && ok; i += stride, ++it) {
     const int c = from_end(i);
     const int64_t tok0 = sp.t0 + (int64_t)c * C;
     const int rows = min(C, sp.len - c * C);
@@ -392,8 +400,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
     }
     if (!skipped) {
       if (warp == 0) {
-        bool landed = it > 0 || tc::mbar_wait_warp(m0_full, 0, abort_flag);
-        landed = landed && tc::mbar_wait_warp(q_full, (uint32_t)it & 1u, abort_flag);
+        landed = __all_sync(0xffffffffu, (it > 0 || tc::mbar_wait_warp(m0_full, 0, abort_flag)) && tc::mbar_wait_warp(q_full, (uint32_t)it & 1u, abort_flag)) != 0;
         tc::tc_fence_after_sync();
         if (landed && tc::elect_one()) {
           constexpr uint32_t idesc = tc::idesc_f16(128, 64, 1, 1, false, true);  // A K-major, B MN-major (token rows)
@@ -410,9 +417,9 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
         }
         __syncwarp();
       }
-      ok = tc::mbar_wait(mma_bar, (uint32_t)it & 1u, abort_flag) && ok;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(mma_bar, (uint32_t)it & 1u, abort_flag)) != 0;
       tc::tc_fence_after_sync();
-      if (tid == 0 && i + stride < c_end) load_qt(c - stride);  // the product has read the images
+      if (ok && tid == 0 && i + stride < c_end) { load_qt(c - stride); ++asked; }  // the product has read the images
       if (ok) {  // accumulator (a d_v row per thread, 32 tokens) -> staged token rows
         const int d = (warp & 3) * 32 + lane, first = 32 * (warp >> 2);
         uint32_t acc[32];
@@ -423,7 +430,7 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
       }
     }
     tc::tc_fence_before_sync();
-    group_sync();  // staged rows complete; the accumulator is free for the next product
+    ok = group_all(ok);  // staged rows complete; the accumulator is free for the next product
     tc::tc_fence_after_sync();
     if (ok) {
 #pragma unroll
@@ -466,6 +473,11 @@ part_finish_kernel(const AveGdnArgs a, const int32_t* chunk_start, const float* 
       }
     }
     group_sync();  // the staged rows have been read
+  }
+  if (!ok) {  // nothing of this group is on its way when the CTA ends
+    if (warp == 0 && landed) tc::drain(mma_bar, (uint32_t)(it - 1) & 1u);
+    if (tid == 0) tc::drain(q_full, (uint32_t)(asked - 1) & 1u);
+    if (threadIdx.x == 0) tc::drain(m0_full, 0u);
   }
   tc::tc_fence_before_sync();
   __syncthreads();
