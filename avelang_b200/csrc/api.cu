@@ -11,6 +11,7 @@ int launch_prefill_d64(const AveGdnArgs& a, cudaStream_t stream);
 size_t prefill_d64_workspace_bytes(const AveGdnArgs& a);
 int launch_prefill_tc(const AveGdnArgs& a, cudaStream_t stream, bool plain, const AveGdnArgs* decode);
 size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain);
+size_t prefill_tc_workspace_least(const AveGdnArgs& a);
 int prefill_tc_launch_count(const AveGdnArgs& a, bool plain);
 int prefill_tc_parts(const AveGdnArgs& a);
 int launch_gated_rmsnorm(const AveGdnNormArgs& a, cudaStream_t stream);
@@ -26,6 +27,9 @@ size_t backward_workspace_bytes(const AveGdnBwdArgs& a, int key_heads);
 
 static size_t prefill_ws_bytes(const AveGdnArgs& a) {
   return a.dk == 128 ? prefill_tc_workspace_bytes(a, false) : prefill_d64_workspace_bytes(a);
+}
+static bool prefill_ws_too_small(const AveGdnArgs& a) {
+  return a.workspace_bytes < (a.dk == 128 ? prefill_tc_workspace_least(a) : prefill_d64_workspace_bytes(a));
 }
 
 static int check_rows(const void* p, int64_t st, int64_t sh, int64_t sb, int elem_bytes) {
@@ -106,7 +110,7 @@ int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream) {
   if (rc != AVE_GDN_OK) return rc;
   if ((int64_t)args->B * args->T == 0 || args->n_seqs == 0) return AVE_GDN_OK;
   if (args->workspace == nullptr || !aligned16(args->workspace)) return AVE_GDN_INVALID_ARGUMENT;
-  if (args->workspace_bytes < prefill_ws_bytes(*args)) return AVE_GDN_WORKSPACE_TOO_SMALL;
+  if (prefill_ws_too_small(*args)) return AVE_GDN_WORKSPACE_TOO_SMALL;
   // d = 128 runs on the tcgen05 scan; d = 64 (the small CPU-reference shape) has a form of its own, with fp32 accuracy
   if (args->dk == 128) return launch_prefill_tc(*args, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
   return launch_prefill_d64(*args, reinterpret_cast<cudaStream_t>(stream));
@@ -129,7 +133,7 @@ int ave_gdn_mixed_step(const AveGdnArgs* decode, const AveGdnArgs* prefill, void
     return rc != AVE_GDN_OK ? rc : ave_gdn_chunk_prefill(prefill, stream);
   }
   if (prefill->workspace == nullptr || !aligned16(prefill->workspace)) return AVE_GDN_INVALID_ARGUMENT;
-  if (prefill->workspace_bytes < prefill_ws_bytes(*prefill)) return AVE_GDN_WORKSPACE_TOO_SMALL;
+  if (prefill_ws_too_small(*prefill)) return AVE_GDN_WORKSPACE_TOO_SMALL;
   return launch_prefill_tc(*prefill, reinterpret_cast<cudaStream_t>(stream), false, decode);
 }
 

@@ -503,55 +503,77 @@ struct WsLayout {
   int seg_begin[9];    // range i covers chunk offsets [seg_begin[i], seg_begin[i+1])
 };
 
-// `plain`: one part, one range, everything on the caller's stream (the schedule of the fixed-scratch entry point).
-WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
-  WsLayout L;
-  L.chunks = a.cu_seqlens ? (int64_t)a.T / C + a.n_seqs : (int64_t)a.B * ((a.T + C - 1) / C);
-  const size_t recs = (size_t)L.chunks * a.Hv;
-  auto up = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
-  // The longest chain is known for dense batches and for packed ones that come with the max_seqlen bound; otherwise only
-  // its bound T is.
-  const int max_chunks = ((a.cu_seqlens != nullptr && a.max_seqlen > 0 ? min(a.max_seqlen, a.T) : a.T) + C - 1) / C;
-  L.max_chunks = max_chunks;
+// The longest chain, in chunks, is known for dense batches and for packed ones that come with the max_seqlen bound; otherwise only its bound T is.
+int longest_chunks(const AveGdnArgs& a) { return ((a.cu_seqlens != nullptr && a.max_seqlen > 0 ? min(a.max_seqlen, a.T) : a.T) + C - 1) / C; }
+
+// Length of the parts after the first and of the first, in chunks.  Part 0 runs one chain and needs no fix-up, a later part runs two chains and its rows wait for
+// the fix-up, so part 0 is made PART0_X4 / 4 times as long as the others; lengths are even.
+int part_length(int chunks, int S) { return max(2, (4 * chunks / (4 * (S - 1) + PART0_X4) + 1) & ~1); }
+int first_part_length(int chunks, int S) { return S > 1 ? max(2, (chunks - (S - 1) * part_length(chunks, S) + 1) & ~1) : 0; }
+
+// Most parts whose 2S - 1 chains per head still get an SM each
+int most_parts(int64_t heads_total) {
+  const int64_t per_head = (NUM_SMS / heads_total + 1) / 2;
+  return per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
+}
+// Two parts take three chains a head.  They are taken while these leave a third of the SMs and the chains are long enough for the
+// fix-up, which with a gate also holds the later part's norms back.
+bool two_parts(int64_t heads_total, int chunks, bool gated) { return 3 * heads_total <= 2 * NUM_SMS / 3 && chunks >= (gated ? 112 : 64); }
+
+// Parts: with few chains most SMs idle while every chain walks its chunks one after the other.  Cutting the sequences into S parts that run at
+// the same time shortens the walk S-fold at the price of a second (transition) chain per later part, a combine and one GEMM-shaped fix-up.  Not
+// with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of beside it.
+int parts_wanted(const AveGdnArgs& a, bool plain) {
   const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
-  const bool push = a.o_peers != nullptr && a.n_peers > 1;
-  // Parts: with few chains most SMs idle while every chain walks its chunks one after the other.  Cutting the sequences into S parts that run at
-  // the same time shortens the walk S-fold at the price of a second (transition) chain per later part, a combine and one GEMM-shaped fix-up.  Not
-  // with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of beside it.
-  // Part 0 runs one chain and needs no fix-up, a later part runs two chains and its rows wait for the fix-up, so part 0 is made PART0_X4 / 4
-  // times as long as the others; lengths are even.
-  auto length = [&](int S) { return max(2, (4 * max_chunks / (4 * (S - 1) + PART0_X4) + 1) & ~1); };
-  auto first_length = [&](int S) { return S > 1 ? max(2, (max_chunks - (S - 1) * length(S) + 1) & ~1) : 0; };
+  const int max_chunks = longest_chunks(a);
+  if (plain || (a.o_peers != nullptr && a.n_peers > 1) || heads_total <= 0 || max_chunks < 12) return 1;
   // What a call with S parts takes beside what it takes anyway, in ns: its longest chain's steps, which get longer with the SMs that hold chains, their
   // start, the fix-up, and what goes with any.  Fitted to 1156 measurements (4 to 96 chains of 8 to 256 chunks, whole and in 2 to 16 parts, with a gate and
   // without; 3.4 % off on the mean, as good with either).
   auto cost = [&](int S) {
-    const int64_t chains = heads_total * (2 * S - 1), steps = S > 1 ? max(length(S), first_length(S)) : max_chunks;
+    const int first = first_part_length(max_chunks, S);
+    const int64_t chains = heads_total * (2 * S - 1), steps = S > 1 ? max(part_length(max_chunks, S), first) : max_chunks;
     return steps * (1870 + 34 * chains / 10) + 122 * chains + (S == 1 ? 0 : S == 2 ? 10500 : 13000 + 460 * (S - 1)) +
-           (S > 1 ? 147 * heads_total * max(0, max_chunks - first_length(S)) / 10 : 0) + 10100 + 3 * heads_total * max_chunks;
+           (S > 1 ? 147 * heads_total * max(0, max_chunks - first) / 10 : 0) + 10100 + 3 * heads_total * max_chunks;
   };
-  L.parts = 1;
-  if (!plain && !push && heads_total > 0 && max_chunks >= 12) {
-    const int64_t per_head = (NUM_SMS / heads_total + 1) / 2;  // chains per head that still get an SM each: 2S - 1
-    int most = per_head < MAX_PARTS ? (int)per_head : MAX_PARTS;
-    while (most > 1 && max_chunks / most < 2) --most;
-    int S = most;
-    for (int i = most - 1; i >= 3; --i) if (cost(i) < cost(S)) S = i;
-    if (max_chunks < 32) {  // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
-      if (most >= 2 && cost(2) < cost(S)) S = 2;
-      L.parts = S >= 2 && heads_total <= 16 && 20 * cost(S) < 19 * cost(1) ? S : 1;
-    } else if (S >= 3) {  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
-      L.parts = 20 * cost(2) < 19 * cost(S) ? 2 : S;
-    } else if (S == 2) {
-      // Two parts take three chains a head.  They are taken while these leave a third of the SMs and the chains are long enough for the
-      // fix-up, which with a gate also holds the later part's norms back.  Both lines are those of slower forms of pass 1, the combine and the fix-up, and
-      // on the safe side: two parts win at them and would win beyond (32 heads gated, whole / two: 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199;
-      // without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
-      L.parts = 3 * heads_total <= 2 * NUM_SMS / 3 && max_chunks >= (a.z != nullptr ? 112 : 64) ? 2 : 1;
-    }
+  int most = most_parts(heads_total);
+  while (most > 1 && max_chunks / most < 2) --most;
+  int S = most;
+  for (int i = most - 1; i >= 3; --i) if (cost(i) < cost(S)) S = i;
+  if (max_chunks < 32) {  // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
+    if (most >= 2 && cost(2) < cost(S)) S = 2;
+    return S >= 2 && heads_total <= 16 && 20 * cost(S) < 19 * cost(1) ? S : 1;
   }
+  if (S >= 3) return 20 * cost(2) < 19 * cost(S) ? 2 : S;  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
+  // Both lines of two parts are those of slower forms of pass 1, the combine and the fix-up: two parts win at them and would win beyond (32 heads gated, whole / two:
+  // 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199; without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
+  return S == 2 && two_parts(heads_total, max_chunks, a.z != nullptr) ? 2 : 1;
+}
+
+// The parts that a call may bring the scratch for instead, with which it then runs: the largest count with eight chunks a part or more.  Its scratch grows
+// with the length, so that a buffer for the longest of a caller's prompts serves the shorter ones; with the wanted parts four heads need 24.0 MB
+// at 20 chunks and 5.4 MB at 21.
+int parts_least(const AveGdnArgs& a, bool plain) {
+  const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
+  const int max_chunks = longest_chunks(a);
+  if (plain || (a.o_peers != nullptr && a.n_peers > 1) || heads_total <= 0 || max_chunks < 32) return 1;
+  int S = most_parts(heads_total);
+  while (S > 1 && max_chunks / S < 8) --S;
+  return S >= 3 || (S == 2 && two_parts(heads_total, max_chunks, a.z != nullptr)) ? S : 1;
+}
+
+WsLayout ws_layout_of(const AveGdnArgs& a, bool plain, int parts) {
+  WsLayout L;
+  L.chunks = a.cu_seqlens ? (int64_t)a.T / C + a.n_seqs : (int64_t)a.B * ((a.T + C - 1) / C);
+  const size_t recs = (size_t)L.chunks * a.Hv;
+  auto up = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
+  const int max_chunks = longest_chunks(a);
+  L.max_chunks = max_chunks;
+  const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
+  const bool push = a.o_peers != nullptr && a.n_peers > 1;
+  L.parts = parts;
   L.part_begin[0] = 0;
-  for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < L.parts ? first_length(L.parts) + (p - 1) * length(L.parts) : (1 << 24);
+  for (int p = 1; p <= MAX_PARTS; ++p) L.part_begin[p] = p < parts ? first_part_length(max_chunks, parts) + (p - 1) * part_length(max_chunks, parts) : (1 << 24);
   // Ranges: with the fused all-gather a launch of its own norms the rows and pushes them to every peer over NVLink, which takes about
   // as long as a chain itself; with few long chains that runs beside the chains of the next range, and only the last range's push is
   // exposed, so the ranges are equal and as many as the event pool allows.  (Without peers ranges do not pay any more: pass 1 of
@@ -583,6 +605,12 @@ WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
   return L;
 }
 
+// `plain`: one part, one range, everything on the caller's stream (the schedule of the fixed-scratch entry point).
+WsLayout ws_layout(const AveGdnArgs& a, bool plain) {
+  const WsLayout L = ws_layout_of(a, plain, parts_wanted(a, plain));
+  return plain || a.workspace == nullptr || a.workspace_bytes >= L.total ? L : ws_layout_of(a, plain, parts_least(a, plain));
+}
+
 }  // namespace
 
 int launch_decode(const AveGdnArgs& a, cudaStream_t stream);
@@ -595,7 +623,13 @@ int launch_gated_rmsnorm_f32in_batched(const AveGdnNormArgs& a, cudaStream_t str
 // 32 heads, one sequence of 203 tokens: 33.9 us with the tables, 31.3 without.
 static bool needs_tables(const AveGdnArgs& a) { return a.cu_seqlens != nullptr && (int64_t)a.n_seqs * a.Hv > NUM_SMS; }
 
-size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain) { return ws_layout(a, plain).total; }
+// What a caller is told to bring, and what a call is refused below
+size_t prefill_tc_workspace_bytes(const AveGdnArgs& a, bool plain) {
+  return max(ws_layout_of(a, plain, parts_wanted(a, plain)).total, ws_layout_of(a, plain, parts_least(a, plain)).total);
+}
+size_t prefill_tc_workspace_least(const AveGdnArgs& a) {
+  return min(ws_layout_of(a, false, parts_wanted(a, false)).total, ws_layout_of(a, false, parts_least(a, false)).total);
+}
 
 int prefill_tc_parts(const AveGdnArgs& a) { return ws_layout(a, false).parts; }
 

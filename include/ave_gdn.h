@@ -112,9 +112,11 @@ typedef struct AveGdnArgs {
 
 /* Chunked prefill (chunk 64, WY/UT form), dense [B,T] or packed varlen via cu_seqlens. */
 int ave_gdn_chunk_prefill(const AveGdnArgs* args, void* stream);
+/* Scratch of a prefill.  What it answers for the longest of a caller's sequences, everything else the same, is enough for the
+ * shorter ones too: a call whose own best schedule would want more runs with fewer parts. */
 size_t ave_gdn_prefill_workspace_bytes(const AveGdnArgs* args);
 /* Number of kernels one ave_gdn_chunk_prefill call with these arguments enqueues (a pure function of the shapes and of
- * which optional tensors are present; no device needed).  0 for invalid arguments. */
+ * which optional tensors are present, and of workspace_bytes where `workspace` is set; no device needed).  0 for invalid arguments. */
 int ave_gdn_prefill_launch_count(const AveGdnArgs* args);
 /* Number of parts the schedule cuts a sequence of the longest length into, which are scanned at the same time (1: whole
  * chains); like the launch count a pure function of the arguments.  0 for invalid arguments. */
