@@ -520,36 +520,6 @@ int most_parts(int64_t heads_total) {
 // fix-up, which with a gate also holds the later part's norms back.
 bool two_parts(int64_t heads_total, int chunks, bool gated) { return 3 * heads_total <= 2 * NUM_SMS / 3 && chunks >= (gated ? 112 : 64); }
 
-// Parts: with few chains most SMs idle while every chain walks its chunks one after the other.  Cutting the sequences into S parts that run at
-// the same time shortens the walk S-fold at the price of a second (transition) chain per later part, a combine and one GEMM-shaped fix-up.  Not
-// with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of beside it.
-int parts_wanted(const AveGdnArgs& a, bool plain) {
-  const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
-  const int max_chunks = longest_chunks(a);
-  if (plain || (a.o_peers != nullptr && a.n_peers > 1) || heads_total <= 0 || max_chunks < 12) return 1;
-  // What a call with S parts takes beside what it takes anyway, in ns: its longest chain's steps, which get longer with the SMs that hold chains, their
-  // start, the fix-up, and what goes with any.  Fitted to 1156 measurements (4 to 96 chains of 8 to 256 chunks, whole and in 2 to 16 parts, with a gate and
-  // without; 3.4 % off on the mean, as good with either).
-  auto cost = [&](int S) {
-    const int first = first_part_length(max_chunks, S);
-    const int64_t chains = heads_total * (2 * S - 1), steps = S > 1 ? max(part_length(max_chunks, S), first) : max_chunks;
-    return steps * (1870 + 34 * chains / 10) + 122 * chains + (S == 1 ? 0 : S == 2 ? 10500 : 13000 + 460 * (S - 1)) +
-           (S > 1 ? 147 * heads_total * max(0, max_chunks - first) / 10 : 0) + 10100 + 3 * heads_total * max_chunks;
-  };
-  int most = most_parts(heads_total);
-  while (most > 1 && max_chunks / most < 2) --most;
-  int S = most;
-  for (int i = most - 1; i >= 3; --i) if (cost(i) < cost(S)) S = i;
-  if (max_chunks < 32) {  // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
-    if (most >= 2 && cost(2) < cost(S)) S = 2;
-    return S >= 2 && heads_total <= 16 && 20 * cost(S) < 19 * cost(1) ? S : 1;
-  }
-  if (S >= 3) return 20 * cost(2) < 19 * cost(S) ? 2 : S;  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
-  // Both lines of two parts are those of slower forms of pass 1, the combine and the fix-up: two parts win at them and would win beyond (32 heads gated, whole / two:
-  // 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199; without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
-  return S == 2 && two_parts(heads_total, max_chunks, a.z != nullptr) ? 2 : 1;
-}
-
 // The parts that a call may bring the scratch for instead, with which it then runs: the largest count with eight chunks a part or more.  Its scratch grows
 // with the length, so that a buffer for the longest of a caller's prompts serves the shorter ones; with the wanted parts four heads need 24.0 MB
 // at 20 chunks and 5.4 MB at 21.
@@ -560,6 +530,45 @@ int parts_least(const AveGdnArgs& a, bool plain) {
   int S = most_parts(heads_total);
   while (S > 1 && max_chunks / S < 8) --S;
   return S >= 3 || (S == 2 && two_parts(heads_total, max_chunks, a.z != nullptr)) ? S : 1;
+}
+
+// Parts: with few chains most SMs idle while every chain walks its chunks one after the other.  Cutting the sequences into S parts that run at
+// the same time shortens the walk S-fold at the price of a second (transition) chain per later part, a combine and one GEMM-shaped fix-up.  Not
+// with the fused all-gather: there the fix-up would push most rows to the peers after the scan instead of beside it.
+int parts_wanted(const AveGdnArgs& a, bool plain) {
+  const int64_t heads_total = (int64_t)a.n_seqs * a.Hv;
+  const int max_chunks = longest_chunks(a);
+  if (plain || (a.o_peers != nullptr && a.n_peers > 1) || heads_total <= 0 || max_chunks < 12) return 1;
+  // What a call with S parts takes beside what it takes anyway, in ns: its longest chain's steps, which get longer with the SMs that hold chains, their
+  // start, the fix-up, and what goes with any.  Fitted to 1156 measurements (4 to 96 chains of 8 to 256 chunks, whole and in 2 to 16 parts, with a gate and
+  // without; 3.4 % off on the mean, as good with either).
+  auto scan = [&](int S) {
+    const int64_t chains = heads_total * (2 * S - 1), steps = S > 1 ? max(part_length(max_chunks, S), first_part_length(max_chunks, S)) : max_chunks;
+    return steps * (1870 + 34 * chains / 10) + 122 * chains;
+  };
+  auto cost = [&](int S) {
+    return scan(S) + (S == 1 ? 0 : S == 2 ? 10500 : 13000 + 460 * (S - 1)) +
+           (S > 1 ? 147 * heads_total * max(0, max_chunks - first_part_length(max_chunks, S)) / 10 : 0) + 10100 + 3 * heads_total * max_chunks;
+  };
+  int most = most_parts(heads_total);
+  while (most > 1 && max_chunks / most < 2) --most;
+  int S = most;
+  for (int i = most - 1; i >= 3; --i) if (cost(i) < cost(S)) S = i;
+  if (max_chunks < 32) {
+    // Of several packed sequences without a bound only the sum is known.  Each may end inside the first part or soon behind it, and what parts take beside
+    // the scan is paid for nothing (whole / parts: 3 x 650 tokens x 4 heads gated 37.8 / 52.6 us, 2 x 975 x 8 51.7 / 59.8; 1853 and 97 x 4 69.8 / 53.7, with its bound 56).
+    if (a.cu_seqlens != nullptr && a.n_seqs > 1 && a.max_seqlen <= 0) return 1;
+    // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
+    if (most >= 2 && cost(2) < cost(S)) S = 2;
+    if (S < 2 || heads_total > 16 || 20 * cost(S) >= 19 * cost(1)) S = 1;
+  } else if (S >= 3) {  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
+    if (20 * cost(2) < 19 * cost(S)) S = 2;
+  } else if (S == 2 && !two_parts(heads_total, max_chunks, a.z != nullptr)) {
+    // Both lines of two parts are those of slower forms of pass 1, the combine and the fix-up: two parts win at them and would win beyond (32 heads gated, whole / two:
+    // 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199; without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
+    S = 1;
+  }
+  return max(S, 1);
 }
 
 WsLayout ws_layout_of(const AveGdnArgs& a, bool plain, int parts) {
