@@ -568,6 +568,11 @@ int parts_wanted(const AveGdnArgs& a, bool plain) {
     // 2048 tokens 96.1 / 86.5 us, 4096 176 / 141, 6144 258 / 199; without a gate 2048 79.7 / 77.0; 48 heads x 8192 gated 382 / 318).
     S = 1;
   }
+  // The single tokens of a mixed step stream their states, 64 KB in and out in about 1.75 us an SM, through the SMs that the chains leave, and the fix-up finds no
+  // room before they are through.  Where they take longer than the scan, not more parts than by the rule above (without the gate, parts / not: 16
+  // heads, 200 single tokens and a prompt of 1700 123 / 99 us, 8 heads, 200 and 1200 74 / 57; 8 heads, 200 and 2500, six parts / five 88 / 81).
+  const int least = parts_least(a, plain);
+  if (least < S && (int64_t)a.token_begin * a.Hv * 1750 > scan(S) * (NUM_SMS - heads_total * (2 * S - 1))) S = least;
   return max(S, 1);
 }
 

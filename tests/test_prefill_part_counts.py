@@ -32,6 +32,11 @@ def test_short_packed_sequences_without_a_bound_stay_whole(built_lib, T, heads, 
     assert _parts(1, 2048, heads, seqs=seqs) > 1
 
 
+@pytest.mark.parametrize("heads, singles, prompt, parts", [(16, 200, 1700, 1), (8, 200, 1200, 1), (8, 200, 2500, 5), (4, 200, 1700, 5), (4, 64, 1500, 7)])
+def test_a_mixed_steps_single_tokens_are_not_held_up(built_lib, heads, singles, prompt, parts):
+    assert _parts(1, singles + prompt, heads, seqs=1, singles=singles) == parts
+
+
 @pytest.mark.parametrize("gated", [False, True])
 def test_every_chain_gets_an_sm(built_lib, gated):
     for heads in (2, 4, 6, 8, 12, 16, 24, 32, 48, 50, 74, 148, 200):
