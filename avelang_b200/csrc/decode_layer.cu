@@ -8,11 +8,12 @@
 // is that of the slot-pool decode kernel: persistent CTAs, the next 64 KiB tile lands in shared memory through a bulk
 // copy while the current one is reduced, updated and streamed out of registers.  A unit is a (sequence, key head); a CTA walks the value
 // heads that share it back to back: q and k are convolved and their history shifted once, by the one CTA that reads them, which is what
-// makes the in-place history update free of races.  CTAs come in clusters of two, which take units in turn; where a cluster's number of units is
-// odd, the two share the last one, half of its value heads each: both read the q and k history, and one shifts it behind a cluster
-// barrier.  The busiest CTA then has 7 tiles where 64 sequences x 16 key heads left it 8 of 6.9 on the mean, and one sequence is twice as many CTAs.
-// A layer with both projections, 32 value heads: 64 sequences 85.0 -> 82.4 us, 1: 32.2 -> 30.4, 9: 37.0 -> 34.5, 20: 51.5 -> 48.2, 100: 116.3 ->
-// 113.4; where the units come out even nothing changes (37: 58.6 and 58.8, 256: 230).
+// makes the in-place history update free of races.  Where the busiest CTA then has fewer tiles, CTAs come in clusters of two, which take units in turn; where a
+// cluster's number of units is odd, the two share the last one, half of its value heads each: both read the q and k history, and one shifts it behind a cluster
+// barrier.  The busiest CTA has 7 tiles where 64 sequences x 16 key heads leave it 8 of 6.9 on the mean, and one sequence is twice as many CTAs.
+// This kernel, 32 value heads, without / with pairs: 1 sequence 9.1 / 6.6 us, 9 12.1 / 8.7, 20 19.8 / 17.7, 64 55.5 / 54.5, 100 83.3 / 82.5.  Elsewhere a cluster only
+// costs (37 sequences x 1 head 5.8 / 6.5, 5 x 16 heads of a key head each 7.1 / 7.3, 64 x 16 24.2 / 24.6, 64 x 4 key heads of eight 51.4 / 52.9), and so does code that could do both
+// (28 sequences 23.1 / 26): the two forms are kernels of their own.
 // Rounding points are those of the separate kernels (convolution outputs are rounded to bf16, g and beta stay fp32), so
 // the fused step leaves the states and histories that conv1d_update + gate_beta + decode_step leave, bit for bit.
 #include "common.cuh"
@@ -23,7 +24,7 @@ namespace {
 
 constexpr int DK = 128, DV = 128, WARPS = 8, ROWS = DK / WARPS;  // rows of the tile per warp; a lane owns 4 columns
 
-template <int WIDTH>
+template <int WIDTH, int pairs>
 __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDecodeLayerArgs a, int n_units) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   float* tile_s = reinterpret_cast<float*>(dyn_smem);  // [DK][DV] fp32
@@ -51,13 +52,14 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
     tc::fence_barrier_init();
   }
   pdl_wait();
-  // this cluster's units: cluster, cluster + clusters, ...; CTA `rank` takes every second of them, and its part of the last of an odd number
-  const int clusters = gridDim.x >> 1, cluster = blockIdx.x >> 1, rank = blockIdx.x & 1;
-  const int n_mine = (n_units - cluster + clusters - 1) / clusters, own = (n_mine >> 1) * r, half = (r + 1) >> 1;  // (own: tiles of whole units)
-  const bool shared = (n_mine & 1) != 0 && r > 1;  // the last unit is walked by both
-  const int n_local = own + ((n_mine & 1) == 0 ? 0 : r == 1 ? (rank == 0 ? 1 : 0) : rank == 0 ? half : r - half);
+  // This cluster's units: cluster, cluster + clusters, ...; with pairs, CTA `rank` takes every second of them, and its part of the last of an odd number.
+  // (Without, a CTA is a cluster of its own.)
+  const int clusters = gridDim.x >> pairs, cluster = blockIdx.x >> pairs, rank = blockIdx.x & pairs;
+  const int n_mine = (n_units - cluster + clusters - 1) / clusters, own = (n_mine >> pairs) * r, half = (r + 1) >> 1;  // (own: tiles of whole units)
+  const bool shared = (n_mine & pairs) != 0;  // the last unit is walked by both
+  const int n_local = own + (!shared ? 0 : rank == 0 ? half : r - half);
   if (n_local == 0) return;
-  auto unit_of = [&](int i) { return cluster + (i < own ? 2 * (i / r) + rank : n_mine - 1) * clusters; };
+  auto unit_of = [&](int i) { return cluster + (i < own ? ((i / r) << pairs) + rank : n_mine - 1) * clusters; };
   auto head_of = [&](int i) { return i < own ? i % r : i - own + rank * half; };  // among the value heads of the unit
   auto slot_of_seq = [&](int n) -> int {  // < 0: the sequence is skipped
     int slot = a.state_indices ? a.state_indices[n] : n;
@@ -218,28 +220,34 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
 int launch_decode_layer(const AveGdnDecodeLayerArgs& a, cudaStream_t stream) {
   const int units = a.n_seqs * a.Hk;
   if (units == 0) return AVE_GDN_OK;
+  using Kernel = void (*)(const AveGdnDecodeLayerArgs, int);
+  static constexpr Kernel kernels[3][2] = {{gdn_decode_layer_kernel<2, 0>, gdn_decode_layer_kernel<2, 1>},
+                                           {gdn_decode_layer_kernel<3, 0>, gdn_decode_layer_kernel<3, 1>},
+                                           {gdn_decode_layer_kernel<4, 0>, gdn_decode_layer_kernel<4, 1>}};
   static bool attr_set_dev[64] = {};
   int dev = 0, sms = 148;
   AVE_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return AVE_GDN_UNSUPPORTED;
   if (!attr_set_dev[dev]) {
-    AVE_CUDA_TRY(cudaFuncSetAttribute(gdn_decode_layer_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, DK * DV * 4));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(gdn_decode_layer_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, DK * DV * 4));
-    AVE_CUDA_TRY(cudaFuncSetAttribute(gdn_decode_layer_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, DK * DV * 4));
-    attr_set_dev[dev] = true;  // repeating the three calls from another thread is harmless
+    for (const auto& of_width : kernels)
+      for (const auto kernel : of_width) AVE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DK * DV * 4));
+    attr_set_dev[dev] = true;  // repeating the calls from another thread is harmless
   }
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (a.width < 2 || a.width > 4) return AVE_GDN_UNSUPPORTED;
-  const auto kernel = a.width == 2 ? gdn_decode_layer_kernel<2> : a.width == 3 ? gdn_decode_layer_kernel<3> : gdn_decode_layer_kernel<4>;
+  // tiles of the busiest CTA, alone and in pairs
+  const int r = a.Hv / a.Hk, ctas = units < 2 * sms ? units : 2 * sms, clusters = units < sms ? units : sms;
+  const int alone = (units + ctas - 1) / ctas * r, most = (units + clusters - 1) / clusters, paired = (most >> 1) * r + ((most & 1) != 0 ? (r + 1) >> 1 : 0);
+  const int pairs = r > 1 && paired < alone ? 1 : 0;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.gridDim = dim3((unsigned)(2 * (units < sms ? units : sms))); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = DK * DV * 4; cfg.stream = stream;
-  cfg.attrs = at; cfg.numAttrs = 2;
-  AVE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, a, units));
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = 2; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(pairs != 0 ? 2 * clusters : ctas)); cfg.blockDim = dim3(256); cfg.dynamicSmemBytes = DK * DV * 4; cfg.stream = stream;
+  cfg.attrs = at; cfg.numAttrs = 1 + pairs;
+  AVE_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernels[a.width - 2][pairs], a, units));
   AVE_CUDA_TRY(cudaGetLastError());
   return AVE_GDN_OK;
 }
