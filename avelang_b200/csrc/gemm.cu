@@ -80,7 +80,7 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
         const TileCoord tcd = tile_coord(tile, mt, nt);
         for (int kb = 0; kb < kb_count; ++kb) {
-          if (!tc::mbar_wait(&empty[s], ph ^ 1u, abort_flag)) goto producer_done;
+          if (!tc::mbar_wait_unrolled(&empty[s], ph ^ 1u, abort_flag)) goto producer_done;
           tc::mbar_expect_tx(&full[s], (uint32_t)(A_BYTES + bn * BK * 2));
           tc::tma_load_2d(smem + s * STAGE_BYTES, &tmA, &full[s], kb * BK, tcd.m * BM);
           tc::tma_load_2d(smem + s * STAGE_BYTES + A_BYTES, &tmB, &full[s], kb * BK, tcd.n * bn);
@@ -96,12 +96,12 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         const uint32_t idesc = tc::idesc_f16(BM, bn, 1, 1, false, false);
         const int buf = local & 1;
         const uint32_t acc_ph = (uint32_t)(local >> 1) & 1u;
-        if (!tc::mbar_wait(&acc_empty[buf], acc_ph ^ 1u, abort_flag)) break;
+        if (!tc::mbar_wait_unrolled(&acc_empty[buf], acc_ph ^ 1u, abort_flag)) break;
         tc::tc_fence_after_sync();
         const uint32_t d = tmem_base + (uint32_t)buf * BN;
         bool ok = true;
         for (int kb = 0; kb < kb_count; ++kb) {
-          if (!tc::mbar_wait(&full[s], ph, abort_flag)) { ok = false; break; }
+          if (!tc::mbar_wait_unrolled(&full[s], ph, abort_flag)) { ok = false; break; }
           tc::tc_fence_after_sync();
           const uint32_t a_addr = tc::smem_u32(smem + s * STAGE_BYTES);
           const uint32_t b_addr = a_addr + A_BYTES;
@@ -124,7 +124,7 @@ gemm_bf16_nt_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       const TileCoord tcd = tile_coord(tile, mt, nt);
       const int buf = local & 1;
       const uint32_t acc_ph = (uint32_t)(local >> 1) & 1u;
-      if (!tc::mbar_wait(&acc_full[buf], acc_ph, abort_flag)) break;
+      if (!tc::mbar_wait_unrolled(&acc_full[buf], acc_ph, abort_flag)) break;
       tc::tc_fence_after_sync();
       const int64_t row = (int64_t)tcd.m * BM + quarter * 32 + lane;
       __nv_bfloat16* crow = C + row * ldc + (int64_t)tcd.n * bn;
@@ -267,7 +267,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   if (warp == 0) {
     int s = 0; uint32_t ph = 0;
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!tc::mbar_wait_warp(&empty[s], ph ^ 1u, &abort_flag)) break;
+      if (!tc::mbar_wait_unrolled(&empty[s], ph ^ 1u, &abort_flag)) break;
       if (tc::elect_one()) {
         uint8_t* st = smem + s * stage_bytes;
         tc::mbar_expect_tx(&full[s], (uint32_t)stage_bytes);
@@ -282,7 +282,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     int s = 0; uint32_t ph = 0;
     bool ok = true;
     for (int kb = kb0; kb < kb1; ++kb) {
-      if (!tc::mbar_wait_warp(&full[s], ph, &abort_flag)) { ok = false; break; }
+      if (!tc::mbar_wait_unrolled(&full[s], ph, &abort_flag)) { ok = false; break; }
       tc::tc_fence_after_sync();
       if (tc::elect_one()) {
         // with fewer than 128 rows in the A tile the MMA reads whatever lies behind it: those lanes are never read back
@@ -303,7 +303,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   }
   __syncwarp();  // the other lanes of the issuing warps must not poll beside them
   // the accumulator is complete, so every operand tile has landed and been read
-  const bool ok = tc::mbar_wait(&acc_full, 0, &abort_flag);
+  const bool ok = tc::mbar_wait_unrolled(&acc_full, 0, &abort_flag);
   tc::tc_fence_after_sync();
   __syncwarp();
   tc::cluster_sync();  // ... in every CTA of the cluster: the rings may be overwritten

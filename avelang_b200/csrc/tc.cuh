@@ -49,6 +49,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
+// The same in a loop that the compiler unrolls and that looks for the flag at every 64th poll, for the GEMM, whose few roles have the room: 4096^3 108.7 us
+// with the other, 106.4 with this, 1000 x 12352 x 2048 42.8 and 42.3.
+__device__ __forceinline__ bool mbar_wait_unrolled(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((it & 63u) == 63u && *abort_flag != 0u) return false;
+  }
+  *abort_flag = 1u;
+  return false;
+}
+
 // Bounded waits for two or three phases at once.  The polls are independent, so the latencies of phases that are
 // already complete overlap instead of adding up.
 __device__ __forceinline__ bool mbar_wait2(uint64_t* b0, uint32_t p0, uint64_t* b1, uint32_t p1, volatile uint32_t* abort_flag) {
