@@ -11,7 +11,7 @@
 // makes the in-place history update free of races.  Where the busiest CTA then has fewer tiles, CTAs come in clusters of two, which take units in turn; where a
 // cluster's number of units is odd, the two share the last one, half of its value heads each: both read the q and k history, and one shifts it behind a cluster
 // barrier.  The busiest CTA has 7 tiles where 64 sequences x 16 key heads leave it 8 of 6.9 on the mean, and one sequence is twice as many CTAs.
-// This kernel, 32 value heads, without / with pairs: 1 sequence 9.1 / 6.6 us, 9 12.1 / 8.7, 20 19.8 / 17.7, 64 55.5 / 54.5, 100 83.3 / 82.5.  Elsewhere a cluster only
+// This kernel, 32 value heads, without / with pairs: 1 sequence 9.0 / 6.9 us, 9 12.0 / 8.5, 20 19.5 / 17.0, 64 55.2 / 52.8, 100 83.0 / 81.3.  Elsewhere a cluster only
 // costs (37 sequences x 1 head 5.8 / 6.5, 5 x 16 heads of a key head each 7.1 / 7.3, 64 x 16 24.2 / 24.6, 64 x 4 key heads of eight 51.4 / 52.9), and so does code that could do both
 // (28 sequences 23.1 / 26): the two forms are kernels of their own.
 // Rounding points are those of the separate kernels (convolution outputs are rounded to bf16, g and beta stay fp32), so
@@ -56,10 +56,10 @@ __global__ void __launch_bounds__(256, 2) gdn_decode_layer_kernel(const AveGdnDe
   // (Without, a CTA is a cluster of its own.)
   const int clusters = gridDim.x >> pairs, cluster = blockIdx.x >> pairs, rank = blockIdx.x & pairs;
   const int n_mine = (n_units - cluster + clusters - 1) / clusters, own = (n_mine >> pairs) * r, half = (r + 1) >> 1;  // (own: tiles of whole units)
-  const bool shared = (n_mine & pairs) != 0;  // the last unit is walked by both
+  const bool shared = (n_mine & pairs) != 0 && r > 1;  // the last unit is walked by both (pairs imply r > 1; said here, 64 sequences take 52.8 us, and 53.7 otherwise)
   const int n_local = own + (!shared ? 0 : rank == 0 ? half : r - half);
   if (n_local == 0) return;
-  auto unit_of = [&](int i) { return cluster + (i < own ? ((i / r) << pairs) + rank : n_mine - 1) * clusters; };
+  auto unit_of = [&](int i) { return cluster + (i < own ? (1 + pairs) * (i / r) + rank : n_mine - 1) * clusters; };
   auto head_of = [&](int i) { return i < own ? i % r : i - own + rank * half; };  // among the value heads of the unit
   auto slot_of_seq = [&](int n) -> int {  // < 0: the sequence is skipped
     int slot = a.state_indices ? a.state_indices[n] : n;

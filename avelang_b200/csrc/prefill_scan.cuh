@@ -12,9 +12,9 @@
 // A step takes 3.9 to 4.2 k cycles, of which the tensor pipe is busy 2.4 k: H K^T 0.85 k, X 0.55 k, its product 0.45 k, Vd 0.35 k, the increment
 // 0.7 k, the new state 0.7 k, each of them about a third hand-over (arrival or commit, wake-up, first load).  What it took to get there from 4.55 k
 // (8192 tokens x 32 heads 313 -> 260 us, 4 heads x 32768 212 -> 186, 262144 packed tokens 4.17 -> 3.75 ms, all with everything around the scan):
-//   - the code of all roles fits the 32 KB of the SM's instruction cache.  It was 44 KB (rolled waits, outputs in a rolled loop, descriptors from
-//     constants and roles that the compiler knows to be uniform took it down), every step fetched 116 lines of 128 bytes, 40 now, from the cache that the SMs of a GPC
-//     share, and chains ran up to a third slower where more of a GPC's SMs held one;
+//   - the code that a step runs fits the 32 KB of the SM's instruction cache (rolled waits, outputs in a rolled loop, descriptors from constants and roles that the
+//     compiler knows to be uniform took the kernel from 83 to 67 KB): every step fetched 116 lines of 128 bytes, 40 now, from the cache that the SMs of a GPC share, and
+//     chains ran up to a third slower where more of a GPC's SMs held one;
 //   - the two groups of epilogue warps hand over by halves: a group's tokens of X and Vd, and features of the state, have barriers of their own, so
 //     that the products begin with one half while the other is converted, and an increment's first features are taken while the rest is formed;
 //   - arrivals that the chain waits for are hardware barriers (30 cycles, an mbarrier 85 to 250);
@@ -121,7 +121,7 @@ chunk_scan_kernel(const AveGdnArgs a, const __grid_constant__ GdnMaps maps, cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  // (a shuffle, so that the compiler knows a role's code to be uniform: an MMA takes 6 instructions then, and 18 with descriptors in vector registers)
+  // (a shuffle, so that the compiler knows a role's code to be uniform)
   const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // what reads nothing that a launch before wrote comes in front of the wait for it
   if (threadIdx.x == 0) {

@@ -558,7 +558,8 @@ int parts_wanted(const AveGdnArgs& a, bool plain) {
     // Of several packed sequences without a bound only the sum is known.  Each may end inside the first part or soon behind it, and what parts take beside
     // the scan is paid for nothing (whole / parts: 3 x 650 tokens x 4 heads gated 37.8 / 52.6 us, 2 x 975 x 8 51.7 / 59.8; 1853 and 97 x 4 69.8 / 53.7, with its bound 56).
     if (a.cu_seqlens != nullptr && a.n_seqs > 1 && a.max_seqlen <= 0) return 1;
-    // short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0)
+    // Short chains: two parts as well, and whole unless parts are clearly ahead (4 heads x 1024 tokens 45.8 -> 40.0 us, 16 x 1536 65.7 -> 58.0).  Not beyond 16 chains: at
+    // 24 two parts win only with a gate, and not always (whole / two, 1536 tokens 74 / 67 us, without a gate 58 / 57; 1024 55 / 56 and 43 / 48).
     if (most >= 2 && cost(2) < cost(S)) S = 2;
     if (S < 2 || heads_total > 16 || 20 * cost(S) >= 19 * cost(1)) S = 1;
   } else if (S >= 3) {  // two only where clearly ahead (24 heads x 2048 tokens 88.6 -> 82.4; 8 heads x 6144 tokens 103 with nine parts, 92.9 with eight)
